@@ -66,6 +66,7 @@ SIGNATURES = {
 }
 
 _lib = None
+_host = None
 
 
 class NativeError(RuntimeError):
@@ -97,3 +98,21 @@ def check(stage: str, status: int) -> None:
         L = lib()
         detail = L.tg_last_error().decode() or L.tg_status_string(status).decode()
         raise NativeError(stage, status, detail)
+
+
+def host():
+    """The compiled host path (``_tg_torch``), bound to the library of ``lib()``.  Raises if it has not been built."""
+    global _host
+    if _host is None:
+        lib()
+        try:
+            from . import _tg_torch as module
+        except ImportError as e:
+            raise RuntimeError("trigrad_b200/_tg_torch is missing or does not fit this torch: build it first "
+                               "(python -m trigrad_b200.build). trigrad_b200 has no CPU or PyTorch fallback.") from e
+        from .util import create_check
+        import torch
+
+        module.bind(LIB_PATH, NativeError, create_check("cuda", torch.float32))
+        _host = module
+    return _host

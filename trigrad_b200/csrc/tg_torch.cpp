@@ -1,0 +1,790 @@
+// Host path of the Python entry points: argument checks, allocations, the per-stream state and the autograd nodes, in
+// C++ over the C ABI of include/trigrad_b200.h.
+//
+// A small render is over in 40 us on the GPU; issued from Python (a dozen torch.empty calls, a ctypes call with 31
+// arguments, a Python autograd Function whose backward has to take the interpreter lock in the engine's thread) one
+// pass of it took 100 us forward only and 360 us with gradients.  Here one call does all of it, without the lock.
+//
+// The kernels are reached through the shared library that trigrad_b200/_native.py loads (bind() gets its path), so this
+// module holds no device code.
+#include <dlfcn.h>
+
+#include <list>
+#include <memory>
+#include <mutex>
+#include <tuple>
+#include <vector>
+
+#include <ATen/Parallel.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/saved_variable.h>
+#include <torch/extension.h>
+
+#include "../../include/trigrad_b200.h"
+
+namespace py = pybind11;
+using at::Tensor;
+using torch::autograd::Node;
+using torch::autograd::SavedVariable;
+using torch::autograd::variable_list;
+
+namespace {
+
+// ---- the library ---------------------------------------------------------------------------------------------------
+struct Api {
+#define TG_FN(name) decltype(&tg_##name) name = nullptr;
+#define TG_FUNCTIONS(F)                                                                                              \
+    F(last_error) F(status_string) F(selection_planes) F(forward_workspace_bytes) F(render_forward)                  \
+    F(render_step_l2) F(backward_scratch_bytes) F(blend_backward) F(blend_backward_corrected) F(blend_backward_l2)   \
+    F(blend_backward_l2_u8) F(unpack_gradients) F(unpack_gradients_rgba) F(project) F(project_backward)              \
+    F(project_clip) F(project_clip_backward) F(unpack_project_backward) F(pack_inputs)
+    TG_FUNCTIONS(TG_FN)
+#undef TG_FN
+};
+Api g;
+PyObject* g_native_error = nullptr;   // trigrad_b200._native.NativeError
+PyObject* g_check_tensor = nullptr;   // trigrad_b200.util check, called to raise the error of a failed check
+
+void bind(const std::string& path, py::object native_error, py::object check_tensor) {
+    void* h = dlopen(path.c_str(), RTLD_NOW | RTLD_LOCAL);
+    if (!h) throw std::runtime_error(std::string("cannot load ") + path + ": " + dlerror());
+#define TG_FN(name)                                                                             \
+    g.name = reinterpret_cast<decltype(&tg_##name)>(dlsym(h, "tg_" #name));                      \
+    if (!g.name) throw std::runtime_error(path + " does not export tg_" #name);
+    TG_FUNCTIONS(TG_FN)
+#undef TG_FN
+    g_native_error = native_error.release().ptr();
+    g_check_tensor = check_tensor.release().ptr();
+}
+
+// A failed library call, thrown without the interpreter lock and translated into NativeError where the lock is held.
+// A std::runtime_error, so that the autograd engine reports it as a RuntimeError (NativeError's base) as well.
+struct LibraryError : std::runtime_error {
+    std::string stage, detail;
+    int status;
+    LibraryError(const char* s, int st, const std::string& d)
+        : std::runtime_error(std::string("trigrad_b200 ") + s + " failed: status " + std::to_string(st) + " (" + d + ")"),
+          stage(s), detail(d), status(st) {}
+};
+void check(const char* stage, int status) {
+    if (status == TG_OK) return;
+    std::string detail = g.last_error();
+    if (detail.empty()) detail = g.status_string(status);
+    throw LibraryError(stage, status, detail);
+}
+
+// ---- argument checks -----------------------------------------------------------------------------------------------
+// Device, dtype, then shape; the error itself (type and text) is raised by the Python helper.  Needs the lock.
+void need(const Tensor& t, const char* name, std::initializer_list<int64_t> shape, at::ScalarType type = at::kFloat) {
+    if (t.is_cuda() && t.scalar_type() == type && t.sizes() == at::IntArrayRef(shape.begin(), shape.size())) return;
+    py::tuple want(shape.size());
+    size_t k = 0;
+    for (int64_t s : shape) want[k++] = py::int_(s);
+    const char* dt = type == at::kFloat ? "float32" : type == at::kInt ? "int32" : "uint8";
+    py::reinterpret_borrow<py::object>(g_check_tensor)(t, name, want, py::module_::import("torch").attr(dt));
+    throw py::value_error(std::string(name) + ": wrong tensor");
+}
+// First dimension of a matrix argument (what `n, _ = t.shape` gives).
+int64_t rows(const Tensor& t, const char* name) {
+    if (t.dim() != 2) throw py::value_error(std::string(name) + " must have two dimensions");
+    return t.size(0);
+}
+int need_int(int64_t v) {
+    TORCH_CHECK(v >= 0 && v <= INT32_MAX, "size out of range");
+    return (int)v;
+}
+void need_tile(int tw, int th) {
+    if ((int64_t)tw * th > 1024) throw py::value_error("tile_width * tile_height must be <= 1024");
+}
+
+template <class T>
+T* data(const Tensor& t) { return t.defined() ? static_cast<T*>(t.data_ptr()) : nullptr; }
+
+// ---- per (device, stream) state ------------------------------------------------------------------------------------
+// Workspace, pinned read-back slots and the estimate of the number of list entries.  `use` is held while a forward call
+// issues its work: two threads that render on one stream take turns (the workspace holds one render's lists).
+struct DeviceState {
+    static constexpr int kSlots = 256;
+    std::mutex use;
+    Tensor workspace, info;      // info [slots,4] int32 pinned: K, longest list, error word, -
+    int slot = 0, last_slot = -1;
+    int64_t k_estimate = 0;
+
+    explicit DeviceState(at::Device device) {
+        workspace = at::empty({0}, at::TensorOptions().dtype(at::kByte).device(device));
+        info = at::zeros({kSlots, 4}, at::TensorOptions().dtype(at::kInt)).pin_memory();
+    }
+    int32_t* words(int s) { return info.data_ptr<int32_t>() + 4 * s; }
+    int next_slot() {
+        const int s = slot;
+        slot = (slot + 1) % kSlots;
+        return s;
+    }
+    // Raise if the kernels of the call that used slot `s` raised the device error word (a bounded wait ran out inside a
+    // kernel, so its outputs are not valid).  The word arrives by an asynchronous copy at the end of that call: it is
+    // certain to be there once a later event of the same stream has completed.
+    void check_error_word(int s) {
+        if (s < 0) return;
+        const int32_t stale = words(s)[2];
+        if (!stale) return;
+        words(s)[2] = 0;
+        throw std::runtime_error("trigrad_b200: an earlier render reported device error word " + std::to_string(stale) +
+                                 " (a bounded wait ran out inside a kernel); its outputs are not valid");
+    }
+    // After a forward call that used slot `s` has returned: it waited for work recorded after the previous call's on
+    // this stream, so the previous call's error word has arrived.
+    void finish_call(int s) {
+        const int prev = last_slot;
+        last_slot = s;
+        if (prev != s) check_error_word(prev);
+    }
+    void* workspace_of(size_t bytes, size_t* have) {
+        if ((size_t)workspace.numel() < bytes + 256)
+            workspace = at::empty({(int64_t)(bytes + bytes / 4 + 512)}, workspace.options());
+        const uintptr_t p = (uintptr_t)workspace.data_ptr(), base = (p + 255) / 256 * 256;
+        *have = (size_t)workspace.numel() - (base - p);
+        return (void*)base;
+    }
+};
+
+// At most kStates of them: a program that keeps making streams gives back the workspace of the one not used for longest.
+constexpr size_t kStates = 128;
+struct StateEntry {
+    int device;
+    cudaStream_t stream;
+    std::shared_ptr<DeviceState> state;
+};
+std::mutex g_states_lock;
+std::list<StateEntry>& states() {
+    static auto* s = new std::list<StateEntry>();   // never destroyed: its tensors must not outlive the CUDA context
+    return *s;
+}
+std::shared_ptr<DeviceState> state_of(int device, cudaStream_t stream) {
+    std::lock_guard<std::mutex> lock(g_states_lock);
+    auto& all = states();
+    for (auto it = all.begin(); it != all.end(); ++it)
+        if (it->device == device && it->stream == stream) {
+            if (it != all.begin()) all.splice(all.begin(), all, it);
+            return it->state;
+        }
+    all.push_front({device, stream, std::make_shared<DeviceState>(at::Device(at::kCUDA, (at::DeviceIndex)device))});
+    if (all.size() > kStates) all.pop_back();
+    return all.front().state;
+}
+
+struct Where {      // device made current for the scope, its current stream
+    c10::cuda::CUDAGuard guard;
+    int device;
+    cudaStream_t stream;
+    explicit Where(const Tensor& t) : guard(t.device()), device(t.get_device()) {
+        stream = c10::cuda::getCurrentCUDAStream(device).stream();
+    }
+};
+
+// ---- forward -------------------------------------------------------------------------------------------------------
+struct View {       // the arguments of a render that are not tensors
+    int W, H, tw, th;
+    double thr;
+    bool sort;
+    int layers;
+    int tiles() const { return ((W + tw - 1) / tw) * ((H + th - 1) / th); }
+    int64_t pixels() const { return (int64_t)W * H; }
+};
+
+// What a forward leaves for its backward, in one allocation (`blob`) beside the lists and the selection.
+struct Saved {
+    View v;
+    int V = 0, T = 0;
+    int64_t K = 0;
+    Tensor blob, ids, selection;
+    float *final_w = nullptr, *geo = nullptr, *attr = nullptr;
+    int32_t *ends = nullptr, *offsets = nullptr;
+    const int32_t* id_list() const { return data<int32_t>(ids); }
+    const int32_t* sel() const { return data<int32_t>(selection); }
+};
+
+struct ForwardOut {
+    Tensor image, depthmap;
+    std::shared_ptr<Saved> saved;
+    std::vector<float> stage_ms;    // five, when asked for
+};
+
+struct L2Step {     // forward, loss and gradients in one call (tg_render_step_l2)
+    const float* target;
+    float *loss, *gV, *gC, *gO;
+    int mode;
+    void* scratch;
+    size_t scratch_bytes;
+};
+
+constexpr size_t kAlign = 256;
+size_t up(size_t x) { return (x + kAlign - 1) / kAlign * kAlign; }
+
+std::shared_ptr<Saved> allocate_saved(const View& v, int V, int T, const at::TensorOptions& options) {
+    auto s = std::make_shared<Saved>();
+    s->v = v; s->V = V; s->T = T;
+    const size_t px = (size_t)v.pixels();
+    size_t off = 0;
+    auto take = [&](size_t bytes) { const size_t at = off; off += up(bytes); return at; };
+    const size_t o_fw = take(4 * px), o_ends = take(4 * px), o_geo = take(4 * (size_t)T * TG_GEO_WORDS),
+                 o_attr = take(4 * (size_t)T * TG_ATTR_WORDS), o_off = take(4 * ((size_t)v.tiles() + 1));
+    s->blob = at::empty({(int64_t)off}, options.dtype(at::kByte));
+    char* p = (char*)s->blob.data_ptr();
+    s->final_w = (float*)(p + o_fw);
+    s->ends = (int32_t*)(p + o_ends);
+    s->geo = (float*)(p + o_geo);
+    s->attr = (float*)(p + o_attr);
+    s->offsets = (int32_t*)(p + o_off);
+    return s;
+}
+
+// `opacities` undefined: packed inputs (indices [T,4], colors [V,4]).  Called without the interpreter lock.
+ForwardOut forward(const Tensor& vertices_, const Tensor& indices_, const Tensor& colors_, const Tensor& opacities_,
+                   const View& v, bool record_timing, bool save_selection, bool cull, int64_t selection_max_bytes,
+                   const L2Step* step = nullptr) {
+    const Tensor vertices = vertices_.contiguous(), indices = indices_.contiguous(), colors = colors_.contiguous();
+    const bool packed = !opacities_.defined();
+    const Tensor opacities = packed ? Tensor() : opacities_.contiguous();
+    const Where w(vertices);
+    const int T = need_int(indices.size(0)), V = need_int(vertices.size(0));
+    const auto options = vertices.options().requires_grad(false);
+    ForwardOut out;
+    out.image = at::empty({v.H, v.W, 4}, options);
+    out.depthmap = at::empty({v.H, v.W}, options);
+    out.saved = allocate_saved(v, V, T, options);
+    Saved& s = *out.saved;
+    const int64_t planes = save_selection ? g.selection_planes(v.sort ? 1 : 0, v.layers) : 0;
+    if (planes > 0 && planes * v.pixels() * 4 <= selection_max_bytes)
+        s.selection = at::empty({planes, v.H, v.W}, options.dtype(at::kInt));
+    if (record_timing) out.stage_ms.resize(5);
+    const unsigned flags = (cull ? TG_FORWARD_CULL_TILES : 0u) | (packed ? TG_INPUT_PACKED : 0u);
+    const auto state = state_of(w.device, w.stream);
+    std::lock_guard<std::mutex> lock(state->use);
+    int64_t cap = std::max<int64_t>(state->k_estimate + state->k_estimate / 4 + 1024, 2 * (int64_t)T + 1024);
+    while (true) {
+        s.ids = at::empty({cap}, options.dtype(at::kInt));
+        size_t have = 0;
+        void* ws = state->workspace_of(g.forward_workspace_bytes(T, v.tiles(), (uint32_t)cap), &have);
+        const int slot = state->next_slot();
+        int32_t* info = state->words(slot);
+        float* ms = record_timing ? out.stage_ms.data() : nullptr;
+        const double n = 4.0 * v.pixels();
+        const int status =
+            step ? g.render_step_l2(data<float>(vertices), data<int32_t>(indices), data<float>(colors), data<float>(opacities),
+                                    T, V, v.W, v.H, v.tw, v.th, (float)v.thr, v.layers, step->target, (float)(2.0 / n),
+                                    (float)(1.0 / n), step->loss, data<float>(out.image), data<float>(out.depthmap),
+                                    s.final_w, s.ends, s.geo, s.attr, data<int32_t>(s.ids), (uint32_t)cap, s.offsets,
+                                    step->gV, step->gC, step->gO, step->mode, ws, have, step->scratch,
+                                    step->scratch_bytes, (uint32_t*)info, ms, flags, w.stream)
+                 : g.render_forward(data<float>(vertices), data<int32_t>(indices), data<float>(colors),
+                                    data<float>(opacities), T, v.W, v.H, v.tw, v.th, (float)v.thr, v.sort ? 1 : 0,
+                                    v.layers, data<float>(out.image), data<float>(out.depthmap), s.final_w, s.ends,
+                                    data<int32_t>(s.selection), s.geo, s.attr, data<int32_t>(s.ids), (uint32_t)cap,
+                                    s.offsets, ws, have, (uint32_t*)info, ms, flags, w.stream);
+        s.K = (uint32_t)info[0];
+        if (status == TG_ERR_CAPACITY) {
+            cap = s.K + s.K / 4 + 1024;
+            continue;
+        }
+        check(step ? "render_step_l2" : "render_forward", status);
+        state->finish_call(slot);
+        state->k_estimate = s.K;
+        return out;
+    }
+}
+
+// ---- backward ------------------------------------------------------------------------------------------------------
+enum class Kind { kReference, kCorrected, kPacked };
+
+// Raise when the forward's error word has arrived by now and is set (no waiting here): lists built by a kernel whose
+// bounded wait ran out must not be walked.
+void check_last_forward(const Where& w) {
+    const auto state = state_of(w.device, w.stream);
+    state->check_error_word(state->last_slot);
+}
+
+// Gradients in the order of the inputs: vertices, colours, opacities - or vertices, rgba with packed inputs.
+std::vector<Tensor> backward(Kind kind, const Saved& s, const Tensor& image, const Tensor& depthmap, Tensor gi, Tensor gd) {
+    const Where w(image);
+    check_last_forward(w);
+    const auto options = image.options().requires_grad(false);
+    std::vector<Tensor> out;
+    out.push_back(at::empty({s.V, 4}, options));
+    if (kind == Kind::kPacked) {
+        out.push_back(at::empty({s.V, 4}, options));
+    } else {
+        out.push_back(at::empty({s.V, 3}, options));
+        out.push_back(at::empty({s.V}, options));
+    }
+    if (!gi.defined() && !gd.defined()) {
+        for (auto& t : out) t.zero_();
+        return out;
+    }
+    gi = gi.defined() ? gi.contiguous() : at::zeros_like(image);      // only the depth map was used downstream
+    gd = gd.defined() ? gd.contiguous() : Tensor();                  // none: taken as zero by the kernel
+    const size_t nscratch = g.backward_scratch_bytes(s.V);
+    const Tensor scratch = at::empty({(int64_t)nscratch}, options.dtype(at::kByte));
+    const View& v = s.v;
+    if (kind == Kind::kPacked) {
+        scratch.zero_();
+        // the sums stay in the packed accumulator, which already has the layout wanted here
+        check("blend_backward", g.blend_backward(s.geo, s.attr, s.id_list(), s.offsets, s.V, v.W, v.H, v.tw, v.th, v.sort,
+                                                 v.layers, data<float>(gi), data<float>(gd), data<float>(image),
+                                                 data<float>(depthmap), s.final_w, s.ends, s.sel(), nullptr, nullptr,
+                                                 nullptr, TG_ACCUMULATE_PACKED, scratch.data_ptr(), nscratch, w.stream));
+        check("unpack_gradients_rgba", g.unpack_gradients_rgba(scratch.data_ptr(), nscratch, s.V, 0.f, nullptr,
+                                                               data<float>(out[0]), data<float>(out[1]), 0, w.stream));
+    } else if (kind == Kind::kCorrected) {
+        check("blend_backward_corrected",
+              g.blend_backward_corrected(s.geo, s.attr, s.id_list(), s.offsets, s.V, v.W, v.H, v.tw, v.th, v.sort, v.layers,
+                                         data<float>(gi), data<float>(gd), data<float>(image), data<float>(depthmap),
+                                         s.final_w, s.ends, data<float>(out[0]), data<float>(out[1]), data<float>(out[2]),
+                                         0, scratch.data_ptr(), nscratch, w.stream));
+    } else {
+        check("blend_backward", g.blend_backward(s.geo, s.attr, s.id_list(), s.offsets, s.V, v.W, v.H, v.tw, v.th, v.sort,
+                                                 v.layers, data<float>(gi), data<float>(gd), data<float>(image),
+                                                 data<float>(depthmap), s.final_w, s.ends, s.sel(), data<float>(out[0]),
+                                                 data<float>(out[1]), data<float>(out[2]), 0, scratch.data_ptr(), nscratch,
+                                                 w.stream));
+    }
+    return out;
+}
+
+struct RenderBackward : public Node {
+    Kind kind = Kind::kReference;
+    std::shared_ptr<Saved> saved;      // null: a mesh without triangles
+    SavedVariable image, depthmap;     // outputs of this node
+    std::vector<Tensor> like;          // mesh without triangles: the shapes of the (zero) gradients
+    std::mutex lock;
+
+    std::string name() const override { return "RenderBackward"; }
+    variable_list apply(variable_list&& grads) override {
+        std::lock_guard<std::mutex> hold(lock);
+        variable_list out;
+        if (!like.empty()) {
+            for (const auto& t : like) out.push_back(at::zeros_like(t));
+            return out;
+        }
+        const Tensor im = image.unpack(shared_from_this()), dm = depthmap.unpack(shared_from_this());
+        TORCH_CHECK(saved, torch::autograd::ERR_BACKWARD_TWICE);
+        at::AutoDispatchBelowADInplaceOrView below_autograd;
+        for (auto& t : backward(kind, *saved, im, dm, grads[0], grads[1])) out.push_back(std::move(t));
+        return out;
+    }
+    void release_variables() override {
+        std::lock_guard<std::mutex> hold(lock);
+        image.reset_data();
+        depthmap.reset_data();
+        saved.reset();
+    }
+};
+
+struct ImageAndDepth {
+    Tensor image, depthmap;
+    std::vector<float> stage_ms;
+};
+
+// Forward with the gradient node attached when gradients are wanted.  Without the interpreter lock.
+ImageAndDepth render_graph(Kind kind, const Tensor& vertices, const Tensor& indices, const Tensor& colors,
+                           const Tensor& opacities, View v, bool record_timing, bool cull_tiles,
+                           int64_t selection_max_bytes) {
+    const int64_t T = indices.size(0);
+    if (v.layers <= 0) v.layers = need_int(T + 1);
+    const bool wants_grad = at::GradMode::is_enabled() && (vertices.requires_grad() || colors.requires_grad() ||
+                                                           (opacities.defined() && opacities.requires_grad()));
+    std::shared_ptr<RenderBackward> node;
+    if (wants_grad) {
+        node = std::shared_ptr<RenderBackward>(new RenderBackward(), torch::autograd::deleteNode);
+        node->kind = kind;
+        if (kind == Kind::kPacked) node->set_next_edges(torch::autograd::collect_next_edges(vertices, colors));
+        else node->set_next_edges(torch::autograd::collect_next_edges(vertices, colors, opacities));
+    }
+    ImageAndDepth r;
+    {
+        at::AutoDispatchBelowADInplaceOrView below_autograd;
+        if (T < 1) {
+            const c10::cuda::CUDAGuard guard(colors.device());
+            const auto options = colors.options().requires_grad(false);
+            r.image = at::zeros({v.H, v.W, 4}, options);
+            r.image.select(2, 3).fill_(1.0);
+            r.depthmap = at::full({v.H, v.W}, INFINITY, options);
+            if (node) {
+                node->like = {vertices.detach(), colors.detach()};
+                if (kind != Kind::kPacked) node->like.push_back(opacities.detach());
+            }
+        } else {
+            // the corrected gradients walk the lists themselves and need no selection; nor does a render nobody differentiates
+            ForwardOut f = forward(vertices, indices, colors, opacities, v, record_timing,
+                                   wants_grad && kind != Kind::kCorrected, cull_tiles, selection_max_bytes);
+            r.image = std::move(f.image);
+            r.depthmap = std::move(f.depthmap);
+            r.stage_ms = std::move(f.stage_ms);
+            if (node) node->saved = std::move(f.saved);
+        }
+    }
+    if (node) {
+        torch::autograd::set_history(r.image, node);
+        torch::autograd::set_history(r.depthmap, node);
+        if (node->saved) {
+            node->image = SavedVariable(r.image, /*is_output=*/true);
+            node->depthmap = SavedVariable(r.depthmap, /*is_output=*/true);
+        }
+    }
+    return r;
+}
+
+// ---- fused mean-squared-error step ---------------------------------------------------------------------------------
+struct Grads {      // where a step's gradients and loss go: the three tensors and the loss, or a packed accumulator
+    Tensor vertices, colors, opacities, loss, packed;
+};
+
+Tensor l2_step(const Tensor& vertices, const Tensor& indices, const Tensor& colors, const Tensor& opacities,
+               const Tensor& target_, const View& v, const Grads& to, bool one_kernel, bool cull,
+               int64_t selection_max_bytes) {
+    const at::AutoDispatchBelowADInplaceOrView below_autograd;
+    const Where w(vertices);
+    const int V = need_int(vertices.size(0));
+    const Tensor target = target_.contiguous();
+    const size_t nscratch = g.backward_scratch_bytes(V);
+    const bool packed = to.packed.defined();
+    L2Step step;
+    step.target = data<float>(target);
+    step.mode = packed ? TG_ACCUMULATE_PACKED : 1;
+    step.loss = packed ? nullptr : data<float>(to.loss);
+    step.gV = packed ? nullptr : data<float>(to.vertices);
+    step.gC = packed ? nullptr : data<float>(to.colors);
+    step.gO = packed ? nullptr : data<float>(to.opacities);
+    const Tensor scratch = packed ? to.packed : at::empty({(int64_t)nscratch}, vertices.options().dtype(at::kByte).requires_grad(false));
+    step.scratch = scratch.data_ptr();
+    step.scratch_bytes = packed ? (size_t)scratch.numel() : nscratch;
+    if (one_kernel) return forward(vertices, indices, colors, opacities, v, false, false, cull, 0, &step).image;
+    const ForwardOut f = forward(vertices, indices, colors, opacities, v, false, true, cull, selection_max_bytes);
+    const Saved& s = *f.saved;
+    TORCH_CHECK_VALUE(s.selection.defined(), "the fused L2 backward needs per_pixel_sort=True and max_layers <= 32");
+    const double n = 4.0 * v.pixels();
+    const int status =
+        target.scalar_type() == at::kByte
+            ? g.blend_backward_l2_u8(s.geo, s.attr, s.id_list(), s.offsets, V, v.W, v.H, v.tw, v.th, 1, v.layers,
+                                     data<uint8_t>(target), (float)(2.0 / n), (float)(1.0 / n), step.loss,
+                                     data<float>(f.image), data<float>(f.depthmap), s.final_w, s.ends, s.sel(), step.gV,
+                                     step.gC, step.gO, step.mode, step.scratch, step.scratch_bytes, w.stream)
+            : g.blend_backward_l2(s.geo, s.attr, s.id_list(), s.offsets, V, v.W, v.H, v.tw, v.th, 1, v.layers,
+                                  step.target, (float)(2.0 / n), (float)(1.0 / n), step.loss, data<float>(f.image),
+                                  data<float>(f.depthmap), s.final_w, s.ends, s.sel(), step.gV, step.gC, step.gO, step.mode,
+                                  step.scratch, step.scratch_bytes, w.stream);
+    check("blend_backward_l2", status);
+    return f.image;
+}
+
+// ---- projection ----------------------------------------------------------------------------------------------------
+struct Matrix { float m[16]; };
+
+Tensor project(const Tensor& points_, const Matrix& pv) {
+    const at::AutoDispatchBelowADInplaceOrView below_autograd;
+    const Tensor points = points_.contiguous();
+    const Where w(points);
+    const Tensor out = at::empty({points.size(0), 4}, points.options().requires_grad(false));
+    check("project", g.project(data<float>(points), need_int(points.size(0)), pv.m, data<float>(out), w.stream));
+    return out;
+}
+
+void project_backward(const Tensor& points_, const Matrix& pv, const Tensor& grad_vertices_, const Tensor& grad_points,
+                      bool accumulate) {
+    const at::AutoDispatchBelowADInplaceOrView below_autograd;
+    const Tensor points = points_.contiguous(), grad_vertices = grad_vertices_.contiguous();
+    const Where w(points);
+    check("project_backward", g.project_backward(data<float>(points), need_int(points.size(0)), pv.m,
+                                                 data<float>(grad_vertices), data<float>(grad_points), accumulate, w.stream));
+}
+
+Tensor world_step(const Tensor& points_, const Matrix& pv, const Tensor& indices, const Tensor& colors,
+                  const Tensor& opacities, const Tensor& target, const View& v, const Grads& to, bool one_kernel,
+                  int64_t selection_max_bytes) {
+    const at::AutoDispatchBelowADInplaceOrView below_autograd;
+    const Tensor points = points_.contiguous();
+    const Where w(points);
+    const Tensor vertices = project(points, pv);
+    if (!to.packed.defined()) {
+        Grads inner = to;
+        inner.vertices = at::zeros_like(vertices);
+        const Tensor image = l2_step(vertices, indices, colors, opacities, target, v, inner, one_kernel, true,
+                                     selection_max_bytes);
+        project_backward(points, pv, inner.vertices, to.vertices, true);
+        return image;
+    }
+    const Tensor image = l2_step(vertices, indices, colors, opacities, target, v, to, one_kernel, true, selection_max_bytes);
+    check("unpack_project_backward",
+          g.unpack_project_backward(to.packed.data_ptr(), (size_t)to.packed.numel(), need_int(points.size(0)),
+                                    data<float>(points), pv.m, (float)(1.0 / (4.0 * v.pixels())), data<float>(to.loss),
+                                    data<float>(to.vertices), data<float>(to.colors), data<float>(to.opacities), w.stream));
+    return image;
+}
+
+// ---- projection with near-plane splitting --------------------------------------------------------------------------
+struct ProjectClipBackward : public Node {
+    SavedVariable points, indices, colors, opacities;
+    Matrix pv;
+    std::mutex lock;
+
+    std::string name() const override { return "ProjectClipBackward"; }
+    variable_list apply(variable_list&& grads) override {
+        std::lock_guard<std::mutex> hold(lock);
+        const Tensor p = points.unpack().detach(), i = indices.unpack(), c = colors.unpack().detach(),
+                     o = opacities.unpack().detach();
+        at::AutoDispatchBelowADInplaceOrView below_autograd;
+        const Where w(p);
+        const int64_t T = i.size(0);
+        const auto options = p.options().requires_grad(false);
+        auto upstream = [&](const Tensor& t, at::IntArrayRef shape) { return t.defined() ? t.contiguous() : at::zeros(shape, options); };
+        const Tensor gv = upstream(grads[0], {6 * T, 4}), gc = upstream(grads[1], {6 * T, 3}), go = upstream(grads[2], {6 * T});
+        variable_list out = {at::zeros_like(p), at::zeros_like(c), at::zeros_like(o)};
+        check("project_clip_backward",
+              g.project_clip_backward(data<float>(p), data<int32_t>(i), data<float>(c), data<float>(o), need_int(T), pv.m,
+                                      data<float>(gv), data<float>(gc), data<float>(go), data<float>(out[0]),
+                                      data<float>(out[1]), data<float>(out[2]), w.stream));
+        return out;
+    }
+    void release_variables() override {
+        std::lock_guard<std::mutex> hold(lock);
+        points.reset_data(); indices.reset_data(); colors.reset_data(); opacities.reset_data();
+    }
+};
+
+std::tuple<Tensor, Tensor, Tensor, Tensor> project_clip(const Tensor& points_, const Tensor& indices_, const Tensor& colors_,
+                                                        const Tensor& opacities_, const Matrix& pv) {
+    const Tensor points = points_.contiguous(), indices = indices_.contiguous(), colors = colors_.contiguous(),
+                 opacities = opacities_.contiguous();
+    std::shared_ptr<ProjectClipBackward> node;
+    if (at::GradMode::is_enabled() && (points.requires_grad() || colors.requires_grad() || opacities.requires_grad())) {
+        node = std::shared_ptr<ProjectClipBackward>(new ProjectClipBackward(), torch::autograd::deleteNode);
+        node->set_next_edges(torch::autograd::collect_next_edges(points, colors, opacities));
+        node->points = SavedVariable(points, false);
+        node->indices = SavedVariable(indices, false);
+        node->colors = SavedVariable(colors, false);
+        node->opacities = SavedVariable(opacities, false);
+        node->pv = pv;
+    }
+    Tensor ov, oi, oc, oo;
+    {
+        at::AutoDispatchBelowADInplaceOrView below_autograd;
+        const Where w(points);
+        const int64_t T = indices.size(0);
+        const auto options = points.options().requires_grad(false);
+        ov = at::empty({6 * T, 4}, options);
+        oi = at::empty({2 * T, 3}, options.dtype(at::kInt));
+        oc = at::empty({6 * T, 3}, options);
+        oo = at::empty({6 * T}, options);
+        check("project_clip", g.project_clip(data<float>(points), data<int32_t>(indices), data<float>(colors),
+                                             data<float>(opacities), need_int(T), pv.m, data<float>(ov), data<int32_t>(oi),
+                                             data<float>(oc), data<float>(oo), w.stream));
+    }
+    if (node) {
+        torch::autograd::set_history(ov, node);
+        torch::autograd::set_history(oc, node);
+        torch::autograd::set_history(oo, node);
+    }
+    return {ov, oi, oc, oo};
+}
+
+// ---- what Python sees ----------------------------------------------------------------------------------------------
+// Checks with the interpreter lock, work without it.
+using Optional = std::optional<Tensor>;
+Tensor or_none(const Optional& t) { return t ? *t : Tensor(); }
+
+View view_of(int64_t W, int64_t H, int64_t tw, int64_t th, double thr, bool sort, int64_t layers) {
+    return {need_int(W), need_int(H), (int)tw, (int)th, thr, sort, (int)std::min<int64_t>(layers, INT32_MAX)};
+}
+
+Matrix matrix_of(const py::buffer& b) {
+    const py::buffer_info i = b.request();
+    if (i.itemsize != 4 || i.format != py::format_descriptor<float>::format() || i.size != 16)
+        throw py::value_error("pv must be a 4x4 matrix");
+    Matrix m;
+    std::copy_n(static_cast<const float*>(i.ptr), 16, m.m);
+    return m;
+}
+
+py::object py_render(int kind, const Tensor& vertices, const Tensor& indices, const Tensor& colors,
+                     const Optional& opacities_, int64_t W, int64_t H, int64_t tw, int64_t th, double thr, bool timing,
+                     bool sort, int64_t layers, bool cull, int64_t selection_max_bytes) {
+    need_tile((int)tw, (int)th);
+    const Tensor opacities = or_none(opacities_);
+    const int64_t V = rows(vertices, "vertices");
+    need(vertices, "vertices", {V, 4});
+    if ((Kind)kind == Kind::kPacked) {
+        need(colors, "rgba", {V, 4});
+        need(indices, "faces", {rows(indices, "faces"), 4}, at::kInt);
+    } else {
+        need(colors, "colors", {V, 3});
+        need(opacities, "opacities", {V});
+        need(indices, "indices", {rows(indices, "indices"), 3}, at::kInt);
+    }
+    const View v = view_of(W, H, tw, th, thr, sort, layers);
+    ImageAndDepth r;
+    {
+        py::gil_scoped_release nogil;
+        r = render_graph((Kind)kind, vertices, indices, colors, opacities, v, timing, cull, selection_max_bytes);
+    }
+    if (!timing) return py::make_tuple(std::move(r.image), std::move(r.depthmap));
+    return py::make_tuple(std::move(r.image), std::move(r.depthmap),
+                          r.stage_ms.empty() ? py::object(py::none()) : py::cast(r.stage_ms));
+}
+
+// The separate tensors a caller of the forward alone gets: views of the one allocation.
+Tensor part(const Saved& s, const void* p, at::ScalarType type, at::IntArrayRef shape) {
+    const int64_t off = (const char*)p - (const char*)s.blob.data_ptr();
+    int64_t n = 4;
+    for (int64_t d : shape) n *= d;
+    return s.blob.narrow(0, off, n).view(type).view(shape);
+}
+
+// opacities None: packed inputs
+py::object py_forward(const Tensor& vertices, const Tensor& indices, const Tensor& colors, const Optional& opacities,
+                      int64_t W, int64_t H, int64_t tw, int64_t th, double thr, bool timing, bool sort, int64_t layers,
+                      bool save_selection, bool cull, int64_t selection_max_bytes) {
+    const View v = view_of(W, H, tw, th, thr, sort, layers);
+    ForwardOut f;
+    Tensor fw, ids, off, geo, attr, ends;
+    {
+        py::gil_scoped_release nogil;
+        at::AutoDispatchBelowADInplaceOrView below_autograd;
+        f = forward(vertices, indices, colors, or_none(opacities), v, timing, save_selection, cull, selection_max_bytes);
+        const Saved& s = *f.saved;
+        fw = part(s, s.final_w, at::kFloat, {v.H, v.W});
+        ids = s.ids.narrow(0, 0, s.K);
+        off = part(s, s.offsets, at::kInt, {v.tiles() + 1});
+        geo = part(s, s.geo, at::kFloat, {s.T, TG_GEO_WORDS});
+        attr = part(s, s.attr, at::kFloat, {s.T, TG_ATTR_WORDS});
+        ends = part(s, s.ends, at::kInt, {v.H, v.W});
+    }
+    return py::make_tuple(f.image, f.depthmap, fw, ids, off, geo, attr, ends,
+                          f.saved->selection.defined() ? py::cast(f.saved->selection) : py::object(py::none()),
+                          timing ? py::cast(f.stage_ms) : py::object(py::none()), f.saved);
+}
+
+py::list py_backward(const std::shared_ptr<Saved>& saved, const Tensor& image, const Tensor& depthmap, const Optional& gi,
+                     const Optional& gd) {
+    std::vector<Tensor> out;
+    {
+        py::gil_scoped_release nogil;
+        at::AutoDispatchBelowADInplaceOrView below_autograd;
+        out = backward(Kind::kReference, *saved, image, depthmap, or_none(gi), or_none(gd));
+    }
+    return py::cast(out);
+}
+
+void need_mesh(const Tensor& positions, const char* name, int64_t components, const Tensor& indices, const Tensor& colors,
+               const Tensor& opacities) {
+    const int64_t V = rows(positions, name);
+    need(positions, name, {V, components});
+    need(colors, "colors", {V, 3});
+    need(opacities, "opacities", {V});
+    need(indices, "indices", {rows(indices, "indices"), 3}, at::kInt);
+}
+
+Tensor py_l2_step(const Tensor& vertices, const Tensor& indices, const Tensor& colors, const Tensor& opacities,
+                  const Tensor& target, int64_t W, int64_t H, int64_t tw, int64_t th, double thr, int64_t layers,
+                  const Optional& gV, const Optional& gC, const Optional& gO, const Optional& loss, const Optional& packed,
+                  bool one_kernel, bool cull, int64_t selection_max_bytes, const py::object& pv) {
+    const bool world = !pv.is_none();
+    need_mesh(vertices, world ? "points" : "vertices", world ? 3 : 4, indices, colors, opacities);
+    need(target, "target", {H, W, 4}, target.scalar_type() == at::kByte && !one_kernel ? at::kByte : at::kFloat);
+    need_tile((int)tw, (int)th);
+    const View v = view_of(W, H, tw, th, thr, true, layers);
+    const Grads to = {or_none(gV), or_none(gC), or_none(gO), or_none(loss), or_none(packed)};
+    const Matrix m = world ? matrix_of(pv.cast<py::buffer>()) : Matrix{};
+    py::gil_scoped_release nogil;
+    return world ? world_step(vertices, m, indices, colors, opacities, target, v, to, one_kernel, selection_max_bytes)
+                 : l2_step(vertices, indices, colors, opacities, target, v, to, one_kernel, cull, selection_max_bytes);
+}
+
+Tensor py_project(const Tensor& points, const py::buffer& pv) {
+    need(points, "points", {rows(points, "points"), 3});
+    const Matrix m = matrix_of(pv);
+    py::gil_scoped_release nogil;
+    return project(points, m);
+}
+
+void py_project_backward(const Tensor& points, const py::buffer& pv, const Tensor& gv, const Tensor& gp, bool accumulate) {
+    const int64_t V = rows(points, "points");
+    need(points, "points", {V, 3});
+    need(gv, "grad_vertices", {V, 4});
+    need(gp, "grad_points", {V, 3});
+    const Matrix m = matrix_of(pv);
+    py::gil_scoped_release nogil;
+    project_backward(points, m, gv, gp, accumulate);
+}
+
+py::tuple py_project_clip(const Tensor& points, const Tensor& indices, const Tensor& colors, const Tensor& opacities,
+                          const py::buffer& pv) {
+    need_mesh(points, "points", 3, indices, colors, opacities);
+    const Matrix m = matrix_of(pv);
+    std::tuple<Tensor, Tensor, Tensor, Tensor> r;
+    {
+        py::gil_scoped_release nogil;
+        r = project_clip(points, indices, colors, opacities, m);
+    }
+    return py::make_tuple(std::get<0>(r), std::get<1>(r), std::get<2>(r), std::get<3>(r));
+}
+
+py::tuple py_pack_mesh(const Tensor& colors_, const Tensor& opacities_, const Tensor& indices_) {
+    const int64_t V = rows(colors_, "colors"), T = rows(indices_, "indices");
+    need(colors_, "colors", {V, 3});
+    need(opacities_, "opacities", {V});
+    need(indices_, "indices", {T, 3}, at::kInt);
+    Tensor rgba, faces;
+    {
+        py::gil_scoped_release nogil;
+        const at::AutoDispatchBelowADInplaceOrView below_autograd;
+        const Tensor colors = colors_.contiguous(), opacities = opacities_.contiguous(), indices = indices_.contiguous();
+        const Where w(colors);
+        rgba = at::empty({V, 4}, colors.options().requires_grad(false));
+        faces = at::empty({T, 4}, indices.options());
+        check("pack_inputs", g.pack_inputs(data<float>(colors), data<float>(opacities), data<int32_t>(indices), need_int(V),
+                                           need_int(T), data<float>(rgba), data<int32_t>(faces), w.stream));
+    }
+    return py::make_tuple(rgba, faces);
+}
+
+void py_unpack_gradients(const Tensor& scratch, int64_t V, int64_t W, int64_t H, const Tensor& gV, const Tensor& gC,
+                         const Tensor& gO, const Optional& loss, bool accumulate) {
+    py::gil_scoped_release nogil;
+    const Where w(gV);
+    check("unpack_gradients",
+          g.unpack_gradients(scratch.data_ptr(), (size_t)scratch.numel(), need_int(V), (float)(1.0 / (4.0 * W * H)),
+                             data<float>(or_none(loss)), data<float>(gV), data<float>(gC), data<float>(gO), accumulate,
+                             w.stream));
+}
+
+}  // namespace
+
+PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+    py::register_exception_translator([](std::exception_ptr p) {
+        try {
+            if (p) std::rethrow_exception(p);
+        } catch (const LibraryError& e) {
+            const py::object error = py::reinterpret_borrow<py::object>(g_native_error)(e.stage, e.status, e.detail);
+            PyErr_SetObject(g_native_error, error.ptr());
+        }
+    });
+    py::class_<Saved, std::shared_ptr<Saved>>(m, "Saved");
+    py::class_<DeviceState, std::shared_ptr<DeviceState>>(m, "DeviceState")
+        .def_readonly("info", &DeviceState::info)
+        .def_readonly("last_slot", &DeviceState::last_slot)
+        .def_readonly("k_estimate", &DeviceState::k_estimate)
+        .def("check_error_word", &DeviceState::check_error_word);
+    m.def("bind", &bind);
+    m.def("state", [](int device, int64_t stream) { return state_of(device, (cudaStream_t)stream); });
+    m.def("render", &py_render);
+    m.def("forward", &py_forward);
+    m.def("backward", &py_backward);
+    m.def("l2_step", &py_l2_step);
+    m.def("project", &py_project);
+    m.def("project_backward", &py_project_backward);
+    m.def("project_clip", &py_project_clip);
+    m.def("pack_mesh", &py_pack_mesh);
+    m.def("unpack_gradients", &py_unpack_gradients);
+}

@@ -16,6 +16,7 @@ from typing import Callable, Sequence
 
 import torch
 
+from . import _native as N
 from . import wrapper as _w
 from .wrapper import render as _render
 
@@ -68,8 +69,6 @@ class PackedGradients:
     """
 
     def __init__(self, num_vertices: int, device):
-        from . import _native as N
-
         self.num_vertices = num_vertices
         self.scratch = torch.zeros(N.lib().tg_backward_scratch_bytes(num_vertices), dtype=torch.uint8, device=device)
 
@@ -79,8 +78,8 @@ class PackedGradients:
     def unpack(self, width: int, height: int, grad_vertices: torch.Tensor, grad_colors: torch.Tensor,
                grad_opacities: torch.Tensor, loss: torch.Tensor, accumulate: bool = False) -> None:
         """Writes (or adds) the sums; ``loss`` receives the sum of the views' mean squared errors."""
-        _w.unpack_gradients_native(self.scratch, self.num_vertices, width, height,
-                                   (grad_vertices, grad_colors, grad_opacities), loss, accumulate)
+        N.host().unpack_gradients(self.scratch, self.num_vertices, width, height, grad_vertices, grad_colors,
+                                  grad_opacities, loss, accumulate)
 
 
 def render_views_l2(points: torch.Tensor, indices: torch.Tensor, colors: torch.Tensor, opacities: torch.Tensor,
@@ -129,41 +128,29 @@ def l2_view_step(vertices: torch.Tensor, indices: torch.Tensor, colors: torch.Te
     """
     if not (1 <= max_layers <= 32):
         raise ValueError("l2_view_step needs 1 <= max_layers <= 32")
-    n, _ = vertices.shape
-    _w.check_tensor(vertices, "vertices", (n, 4))
+    if one_kernel and target.dtype == torch.uint8:
+        # 8-bit RGBA target (value / 255): a quarter of the bytes per view; the two-kernel path reads it directly
+        raise ValueError("the one-kernel step takes a float32 target")
+    if indices.shape[0] < 1:
+        return _empty_mesh_step(vertices, 4, colors, opacities, target, packed, loss)
+    return N.host().l2_step(vertices, indices, colors, opacities, target, width, height, tile_width, tile_height,
+                            early_stopping_threshold, max_layers, grad_vertices, grad_colors, grad_opacities, loss,
+                            None if packed is None else packed.scratch, one_kernel and tile_width * tile_height <= 256,
+                            cull_tiles, _w.SELECTION_MAX_BYTES, None)
+
+
+def _empty_mesh_step(positions, components, colors, opacities, target, packed, loss):
+    """The background's loss; no gradients and no image."""
+    n, _ = positions.shape
+    _w.check_tensor(positions, "positions", (n, components))
     _w.check_tensor(colors, "colors", (n, 3))
     _w.check_tensor(opacities, "opacities", (n,))
-    m, _ = indices.shape
-    _w.check_tensor(indices, "indices", (m, 3), torch.int32)
-    if target.dtype == torch.uint8:
-        # 8-bit RGBA target (value / 255): a quarter of the bytes per view; the two-kernel path reads it directly
-        if one_kernel:
-            raise ValueError("the one-kernel step takes a float32 target")
-        _w.check_tensor(target, "target", (height, width, 4), torch.uint8)
-    else:
-        _w.check_tensor(target, "target", (height, width, 4))
-    if tile_width * tile_height > 1024:
-        raise ValueError("tile_width * tile_height must be <= 1024")
-    if m < 1:
-        if packed is not None:
-            raise ValueError("a mesh without triangles cannot use the packed accumulator")
-        tf = target.float() / 255 if target.dtype == torch.uint8 else target
-        loss += torch.mean((torch.tensor([0.0, 0.0, 0.0, 1.0], device=target.device) - tf) ** 2)
-        return None
-    grads = (grad_vertices, grad_colors, grad_opacities)
-    if one_kernel and tile_width * tile_height <= 256:
-        # forward, loss and gradients in one native call (one compositing kernel for both directions)
-        return _w.step_l2_native(vertices.contiguous(), indices.contiguous(), colors.contiguous(), opacities.contiguous(),
-                                 target, width, height, tile_width, tile_height, early_stopping_threshold, max_layers,
-                                 grads, loss, accumulate=True,
-                                 packed_scratch=None if packed is None else packed.scratch, cull_tiles=cull_tiles)[0]
-    (image, depthmap, final_weights, sorted_ids, offsets, tri_geo, tri_attr, ends, selection, _) = _w.forward_native(
-        vertices.contiguous(), indices.contiguous(), colors.contiguous(), opacities.contiguous(), width, height,
-        tile_width, tile_height, early_stopping_threshold, False, True, max_layers, cull_tiles=cull_tiles)
-    saved = (sorted_ids, offsets, tri_geo, tri_attr, image, depthmap, final_weights, ends, selection)
-    _w.backward_l2_native(target, saved, n, width, height, tile_width, tile_height, True, max_layers, grads, loss,
-                          accumulate=True, packed_scratch=None if packed is None else packed.scratch)
-    return image
+    _w.check_tensor(target, "target", dtype=None if target.dtype != torch.uint8 else torch.uint8)
+    if packed is not None:
+        raise ValueError("a mesh without triangles cannot use the packed accumulator")
+    tf = target.float() / 255 if target.dtype == torch.uint8 else target
+    loss += torch.mean((torch.tensor([0.0, 0.0, 0.0, 1.0], device=target.device) - tf) ** 2)
+    return None
 
 
 def _pv_host(pv):
@@ -180,37 +167,13 @@ def _pv_host(pv):
 
 def project_native(points: torch.Tensor, pv) -> torch.Tensor:
     """World points (V,3) -> render vertices (V,4) in one kernel (``tg_project``); ``pv`` best given on the host."""
-    import ctypes as C
-
-    from . import _native as N
-
-    _w.check_tensor(points, "points", (points.shape[0], 3))
-    m = _pv_host(pv)
-    out = torch.empty((points.shape[0], 4), dtype=torch.float32, device=points.device)
-    with torch.cuda.device(points.device):
-        stream = torch.cuda.current_stream(points.device).cuda_stream
-        N.check("project", N.lib().tg_project(C.c_void_p(points.data_ptr()), points.shape[0], m.ctypes.data_as(C.c_void_p),
-                                              C.c_void_p(out.data_ptr()), C.c_void_p(stream)))
-    return out
+    return N.host().project(points, _pv_host(pv))
 
 
 def project_backward_native(points: torch.Tensor, pv, grad_vertices: torch.Tensor, grad_points: torch.Tensor,
                             accumulate: bool = True) -> torch.Tensor:
     """``grad_points (V,3)`` += (or =) the vector-Jacobian product of ``project_native`` with ``grad_vertices (V,4)``."""
-    import ctypes as C
-
-    from . import _native as N
-
-    V = points.shape[0]
-    _w.check_tensor(points, "points", (V, 3))
-    _w.check_tensor(grad_vertices, "grad_vertices", (V, 4))
-    _w.check_tensor(grad_points, "grad_points", (V, 3))
-    m = _pv_host(pv)
-    with torch.cuda.device(points.device):
-        stream = torch.cuda.current_stream(points.device).cuda_stream
-        N.check("project_backward", N.lib().tg_project_backward(
-            C.c_void_p(points.data_ptr()), V, m.ctypes.data_as(C.c_void_p), C.c_void_p(grad_vertices.data_ptr()),
-            C.c_void_p(grad_points.data_ptr()), int(bool(accumulate)), C.c_void_p(stream)))
+    N.host().project_backward(points, _pv_host(pv), grad_vertices, grad_points, accumulate)
     return grad_points
 
 
@@ -228,28 +191,16 @@ def l2_world_view_step(points: torch.Tensor, pv, indices: torch.Tensor, colors: 
     through the projection's VJP into the three tensors and ``loss`` with atomic additions and leaves the
     accumulator zero again: no per-view clear, no render-space gradient tensor, and views on several streams may
     add into the same tensors."""
-    m = _pv_host(pv)
-    verts = project_native(points, m)
-    if packed is not None:
-        import ctypes as C
-
-        from . import _native as N
-
-        image = l2_view_step(verts, indices, colors, opacities, target, width, height, None, None, None, None, tile_width,
-                             tile_height, early_stopping_threshold, max_layers, one_kernel, packed=packed)
-        with torch.cuda.device(points.device):
-            stream = torch.cuda.current_stream(points.device).cuda_stream
-            N.check("unpack_project_backward", N.lib().tg_unpack_project_backward(
-                C.c_void_p(packed.scratch.data_ptr()), packed.scratch.numel(), points.shape[0],
-                C.c_void_p(points.data_ptr()), m.ctypes.data_as(C.c_void_p), 1.0 / float(width * height * 4),
-                C.c_void_p(loss.data_ptr()), C.c_void_p(grad_points.data_ptr()), C.c_void_p(grad_colors.data_ptr()),
-                C.c_void_p(grad_opacities.data_ptr()), C.c_void_p(stream)))
-        return image
-    gverts = torch.zeros_like(verts)
-    image = l2_view_step(verts, indices, colors, opacities, target, width, height, gverts, grad_colors, grad_opacities, loss,
-                         tile_width, tile_height, early_stopping_threshold, max_layers, one_kernel)
-    project_backward_native(points, m, gverts, grad_points, accumulate=True)
-    return image
+    if not (1 <= max_layers <= 32):
+        raise ValueError("l2_world_view_step needs 1 <= max_layers <= 32")
+    if one_kernel and target.dtype == torch.uint8:
+        raise ValueError("the one-kernel step takes a float32 target")
+    if indices.shape[0] < 1:
+        return _empty_mesh_step(points, 3, colors, opacities, target, packed, loss)
+    return N.host().l2_step(points, indices, colors, opacities, target, width, height, tile_width, tile_height,
+                            early_stopping_threshold, max_layers, grad_points, grad_colors, grad_opacities, loss,
+                            None if packed is None else packed.scratch, one_kernel and tile_width * tile_height <= 256,
+                            True, _w.SELECTION_MAX_BYTES, _pv_host(pv))
 
 
 def allreduce_gradients(grads: GradBuffer, loss: torch.Tensor | None = None, group=None) -> None:
