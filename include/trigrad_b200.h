@@ -288,6 +288,11 @@ int tg_blend_step_l2(const float* tri_geo, const float* tri_attr, const int32_t*
  *                tg_pack_inputs converts, tg_unpack_gradients_rgba returns the gradients in the same layout.
  */
 #define TG_INPUT_PACKED 2u
+/*                TG_INFO_MAPPED: info_host is pinned host memory that kernels can write under the same address (what
+ *                cudaHostAlloc gives under unified addressing; the caller vouches for it).  K then comes straight from
+ *                the kernel that counts it instead of by a copy.
+ */
+#define TG_INFO_MAPPED 4u
 size_t tg_forward_workspace_bytes(int T, int tiles, uint32_t list_capacity);
 int tg_render_forward(const float* vertices, const int32_t* indices, const float* colors, const float* opacities,
                       int T, int W, int H, int tile_w, int tile_h, float early_stopping_threshold,

@@ -14,34 +14,32 @@ inline size_t align_up(size_t x, size_t a = 256) { return (x + a - 1) / a * a; }
 
 // Carves the caller's workspace; the same function sizes it.
 struct ForwardWorkspace {
-    uint32_t* tri_offsets;
-    uint64_t* entries;
-    // Everything from `status` up to `clear_end` must be zero when the kernels start: one memset.
-    uint32_t* status;
-    void* scan_scratch;        // binning kernel: finished-CTA counter, totals of its CTAs
-    void* tile_scan_scratch;   // device-wide scan of the tile counts (only beyond kTileScanByLastCta tiles)
+    tg_host::BinBuffers bin = {};
     uint32_t* long_list;       // work lists of the per-tile sort; only their six head words need clearing
-    uint32_t* tile_cursor;     // [tiles]
-    uint32_t* tile_order;      // [tiles] launch order of the compositing kernel, when the binning kernel wrote one
-    char* clear_end;
     size_t total;
 
-    ForwardWorkspace(void* base, int T, int tiles, uint32_t cap) {
+    ForwardWorkspace(void* base, int tiles, uint32_t cap) {
         size_t off = 0;
         auto take = [&](size_t bytes) {
             void* p = base ? (void*)((char*)base + off) : nullptr;
             off += align_up(bytes ? bytes : 1);
             return p;
         };
-        tri_offsets = (uint32_t*)take(sizeof(uint32_t) * ((size_t)T + 2));   // [T] = K, [T+1] = longest tile list
-        entries = (uint64_t*)take(sizeof(uint64_t) * (size_t)cap);
-        status = (uint32_t*)take(sizeof(uint32_t) * 4);
-        scan_scratch = take(tg_host::preprocess_scan_scratch_bytes(T));
-        tile_scan_scratch = take(tiles > tg::kTileScanByLastCta ? tg_scan_scratch_bytes(tiles) : 0);
-        tile_cursor = (uint32_t*)take(sizeof(uint32_t) * (size_t)tiles);
+        const bool device_scan = tiles > tg::kTileScanByLastCta;
+        bin.entries = (uint64_t*)take(sizeof(uint64_t) * (size_t)cap);
+        bin.pairs = (uint4*)take(sizeof(uint4) * (size_t)cap);
+        bin.tables = (float4*)take(sizeof(float4) * ((size_t)tiles + 1));     // tiles_x + tiles_y <= tiles + 1
+        bin.info = (uint32_t*)take(sizeof(uint32_t) * 2);
+        // everything from `status` up to the head of the work lists must be zero when the kernels start: one clear
+        bin.status = (uint32_t*)take(sizeof(uint32_t) * 4);
+        bin.counters = (uint32_t*)take(sizeof(uint32_t) * 2);
+        bin.tile_scan_scratch = take(device_scan ? tg_scan_scratch_bytes(tiles) : 0);
+        bin.tile_counts = (uint32_t*)take(sizeof(uint32_t) * (size_t)tiles);
         long_list = (uint32_t*)take(tg_host::tile_sort_scratch_bytes(tiles));
-        clear_end = (char*)long_list + 6 * sizeof(uint32_t);
-        tile_order = (uint32_t*)take(sizeof(uint32_t) * (size_t)tiles);
+        bin.clear = bin.status;
+        bin.clear_words = base ? (size_t)(long_list + 6 - bin.clear) : 0;
+        bin.tile_order = (uint32_t*)take(sizeof(uint32_t) * (size_t)tiles);
+        if (device_scan) bin.tile_order = nullptr;
         total = off;
     }
 };
@@ -89,45 +87,48 @@ static int build_tile_lists(const float* vertices, const int32_t* indices, const
     TG_REQUIRE(list_capacity < 0x80000000u, "list capacity must stay below 2^31");
     const int tiles_x = (W + tw - 1) / tw, tiles_y = (H + th - 1) / th;
     const int tiles = tiles_x * tiles_y;
-    TG_REQUIRE((flags & ~(unsigned)(TG_FORWARD_CULL_TILES | TG_INPUT_PACKED)) == 0, "unknown flag");
+    TG_REQUIRE((flags & ~(unsigned)(TG_FORWARD_CULL_TILES | TG_INPUT_PACKED | TG_INFO_MAPPED)) == 0, "unknown flag");
     const bool packed = (flags & TG_INPUT_PACKED) != 0;
-    // beyond 65536 tiles the tile counts go through the device-wide scan, which the culling variant does not feed
-    const bool cull = (flags & TG_FORWARD_CULL_TILES) != 0 && tiles <= tg::kTileScanByLastCta;
-    const ForwardWorkspace ws(workspace, T, tiles, list_capacity);
-    *device_status = ws.status;
+    const bool device_scan = tiles > tg::kTileScanByLastCta;
+    // beyond 65536 tiles the lists are the reference's
+    const bool cull = (flags & TG_FORWARD_CULL_TILES) != 0 && !device_scan;
+    const ForwardWorkspace ws(workspace, tiles, list_capacity);
+    // the only kernel of this path that can raise the error word is the scan
+    *device_status = device_scan ? ws.bin.status : nullptr;
     *tile_order_out = nullptr;
     if (workspace_bytes < ws.total) {
         tg_host::set_error("forward workspace: need %zu bytes, got %zu", ws.total, workspace_bytes);
         return TG_ERR_WORKSPACE;
     }
-    info_host[0] = kNotArrived;     // K < 2^31, so this value means "the copy of K has not landed yet"
+    info_host[0] = kNotArrived;     // K < 2^31, so this value means "K has not landed yet"
     info_host[1] = 0;
     info_host[2] = 0;
     TG_REQUIRE(list_capacity == 0 || sorted_ids != nullptr, "null sorted_ids");
-    cudaEvent_t k_ready;
-    if (int st = scratch_event(&k_ready)) return st;
+    // mapped: the binning kernel writes K where the host looks; otherwise a copy brings it
+    const bool mapped = (flags & TG_INFO_MAPPED) != 0 && T > 0;
+    cudaEvent_t k_ready = nullptr;
+    if (!mapped)
+        if (int st = scratch_event(&k_ready)) return st;
 
     timer.mark();                                                    // [0] start of "init"
-    // error word, scan tickets and look-back words, tile counters, head of the sort's work list: one clear
-    TG_CUDA(cudaMemsetAsync(ws.status, 0, (size_t)(ws.clear_end - (char*)ws.status), s));
     timer.mark();                                                    // [1] start of "bary_transforms"
-    // per-triangle records, triangle offsets, per-tile counts and tile offsets
-    int st = tg_host::preprocess_scan(vertices, indices, colors, opacities, T, W, H, tw, th, tri_geo, tri_attr,
-                                      ws.tri_offsets, ws.scan_scratch, ws.status, ws.tile_cursor, offsets,
-                                      ws.tile_scan_scratch, cull, packed, ws.tile_order, s);
+    // per-triangle records, (triangle, tile) pairs with their depth keys, tile offsets
+    int st = tg_host::bin_triangles(vertices, indices, colors, opacities, T, W, H, tw, th, tri_geo, tri_attr, ws.bin,
+                                    offsets, list_capacity, mapped ? info_host : nullptr, cull, packed, s);
     if (st) return st;
     timer.mark();                                                    // [2] start of "per_tile_lists"
-    TG_CUDA(cudaMemcpyAsync(&info_host[0], ws.tri_offsets + T, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    TG_CUDA(cudaEventRecord(k_ready, s));
-    // Entries are written while K travels to the host: the kernel drops those beyond the capacity, and
-    // nothing that reads them is launched before K has been checked.
-    st = tg_host::emit_entries(vertices, indices, T, W, H, tw, th, ws.tri_offsets, ws.scan_scratch, ws.tile_cursor,
-                               ws.entries, list_capacity, cull ? tri_geo : nullptr, packed, s);
+    if (!mapped) {
+        TG_CUDA(cudaMemcpyAsync(&info_host[0], ws.bin.info, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+        TG_CUDA(cudaEventRecord(k_ready, s));
+    }
+    // The entries move to their tiles while K travels to the host: the kernel does nothing when K exceeds the capacity,
+    // and nothing that reads them is launched before K has been checked.
+    st = tg_host::scatter_entries(ws.bin, list_capacity, offsets, tiles, T, s);
     if (st) return st;
-    // K arrives by an 8-byte copy into (preferably pinned) host memory.  Watching the word itself is quicker than
+    // K arrives in (preferably pinned) host memory.  Watching the word itself is quicker than
     // waking up from cudaEventSynchronize (the compositing kernels cannot be launched before K is known, so every
     // microsecond here is an idle GPU once the entry writer has finished); after a bounded while, or for pageable
-    // memory where the copy has completed by now anyway, the event is waited for in the ordinary way, which also
+    // memory where the copy has completed by now anyway, the event (the stream, without a copy) is waited for in the ordinary way, which also
     // surfaces any error of the kernels before it.
     {
         const volatile uint32_t* watched = info_host;
@@ -142,7 +143,7 @@ static int build_tile_lists(const float* vertices, const int32_t* indices, const
             if ((spins & 0xfffu) == 0 && std::chrono::steady_clock::now() - t0 > std::chrono::milliseconds(200)) break;
         }
         std::atomic_thread_fence(std::memory_order_acquire);
-        if (info_host[0] == kNotArrived) TG_CUDA(cudaEventSynchronize(k_ready));
+        if (info_host[0] == kNotArrived) TG_CUDA(mapped ? cudaStreamSynchronize(s) : cudaEventSynchronize(k_ready));
     }
     if (info_host[0] == kNotArrived) {
         tg_host::set_error("the number of list entries never reached the host");
@@ -152,14 +153,14 @@ static int build_tile_lists(const float* vertices, const int32_t* indices, const
     // the longest-list word carries "a launch order of the tiles was written" in its top bit
     const bool have_order = (info_host[1] & tg::kOrderWrittenBit) != 0 && info_host[1] != UINT32_MAX;
     if (info_host[1] != UINT32_MAX) info_host[1] &= ~tg::kOrderWrittenBit;
-    *tile_order_out = have_order ? ws.tile_order : nullptr;
+    *tile_order_out = have_order ? ws.bin.tile_order : nullptr;
     if (K > list_capacity) {
         tg_host::set_error("K = %u exceeds the list capacity %u", K, list_capacity);
         return TG_ERR_CAPACITY;
     }
     timer.mark();                                                    // [3] start of "sorting"
     if (K > 0) {
-        st = tg_host::sort_tile_lists(ws.entries, offsets, tiles, sorted_ids, ws.long_list, true, false, info_host[1], s);
+        st = tg_host::sort_tile_lists(ws.bin.entries, offsets, tiles, sorted_ids, ws.long_list, true, false, info_host[1], s);
         if (st) return st;
     }
     return TG_OK;
@@ -186,9 +187,9 @@ static int finish_timing(StageTimer& timer, float* stage_ms_host, const uint32_t
 extern "C" {
 
 size_t tg_forward_workspace_bytes(int T, int tiles, uint32_t list_capacity) {
-    if (T < 0) T = 0;
     if (tiles < 0) tiles = 0;
-    return ForwardWorkspace(nullptr, T, tiles, list_capacity).total;
+    (void)T;
+    return ForwardWorkspace(nullptr, tiles, list_capacity).total;
 }
 
 int tg_render_forward(const float* vertices, const int32_t* indices, const float* colors, const float* opacities, int T,
@@ -213,7 +214,7 @@ int tg_render_forward(const float* vertices, const int32_t* indices, const float
     if (st) return st;
     timer.mark();                                                    // [5] end
     // device error word: valid on the host once the stream has been synchronised
-    TG_CUDA(cudaMemcpyAsync(&info_host[2], device_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    if (device_status) TG_CUDA(cudaMemcpyAsync(&info_host[2], device_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
     return finish_timing(timer, stage_ms_host, info_host, s);
 }
 
@@ -242,7 +243,7 @@ int tg_render_step_l2(const float* vertices, const int32_t* indices, const float
     tg_host::set_tile_order(nullptr);
     if (st) return st;
     timer.mark();                                                    // [5] end
-    TG_CUDA(cudaMemcpyAsync(&info_host[2], device_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    if (device_status) TG_CUDA(cudaMemcpyAsync(&info_host[2], device_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
     return finish_timing(timer, stage_ms_host, info_host, s);
 }
 

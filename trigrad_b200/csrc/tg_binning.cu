@@ -12,13 +12,15 @@ namespace tg {
 // Stage 1: preprocess.  One thread per triangle: gathers its three vertices and attributes,
 // counts the tiles its bounding box touches and writes the two packed records the compositing
 // kernels stream.  HBM-bound: reads 12 B + 3 gathers of (16+12+4) B, writes 4 + 64 + 96 B.
+struct TriSetup { float m[9], x[3], y[3], z[3]; };    // what the binning kernel needs of a triangle
+
 __device__ __forceinline__ uint32_t preprocess_triangle(int t, const float4* __restrict__ vertices,
                                                         const int* __restrict__ indices,
                                                         const float* __restrict__ colors,
                                                         const float* __restrict__ opacities, int W, int H, int tw,
                                                         int th, int tiles_x, int tiles_y, int4* __restrict__ tri_rects,
                                                         float4* __restrict__ tri_geo, float4* __restrict__ tri_attr,
-                                                        Rect& r, float* m_out = nullptr, bool packed = false) {
+                                                        Rect& r, TriSetup* out = nullptr, bool packed = false) {
     // packed inputs: faces as [T,4] int32 and colours as [V,4] (r, g, b, opacity), one 16-byte load each instead
     // of the reference's 12-byte strides (util.h:457-573); the branch is uniform over the grid
     int ia, ib, ic;
@@ -46,10 +48,7 @@ __device__ __forceinline__ uint32_t preprocess_triangle(int t, const float4* __r
     float m6 = div(sub(a.y, b.y), denom);
     float m7 = div(sub(b.x, a.x), denom);
     float m8 = div(sub(mul(a.x, b.y), mul(b.x, a.y)), denom);
-    if (m_out) {
-        m_out[0] = m0; m_out[1] = m1; m_out[2] = m2; m_out[3] = m3; m_out[4] = m4; m_out[5] = m5; m_out[6] = m6;
-        m_out[7] = m7; m_out[8] = m8;
-    }
+    if (out) *out = {{m0, m1, m2, m3, m4, m5, m6, m7, m8}, {a.x, b.x, c.x}, {a.y, b.y, c.y}, {a.z, b.z, c.z}};
 
     // Lower bound of the per-pixel sort depth: with weights of one sign the interpolated depth is
     // a convex combination of the vertex depths; a relative margin covers fp32 rounding.
@@ -224,108 +223,109 @@ __global__ void __launch_bounds__(32) bounded_wait_selftest_kernel(uint64_t* par
     if (lane_id() == 0) *excl_out = excl;
 }
 
-// Stages 1 and 2 as the forward path runs them: the CTA that preprocesses 256 triangles scans their
-// tile counts among themselves (`tri_offsets[t]` = entries of the CTA's earlier triangles) and leaves
-// its total in `part_total`; no CTA waits for another.  The writer of the entries only needs these local
-// offsets, because it places every entry through its tile's cursor.
-//
-// The CTA also counts its (triangle, tile) entries per tile, one thread per entry, and the CTA that
-// finishes last adds up the totals (K) and turns the tile counts into the exclusive tile offsets, in place
-// (`tile_cursor[t]` = first slot of tile t, advanced later by the entry writer) and in `bin.offsets`.
-struct TileBinArgs {
-    uint32_t* tile_cursor;   // [tiles], zero on entry
-    int32_t* offsets;        // [tiles + 1], written when scan_here
-    uint32_t* done;          // zero on entry: counts finished CTAs
-    int tiles;
-    int scan_here;           // 1: the last CTA scans the tile counts; 0: the host launches a scan
-    uint32_t* longest;       // written when scan_here: the largest tile count
-    uint32_t* part_total;    // [CTAs] entries of each CTA's triangles
-    uint32_t* k_out;         // K = all entries
-    uint32_t* order;         // [tiles] or null: tiles by descending list-length class, written when scan_here and
-                             // the lists are long and uneven enough to matter; *longest then carries kOrderWrittenBit
+// ---- the forward path's binning: shared pieces ------------------------------------------------------------------
+// Pixel-centre extent and NDC borders of every tile column and row, in the exact arithmetic of the coverage test and of
+// the clipper (double divisions): computed once per call instead of once per (triangle, tile) pair.
+struct TileTables {
+    const float4* cols;      // [tiles_x] (first centre, last centre, lower border, upper border)
+    const float4* rows;      // [tiles_y]
 };
 
-// Exclusive scan of cursor[0..tiles) by one CTA of 256 threads, in place, copy in offsets[0..tiles].
-// Rounds of 2048 counts: coalesced loads into shared memory, eight consecutive counts per thread,
-// coalesced stores (a single SM issues too few memory requests per clock for anything strided).
-constexpr int kTileScanRound = 2048;
-__device__ uint32_t tile_offsets_by_one_cta(uint32_t* cursor, int32_t* offsets, int tiles, uint32_t* longest,
-                                        uint32_t* s_buf /*[2048]*/, uint32_t* s_warp /*[8]*/,
-                                        uint32_t* k_out = nullptr) {
-    constexpr int kPer = kTileScanRound / 256;
+__device__ __forceinline__ float4 tile_span(int i, int tile, int extent) {
+    return make_float4(pixel_coord(i * tile, extent), pixel_coord(min((i + 1) * tile, extent) - 1, extent),
+                       sub(mul(div((float)(i * tile), (float)extent), 2.f), 1.f),
+                       sub(mul(div((float)((i + 1) * tile), (float)extent), 2.f), 1.f));
+}
+
+// Clears the counters of the binning kernel and fills the tile tables: first kernel of a forward.
+__global__ void __launch_bounds__(256) bin_init_kernel(uint32_t* __restrict__ clear, size_t clear_words, float4* __restrict__ cols,
+                                                       float4* __restrict__ rows, int tiles_x, int tiles_y, int W, int H,
+                                                       int tw, int th) {
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < clear_words) clear[i] = 0;
+    if (i < (size_t)tiles_x) cols[i] = tile_span((int)i, tw, W);
+    else if (i < (size_t)tiles_x + tiles_y) rows[i - tiles_x] = tile_span((int)(i - tiles_x), th, H);
+}
+
+// Exclusive scan of counts[0..tiles) by one CTA of 256 threads into offsets[0..tiles]; returns the largest count.
+// 16 consecutive counts per thread and round, fetched by four independent 16-byte loads one round ahead: the rounds are
+// bound by the latency of those loads.
+constexpr int kTileScanPer = 16;
+constexpr int kTileScanRound = 256 * kTileScanPer;
+__device__ __forceinline__ void load_counts(const uint32_t* counts, int first, int tiles, uint4 (&v)[4]) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const int i = first + 4 * k;
+        if (i + 3 < tiles) {
+            v[k] = __ldcg(reinterpret_cast<const uint4*>(counts + i));
+        } else {
+            v[k].x = i < tiles ? __ldcg(counts + i) : 0u;
+            v[k].y = i + 1 < tiles ? __ldcg(counts + i + 1) : 0u;
+            v[k].z = i + 2 < tiles ? __ldcg(counts + i + 2) : 0u;
+            v[k].w = 0u;
+        }
+    }
+}
+__device__ uint32_t tile_offsets_by_one_cta(const uint32_t* counts, int32_t* offsets, int tiles, uint32_t* s_warp /*[8]*/) {
     const int tid = threadIdx.x, warp = tid >> 5;
     uint32_t carry = 0, biggest = 0;
+    uint4 ahead[4];
+    load_counts(counts, tid * kTileScanPer, tiles, ahead);
     for (int base = 0; base < tiles; base += kTileScanRound) {
-        __syncthreads();                      // s_buf and s_warp free again
+        const int first = base + tid * kTileScanPer;
+        uint32_t v[kTileScanPer], mine = 0;
 #pragma unroll
-        for (int k = 0; k < kPer; k++) {
-            const int i = base + k * 256 + tid;
-            s_buf[k * 256 + tid] = (i < tiles) ? __ldcg(cursor + i) : 0u;
-        }
-        __syncthreads();
-        uint32_t v[kPer], mine = 0;
+        for (int k = 0; k < 4; k++) { v[4 * k] = ahead[k].x; v[4 * k + 1] = ahead[k].y; v[4 * k + 2] = ahead[k].z; v[4 * k + 3] = ahead[k].w; }
+        if (base + kTileScanRound < tiles) load_counts(counts, first + kTileScanRound, tiles, ahead);
 #pragma unroll
-        for (int k = 0; k < kPer; k++) {
-            v[k] = s_buf[tid * kPer + k];
-            mine += v[k];
-            biggest = max(biggest, v[k]);
-        }
+        for (int k = 0; k < kTileScanPer; k++) { mine += v[k]; biggest = max(biggest, v[k]); }
         uint32_t incl = mine;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
             uint32_t y = __shfl_up_sync(0xffffffffu, incl, d);
             if (lane_id() >= (unsigned)d) incl += y;
         }
+        __syncthreads();                      // s_warp free again
         if (lane_id() == 31) s_warp[warp] = incl;
         __syncthreads();
-        uint32_t warp_off = 0, total = 0;
+        uint32_t run = carry + incl - mine;
 #pragma unroll
         for (int w = 0; w < 8; w++) {
-            uint32_t x = s_warp[w];
-            if (w < warp) warp_off += x;
-            total += x;
+            const uint32_t x = s_warp[w];
+            if (w < warp) run += x;
+            carry += x;
         }
-        uint32_t run = carry + warp_off + incl - mine;
 #pragma unroll
-        for (int k = 0; k < kPer; k++) {
-            s_buf[tid * kPer + k] = run;
-            run += v[k];
-        }
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < kPer; k++) {
-            const int i = base + k * 256 + tid;
-            if (i < tiles) {
-                const uint32_t x = s_buf[k * 256 + tid];
-                cursor[i] = x;
-                offsets[i] = (int32_t)x;
+        for (int k = 0; k < kTileScanPer; k += 4) {
+            const uint4 o = make_uint4(run, run + v[k], run + v[k] + v[k + 1], run + v[k] + v[k + 1] + v[k + 2]);
+            run = o.w + v[k + 3];
+            const int i = first + k;
+            if (i + 3 < tiles && ((uintptr_t)offsets & 15) == 0) {
+                *reinterpret_cast<uint4*>(offsets + i) = o;
+            } else {
+                if (i < tiles) offsets[i] = (int32_t)o.x;
+                if (i + 1 < tiles) offsets[i + 1] = (int32_t)o.y;
+                if (i + 2 < tiles) offsets[i + 2] = (int32_t)o.z;
+                if (i + 3 < tiles) offsets[i + 3] = (int32_t)o.w;
             }
         }
-        carry += total;
     }
-    if (tid == 0) {
-        offsets[tiles] = (int32_t)carry;
-        if (k_out) *k_out = carry;
-    }
+    if (tid == 0) offsets[tiles] = (int32_t)carry;
     biggest = __reduce_max_sync(0xffffffffu, biggest);
     __syncthreads();
     if (lane_id() == 0) s_warp[warp] = biggest;
     __syncthreads();
-    if (tid == 0) {
 #pragma unroll
-        for (int w = 1; w < 8; w++) biggest = max(biggest, s_warp[w]);
-        *longest = biggest;
-        s_warp[0] = biggest;
-    }
-    __syncthreads();
-    return s_warp[0];
+    for (int w = 0; w < 8; w++) biggest = max(biggest, s_warp[w]);
+    return biggest;
 }
 
 // Launch order for the compositing kernel: tiles grouped by the class floor(log2(length)) + 1 of their list length,
 // longest class first (empty tiles last).  With one CTA per tile in scan order a tile whose list is as long as
 // everything else an SM processes can start late and leave the other SMs idle (a view of a fine mesh: 28 % of the
 // SM time); long lists first removes that tail.  Worth its two passes over the offsets only when lists are long and
-// uneven and the tiles are few enough for one CTA (a 1920x1080 image: 8160 tiles, 5 us).
+// uneven and the tiles are few enough for one CTA (a 1920x1080 image: 8160 tiles, 5 us); an extra CTA of the scatter kernel
+// makes it while the others move the entries.
 constexpr uint32_t kOrderMinLongest = 256;
 constexpr int kOrderMaxTiles = 16384;
 constexpr uint32_t kOrderMinMean = 64;
@@ -354,128 +354,6 @@ __device__ void tile_order_by_one_cta(const int32_t* offsets, int tiles, uint32_
         if (cls <= 32 && (int)lane == leader) base = atomicAdd(&s_hist[cls], (uint32_t)__popc(peers));
         base = __shfl_sync(0xffffffffu, base, leader);
         if (cls <= 32) order[base + __popc(peers & lt_mask)] = (uint32_t)i;
-    }
-}
-
-// CULL: a (triangle, tile) pair of the bounding rectangle is counted only if the triangle can cover the centre of
-// some pixel of the tile (rect_may_cover on the tile's pixel-centre rectangle): the exact test the reference
-// leaves open (render.cu:110).  K is then the sum of the tile counts, not of the rectangle sizes.
-// MINB: CTAs per SM the register budget is set for.  Six (40 registers) keeps a mesh of up to 888 x 256 triangles
-// resident in a single wave; larger meshes run several waves anyway and gain from more registers per thread
-// (more of a triangle's gathers in flight at once).
-#ifndef TG_PREPROCESS_MINB_LARGE
-#define TG_PREPROCESS_MINB_LARGE 5
-#endif
-template <bool CULL, int MINB>
-__global__ void __launch_bounds__(256, MINB) preprocess_count_kernel(const float4* __restrict__ vertices,
-                                                               const int* __restrict__ indices,
-                                                               const float* __restrict__ colors,
-                                                               const float* __restrict__ opacities, int T, int W, int H,
-                                                               int tw, int th, int tiles_x, int tiles_y,
-                                                               float4* __restrict__ tri_geo, float4* __restrict__ tri_attr,
-                                                               uint32_t* __restrict__ tri_offsets /*[T], CTA-local*/,
-                                                               TileBinArgs bin, int packed) {
-    __shared__ uint32_t s_warp[8];
-    __shared__ uint32_t s_buf[kTileScanRound];
-    uint32_t* s_loc = s_buf;                 // [257] exclusive offsets of the CTA's triangles within the CTA
-    int* s_rect = (int*)s_buf + 257;         // [768] x0, y0, rows of each triangle's tile rectangle
-    __shared__ bool s_last;
-    __shared__ uint32_t s_k_upper;
-    __shared__ float s_m[CULL ? 9 * 256 : 1];   // barycentric matrices of the CTA's triangles, component-major
-    const int tid = threadIdx.x;
-    const int p = blockIdx.x, num_parts = gridDim.x;
-    const int t = p * 256 + tid;
-    Rect r = {0, 0, 0, 0};
-    float m[9];
-    const uint32_t count = (t < T) ? preprocess_triangle(t, vertices, indices, colors, opacities, W, H, tw, th, tiles_x,
-                                                         tiles_y, nullptr, tri_geo, tri_attr, r, CULL ? m : nullptr, packed != 0)
-                                   : 0u;
-    if (CULL && count) {
-#pragma unroll
-        for (int k = 0; k < 9; k++) s_m[k * 256 + tid] = m[k];
-    }
-    uint32_t incl = count;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        uint32_t y = __shfl_up_sync(0xffffffffu, incl, d);
-        if (lane_id() >= (unsigned)d) incl += y;
-    }
-    const int warp = tid >> 5;
-    if (lane_id() == 31) s_warp[warp] = incl;
-    __syncthreads();
-    uint32_t warp_off = 0, total = 0;
-#pragma unroll
-    for (int w = 0; w < 8; w++) {
-        uint32_t x = s_warp[w];
-        if (w < warp) warp_off += x;
-        total += x;
-    }
-    const uint32_t local_excl = warp_off + incl - count;
-    s_loc[tid] = local_excl;
-    s_rect[3 * tid] = r.x0;
-    s_rect[3 * tid + 1] = r.y0;
-    s_rect[3 * tid + 2] = r.y1 - r.y0 + 1;
-    if (tid == 0) {
-        s_loc[256] = total;
-        bin.part_total[p] = total;
-    }
-    if (t < T) tri_offsets[t] = local_excl;
-    __syncthreads();
-
-    for (uint32_t e = tid; e < total; e += 256) {
-        int lo = 0, hi = 256;                 // largest i with s_loc[i] <= e
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (s_loc[mid] <= e) lo = mid; else hi = mid;
-        }
-        const uint32_t local = e - s_loc[lo];
-        const uint32_t ny = (uint32_t)s_rect[3 * lo + 2];
-        const int tx = s_rect[3 * lo] + (int)(local / ny), ty = s_rect[3 * lo + 1] + (int)(local % ny);
-        if (CULL) {
-            float mm[9];
-#pragma unroll
-            for (int k = 0; k < 9; k++) mm[k] = s_m[k * 256 + lo];
-            if (!rect_may_cover(mm, tile_pixel_rect(tx, ty, W, H, tw, th))) continue;
-        }
-        atomicAdd(&bin.tile_cursor[ty * tiles_x + tx], 1u);
-    }
-    __syncthreads();                          // the CTA's counts are issued; one cumulative fence publishes them
-    if (tid == 0) {
-        __threadfence();
-        s_last = (atomicAdd(bin.done, 1u) == (uint32_t)num_parts - 1u);
-    }
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    // K: sum of the CTA totals
-    uint32_t k = 0;
-    for (int i = tid; i < num_parts; i += 256) k += __ldcg(bin.part_total + i);
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) k += __shfl_xor_sync(0xffffffffu, k, d);
-    __syncthreads();
-    if (lane_id() == 0) s_warp[warp] = k;
-    __syncthreads();
-    if (tid == 0) {
-        k = 0;
-#pragma unroll
-        for (int w = 0; w < 8; w++) k += s_warp[w];
-        if (!CULL) *bin.k_out = k;
-        s_k_upper = k;                       // with culling an upper bound of K (sum of the rectangle sizes)
-    }
-    __syncthreads();
-    if (bin.scan_here) {
-        const uint32_t biggest = tile_offsets_by_one_cta(bin.tile_cursor, bin.offsets, bin.tiles, bin.longest, s_buf, s_warp,
-                                                         CULL ? bin.k_out : nullptr);
-        // the launch order costs two more passes over the offsets: only for images of at most 16384 tiles whose
-        // lists are long on average (from the rectangle sizes) and uneven (the longest one at least 256 entries)
-        if (bin.order && bin.tiles <= kOrderMaxTiles && s_k_upper >= kOrderMinMean * (uint32_t)bin.tiles &&
-            biggest >= kOrderMinLongest) {
-            __syncthreads();                      // the offsets written above are read back by other threads
-            tile_order_by_one_cta(bin.offsets, bin.tiles, bin.order, s_buf);
-            // the host reads the longest list length together with K: its top bit says "an order was written"
-            // (lengths stay below 2^31), so that the compositing kernel is given the order only when there is one
-            if (tid == 0) *bin.longest = biggest | kOrderWrittenBit;
-        }
     }
 }
 
@@ -526,13 +404,9 @@ __device__ __forceinline__ int clip_pass(const float2* in, int n_in, float2* out
     return n_out;
 }
 
-struct TriXYZ { float ax, ay, az, bx, by, bz, cx, cy, cz; };
+struct TriXYZ { float ax, ay, bx, by, cx, cy; };
 
-__device__ float tile_key(const TriXYZ& v, const Plane& pl, int tx, int ty, int W, int H, int tw, int th) {
-    const float xmin = sub(mul(div((float)(tx * tw), (float)W), 2.f), 1.f);
-    const float xmax = sub(mul(div((float)((tx + 1) * tw), (float)W), 2.f), 1.f);
-    const float ymin = sub(mul(div((float)(ty * th), (float)H), 2.f), 1.f);
-    const float ymax = sub(mul(div((float)((ty + 1) * th), (float)H), 2.f), 1.f);
+__device__ float tile_key(const TriXYZ& v, const Plane& pl, float xmin, float xmax, float ymin, float ymax) {
     // triangle entirely inside the tile: the clipper would return it unchanged
     const float lox = fminf(fminf(v.ax, v.bx), v.cx), hix = fmaxf(fmaxf(v.ax, v.bx), v.cx);
     const float loy = fminf(fminf(v.ay, v.by), v.cy), hiy = fmaxf(fmaxf(v.ay, v.by), v.cy);
@@ -558,58 +432,43 @@ __device__ float tile_key(const TriXYZ& v, const Plane& pl, int tx, int ty, int 
     return md;
 }
 
-// One CTA takes 256 consecutive triangles.  Phase 1 (a thread per triangle) gathers the vertices and
-// stages rectangle, depth plane and first output slot in shared memory.  Phase 2 (a thread per
-// OUTPUT entry) finds its triangle by binary search over the staged offsets, so that a triangle
+// Stage entry point: entries with their radix keys in emission order.  One CTA takes 256 consecutive triangles.  Phase 1
+// (a thread per triangle) gathers the vertices and stages rectangle, depth plane and first output slot in shared memory.
+// Phase 2 (a thread per OUTPUT entry) finds its triangle by binary search over the staged offsets, so that a triangle
 // touching many tiles is spread over the whole CTA and no lane idles behind a long neighbour.
-// When `hist.hist` is set the digits of the written keys are counted on the fly, which saves the
-// radix sort its own histogram pass over the keys.
 struct __align__(16) EmitTri {
-    float ax, ay, az, bx, by, bz, cx, cy, cz;
+    float ax, ay, bx, by, cx, cy;
     float A, B, C;
-    int x0, y0, ny, pad;
+    int x0, y0, ny;
 };
-struct EmitMat { float m[9]; };   // CULL only: the triangle's barycentric matrix (from its packed record)
 constexpr int kEmitThreads = 256;
 
-//
-// DIRECT: the tile offsets are known already; every entry takes the next free slot of its tile
-// (`tile_cursor`, arrival order) and is stored there as (ordered depth << 32 | triangle), ready for the
-// per-tile sort.  `keys` is that array, `ids` is unused.
-// CULL (with DIRECT): pairs that the culling preprocess_count_kernel did not count are skipped by the same test.
-template <bool DIRECT, bool CULL>
+__device__ __forceinline__ int find_segment(const uint32_t* first, int n, uint32_t e) {   // largest i with first[i] <= e
+    int lo = 0, hi = n;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (first[mid] <= e) lo = mid; else hi = mid;
+    }
+    return lo;
+}
+
 __global__ void __launch_bounds__(kEmitThreads) emit_keys_kernel(const float4* __restrict__ vertices,
                                                                  const int* __restrict__ indices, int T, int W, int H,
                                                                  int tw, int th, int tiles_x, int tiles_y,
                                                                  const uint32_t* __restrict__ tri_offsets,
                                                                  uint64_t* __restrict__ keys, uint32_t* __restrict__ ids,
-                                                                 uint32_t capacity, HistArgs hist,
-                                                                 uint32_t* __restrict__ tile_cursor,
-                                                                 const uint32_t* __restrict__ part_total,
-                                                                 const float4* __restrict__ tri_geo, int packed) {
+                                                                 uint32_t capacity) {
     __shared__ EmitTri s_tri[kEmitThreads];
-    __shared__ EmitMat s_mat[CULL ? kEmitThreads : 1];
     __shared__ uint32_t s_off[kEmitThreads + 1];
-    __shared__ uint32_t s_hist[DIRECT ? 1 : kMaxPasses * kRadix];     // digit counts of the radix route only
-    __shared__ uint32_t s_warp_tot[kSortWarps];
-    __shared__ bool s_last;
     const int tid = threadIdx.x;
     const int t0 = blockIdx.x * kEmitThreads;
     const int ntri = min(kEmitThreads, T - t0);
-    if (!DIRECT && hist.hist)
-        for (int i = tid; i < hist.passes * kRadix; i += kEmitThreads) s_hist[i] = 0;
     if (tid < ntri) {
         const int t = t0 + tid;
-        int ia, ib, ic;
-        if (packed) {
-            const int4 f = reinterpret_cast<const int4*>(indices)[t];
-            ia = f.x; ib = f.y; ic = f.z;
-        } else {
-            ia = indices[3 * (size_t)t]; ib = indices[3 * (size_t)t + 1]; ic = indices[3 * (size_t)t + 2];
-        }
-        const float4 a = vertices[ia], b = vertices[ib], c = vertices[ic];
+        const float4 a = vertices[indices[3 * (size_t)t]], b = vertices[indices[3 * (size_t)t + 1]],
+                     c = vertices[indices[3 * (size_t)t + 2]];
         EmitTri e;
-        e.ax = a.x; e.ay = a.y; e.az = a.z; e.bx = b.x; e.by = b.y; e.bz = b.z; e.cx = c.x; e.cy = c.y; e.cz = c.z;
+        e.ax = a.x; e.ay = a.y; e.bx = b.x; e.by = b.y; e.cx = c.x; e.cy = c.y;
         Rect r;
         if (tile_rect(a.x, a.y, b.x, b.y, c.x, c.y, W, H, tw, th, tiles_x, tiles_y, r)) {
             const Plane pl = depth_plane(a.x, a.y, a.z, b.x, b.y, b.z, c.x, c.y, c.z);
@@ -617,51 +476,203 @@ __global__ void __launch_bounds__(kEmitThreads) emit_keys_kernel(const float4* _
         } else {
             e.A = e.B = e.C = 0.f;
         }
-        e.x0 = r.x0; e.y0 = r.y0; e.ny = r.y1 - r.y0 + 1; e.pad = 0;
+        e.x0 = r.x0; e.y0 = r.y0; e.ny = r.y1 - r.y0 + 1;
         s_tri[tid] = e;
         s_off[tid] = tri_offsets[t];
-        if (CULL) {
-            const float4 g0 = tri_geo[4 * (size_t)t], g1 = tri_geo[4 * (size_t)t + 1], g2 = tri_geo[4 * (size_t)t + 2];
-            s_mat[tid] = {{g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w, g2.x}};
-        }
     }
-    // DIRECT: the offsets are local to the 256 triangles of the CTA and its total stands in a separate array
-    if (tid == 0) s_off[ntri] = DIRECT ? part_total[blockIdx.x] : tri_offsets[t0 + ntri];
+    if (tid == 0) s_off[ntri] = tri_offsets[t0 + ntri];
     __syncthreads();
     const uint32_t first = s_off[0], total = s_off[ntri] - first;
     for (uint32_t e = tid; e < total; e += kEmitThreads) {
         const uint32_t ge = first + e;
-        // largest i in [0, ntri) with s_off[i] <= ge (triangles without entries have equal offsets)
-        int lo = 0, hi = ntri;
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (s_off[mid] <= ge) lo = mid; else hi = mid;
-        }
+        const int lo = find_segment(s_off, ntri, ge);      // triangles without entries have equal offsets
         const EmitTri& tr = s_tri[lo];
         const uint32_t local = ge - s_off[lo];
         const int tx = tr.x0 + (int)(local / (uint32_t)tr.ny), ty = tr.y0 + (int)(local % (uint32_t)tr.ny);
-        if (CULL && !rect_may_cover(s_mat[lo].m, tile_pixel_rect(tx, ty, W, H, tw, th))) continue;
-        const TriXYZ v = {tr.ax, tr.ay, tr.az, tr.bx, tr.by, tr.bz, tr.cx, tr.cy, tr.cz};
-        const Plane pl = {tr.A, tr.B, tr.C};
-        // DIRECT: the slot does not depend on the key, so its atomic (a round trip to L2) is issued first and
-        // travels while the polygon is clipped
-        uint32_t pos = 0;
-        if (DIRECT) pos = atomicAdd(&tile_cursor[ty * tiles_x + tx], 1u);
-        const float depth = tile_key(v, pl, tx, ty, W, H, tw, th);
-        if (DIRECT) {
-            if (pos < capacity) keys[pos] = ((uint64_t)float_to_ordered(depth) << 32) | (uint32_t)(t0 + lo);
-            continue;
-        }
-        const uint64_t key = ((uint64_t)(uint32_t)(ty * tiles_x + tx) << 32) | float_to_ordered(depth);
+        const float4 cx = tile_span(tx, tw, W), cy = tile_span(ty, th, H);
+        const float depth = tile_key({tr.ax, tr.ay, tr.bx, tr.by, tr.cx, tr.cy}, {tr.A, tr.B, tr.C}, cx.z, cx.w, cy.z, cy.w);
         if (ge < capacity) {                       // the host guarantees K <= capacity before the result is used
-            keys[ge] = key;
+            keys[ge] = ((uint64_t)(uint32_t)(ty * tiles_x + tx) << 32) | float_to_ordered(depth);
             ids[ge] = (uint32_t)(t0 + lo);
-            if (hist.hist) hist_count(s_hist, key, hist);
         }
     }
-    if (!DIRECT && hist.hist) {
+}
+
+// ---- the forward path's binning ----------------------------------------------------------------------------------
+// One pass over the triangles makes everything: the packed records, the (triangle, tile) pairs with their depth keys and
+// the tile counts.  A CTA takes `per_cta` consecutive triangles.  Phase 1, a thread per triangle: gathers, records, tile
+// rectangle; matrix, corners and depth plane stay in shared memory.  Phase 2, a thread per pair of the rectangles: the
+// pairs that are to be listed (all, or with CULL those that can cover a pixel centre of their tile, the exact test the
+// reference leaves open, render.cu:110) go to a queue in shared memory.  Phase 3, a thread per queued pair, so that the
+// clipper runs with full warps: the pair's rank in its tile from one atomic on the tile's count (issued before the clip,
+// which hides its latency), its depth key, and one 16-byte record (key, triangle, tile, rank) to the next free slot.
+// The CTA that finishes last turns the counts into tile offsets; the scatter kernel then moves every entry to
+// offset + rank.  Against counting and writing in two kernels, which gathered, tested and searched twice, B200: 1280
+// triangles 256x256 27 -> 15 us, 200k triangles full HD 65 -> 59, 1.3M triangles 281 -> 235, 3000 large triangles
+// 294 -> 28.
+struct BinArgs {
+    uint32_t* tile_counts;   // [tiles], zero on entry
+    int32_t* offsets;        // [tiles + 1], written when scan_here
+    uint32_t* counters;      // [2], zero on entry: finished CTAs, slots handed out (K in the end)
+    uint32_t* info;          // [2] K, and when scan_here the longest list (kOrderWrittenBit: a launch order is wanted)
+    uint32_t* info_host;     // the same two words in mapped host memory, or null
+    uint4* pairs;            // [capacity]
+    uint32_t capacity;
+    int tiles, tiles_x, tiles_y;
+    int scan_here;           // 1: the last CTA scans the tile counts; 0: the host launches a scan
+    int want_order;
+    TileTables tables;
+};
+
+constexpr int kBinQueue = 1024;
+constexpr int kBinWords = 18;        // matrix 9, corners 6, depth plane 3
+
+template <bool CULL>
+__global__ void __launch_bounds__(256, 4) bin_kernel(const float4* __restrict__ vertices, const int* __restrict__ indices,
+                                                     const float* __restrict__ colors, const float* __restrict__ opacities,
+                                                     int T, int per_cta, int W, int H, int tw, int th,
+                                                     float4* __restrict__ tri_geo, float4* __restrict__ tri_attr,
+                                                     BinArgs bin, int packed) {
+    __shared__ float s_tri[kBinWords][256];
+    __shared__ int s_x0[256], s_y0[256], s_ny[256];
+    __shared__ uint32_t s_loc[257];
+    __shared__ uint32_t s_qx[kBinQueue], s_qy[kBinQueue];     // tile column | tile row << 8 | triangle of the CTA
+    __shared__ uint32_t s_warp[8];
+    __shared__ uint32_t s_queued, s_base;
+    __shared__ bool s_last;
+    const int tid = threadIdx.x, warp = tid >> 5;
+    const int t0 = blockIdx.x * per_cta, ntri = min(per_cta, T - t0);
+    uint32_t count = 0;
+    if (tid < ntri) {
+        Rect r;
+        TriSetup ts;
+        count = preprocess_triangle(t0 + tid, vertices, indices, colors, opacities, W, H, tw, th, bin.tiles_x, bin.tiles_y,
+                                    nullptr, tri_geo, tri_attr, r, &ts, packed != 0);
+        if (count) {
+            const Plane pl = depth_plane(ts.x[0], ts.y[0], ts.z[0], ts.x[1], ts.y[1], ts.z[1], ts.x[2], ts.y[2], ts.z[2]);
+#pragma unroll
+            for (int k = 0; k < 9; k++) s_tri[k][tid] = ts.m[k];
+#pragma unroll
+            for (int k = 0; k < 3; k++) { s_tri[9 + 2 * k][tid] = ts.x[k]; s_tri[10 + 2 * k][tid] = ts.y[k]; }
+            s_tri[15][tid] = pl.A; s_tri[16][tid] = pl.B; s_tri[17][tid] = pl.C;
+            s_x0[tid] = r.x0; s_y0[tid] = r.y0; s_ny[tid] = r.y1 - r.y0 + 1;
+        }
+    }
+    uint32_t incl = count;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        uint32_t y = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane_id() >= (unsigned)d) incl += y;
+    }
+    if (lane_id() == 31) s_warp[warp] = incl;
+    if (tid == 0) s_queued = 0;
+    __syncthreads();
+    uint32_t warp_off = 0, total = 0;
+#pragma unroll
+    for (int w = 0; w < 8; w++) {
+        const uint32_t x = s_warp[w];
+        if (w < warp) warp_off += x;
+        total += x;
+    }
+    s_loc[tid] = warp_off + incl - count;
+    if (tid == 0) s_loc[256] = total;
+    __syncthreads();
+
+    for (uint32_t base = 0; base < total; base += 256) {
+        const uint32_t e = base + tid;
+        bool keep = false;
+        int lo = 0, tx = 0, ty = 0;
+        if (e < total) {
+            lo = find_segment(s_loc, ntri, e);
+            const uint32_t local = e - s_loc[lo], ny = (uint32_t)s_ny[lo];
+            tx = s_x0[lo] + (int)(local / ny);
+            ty = s_y0[lo] + (int)(local % ny);
+            keep = true;
+            if (CULL) {
+                const float4 cx = __ldg(bin.tables.cols + tx), cy = __ldg(bin.tables.rows + ty);
+                float m[9];
+#pragma unroll
+                for (int k = 0; k < 9; k++) m[k] = s_tri[k][lo];
+                keep = rect_may_cover(m, {cx.x, cx.y, cy.x, cy.y});
+            }
+        }
+        const unsigned kept = __ballot_sync(0xffffffffu, keep);
+        uint32_t slot = 0;
+        if (lane_id() == 0 && kept) slot = atomicAdd(&s_queued, (uint32_t)__popc(kept));
+        slot = __shfl_sync(0xffffffffu, slot, 0) + __popc(kept & ((1u << lane_id()) - 1u));
+        if (keep) {
+            s_qx[slot] = (uint32_t)tx;
+            s_qy[slot] = ((uint32_t)ty << 8) | (uint32_t)lo;
+        }
         __syncthreads();
-        hist_flush_and_finish(s_hist, s_warp_tot, &s_last, hist);
+        const uint32_t queued = s_queued;
+        if (queued == 0 || (queued + 256 <= kBinQueue && base + 256 < total)) {
+            __syncthreads();              // everyone has read s_queued before the next round adds to it
+            continue;
+        }
+        if (tid == 0) s_base = atomicAdd(bin.counters + 1, queued);
+        __syncthreads();
+        for (uint32_t q = tid; q < queued; q += 256) {
+            const int qx = (int)s_qx[q], qy = (int)(s_qy[q] >> 8), lt = (int)(s_qy[q] & 255u);
+            const uint32_t tile = (uint32_t)(qy * bin.tiles_x + qx);
+            const uint32_t rank = atomicAdd(bin.tile_counts + tile, 1u);
+            const float4 cx = __ldg(bin.tables.cols + qx), cy = __ldg(bin.tables.rows + qy);
+            const TriXYZ v = {s_tri[9][lt], s_tri[10][lt], s_tri[11][lt], s_tri[12][lt], s_tri[13][lt], s_tri[14][lt]};
+            const Plane pl = {s_tri[15][lt], s_tri[16][lt], s_tri[17][lt]};
+            const float depth = tile_key(v, pl, cx.z, cx.w, cy.z, cy.w);
+            const uint32_t pos = s_base + q;
+            if (pos < bin.capacity)          // the host checks K before anything that reads the entries is used
+                bin.pairs[pos] = make_uint4((uint32_t)(t0 + lt), float_to_ordered(depth), tile, rank);
+        }
+        __syncthreads();
+        if (tid == 0) s_queued = 0;
+        __syncthreads();
+    }
+    __syncthreads();                          // the CTA's counts are issued; one cumulative fence publishes them
+    if (tid == 0) {
+        __threadfence();
+        s_last = (atomicAdd(bin.counters, 1u) == gridDim.x - 1u);
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    const uint32_t K = __ldcg(bin.counters + 1);
+    uint32_t longest = UINT32_MAX;            // not known
+    if (bin.scan_here) {
+        longest = tile_offsets_by_one_cta(bin.tile_counts, bin.offsets, bin.tiles, s_warp);
+        // the launch order costs two passes over the offsets: only for images of at most 16384 tiles whose lists are
+        // long on average and uneven (the longest one at least 256 entries)
+        if (bin.want_order && bin.tiles <= kOrderMaxTiles && K >= kOrderMinMean * (uint32_t)bin.tiles && longest >= kOrderMinLongest)
+            longest |= kOrderWrittenBit;
+    }
+    if (tid == 0) {
+        bin.info[0] = K;
+        bin.info[1] = longest;
+        if (bin.info_host) {                  // K last: the host watches that word
+            *(volatile uint32_t*)(bin.info_host + 1) = longest;
+            __threadfence_system();
+            *(volatile uint32_t*)bin.info_host = K;
+        }
+    }
+}
+
+// Every entry to its place: offset of its tile plus its rank there.  The last CTA makes the launch order of the
+// compositing kernel instead when one is wanted.
+__global__ void __launch_bounds__(256) scatter_entries_kernel(const uint4* __restrict__ pairs, const uint32_t* __restrict__ info,
+                                                              uint32_t capacity, const int32_t* __restrict__ offsets,
+                                                              uint64_t* __restrict__ entries, uint32_t* __restrict__ order,
+                                                              int tiles) {
+    __shared__ uint32_t s_hist[33];
+    const uint32_t K = info[0];
+    if (K > capacity) return;
+    if (blockIdx.x == gridDim.x - 1) {
+        if (order && info[1] != UINT32_MAX && (info[1] & kOrderWrittenBit)) tile_order_by_one_cta(offsets, tiles, order, s_hist);
+        return;
+    }
+    const uint32_t stride = (gridDim.x - 1) * 256;
+    for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < K; i += stride) {
+        const uint4 p = pairs[i];
+        entries[(uint32_t)__ldg(offsets + p.z) + p.w] = ((uint64_t)p.y << 32) | p.x;
     }
 }
 
@@ -713,100 +724,63 @@ static int check_dims_internal(int T, int W, int H, int tw, int th) {
     return TG_OK;
 }
 
-// finished-CTA counter (4, zero on entry) + pad (4) + one total per CTA of 256 triangles
-size_t preprocess_scan_scratch_bytes(int T) { return 8 + 4 * ((size_t)(T > 0 ? (T + 255) / 256 : 0) + 1); }
-
-// Per-triangle records, CTA-local triangle offsets (`tri_offsets[T + 2]`: [t] local to the triangle's
-// CTA of 256, [T] = K, [T + 1] = longest tile list), tile offsets in `tile_cursor[tiles]` and
-// `offsets[tiles + 1]`.  The first word of `scratch` and `tile_cursor` must have been zeroed by the caller.
-// Beyond kTileScanByLastCta tiles a device-wide scan makes the tile offsets, for which `tile_scan_scratch`
-// (zeroed, tg_scan_scratch_bytes(tiles) bytes) is needed, and [T + 1] is set to UINT32_MAX (not known).
-int preprocess_scan(const float* vertices, const int32_t* indices, const float* colors, const float* opacities, int T,
-                    int W, int H, int tw, int th, float* tri_geo, float* tri_attr, uint32_t* tri_offsets, void* scratch,
-                    uint32_t* status, uint32_t* tile_cursor, int32_t* offsets, void* tile_scan_scratch, bool cull,
-                    bool packed, uint32_t* tile_order, cudaStream_t stream) {
+// Per-triangle records, (triangle, tile) pairs and tile offsets: bin_init_kernel, bin_kernel and scatter_entries_kernel
+// (declared in tg_common.cuh with what each argument is).
+int bin_triangles(const float* vertices, const int32_t* indices, const float* colors, const float* opacities, int T, int W,
+                  int H, int tw, int th, float* tri_geo, float* tri_attr, const BinBuffers& b, int32_t* offsets,
+                  uint32_t list_capacity, uint32_t* info_host, bool cull, bool packed, cudaStream_t stream) {
     if (int s = check_dims_internal(T, W, H, tw, th)) return s;
-    TG_REQUIRE(tri_offsets && scratch && status && tile_cursor && offsets, "null pointer");
+    TG_REQUIRE(offsets, "null pointer");
     const int tiles_x = (W + tw - 1) / tw, tiles_y = (H + th - 1) / th;
     const int tiles = tiles_x * tiles_y;
-    if (T == 0) {
-        TG_CUDA(cudaMemsetAsync(tri_offsets, 0, sizeof(uint32_t) * 2, stream));
-        TG_CUDA(cudaMemsetAsync(offsets, 0, sizeof(int32_t) * ((size_t)tiles + 1), stream));
-        return TG_OK;
-    }
-    TG_REQUIRE(vertices && indices && colors && (packed || opacities) && tri_geo && tri_attr, "null pointer");
+    TG_REQUIRE(T == 0 || (vertices && indices && colors && (packed || opacities) && tri_geo && tri_attr), "null pointer");
     TG_REQUIRE(((uintptr_t)vertices & 15) == 0 && ((uintptr_t)tri_geo & 15) == 0 && ((uintptr_t)tri_attr & 15) == 0,
                "vertices / tri_geo / tri_attr must be 16-byte aligned");
     TG_REQUIRE(!packed || ((((uintptr_t)indices | (uintptr_t)colors) & 15) == 0),
                "packed faces [T,4] and colours [V,4] must be 16-byte aligned");
     const bool by_last_cta = tiles <= tg::kTileScanByLastCta;
-    TG_REQUIRE(by_last_cta || tile_scan_scratch, "null tile scan scratch");
-    const tg::TileBinArgs bin = {tile_cursor, offsets, (uint32_t*)scratch, tiles, by_last_cta ? 1 : 0,
-                                 tri_offsets + T + 1, (uint32_t*)scratch + 2, tri_offsets + T,
-                                 by_last_cta ? tile_order : nullptr};
     TG_REQUIRE(!cull || by_last_cta, "tile culling is limited to 65536 tiles");
-    const int grid = (T + 255) / 256;
-    const bool one_wave = grid <= 148 * 6;      // all CTAs resident at once at six per SM
-#define TG_LAUNCH_PREPROCESS(CULLV, MINBV)                                                                             \
-    tg::preprocess_count_kernel<CULLV, MINBV><<<grid, 256, 0, stream>>>(                                               \
-        (const float4*)vertices, indices, colors, opacities, T, W, H, tw, th, tiles_x, tiles_y, (float4*)tri_geo,      \
-        (float4*)tri_attr, tri_offsets, bin, packed ? 1 : 0)
-    if (cull) {
-        if (one_wave) TG_LAUNCH_PREPROCESS(true, 6); else TG_LAUNCH_PREPROCESS(true, TG_PREPROCESS_MINB_LARGE);
-    } else {
-        if (one_wave) TG_LAUNCH_PREPROCESS(false, 6); else TG_LAUNCH_PREPROCESS(false, TG_PREPROCESS_MINB_LARGE);
+    float4* rows = b.tables + tiles_x;
+    const size_t init = b.clear_words > (size_t)tiles_x + tiles_y ? b.clear_words : (size_t)tiles_x + tiles_y;
+    tg::bin_init_kernel<<<(unsigned)((init + 255) / 256), 256, 0, stream>>>(b.clear, b.clear_words, b.tables, rows, tiles_x,
+                                                                          tiles_y, W, H, tw, th);
+    TG_LAUNCH_CHECK("bin_init_kernel");
+    if (T == 0) {
+        TG_CUDA(cudaMemsetAsync(b.info, 0, sizeof(uint32_t) * 2, stream));
+        TG_CUDA(cudaMemsetAsync(offsets, 0, sizeof(int32_t) * ((size_t)tiles + 1), stream));
+        return TG_OK;
     }
-#undef TG_LAUNCH_PREPROCESS
-    TG_LAUNCH_CHECK("preprocess_count_kernel");
+    const tg::BinArgs bin = {b.tile_counts, offsets, b.counters, b.info, info_host, b.pairs, list_capacity, tiles, tiles_x,
+                             tiles_y, by_last_cta ? 1 : 0, b.tile_order ? 1 : 0, {b.tables, rows}};
+    // Triangles per CTA: 256 where that fills the GPU; fewer below, so that a mesh of few triangles that cover many tiles
+    // each still spreads over all SMs (four CTAs on each).
+    constexpr int kWave = 148 * 4;
+    const int per_cta = T >= 256 * kWave ? 256 : (T + kWave - 1) / kWave;
+    const int grid = (T + per_cta - 1) / per_cta;
+    auto kernel = cull ? tg::bin_kernel<true> : tg::bin_kernel<false>;
+    kernel<<<grid, 256, 0, stream>>>((const float4*)vertices, indices, colors, opacities, T, per_cta, W, H, tw, th,
+                                     (float4*)tri_geo, (float4*)tri_attr, bin, packed ? 1 : 0);
+    TG_LAUNCH_CHECK("bin_kernel");
     if (!by_last_cta) {
-        // counts -> offsets by the device-wide scan, then the cursors start at the offsets
         const int parts = (tiles + tg::kScanTile - 1) / tg::kScanTile;
-        tg::scan_kernel<<<parts, tg::kScanThreads, 0, stream>>>(tile_cursor, (uint32_t*)offsets, tiles, parts,
-                                                                 (uint32_t*)tile_scan_scratch,
-                                                                 (uint64_t*)((char*)tile_scan_scratch + 8), status);
+        tg::scan_kernel<<<parts, tg::kScanThreads, 0, stream>>>(b.tile_counts, (uint32_t*)offsets, tiles, parts,
+                                                                 (uint32_t*)b.tile_scan_scratch,
+                                                                 (uint64_t*)((char*)b.tile_scan_scratch + 8), b.status);
         TG_LAUNCH_CHECK("scan_kernel");
-        TG_CUDA(cudaMemcpyAsync(tile_cursor, offsets, sizeof(uint32_t) * (size_t)tiles, cudaMemcpyDeviceToDevice, stream));
-        TG_CUDA(cudaMemsetAsync(tri_offsets + T + 1, 0xff, sizeof(uint32_t), stream));
     }
     return TG_OK;
 }
 
-int emit_keys(const float* vertices, const int32_t* indices, int T, int W, int H, int tw, int th,
-              const uint32_t* tri_offsets, uint64_t* keys, uint32_t* ids, uint32_t capacity, const tg::HistArgs& hist,
-              cudaStream_t stream) {
-    if (int s = check_dims_internal(T, W, H, tw, th)) return s;
-    if (T == 0) return TG_OK;
-    TG_REQUIRE(vertices && indices && tri_offsets && keys && ids, "null pointer");
-    const int tiles_x = (W + tw - 1) / tw, tiles_y = (H + th - 1) / th;
-    tg::emit_keys_kernel<false, false><<<(T + tg::kEmitThreads - 1) / tg::kEmitThreads, tg::kEmitThreads, 0, stream>>>(
-        (const float4*)vertices, indices, T, W, H, tw, th, tiles_x, tiles_y, tri_offsets, keys, ids, capacity, hist,
-        nullptr, nullptr, nullptr, 0);
-    TG_LAUNCH_CHECK("emit_keys_kernel");
+int scatter_entries(const BinBuffers& b, uint32_t list_capacity, const int32_t* offsets, int tiles, int T, cudaStream_t stream) {
+    if (T == 0 || list_capacity == 0) return TG_OK;
+    // K is not known on the host yet: as many CTAs as its upper bound fills, at most four per SM, and one for the order
+    const uint32_t want = (list_capacity + 1023) / 1024;
+    const int grid = (int)(want < 148 * 4 ? want : 148 * 4) + 1;
+    tg::scatter_entries_kernel<<<grid, 256, 0, stream>>>(b.pairs, b.info, list_capacity, offsets, b.entries, b.tile_order, tiles);
+    TG_LAUNCH_CHECK("scatter_entries_kernel");
     return TG_OK;
 }
 
-// Entries written straight into their tile's segment of `entries` (capacity slots), unsorted within it.
-// `tri_offsets` and `scan_scratch` as preprocess_scan left them (CTA-local offsets, CTA totals).
-int emit_entries(const float* vertices, const int32_t* indices, int T, int W, int H, int tw, int th,
-                 const uint32_t* tri_offsets, const void* scan_scratch, uint32_t* tile_cursor, uint64_t* entries,
-                 uint32_t capacity, const float* tri_geo_for_cull, bool packed, cudaStream_t stream) {
-    if (int s = check_dims_internal(T, W, H, tw, th)) return s;
-    if (T == 0 || capacity == 0) return TG_OK;
-    TG_REQUIRE(vertices && indices && tri_offsets && scan_scratch && tile_cursor && entries, "null pointer");
-    const int tiles_x = (W + tw - 1) / tw, tiles_y = (H + th - 1) / th;
-    const tg::HistArgs none = {nullptr, nullptr, 0, 0, 0};
-    const int grid = (T + tg::kEmitThreads - 1) / tg::kEmitThreads;
-    if (tri_geo_for_cull)
-        tg::emit_keys_kernel<true, true><<<grid, tg::kEmitThreads, 0, stream>>>(
-            (const float4*)vertices, indices, T, W, H, tw, th, tiles_x, tiles_y, tri_offsets, entries, nullptr, capacity,
-            none, tile_cursor, (const uint32_t*)scan_scratch + 2, (const float4*)tri_geo_for_cull, packed ? 1 : 0);
-    else
-        tg::emit_keys_kernel<true, false><<<grid, tg::kEmitThreads, 0, stream>>>(
-            (const float4*)vertices, indices, T, W, H, tw, th, tiles_x, tiles_y, tri_offsets, entries, nullptr, capacity,
-            none, tile_cursor, (const uint32_t*)scan_scratch + 2, nullptr, packed ? 1 : 0);
-    TG_LAUNCH_CHECK("emit_entries_kernel");
-    return TG_OK;
-}
 static std::atomic<unsigned long long> g_launches{0};
 void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 }  // namespace tg_host
@@ -967,9 +941,14 @@ int tg_selftest_bounded_wait(void* scratch, size_t scratch_bytes, uint32_t* stat
 
 int tg_emit_keys(const float* vertices, const int32_t* indices, int T, int W, int H, int tw, int th,
                  const uint32_t* tri_offsets, uint64_t* keys, uint32_t* ids, uint32_t capacity, tg_stream_t stream) {
-    const tg::HistArgs no_hist = {nullptr, nullptr, 0, 0, 0};
-    return tg_host::emit_keys(vertices, indices, T, W, H, tw, th, tri_offsets, keys, ids, capacity, no_hist,
-                              (cudaStream_t)stream);
+    if (int s = check_dims(T, W, H, tw, th)) return s;
+    if (T == 0) return TG_OK;
+    TG_REQUIRE(vertices && indices && tri_offsets && keys && ids, "null pointer");
+    const int tiles_x = (W + tw - 1) / tw, tiles_y = (H + th - 1) / th;
+    tg::emit_keys_kernel<<<(T + tg::kEmitThreads - 1) / tg::kEmitThreads, tg::kEmitThreads, 0, (cudaStream_t)stream>>>(
+        (const float4*)vertices, indices, T, W, H, tw, th, tiles_x, tiles_y, tri_offsets, keys, ids, capacity);
+    TG_LAUNCH_CHECK("emit_keys_kernel");
+    return TG_OK;
 }
 
 int tg_tile_ranges(const uint64_t* sorted_keys, uint32_t n, int tiles, int32_t* offsets, tg_stream_t stream) {

@@ -1,5 +1,4 @@
-// Radix-sort constants and the digit-histogram helpers shared by the sort kernels and by the key
-// emission kernel (which can count the digits of the keys it writes, saving one read of them).
+// Radix-sort constants and digit-histogram helpers, and the host functions that the .cu files share.
 #pragma once
 #include "tg_common.cuh"
 
@@ -84,23 +83,31 @@ __device__ __forceinline__ void hist_flush_and_finish(uint32_t* s_hist, uint32_t
 
 namespace tg_host {
 // Internal (not part of the C ABI): the pieces tg_render_forward strings together.
-int emit_keys(const float* vertices, const int32_t* indices, int T, int W, int H, int tw, int th,
-              const uint32_t* tri_offsets, uint64_t* keys, uint32_t* ids, uint32_t capacity, const tg::HistArgs& hist,
-              cudaStream_t stream);
 int sort_pairs(uint64_t* keys_a, uint64_t* keys_b, uint32_t* vals_a, uint32_t* vals_b, uint32_t n, int begin_bit,
                int end_bit, void* scratch, size_t scratch_bytes, uint32_t* status, int* result_in_b_host,
                bool scratch_prepared, cudaStream_t stream);
 size_t sort_scratch_clear_bytes(uint32_t n, int passes);
-size_t preprocess_scan_scratch_bytes(int T);
-int preprocess_scan(const float* vertices, const int32_t* indices, const float* colors, const float* opacities, int T,
-                    int W, int H, int tw, int th, float* tri_geo, float* tri_attr, uint32_t* tri_offsets, void* scratch,
-                    uint32_t* status, uint32_t* tile_cursor, int32_t* offsets, void* tile_scan_scratch, bool cull,
-                    bool packed, uint32_t* tile_order, cudaStream_t stream);
-int emit_entries(const float* vertices, const int32_t* indices, int T, int W, int H, int tw, int th,
-                 const uint32_t* tri_offsets, const void* scan_scratch, uint32_t* tile_cursor, uint64_t* entries,
-                 uint32_t capacity, const float* tri_geo_for_cull, bool packed, cudaStream_t stream);
 void set_tile_order(const uint32_t* order, uint32_t longest_list = 0);
 size_t tile_sort_scratch_bytes(int tiles);
+// Workspace of the binning kernels (bin_triangles, scatter_entries).
+struct BinBuffers {
+    uint32_t* clear;             // zeroed by the first kernel: `clear_words` words that hold the next three and the head
+    size_t clear_words;          //   words of the sort's work lists
+    uint32_t* status;            // device error word
+    uint32_t* counters;          // [2]
+    uint32_t* tile_counts;       // [tiles], 16-byte aligned
+    void* tile_scan_scratch;     // device-wide scan of the tile counts, only beyond kTileScanByLastCta tiles; zeroed too
+    float4* tables;              // [tiles_x + tiles_y]
+    uint32_t* info;              // [2] K, longest list (UINT32_MAX: not known)
+    uint4* pairs;                // [list capacity]
+    uint64_t* entries;           // [list capacity]
+    uint32_t* tile_order;        // [tiles] or null
+};
+// `info_host`: mapped host memory that receives the two info words (K last), or null.
+int bin_triangles(const float* vertices, const int32_t* indices, const float* colors, const float* opacities, int T, int W,
+                  int H, int tw, int th, float* tri_geo, float* tri_attr, const BinBuffers& b, int32_t* offsets,
+                  uint32_t list_capacity, uint32_t* info_host, bool cull, bool packed, cudaStream_t stream);
+int scatter_entries(const BinBuffers& b, uint32_t list_capacity, const int32_t* offsets, int tiles, int T, cudaStream_t stream);
 int sort_tile_lists(uint64_t* entries, const int32_t* offsets, int tiles, int32_t* sorted_ids, uint32_t* lists,
                     bool scratch_prepared, bool write_back, uint32_t longest, cudaStream_t stream);
 }  // namespace tg_host

@@ -260,7 +260,7 @@ ForwardOut forward(const Tensor& vertices_, const Tensor& indices_, const Tensor
     if (planes > 0 && planes * v.pixels() * 4 <= selection_max_bytes)
         s.selection = at::empty({planes, v.H, v.W}, options.dtype(at::kInt));
     if (record_timing) out.stage_ms.resize(5);
-    const unsigned flags = (cull ? TG_FORWARD_CULL_TILES : 0u) | (packed ? TG_INPUT_PACKED : 0u);
+    const unsigned flags = (cull ? TG_FORWARD_CULL_TILES : 0u) | (packed ? TG_INPUT_PACKED : 0u) | TG_INFO_MAPPED;
     const auto state = state_of(w.device, w.stream);
     std::lock_guard<std::mutex> lock(state->use);
     int64_t cap = std::max<int64_t>(state->k_estimate + state->k_estimate / 4 + 1024, 2 * (int64_t)T + 1024);
