@@ -265,11 +265,12 @@ int tg_blend_step_l2(const float* tri_geo, const float* tri_attr, const int32_t*
  *                the first word, so pinned memory makes this quick; the reference synchronises at the same
  *                point, src/trigrad/render.cu:290).  [2] receives the device error
  *                word (0 = fine) by an asynchronous copy: it is valid after the caller next
- *                synchronises the stream.  [3] is not used.
+ *                synchronises the stream.  [3] receives, with K, the number of list slots the call used: K plus the
+ *                pairs that TG_FORWARD_CULL_TILES dropped.
  *   stage_ms_host  NULL or float[5]: milliseconds of {init, per_tile_lists, sorting,
  *                bary_transforms, rasterization} measured with CUDA events (synchronises)
- * If K > list_capacity nothing past the scan is run and TG_ERR_CAPACITY is returned with info_host[0]
- * set; call again with a larger list and workspace.
+ * If the slots exceed list_capacity nothing past the binning is run and TG_ERR_CAPACITY is returned with the
+ * capacity needed in info_host[0]; call again with a larger list and workspace.
  *   flags        0, or TG_FORWARD_CULL_TILES: a (triangle, tile) pair of the bounding rectangle is listed only if
  *                the triangle can cover the centre of some pixel of that tile - the exact overlap test the
  *                reference leaves as a TODO (src/trigrad/render.cu:110; its lists hold every tile of the bounding

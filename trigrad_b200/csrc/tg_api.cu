@@ -29,7 +29,7 @@ struct ForwardWorkspace {
         bin.entries = (uint64_t*)take(sizeof(uint64_t) * (size_t)cap);
         bin.pairs = (uint4*)take(sizeof(uint4) * (size_t)cap);
         bin.tables = (float4*)take(sizeof(float4) * ((size_t)tiles + 1));     // tiles_x + tiles_y <= tiles + 1
-        bin.info = (uint32_t*)take(sizeof(uint32_t) * 2);
+        bin.info = (uint32_t*)take(sizeof(uint32_t) * 3);
         // everything from `status` up to the head of the work lists must be zero when the kernels start: one clear
         bin.status = (uint32_t*)take(sizeof(uint32_t) * 4);
         bin.counters = (uint32_t*)take(sizeof(uint32_t) * 2);
@@ -103,6 +103,7 @@ static int build_tile_lists(const float* vertices, const int32_t* indices, const
     info_host[0] = kNotArrived;     // K < 2^31, so this value means "K has not landed yet"
     info_host[1] = 0;
     info_host[2] = 0;
+    info_host[3] = 0;
     TG_REQUIRE(list_capacity == 0 || sorted_ids != nullptr, "null sorted_ids");
     // mapped: the binning kernel writes K where the host looks; otherwise a copy brings it
     const bool mapped = (flags & TG_INFO_MAPPED) != 0 && T > 0;
@@ -118,6 +119,8 @@ static int build_tile_lists(const float* vertices, const int32_t* indices, const
     if (st) return st;
     timer.mark();                                                    // [2] start of "per_tile_lists"
     if (!mapped) {
+        // [3] first: the host watches the word K arrives in
+        TG_CUDA(cudaMemcpyAsync(&info_host[3], ws.bin.info + 2, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
         TG_CUDA(cudaMemcpyAsync(&info_host[0], ws.bin.info, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
         TG_CUDA(cudaEventRecord(k_ready, s));
     }
@@ -154,8 +157,10 @@ static int build_tile_lists(const float* vertices, const int32_t* indices, const
     const bool have_order = (info_host[1] & tg::kOrderWrittenBit) != 0 && info_host[1] != UINT32_MAX;
     if (info_host[1] != UINT32_MAX) info_host[1] &= ~tg::kOrderWrittenBit;
     *tile_order_out = have_order ? ws.bin.tile_order : nullptr;
-    if (K > list_capacity) {
-        tg_host::set_error("K = %u exceeds the list capacity %u", K, list_capacity);
+    const uint32_t slots = info_host[3];            // K and the holes of culled pairs
+    if (K > list_capacity || slots > list_capacity) {
+        info_host[0] = K > slots ? K : slots;
+        tg_host::set_error("%u entries and culled pairs exceed the list capacity %u", info_host[0], list_capacity);
         return TG_ERR_CAPACITY;
     }
     timer.mark();                                                    // [3] start of "sorting"

@@ -9,33 +9,51 @@
 namespace tg {
 
 // ================================================================================================
-// Stage 1: preprocess.  One thread per triangle: gathers its three vertices and attributes,
-// counts the tiles its bounding box touches and writes the two packed records the compositing
-// kernels stream.  HBM-bound: reads 12 B + 3 gathers of (16+12+4) B, writes 4 + 64 + 96 B.
-struct TriSetup { float m[9], x[3], y[3], z[3]; };    // what the binning kernel needs of a triangle
-
-__device__ __forceinline__ uint32_t preprocess_triangle(int t, const float4* __restrict__ vertices,
-                                                        const int* __restrict__ indices,
-                                                        const float* __restrict__ colors,
-                                                        const float* __restrict__ opacities, int W, int H, int tw,
-                                                        int th, int tiles_x, int tiles_y, int4* __restrict__ tri_rects,
-                                                        float4* __restrict__ tri_geo, float4* __restrict__ tri_attr,
-                                                        Rect& r, TriSetup* out = nullptr, bool packed = false) {
-    // packed inputs: faces as [T,4] int32 and colours as [V,4] (r, g, b, opacity), one 16-byte load each instead
-    // of the reference's 12-byte strides (util.h:457-573); the branch is uniform over the grid
+// Stage 1: a triangle's gathers and its two packed records (64 and 96 bytes), which the compositing kernels stream.
+struct TriInput {
     int ia, ib, ic;
+    float4 a, b, c;         // vertices
+    float4 ra, rb, rc;      // (r, g, b, opacity)
+};
+
+// packed inputs: faces as [T,4] int32 and colours as [V,4] (r, g, b, opacity), one 16-byte load each instead of the
+// reference's 12-byte strides (util.h:457-573); the branch is uniform over the grid
+__device__ __forceinline__ TriInput load_triangle(int t, const float4* __restrict__ vertices, const int* __restrict__ indices,
+                                                  const float* __restrict__ colors, const float* __restrict__ opacities,
+                                                  bool packed) {
+    TriInput in;
     if (packed) {
         const int4 f = reinterpret_cast<const int4*>(indices)[t];
-        ia = f.x; ib = f.y; ic = f.z;
+        in.ia = f.x; in.ib = f.y; in.ic = f.z;
     } else {
-        ia = indices[3 * (size_t)t]; ib = indices[3 * (size_t)t + 1]; ic = indices[3 * (size_t)t + 2];
+        in.ia = indices[3 * (size_t)t]; in.ib = indices[3 * (size_t)t + 1]; in.ic = indices[3 * (size_t)t + 2];
     }
-    float4 a = vertices[ia], b = vertices[ib], c = vertices[ic];
+    in.a = vertices[in.ia]; in.b = vertices[in.ib]; in.c = vertices[in.ic];
+    if (packed) {
+        const float4* rgba = reinterpret_cast<const float4*>(colors);
+        in.ra = rgba[in.ia]; in.rb = rgba[in.ib]; in.rc = rgba[in.ic];
+    } else {
+        const float* ca = colors + 3 * (size_t)in.ia;
+        const float* cb = colors + 3 * (size_t)in.ib;
+        const float* cc = colors + 3 * (size_t)in.ic;
+        in.ra = make_float4(ca[0], ca[1], ca[2], opacities[in.ia]);
+        in.rb = make_float4(cb[0], cb[1], cb[2], opacities[in.ib]);
+        in.rc = make_float4(cc[0], cc[1], cc[2], opacities[in.ic]);
+    }
+    return in;
+}
 
-    bool ok = tile_rect(a.x, a.y, b.x, b.y, c.x, c.y, W, H, tw, th, tiles_x, tiles_y, r);
-    const uint32_t count = ok ? (uint32_t)(r.x1 - r.x0 + 1) * (uint32_t)(r.y1 - r.y0 + 1) : 0u;
-    if (tri_rects) tri_rects[t] = make_int4(r.x0, r.y0, r.x1, r.y1);
+__device__ __forceinline__ void make_attr(const TriInput& in, float4 (&q)[6]) {
+    q[0] = make_float4(in.ra.w, in.rb.w, in.rc.w, in.ra.x);
+    q[1] = make_float4(in.ra.y, in.ra.z, in.rb.x, in.rb.y);
+    q[2] = make_float4(in.rb.z, in.rc.x, in.rc.y, in.rc.z);
+    q[3] = make_float4(div(1.f, in.a.w), div(1.f, in.b.w), div(1.f, in.c.w), __int_as_float(in.ia));
+    q[4] = make_float4(__int_as_float(in.ib), __int_as_float(in.ic), in.a.x, in.a.y);
+    q[5] = make_float4(in.b.x, in.b.y, in.c.x, in.c.y);
+}
 
+__device__ __forceinline__ void make_geo(const TriInput& in, float4 (&g)[4]) {
+    const float4 a = in.a, b = in.b, c = in.c;
     // barycentric matrix, reference render.cu:324-336: plain mul/sub/div
     float denom = add(add(mul(a.x, sub(b.y, c.y)), mul(b.x, sub(c.y, a.y))), mul(c.x, sub(a.y, b.y)));
     if (fabsf(denom) < kEffZero) denom = 1.0f;
@@ -48,8 +66,6 @@ __device__ __forceinline__ uint32_t preprocess_triangle(int t, const float4* __r
     float m6 = div(sub(a.y, b.y), denom);
     float m7 = div(sub(b.x, a.x), denom);
     float m8 = div(sub(mul(a.x, b.y), mul(b.x, a.y)), denom);
-    if (out) *out = {{m0, m1, m2, m3, m4, m5, m6, m7, m8}, {a.x, b.x, c.x}, {a.y, b.y, c.y}, {a.z, b.z, c.z}};
-
     // Lower bound of the per-pixel sort depth: with weights of one sign the interpolated depth is
     // a convex combination of the vertex depths; a relative margin covers fp32 rounding.
     float zlow = -INFINITY;
@@ -60,33 +76,10 @@ __device__ __forceinline__ uint32_t preprocess_triangle(int t, const float4* __r
         float lo = zmin - 4e-6f * zabs;
         if (isfinite(lo)) zlow = lo;
     }
-
-    float4* g = tri_geo + 4 * (size_t)t;
     g[0] = make_float4(m0, m1, m2, m3);
     g[1] = make_float4(m4, m5, m6, m7);
     g[2] = make_float4(m8, a.z, b.z, c.z);
     g[3] = make_float4(a.w, b.w, c.w, zlow);
-
-    float4* q = tri_attr + 6 * (size_t)t;
-    float4 ra, rb, rc;   // (r, g, b, opacity) of the three vertices
-    if (packed) {
-        const float4* rgba = reinterpret_cast<const float4*>(colors);
-        ra = rgba[ia]; rb = rgba[ib]; rc = rgba[ic];
-    } else {
-        const float* ca = colors + 3 * (size_t)ia;
-        const float* cb = colors + 3 * (size_t)ib;
-        const float* cc = colors + 3 * (size_t)ic;
-        ra = make_float4(ca[0], ca[1], ca[2], opacities[ia]);
-        rb = make_float4(cb[0], cb[1], cb[2], opacities[ib]);
-        rc = make_float4(cc[0], cc[1], cc[2], opacities[ic]);
-    }
-    q[0] = make_float4(ra.w, rb.w, rc.w, ra.x);
-    q[1] = make_float4(ra.y, ra.z, rb.x, rb.y);
-    q[2] = make_float4(rb.z, rc.x, rc.y, rc.z);
-    q[3] = make_float4(div(1.f, a.w), div(1.f, b.w), div(1.f, c.w), __int_as_float(ia));
-    q[4] = make_float4(__int_as_float(ib), __int_as_float(ic), a.x, a.y);
-    q[5] = make_float4(b.x, b.y, c.x, c.y);
-    return count;
 }
 
 __global__ void __launch_bounds__(256) preprocess_kernel(const float4* __restrict__ vertices,
@@ -98,9 +91,18 @@ __global__ void __launch_bounds__(256) preprocess_kernel(const float4* __restric
                                                          float4* __restrict__ tri_geo, float4* __restrict__ tri_attr) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= T) return;
+    const TriInput in = load_triangle(t, vertices, indices, colors, opacities, false);
     Rect r;
-    tri_counts[t] = preprocess_triangle(t, vertices, indices, colors, opacities, W, H, tw, th, tiles_x, tiles_y, tri_rects,
-                                        tri_geo, tri_attr, r);
+    const bool ok = tile_rect(in.a.x, in.a.y, in.b.x, in.b.y, in.c.x, in.c.y, W, H, tw, th, tiles_x, tiles_y, r);
+    tri_counts[t] = ok ? (uint32_t)(r.x1 - r.x0 + 1) * (uint32_t)(r.y1 - r.y0 + 1) : 0u;
+    if (tri_rects) tri_rects[t] = make_int4(r.x0, r.y0, r.x1, r.y1);
+    float4 g[4], q[6];
+    make_geo(in, g);
+    make_attr(in, q);
+#pragma unroll
+    for (int k = 0; k < 4; k++) tri_geo[4 * (size_t)t + k] = g[k];
+#pragma unroll
+    for (int k = 0; k < 6; k++) tri_attr[6 * (size_t)t + k] = q[k];
 }
 
 // ================================================================================================
@@ -247,7 +249,8 @@ __global__ void __launch_bounds__(256) bin_init_kernel(uint32_t* __restrict__ cl
     else if (i < (size_t)tiles_x + tiles_y) rows[i - tiles_x] = tile_span((int)(i - tiles_x), th, H);
 }
 
-// Exclusive scan of counts[0..tiles) by one CTA of 256 threads into offsets[0..tiles]; returns the largest count.
+// Exclusive scan of counts[0..tiles) by one CTA of 256 threads into offsets[0..tiles]; returns the largest count,
+// the sum in `total`.
 // 16 consecutive counts per thread and round, fetched by four independent 16-byte loads one round ahead: the rounds are
 // bound by the latency of those loads.
 constexpr int kTileScanPer = 16;
@@ -266,7 +269,8 @@ __device__ __forceinline__ void load_counts(const uint32_t* counts, int first, i
         }
     }
 }
-__device__ uint32_t tile_offsets_by_one_cta(const uint32_t* counts, int32_t* offsets, int tiles, uint32_t* s_warp /*[8]*/) {
+__device__ uint32_t tile_offsets_by_one_cta(const uint32_t* counts, int32_t* offsets, int tiles, uint32_t* s_warp /*[8]*/,
+                                            uint32_t& total) {
     const int tid = threadIdx.x, warp = tid >> 5;
     uint32_t carry = 0, biggest = 0;
     uint4 ahead[4];
@@ -311,6 +315,7 @@ __device__ uint32_t tile_offsets_by_one_cta(const uint32_t* counts, int32_t* off
         }
     }
     if (tid == 0) offsets[tiles] = (int32_t)carry;
+    total = carry;
     biggest = __reduce_max_sync(0xffffffffu, biggest);
     __syncthreads();
     if (lane_id() == 0) s_warp[warp] = biggest;
@@ -365,7 +370,7 @@ struct Plane { float A, B, C; };
 __device__ __forceinline__ Plane depth_plane(float ax, float ay, float az, float bx, float by, float bz, float cx,
                                              float cy, float cz) {
     float det = add(add(mul(ax, sub(by, cy)), mul(bx, sub(cy, ay))), mul(cx, sub(ay, by)));
-    float id = (float)__ddiv_rn(1.0, (double)det);
+    float id = (float)__drcp_rn((double)det);
     Plane p;
     p.A = mul(add(add(mul(az, sub(by, cy)), mul(bz, sub(cy, ay))), mul(cz, sub(ay, by))), id);
     p.B = mul(add(add(mul(ax, sub(bz, cz)), mul(bx, sub(cz, az))), mul(cx, sub(az, bz))), id);
@@ -377,59 +382,71 @@ __device__ __forceinline__ Plane depth_plane(float ax, float ay, float az, float
 
 __device__ __forceinline__ float plane_depth(const Plane& p, float x, float y) { return fma_(p.A, x, fma_(p.B, y, p.C)); }
 
-// One Sutherland-Hodgman pass against an axis-aligned half-plane (reference render.cu:159-189).
-template <int AXIS>
-__device__ __forceinline__ int clip_pass(const float2* in, int n_in, float2* out, float bound) {
+// One Sutherland-Hodgman pass against an axis-aligned half-plane (reference render.cu:159-189) over the `n_in` vertices
+// poly[0], poly[stride], ...; `emit` receives the vertices of the clipped polygon in order and may write them back to
+// the same places: two vertices are read ahead, and a pass over the at most six vertices of a polygon that is convex but
+// for the rounding of its corners never gets further ahead of its reads.
+template <int AXIS, class Emit>
+__device__ __forceinline__ void clip_pass(const float2* poly, int stride, int n_in, float bound, Emit&& emit) {
     auto dist = [&](const float2& p) -> float {
         if (AXIS == 0) return sub(p.x, bound);
         if (AXIS == 1) return sub(bound, p.x);
         if (AXIS == 2) return sub(p.y, bound);
         return sub(bound, p.y);
     };
-    int n_out = 0;
-    float2 p0 = in[n_in - 1];
+    float2 p0 = poly[(n_in - 1) * stride], p1 = poly[0], p2 = poly[min(1, n_in - 1) * stride];
     float d0 = dist(p0);
     bool in0 = d0 >= 0.f;
+#pragma unroll 1
     for (int i = 0; i < n_in; i++) {
-        float2 p1 = in[i];
-        float d1 = dist(p1);
-        bool in1 = d1 >= 0.f;
+        const float2 p3 = poly[min(i + 2, n_in - 1) * stride];
+        const float d1 = dist(p1);
+        const bool in1 = d1 >= 0.f;
         if (in1 != in0) {
-            float t = div(d0, sub(d0, d1));
-            out[n_out++] = make_float2(fma_(t, sub(p1.x, p0.x), p0.x), fma_(t, sub(p1.y, p0.y), p0.y));
+            const float t = div(d0, sub(d0, d1));
+            emit(make_float2(fma_(t, sub(p1.x, p0.x), p0.x), fma_(t, sub(p1.y, p0.y), p0.y)));
         }
-        if (in1) out[n_out++] = p1;
+        if (in1) emit(p1);
         p0 = p1; d0 = d1; in0 = in1;
+        p1 = p2; p2 = p3;
     }
-    return n_out;
 }
 
 struct TriXYZ { float ax, ay, bx, by, cx, cy; };
 
-__device__ float tile_key(const TriXYZ& v, const Plane& pl, float xmin, float xmax, float ymin, float ymax) {
-    // triangle entirely inside the tile: the clipper would return it unchanged
+// Triangle entirely inside the tile: the clipper would return it unchanged.
+__device__ __forceinline__ bool inside_tile(const TriXYZ& v, float xmin, float xmax, float ymin, float ymax) {
     const float lox = fminf(fminf(v.ax, v.bx), v.cx), hix = fmaxf(fmaxf(v.ax, v.bx), v.cx);
     const float loy = fminf(fminf(v.ay, v.by), v.cy), hiy = fmaxf(fmaxf(v.ay, v.by), v.cy);
-    if (sub(lox, xmin) >= 0.f && sub(xmax, hix) >= 0.f && sub(loy, ymin) >= 0.f && sub(ymax, hiy) >= 0.f) {
+    return sub(lox, xmin) >= 0.f && sub(xmax, hix) >= 0.f && sub(loy, ymin) >= 0.f && sub(ymax, hiy) >= 0.f;
+}
+
+// The polygon of a clip lives in shared memory, a column of kPolySlots float2 per thread of the CTA (no bank conflicts
+// whatever slot a lane is at).  In local memory the two arrays of a thread made 131 KB of L1 working set per SM, more
+// than L1 has beside the CTAs' shared memory (200k triangles, full HD: 55 us against 40).
+constexpr int kPolySlots = 8;
+__device__ __forceinline__ float tile_key(const TriXYZ& v, const Plane& pl, float xmin, float xmax, float ymin, float ymax,
+                                          float2* poly, int stride) {
+    if (inside_tile(v, xmin, xmax, ymin, ymax)) {
         float md0 = fminf(FLT_MAX, plane_depth(pl, v.ax, v.ay));
         md0 = fminf(md0, plane_depth(pl, v.bx, v.by));
         return fminf(md0, plane_depth(pl, v.cx, v.cy));
     }
-    float2 poly[8], buf[8];
     poly[0] = make_float2(v.ax, v.ay);
-    poly[1] = make_float2(v.bx, v.by);
-    poly[2] = make_float2(v.cx, v.cy);
-    int n = clip_pass<0>(poly, 3, buf, xmin);
-    if (n <= 0) return 1e30f;
-    n = clip_pass<1>(buf, n, poly, xmax);
-    if (n <= 0) return 1e30f;
-    n = clip_pass<2>(poly, n, buf, ymin);
-    if (n <= 0) return 1e30f;
-    n = clip_pass<3>(buf, n, poly, ymax);
-    if (n <= 0) return 1e30f;
+    poly[stride] = make_float2(v.bx, v.by);
+    poly[2 * stride] = make_float2(v.cx, v.cy);
+    int n = 3, m = 0;
+    auto keep = [&](float2 p) { poly[min(m++, kPolySlots - 1) * stride] = p; };
+    auto next = [&]() { n = min(m, kPolySlots); m = 0; return n > 0; };
+    clip_pass<0>(poly, stride, n, xmin, keep);
+    if (!next()) return 1e30f;
+    clip_pass<1>(poly, stride, n, xmax, keep);
+    if (!next()) return 1e30f;
+    clip_pass<2>(poly, stride, n, ymin, keep);
+    if (!next()) return 1e30f;
     float md = FLT_MAX;
-    for (int i = 0; i < n; i++) md = fminf(md, plane_depth(pl, poly[i].x, poly[i].y));
-    return md;
+    clip_pass<3>(poly, stride, n, ymax, [&](float2 p) { md = fminf(md, plane_depth(pl, p.x, p.y)); m++; });
+    return m <= 0 ? 1e30f : md;
 }
 
 // Stage entry point: entries with their radix keys in emission order.  One CTA takes 256 consecutive triangles.  Phase 1
@@ -460,6 +477,7 @@ __global__ void __launch_bounds__(kEmitThreads) emit_keys_kernel(const float4* _
                                                                  uint32_t capacity) {
     __shared__ EmitTri s_tri[kEmitThreads];
     __shared__ uint32_t s_off[kEmitThreads + 1];
+    __shared__ float2 s_poly[kPolySlots * kEmitThreads];
     const int tid = threadIdx.x;
     const int t0 = blockIdx.x * kEmitThreads;
     const int ntri = min(kEmitThreads, T - t0);
@@ -490,7 +508,8 @@ __global__ void __launch_bounds__(kEmitThreads) emit_keys_kernel(const float4* _
         const uint32_t local = ge - s_off[lo];
         const int tx = tr.x0 + (int)(local / (uint32_t)tr.ny), ty = tr.y0 + (int)(local % (uint32_t)tr.ny);
         const float4 cx = tile_span(tx, tw, W), cy = tile_span(ty, th, H);
-        const float depth = tile_key({tr.ax, tr.ay, tr.bx, tr.by, tr.cx, tr.cy}, {tr.A, tr.B, tr.C}, cx.z, cx.w, cy.z, cy.w);
+        const float depth = tile_key({tr.ax, tr.ay, tr.bx, tr.by, tr.cx, tr.cy}, {tr.A, tr.B, tr.C}, cx.z, cx.w, cy.z, cy.w,
+                                     s_poly + tid, kEmitThreads);
         if (ge < capacity) {                       // the host guarantees K <= capacity before the result is used
             keys[ge] = ((uint64_t)(uint32_t)(ty * tiles_x + tx) << 32) | float_to_ordered(depth);
             ids[ge] = (uint32_t)(t0 + lo);
@@ -500,22 +519,23 @@ __global__ void __launch_bounds__(kEmitThreads) emit_keys_kernel(const float4* _
 
 // ---- the forward path's binning ----------------------------------------------------------------------------------
 // One pass over the triangles makes everything: the packed records, the (triangle, tile) pairs with their depth keys and
-// the tile counts.  A CTA takes `per_cta` consecutive triangles.  Phase 1, a thread per triangle: gathers, records, tile
-// rectangle; matrix, corners and depth plane stay in shared memory.  Phase 2, a thread per pair of the rectangles: the
-// pairs that are to be listed (all, or with CULL those that can cover a pixel centre of their tile, the exact test the
-// reference leaves open, render.cu:110) go to a queue in shared memory.  Phase 3, a thread per queued pair, so that the
-// clipper runs with full warps: the pair's rank in its tile from one atomic on the tile's count (issued before the clip,
-// which hides its latency), its depth key, and one 16-byte record (key, triangle, tile, rank) to the next free slot.
+// the tile counts.  A CTA takes `per_cta` consecutive triangles, up to 32 per warp.  Phase 1, a lane per triangle: gathers,
+// records, tile rectangle; matrix, corners and depth plane stay in shared memory.  Phase 2, a thread per pair of the
+// CTA's rectangles: with CULL, pairs that cannot cover a pixel centre of their tile leave a hole (the exact test the
+// reference leaves open, render.cu:110).  The others take their rank in the tile from one atomic on the tile's count
+// (issued before the depth key, which hides its latency) and leave one 16-byte record (key, triangle, tile, rank).  Pairs
+// that need the polygon clipper are put off to the end of the CTA when they are few in a warp, and run there with full
+// warps.
 // The CTA that finishes last turns the counts into tile offsets; the scatter kernel then moves every entry to
-// offset + rank.  Against counting and writing in two kernels, which gathered, tested and searched twice, B200: 1280
-// triangles 256x256 27 -> 15 us, 200k triangles full HD 65 -> 59, 1.3M triangles 281 -> 235, 3000 large triangles
-// 294 -> 28.
+// offset + rank.  Against counting and writing in two kernels, which gathered, tested and searched twice, B200: 1.3M triangles of a pixel
+// each, full HD: 281 -> 188 us; 200k triangles, full HD: 65 -> 46; 2M triangles, 4K: 791 -> 510; 3000 triangles of 200
+// tiles each: 294 -> 28.  Bound by instruction issue and shared-memory wavefronts (61 %) in turns with the barriers.
 struct BinArgs {
     uint32_t* tile_counts;   // [tiles], zero on entry
     int32_t* offsets;        // [tiles + 1], written when scan_here
-    uint32_t* counters;      // [2], zero on entry: finished CTAs, slots handed out (K in the end)
-    uint32_t* info;          // [2] K, and when scan_here the longest list (kOrderWrittenBit: a launch order is wanted)
-    uint32_t* info_host;     // the same two words in mapped host memory, or null
+    uint32_t* counters;      // [2], zero on entry: finished CTAs, slots handed out
+    uint32_t* info;          // [3] K, when scan_here the longest list (kOrderWrittenBit: a launch order is wanted), slots
+    uint32_t* info_host;     // words 0, 1 and 3 of mapped host memory receive them too, or null
     uint4* pairs;            // [capacity]
     uint32_t capacity;
     int tiles, tiles_x, tiles_y;
@@ -524,109 +544,175 @@ struct BinArgs {
     TileTables tables;
 };
 
-constexpr int kBinQueue = 1024;
-constexpr int kBinWords = 18;        // matrix 9, corners 6, depth plane 3
+constexpr uint32_t kHole = 0xffffffffu;      // tile word of a pair that is not listed
+constexpr int kBinWarps = 8;
+constexpr int kBinQueue = 512;       // clip queue of a CTA
+// Shared memory of a warp, in words: first the staging area of its records (pitch 5 quads for the 4 of a geometry
+// record, 7 for the 6 of half the warp's attribute records: 16-byte accesses of consecutive lanes then fall on different
+// banks), then, component-major, what the pairs need of its triangles: matrix 9, corners 6, depth plane 3, tile
+// rectangle (x0, y0, rows), first pair.
+constexpr int kBinWarpWords = 22 * 32 + 4;
+constexpr size_t kBinSmem = sizeof(float) * kBinWarps * kBinWarpWords + sizeof(float2) * kPolySlots * 32 * kBinWarps;
+constexpr int kTriMatrix = 0, kTriCorners = 9, kTriPlane = 15, kTriX0 = 18, kTriY0 = 19, kTriRows = 20, kTriFirst = 21;
+static_assert(32 * 20 <= kBinWarpWords && 16 * 28 <= kBinWarpWords, "the triangles' data replace the staging area");
+
+// Key and record of one listed pair: triangle `lt` of the CTA with its data at `tri` (lane stride 32), tile (tx, ty).
+__device__ __forceinline__ void write_pair(const BinArgs& bin, const float* tri, int t, uint32_t tx, uint32_t ty, uint32_t pos,
+                                           const float4& cx, const float4& cy, float2* poly) {
+    const uint32_t tile = ty * (uint32_t)bin.tiles_x + tx;
+    const uint32_t rank = atomicAdd(bin.tile_counts + tile, 1u);     // travels while the key is computed
+    const float* v = tri + 32 * kTriCorners;
+    const float* p = tri + 32 * kTriPlane;
+    const float depth = tile_key({v[0], v[32], v[64], v[96], v[128], v[160]}, {p[0], p[32], p[64]}, cx.z, cx.w, cy.z, cy.w,
+                                 poly, 32 * kBinWarps);
+    if (pos < bin.capacity)              // the host checks K before anything that reads the entries is used
+        bin.pairs[pos] = make_uint4((uint32_t)t, float_to_ordered(depth), tile, rank);
+}
 
 template <bool CULL>
-__global__ void __launch_bounds__(256, 4) bin_kernel(const float4* __restrict__ vertices, const int* __restrict__ indices,
-                                                     const float* __restrict__ colors, const float* __restrict__ opacities,
-                                                     int T, int per_cta, int W, int H, int tw, int th,
-                                                     float4* __restrict__ tri_geo, float4* __restrict__ tri_attr,
-                                                     BinArgs bin, int packed) {
-    __shared__ float s_tri[kBinWords][256];
-    __shared__ int s_x0[256], s_y0[256], s_ny[256];
-    __shared__ uint32_t s_loc[257];
-    __shared__ uint32_t s_qx[kBinQueue], s_qy[kBinQueue];     // tile column | tile row << 8 | triangle of the CTA
-    __shared__ uint32_t s_warp[8];
+__global__ void __launch_bounds__(32 * kBinWarps, 4) bin_kernel(const float4* __restrict__ vertices,
+                                                                const int* __restrict__ indices,
+                                                                const float* __restrict__ colors,
+                                                                const float* __restrict__ opacities, int T, int per_cta,
+                                                                int W, int H, int tw, int th, double inv_tw, double inv_th,
+                                                                float4* __restrict__ tri_geo, float4* __restrict__ tri_attr,
+                                                                BinArgs bin, int packed) {
+    extern __shared__ __align__(16) char s_dynamic[];
+    float (*s_tri)[kBinWarpWords] = reinterpret_cast<float (*)[kBinWarpWords]>(s_dynamic);
+    float2* s_poly = reinterpret_cast<float2*>(s_dynamic + sizeof(float) * kBinWarps * kBinWarpWords);
+    __shared__ uint32_t s_qx[kBinQueue], s_qy[kBinQueue], s_qe[kBinQueue];   // tile column, tile row << 8 | triangle, pair
+    __shared__ uint32_t s_first[kBinWarps + 1];       // first pair of every warp's triangles
     __shared__ uint32_t s_queued, s_base;
+    __shared__ uint32_t s_warp[8];
     __shared__ bool s_last;
-    const int tid = threadIdx.x, warp = tid >> 5;
-    const int t0 = blockIdx.x * per_cta, ntri = min(per_cta, T - t0);
-    uint32_t count = 0;
-    if (tid < ntri) {
-        Rect r;
-        TriSetup ts;
-        count = preprocess_triangle(t0 + tid, vertices, indices, colors, opacities, W, H, tw, th, bin.tiles_x, bin.tiles_y,
-                                    nullptr, tri_geo, tri_attr, r, &ts, packed != 0);
-        if (count) {
-            const Plane pl = depth_plane(ts.x[0], ts.y[0], ts.z[0], ts.x[1], ts.y[1], ts.z[1], ts.x[2], ts.y[2], ts.z[2]);
-#pragma unroll
-            for (int k = 0; k < 9; k++) s_tri[k][tid] = ts.m[k];
-#pragma unroll
-            for (int k = 0; k < 3; k++) { s_tri[9 + 2 * k][tid] = ts.x[k]; s_tri[10 + 2 * k][tid] = ts.y[k]; }
-            s_tri[15][tid] = pl.A; s_tri[16][tid] = pl.B; s_tri[17][tid] = pl.C;
-            s_x0[tid] = r.x0; s_y0[tid] = r.y0; s_ny[tid] = r.y1 - r.y0 + 1;
-        }
-    }
-    uint32_t incl = count;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        uint32_t y = __shfl_up_sync(0xffffffffu, incl, d);
-        if (lane_id() >= (unsigned)d) incl += y;
-    }
-    if (lane_id() == 31) s_warp[warp] = incl;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const unsigned below = (1u << lane) - 1u;
+    const int per_warp = (per_cta + kBinWarps - 1) / kBinWarps;
+    const int t_cta = blockIdx.x * per_cta, t0 = t_cta + warp * per_warp;
+    const int ntri = min(min(per_warp, per_cta - warp * per_warp), T - t0);
     if (tid == 0) s_queued = 0;
-    __syncthreads();
-    uint32_t warp_off = 0, total = 0;
+    float* mine = s_tri[warp];
+    float4* stage = reinterpret_cast<float4*>(mine);
+    uint32_t total = 0;
+    if (ntri > 0) {
+        uint32_t count = 0;
+        TriInput in = {};
+        if (lane < ntri) in = load_triangle(t0 + lane, vertices, indices, colors, opacities, packed != 0);
+        // the records leave through shared memory, so that the warp's stores are whole consecutive lines
+        float4 q[6];
+        make_attr(in, q);
 #pragma unroll
-    for (int w = 0; w < 8; w++) {
-        const uint32_t x = s_warp[w];
-        if (w < warp) warp_off += x;
-        total += x;
-    }
-    s_loc[tid] = warp_off + incl - count;
-    if (tid == 0) s_loc[256] = total;
-    __syncthreads();
-
-    for (uint32_t base = 0; base < total; base += 256) {
-        const uint32_t e = base + tid;
-        bool keep = false;
-        int lo = 0, tx = 0, ty = 0;
-        if (e < total) {
-            lo = find_segment(s_loc, ntri, e);
-            const uint32_t local = e - s_loc[lo], ny = (uint32_t)s_ny[lo];
-            tx = s_x0[lo] + (int)(local / ny);
-            ty = s_y0[lo] + (int)(local % ny);
-            keep = true;
-            if (CULL) {
-                const float4 cx = __ldg(bin.tables.cols + tx), cy = __ldg(bin.tables.rows + ty);
-                float m[9];
+        for (int half = 0; half < 2; half++) {
+            const int n = min(16, ntri - 16 * half);
+            if ((lane >> 4) == half) {
 #pragma unroll
-                for (int k = 0; k < 9; k++) m[k] = s_tri[k][lo];
-                keep = rect_may_cover(m, {cx.x, cx.y, cy.x, cy.y});
+                for (int k = 0; k < 6; k++) stage[7 * (lane & 15) + k] = q[k];
+            }
+            __syncwarp();
+            for (int i = lane; i < 6 * n; i += 32) tri_attr[6 * ((size_t)t0 + 16 * half) + i] = stage[7 * (i / 6) + i % 6];
+            __syncwarp();
+        }
+        float4 g[4];
+        if (lane < ntri) {
+            make_geo(in, g);
+#pragma unroll
+            for (int k = 0; k < 4; k++) stage[5 * lane + k] = g[k];
+        }
+        __syncwarp();
+        for (int i = lane; i < 4 * ntri; i += 32) tri_geo[4 * (size_t)t0 + i] = stage[5 * (i >> 2) + (i & 3)];
+        __syncwarp();
+        if (lane < ntri) {
+            Rect r;
+            float* d = mine + lane;
+            if (tile_rect(in.a.x, in.a.y, in.b.x, in.b.y, in.c.x, in.c.y, W, H, tw, th, bin.tiles_x, bin.tiles_y, r, inv_tw, inv_th)) {
+                count = (uint32_t)(r.x1 - r.x0 + 1) * (uint32_t)(r.y1 - r.y0 + 1);
+                const Plane pl = depth_plane(in.a.x, in.a.y, in.a.z, in.b.x, in.b.y, in.b.z, in.c.x, in.c.y, in.c.z);
+                const float m[9] = {g[0].x, g[0].y, g[0].z, g[0].w, g[1].x, g[1].y, g[1].z, g[1].w, g[2].x};
+                const float rest[9] = {in.a.x, in.a.y, in.b.x, in.b.y, in.c.x, in.c.y, pl.A, pl.B, pl.C};
+#pragma unroll
+                for (int k = 0; k < 9; k++) { d[32 * (kTriMatrix + k)] = m[k]; d[32 * (kTriCorners + k)] = rest[k]; }
+                d[32 * kTriX0] = __int_as_float(r.x0);
+                d[32 * kTriY0] = __int_as_float(r.y0);
+                d[32 * kTriRows] = __int_as_float(r.y1 - r.y0 + 1);
             }
         }
-        const unsigned kept = __ballot_sync(0xffffffffu, keep);
-        uint32_t slot = 0;
-        if (lane_id() == 0 && kept) slot = atomicAdd(&s_queued, (uint32_t)__popc(kept));
-        slot = __shfl_sync(0xffffffffu, slot, 0) + __popc(kept & ((1u << lane_id()) - 1u));
-        if (keep) {
-            s_qx[slot] = (uint32_t)tx;
-            s_qy[slot] = ((uint32_t)ty << 8) | (uint32_t)lo;
+        uint32_t incl = count;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= d) incl += y;
         }
-        __syncthreads();
-        const uint32_t queued = s_queued;
-        if (queued == 0 || (queued + 256 <= kBinQueue && base + 256 < total)) {
-            __syncthreads();              // everyone has read s_queued before the next round adds to it
-            continue;
+        total = __shfl_sync(0xffffffffu, incl, 31);
+        mine[32 * kTriFirst + lane] = __uint_as_float(incl - count);
+    }
+    if (lane == 0) s_warp[warp] = total;
+    __syncthreads();
+    // Every pair of the rectangles has its slot; those that are not listed leave a hole there.
+    if (tid == 0) {
+        uint32_t sum = 0;
+#pragma unroll
+        for (int w = 0; w < kBinWarps; w++) { s_first[w] = sum; sum += s_warp[w]; }
+        s_first[kBinWarps] = sum;
+        s_base = sum ? atomicAdd(bin.counters + 1, sum) : 0u;
+    }
+    __syncthreads();
+    // The CTA's pairs in chunks of 32, whichever warp prepared the triangle
+    const uint32_t all = s_first[kBinWarps], slot0 = s_base;
+    for (uint32_t base = 32 * warp; base < all; base += 32 * kBinWarps) {
+        const uint32_t e = base + lane;
+        bool keep = false, inside = false;
+        int ct = 0;                                  // triangle: warp << 5 | lane that prepared it
+        uint32_t tx = 0, ty = 0;
+        float4 cx, cy;
+        if (e < all) {
+            const int w = find_segment(s_first, kBinWarps, e);
+            const uint32_t ew = e - s_first[w];
+            const uint32_t* first_pair = reinterpret_cast<const uint32_t*>(s_tri[w] + 32 * kTriFirst);
+            const int lt = find_segment(first_pair, 32, ew);
+            ct = (w << 5) | lt;
+            const float* d = s_tri[w] + lt;
+            const uint32_t local = ew - first_pair[lt], rows = __float_as_uint(d[32 * kTriRows]);
+            const uint32_t col = rows == 1 ? local : local / rows;
+            tx = __float_as_uint(d[32 * kTriX0]) + col;
+            ty = __float_as_uint(d[32 * kTriY0]) + (local - col * rows);
+            cx = __ldg(bin.tables.cols + tx);
+            cy = __ldg(bin.tables.rows + ty);
+            keep = true;
+            if (CULL) {
+                float m[9];
+#pragma unroll
+                for (int k = 0; k < 9; k++) m[k] = d[32 * (kTriMatrix + k)];
+                keep = rect_may_cover(m, {cx.x, cx.y, cy.x, cy.y});
+                if (!keep && slot0 + e < bin.capacity) bin.pairs[slot0 + e] = make_uint4(0, 0, kHole, 0);
+            }
+            const float* v = d + 32 * kTriCorners;
+            inside = inside_tile({v[0], v[32], v[64], v[96], v[128], v[160]}, cx.z, cx.w, cy.z, cy.w);
         }
-        if (tid == 0) s_base = atomicAdd(bin.counters + 1, queued);
-        __syncthreads();
-        for (uint32_t q = tid; q < queued; q += 256) {
-            const int qx = (int)s_qx[q], qy = (int)(s_qy[q] >> 8), lt = (int)(s_qy[q] & 255u);
-            const uint32_t tile = (uint32_t)(qy * bin.tiles_x + qx);
-            const uint32_t rank = atomicAdd(bin.tile_counts + tile, 1u);
-            const float4 cx = __ldg(bin.tables.cols + qx), cy = __ldg(bin.tables.rows + qy);
-            const TriXYZ v = {s_tri[9][lt], s_tri[10][lt], s_tri[11][lt], s_tri[12][lt], s_tri[13][lt], s_tri[14][lt]};
-            const Plane pl = {s_tri[15][lt], s_tri[16][lt], s_tri[17][lt]};
-            const float depth = tile_key(v, pl, cx.z, cx.w, cy.z, cy.w);
-            const uint32_t pos = s_base + q;
-            if (pos < bin.capacity)          // the host checks K before anything that reads the entries is used
-                bin.pairs[pos] = make_uint4((uint32_t)(t0 + lt), float_to_ordered(depth), tile, rank);
+        // Pairs that need the clipper (a triangle across tile borders) wait for the CTA's queue and run there with full
+        // warps, unless most lanes of this warp need it anyway or the queue is full.
+        const unsigned clip = __ballot_sync(0xffffffffu, keep && !inside);
+        bool now = keep;
+        if (clip && __popc(clip) < 20) {
+            uint32_t at = 0;
+            if (lane == 0) at = atomicAdd(&s_queued, (uint32_t)__popc(clip));
+            at = __shfl_sync(0xffffffffu, at, 0) + __popc(clip & below);
+            if (keep && !inside && at < kBinQueue) {
+                s_qx[at] = tx;
+                s_qy[at] = (ty << 8) | (uint32_t)ct;
+                s_qe[at] = e;
+                now = false;
+            }
         }
-        __syncthreads();
-        if (tid == 0) s_queued = 0;
-        __syncthreads();
+        if (now) write_pair(bin, s_tri[ct >> 5] + (ct & 31), t_cta + (ct >> 5) * per_warp + (ct & 31), tx, ty, slot0 + e, cx, cy,
+                            s_poly + tid);
+    }
+    __syncthreads();
+    const uint32_t queued = min(s_queued, (uint32_t)kBinQueue);
+    for (uint32_t q = tid; q < queued; q += 32 * kBinWarps) {
+        const uint32_t tx = s_qx[q], ty = s_qy[q] >> 8;
+        const int ct = (int)(s_qy[q] & 255u);
+        write_pair(bin, s_tri[ct >> 5] + (ct & 31), t_cta + (ct >> 5) * per_warp + (ct & 31), tx, ty, slot0 + s_qe[q],
+                   __ldg(bin.tables.cols + tx), __ldg(bin.tables.rows + ty), s_poly + tid);
     }
     __syncthreads();                          // the CTA's counts are issued; one cumulative fence publishes them
     if (tid == 0) {
@@ -636,10 +722,10 @@ __global__ void __launch_bounds__(256, 4) bin_kernel(const float4* __restrict__ 
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    const uint32_t K = __ldcg(bin.counters + 1);
-    uint32_t longest = UINT32_MAX;            // not known
+    const uint32_t slots = __ldcg(bin.counters + 1);
+    uint32_t K = slots, longest = UINT32_MAX;            // longest: not known
     if (bin.scan_here) {
-        longest = tile_offsets_by_one_cta(bin.tile_counts, bin.offsets, bin.tiles, s_warp);
+        longest = tile_offsets_by_one_cta(bin.tile_counts, bin.offsets, bin.tiles, s_warp, K);
         // the launch order costs two passes over the offsets: only for images of at most 16384 tiles whose lists are
         // long on average and uneven (the longest one at least 256 entries)
         if (bin.want_order && bin.tiles <= kOrderMaxTiles && K >= kOrderMinMean * (uint32_t)bin.tiles && longest >= kOrderMinLongest)
@@ -648,10 +734,13 @@ __global__ void __launch_bounds__(256, 4) bin_kernel(const float4* __restrict__ 
     if (tid == 0) {
         bin.info[0] = K;
         bin.info[1] = longest;
+        bin.info[2] = slots;
         if (bin.info_host) {                  // K last: the host watches that word
-            *(volatile uint32_t*)(bin.info_host + 1) = longest;
+            volatile uint32_t* h = bin.info_host;
+            h[1] = longest;
+            h[3] = slots;
             __threadfence_system();
-            *(volatile uint32_t*)bin.info_host = K;
+            h[0] = K;
         }
     }
 }
@@ -663,16 +752,28 @@ __global__ void __launch_bounds__(256) scatter_entries_kernel(const uint4* __res
                                                               uint64_t* __restrict__ entries, uint32_t* __restrict__ order,
                                                               int tiles) {
     __shared__ uint32_t s_hist[33];
-    const uint32_t K = info[0];
-    if (K > capacity) return;
+    const uint32_t n = info[2];               // slots, holes included
+    if (n > capacity) return;
     if (blockIdx.x == gridDim.x - 1) {
         if (order && info[1] != UINT32_MAX && (info[1] & kOrderWrittenBit)) tile_order_by_one_cta(offsets, tiles, order, s_hist);
         return;
     }
-    const uint32_t stride = (gridDim.x - 1) * 256;
-    for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < K; i += stride) {
-        const uint4 p = pairs[i];
-        entries[(uint32_t)__ldg(offsets + p.z) + p.w] = ((uint64_t)p.y << 32) | p.x;
+    // four entries per thread in flight: each is a chain of two loads and a scattered store
+    const uint32_t stride = (gridDim.x - 1) * 1024;
+    for (uint32_t i = blockIdx.x * 1024 + threadIdx.x; i < n; i += stride) {
+        uint4 p[4];
+        uint32_t off[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            p[k].z = kHole;
+            if (i + 256 * k < n) p[k] = __ldcs(pairs + i + 256 * k);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (p[k].z != kHole) off[k] = (uint32_t)__ldg(offsets + p[k].z);
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (p[k].z != kHole) entries[off[k] + p[k].w] = ((uint64_t)p[k].y << 32) | p[k].x;
     }
 }
 
@@ -724,6 +825,20 @@ static int check_dims_internal(int T, int W, int H, int tw, int th) {
     return TG_OK;
 }
 
+// Opt-in shared memory of a kernel, set once per device (`slot`: which kernel; setting it twice is harmless).
+static int allow_smem(const void* kernel, size_t bytes, int slot) {
+    constexpr int kMaxDevices = 64;
+    static std::atomic<bool> set[2][kMaxDevices];
+    int dev = 0;
+    TG_CUDA(cudaGetDevice(&dev));
+    TG_REQUIRE(dev >= 0 && dev < kMaxDevices, "device index outside the supported range");
+    if (!set[slot][dev].load(std::memory_order_acquire)) {
+        TG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+        set[slot][dev].store(true, std::memory_order_release);
+    }
+    return TG_OK;
+}
+
 // Per-triangle records, (triangle, tile) pairs and tile offsets: bin_init_kernel, bin_kernel and scatter_entries_kernel
 // (declared in tg_common.cuh with what each argument is).
 int bin_triangles(const float* vertices, const int32_t* indices, const float* colors, const float* opacities, int T, int W,
@@ -746,7 +861,7 @@ int bin_triangles(const float* vertices, const int32_t* indices, const float* co
                                                                           tiles_y, W, H, tw, th);
     TG_LAUNCH_CHECK("bin_init_kernel");
     if (T == 0) {
-        TG_CUDA(cudaMemsetAsync(b.info, 0, sizeof(uint32_t) * 2, stream));
+        TG_CUDA(cudaMemsetAsync(b.info, 0, sizeof(uint32_t) * 3, stream));
         TG_CUDA(cudaMemsetAsync(offsets, 0, sizeof(int32_t) * ((size_t)tiles + 1), stream));
         return TG_OK;
     }
@@ -755,11 +870,14 @@ int bin_triangles(const float* vertices, const int32_t* indices, const float* co
     // Triangles per CTA: 256 where that fills the GPU; fewer below, so that a mesh of few triangles that cover many tiles
     // each still spreads over all SMs (four CTAs on each).
     constexpr int kWave = 148 * 4;
-    const int per_cta = T >= 256 * kWave ? 256 : (T + kWave - 1) / kWave;
+    const int per_cta = T >= 32 * tg::kBinWarps * kWave ? 32 * tg::kBinWarps : (T + kWave - 1) / kWave;
     const int grid = (T + per_cta - 1) / per_cta;
+    auto inverse = [](int n) { return (n & (n - 1)) == 0 ? 1.0 / n : 0.0; };
     auto kernel = cull ? tg::bin_kernel<true> : tg::bin_kernel<false>;
-    kernel<<<grid, 256, 0, stream>>>((const float4*)vertices, indices, colors, opacities, T, per_cta, W, H, tw, th,
-                                     (float4*)tri_geo, (float4*)tri_attr, bin, packed ? 1 : 0);
+    if (int st = allow_smem((const void*)kernel, tg::kBinSmem, cull ? 1 : 0)) return st;
+    kernel<<<grid, 32 * tg::kBinWarps, tg::kBinSmem, stream>>>((const float4*)vertices, indices, colors, opacities, T, per_cta, W, H,
+                                                    tw, th, inverse(tw), inverse(th), (float4*)tri_geo, (float4*)tri_attr,
+                                                    bin, packed ? 1 : 0);
     TG_LAUNCH_CHECK("bin_kernel");
     if (!by_last_cta) {
         const int parts = (tiles + tg::kScanTile - 1) / tg::kScanTile;
@@ -773,9 +891,9 @@ int bin_triangles(const float* vertices, const int32_t* indices, const float* co
 
 int scatter_entries(const BinBuffers& b, uint32_t list_capacity, const int32_t* offsets, int tiles, int T, cudaStream_t stream) {
     if (T == 0 || list_capacity == 0) return TG_OK;
-    // K is not known on the host yet: as many CTAs as its upper bound fills, at most four per SM, and one for the order
+    // K is not known on the host yet: as many CTAs as its upper bound fills, at most eight per SM, and one for the order
     const uint32_t want = (list_capacity + 1023) / 1024;
-    const int grid = (int)(want < 148 * 4 ? want : 148 * 4) + 1;
+    const int grid = (int)(want < 148 * 8 ? want : 148 * 8) + 1;
     tg::scatter_entries_kernel<<<grid, 256, 0, stream>>>(b.pairs, b.info, list_capacity, offsets, b.entries, b.tile_order, tiles);
     TG_LAUNCH_CHECK("scatter_entries_kernel");
     return TG_OK;

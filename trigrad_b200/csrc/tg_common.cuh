@@ -36,9 +36,11 @@ struct Rect { int x0, y0, x1, y1; };
 
 // Tile rectangle of a triangle's bounding box; returns false for degenerate / non-finite input.
 // Same rule as reference render.cu:51-76: float add, then double multiply/divide, cast, clamp,
-// truncate.
+// truncate.  inv_tw / inv_th: exact reciprocals of power-of-two tile sizes, or 0 (the product is then the quotient, bit for
+// bit, and 20 instructions shorter).
 __device__ __forceinline__ bool tile_rect(float ax, float ay, float bx, float by, float cx, float cy, int W, int H,
-                                          int tw, int th, int tiles_x, int tiles_y, Rect& r) {
+                                          int tw, int th, int tiles_x, int tiles_y, Rect& r, double inv_tw = 0.0,
+                                          double inv_th = 0.0) {
     float ux = sub(bx, ax), uy = sub(by, ay), vx = sub(cx, ax), vy = sub(cy, ay);
     float v = sub(mul(ux, vy), mul(uy, vx));
     if (fabsf(v) < kEffZero || isnan(v) || isinf(v)) {
@@ -47,17 +49,18 @@ __device__ __forceinline__ bool tile_rect(float ax, float ay, float bx, float by
     }
     float minx = fminf(fminf(ax, bx), cx), miny = fminf(fminf(ay, by), cy);
     float maxx = fmaxf(fmaxf(ax, bx), cx), maxy = fmaxf(fmaxf(ay, by), cy);
-    auto to_tile = [](float m, int extent, int tile, int ntiles) -> int {
-        double d = __ddiv_rn(__dmul_rn(__dmul_rn((double)add(m, 1.0f), 0.5), (double)extent), (double)tile);
+    auto to_tile = [](float m, int extent, int tile, int ntiles, double inv) -> int {
+        double d = __dmul_rn(__dmul_rn((double)add(m, 1.0f), 0.5), (double)extent);
+        d = inv != 0.0 ? __dmul_rn(d, inv) : __ddiv_rn(d, (double)tile);
         float f = (float)d;
         float hi = (float)(ntiles - 1);
         f = (f < 0.0f) ? 0.0f : ((hi < f) ? hi : f);
         return (int)f;
     };
-    r.x0 = to_tile(minx, W, tw, tiles_x);
-    r.y0 = to_tile(miny, H, th, tiles_y);
-    r.x1 = to_tile(maxx, W, tw, tiles_x);
-    r.y1 = to_tile(maxy, H, th, tiles_y);
+    r.x0 = to_tile(minx, W, tw, tiles_x, inv_tw);
+    r.y0 = to_tile(miny, H, th, tiles_y, inv_th);
+    r.x1 = to_tile(maxx, W, tw, tiles_x, inv_tw);
+    r.y1 = to_tile(maxy, H, th, tiles_y, inv_th);
     return true;
 }
 

@@ -98,12 +98,12 @@ struct BinBuffers {
     uint32_t* tile_counts;       // [tiles], 16-byte aligned
     void* tile_scan_scratch;     // device-wide scan of the tile counts, only beyond kTileScanByLastCta tiles; zeroed too
     float4* tables;              // [tiles_x + tiles_y]
-    uint32_t* info;              // [2] K, longest list (UINT32_MAX: not known)
+    uint32_t* info;              // [3] K, longest list (UINT32_MAX: not known), slots of `pairs` in use
     uint4* pairs;                // [list capacity]
     uint64_t* entries;           // [list capacity]
     uint32_t* tile_order;        // [tiles] or null
 };
-// `info_host`: mapped host memory that receives the two info words (K last), or null.
+// `info_host`: mapped host memory whose words 0, 1 and 3 receive the three info words (K last), or null.
 int bin_triangles(const float* vertices, const int32_t* indices, const float* colors, const float* opacities, int T, int W,
                   int H, int tw, int th, float* tri_geo, float* tri_attr, const BinBuffers& b, int32_t* offsets,
                   uint32_t list_capacity, uint32_t* info_host, bool cull, bool packed, cudaStream_t stream);

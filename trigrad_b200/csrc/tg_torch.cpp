@@ -286,12 +286,12 @@ ForwardOut forward(const Tensor& vertices_, const Tensor& indices_, const Tensor
                                     s.offsets, ws, have, (uint32_t*)info, ms, flags, w.stream);
         s.K = (uint32_t)info[0];
         if (status == TG_ERR_CAPACITY) {
-            cap = s.K + s.K / 4 + 1024;
+            cap = s.K + s.K / 4 + 1024;              // what the call says it needs
             continue;
         }
         check(step ? "render_step_l2" : "render_forward", status);
         state->finish_call(slot);
-        state->k_estimate = s.K;
+        state->k_estimate = std::max<int64_t>(s.K, (uint32_t)info[3]);
         return out;
     }
 }
