@@ -527,6 +527,65 @@ __device__ __forceinline__ void emit_contrib(const Contrib& c, float4* __restric
     }
 }
 
+// Sum of the contributions of the lanes with `in` (one triangle), added by 24 lanes with one instruction: a reduction by
+// halves in which a lane keeps half of its 24 values and hands the other half to its partner (12 + 6 + 3 + 2 + 1
+// exchanges instead of 5 x 21) and ends up with the total of one value of the triangle's three 32-byte slots.  All lanes
+// of the warp must call; `leader` is one of those with `in`.
+__device__ __forceinline__ void reduce_group(const Contrib& c, bool in, int leader, float4* __restrict__ gpack) {
+    const int lane = lane_id();
+    float v[24];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+#pragma unroll
+        for (int q = 0; q < 7; q++) v[8 * k + q] = in ? c.v[k][q] : 0.f;
+        v[8 * k + 7] = 0.f;
+    }
+    const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4, b1 = lane & 2, b0 = lane & 1;
+#pragma unroll
+    for (int i = 0; i < 12; i++) v[i] = (b4 ? v[i + 12] : v[i]) + __shfl_xor_sync(0xffffffffu, b4 ? v[i] : v[i + 12], 16);
+#pragma unroll
+    for (int i = 0; i < 6; i++) v[i] = (b3 ? v[i + 6] : v[i]) + __shfl_xor_sync(0xffffffffu, b3 ? v[i] : v[i + 6], 8);
+#pragma unroll
+    for (int i = 0; i < 3; i++) v[i] = (b2 ? v[i + 3] : v[i]) + __shfl_xor_sync(0xffffffffu, b2 ? v[i] : v[i + 3], 4);
+    v[3] = 0.f;
+#pragma unroll
+    for (int i = 0; i < 2; i++) v[i] = (b1 ? v[i + 2] : v[i]) + __shfl_xor_sync(0xffffffffu, b1 ? v[i] : v[i + 2], 2);
+    v[0] = (b0 ? v[1] : v[0]) + __shfl_xor_sync(0xffffffffu, b0 ? v[0] : v[1], 1);
+    const int at = (lane >> 4) * 12 + ((lane >> 3) & 1) * 6 + ((lane >> 2) & 1) * 3 + (lane & 3);   // this lane's value
+    const int v0 = __shfl_sync(0xffffffffu, c.vid[0], leader), v1 = __shfl_sync(0xffffffffu, c.vid[1], leader),
+              v2 = __shfl_sync(0xffffffffu, c.vid[2], leader);
+    const int vid = at < 8 ? v0 : at < 16 ? v1 : v2;
+    if ((lane & 3) != 3 && (at & 7) != 7) atomicAdd(reinterpret_cast<float*>(gpack + 2 * (size_t)vid) + (at & 7), v[0]);
+}
+
+// From this many lanes on the reduction is cheaper than the lanes' own six vector reductions to the same three slots.
+constexpr int kGroupMin = 6;
+
+// Contributions of a warp whose lanes with `has` hold one and the same triangle.  All lanes must call.
+__device__ __forceinline__ void emit_uniform(const Contrib& c, bool has, float4* __restrict__ gpack) {
+    const unsigned group = __ballot_sync(0xffffffffu, has);
+    if (__popc(group) >= kGroupMin) reduce_group(c, has, __ffs(group) - 1, gpack);
+    else if (has) emit_contrib(c, gpack);
+    __syncwarp();
+}
+
+// The same for lanes with triangles of their own (`id`): pixels next to each other under large triangles mostly blend the
+// same triangle at the same place of their sequences.  All lanes must call.
+__device__ __forceinline__ void emit_warp(const Contrib& c, bool has, int id, float4* __restrict__ gpack) {
+    const unsigned peers = __match_any_sync(0xffffffffu, has ? id : -1 - (int)lane_id());
+    const bool big = has && __popc(peers) >= kGroupMin;
+    unsigned todo = __ballot_sync(0xffffffffu, big);
+#pragma unroll 1
+    for (int it = 0; it < 32 / kGroupMin && todo != 0; ++it) {
+        const int leader = __ffs(todo) - 1;
+        const unsigned group = __shfl_sync(0xffffffffu, peers, leader);
+        todo &= ~group;
+        reduce_group(c, (group >> lane_id()) & 1u, leader, gpack);
+    }
+    if (has && !big) emit_contrib(c, gpack);
+    __syncwarp();
+}
+
 __device__ __forceinline__ void backward_one(const float* w, const AttrRec& a, const Bary& b, float px, float py,
                                              const PixelGrad& pg, BackState& st, Contrib& out) {
     const float bw0 = b.x * w[0], bw1 = b.y * w[1], bw2 = b.z * w[2];
@@ -1114,18 +1173,25 @@ __global__ void __launch_bounds__(MAXT) blend_backward_kernel(BlendParams P, Bac
             if (!__syncthreads_or(go)) break;
             const int bs = min(kBatchLayers, remaining);
             const int found = select_sweep(P, c, go, bs, lastDepth, lastJ, dl, jl, s_geo, s_id);
-            if (go) {
-                const int n = min(found, remaining);
-                for (int i = n - 1; i >= 0; --i) {          // reference render.cu:684-688
-                    const int id = P.ids[jl[i]];
+            const int n = go ? min(found, remaining) : 0;
+            const int rounds = __reduce_max_sync(0xffffffffu, n);
+            // back to front inside the batch (reference render.cu:684-688); the first of the rounds starts at every lane's
+            // last fragment
+            for (int s = 0; s < rounds; ++s) {
+                const int i = n - 1 - s;
+                int id = -1;
+                Contrib ct = {};
+                if (i >= 0) {
+                    id = P.ids[jl[i]];
                     float m[9], w[3];
                     load_geo(P.geo, id, m, w);
                     const Bary b = apply_bary(m, c.px, c.py);
                     const AttrRec a = load_attr<true>(P.attr, id);
-                    Contrib ct;
                     backward_one(w, a, b, c.px, c.py, pg, st, ct);
-                    emit_contrib(ct, gpack);
                 }
+                emit_warp(ct, i >= 0, id, gpack);
+            }
+            if (go) {
                 if (n > 0) {
                     lastDepth = dl[n - 1];
                     lastJ = jl[n - 1];
@@ -1153,14 +1219,15 @@ __global__ void __launch_bounds__(MAXT) blend_backward_kernel(BlendParams P, Bac
             while (mask) {
                 const int r = __ffsll((long long)mask) - 1;
                 mask &= mask - 1;
-                if (first + r >= limit) continue;
                 const float* g = reinterpret_cast<const float*>(s_geo + kStagedQuads * r);
                 const Bary b = apply_bary(g, c.px, c.py);
-                if (!covered(b)) continue;
-                const AttrRec a = load_attr<true>(P.attr, s_id[r]);
-                Contrib ct;
-                backward_one(g + 12, a, b, c.px, c.py, pg, st, ct);
-                emit_contrib(ct, gpack);
+                const bool has = first + r < limit && covered(b);
+                Contrib ct = {};
+                if (has) {
+                    const AttrRec a = load_attr<true>(P.attr, s_id[r]);
+                    backward_one(g + 12, a, b, c.px, c.py, pg, st, ct);
+                }
+                emit_uniform(ct, has, gpack);
             }
         }
     }
@@ -1252,18 +1319,22 @@ __global__ void __launch_bounds__(MAXT) blend_backward_corrected_kernel(BlendPar
             if (!__syncthreads_or(go)) break;
             const int bs = min(kBatchLayers, remaining);
             const int found = select_sweep(P, c, go, bs, lastDepth, lastJ, dl, jl, s_geo, s_id);
-            if (go) {
-                const int n = min(found, remaining);
-                for (int i = 0; i < n; ++i) {
-                    const int id = P.ids[jl[i]];
+            const int n = go ? min(found, remaining) : 0;
+            const int rounds = __reduce_max_sync(0xffffffffu, n);
+            for (int i = 0; i < rounds; ++i) {
+                int id = -1;
+                Contrib ct = {};
+                if (i < n) {
+                    id = P.ids[jl[i]];
                     float m[9], w[3];
                     load_geo(P.geo, id, m, w);
                     const Bary b = apply_bary(m, c.px, c.py);
                     const AttrRec a = load_attr<true>(P.attr, id);
-                    Contrib ct;
                     backward_one_prefix(w, a, b, c.px, c.py, pg, fin, pf, ct);
-                    emit_contrib(ct, gpack);
                 }
+                emit_warp(ct, i < n, id, gpack);
+            }
+            if (go) {
                 if (n > 0) {
                     lastDepth = dl[n - 1];
                     lastJ = jl[n - 1];
@@ -1287,15 +1358,16 @@ __global__ void __launch_bounds__(MAXT) blend_backward_corrected_kernel(BlendPar
                 while (mask) {
                     const int r = __ffsll((long long)mask) - 1;
                     mask &= mask - 1;
-                    if (done) continue;
                     const float* g = reinterpret_cast<const float*>(s_geo + kStagedQuads * r);
                     const Bary b = apply_bary(g, c.px, c.py);
-                    if (!covered(b)) continue;
-                    const AttrRec a = load_attr<true>(P.attr, s_id[r]);
-                    Contrib ct;
-                    backward_one_prefix(g + 12, a, b, c.px, c.py, pg, fin, pf, ct);
-                    emit_contrib(ct, gpack);
-                    if (++processed >= limit) done = true;
+                    const bool has = !done && covered(b);
+                    Contrib ct = {};
+                    if (has) {
+                        const AttrRec a = load_attr<true>(P.attr, s_id[r]);
+                        backward_one_prefix(g + 12, a, b, c.px, c.py, pg, fin, pf, ct);
+                        if (++processed >= limit) done = true;
+                    }
+                    emit_uniform(ct, has, gpack);
                 }
             }
             if (__syncthreads_and(done)) break;
