@@ -70,7 +70,7 @@ def build_extension(force: bool = False, verbose: bool = False) -> str:
 
 
 def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) -> str:
-    build_extension(force, verbose)
+    build_extension(verbose=verbose)
     if not force and not is_stale():
         return LIB
     objdir = os.path.join(HERE, "build")

@@ -825,16 +825,13 @@ static int check_dims_internal(int T, int W, int H, int tw, int th) {
     return TG_OK;
 }
 
-// Opt-in shared memory of a kernel, set once per device (`slot`: which kernel; setting it twice is harmless).
-static int allow_smem(const void* kernel, size_t bytes, int slot) {
-    constexpr int kMaxDevices = 64;
-    static std::atomic<bool> set[2][kMaxDevices];
+int allow_smem(const void* kernel, size_t bytes, SmemAllowed& allowed) {
     int dev = 0;
     TG_CUDA(cudaGetDevice(&dev));
-    TG_REQUIRE(dev >= 0 && dev < kMaxDevices, "device index outside the supported range");
-    if (!set[slot][dev].load(std::memory_order_acquire)) {
+    TG_REQUIRE(dev >= 0 && dev < SmemAllowed::kMaxDevices, "device index outside the supported range");
+    if (!allowed.set[dev].load(std::memory_order_acquire)) {
         TG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-        set[slot][dev].store(true, std::memory_order_release);
+        allowed.set[dev].store(true, std::memory_order_release);
     }
     return TG_OK;
 }
@@ -874,7 +871,8 @@ int bin_triangles(const float* vertices, const int32_t* indices, const float* co
     const int grid = (T + per_cta - 1) / per_cta;
     auto inverse = [](int n) { return (n & (n - 1)) == 0 ? 1.0 / n : 0.0; };
     auto kernel = cull ? tg::bin_kernel<true> : tg::bin_kernel<false>;
-    if (int st = allow_smem((const void*)kernel, tg::kBinSmem, cull ? 1 : 0)) return st;
+    static SmemAllowed allowed[2];
+    if (int st = allow_smem((const void*)kernel, tg::kBinSmem, allowed[cull ? 1 : 0])) return st;
     kernel<<<grid, 32 * tg::kBinWarps, tg::kBinSmem, stream>>>((const float4*)vertices, indices, colors, opacities, T, per_cta, W, H,
                                                     tw, th, inverse(tw), inverse(th), (float4*)tri_geo, (float4*)tri_attr,
                                                     bin, packed ? 1 : 0);

@@ -56,6 +56,12 @@ __device__ __forceinline__ void load_geo(const float4* geo, int id, float* m, fl
 }
 
 constexpr int kAttrQuads = TG_ATTR_WORDS / 4;
+// Brings a triangle's records towards L1: the backward knows the fragment after the current one (3 % of its time).
+__device__ __forceinline__ void prefetch_record(const BlendParams& P, int id) {
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(P.geo + 4 * (size_t)id));
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(P.attr + kAttrQuads * (size_t)id));
+}
+
 struct AttrRec { float o[3]; float c[9]; float iw[3]; int vid[3]; float xy[6]; };
 
 // FULL = false loads only what the forward pass needs (opacities, colours, 1/w).
@@ -514,11 +520,6 @@ __device__ __forceinline__ void red_add_v4(float4* addr, float a, float b, float
     asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b), "f"(c), "f"(d));
 }
 
-// process_backward of the reference (render.cu:455-538) for one fragment of one pixel; adds this
-// pixel's contribution for the triangle's three vertices into `gpack`.  The interpolation VJPs
-// (util.h:299-355) share 1/den; vertex-position gradients follow the reference's expanded partial
-// derivatives (util.h:405-455) term by term: for small triangles their fp32 cancellation is
-// systematic and part of what "the same result" means.
 __device__ __forceinline__ void emit_contrib(const Contrib& c, float4* __restrict__ gpack) {
 #pragma unroll
     for (int k = 0; k < 3; k++) {
@@ -586,88 +587,6 @@ __device__ __forceinline__ void emit_warp(const Contrib& c, bool has, int id, fl
     __syncwarp();
 }
 
-__device__ __forceinline__ void backward_one(const float* w, const AttrRec& a, const Bary& b, float px, float py,
-                                             const PixelGrad& pg, BackState& st, Contrib& out) {
-    const float bw0 = b.x * w[0], bw1 = b.y * w[1], bw2 = b.z * w[2];
-    const float den = bw0 + bw1 + bw2;
-    const bool ok = !(den * den < kEffZero);
-    const float inv = rcp_fast(den);
-    const float o_raw = (bw0 * a.o[0] + bw1 * a.o[1] + bw2 * a.o[2]) * inv;
-    const float o = fminf(fmaxf(o_raw, 0.f), kMaxOpacity);
-    const float cr = (bw0 * a.c[0] + bw1 * a.c[3] + bw2 * a.c[6]) * inv;
-    const float cg = (bw0 * a.c[1] + bw1 * a.c[4] + bw2 * a.c[7]) * inv;
-    const float cb = (bw0 * a.c[2] + bw1 * a.c[5] + bw2 * a.c[8]) * inv;
-    const float iw0 = a.iw[0], iw1 = a.iw[1], iw2 = a.iw[2];
-    const float denz = b.x + b.y + b.z;
-    const bool okz = !(denz * denz < kEffZero);
-    const float invz = rcp_fast(denz);
-    const float z = (b.x * iw0 + b.y * iw1 + b.z * iw2) * invz;
-    const float iom = rcp_fast(1.f - o);
-
-    const float drgb_do = ((cr * st.alpha - st.sr) * pg.gr + (cg * st.alpha - st.sg) * pg.gg + (cb * st.alpha - st.sb) * pg.gb -
-                           pg.ga * pg.final_alpha) * iom;
-    st.alpha = st.alpha * iom;
-    const float ao = st.alpha * o;
-    st.sr += cr * ao;
-    st.sg += cg * ao;
-    st.sb += cb * ao;
-    const float ddw_do = st.alpha - st.oa * iom;
-    const float dud_do = st.alpha * z - st.zoa * iom;
-    st.oa += ao;
-    st.zoa += z * ao;
-    const bool has_w = !(pg.final_weight < kEffZero);
-    const float inv_fw = has_w ? rcp_fast(pg.final_weight) : 0.f;
-    const float dd_do = (dud_do - pg.final_depth * ddw_do) * inv_fw * pg.gd;
-    const float d_do = drgb_do + (has_w ? dd_do : 0.f);
-
-    // upstream of the four weighted interpolations (0 where the reference's guard returns zeros)
-    const float uo = ok ? d_do * inv : 0.f;
-    const float ur = ok ? ao * pg.gr * inv : 0.f, ug = ok ? ao * pg.gg * inv : 0.f, ub = ok ? ao * pg.gb * inv : 0.f;
-    // e_k = sum over attributes of upstream * (a_k - value): d/d(b_k w_k) of the interpolated values
-    const float e0 = uo * (a.o[0] - o_raw) + ur * (a.c[0] - cr) + ug * (a.c[1] - cg) + ub * (a.c[2] - cb);
-    const float e1 = uo * (a.o[1] - o_raw) + ur * (a.c[3] - cr) + ug * (a.c[4] - cg) + ub * (a.c[5] - cb);
-    const float e2 = uo * (a.o[2] - o_raw) + ur * (a.c[6] - cr) + ug * (a.c[7] - cg) + ub * (a.c[8] - cb);
-    // depth interpolation (values 1/w, unit weights)
-    const float uz = (okz && has_w) ? ao * pg.gd * inv_fw * invz : 0.f;
-    const float z0 = uz * (iw0 - z), z1 = uz * (iw1 - z), z2 = uz * (iw2 - z);
-    const float g0 = w[0] * e0 + z0, g1 = w[1] * e1 + z1, g2 = w[2] * e2 + z2;       // d/d bary
-    // d/dw: weighted interpolations, plus (as the reference does, render.cu:530) the gradient w.r.t. the unit
-    // weights of the depth interpolation, plus the chain through the values 1/w
-    const float gw0 = b.x * e0 + b.x * z0 - uz * b.x * iw0 * iw0;
-    const float gw1 = b.y * e1 + b.y * z1 - uz * b.y * iw1 * iw1;
-    const float gw2 = b.z * e2 + b.z * z2 - uz * b.z * iw2 * iw2;
-
-    // barycentric_backward: l by cross products, then the expanded partials
-    const float ax = a.xy[0], ay = a.xy[1], bx = a.xy[2], by = a.xy[3], cx = a.xy[4], cy = a.xy[5];
-    float gxy[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    const float d = ax * (by - cy) + bx * (-ay + cy) + cx * (ay - by);
-    if (!(fabsf(d) < kEffZero)) {
-        const float iT = rcp_fast((bx - ax) * (cy - ay) - (by - ay) * (cx - ax));
-        const float lx = ((bx - px) * (cy - py) - (by - py) * (cx - px)) * iT;
-        const float ly = ((cx - px) * (ay - py) - (cy - py) * (ax - px)) * iT;
-        const float lz = ((ax - px) * (by - py) - (ay - py) * (bx - px)) * iT;
-        const float id = rcp_fast(d);
-        gxy[0] = (g0 * (lx * (-by + cy)) + g1 * (-cy - ly * (by - cy) + py) + g2 * (by - lz * (by - cy) - py)) * id;
-        gxy[1] = (g0 * (lx * (bx - cx)) + g1 * (cx + ly * (bx - cx) - px) + g2 * (-bx + lz * (bx - cx) + px)) * id;
-        gxy[2] = (g0 * (cy + lx * (ay - cy) - py) + g1 * (ly * (ay - cy)) + g2 * (-ay + lz * (ay - cy) + py)) * id;
-        gxy[3] = (g0 * (-cx - lx * (ax - cx) + px) + g1 * (ly * (-ax + cx)) + g2 * (ax - lz * (ax - cx) - px)) * id;
-        gxy[4] = (g0 * (-by - lx * (ay - by) + py) + g1 * (ay - ly * (ay - by) - py) + g2 * (lz * (-ay + by))) * id;
-        gxy[5] = (g0 * (bx + lx * (ax - bx) - px) + g1 * (-ax + ly * (ax - bx) + px) + g2 * (lz * (ax - bx))) * id;
-    }
-    const float gw[3] = {gw0, gw1, gw2}, bwk[3] = {bw0, bw1, bw2};
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-        out.vid[k] = a.vid[k];
-        out.v[k][0] = gxy[2 * k];
-        out.v[k][1] = gxy[2 * k + 1];
-        out.v[k][2] = gw[k];
-        out.v[k][3] = uo * bwk[k];
-        out.v[k][4] = ur * bwk[k];
-        out.v[k][5] = ug * bwk[k];
-        out.v[k][6] = ub * bwk[k];
-    }
-}
-
 struct BackwardIn {
     const float4* gimage;
     const float* gdepth;
@@ -687,6 +606,8 @@ struct BackwardIn {
 };
 constexpr int kLossPartials = 64;
 
+// DEPTH = false: no gradient flows into the depth map, so neither it nor the final weight is read.
+template <bool DEPTH = true>
 __device__ __forceinline__ int load_pixel_state(const TileCtx& c, const BlendParams& P, const BackwardIn& in,
                                                 PixelGrad& pg, BackState& st, float* sq_diff = nullptr) {
     pg = PixelGrad{};
@@ -712,77 +633,15 @@ __device__ __forceinline__ int load_pixel_state(const TileCtx& c, const BlendPar
     } else {
         const float4 gi = in.gimage[index];
         pg.gr = gi.x; pg.gg = gi.y; pg.gb = gi.z; pg.ga = gi.w;
-        pg.gd = in.gdepth ? in.gdepth[index] : 0.f;      // no depth-map gradient given: zero
+        pg.gd = DEPTH && in.gdepth ? in.gdepth[index] : 0.f;      // no depth-map gradient given: zero
     }
     pg.final_alpha = img.w;
-    pg.final_weight = in.final_w[index];
-    pg.final_depth = in.depthmap[index];
+    if (DEPTH) {
+        pg.final_weight = in.final_w[index];
+        pg.final_depth = in.depthmap[index];
+    }
     st.alpha = pg.final_alpha;
     return min(in.ends[index], P.max_layers);
-}
-
-// Default mode with the per-pixel fragment ids saved by the forward pass: no list search, no shared
-// memory, no barriers - every thread walks its own fragments last to first.
-template <int MAXT>
-__global__ void __launch_bounds__(MAXT, MAXT <= 256 ? 4 : 1) blend_backward_saved_kernel(BlendParams P, BackwardIn in,
-                                                                    const int* __restrict__ sel,
-                                                                    float4* __restrict__ gpack) {
-    __shared__ float s_coord[kMaxTileCoords];
-    const TileCtx c = tile_context(P, s_coord);
-    PixelGrad pg;
-    BackState st;
-    float sq = 0.f;
-    const int n = load_pixel_state(c, P, in, pg, st, &sq);
-    const size_t plane = (size_t)P.W * P.H, index = (size_t)c.iy * P.W + c.ix;
-    const int lane = lane_id();
-    if (in.l2_target || in.l2_target_u8) {
-        // loss: warp sum, then one atomic per warp into one of 64 partial sums (spread addresses)
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, d);
-        if (lane == 0 && sq != 0.f) atomicAdd(in.l2_partials + ((blockIdx.x * 8 + (threadIdx.x >> 5)) & (kLossPartials - 1)), sq);
-    }
-    int nmax = n;
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) nmax = max(nmax, __shfl_xor_sync(0xffffffffu, nmax, d));
-    // 2x2 pixel quads of the warp's 8x4 block: lanes L, L^1, L^8, L^9
-    const unsigned quad = 0x303u << (lane & ~9);
-    // ids are fetched one fragment ahead of their use
-    int id_next = (n > 0) ? sel[(size_t)(n - 1) * plane + index] : 0;
-    for (int s = 0; s < nmax; s++) {
-        const int k = n - 1 - s;
-        const bool has = k >= 0;
-        const int id = has ? id_next : -1 - lane;          // distinct negatives never match
-        if (k > 0) id_next = sel[(size_t)(k - 1) * plane + index];
-        Contrib ct;
-#pragma unroll
-        for (int j = 0; j < 3; j++) {
-            ct.vid[j] = 0;
-#pragma unroll
-            for (int q = 0; q < 7; q++) ct.v[j][q] = 0.f;
-        }
-        if (has) {
-            float m[9], w[3];
-            load_geo(P.geo, id, m, w);
-            const AttrRec a = load_attr<true>(P.attr, id);
-            const Bary b = apply_bary(m, c.px, c.py);
-            backward_one(w, a, b, c.px, c.py, pg, st, ct);
-        }
-        // Pixels of one quad that hold the same triangle are summed with two shuffle rounds and one
-        // lane issues the reductions: fewer, fuller vector atomics.
-        const unsigned peers = __match_any_sync(0xffffffffu, id);
-        const bool full4 = has && ((peers & quad) == quad);
-#pragma unroll
-        for (int j = 0; j < 3; j++) {
-#pragma unroll
-            for (int q = 0; q < 7; q++) {
-                float t = ct.v[j][q];
-                t += __shfl_xor_sync(0xffffffffu, t, 1);
-                t += __shfl_xor_sync(0xffffffffu, t, 8);
-                if (full4) ct.v[j][q] = t;
-            }
-        }
-        if (has && (!full4 || (lane & 9) == 0)) emit_contrib(ct, gpack);
-    }
 }
 
 // ---- default mode, two-part gradient with a per-warp queue ------------------------------------------
@@ -791,8 +650,9 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? 4 : 1) blend_backward_save
 // the work is split: part A (per pixel, back to front) runs the recurrence and produces the upstream
 // gradients of the fragment's interpolations; these go into a queue in shared memory; part B (the
 // expensive barycentric partials and the 21 per-vertex outputs) pops 32 queued fragments at a time and
-// so runs with full warps.  The arithmetic per fragment is that of backward_one.  A warp whose lanes are
-// busy anyway (deep overlap, or one opaque layer everywhere) skips the queue.
+// so runs with full warps.  A warp whose lanes are busy anyway (deep overlap, or one opaque layer everywhere) skips the
+// queue.  (Bound by L1 data wavefronts, 78 %, and by the latency of the gathers.)
+// DEPTH = false (everywhere below): no gradient flows into the depth map, the terms that it feeds are left out.
 struct QueuedFragment {
     float px, py;
     int id;
@@ -800,11 +660,40 @@ struct QueuedFragment {
     float o_raw, cr, cg, cb, z;
     float uo, ur, ug, ub, uz;
 };
-constexpr int kQueueFields = 16, kQueueSlots = 64;
+// A warp's queue: 64 slots of 4 quads, 5 apart (the odd pitch spreads consecutive slots over the banks).
+constexpr int kQueueSlots = 64, kQueuePitch = 5, kQueueQuads = kQueueSlots * kQueuePitch;
+
+template <bool DEPTH>
+__device__ __forceinline__ void queue_push(float4* q, int slot, const QueuedFragment& f) {
+    q += kQueuePitch * slot;
+    q[0] = make_float4(f.px, f.py, __int_as_float(f.id), f.bx);
+    q[1] = make_float4(f.by, f.bz, f.o_raw, f.cr);
+    q[2] = make_float4(f.cg, f.cb, f.uo, f.ur);
+    if (DEPTH) q[3] = make_float4(f.ug, f.ub, f.z, f.uz);
+    else *reinterpret_cast<float2*>(q + 3) = make_float2(f.ug, f.ub);
+}
+template <bool DEPTH>
+__device__ __forceinline__ QueuedFragment queue_pop(const float4* q, int slot) {
+    QueuedFragment f;
+    q += kQueuePitch * slot;
+    const float4 a = q[0], b = q[1], c = q[2];
+    f.px = a.x; f.py = a.y; f.id = __float_as_int(a.z); f.bx = a.w;
+    f.by = b.x; f.bz = b.y; f.o_raw = b.z; f.cr = b.w;
+    f.cg = c.x; f.cb = c.y; f.uo = c.z; f.ur = c.w;
+    if (DEPTH) {
+        const float4 d = q[3];
+        f.ug = d.x; f.ub = d.y; f.z = d.z; f.uz = d.w;
+    } else {
+        const float2 d = *reinterpret_cast<const float2*>(q + 3);
+        f.ug = d.x; f.ub = d.y; f.z = 0.f; f.uz = 0.f;
+    }
+    return f;
+}
 
 // Part A, second half: the transmittance recurrence of render.cu:455-538 for one fragment (back to
 // front) and the upstream gradients of its interpolations.  inv_den / inv_denz are the reciprocals of
 // the interpolation denominators, or 0 where the reference's guard returns zero gradients.
+template <bool DEPTH>
 __device__ __forceinline__ void backward_recurrence(float o_raw, float cr, float cg, float cb, float z, float inv_den,
                                                     float inv_denz, const PixelGrad& pg, BackState& st,
                                                     QueuedFragment& f) {
@@ -817,23 +706,28 @@ __device__ __forceinline__ void backward_recurrence(float o_raw, float cr, float
     st.sr += cr * ao;
     st.sg += cg * ao;
     st.sb += cb * ao;
-    const float ddw_do = st.alpha - st.oa * iom;
-    const float dud_do = st.alpha * z - st.zoa * iom;
-    st.oa += ao;
-    st.zoa += z * ao;
-    const bool has_w = !(pg.final_weight < kEffZero);
-    const float inv_fw = has_w ? rcp_fast(pg.final_weight) : 0.f;
-    const float dd_do = (dud_do - pg.final_depth * ddw_do) * inv_fw * pg.gd;
-    const float d_do = drgb_do + (has_w ? dd_do : 0.f);
+    float d_do = drgb_do, uz = 0.f;
+    if (DEPTH) {
+        const float ddw_do = st.alpha - st.oa * iom;
+        const float dud_do = st.alpha * z - st.zoa * iom;
+        st.oa += ao;
+        st.zoa += z * ao;
+        const bool has_w = !(pg.final_weight < kEffZero);
+        const float inv_fw = has_w ? rcp_fast(pg.final_weight) : 0.f;
+        const float dd_do = (dud_do - pg.final_depth * ddw_do) * inv_fw * pg.gd;
+        d_do = drgb_do + (has_w ? dd_do : 0.f);
+        uz = has_w ? ao * pg.gd * inv_fw * inv_denz : 0.f;
+    }
     f.o_raw = o_raw; f.cr = cr; f.cg = cg; f.cb = cb; f.z = z;
     f.uo = d_do * inv_den;
     f.ur = ao * pg.gr * inv_den;
     f.ug = ao * pg.gg * inv_den;
     f.ub = ao * pg.gb * inv_den;
-    f.uz = has_w ? ao * pg.gd * inv_fw * inv_denz : 0.f;
+    f.uz = uz;
 }
 
 // Part A: interpolations of the fragment (approximate reciprocals), then the recurrence.
+template <bool DEPTH>
 __device__ __forceinline__ void backward_state(const float* w, const AttrRec& a, const Bary& b, const PixelGrad& pg,
                                                BackState& st, QueuedFragment& f) {
     const float bw0 = b.x * w[0], bw1 = b.y * w[1], bw2 = b.z * w[2];
@@ -844,26 +738,42 @@ __device__ __forceinline__ void backward_state(const float* w, const AttrRec& a,
     const float cr = (bw0 * a.c[0] + bw1 * a.c[3] + bw2 * a.c[6]) * inv;
     const float cg = (bw0 * a.c[1] + bw1 * a.c[4] + bw2 * a.c[7]) * inv;
     const float cb = (bw0 * a.c[2] + bw1 * a.c[5] + bw2 * a.c[8]) * inv;
-    const float denz = b.x + b.y + b.z;
-    const bool okz = !(denz * denz < kEffZero);
-    const float invz = rcp_fast(denz);
-    const float z = (b.x * a.iw[0] + b.y * a.iw[1] + b.z * a.iw[2]) * invz;
+    float z = 0.f, inv_denz = 0.f;
+    if (DEPTH) {
+        const float denz = b.x + b.y + b.z;
+        const bool okz = !(denz * denz < kEffZero);
+        const float invz = rcp_fast(denz);
+        z = (b.x * a.iw[0] + b.y * a.iw[1] + b.z * a.iw[2]) * invz;
+        inv_denz = okz ? invz : 0.f;
+    }
     f.bx = b.x; f.by = b.y; f.bz = b.z;
-    backward_recurrence(o_raw, cr, cg, cb, z, ok ? inv : 0.f, okz ? invz : 0.f, pg, st, f);
+    backward_recurrence<DEPTH>(o_raw, cr, cg, cb, z, ok ? inv : 0.f, inv_denz, pg, st, f);
 }
 
-// Part B: from the upstream gradients to the contribution for the triangle's three vertices.
+// Part B: from the upstream gradients to the contribution for the triangle's three vertices: process_backward of the
+// reference (render.cu:455-538).  The interpolation VJPs (util.h:299-355) share 1/den; vertex-position gradients follow
+// the reference's expanded partial derivatives (util.h:405-455) term by term: for small triangles their fp32
+// cancellation is systematic and part of what "the same result" means.
+template <bool DEPTH>
 __device__ __forceinline__ void backward_outputs(const float* w, const AttrRec& a, const QueuedFragment& f, Contrib& out) {
-    const float uo = f.uo, ur = f.ur, ug = f.ug, ub = f.ub, uz = f.uz;
+    const float uo = f.uo, ur = f.ur, ug = f.ug, ub = f.ub;
+    // e_k = sum over attributes of upstream * (a_k - value): d/d(b_k w_k) of the interpolated values
     const float e0 = uo * (a.o[0] - f.o_raw) + ur * (a.c[0] - f.cr) + ug * (a.c[1] - f.cg) + ub * (a.c[2] - f.cb);
     const float e1 = uo * (a.o[1] - f.o_raw) + ur * (a.c[3] - f.cr) + ug * (a.c[4] - f.cg) + ub * (a.c[5] - f.cb);
     const float e2 = uo * (a.o[2] - f.o_raw) + ur * (a.c[6] - f.cr) + ug * (a.c[7] - f.cg) + ub * (a.c[8] - f.cb);
-    const float iw0 = a.iw[0], iw1 = a.iw[1], iw2 = a.iw[2];
-    const float z0 = uz * (iw0 - f.z), z1 = uz * (iw1 - f.z), z2 = uz * (iw2 - f.z);
-    const float g0 = w[0] * e0 + z0, g1 = w[1] * e1 + z1, g2 = w[2] * e2 + z2;
-    const float gw0 = f.bx * e0 + f.bx * z0 - uz * f.bx * iw0 * iw0;
-    const float gw1 = f.by * e1 + f.by * z1 - uz * f.by * iw1 * iw1;
-    const float gw2 = f.bz * e2 + f.bz * z2 - uz * f.bz * iw2 * iw2;
+    float g0 = w[0] * e0, g1 = w[1] * e1, g2 = w[2] * e2;                        // d/d bary
+    float gw0 = f.bx * e0, gw1 = f.by * e1, gw2 = f.bz * e2;                     // d/dw
+    if (DEPTH) {
+        // depth interpolation (values 1/w, unit weights); d/dw as the reference does it (render.cu:530): also the gradient
+        // w.r.t. the unit weights, plus the chain through the values 1/w
+        const float uz = f.uz, iw0 = a.iw[0], iw1 = a.iw[1], iw2 = a.iw[2];
+        const float z0 = uz * (iw0 - f.z), z1 = uz * (iw1 - f.z), z2 = uz * (iw2 - f.z);
+        g0 += z0; g1 += z1; g2 += z2;
+        gw0 = gw0 + f.bx * z0 - uz * f.bx * iw0 * iw0;
+        gw1 = gw1 + f.by * z1 - uz * f.by * iw1 * iw1;
+        gw2 = gw2 + f.bz * z2 - uz * f.bz * iw2 * iw2;
+    }
+    // barycentric_backward: l by cross products, then the expanded partials
     const float px = f.px, py = f.py;
     const float ax = a.xy[0], ay = a.xy[1], bx = a.xy[2], by = a.xy[3], cx = a.xy[4], cy = a.xy[5];
     float gxy[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -895,129 +805,146 @@ __device__ __forceinline__ void backward_outputs(const float* w, const AttrRec& 
     }
 }
 
-// Part B for the fragments in queue slots first .. first + count - 1 (count <= 32), one per lane.
-// Consecutive slots that hold the same triangle (neighbouring pixels mostly do) are summed over runs of
-// up to four with two shuffle rounds before the vector reductions are issued (a third round, runs of
-// eight, costs more in shuffles than it saves in reductions).
-__device__ __forceinline__ void drain_queue(const BlendParams& P, float (*q)[kQueueSlots], int first, int count,
-                                            float4* __restrict__ gpack) {
-    const int lane = lane_id();
-    const bool valid = lane < count;
+// Both parts for one fragment of one pixel.
+template <bool DEPTH = true>
+__device__ __forceinline__ void backward_one(const float* w, const AttrRec& a, const Bary& b, float px, float py,
+                                             const PixelGrad& pg, BackState& st, Contrib& out) {
     QueuedFragment f;
-    const int slot = first + (valid ? lane : 0);
-    f.px = q[0][slot]; f.py = q[1][slot]; f.id = __float_as_int(q[2][slot]);
-    f.bx = q[3][slot]; f.by = q[4][slot]; f.bz = q[5][slot];
-    f.o_raw = q[6][slot]; f.cr = q[7][slot]; f.cg = q[8][slot]; f.cb = q[9][slot]; f.z = q[10][slot];
-    f.uo = q[11][slot]; f.ur = q[12][slot]; f.ug = q[13][slot]; f.ub = q[14][slot]; f.uz = q[15][slot];
-    const int id = valid ? f.id : -1 - lane;
-    Contrib ct;
-#pragma unroll
-    for (int j = 0; j < 3; j++) {
-        ct.vid[j] = 0;
-#pragma unroll
-        for (int k = 0; k < 7; k++) ct.v[j][k] = 0.f;
-    }
-    if (valid) {
-        const float4 g3 = __ldg(P.geo + 4 * (size_t)id + 3);
-        const float w[3] = {g3.x, g3.y, g3.z};
-        const AttrRec a = load_attr<true>(P.attr, id);
-        backward_outputs(w, a, f, ct);
-    }
-    // runs of equal triangle ids in lane order
-    const int prev = __shfl_up_sync(0xffffffffu, id, 1);
-    const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || prev != id);
-    const unsigned above = (lane == 31) ? 1u : (heads >> (lane + 1));      // head flags of lanes lane+1 .. (bit 0 = next lane)
-    const bool same1 = (above & 1u) == 0 && lane + 1 < 32;
-    const bool same2 = (above & 3u) == 0 && lane + 2 < 32;
-    const int run_start = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
-#pragma unroll
-    for (int j = 0; j < 3; j++) {
-#pragma unroll
-        for (int k = 0; k < 7; k++) {
-            float t = ct.v[j][k], u;
-            u = __shfl_down_sync(0xffffffffu, t, 1); if (same1) t += u;
-            u = __shfl_down_sync(0xffffffffu, t, 2); if (same2) t += u;
-            ct.v[j][k] = t;
-        }
-    }
-    if (valid && ((lane - run_start) & 3) == 0) emit_contrib(ct, gpack);
+    f.px = px; f.py = py; f.id = 0;
+    backward_state<DEPTH>(w, a, b, pg, st, f);
+    backward_outputs<DEPTH>(w, a, f, out);
 }
 
-// Whole fragments per round, for warps whose lanes are busy anyway.  Pixels of one 2x2 quad (lanes L, L^1,
-// L^8, L^9 of the warp's 8x4 block) that hold the same triangle are summed before one lane issues the
-// reductions.  Kept out of line so that it does not weigh on the register allocation of the queued path.
+// Contributions of a warp's lanes (triangles `id`) with as few atomics as their triangles allow.  All lanes must call.
+// The lanes' rows go to shared memory ordered by triangle, sixteen at a time; 24 lanes add the columns up and send each
+// triangle's three 32-byte slots with one instruction.  The vertex ids ride in the unused eighth word of every slot.
+// (Adding up to four neighbouring lanes with 42 shuffles and six vector reductions per run took as long where a triangle
+// has one or two of the 32 fragments, and 17 % longer where a few triangles have them all: 2M overlapping triangles, 4K,
+// 944 us against 804.)
+// `rows`: kRowsQuads quads of shared memory of this warp.
+constexpr int kRowQuads = 7;                  // 6 used; the odd pitch spreads the rows over the banks
+constexpr int kRowsQuads = 16 * kRowQuads;
+__device__ __forceinline__ void emit_lanes(const Contrib& c, bool valid, int id, float4* rows, float4* __restrict__ gpack) {
+    const int lane = lane_id();
+    const unsigned peers = __match_any_sync(0xffffffffu, valid ? id : -1 - lane);      // distinct negatives never match
+    const unsigned below = (1u << lane) - 1u;
+    const bool leads = valid && (peers & below) == 0;
+    const int size = leads ? __popc(peers) : 0;
+    int incl = size;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += y;
+    }
+    const int total = __shfl_sync(0xffffffffu, incl, 31);
+    const int place = __shfl_sync(0xffffffffu, incl - size, __ffs(peers) - 1) + __popc(peers & below);
+    const unsigned ends = __reduce_or_sync(0xffffffffu, leads ? 1u << (incl - 1) : 0u);   // last row of every triangle
+    const float* column = reinterpret_cast<const float*>(rows) + min(lane, 4 * kRowQuads - 1);
+    const int* ids = reinterpret_cast<const int*>(rows) + (min(lane, 23) | 7);
+    const bool adds = lane < 24 && (lane & 7) != 7;
+    float sum = 0.f;
+#pragma unroll 1
+    for (int half = 0; half < total; half += 16) {
+        __syncwarp();                     // the rows before have been added up
+        if (valid && place >= half && place < half + 16) {
+            float4* row = rows + kRowQuads * (place - half);
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                row[2 * k] = make_float4(c.v[k][0], c.v[k][1], c.v[k][2], c.v[k][3]);
+                row[2 * k + 1] = make_float4(c.v[k][4], c.v[k][5], c.v[k][6], __int_as_float(c.vid[k]));
+            }
+        }
+        __syncwarp();
+        const int n = min(16, total - half);
+        const unsigned end_bits = ends >> half;
+#pragma unroll 1
+        for (int j = 0; j < n; j += 4) {
+            float x[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) x[k] = column[4 * kRowQuads * (j + k)];     // rows past `total` end no triangle
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                sum += x[k];
+                if ((end_bits >> (j + k)) & 1u) {
+                    const int vid = ids[4 * kRowQuads * (j + k)];
+                    if (adds) atomicAdd(reinterpret_cast<float*>(gpack + 2 * (size_t)vid) + (lane & 7), sum);
+                    sum = 0.f;
+                }
+            }
+        }
+    }
+    __syncwarp();
+}
+
+// Part B for the fragments in queue slots first .. first + count - 1 (count <= 32), one per lane.  The slots from `first`
+// on, at least 33 of them, are free once the fragments are in registers.
+static_assert(kRowsQuads <= 33 * kQueuePitch, "rows in the free part of the queue");
+template <bool DEPTH>
+__device__ __forceinline__ void drain_queue(const BlendParams& P, float4* q, int first, int count, float4* __restrict__ gpack) {
+    const int lane = lane_id();
+    const bool valid = lane < count;
+    const QueuedFragment f = queue_pop<DEPTH>(q, first + (valid ? lane : 0));
+    Contrib ct = {};
+    if (valid) {
+        const float4 g3 = __ldg(P.geo + 4 * (size_t)f.id + 3);
+        const float w[3] = {g3.x, g3.y, g3.z};
+        const AttrRec a = load_attr<true>(P.attr, f.id);
+        backward_outputs<DEPTH>(w, a, f, ct);
+    }
+    __syncwarp();
+    emit_lanes(ct, valid, f.id, q + kQueuePitch * first, gpack);
+}
+
+// Whole fragments per round, for warps whose lanes are busy anyway.  Kept out of line so that it does not weigh on the
+// register allocation of the queued path.
+template <bool DEPTH>
 __device__ __noinline__ void backward_rounds_direct(const BlendParams& P, float px, float py, PixelGrad pg, BackState st,
                                                     int n, int nmax, int id_next, const int* __restrict__ sel_pixel,
-                                                    size_t plane, float4* __restrict__ gpack) {
-    const int lane = lane_id();
-    const unsigned quad = 0x303u << (lane & ~9);
+                                                    size_t plane, float4* rows, float4* __restrict__ gpack) {
     for (int s = 0; s < nmax; s++) {
         const int k = n - 1 - s;
         const bool has = k >= 0;
-        const int id = has ? id_next : -1 - lane;          // distinct negatives never match
+        const int id = id_next;
         if (k > 0) id_next = sel_pixel[(size_t)(k - 1) * plane];
-        Contrib ct;
-#pragma unroll
-        for (int j = 0; j < 3; j++) {
-            ct.vid[j] = 0;
-#pragma unroll
-            for (int i = 0; i < 7; i++) ct.v[j][i] = 0.f;
-        }
+        Contrib ct = {};
         if (has) {
             float m[9], w[3];
             load_geo(P.geo, id, m, w);
             const AttrRec a = load_attr<true>(P.attr, id);
             const Bary b = apply_bary(m, px, py);
-            backward_one(w, a, b, px, py, pg, st, ct);
+            backward_one<DEPTH>(w, a, b, px, py, pg, st, ct);
         }
-        const unsigned peers = __match_any_sync(0xffffffffu, id);
-        const bool full4 = has && ((peers & quad) == quad);
-#pragma unroll
-        for (int j = 0; j < 3; j++) {
-#pragma unroll
-            for (int i = 0; i < 7; i++) {
-                float t = ct.v[j][i];
-                t += __shfl_xor_sync(0xffffffffu, t, 1);
-                t += __shfl_xor_sync(0xffffffffu, t, 8);
-                if (full4) ct.v[j][i] = t;
-            }
-        }
-        if (has && (!full4 || (lane & 9) == 0)) emit_contrib(ct, gpack);
+        emit_lanes(ct, has, id, rows, gpack);
     }
 }
 
-template <int MAXT>
-__global__ void __launch_bounds__(MAXT, 1024 / MAXT) blend_backward_queued_kernel(BlendParams P, BackwardIn in,
+template <int MAXT, bool DEPTH>
+__global__ void __launch_bounds__(MAXT, DEPTH ? 7 : 8) blend_backward_queued_kernel(BlendParams P, BackwardIn in,
                                                                         const int* __restrict__ sel,
                                                                         float4* __restrict__ gpack) {
     static_assert(MAXT % 32 == 0 && MAXT <= 256, "one queue per warp, at most 8 warps");
     __shared__ float s_coord[MAXT + 2];      // tile_w + tile_h <= tile_w * tile_h + 1 <= MAXT + 1
-    __shared__ float s_queue[MAXT / 32][kQueueFields][kQueueSlots];
+    __shared__ float4 s_queue[MAXT / 32][kQueueQuads];
     const TileCtx c = tile_context(P, s_coord);
     PixelGrad pg;
     BackState st;
     float sq = 0.f;
-    const int n = load_pixel_state(c, P, in, pg, st, &sq);
+    const int n = load_pixel_state<DEPTH>(c, P, in, pg, st, &sq);
     const size_t plane = (size_t)P.W * P.H, index = (size_t)c.iy * P.W + c.ix;
     const int lane = lane_id();
-    float (*q)[kQueueSlots] = s_queue[threadIdx.x >> 5];
+    float4* q = s_queue[threadIdx.x >> 5];
+    int id_next = (n > 0) ? sel[(size_t)(n - 1) * plane + index] : 0;   // ids are fetched one fragment ahead
     if (in.l2_target || in.l2_target_u8) {
         // loss: warp sum, then one atomic per warp into one of 64 partial sums (spread addresses)
 #pragma unroll
         for (int d = 16; d > 0; d >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, d);
         if (lane == 0 && sq != 0.f) atomicAdd(in.l2_partials + ((blockIdx.x * 8 + (threadIdx.x >> 5)) & (kLossPartials - 1)), sq);
     }
-    int nmax = n;
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) nmax = max(nmax, __shfl_xor_sync(0xffffffffu, nmax, d));
-    int nsum = n;
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) nsum += __shfl_xor_sync(0xffffffffu, nsum, d);
-    int id_next = (n > 0) ? sel[(size_t)(n - 1) * plane + index] : 0;   // ids are fetched one fragment ahead
+    const int nmax = __reduce_max_sync(0xffffffffu, n), nsum = __reduce_add_sync(0xffffffffu, n);
     if (nsum * 10 >= nmax * 32 * 9) {
         // Nearly all lanes have a fragment in every round (90 % or more): the queue would cost more than the idle
         // lanes do.
-        backward_rounds_direct(P, c.px, c.py, pg, st, n, nmax, id_next, sel + index, plane, gpack);
+        backward_rounds_direct<DEPTH>(P, c.px, c.py, pg, st, n, nmax, id_next, sel + index, plane, q, gpack);
         return;
     }
     int queued = 0;                                    // uniform over the warp
@@ -1031,24 +958,22 @@ __global__ void __launch_bounds__(MAXT, 1024 / MAXT) blend_backward_queued_kerne
             float m[9], w[3];
             load_geo(P.geo, id, m, w);
             const AttrRec a = load_attr<false>(P.attr, id);
+            if (k > 0) prefetch_record(P, id_next);
             const Bary b = apply_bary(m, c.px, c.py);
             QueuedFragment f;
-            backward_state(w, a, b, pg, st, f);
-            const int slot = queued + __popc(pushing & ((1u << lane) - 1u));
-            q[0][slot] = c.px; q[1][slot] = c.py; q[2][slot] = __int_as_float(id);
-            q[3][slot] = f.bx; q[4][slot] = f.by; q[5][slot] = f.bz;
-            q[6][slot] = f.o_raw; q[7][slot] = f.cr; q[8][slot] = f.cg; q[9][slot] = f.cb; q[10][slot] = f.z;
-            q[11][slot] = f.uo; q[12][slot] = f.ur; q[13][slot] = f.ug; q[14][slot] = f.ub; q[15][slot] = f.uz;
+            f.px = c.px; f.py = c.py; f.id = id;
+            backward_state<DEPTH>(w, a, b, pg, st, f);
+            queue_push<DEPTH>(q, queued + __popc(pushing & ((1u << lane) - 1u)), f);
         }
         queued += __popc(pushing);
         __syncwarp();
         if (queued >= 32) {
             queued -= 32;
-            drain_queue(P, q, queued, 32, gpack);
+            drain_queue<DEPTH>(P, q, queued, 32, gpack);
             __syncwarp();
         }
     }
-    if (queued > 0) drain_queue(P, q, 0, queued, gpack);
+    if (queued > 0) drain_queue<DEPTH>(P, q, 0, queued, gpack);
 }
 
 // ---- one optimisation step of one view in a single kernel -------------------------------------------
@@ -1067,7 +992,7 @@ __global__ void __launch_bounds__(MAXT, 4) blend_step_l2_kernel(BlendParams P, f
     __shared__ float4 s_geo[kChunk * kStagedQuads];
     __shared__ int s_id[kChunk];
     __shared__ float s_coord[kMaxTileCoords];
-    __shared__ float s_queue[MAXT / 32][kQueueFields][kQueueSlots];
+    extern __shared__ float4 s_step[];       // queues of the warps
     const TileCtx c = tile_context(P, s_coord);
     const int lane = lane_id();
     PixelAcc acc;
@@ -1120,10 +1045,8 @@ __global__ void __launch_bounds__(MAXT, 4) blend_step_l2_kernel(BlendParams P, f
     for (int d = 16; d > 0; d >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, d);
     if (lane == 0 && sq != 0.f) atomicAdd(l2_partials + ((blockIdx.x * 8 + (threadIdx.x >> 5)) & (kLossPartials - 1)), sq);
 
-    float (*q)[kQueueSlots] = s_queue[threadIdx.x >> 5];
-    int nmax = n;
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) nmax = max(nmax, __shfl_xor_sync(0xffffffffu, nmax, d));
+    float4* q = s_step + kQueueQuads * (threadIdx.x >> 5);
+    const int nmax = __reduce_max_sync(0xffffffffu, n);
     int queued = 0;                                    // uniform over the warp
     for (int s = 0; s < nmax; s++) {
         const int k = n - 1 - s;
@@ -1132,23 +1055,20 @@ __global__ void __launch_bounds__(MAXT, 4) blend_step_l2_kernel(BlendParams P, f
         if (has) {
             const float4 k0 = kept[k][0], k1 = kept[k][1], k2 = kept[k][2];
             QueuedFragment f;
+            f.px = c.px; f.py = c.py; f.id = __float_as_int(k2.z);
             f.bx = k0.x; f.by = k0.y; f.bz = k0.z;
-            backward_recurrence(k0.w, k1.x, k1.y, k1.z, k1.w, k2.x, k2.y, pg, st, f);
-            const int slot = queued + __popc(pushing & ((1u << lane) - 1u));
-            q[0][slot] = c.px; q[1][slot] = c.py; q[2][slot] = k2.z;
-            q[3][slot] = f.bx; q[4][slot] = f.by; q[5][slot] = f.bz;
-            q[6][slot] = f.o_raw; q[7][slot] = f.cr; q[8][slot] = f.cg; q[9][slot] = f.cb; q[10][slot] = f.z;
-            q[11][slot] = f.uo; q[12][slot] = f.ur; q[13][slot] = f.ug; q[14][slot] = f.ub; q[15][slot] = f.uz;
+            backward_recurrence<false>(k0.w, k1.x, k1.y, k1.z, k1.w, k2.x, k2.y, pg, st, f);
+            queue_push<false>(q, queued + __popc(pushing & ((1u << lane) - 1u)), f);
         }
         queued += __popc(pushing);
         __syncwarp();
         if (queued >= 32) {
             queued -= 32;
-            drain_queue(P, q, queued, 32, gpack);
+            drain_queue<false>(P, q, queued, 32, gpack);
             __syncwarp();
         }
     }
-    if (queued > 0) drain_queue(P, q, 0, queued, gpack);
+    if (queued > 0) drain_queue<false>(P, q, 0, queued, gpack);
 }
 
 // General path (any max_layers, both modes): searches the list again as the reference does.
@@ -1287,7 +1207,7 @@ __device__ __forceinline__ void backward_one_prefix(const float* w, const AttrRe
     f.ug = ao * pg.gg * inv_den;
     f.ub = ao * pg.gb * inv_den;
     f.uz = (has_w && okz) ? ao * pg.gd * inv_fw * invz : 0.f;
-    backward_outputs(w, a, f, out);
+    backward_outputs<true>(w, a, f, out);
 }
 
 template <bool SORT, int MAXT>
@@ -1533,24 +1453,23 @@ static int backward_impl(const float* tri_geo, const float* tri_attr, const int3
     const tg::BackwardIn in = {(const float4*)grad_image, grad_depthmap, (const float4*)image, depthmap, final_weights,
                                ends, target_u8 ? nullptr : (const float4*)l2_target, l2_grad_scale, partials,
                                target_u8 ? (const uchar4*)l2_target : nullptr};
-    if (threads <= 256) {
-        if (saved) {
-            // The queued kernel walks the per-pixel selection, not the tile lists, so its blocks need not be the
-            // forward's tiles: 16x8 pixels (four warps) finish more evenly than whole tiles do, and a block's
-            // registers come free only when its slowest warp is done (config 3: 179 -> 173 µs; 64 threads the
-            // same, 32 threads slower again).
-            tg::BlendParams Q = P;
-            Q.tw = 16; Q.th = 8;
-            Q.tiles_x = (W + Q.tw - 1) / Q.tw;
-            Q.offsets = nullptr; Q.ids = nullptr; Q.order = nullptr;
-            const int blocks = Q.tiles_x * ((H + Q.th - 1) / Q.th);
-            tg::blend_backward_queued_kernel<128><<<blocks, 128, 0, s>>>(Q, in, selection, gpack);
-        }
-        else if (per_pixel_sort) tg::blend_backward_kernel<true, 256><<<tiles, threads, 0, s>>>(P, in, gpack);
+    if (saved) {
+        // The queued kernel walks the per-pixel selection, not the tile lists, so its blocks need not be the
+        // forward's tiles: 16x8 pixels (four warps) finish more evenly than whole tiles do, and a block's
+        // registers come free only when its slowest warp is done (config 3: 179 -> 173 µs; 64 threads the
+        // same, 32 threads slower again).
+        tg::BlendParams Q = P;
+        Q.tw = 16; Q.th = 8;
+        Q.tiles_x = (W + Q.tw - 1) / Q.tw;
+        Q.offsets = nullptr; Q.ids = nullptr; Q.order = nullptr;
+        const int blocks = Q.tiles_x * ((H + Q.th - 1) / Q.th);
+        if (grad_depthmap) tg::blend_backward_queued_kernel<128, true><<<blocks, 128, 0, s>>>(Q, in, selection, gpack);
+        else tg::blend_backward_queued_kernel<128, false><<<blocks, 128, 0, s>>>(Q, in, selection, gpack);
+    } else if (threads <= 256) {
+        if (per_pixel_sort) tg::blend_backward_kernel<true, 256><<<tiles, threads, 0, s>>>(P, in, gpack);
         else tg::blend_backward_kernel<false, 256><<<tiles, threads, 0, s>>>(P, in, gpack);
     } else {
-        if (saved) tg::blend_backward_saved_kernel<1024><<<tiles, threads, 0, s>>>(P, in, selection, gpack);
-        else if (per_pixel_sort) tg::blend_backward_kernel<true, 1024><<<tiles, threads, 0, s>>>(P, in, gpack);
+        if (per_pixel_sort) tg::blend_backward_kernel<true, 1024><<<tiles, threads, 0, s>>>(P, in, gpack);
         else tg::blend_backward_kernel<false, 1024><<<tiles, threads, 0, s>>>(P, in, gpack);
     }
     TG_LAUNCH_CHECK("blend_backward_kernel");
@@ -1590,7 +1509,10 @@ int tg_blend_step_l2(const float* tri_geo, const float* tri_attr, const int32_t*
     P.order = tg_host::g_tile_order;
     const int tiles = P.tiles_x * ((H + th - 1) / th);
     const int threads = ((tw * th + 31) / 32) * 32;
-    tg::blend_step_l2_kernel<256><<<tiles, threads, 0, s>>>(P, (float4*)image, depthmap, final_weights, ends,
+    static tg_host::SmemAllowed allowed;
+    constexpr size_t smem = 8 * sizeof(float4) * tg::kQueueQuads;
+    if (int st = tg_host::allow_smem((const void*)tg::blend_step_l2_kernel<256>, smem, allowed)) return st;
+    tg::blend_step_l2_kernel<256><<<tiles, threads, smem, s>>>(P, (float4*)image, depthmap, final_weights, ends,
                                                             (const float4*)target, grad_scale, partials, gpack);
     TG_LAUNCH_CHECK("blend_step_l2_kernel");
     if (packed) return TG_OK;

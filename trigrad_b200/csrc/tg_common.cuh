@@ -10,6 +10,8 @@
 #include <float.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "../../include/trigrad_b200.h"
 
 namespace tg {
@@ -145,6 +147,12 @@ namespace tg_host {
 void set_error(const char* fmt, ...);
 int cuda_fail(cudaError_t e, const char* what);
 void count_launch();
+// Opt-in shared memory of a kernel, set once per device (setting it twice is harmless).
+struct SmemAllowed {
+    static constexpr int kMaxDevices = 64;
+    std::atomic<bool> set[kMaxDevices];
+};
+int allow_smem(const void* kernel, size_t bytes, SmemAllowed& allowed);
 }  // namespace tg_host
 
 #define TG_CUDA(call)                                                   \

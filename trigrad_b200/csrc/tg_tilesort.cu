@@ -350,17 +350,9 @@ int sort_tile_lists(uint64_t* entries, const int32_t* offsets, int tiles, int32_
         TG_LAUNCH_CHECK("tile_sort_mid_kernel");
     }
     if (longest > (uint32_t)tg::kTileSortShort) {
-        constexpr int kMaxDevices = 64;
-        static std::atomic<bool> attr_set[kMaxDevices];   // zero-initialised; setting the attribute twice is harmless
+        static SmemAllowed allowed;
         const size_t long_smem = sizeof(uint64_t) * tg::kLongSmemWords;
-        int dev = 0;
-        TG_CUDA(cudaGetDevice(&dev));
-        TG_REQUIRE(dev >= 0 && dev < kMaxDevices, "device index outside the supported range");
-        if (!attr_set[dev].load(std::memory_order_acquire)) {
-            TG_CUDA(cudaFuncSetAttribute(tg::tile_sort_long_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)long_smem));
-            attr_set[dev].store(true, std::memory_order_release);
-        }
+        if (int st = allow_smem((const void*)tg::tile_sort_long_kernel, long_smem, allowed)) return st;
         const int grid = tiles < 148 ? tiles : 148;
         tg::tile_sort_long_kernel<<<grid, tg::kTileSortLongThreads, long_smem, s>>>(entries, offsets, sorted_ids, lists,
                                                                                      write_back ? 1 : 0);
