@@ -122,6 +122,7 @@ struct TileCtx {
     bool active;
     float px, py;
     WarpRect rect;
+    const float *s_x, *s_y;     // centres of the 8 columns and 4 rows of the warp's block, null without 8x4 blocks
 };
 
 // Pixel-centre coordinates need double arithmetic (one rounding, reference render.cu:561-562); the
@@ -155,6 +156,8 @@ __device__ __forceinline__ TileCtx tile_context(const BlendParams& P, float* s_c
     c.start = P.offsets ? P.offsets[c.tile] : 0;
     c.end = P.offsets ? P.offsets[c.tile + 1] : 0;
     __syncthreads();
+    c.s_x = blocks ? s_coord + bx0 : nullptr;
+    c.s_y = s_coord + P.tw + by0;
     c.px = s_coord[min(lx, P.tw - 1)];
     c.py = s_coord[P.tw + min(ly, P.th - 1)];
     if (blocks) {
@@ -261,43 +264,294 @@ __device__ __forceinline__ void cp_async16(float4* smem_dst, const float4* gmem_
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
-// One selection sweep over the whole tile list (select_next_k_in_tile, reference render.cu:375-415):
-// keeps the `bs` covered fragments smallest in (depth, j) among those after (lastDepth, lastJ).
-// All threads of the CTA must call it; `go` says whether this thread collects.
-// `s_attr`, when given, receives the attribute quads of the chunk as well (stage_attr_chunk).
-// `s_geo2` / `s_id2`, when given, are a second pair of staging buffers: a list of more than one chunk is then streamed
+// The nearest fragments a pixel has collected in a sweep: at most `bs` words (ordered depth << 32 | list position),
+// ascending.  One word per fragment, because the array lives in local memory.
+struct Batch {
+    uint64_t key[kBatchLayers];
+    int found;
+    float dfar;      // depth of the last one; -inf while the batch is empty, so the first fragment is appended
+};
+__device__ __forceinline__ float ordered_to_float(uint32_t u) {
+    return __uint_as_float((u & 0x80000000u) ? u & 0x7fffffffu : ~u);
+}
+
+// Fragment of the covering record (list position j) into the batch, unless it does not lie behind `last`.
+__device__ __forceinline__ void collect(Batch& s, int bs, uint64_t last, const Bary& b, const float4& q2, const float4& q3, int j) {
+    const float d = interp_rn(b, q2.y, q2.z, q2.w, q3.x, q3.y, q3.z);
+    const uint64_t key = ((uint64_t)float_to_ordered(d) << 32) | (uint32_t)j;
+    if (key <= last) return;
+    // the farthest kept depth stays in a register: lists come roughly front to back, so most
+    // fragments go to the end of the batch (ties keep list order) or, once it is full, nowhere
+    if (d >= s.dfar) {
+        if (s.found == bs) return;
+        s.key[s.found++] = key;
+        s.dfar = d;
+        return;
+    }
+    int pos = (s.found < bs) ? s.found : (bs - 1);
+    while (pos > 0) {
+        const uint64_t before = s.key[pos - 1];
+        if (key >= before) break;
+        s.key[pos--] = before;
+    }
+    s.key[pos] = key;
+    if (s.found < bs) s.found++;
+    s.dfar = ordered_to_float((uint32_t)(s.key[s.found - 1] >> 32));
+}
+
+// Two correctly rounded single-precision FMAs in one instruction.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("{ .reg .b64 a, b, c, d;\n\t"
+        "mov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\t"
+        "fma.rn.f32x2 d, a, b, c;\n\tmov.b64 {%0, %1}, d; }"
+        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
+
+// Coverage of `rows` rows of the warp's 8x4 pixel block, from row `row` on, by the record whose matrix is in m: bit
+// 8 * row + column, decided with the operations of apply_bary and covered().
+__device__ __forceinline__ unsigned cover_rows(const float* m, const float* s_x /*[8], 16-byte aligned*/, const float* s_y,
+                                               int row, int rows) {
+    const float4 xa = *reinterpret_cast<const float4*>(s_x), xb = *reinterpret_cast<const float4*>(s_x + 4);
+    const float2 x[4] = {{xa.x, xa.y}, {xa.z, xa.w}, {xb.x, xb.y}, {xb.z, xb.w}};
+    unsigned cover = 0;
+#pragma unroll 1
+    for (int k = row; k < row + rows; k++) {
+        const float py = s_y[k];
+        const float c0 = fma_(m[1], py, m[2]), c1 = fma_(m[4], py, m[5]), c2 = fma_(m[7], py, m[8]);
+        unsigned bits = 0;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const float2 u = fma2({m[0], m[0]}, x[i], {c0, c0}), v = fma2({m[3], m[3]}, x[i], {c1, c1}),
+                         t = fma2({m[6], m[6]}, x[i], {c2, c2});
+            if (!(fminf(fminf(u.x, v.x), t.x) < kEffZero)) bits |= 1u << (2 * i);
+            if (!(fminf(fminf(u.y, v.y), t.y) < kEffZero)) bits |= 2u << (2 * i);
+        }
+        cover |= bits << (8 * k);
+    }
+    return cover;
+}
+
+// 32x32 bit matrix, one row per lane, transposed: bit k of lane p becomes bit p of lane k.
+__device__ __forceinline__ unsigned transpose_bits(unsigned x) {
+    const unsigned lane = lane_id();
+    unsigned m = 0x0000ffffu;
+#pragma unroll
+    for (int j = 16; j > 0; j >>= 1) {
+        const unsigned y = __shfl_xor_sync(0xffffffffu, x, j);
+        x = (lane & j) ? ((x & ~m) | ((y & ~m) >> j)) : ((x & m) | ((y & m) << j));
+        m ^= m << (j >> 1);
+    }
+    return x;
+}
+
+// One staged chunk of n <= 64 records: the warp's lanes with `go` collect the fragments that cover their pixels, in list
+// order.  first: list position of record 0, or s_j: the records' list positions.
+// The records that survive the warp's cull are tested against all 32 pixels by a lane each (two or four lanes when they
+// are few), the bits are transposed, and every pixel then visits only the records that cover it: a triangle of a pixel
+// or two costs a share of the warp's test instead of 20 instructions with one lane busy.  s_slot: 64 bytes per warp.
+// Tiles without 8x4 blocks test one record at a time with the pixels in the lanes; so does a warp (from then on: `dense`)
+// in which some pixel turned out to be covered by more than half of the records.
+// Forward kernel, B200: 1.3M triangles of a pixel, full HD 272 -> 180 us; 1280 triangles 256x256 8.4 -> 6.2; 2M
+// triangles, 4K 650 -> 617; 200k triangles, full HD 109 -> 110 (there a survivor covers a third of the lanes).
+constexpr int kFewRecords = 3;      // up to this many survivors are tested one at a time in any case
+__device__ __forceinline__ void process_chunk(const TileCtx& c, bool go, int bs, uint64_t last, Batch& s, bool& dense,
+                                              const float4* geo, int n, int first, const int* s_j, uint8_t* s_slot) {
+    // Once every collecting lane of the warp holds a full batch, a record whose depth lower bound is
+    // not below the farthest kept depth of any lane cannot enter any lane's batch (ties lose).
+    float cut = INFINITY;
+    if (__all_sync(0xffffffffu, !go || s.found == bs)) {
+        cut = go ? s.dfar : -INFINITY;
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) cut = fmaxf(cut, __shfl_xor_sync(0xffffffffu, cut, d));
+    }
+    const unsigned long long mask = warp_cull(geo, n, c.rect, cut);
+    const unsigned m0 = (unsigned)mask, m1 = (unsigned)(mask >> 32);
+    const int survivors = __popc(m0) + __popc(m1);
+    if (c.s_x == nullptr || survivors <= kFewRecords || dense) {
+        // the two 32-bit halves of the mask one after the other: bit scans on 32-bit words are cheaper
+#pragma unroll 1
+        for (int half = 0; half < 2; half++) {
+            unsigned bits = half ? m1 : m0;
+            while (bits) {
+                const int r = __ffs((int)bits) - 1 + 32 * half;
+                bits &= bits - 1;
+                // all lanes read the same record: broadcast 16-byte loads
+                const float4* rec = geo + kStagedQuads * r;
+                const float4 q0 = rec[0], q1 = rec[1], q2 = rec[2];
+                const float m[9] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w, q2.x};
+                const Bary b = apply_bary(m, c.px, c.py);
+                // one minimum instead of three comparisons: fminf skips NaN operands, so the result is below
+                // kEffZero exactly when one of the three is (and NaN, i.e. "covered", when all three are NaN)
+                if (!go || fminf(fminf(b.x, b.y), b.z) < kEffZero) continue;
+                collect(s, bs, last, b, q2, rec[3], s_j ? s_j[r] : first + r);
+            }
+        }
+        return;
+    }
+    const int lane = lane_id();
+    const unsigned below = (1u << lane) - 1u;
+    __syncwarp();                 // the slots of the chunk before have been read
+    if ((m0 >> lane) & 1u) s_slot[__popc(m0 & below)] = (uint8_t)lane;
+    if ((m1 >> lane) & 1u) s_slot[__popc(m0) + __popc(m1 & below)] = (uint8_t)(lane + 32);
+    __syncwarp();
+#pragma unroll 1
+    for (int base = 0; base < survivors; base += 32) {
+        const int count = min(32, survivors - base);
+        const int shift = count <= 8 ? 2 : count <= 16 ? 1 : 0;      // log2 of the lanes per record
+        const int k = lane & (31 >> shift), part = lane >> (5 - shift);
+        unsigned cover = 0;
+        if (k < count) {
+            const float4* rec = geo + kStagedQuads * s_slot[base + k];
+            const float4 q0 = rec[0], q1 = rec[1];
+            const float m[9] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w, rec[2].x};
+            cover = cover_rows(m, c.s_x, c.s_y, part * (4 >> shift), 4 >> shift);
+        }
+        __syncwarp();
+        if (shift >= 1) cover |= __shfl_xor_sync(0xffffffffu, cover, 16);
+        if (shift == 2) cover |= __shfl_xor_sync(0xffffffffu, cover, 8);
+        unsigned mine = transpose_bits(lane < count ? cover : 0u);
+        if (!go) mine = 0;
+        dense = 2 * __reduce_max_sync(0xffffffffu, (unsigned)__popc(mine)) > (unsigned)count;
+        while (mine) {
+            const int r = s_slot[base + __ffs((int)mine) - 1];
+            mine &= mine - 1;
+            const float4* rec = geo + kStagedQuads * r;
+            const float4 q0 = rec[0], q1 = rec[1], q2 = rec[2];
+            const float m[9] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w, q2.x};
+            collect(s, bs, last, apply_bary(m, c.px, c.py), q2, rec[3], s_j ? s_j[r] : first + r);
+        }
+        __syncwarp();
+    }
+}
+
+// Shared memory of a sweep.  `attr`, when given, receives the attribute quads of the chunk as well (stage_attr_chunk).
+// `geo2` / `id2`, when given, are a second pair of staging buffers: a list of more than one chunk is then streamed
 // (CTAs of 256 threads: one quad per thread and chunk) - the records of chunk k + 1 travel by asynchronous copies
 // while chunk k is processed, their ids having been fetched one iteration earlier still, and one barrier per chunk
 // replaces the two of the load-then-process loop.
+constexpr int kFilterBatch = 1024;
+struct SweepScratch {
+    uint16_t keep[kFilterBatch];     // entries of a filtered batch, as offsets
+    int j[kChunk];                   // list positions of a filtered chunk
+    uint32_t count[33];              // per warp and quarter of a batch
+    uint8_t slot[32][64];            // per warp, see process_chunk
+};
+struct SweepSmem {
+    float4* geo;
+    int* id;
+    SweepScratch* scratch;
+    float4* attr;
+    float4* geo2;
+    int* id2;
+};
+
+// The rest of a tile list, from `pos` on, once every collecting pixel of the CTA holds a full batch: only entries whose
+// depth lower bound is below the farthest kept depth of some pixel can still matter.  Lists are sorted by depth, so these
+// are few: 1024 entries at a time the CTA reads just that word, and stages the ones that pass, 64 at a time (2M triangles
+// piled up in the middle of a 4K image: most of a list of 5000 lies behind the 32 layers).
+__device__ __forceinline__ void sweep_filtered(const BlendParams& P, const TileCtx& c, bool go, bool warp_go, int bs, uint64_t last,
+                                            Batch& s, bool& dense, const SweepSmem& sm, int pos) {
+    const int tid = threadIdx.x, warp = tid >> 5, nt = blockDim.x, warps = nt >> 5;
+    const int per = nt <= 256 ? 4 : 1;          // per * warps <= 32 counts
+    SweepScratch& x = *sm.scratch;
+    const float* zlow = reinterpret_cast<const float*>(P.geo) + 15;
+    for (; pos < c.end; pos += per * nt) {
+        float cut = go ? s.dfar : -INFINITY;
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) cut = fmaxf(cut, __shfl_xor_sync(0xffffffffu, cut, d));
+        __syncthreads();
+        if (lane_id() == 0) x.count[warp] = __float_as_uint(cut);
+        __syncthreads();
+        cut = (int)lane_id() < warps ? __uint_as_float(x.count[lane_id()]) : -INFINITY;
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) cut = fmaxf(cut, __shfl_xor_sync(0xffffffffu, cut, d));
+        __syncthreads();
+        float z[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int j = pos + k * nt + tid;
+            z[k] = (k < per && j < c.end) ? __ldg(zlow + 16 * (size_t)P.ids[j]) : INFINITY;
+        }
+        unsigned kept[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            kept[k] = __ballot_sync(0xffffffffu, z[k] < cut);
+            if (k < per && lane_id() == 0) x.count[k * warps + warp] = (uint32_t)__popc(kept[k]);
+        }
+        __syncthreads();
+        if (warp == 0) {
+            const uint32_t mine = (int)lane_id() < per * warps ? x.count[lane_id()] : 0u;
+            uint32_t incl = mine;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, incl, d);
+                if ((int)lane_id() >= d) incl += y;
+            }
+            x.count[lane_id()] = incl - mine;
+            if (lane_id() == 31) x.count[32] = incl;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (k < per && z[k] < cut)
+                x.keep[x.count[k * warps + warp] + __popc(kept[k] & ((1u << lane_id()) - 1u))] = (uint16_t)(k * nt + tid);
+        const int total = (int)x.count[32];
+        __syncthreads();
+        for (int c0 = 0; c0 < total; c0 += kChunk) {
+            const int n = min(kChunk, total - c0);
+            for (int i = tid; i < n * 4; i += nt) {
+                const int rec = i >> 2, q = i & 3, j = pos + x.keep[c0 + rec];
+                const int id = P.ids[j];
+                if (q == 0) x.j[rec] = j;
+                sm.geo[staged_quad(rec, q)] = __ldg(P.geo + 4 * (size_t)id + q);
+            }
+            __syncthreads();
+            if (warp_go) process_chunk(c, go, bs, last, s, dense, sm.geo, n, 0, x.j, x.slot[warp]);
+            __syncthreads();
+        }
+    }
+}
+
+// One selection sweep over the whole tile list (select_next_k_in_tile, reference render.cu:375-415):
+// keeps the `bs` covered fragments smallest in (depth, j) among those behind `last` (a word of a batch, 0 for the first).
+// All threads of the CTA must call it; `go` says whether this thread collects.
 // (STREAM is a template parameter so that callers which never stream carry none of its state.)
-template <bool STREAM = false>
-__device__ __forceinline__ int select_sweep(const BlendParams& P, const TileCtx& c, bool go, int bs, float lastDepth,
-                                            int lastJ, float* dl, int* jl, float4* s_geo, int* s_id,
-                                            float4* s_attr = nullptr, float4* s_geo2 = nullptr, int* s_id2 = nullptr) {
-    int found = 0;
-    float dfar = -INFINITY;     // dl[found - 1]; -inf while the batch is empty, so the first fragment is appended
+template <bool STREAM = false, bool FILTER = true>
+__device__ __forceinline__ void select_sweep(const BlendParams& P, const TileCtx& c, bool go, int bs, uint64_t last,
+                                             Batch& s, const SweepSmem& sm) {
+    s.found = 0;
+    s.dfar = -INFINITY;
+    bool dense = false;         // see process_chunk
     const bool warp_go = __any_sync(0xffffffffu, go);
-    const bool streamed = STREAM && s_geo2 != nullptr && c.end - c.start > kChunk && blockDim.x == 4 * kChunk;
+    uint8_t* s_slot = sm.scratch->slot[threadIdx.x >> 5];
+    const bool streamed = STREAM && sm.geo2 != nullptr && c.end - c.start > kChunk && blockDim.x == 4 * kChunk;
     const int my_rec = threadIdx.x >> 2, my_q = threadIdx.x & 3;
     int id_ahead = -1;          // streamed: id of this thread's record in the chunk after the one being copied
     if (streamed) {
         __syncthreads();        // whoever read the buffers before (an earlier sweep) is done
         const int id = P.ids[c.start + my_rec];                       // chunk 0 is full: the list is longer
-        if (my_q == 0) s_id[my_rec] = id;
-        cp_async16(s_geo + staged_quad(my_rec, my_q), P.geo + 4 * (size_t)id + my_q);
+        if (my_q == 0) sm.id[my_rec] = id;
+        cp_async16(sm.geo + staged_quad(my_rec, my_q), P.geo + 4 * (size_t)id + my_q);
         cp_async_commit();
         if (my_rec < c.end - c.start - kChunk) id_ahead = P.ids[c.start + kChunk + my_rec];
     }
     int chunk = 0;
     for (int first = c.start; first < c.end; first += kChunk, chunk++) {
         const int n = min(kChunk, c.end - first);
-        const float4* geo_now = s_geo;          // the staged records of this chunk
+        const float4* geo_now = sm.geo;         // the staged records of this chunk
+        const bool full = !go || s.found == bs;
         if (streamed) {
-            float4* other_geo = s_geo2;         // buffers the next chunk is copied into
-            int* other_id = s_id2;
-            if (chunk & 1) { geo_now = s_geo2; other_geo = s_geo; other_id = s_id; }
+            float4* other_geo = sm.geo2;        // buffers the next chunk is copied into
+            int* other_id = sm.id2;
+            if (chunk & 1) { geo_now = sm.geo2; other_geo = sm.geo; other_id = sm.id; }
             cp_async_wait_all();
-            __syncthreads();    // this chunk has landed for everyone, and everyone has left the chunk before
+            // this chunk has landed for everyone, and everyone has left the chunk before
+            if (__syncthreads_and(full) && c.end - first > kChunk) {
+                sweep_filtered(P, c, go, warp_go, bs, last, s, dense, sm, first);
+                break;
+            }
             if (first + kChunk < c.end) {
                 if (id_ahead >= 0) {
                     if (my_q == 0) other_id[my_rec] = id_ahead;
@@ -308,63 +562,18 @@ __device__ __forceinline__ int select_sweep(const BlendParams& P, const TileCtx&
                 id_ahead = (first2 < c.end && my_rec < c.end - first2) ? P.ids[first2 + my_rec] : -1;
             }
         } else {
-            __syncthreads();
-            stage_chunk(P, first, n, s_geo, s_id);
-            if (s_attr) stage_attr_chunk(P, first, n, s_attr);
-            __syncthreads();
-        }
-        if (!warp_go) continue;
-        // Once every collecting lane of the warp holds a full batch, a record whose depth lower bound is
-        // not below the farthest kept depth of any lane cannot enter any lane's batch (ties lose).
-        float cut = go ? ((found == bs) ? dfar : INFINITY) : -INFINITY;
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) cut = fmaxf(cut, __shfl_xor_sync(0xffffffffu, cut, d));
-        const unsigned long long mask = warp_cull(geo_now, n, c.rect, cut);
-        // the two 32-bit halves of the mask one after the other: bit scans on 32-bit words are cheaper than on the
-        // 64-bit one, and this loop runs once per surviving record and warp
-#pragma unroll 1
-        for (int half = 0; half < 2; half++) {
-            unsigned bits = half ? (unsigned)(mask >> 32) : (unsigned)mask;
-            while (bits) {
-                const int r = __ffs((int)bits) - 1 + 32 * half;
-                bits &= bits - 1;
-                // all lanes read the same record: broadcast 16-byte loads
-                const float4* rec = geo_now + kStagedQuads * r;
-                const float4 q0 = rec[0], q1 = rec[1], q2 = rec[2];
-                const float m[9] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w, q2.x};
-                const Bary b = apply_bary(m, c.px, c.py);
-                // one minimum instead of three comparisons: fminf skips NaN operands, so the result is below
-                // kEffZero exactly when one of the three is (and NaN, i.e. "covered", when all three are NaN)
-                if (!go || fminf(fminf(b.x, b.y), b.z) < kEffZero) continue;
-                const float4 q3 = rec[3];
-                const float d = interp_rn(b, q2.y, q2.z, q2.w, q3.x, q3.y, q3.z);
-                const int j = first + r;
-                if (d < lastDepth) continue;
-                if (d == lastDepth && j <= lastJ) continue;
-                // the farthest kept depth stays in a register: lists come roughly front to back, so most
-                // fragments go to the end of the batch (ties keep list order) or, once it is full, nowhere
-                if (d >= dfar) {
-                    if (found == bs) continue;
-                    dl[found] = d;
-                    jl[found] = j;
-                    dfar = d;
-                    found++;
-                    continue;
-                }
-                int pos = (found < bs) ? found : (bs - 1);
-                while (pos > 0 && d < dl[pos - 1]) {
-                    dl[pos] = dl[pos - 1];
-                    jl[pos] = jl[pos - 1];
-                    pos--;
-                }
-                dl[pos] = d;
-                jl[pos] = j;
-                if (found < bs) found++;
-                dfar = dl[found - 1];
+            if (!FILTER) {
+                __syncthreads();
+            } else if (__syncthreads_and(full) && c.end - first > kChunk) {
+                sweep_filtered(P, c, go, warp_go, bs, last, s, dense, sm, first);
+                break;
             }
+            stage_chunk(P, first, n, sm.geo, sm.id);
+            if (sm.attr) stage_attr_chunk(P, first, n, sm.attr);
+            __syncthreads();
         }
+        if (warp_go) process_chunk(c, go, bs, last, s, dense, geo_now, n, first, nullptr, s_slot);
     }
-    return found;
 }
 
 __device__ __forceinline__ void store_pixel(const TileCtx& c, const BlendParams& P, PixelAcc& acc, float4* image,
@@ -385,14 +594,15 @@ __device__ __forceinline__ void store_pixel(const TileCtx& c, const BlendParams&
 // STREAM: lists of more than one chunk are streamed through two staging buffers (select_sweep); instantiated
 // separately because the state it carries costs the one-chunk tiles a few spilled registers.
 template <bool SORT, int MAXT, bool STREAM = false>
-__global__ void __launch_bounds__(MAXT, MAXT <= 256 ? 5 : 1) blend_forward_kernel(BlendParams P, float4* __restrict__ image,
+__global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (SORT ? 4 : 5) : 1) blend_forward_kernel(BlendParams P, float4* __restrict__ image,
                                                              float* __restrict__ depthmap, float* __restrict__ final_w,
                                                              int* __restrict__ ends, int* __restrict__ sel) {
     __shared__ float4 s_geo[kChunk * kStagedQuads];
     __shared__ float4 s_attr[SORT ? kChunk * kStagedQuads : 1];   // one-chunk lists: attributes; longer ones: 2nd buffer
     __shared__ int s_id[kChunk];
     __shared__ int s_id2[STREAM ? kChunk : 1];
-    __shared__ float s_coord[kMaxTileCoords];
+    __shared__ __align__(16) float s_coord[kMaxTileCoords];
+    __shared__ SweepScratch s_scratch;
     const int this_tile = tile_of_block(P);
     if (P.offsets[this_tile] == P.offsets[this_tile + 1]) {
         // a tile without entries: background, and no need for pixel-centre coordinates (any pixel order will do)
@@ -411,10 +621,8 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? 5 : 1) blend_forward_kerne
     PixelAcc acc;
 
     if (SORT) {
-        float dl[kBatchLayers];
-        int jl[kBatchLayers];
-        float lastDepth = -INFINITY;
-        int lastJ = -1;
+        Batch batch;
+        uint64_t last = 0;
         bool want = c.active;
         const size_t plane = (size_t)P.W * P.H, index = (size_t)c.iy * P.W + c.ix;
         while (true) {
@@ -427,13 +635,14 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? 5 : 1) blend_forward_kerne
             // number of pixels that found something, whether staging the attributes pays was slower: the loads then
             // wait alone behind a barrier.)
             const bool one_chunk = c.end - c.start <= kChunk;
-            const int found = select_sweep<STREAM>(P, c, go, bs, lastDepth, lastJ, dl, jl, s_geo, s_id,
-                                                   one_chunk ? s_attr : nullptr, one_chunk ? nullptr : s_attr, s_id2);
+            select_sweep<STREAM, (STREAM || MAXT > 256)>(P, c, go, bs, last, batch,
+                                 {s_geo, s_id, &s_scratch, one_chunk ? s_attr : nullptr, one_chunk ? nullptr : s_attr, s_id2});
+            const int found = batch.found;
             if (go) {
                 const int n = min(found, P.max_layers - acc.blended);
                 for (int i = 0; i < n; i++) {
                     if (one_chunk) {
-                        const int r = jl[i] - c.start;
+                        const int r = (int)(uint32_t)batch.key[i] - c.start;
                         const StagedGeo g = load_staged(s_geo, r);
                         const Bary b = apply_bary(g.m, c.px, c.py);
                         const AttrRec a = staged_attr(s_attr, r);
@@ -441,7 +650,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? 5 : 1) blend_forward_kerne
                         blend_one(b, g.w, a, acc);
                         continue;
                     }
-                    const int id = P.ids[jl[i]];
+                    const int id = P.ids[(uint32_t)batch.key[i]];
                     float m[9], w[3];
                     load_geo(P.geo, id, m, w);
                     const Bary b = apply_bary(m, c.px, c.py);
@@ -450,8 +659,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? 5 : 1) blend_forward_kerne
                     blend_one(b, w, a, acc);
                 }
                 if (n > 0) {
-                    lastDepth = dl[n - 1];
-                    lastJ = jl[n - 1];
+                    last = batch.key[n - 1];
                 }
                 // fewer than a full batch found: the sweep saw every remaining fragment, nothing is left
                 if (found < bs) want = false;
@@ -923,7 +1131,7 @@ __global__ void __launch_bounds__(MAXT, DEPTH ? 7 : 8) blend_backward_queued_ker
                                                                         const int* __restrict__ sel,
                                                                         float4* __restrict__ gpack) {
     static_assert(MAXT % 32 == 0 && MAXT <= 256, "one queue per warp, at most 8 warps");
-    __shared__ float s_coord[MAXT + 2];      // tile_w + tile_h <= tile_w * tile_h + 1 <= MAXT + 1
+    __shared__ __align__(16) float s_coord[MAXT + 2];      // tile_w + tile_h <= tile_w * tile_h + 1 <= MAXT + 1
     __shared__ float4 s_queue[MAXT / 32][kQueueQuads];
     const TileCtx c = tile_context(P, s_coord);
     PixelGrad pg;
@@ -991,7 +1199,8 @@ __global__ void __launch_bounds__(MAXT, 4) blend_step_l2_kernel(BlendParams P, f
     static_assert(MAXT == 256, "the per-warp queues are sized for 8 warps");
     __shared__ float4 s_geo[kChunk * kStagedQuads];
     __shared__ int s_id[kChunk];
-    __shared__ float s_coord[kMaxTileCoords];
+    __shared__ __align__(16) float s_coord[kMaxTileCoords];
+    __shared__ SweepScratch s_scratch;
     extern __shared__ float4 s_step[];       // queues of the warps
     const TileCtx c = tile_context(P, s_coord);
     const int lane = lane_id();
@@ -999,16 +1208,15 @@ __global__ void __launch_bounds__(MAXT, 4) blend_step_l2_kernel(BlendParams P, f
     float4 kept[kBatchLayers][3];   // per blended fragment: (b.x, b.y, b.z, o_raw), (cr, cg, cb, z), (1/den, 1/denz, id, -)
     int n = 0;
     {
-        float dl[kBatchLayers];
-        int jl[kBatchLayers];
+        Batch batch;
         const bool go = c.active && acc.alpha > P.thr && P.max_layers > 0;
         if (__syncthreads_or(go)) {
             const int bs = min(kBatchLayers, P.max_layers);
-            const int found = select_sweep(P, c, go, bs, -INFINITY, -1, dl, jl, s_geo, s_id);
+            select_sweep(P, c, go, bs, 0, batch, {s_geo, s_id, &s_scratch, nullptr, nullptr, nullptr});
             if (go) {
-                n = min(found, P.max_layers);
+                n = min(batch.found, P.max_layers);
                 for (int i = 0; i < n; i++) {
-                    const int id = P.ids[jl[i]];
+                    const int id = P.ids[(uint32_t)batch.key[i]];
                     float m[9], w[3];
                     load_geo(P.geo, id, m, w);
                     const Bary b = apply_bary(m, c.px, c.py);
@@ -1073,27 +1281,26 @@ __global__ void __launch_bounds__(MAXT, 4) blend_step_l2_kernel(BlendParams P, f
 
 // General path (any max_layers, both modes): searches the list again as the reference does.
 template <bool SORT, int MAXT>
-__global__ void __launch_bounds__(MAXT) blend_backward_kernel(BlendParams P, BackwardIn in, float4* __restrict__ gpack) {
+__global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (SORT ? 3 : 4) : 1) blend_backward_kernel(BlendParams P, BackwardIn in, float4* __restrict__ gpack) {
     __shared__ float4 s_geo[kChunk * kStagedQuads];
     __shared__ int s_id[kChunk];
-    __shared__ float s_coord[kMaxTileCoords];
+    __shared__ __align__(16) float s_coord[kMaxTileCoords];
     const TileCtx c = tile_context(P, s_coord);
     PixelGrad pg;
     BackState st;
     const int limit = load_pixel_state(c, P, in, pg, st);
 
     if (SORT) {
-        float dl[kBatchLayers];
-        int jl[kBatchLayers];
-        float lastDepth = -INFINITY;
-        int lastJ = -1;
+        __shared__ SweepScratch s_scratch;
+        Batch batch;
+        uint64_t last = 0;
         int remaining = limit;
         while (true) {
             const bool go = remaining > 0;
             if (!__syncthreads_or(go)) break;
             const int bs = min(kBatchLayers, remaining);
-            const int found = select_sweep(P, c, go, bs, lastDepth, lastJ, dl, jl, s_geo, s_id);
-            const int n = go ? min(found, remaining) : 0;
+            select_sweep(P, c, go, bs, last, batch, {s_geo, s_id, &s_scratch, nullptr, nullptr, nullptr});
+            const int n = go ? min(batch.found, remaining) : 0;
             const int rounds = __reduce_max_sync(0xffffffffu, n);
             // back to front inside the batch (reference render.cu:684-688); the first of the rounds starts at every lane's
             // last fragment
@@ -1102,7 +1309,7 @@ __global__ void __launch_bounds__(MAXT) blend_backward_kernel(BlendParams P, Bac
                 int id = -1;
                 Contrib ct = {};
                 if (i >= 0) {
-                    id = P.ids[jl[i]];
+                    id = P.ids[(uint32_t)batch.key[i]];
                     float m[9], w[3];
                     load_geo(P.geo, id, m, w);
                     const Bary b = apply_bary(m, c.px, c.py);
@@ -1113,8 +1320,7 @@ __global__ void __launch_bounds__(MAXT) blend_backward_kernel(BlendParams P, Bac
             }
             if (go) {
                 if (n > 0) {
-                    lastDepth = dl[n - 1];
-                    lastJ = jl[n - 1];
+                    last = batch.key[n - 1];
                     remaining -= n;
                 } else {
                     remaining = 0;
@@ -1211,11 +1417,11 @@ __device__ __forceinline__ void backward_one_prefix(const float* w, const AttrRe
 }
 
 template <bool SORT, int MAXT>
-__global__ void __launch_bounds__(MAXT) blend_backward_corrected_kernel(BlendParams P, BackwardIn in,
+__global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (SORT ? 3 : 4) : 1) blend_backward_corrected_kernel(BlendParams P, BackwardIn in,
                                                                         float4* __restrict__ gpack) {
     __shared__ float4 s_geo[kChunk * kStagedQuads];
     __shared__ int s_id[kChunk];
-    __shared__ float s_coord[kMaxTileCoords];
+    __shared__ __align__(16) float s_coord[kMaxTileCoords];
     const TileCtx c = tile_context(P, s_coord);
     PixelGrad pg;
     BackState unused;
@@ -1229,23 +1435,22 @@ __global__ void __launch_bounds__(MAXT) blend_backward_corrected_kernel(BlendPar
     PrefixState pf;
 
     if (SORT) {
-        float dl[kBatchLayers];
-        int jl[kBatchLayers];
-        float lastDepth = -INFINITY;
-        int lastJ = -1;
+        __shared__ SweepScratch s_scratch;
+        Batch batch;
+        uint64_t last = 0;
         int remaining = limit;
         while (true) {
             const bool go = remaining > 0;
             if (!__syncthreads_or(go)) break;
             const int bs = min(kBatchLayers, remaining);
-            const int found = select_sweep(P, c, go, bs, lastDepth, lastJ, dl, jl, s_geo, s_id);
-            const int n = go ? min(found, remaining) : 0;
+            select_sweep(P, c, go, bs, last, batch, {s_geo, s_id, &s_scratch, nullptr, nullptr, nullptr});
+            const int n = go ? min(batch.found, remaining) : 0;
             const int rounds = __reduce_max_sync(0xffffffffu, n);
             for (int i = 0; i < rounds; ++i) {
                 int id = -1;
                 Contrib ct = {};
                 if (i < n) {
-                    id = P.ids[jl[i]];
+                    id = P.ids[(uint32_t)batch.key[i]];
                     float m[9], w[3];
                     load_geo(P.geo, id, m, w);
                     const Bary b = apply_bary(m, c.px, c.py);
@@ -1256,8 +1461,7 @@ __global__ void __launch_bounds__(MAXT) blend_backward_corrected_kernel(BlendPar
             }
             if (go) {
                 if (n > 0) {
-                    lastDepth = dl[n - 1];
-                    lastJ = jl[n - 1];
+                    last = batch.key[n - 1];
                     remaining -= n;
                 } else {
                     remaining = 0;
