@@ -15,7 +15,7 @@ inline size_t align_up(size_t x, size_t a = 256) { return (x + a - 1) / a * a; }
 // Carves the caller's workspace; the same function sizes it.
 struct ForwardWorkspace {
     tg_host::BinBuffers bin = {};
-    uint32_t* long_list;       // work lists of the per-tile sort; only their six head words need clearing
+    uint32_t* long_list;       // work lists of the per-tile sort
     size_t total;
 
     ForwardWorkspace(void* base, int tiles, uint32_t cap) {
@@ -26,20 +26,22 @@ struct ForwardWorkspace {
             return p;
         };
         const bool device_scan = tiles > tg::kTileScanByLastCta;
-        bin.entries = (uint64_t*)take(sizeof(uint64_t) * (size_t)cap);
-        bin.pairs = (uint4*)take(sizeof(uint4) * (size_t)cap);
+        // what outlives a call (TG_WORKSPACE_READY) lies first, at places that do not depend on the list capacity
         bin.tables = (float4*)take(sizeof(float4) * ((size_t)tiles + 1));     // tiles_x + tiles_y <= tiles + 1
-        bin.info = (uint32_t*)take(sizeof(uint32_t) * 3);
-        // everything from `status` up to the head of the work lists must be zero when the kernels start: one clear
+        // everything from `status` up to the end of the tile counts must be zero when the kernels start
         bin.status = (uint32_t*)take(sizeof(uint32_t) * 4);
         bin.counters = (uint32_t*)take(sizeof(uint32_t) * 2);
         bin.tile_scan_scratch = take(device_scan ? tg_scan_scratch_bytes(tiles) : 0);
         bin.tile_counts = (uint32_t*)take(sizeof(uint32_t) * (size_t)tiles);
-        long_list = (uint32_t*)take(tg_host::tile_sort_scratch_bytes(tiles));
         bin.clear = bin.status;
-        bin.clear_words = base ? (size_t)(long_list + 6 - bin.clear) : 0;
+        bin.clear_words = base ? (size_t)(bin.tile_counts + tiles - bin.clear) : 0;
+        bin.info = (uint32_t*)take(sizeof(uint32_t) * 3);
+        long_list = (uint32_t*)take(tg_host::tile_sort_scratch_bytes(tiles));
+        bin.list_heads = long_list;
         bin.tile_order = (uint32_t*)take(sizeof(uint32_t) * (size_t)tiles);
         if (device_scan) bin.tile_order = nullptr;
+        bin.entries = (uint64_t*)take(sizeof(uint64_t) * (size_t)cap);
+        bin.pairs = (uint4*)take(sizeof(uint4) * (size_t)cap);
         total = off;
     }
 };
@@ -73,67 +75,60 @@ struct StageTimer {
 
 }  // namespace
 
-// Everything before compositing: per-triangle records, tile offsets, sorted tile lists (timer marks 0-3).
-static int build_tile_lists(const float* vertices, const int32_t* indices, const float* colors, const float* opacities,
-                            int T, int W, int H, int tw, int th, int max_layers, float* tri_geo, float* tri_attr,
-                            int32_t* sorted_ids, uint32_t list_capacity, int32_t* offsets, void* workspace,
-                            size_t workspace_bytes, uint32_t* info_host, unsigned flags, StageTimer& timer,
-                            uint32_t** device_status, const uint32_t** tile_order_out, cudaStream_t s) {
-    TG_REQUIRE(T >= 0 && W > 0 && H > 0 && tw > 0 && th > 0, "sizes");
-    TG_REQUIRE(tw * th <= 1024, "tile_width * tile_height must be <= 1024");
-    TG_REQUIRE(max_layers >= 1, "max_layers must be >= 1");
-    TG_REQUIRE(workspace && info_host && offsets, "null pointer");
-    TG_REQUIRE(((uintptr_t)workspace & 255) == 0, "workspace must be 256-byte aligned");
-    TG_REQUIRE(list_capacity < 0x80000000u, "list capacity must stay below 2^31");
-    const int tiles_x = (W + tw - 1) / tw, tiles_y = (H + th - 1) / th;
-    const int tiles = tiles_x * tiles_y;
-    TG_REQUIRE((flags & ~(unsigned)(TG_FORWARD_CULL_TILES | TG_INPUT_PACKED | TG_INFO_MAPPED)) == 0, "unknown flag");
-    const bool packed = (flags & TG_INPUT_PACKED) != 0;
-    const bool device_scan = tiles > tg::kTileScanByLastCta;
-    // beyond 65536 tiles the lists are the reference's
-    const bool cull = (flags & TG_FORWARD_CULL_TILES) != 0 && !device_scan;
-    const ForwardWorkspace ws(workspace, tiles, list_capacity);
-    // the only kernel of this path that can raise the error word is the scan
-    *device_status = device_scan ? ws.bin.status : nullptr;
-    *tile_order_out = nullptr;
-    if (workspace_bytes < ws.total) {
-        tg_host::set_error("forward workspace: need %zu bytes, got %zu", ws.total, workspace_bytes);
-        return TG_ERR_WORKSPACE;
-    }
-    info_host[0] = kNotArrived;     // K < 2^31, so this value means "K has not landed yet"
-    info_host[1] = 0;
-    info_host[2] = 0;
-    info_host[3] = 0;
-    TG_REQUIRE(list_capacity == 0 || sorted_ids != nullptr, "null sorted_ids");
-    // mapped: the binning kernel writes K where the host looks; otherwise a copy brings it
-    const bool mapped = (flags & TG_INFO_MAPPED) != 0 && T > 0;
+// Tile lists of a call, in two steps: start() launches everything up to the unsorted lists, wait() waits for K and checks
+// it against the capacity (timer marks 0-2 and 3).
+struct TileLists {
+    ForwardWorkspace ws;
+    int tiles;
+    bool device_scan, mapped;
     cudaEvent_t k_ready = nullptr;
-    if (!mapped)
-        if (int st = scratch_event(&k_ready)) return st;
+    uint32_t* device_status;               // error word, null where no kernel of the path can raise it
+    uint32_t K = 0, longest = 0;
+    const uint32_t* order = nullptr;       // launch order of the compositing kernel, when one was written
 
-    timer.mark();                                                    // [0] start of "init"
-    timer.mark();                                                    // [1] start of "bary_transforms"
-    // per-triangle records, (triangle, tile) pairs with their depth keys, tile offsets
-    int st = tg_host::bin_triangles(vertices, indices, colors, opacities, T, W, H, tw, th, tri_geo, tri_attr, ws.bin,
-                                    offsets, list_capacity, mapped ? info_host : nullptr, cull, packed, s);
-    if (st) return st;
-    timer.mark();                                                    // [2] start of "per_tile_lists"
-    if (!mapped) {
-        // [3] first: the host watches the word K arrives in
-        TG_CUDA(cudaMemcpyAsync(&info_host[3], ws.bin.info + 2, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-        TG_CUDA(cudaMemcpyAsync(&info_host[0], ws.bin.info, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-        TG_CUDA(cudaEventRecord(k_ready, s));
+    TileLists(void* workspace, int T, int W, int H, int tw, int th, uint32_t cap, unsigned flags)
+        : ws(workspace, ((W + tw - 1) / tw) * ((H + th - 1) / th), cap), tiles(((W + tw - 1) / tw) * ((H + th - 1) / th)),
+          device_scan(tiles > tg::kTileScanByLastCta), mapped((flags & TG_INFO_MAPPED) != 0 && T > 0),
+          device_status(device_scan ? ws.bin.status : nullptr) {}       // only the scan waits
+
+    int start(const float* vertices, const int32_t* indices, const float* colors, const float* opacities, int T, int W, int H,
+              int tw, int th, float* tri_geo, float* tri_attr, int32_t* sorted_ids, uint32_t cap, int32_t* offsets,
+              size_t workspace_bytes, uint32_t* info_host, unsigned flags, StageTimer& timer, cudaStream_t s) {
+        if (workspace_bytes < ws.total) {
+            tg_host::set_error("forward workspace: need %zu bytes, got %zu", ws.total, workspace_bytes);
+            return TG_ERR_WORKSPACE;
+        }
+        TG_REQUIRE(cap == 0 || sorted_ids != nullptr, "null sorted_ids");
+        info_host[0] = kNotArrived;     // K < 2^31, so this value means "K has not landed yet"
+        info_host[1] = info_host[2] = info_host[3] = 0;
+        if (!mapped)
+            if (int st = scratch_event(&k_ready)) return st;
+        // beyond 65536 tiles the lists are the reference's
+        const bool cull = (flags & TG_FORWARD_CULL_TILES) != 0 && !device_scan;
+        timer.mark();                                                    // [0] start of "init"
+        timer.mark();                                                    // [1] start of "bary_transforms"
+        // per-triangle records, (triangle, tile) pairs with their depth keys, tile offsets
+        if (int st = tg_host::bin_triangles(vertices, indices, colors, opacities, T, W, H, tw, th, tri_geo, tri_attr, ws.bin,
+                                            offsets, cap, mapped ? info_host : nullptr, cull, (flags & TG_INPUT_PACKED) != 0,
+                                            (flags & TG_WORKSPACE_READY) != 0, s))
+            return st;
+        timer.mark();                                                    // [2] start of "per_tile_lists"
+        if (!mapped) {
+            // [3] first: the host watches the word K arrives in
+            TG_CUDA(cudaMemcpyAsync(&info_host[3], ws.bin.info + 2, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+            TG_CUDA(cudaMemcpyAsync(&info_host[0], ws.bin.info, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+            TG_CUDA(cudaEventRecord(k_ready, s));
+        }
+        // The entries move to their tiles while K travels to the host: the kernel does nothing when K exceeds the capacity.
+        return tg_host::scatter_entries(ws.bin, cap, offsets, tiles, T, s);
     }
-    // The entries move to their tiles while K travels to the host: the kernel does nothing when K exceeds the capacity,
-    // and nothing that reads them is launched before K has been checked.
-    st = tg_host::scatter_entries(ws.bin, list_capacity, offsets, tiles, T, s);
-    if (st) return st;
-    // K arrives in (preferably pinned) host memory.  Watching the word itself is quicker than
-    // waking up from cudaEventSynchronize (the compositing kernels cannot be launched before K is known, so every
-    // microsecond here is an idle GPU once the entry writer has finished); after a bounded while, or for pageable
-    // memory where the copy has completed by now anyway, the event (the stream, without a copy) is waited for in the ordinary way, which also
+
+    // K arrives in (preferably pinned) host memory.  Watching the word itself is quicker than waking up from
+    // cudaEventSynchronize (unless the lists were expected to be short the compositing kernel cannot be launched before K
+    // is known, so every microsecond here is an idle GPU); after a bounded while, or for pageable memory where the copy has
+    // completed by now anyway, the event (the stream, without a copy) is waited for in the ordinary way, which also
     // surfaces any error of the kernels before it.
-    {
+    int wait(uint32_t cap, uint32_t* info_host, cudaStream_t s) {
         const volatile uint32_t* watched = info_host;
         const auto t0 = std::chrono::steady_clock::now();
         for (uint32_t spins = 1; *watched == kNotArrived; ++spins) {
@@ -147,27 +142,41 @@ static int build_tile_lists(const float* vertices, const int32_t* indices, const
         }
         std::atomic_thread_fence(std::memory_order_acquire);
         if (info_host[0] == kNotArrived) TG_CUDA(mapped ? cudaStreamSynchronize(s) : cudaEventSynchronize(k_ready));
+        if (info_host[0] == kNotArrived) {
+            tg_host::set_error("the number of list entries never reached the host");
+            return TG_ERR_CUDA;
+        }
+        K = info_host[0];
+        // the longest-list word carries "a launch order of the tiles was written" in its top bit
+        const bool have_order = (info_host[1] & tg::kOrderWrittenBit) != 0 && info_host[1] != UINT32_MAX;
+        if (info_host[1] != UINT32_MAX) info_host[1] &= ~tg::kOrderWrittenBit;
+        longest = info_host[1];
+        if (have_order) order = ws.bin.tile_order;
+        const uint32_t slots = info_host[3];            // K and the holes of culled pairs
+        if (K > cap || slots > cap) {
+            info_host[0] = K > slots ? K : slots;
+            tg_host::set_error("%u entries and culled pairs exceed the list capacity %u", info_host[0], cap);
+            return TG_ERR_CAPACITY;
+        }
+        return TG_OK;
     }
-    if (info_host[0] == kNotArrived) {
-        tg_host::set_error("the number of list entries never reached the host");
-        return TG_ERR_CUDA;
+
+    int sort(int32_t* sorted_ids, const int32_t* offsets, cudaStream_t s) {
+        if (K == 0) return TG_OK;
+        return tg_host::sort_tile_lists(ws.bin.entries, offsets, tiles, sorted_ids, ws.long_list, true, false, longest, s);
     }
-    const uint32_t K = info_host[0];
-    // the longest-list word carries "a launch order of the tiles was written" in its top bit
-    const bool have_order = (info_host[1] & tg::kOrderWrittenBit) != 0 && info_host[1] != UINT32_MAX;
-    if (info_host[1] != UINT32_MAX) info_host[1] &= ~tg::kOrderWrittenBit;
-    *tile_order_out = have_order ? ws.bin.tile_order : nullptr;
-    const uint32_t slots = info_host[3];            // K and the holes of culled pairs
-    if (K > list_capacity || slots > list_capacity) {
-        info_host[0] = K > slots ? K : slots;
-        tg_host::set_error("%u entries and culled pairs exceed the list capacity %u", info_host[0], list_capacity);
-        return TG_ERR_CAPACITY;
-    }
-    timer.mark();                                                    // [3] start of "sorting"
-    if (K > 0) {
-        st = tg_host::sort_tile_lists(ws.bin.entries, offsets, tiles, sorted_ids, ws.long_list, true, false, info_host[1], s);
-        if (st) return st;
-    }
+};
+
+static int check_forward_args(int T, int W, int H, int tw, int th, int max_layers, const void* workspace,
+                              const void* info_host, const void* offsets, uint32_t list_capacity, unsigned flags) {
+    TG_REQUIRE(T >= 0 && W > 0 && H > 0 && tw > 0 && th > 0, "sizes");
+    TG_REQUIRE(tw * th <= 1024, "tile_width * tile_height must be <= 1024");
+    TG_REQUIRE(max_layers >= 1, "max_layers must be >= 1");
+    TG_REQUIRE(workspace && info_host && offsets, "null pointer");
+    TG_REQUIRE(((uintptr_t)workspace & 255) == 0, "workspace must be 256-byte aligned");
+    TG_REQUIRE(list_capacity < 0x80000000u, "list capacity must stay below 2^31");
+    TG_REQUIRE((flags & ~31u) == 0, "unknown flag");
+    TG_REQUIRE(!(flags & TG_EXPECT_SHORT_LISTS) || (flags & TG_INFO_MAPPED), "TG_EXPECT_SHORT_LISTS needs TG_INFO_MAPPED");
     return TG_OK;
 }
 
@@ -206,20 +215,41 @@ int tg_render_forward(const float* vertices, const int32_t* indices, const float
     TG_REQUIRE(image && depthmap && final_weights && ends, "null pointer");
     cudaStream_t s = (cudaStream_t)stream;
     StageTimer timer(stage_ms_host != nullptr, s);
-    uint32_t* device_status = nullptr;
-    const uint32_t* tile_order = nullptr;
-    int st = build_tile_lists(vertices, indices, colors, opacities, T, W, H, tw, th, max_layers, tri_geo, tri_attr,
-                              sorted_ids, list_capacity, offsets, workspace, workspace_bytes, info_host, flags, timer, &device_status, &tile_order, s);
-    if (st) return st;
-    timer.mark();                                                    // [4] start of "rasterization"
-    tg_host::set_tile_order(tile_order, info_host[1]);      // with the longest list: long lists are streamed
-    st = tg_blend_forward(tri_geo, tri_attr, sorted_ids, offsets, W, H, tw, th, thr, per_pixel_sort, max_layers, image,
-                          depthmap, final_weights, ends, selection, stream);
-    tg_host::set_tile_order(nullptr);
+    if (int st = check_forward_args(T, W, H, tw, th, max_layers, workspace, info_host, offsets, list_capacity, flags)) return st;
+    TileLists lists(workspace, T, W, H, tw, th, list_capacity, flags);
+    if (int st = lists.start(vertices, indices, colors, opacities, T, W, H, tw, th, tri_geo, tri_attr, sorted_ids, list_capacity,
+                             offsets, workspace_bytes, info_host, flags, timer, s))
+        return st;
+    // Lists of up to kFusedList entries are sorted by the compositing kernel itself in images of few tiles.  Where the
+    // caller expects nothing longer it is launched right away, and checks on the device what the host is told afterwards.
+    auto composite_short = [&]() {
+        return tg_host::blend_forward_short(tri_geo, tri_attr, lists.ws.bin.entries, lists.ws.bin.info, list_capacity, sorted_ids,
+                                            offsets, W, H, tw, th, thr, per_pixel_sort, max_layers, image, depthmap,
+                                            final_weights, ends, selection, s);
+    };
+    const bool can = lists.tiles <= tg::kFusedTiles && T > 0;
+    const bool early = can && (flags & TG_EXPECT_SHORT_LISTS) != 0 && stage_ms_host == nullptr;
+    if (early)
+        if (int st = composite_short()) return st;
+    if (int st = lists.wait(list_capacity, info_host, s)) return st;
+    timer.mark();                                                    // [3] start of "sorting"
+    int st = TG_OK;
+    if (can && lists.longest <= tg::kFusedList) {
+        timer.mark();                                                // [4] start of "rasterization"
+        if (!early) st = composite_short();
+    } else {
+        if ((st = lists.sort(sorted_ids, offsets, s))) return st;
+        timer.mark();                                                // [4]
+        tg_host::set_tile_order(lists.order, lists.longest);         // with the longest list: long lists are streamed
+        st = tg_blend_forward(tri_geo, tri_attr, sorted_ids, offsets, W, H, tw, th, thr, per_pixel_sort, max_layers, image,
+                              depthmap, final_weights, ends, selection, stream);
+        tg_host::set_tile_order(nullptr);
+    }
     if (st) return st;
     timer.mark();                                                    // [5] end
     // device error word: valid on the host once the stream has been synchronised
-    if (device_status) TG_CUDA(cudaMemcpyAsync(&info_host[2], device_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    if (lists.device_status)
+        TG_CUDA(cudaMemcpyAsync(&info_host[2], lists.device_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
     return finish_timing(timer, stage_ms_host, info_host, s);
 }
 
@@ -235,20 +265,24 @@ int tg_render_step_l2(const float* vertices, const int32_t* indices, const float
     TG_REQUIRE(tw * th <= 256 && max_layers <= 32, "the one-kernel step needs tiles of at most 256 pixels and max_layers <= 32");
     cudaStream_t s = (cudaStream_t)stream;
     StageTimer timer(stage_ms_host != nullptr, s);
-    uint32_t* device_status = nullptr;
-    const uint32_t* tile_order = nullptr;
-    int st = build_tile_lists(vertices, indices, colors, opacities, T, W, H, tw, th, max_layers, tri_geo, tri_attr,
-                              sorted_ids, list_capacity, offsets, workspace, workspace_bytes, info_host, flags, timer, &device_status, &tile_order, s);
+    if (int st = check_forward_args(T, W, H, tw, th, max_layers, workspace, info_host, offsets, list_capacity, flags)) return st;
+    TileLists lists(workspace, T, W, H, tw, th, list_capacity, flags);
+    int st = lists.start(vertices, indices, colors, opacities, T, W, H, tw, th, tri_geo, tri_attr, sorted_ids, list_capacity,
+                         offsets, workspace_bytes, info_host, flags, timer, s);
     if (st) return st;
+    if ((st = lists.wait(list_capacity, info_host, s))) return st;
+    timer.mark();                                                    // [3] start of "sorting"
+    if ((st = lists.sort(sorted_ids, offsets, s))) return st;
     timer.mark();                                                    // [4] start of "rasterization" (here: forward + backward)
-    tg_host::set_tile_order(tile_order);
+    tg_host::set_tile_order(lists.order);
     st = tg_blend_step_l2(tri_geo, tri_attr, sorted_ids, offsets, V, W, H, tw, th, thr, max_layers, target, grad_scale,
                           loss_scale, loss_out, image, depthmap, final_weights, ends, grad_vertices, grad_colors,
                           grad_opacities, accumulate, scratch, scratch_bytes, stream);
     tg_host::set_tile_order(nullptr);
     if (st) return st;
     timer.mark();                                                    // [5] end
-    if (device_status) TG_CUDA(cudaMemcpyAsync(&info_host[2], device_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    if (lists.device_status)
+        TG_CUDA(cudaMemcpyAsync(&info_host[2], lists.device_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
     return finish_timing(timer, stage_ms_host, info_host, s);
 }
 

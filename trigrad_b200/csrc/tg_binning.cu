@@ -750,8 +750,14 @@ __global__ void __launch_bounds__(32 * kBinWarps, 4) bin_kernel(const float4* __
 __global__ void __launch_bounds__(256) scatter_entries_kernel(const uint4* __restrict__ pairs, const uint32_t* __restrict__ info,
                                                               uint32_t capacity, const int32_t* __restrict__ offsets,
                                                               uint64_t* __restrict__ entries, uint32_t* __restrict__ order,
-                                                              int tiles) {
+                                                              int tiles, uint32_t* __restrict__ tile_counts,
+                                                              uint32_t* __restrict__ counters, uint32_t* __restrict__ list_heads) {
     __shared__ uint32_t s_hist[33];
+    // the binning kernel is done with its counters: zero for the next call
+    const uint32_t me = blockIdx.x * 256 + threadIdx.x;
+    for (uint32_t i = me; i < (uint32_t)tiles; i += gridDim.x * 256) tile_counts[i] = 0;
+    if (me < 2) counters[me] = 0;
+    if (me < 6) list_heads[me] = 0;
     const uint32_t n = info[2];               // slots, holes included
     if (n > capacity) return;
     if (blockIdx.x == gridDim.x - 1) {
@@ -840,7 +846,7 @@ int allow_smem(const void* kernel, size_t bytes, SmemAllowed& allowed) {
 // (declared in tg_common.cuh with what each argument is).
 int bin_triangles(const float* vertices, const int32_t* indices, const float* colors, const float* opacities, int T, int W,
                   int H, int tw, int th, float* tri_geo, float* tri_attr, const BinBuffers& b, int32_t* offsets,
-                  uint32_t list_capacity, uint32_t* info_host, bool cull, bool packed, cudaStream_t stream) {
+                  uint32_t list_capacity, uint32_t* info_host, bool cull, bool packed, bool ready, cudaStream_t stream) {
     if (int s = check_dims_internal(T, W, H, tw, th)) return s;
     TG_REQUIRE(offsets, "null pointer");
     const int tiles_x = (W + tw - 1) / tw, tiles_y = (H + th - 1) / th;
@@ -853,10 +859,12 @@ int bin_triangles(const float* vertices, const int32_t* indices, const float* co
     const bool by_last_cta = tiles <= tg::kTileScanByLastCta;
     TG_REQUIRE(!cull || by_last_cta, "tile culling is limited to 65536 tiles");
     float4* rows = b.tables + tiles_x;
-    const size_t init = b.clear_words > (size_t)tiles_x + tiles_y ? b.clear_words : (size_t)tiles_x + tiles_y;
-    tg::bin_init_kernel<<<(unsigned)((init + 255) / 256), 256, 0, stream>>>(b.clear, b.clear_words, b.tables, rows, tiles_x,
-                                                                          tiles_y, W, H, tw, th);
-    TG_LAUNCH_CHECK("bin_init_kernel");
+    if (!ready || !by_last_cta) {
+        const size_t init = b.clear_words > (size_t)tiles_x + tiles_y ? b.clear_words : (size_t)tiles_x + tiles_y;
+        tg::bin_init_kernel<<<(unsigned)((init + 255) / 256), 256, 0, stream>>>(b.clear, b.clear_words, b.tables, rows, tiles_x,
+                                                                              tiles_y, W, H, tw, th);
+        TG_LAUNCH_CHECK("bin_init_kernel");
+    }
     if (T == 0) {
         TG_CUDA(cudaMemsetAsync(b.info, 0, sizeof(uint32_t) * 3, stream));
         TG_CUDA(cudaMemsetAsync(offsets, 0, sizeof(int32_t) * ((size_t)tiles + 1), stream));
@@ -888,11 +896,12 @@ int bin_triangles(const float* vertices, const int32_t* indices, const float* co
 }
 
 int scatter_entries(const BinBuffers& b, uint32_t list_capacity, const int32_t* offsets, int tiles, int T, cudaStream_t stream) {
-    if (T == 0 || list_capacity == 0) return TG_OK;
+    if (T == 0) return TG_OK;
     // K is not known on the host yet: as many CTAs as its upper bound fills, at most eight per SM, and one for the order
     const uint32_t want = (list_capacity + 1023) / 1024;
     const int grid = (int)(want < 148 * 8 ? want : 148 * 8) + 1;
-    tg::scatter_entries_kernel<<<grid, 256, 0, stream>>>(b.pairs, b.info, list_capacity, offsets, b.entries, b.tile_order, tiles);
+    tg::scatter_entries_kernel<<<grid, 256, 0, stream>>>(b.pairs, b.info, list_capacity, offsets, b.entries, b.tile_order, tiles,
+                                                              b.tile_counts, b.counters, b.list_heads);
     TG_LAUNCH_CHECK("scatter_entries_kernel");
     return TG_OK;
 }

@@ -19,7 +19,7 @@
 // recurrences; every lane adds its contribution with 128-bit vector reductions
 // (red.global.add.v4.f32) into a packed per-vertex buffer (x, y, w, opacity | r, g, b, -) that a
 // small kernel then unpacks into grad_vertices / grad_colors / grad_opacities.
-#include "tg_common.cuh"
+#include "tg_radix.cuh"
 
 namespace tg {
 
@@ -593,16 +593,33 @@ __device__ __forceinline__ void store_pixel(const TileCtx& c, const BlendParams&
 // fragment (k < ends).  Only written when it is not null (per-pixel mode, max_layers <= 32).
 // STREAM: lists of more than one chunk are streamed through two staging buffers (select_sweep); instantiated
 // separately because the state it carries costs the one-chunk tiles a few spilled registers.
-template <bool SORT, int MAXT, bool STREAM = false>
+// FUSED: the lists (at most kFusedList entries) are still unsorted; the CTA sorts its own, by counting smaller words.  That
+// is one launch and one trip through memory less, most of a small render's time.
+struct UnsortedLists {
+    const uint64_t* entries;      // ordered depth << 32 | triangle, grouped by tile
+    const uint32_t* info;         // K, longest list, slots
+    uint32_t capacity;
+    int* sorted_ids;
+};
+template <bool SORT, int MAXT, bool STREAM = false, bool FUSED = false>
 __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (SORT ? 4 : 5) : 1) blend_forward_kernel(BlendParams P, float4* __restrict__ image,
                                                              float* __restrict__ depthmap, float* __restrict__ final_w,
-                                                             int* __restrict__ ends, int* __restrict__ sel) {
+                                                             int* __restrict__ ends, int* __restrict__ sel,
+                                                             UnsortedLists unsorted = {}) {
     __shared__ float4 s_geo[kChunk * kStagedQuads];
     __shared__ float4 s_attr[SORT ? kChunk * kStagedQuads : 1];   // one-chunk lists: attributes; longer ones: 2nd buffer
     __shared__ int s_id[kChunk];
     __shared__ int s_id2[STREAM ? kChunk : 1];
     __shared__ __align__(16) float s_coord[kMaxTileCoords];
     __shared__ SweepScratch s_scratch;
+    __shared__ uint64_t s_key[FUSED ? kFusedList : 1];
+    __shared__ int s_rank[FUSED ? kFusedList : 1];
+    __shared__ int s_list[FUSED ? kFusedList : 1];
+    if (FUSED) {
+        // launched before the host knows: nothing to do when the lists are too long or incomplete
+        const uint32_t slots = unsorted.info[2], longest = unsorted.info[1] & ~kOrderWrittenBit;
+        if (slots > unsorted.capacity || longest > kFusedList) return;
+    }
     const int this_tile = tile_of_block(P);
     if (P.offsets[this_tile] == P.offsets[this_tile + 1]) {
         // a tile without entries: background, and no need for pixel-centre coordinates (any pixel order will do)
@@ -617,7 +634,36 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (SORT ? 4 : 5) : 1) blend_
         }
         return;
     }
-    const TileCtx c = tile_context(P, s_coord);
+    if (FUSED) {
+        const int first = P.offsets[this_tile], n = P.offsets[this_tile + 1] - first;
+        for (int i = threadIdx.x; i < n; i += blockDim.x) {
+            s_key[i] = unsorted.entries[first + i];
+            s_rank[i] = 0;
+        }
+    }
+    const TileCtx c = tile_context(P, s_coord);      // its barrier makes the words above visible
+    if (FUSED) {
+        const int n = c.end - c.start, nt = blockDim.x;
+        // several threads per word where the CTA has them, each counting over a part of the list
+        const int words = n <= 32 ? 32 : n <= 64 ? 64 : (int)kFusedList, parts = max(1, nt / words);
+        const int step = (n + parts - 1) / parts, part = threadIdx.x / words;
+        if (part < parts) {
+            for (int i = threadIdx.x % words; i < n; i += (parts > 1 ? words : nt)) {
+                const uint64_t mine = s_key[i];
+                int below = 0;
+                for (int j = part * step; j < min(n, (part + 1) * step); j++) below += s_key[j] < mine ? 1 : 0;
+                if (below) atomicAdd(&s_rank[i], below);
+            }
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < n; i += nt) {
+            const int id = (int)(uint32_t)s_key[i], at = s_rank[i];
+            s_list[at] = id;
+            unsorted.sorted_ids[c.start + at] = id;
+        }
+        P.ids = s_list - c.start;
+        __syncthreads();
+    }
     PixelAcc acc;
 
     if (SORT) {
@@ -635,7 +681,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (SORT ? 4 : 5) : 1) blend_
             // number of pixels that found something, whether staging the attributes pays was slower: the loads then
             // wait alone behind a barrier.)
             const bool one_chunk = c.end - c.start <= kChunk;
-            select_sweep<STREAM, (STREAM || MAXT > 256)>(P, c, go, bs, last, batch,
+            select_sweep<STREAM, (STREAM || MAXT > 256) && !FUSED>(P, c, go, bs, last, batch,
                                  {s_geo, s_id, &s_scratch, one_chunk ? s_attr : nullptr, one_chunk ? nullptr : s_attr, s_id2});
             const int found = batch.found;
             if (go) {
@@ -1587,6 +1633,25 @@ void set_tile_order(const uint32_t* order, uint32_t longest_list) {
     g_tile_order = order;
     g_longest_list = longest_list;
 }
+
+int blend_forward_short(const float* tri_geo, const float* tri_attr, const uint64_t* entries, const uint32_t* info,
+                        uint32_t capacity, int32_t* sorted_ids, const int32_t* offsets, int W, int H, int tw, int th, float thr,
+                        int per_pixel_sort, int max_layers, float* image, float* depthmap, float* final_weights,
+                        int32_t* ends, int32_t* selection, cudaStream_t s) {
+    TG_REQUIRE(((uintptr_t)image & 15) == 0, "image must be 16-byte aligned");
+    if (tg_selection_planes(per_pixel_sort, max_layers) == 0) selection = nullptr;
+    const tg::BlendParams P = make_params(tri_geo, tri_attr, nullptr, offsets, W, H, tw, th, thr, max_layers);
+    const tg::UnsortedLists lists = {entries, info, capacity, sorted_ids};
+    const int tiles = P.tiles_x * ((H + th - 1) / th);
+    const int threads = ((tw * th + 31) / 32) * 32;
+    auto kernel = threads <= 256 ? (per_pixel_sort ? tg::blend_forward_kernel<true, 256, false, true>
+                                                   : tg::blend_forward_kernel<false, 256, false, true>)
+                                 : (per_pixel_sort ? tg::blend_forward_kernel<true, 1024, false, true>
+                                                   : tg::blend_forward_kernel<false, 1024, false, true>);
+    kernel<<<tiles, threads, 0, s>>>(P, (float4*)image, depthmap, final_weights, ends, selection, lists);
+    TG_LAUNCH_CHECK("blend_forward_kernel (short lists)");
+    return TG_OK;
+}
 }  // namespace tg_host
 
 extern "C" {
@@ -1608,12 +1673,12 @@ int tg_blend_forward(const float* tri_geo, const float* tri_attr, const int32_t*
     if (threads <= 256) {
         // lists well beyond one staged chunk (the binning kernel of the same call reported the longest): stream them
         if (per_pixel_sort && threads == 256 && tg_host::g_longest_list > 2u * tg::kChunk)
-            tg::blend_forward_kernel<true, 256, true><<<tiles, threads, 0, s>>>(P, img, depthmap, final_weights, ends, selection);
-        else if (per_pixel_sort) tg::blend_forward_kernel<true, 256><<<tiles, threads, 0, s>>>(P, img, depthmap, final_weights, ends, selection);
-        else tg::blend_forward_kernel<false, 256><<<tiles, threads, 0, s>>>(P, img, depthmap, final_weights, ends, nullptr);
+            tg::blend_forward_kernel<true, 256, true><<<tiles, threads, 0, s>>>(P, img, depthmap, final_weights, ends, selection, {});
+        else if (per_pixel_sort) tg::blend_forward_kernel<true, 256><<<tiles, threads, 0, s>>>(P, img, depthmap, final_weights, ends, selection, {});
+        else tg::blend_forward_kernel<false, 256><<<tiles, threads, 0, s>>>(P, img, depthmap, final_weights, ends, nullptr, {});
     } else {
-        if (per_pixel_sort) tg::blend_forward_kernel<true, 1024><<<tiles, threads, 0, s>>>(P, img, depthmap, final_weights, ends, selection);
-        else tg::blend_forward_kernel<false, 1024><<<tiles, threads, 0, s>>>(P, img, depthmap, final_weights, ends, nullptr);
+        if (per_pixel_sort) tg::blend_forward_kernel<true, 1024><<<tiles, threads, 0, s>>>(P, img, depthmap, final_weights, ends, selection, {});
+        else tg::blend_forward_kernel<false, 1024><<<tiles, threads, 0, s>>>(P, img, depthmap, final_weights, ends, nullptr, {});
     }
     TG_LAUNCH_CHECK("blend_forward_kernel");
     return TG_OK;

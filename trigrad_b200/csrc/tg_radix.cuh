@@ -20,6 +20,12 @@ constexpr int kHistDoneWord = 8;
 constexpr int kTileScanByLastCta = 65536;
 // Top bit of the longest-list word the binning kernel reports: a launch order of the tiles was written.
 constexpr uint32_t kOrderWrittenBit = 0x80000000u;
+// Longest tile list that the compositing kernel sorts itself, in images of at most kFusedTiles tiles: two waves of its
+// CTAs.  There a launch and a trip through memory count (1280 triangles, 256x256: 36 -> 27 us with the early launch); with
+// many waves the sort inside takes more of the SMs' time than the kernel of its own does (200k triangles, 1920x1080: 124 us
+// against 110 + 6).
+constexpr uint32_t kFusedList = 128;
+constexpr int kFusedTiles = 2 * 4 * 148;
 
 // Exclusive scan of one value per thread over the first 256 threads of a CTA (all threads of the CTA
 // must call it; threads beyond 256 pass 0 and ignore the result).
@@ -87,12 +93,18 @@ int sort_pairs(uint64_t* keys_a, uint64_t* keys_b, uint32_t* vals_a, uint32_t* v
                int end_bit, void* scratch, size_t scratch_bytes, uint32_t* status, int* result_in_b_host,
                bool scratch_prepared, cudaStream_t stream);
 size_t sort_scratch_clear_bytes(uint32_t n, int passes);
+// Forward compositing with the sort of the tile lists (at most kFusedList entries each, `info` as the binning kernel left
+// it) in the same kernel, which does nothing when a list is longer or the slots exceed `capacity`.
+int blend_forward_short(const float* tri_geo, const float* tri_attr, const uint64_t* entries, const uint32_t* info,
+                        uint32_t capacity, int32_t* sorted_ids, const int32_t* offsets, int W, int H, int tw, int th, float thr,
+                        int per_pixel_sort, int max_layers, float* image, float* depthmap, float* final_weights,
+                        int32_t* ends, int32_t* selection, cudaStream_t stream);
 void set_tile_order(const uint32_t* order, uint32_t longest_list = 0);
 size_t tile_sort_scratch_bytes(int tiles);
 // Workspace of the binning kernels (bin_triangles, scatter_entries).
 struct BinBuffers {
-    uint32_t* clear;             // zeroed by the first kernel: `clear_words` words that hold the next three and the head
-    size_t clear_words;          //   words of the sort's work lists
+    uint32_t* clear;             // zeroed by the first kernel: `clear_words` words that hold the next four
+    size_t clear_words;
     uint32_t* status;            // device error word
     uint32_t* counters;          // [2]
     uint32_t* tile_counts;       // [tiles], 16-byte aligned
@@ -102,11 +114,13 @@ struct BinBuffers {
     uint4* pairs;                // [list capacity]
     uint64_t* entries;           // [list capacity]
     uint32_t* tile_order;        // [tiles] or null
+    uint32_t* list_heads;        // [6] heads of the tile sort's work lists, zeroed by scatter_entries
 };
+// `ready`: the counters are zero and the tables valid from a call before (scatter_entries leaves them so).
 // `info_host`: mapped host memory whose words 0, 1 and 3 receive the three info words (K last), or null.
 int bin_triangles(const float* vertices, const int32_t* indices, const float* colors, const float* opacities, int T, int W,
                   int H, int tw, int th, float* tri_geo, float* tri_attr, const BinBuffers& b, int32_t* offsets,
-                  uint32_t list_capacity, uint32_t* info_host, bool cull, bool packed, cudaStream_t stream);
+                  uint32_t list_capacity, uint32_t* info_host, bool cull, bool packed, bool ready, cudaStream_t stream);
 int scatter_entries(const BinBuffers& b, uint32_t list_capacity, const int32_t* offsets, int tiles, int T, cudaStream_t stream);
 int sort_tile_lists(uint64_t* entries, const int32_t* offsets, int tiles, int32_t* sorted_ids, uint32_t* lists,
                     bool scratch_prepared, bool write_back, uint32_t longest, cudaStream_t stream);

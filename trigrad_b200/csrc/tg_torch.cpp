@@ -112,6 +112,9 @@ struct DeviceState {
     Tensor workspace, info;      // info [slots,4] int32 pinned: K, longest list, error word, -
     int slot = 0, last_slot = -1;
     int64_t k_estimate = 0;
+    bool short_lists = false;          // the last forward had no tile list beyond kShortList entries
+    // image and tile size of the last successful forward, whose counters and tables the workspace still holds; W = 0: none
+    int ready[4] = {0, 0, 0, 0};
 
     explicit DeviceState(at::Device device) {
         workspace = at::empty({0}, at::TensorOptions().dtype(at::kByte).device(device));
@@ -142,8 +145,10 @@ struct DeviceState {
         if (prev != s) check_error_word(prev);
     }
     void* workspace_of(size_t bytes, size_t* have) {
-        if ((size_t)workspace.numel() < bytes + 256)
+        if ((size_t)workspace.numel() < bytes + 256) {
             workspace = at::empty({(int64_t)(bytes + bytes / 4 + 512)}, workspace.options());
+            ready[0] = 0;
+        }
         const uintptr_t p = (uintptr_t)workspace.data_ptr(), base = (p + 255) / 256 * 256;
         *have = (size_t)workspace.numel() - (base - p);
         return (void*)base;
@@ -220,6 +225,7 @@ struct L2Step {     // forward, loss and gradients in one call (tg_render_step_l
     size_t scratch_bytes;
 };
 
+constexpr uint32_t kShortList = 128;      // what the compositing kernel sorts itself
 constexpr size_t kAlign = 256;
 size_t up(size_t x) { return (x + kAlign - 1) / kAlign * kAlign; }
 
@@ -260,7 +266,7 @@ ForwardOut forward(const Tensor& vertices_, const Tensor& indices_, const Tensor
     if (planes > 0 && planes * v.pixels() * 4 <= selection_max_bytes)
         s.selection = at::empty({planes, v.H, v.W}, options.dtype(at::kInt));
     if (record_timing) out.stage_ms.resize(5);
-    const unsigned flags = (cull ? TG_FORWARD_CULL_TILES : 0u) | (packed ? TG_INPUT_PACKED : 0u) | TG_INFO_MAPPED;
+    const unsigned fixed_flags = (cull ? TG_FORWARD_CULL_TILES : 0u) | (packed ? TG_INPUT_PACKED : 0u) | TG_INFO_MAPPED;
     const auto state = state_of(w.device, w.stream);
     std::lock_guard<std::mutex> lock(state->use);
     int64_t cap = std::max<int64_t>(state->k_estimate + state->k_estimate / 4 + 1024, 2 * (int64_t)T + 1024);
@@ -268,6 +274,11 @@ ForwardOut forward(const Tensor& vertices_, const Tensor& indices_, const Tensor
         s.ids = at::empty({cap}, options.dtype(at::kInt));
         size_t have = 0;
         void* ws = state->workspace_of(g.forward_workspace_bytes(T, v.tiles(), (uint32_t)cap), &have);
+        const int key[4] = {v.W, v.H, v.tw, v.th};
+        const bool ready = std::equal(key, key + 4, state->ready);
+        state->ready[0] = 0;                     // until this call has succeeded
+        const unsigned flags = fixed_flags | (ready ? TG_WORKSPACE_READY : 0u) |
+                               (state->short_lists && !step ? TG_EXPECT_SHORT_LISTS : 0u);
         const int slot = state->next_slot();
         int32_t* info = state->words(slot);
         float* ms = record_timing ? out.stage_ms.data() : nullptr;
@@ -290,6 +301,8 @@ ForwardOut forward(const Tensor& vertices_, const Tensor& indices_, const Tensor
             continue;
         }
         check(step ? "render_step_l2" : "render_forward", status);
+        std::copy(key, key + 4, state->ready);
+        state->short_lists = (uint32_t)info[1] <= kShortList;
         state->finish_call(slot);
         state->k_estimate = std::max<int64_t>(s.K, (uint32_t)info[3]);
         return out;
