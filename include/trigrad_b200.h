@@ -229,7 +229,10 @@ int tg_blend_backward_l2_u8(const float* tri_geo, const float* tri_attr, const i
  * writes three gradient tensors per call (src/trigrad/render.cu:789-791).
  */
 #define TG_ACCUMULATE_PACKED 2
-int tg_unpack_gradients(const void* scratch, size_t scratch_bytes, int V, float loss_scale, float* loss_out,
+/* Added to `accumulate` of tg_unpack_gradients and tg_unpack_gradients_rgba: the accumulator is zero again when the
+ * kernel ends (only the words that were not are written), ready for the next step without a clear. */
+#define TG_UNPACK_CLEAR 4
+int tg_unpack_gradients(void* scratch, size_t scratch_bytes, int V, float loss_scale, float* loss_out,
                         float* grad_vertices, float* grad_colors, float* grad_opacities, int accumulate,
                         tg_stream_t stream);
 
@@ -239,7 +242,7 @@ int tg_unpack_gradients(const void* scratch, size_t scratch_bytes, int V, float 
 int tg_pack_inputs(const float* colors, const float* opacities, const int32_t* indices, int V, int T, float* rgba,
                    int32_t* faces, tg_stream_t stream);
 /* tg_unpack_gradients for the packed layout: grad_vertices [V,4] and grad_rgba [V,4] = (dr, dg, db, dopacity). */
-int tg_unpack_gradients_rgba(const void* scratch, size_t scratch_bytes, int V, float loss_scale, float* loss_out,
+int tg_unpack_gradients_rgba(void* scratch, size_t scratch_bytes, int V, float loss_scale, float* loss_out,
                              float* grad_vertices, float* grad_rgba, int accumulate, tg_stream_t stream);
 
 /* ---- forward + backward of mean((image - target)^2) in one kernel --------------------------------

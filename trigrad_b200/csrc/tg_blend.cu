@@ -1545,21 +1545,40 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (SORT ? 3 : 4) : 1) blend_
     }
 }
 
-// Packed accumulator -> the three gradient tensors of the reference (render.cu:789-791).
-__global__ void __launch_bounds__(256) unpack_gradients_kernel(const float4* __restrict__ gpack, int V,
-                                                               float4* __restrict__ gV, float* __restrict__ gC,
-                                                               float* __restrict__ gO, int accumulate,
-                                                               const float* __restrict__ l2_partials, float l2_loss_scale,
-                                                               float* __restrict__ l2_loss_out) {
-    if (l2_loss_out && blockIdx.x == 0 && threadIdx.x < 32) {
-        float x = l2_partials[threadIdx.x] + l2_partials[threadIdx.x + 32];
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) x += __shfl_xor_sync(0xffffffffu, x, d);
-        if (threadIdx.x == 0) *l2_loss_out = (accumulate ? *l2_loss_out : 0.f) + x * l2_loss_scale;
+// One vertex of the packed accumulator; with `clear` its words are zeroed behind the read.  False: all zero.
+__device__ __forceinline__ bool take_vertex(float4* gpack, int v, bool clear, float4& a, float4& b) {
+    a = gpack[2 * (size_t)v];
+    b = gpack[2 * (size_t)v + 1];
+    const bool any = a.x != 0.f || a.y != 0.f || a.z != 0.f || a.w != 0.f || b.x != 0.f || b.y != 0.f || b.z != 0.f;
+    if (clear && any) {
+        gpack[2 * (size_t)v] = make_float4(0.f, 0.f, 0.f, 0.f);
+        gpack[2 * (size_t)v + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
+    return any;
+}
+__device__ __forceinline__ void unpack_loss(float* partials, float scale, float* loss_out, bool accumulate, bool clear) {
+    if (blockIdx.x != 0 || threadIdx.x >= 32 || (!loss_out && !clear)) return;
+    float x = partials[threadIdx.x] + partials[threadIdx.x + 32];
+    if (clear) {
+        partials[threadIdx.x] = 0.f;
+        partials[threadIdx.x + 32] = 0.f;
+    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) x += __shfl_xor_sync(0xffffffffu, x, d);
+    if (threadIdx.x == 0 && loss_out) *loss_out = (accumulate ? *loss_out : 0.f) + x * scale;
+}
+
+// Packed accumulator -> the three gradient tensors of the reference (render.cu:789-791).  Bound by DRAM: 32 bytes read per
+// vertex, and 32 written or, adding to the tensors, touched only for vertices that received something.
+__global__ void __launch_bounds__(256) unpack_gradients_kernel(float4* __restrict__ gpack, int V, float4* __restrict__ gV,
+                                                               float* __restrict__ gC, float* __restrict__ gO, int accumulate,
+                                                               int clear, float* __restrict__ l2_partials,
+                                                               float l2_loss_scale, float* __restrict__ l2_loss_out) {
+    unpack_loss(l2_partials, l2_loss_scale, l2_loss_out, accumulate != 0, clear != 0);
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= V) return;
-    const float4 a = gpack[2 * (size_t)v], b = gpack[2 * (size_t)v + 1];
+    float4 a, b;
+    if (!take_vertex(gpack, v, clear != 0, a, b) && accumulate) return;
     float4 ov = make_float4(a.x, a.y, 0.f, a.z);
     float c0 = b.x, c1 = b.y, c2 = b.z, o = a.w;
     if (accumulate) {
@@ -1574,19 +1593,15 @@ __global__ void __launch_bounds__(256) unpack_gradients_kernel(const float4* __r
 }
 
 // The same for the packed input layout: colour and opacity gradients as one [V,4] array (dr, dg, db, dopacity).
-__global__ void __launch_bounds__(256) unpack_gradients_rgba_kernel(const float4* __restrict__ gpack, int V,
-                                                                    float4* __restrict__ gV, float4* __restrict__ gRGBA,
-                                                                    int accumulate, const float* __restrict__ l2_partials,
-                                                                    float l2_loss_scale, float* __restrict__ l2_loss_out) {
-    if (l2_loss_out && blockIdx.x == 0 && threadIdx.x < 32) {
-        float x = l2_partials[threadIdx.x] + l2_partials[threadIdx.x + 32];
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) x += __shfl_xor_sync(0xffffffffu, x, d);
-        if (threadIdx.x == 0) *l2_loss_out = (accumulate ? *l2_loss_out : 0.f) + x * l2_loss_scale;
-    }
+__global__ void __launch_bounds__(256) unpack_gradients_rgba_kernel(float4* __restrict__ gpack, int V, float4* __restrict__ gV,
+                                                                    float4* __restrict__ gRGBA, int accumulate, int clear,
+                                                                    float* __restrict__ l2_partials, float l2_loss_scale,
+                                                                    float* __restrict__ l2_loss_out) {
+    unpack_loss(l2_partials, l2_loss_scale, l2_loss_out, accumulate != 0, clear != 0);
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= V) return;
-    const float4 a = gpack[2 * (size_t)v], b = gpack[2 * (size_t)v + 1];
+    float4 a, b;
+    if (!take_vertex(gpack, v, clear != 0, a, b) && accumulate) return;
     float4 ov = make_float4(a.x, a.y, 0.f, a.z), oc = make_float4(b.x, b.y, b.z, a.w);
     if (accumulate) {
         const float4 pv = gV[v], pc = gRGBA[v];
@@ -1744,7 +1759,7 @@ static int backward_impl(const float* tri_geo, const float* tri_attr, const int3
     TG_LAUNCH_CHECK("blend_backward_kernel");
     if (packed) return TG_OK;
     tg::unpack_gradients_kernel<<<(V + 255) / 256, 256, 0, s>>>(gpack, V, (float4*)grad_vertices, grad_colors,
-                                                              grad_opacities, accumulate, partials, l2_loss_scale,
+                                                              grad_opacities, accumulate, 0, partials, l2_loss_scale,
                                                               l2_target ? l2_loss_out : nullptr);
     TG_LAUNCH_CHECK("unpack_gradients_kernel");
     return TG_OK;
@@ -1786,45 +1801,49 @@ int tg_blend_step_l2(const float* tri_geo, const float* tri_attr, const int32_t*
     TG_LAUNCH_CHECK("blend_step_l2_kernel");
     if (packed) return TG_OK;
     tg::unpack_gradients_kernel<<<(V + 255) / 256, 256, 0, s>>>(gpack, V, (float4*)grad_vertices, grad_colors,
-                                                              grad_opacities, accumulate, partials, loss_scale, loss_out);
+                                                              grad_opacities, accumulate, 0, partials, loss_scale, loss_out);
     TG_LAUNCH_CHECK("unpack_gradients_kernel");
     return TG_OK;
 }
 
-int tg_unpack_gradients(const void* scratch, size_t scratch_bytes, int V, float loss_scale, float* loss_out,
+int tg_unpack_gradients(void* scratch, size_t scratch_bytes, int V, float loss_scale, float* loss_out,
                         float* grad_vertices, float* grad_colors, float* grad_opacities, int accumulate,
                         tg_stream_t stream) {
     TG_REQUIRE(V > 0, "V must be positive");
     TG_REQUIRE(scratch && grad_vertices && grad_colors && grad_opacities, "null pointer");
-    TG_REQUIRE(accumulate == 0 || accumulate == 1, "accumulate must be 0 or 1");
+    const int clear = accumulate & TG_UNPACK_CLEAR;
+    accumulate &= ~TG_UNPACK_CLEAR;
+    TG_REQUIRE(accumulate == 0 || accumulate == 1, "accumulate must be 0 or 1 (+ TG_UNPACK_CLEAR)");
     TG_REQUIRE(((uintptr_t)grad_vertices & 15) == 0 && ((uintptr_t)scratch & 15) == 0,
                "grad_vertices / scratch must be 16-byte aligned");
     if (scratch_bytes < tg_backward_scratch_bytes(V)) {
         tg_host::set_error("backward scratch: need %zu bytes, got %zu", tg_backward_scratch_bytes(V), scratch_bytes);
         return TG_ERR_WORKSPACE;
     }
-    const float* partials = (const float*)((const char*)scratch + (size_t)V * 32);
+    float* partials = (float*)((char*)scratch + (size_t)V * 32);
     tg::unpack_gradients_kernel<<<(V + 255) / 256, 256, 0, (cudaStream_t)stream>>>(
-        (const float4*)scratch, V, (float4*)grad_vertices, grad_colors, grad_opacities, accumulate, partials, loss_scale,
+        (float4*)scratch, V, (float4*)grad_vertices, grad_colors, grad_opacities, accumulate, clear, partials, loss_scale,
         loss_out);
     TG_LAUNCH_CHECK("unpack_gradients_kernel");
     return TG_OK;
 }
 
-int tg_unpack_gradients_rgba(const void* scratch, size_t scratch_bytes, int V, float loss_scale, float* loss_out,
+int tg_unpack_gradients_rgba(void* scratch, size_t scratch_bytes, int V, float loss_scale, float* loss_out,
                              float* grad_vertices, float* grad_rgba, int accumulate, tg_stream_t stream) {
     TG_REQUIRE(V > 0, "V must be positive");
     TG_REQUIRE(scratch && grad_vertices && grad_rgba, "null pointer");
-    TG_REQUIRE(accumulate == 0 || accumulate == 1, "accumulate must be 0 or 1");
+    const int clear = accumulate & TG_UNPACK_CLEAR;
+    accumulate &= ~TG_UNPACK_CLEAR;
+    TG_REQUIRE(accumulate == 0 || accumulate == 1, "accumulate must be 0 or 1 (+ TG_UNPACK_CLEAR)");
     TG_REQUIRE((((uintptr_t)grad_vertices | (uintptr_t)grad_rgba | (uintptr_t)scratch) & 15) == 0,
                "grad_vertices / grad_rgba / scratch must be 16-byte aligned");
     if (scratch_bytes < tg_backward_scratch_bytes(V)) {
         tg_host::set_error("backward scratch: need %zu bytes, got %zu", tg_backward_scratch_bytes(V), scratch_bytes);
         return TG_ERR_WORKSPACE;
     }
-    const float* partials = (const float*)((const char*)scratch + (size_t)V * 32);
+    float* partials = (float*)((char*)scratch + (size_t)V * 32);
     tg::unpack_gradients_rgba_kernel<<<(V + 255) / 256, 256, 0, (cudaStream_t)stream>>>(
-        (const float4*)scratch, V, (float4*)grad_vertices, (float4*)grad_rgba, accumulate, partials, loss_scale, loss_out);
+        (float4*)scratch, V, (float4*)grad_vertices, (float4*)grad_rgba, accumulate, clear, partials, loss_scale, loss_out);
     TG_LAUNCH_CHECK("unpack_gradients_rgba_kernel");
     return TG_OK;
 }
@@ -1877,7 +1896,7 @@ int tg_blend_backward_corrected(const float* tri_geo, const float* tri_attr, con
     }
     TG_LAUNCH_CHECK("blend_backward_corrected_kernel");
     tg::unpack_gradients_kernel<<<(V + 255) / 256, 256, 0, s>>>(gpack, V, (float4*)grad_vertices, grad_colors,
-                                                              grad_opacities, accumulate, partials, 0.f, nullptr);
+                                                              grad_opacities, accumulate, 0, partials, 0.f, nullptr);
     TG_LAUNCH_CHECK("unpack_gradients_kernel");
     return TG_OK;
 }

@@ -116,6 +116,11 @@ struct DeviceState {
     // image and tile size of the last successful forward, whose counters and tables the workspace still holds; W = 0: none
     int ready[4] = {0, 0, 0, 0};
 
+    // Packed gradient accumulator, kept zero between calls (`accumulator_zero`: the last call left it so): the kernel that
+    // unpacks it zeroes what it reads, so that no call clears 32 bytes per vertex first.
+    Tensor accumulator;
+    bool accumulator_zero = false;
+
     explicit DeviceState(at::Device device) {
         workspace = at::empty({0}, at::TensorOptions().dtype(at::kByte).device(device));
         info = at::zeros({kSlots, 4}, at::TensorOptions().dtype(at::kInt)).pin_memory();
@@ -153,6 +158,29 @@ struct DeviceState {
         *have = (size_t)workspace.numel() - (base - p);
         return (void*)base;
     }
+};
+
+// The state's accumulator for the time of one backward (under `use`), or a fresh one where it would keep more than
+// kAccumulatorMax bytes alive.
+constexpr size_t kAccumulatorMax = size_t(256) << 20;
+struct Accumulator {
+    DeviceState& state;
+    Tensor t;
+    bool kept;
+    Accumulator(DeviceState& s, size_t bytes, const at::TensorOptions& byte_options) : state(s), kept(bytes <= kAccumulatorMax) {
+        if (!kept) {
+            t = at::zeros({(int64_t)bytes}, byte_options);
+            return;
+        }
+        if (!state.accumulator.defined() || (size_t)state.accumulator.numel() < bytes) {
+            state.accumulator = at::zeros({(int64_t)bytes}, byte_options);
+        } else if (!state.accumulator_zero) {
+            state.accumulator.zero_();
+        }
+        state.accumulator_zero = false;
+        t = state.accumulator;
+    }
+    void unpacked() { state.accumulator_zero = kept; }       // by a kernel with TG_UNPACK_CLEAR
 };
 
 // At most kStates of them: a program that keeps making streams gives back the workspace of the one not used for longest.
@@ -339,30 +367,30 @@ std::vector<Tensor> backward(Kind kind, const Saved& s, const Tensor& image, con
     gi = gi.defined() ? gi.contiguous() : at::zeros_like(image);      // only the depth map was used downstream
     gd = gd.defined() ? gd.contiguous() : Tensor();                  // none: taken as zero by the kernel
     const size_t nscratch = g.backward_scratch_bytes(s.V);
-    const Tensor scratch = at::empty({(int64_t)nscratch}, options.dtype(at::kByte));
     const View& v = s.v;
-    if (kind == Kind::kPacked) {
-        scratch.zero_();
-        // the sums stay in the packed accumulator, which already has the layout wanted here
-        check("blend_backward", g.blend_backward(s.geo, s.attr, s.id_list(), s.offsets, s.V, v.W, v.H, v.tw, v.th, v.sort,
-                                                 v.layers, data<float>(gi), data<float>(gd), data<float>(image),
-                                                 data<float>(depthmap), s.final_w, s.ends, s.sel(), nullptr, nullptr,
-                                                 nullptr, TG_ACCUMULATE_PACKED, scratch.data_ptr(), nscratch, w.stream));
-        check("unpack_gradients_rgba", g.unpack_gradients_rgba(scratch.data_ptr(), nscratch, s.V, 0.f, nullptr,
-                                                               data<float>(out[0]), data<float>(out[1]), 0, w.stream));
-    } else if (kind == Kind::kCorrected) {
+    const auto state = state_of(w.device, w.stream);
+    std::lock_guard<std::mutex> lock(state->use);
+    if (kind == Kind::kCorrected) {
+        const Tensor scratch = at::empty({(int64_t)nscratch}, options.dtype(at::kByte));
         check("blend_backward_corrected",
               g.blend_backward_corrected(s.geo, s.attr, s.id_list(), s.offsets, s.V, v.W, v.H, v.tw, v.th, v.sort, v.layers,
                                          data<float>(gi), data<float>(gd), data<float>(image), data<float>(depthmap),
                                          s.final_w, s.ends, data<float>(out[0]), data<float>(out[1]), data<float>(out[2]),
                                          0, scratch.data_ptr(), nscratch, w.stream));
-    } else {
-        check("blend_backward", g.blend_backward(s.geo, s.attr, s.id_list(), s.offsets, s.V, v.W, v.H, v.tw, v.th, v.sort,
-                                                 v.layers, data<float>(gi), data<float>(gd), data<float>(image),
-                                                 data<float>(depthmap), s.final_w, s.ends, s.sel(), data<float>(out[0]),
-                                                 data<float>(out[1]), data<float>(out[2]), 0, scratch.data_ptr(), nscratch,
-                                                 w.stream));
+        return out;
     }
+    Accumulator sums(*state, nscratch, options.dtype(at::kByte));
+    check("blend_backward", g.blend_backward(s.geo, s.attr, s.id_list(), s.offsets, s.V, v.W, v.H, v.tw, v.th, v.sort,
+                                             v.layers, data<float>(gi), data<float>(gd), data<float>(image),
+                                             data<float>(depthmap), s.final_w, s.ends, s.sel(), nullptr, nullptr, nullptr,
+                                             TG_ACCUMULATE_PACKED, sums.t.data_ptr(), nscratch, w.stream));
+    if (kind == Kind::kPacked)
+        check("unpack_gradients_rgba", g.unpack_gradients_rgba(sums.t.data_ptr(), nscratch, s.V, 0.f, nullptr, data<float>(out[0]),
+                                                               data<float>(out[1]), TG_UNPACK_CLEAR, w.stream));
+    else
+        check("unpack_gradients", g.unpack_gradients(sums.t.data_ptr(), nscratch, s.V, 0.f, nullptr, data<float>(out[0]),
+                                                     data<float>(out[1]), data<float>(out[2]), TG_UNPACK_CLEAR, w.stream));
+    sums.unpacked();
     return out;
 }
 
@@ -463,32 +491,48 @@ Tensor l2_step(const Tensor& vertices, const Tensor& indices, const Tensor& colo
     const Tensor target = target_.contiguous();
     const size_t nscratch = g.backward_scratch_bytes(V);
     const bool packed = to.packed.defined();
-    L2Step step;
-    step.target = data<float>(target);
-    step.mode = packed ? TG_ACCUMULATE_PACKED : 1;
-    step.loss = packed ? nullptr : data<float>(to.loss);
-    step.gV = packed ? nullptr : data<float>(to.vertices);
-    step.gC = packed ? nullptr : data<float>(to.colors);
-    step.gO = packed ? nullptr : data<float>(to.opacities);
-    const Tensor scratch = packed ? to.packed : at::empty({(int64_t)nscratch}, vertices.options().dtype(at::kByte).requires_grad(false));
-    step.scratch = scratch.data_ptr();
-    step.scratch_bytes = packed ? (size_t)scratch.numel() : nscratch;
-    if (one_kernel) return forward(vertices, indices, colors, opacities, v, false, false, cull, 0, &step).image;
+    const double n = 4.0 * v.pixels();
+    const auto byte_options = vertices.options().dtype(at::kByte).requires_grad(false);
+    if (one_kernel) {
+        const Tensor scratch = packed ? to.packed : at::empty({(int64_t)nscratch}, byte_options);
+        L2Step step;
+        step.target = data<float>(target);
+        step.mode = packed ? TG_ACCUMULATE_PACKED : 1;
+        step.loss = packed ? nullptr : data<float>(to.loss);
+        step.gV = packed ? nullptr : data<float>(to.vertices);
+        step.gC = packed ? nullptr : data<float>(to.colors);
+        step.gO = packed ? nullptr : data<float>(to.opacities);
+        step.scratch = scratch.data_ptr();
+        step.scratch_bytes = (size_t)scratch.numel();
+        return forward(vertices, indices, colors, opacities, v, false, false, cull, 0, &step).image;
+    }
     const ForwardOut f = forward(vertices, indices, colors, opacities, v, false, true, cull, selection_max_bytes);
     const Saved& s = *f.saved;
     TORCH_CHECK_VALUE(s.selection.defined(), "the fused L2 backward needs per_pixel_sort=True and max_layers <= 32");
-    const double n = 4.0 * v.pixels();
-    const int status =
-        target.scalar_type() == at::kByte
-            ? g.blend_backward_l2_u8(s.geo, s.attr, s.id_list(), s.offsets, V, v.W, v.H, v.tw, v.th, 1, v.layers,
-                                     data<uint8_t>(target), (float)(2.0 / n), (float)(1.0 / n), step.loss,
-                                     data<float>(f.image), data<float>(f.depthmap), s.final_w, s.ends, s.sel(), step.gV,
-                                     step.gC, step.gO, step.mode, step.scratch, step.scratch_bytes, w.stream)
-            : g.blend_backward_l2(s.geo, s.attr, s.id_list(), s.offsets, V, v.W, v.H, v.tw, v.th, 1, v.layers,
-                                  step.target, (float)(2.0 / n), (float)(1.0 / n), step.loss, data<float>(f.image),
-                                  data<float>(f.depthmap), s.final_w, s.ends, s.sel(), step.gV, step.gC, step.gO, step.mode,
-                                  step.scratch, step.scratch_bytes, w.stream);
-    check("blend_backward_l2", status);
+    auto backward_into = [&](const Tensor& sums) {
+        check("blend_backward_l2",
+              target.scalar_type() == at::kByte
+                  ? g.blend_backward_l2_u8(s.geo, s.attr, s.id_list(), s.offsets, V, v.W, v.H, v.tw, v.th, 1, v.layers,
+                                           data<uint8_t>(target), (float)(2.0 / n), (float)(1.0 / n), nullptr,
+                                           data<float>(f.image), data<float>(f.depthmap), s.final_w, s.ends, s.sel(), nullptr,
+                                           nullptr, nullptr, TG_ACCUMULATE_PACKED, sums.data_ptr(), (size_t)sums.numel(), w.stream)
+                  : g.blend_backward_l2(s.geo, s.attr, s.id_list(), s.offsets, V, v.W, v.H, v.tw, v.th, 1, v.layers,
+                                        data<float>(target), (float)(2.0 / n), (float)(1.0 / n), nullptr,
+                                        data<float>(f.image), data<float>(f.depthmap), s.final_w, s.ends, s.sel(), nullptr,
+                                        nullptr, nullptr, TG_ACCUMULATE_PACKED, sums.data_ptr(), (size_t)sums.numel(), w.stream));
+    };
+    if (packed) {
+        backward_into(to.packed);
+        return f.image;
+    }
+    const auto state = state_of(w.device, w.stream);
+    std::lock_guard<std::mutex> lock(state->use);
+    Accumulator sums(*state, nscratch, byte_options);
+    backward_into(sums.t);
+    check("unpack_gradients", g.unpack_gradients(sums.t.data_ptr(), nscratch, V, (float)(1.0 / n), data<float>(to.loss),
+                                                 data<float>(to.vertices), data<float>(to.colors), data<float>(to.opacities),
+                                                 1 | TG_UNPACK_CLEAR, w.stream));
+    sums.unpacked();
     return f.image;
 }
 
