@@ -1,0 +1,63 @@
+"""Single kernels at the sizes where they change their method: ends of length classes, remainders of chunks."""
+import numpy as np
+import pytest
+import torch
+
+import helpers as Hh
+import oracle as O
+from trigrad_b200 import scenes as S
+from trigrad_b200 import wrapper as Wr
+
+pytestmark = pytest.mark.gpu
+
+
+def _ordered(depth):
+    u = depth.astype(np.float32).view(np.uint32)
+    return np.where(u >> 31 != 0, ~u, u | np.uint32(0x80000000)).astype(np.uint64)
+
+
+@pytest.mark.parametrize("lengths", [[129, 3, 1023, 1024], [1025, 0, 4096, 8191], [8192, 8193, 130], [24575, 24576, 24577]],
+                         ids=lambda x: "_".join(map(str, x)))
+@pytest.mark.parametrize("depths", ["uniform", "two_layers", "clustered", "empty_clips"])
+def test_bucket_sort_of_tile_lists(lengths, depths):
+    """Finite depths with a few equal ones; the clustered ones overflow the buckets and take the network."""
+    rng = np.random.default_rng(len(lengths) + lengths[0])
+    offsets = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int32)
+    n = int(offsets[-1])
+    d = {"uniform": rng.uniform(-3, 10, n), "two_layers": rng.choice([1.0, 4.0], n) + rng.uniform(0, 0.02, n),
+         "clustered": 2 + rng.normal(0, 1e-4, n) ** 3, "empty_clips": rng.uniform(0.1, 10, n)}[depths].astype(np.float32)
+    d[5::50] = d[4::50][:len(d[5::50])]
+    if depths == "empty_clips":
+        d[::997] = 1e30
+    entries, expect = np.empty(n, np.uint64), np.empty(n, np.uint64)
+    for a, b in zip(offsets[:-1], offsets[1:]):
+        entries[a:b] = (_ordered(d[a:b]) << np.uint64(32)) | rng.permutation(int(b - a)).astype(np.uint64)
+        expect[a:b] = np.sort(entries[a:b])
+    dev = Hh.cuda(entries.view(np.int64))
+    ids = Hh.sort_tile_lists(dev, Hh.cuda(offsets))
+    torch.cuda.synchronize()
+    assert np.array_equal(dev.cpu().numpy().view(np.uint64), expect)
+    assert np.array_equal(ids.cpu().numpy().view(np.uint32), (expect & np.uint64(0xFFFFFFFF)).astype(np.uint32))
+
+
+@pytest.mark.parametrize("triangles,edge,width,height,tile,layers", [
+    (3000, 0.9, 61, 45, 16, 32),        # long lists, every pixel full early: the rest of the list is filtered
+    (3000, 0.9, 40, 33, 32, 8),         # the same with one CTA of 1024 threads, small batches
+    (20000, 0.02, 100, 77, 16, 32),     # small triangles: records tested by a lane each, last block cut by the image
+    (20000, 0.02, 90, 70, 8, 70),       # several batches
+    (129, 0.5, 33, 17, 16, 32),         # lists just beyond what the compositing kernel sorts itself
+    (128, 0.5, 33, 17, 16, 32),
+    (65, 0.5, 31, 31, 4, 5),
+])
+def test_forward_methods_agree_with_the_oracle(triangles, edge, width, height, tile, layers):
+    sc = S.random_triangles(triangles, width, height, edge, 0.4, name="methods", seed=triangles + tile)
+    sc.tile_width = sc.tile_height = tile
+    of = O.forward(sc.vertices, sc.indices, sc.colors, sc.opacities, width, height, tile, tile, 1e-6, True, layers)
+    for repeat in range(2):             # the second call finds the workspace and the guess of the first
+        out = Wr.forward_native(*Hh.scene_tensors(sc), width, height, tile, tile, 1e-6, False, True, layers, cull_tiles=True)
+        torch.cuda.synchronize()
+        assert np.array_equal(out[7].cpu().numpy(), of.ends)
+        assert np.array_equal(out[0].cpu().numpy().view(np.uint32), of.image.view(np.uint32))
+        assert np.array_equal(out[1].cpu().numpy().view(np.uint32), of.depthmap.view(np.uint32))
+    li = O.build_lists(sc.vertices, sc.indices, width, height, tile, tile, cull=True)
+    assert np.array_equal(out[4].cpu().numpy(), li.offsets) and np.array_equal(out[3].cpu().numpy(), li.ids)

@@ -249,12 +249,13 @@ __global__ void __launch_bounds__(256) bin_init_kernel(uint32_t* __restrict__ cl
     else if (i < (size_t)tiles_x + tiles_y) rows[i - tiles_x] = tile_span((int)(i - tiles_x), th, H);
 }
 
-// Exclusive scan of counts[0..tiles) by one CTA of 256 threads into offsets[0..tiles]; returns the largest count,
+// Exclusive scan of counts[0..tiles) by one CTA of the binning kernel into offsets[0..tiles]; returns the largest count,
 // the sum in `total`.
 // 16 consecutive counts per thread and round, fetched by four independent 16-byte loads one round ahead: the rounds are
 // bound by the latency of those loads.
+constexpr int kBinWarps = 4;         // warps of a CTA of the binning kernel (two and eight: 3 to 7 % slower)
 constexpr int kTileScanPer = 16;
-constexpr int kTileScanRound = 256 * kTileScanPer;
+constexpr int kTileScanRound = 32 * kBinWarps * kTileScanPer;
 __device__ __forceinline__ void load_counts(const uint32_t* counts, int first, int tiles, uint4 (&v)[4]) {
 #pragma unroll
     for (int k = 0; k < 4; k++) {
@@ -269,7 +270,7 @@ __device__ __forceinline__ void load_counts(const uint32_t* counts, int first, i
         }
     }
 }
-__device__ uint32_t tile_offsets_by_one_cta(const uint32_t* counts, int32_t* offsets, int tiles, uint32_t* s_warp /*[8]*/,
+__device__ uint32_t tile_offsets_by_one_cta(const uint32_t* counts, int32_t* offsets, int tiles, uint32_t* s_warp /*[kBinWarps]*/,
                                             uint32_t& total) {
     const int tid = threadIdx.x, warp = tid >> 5;
     uint32_t carry = 0, biggest = 0;
@@ -294,7 +295,7 @@ __device__ uint32_t tile_offsets_by_one_cta(const uint32_t* counts, int32_t* off
         __syncthreads();
         uint32_t run = carry + incl - mine;
 #pragma unroll
-        for (int w = 0; w < 8; w++) {
+        for (int w = 0; w < kBinWarps; w++) {
             const uint32_t x = s_warp[w];
             if (w < warp) run += x;
             carry += x;
@@ -321,7 +322,7 @@ __device__ uint32_t tile_offsets_by_one_cta(const uint32_t* counts, int32_t* off
     if (lane_id() == 0) s_warp[warp] = biggest;
     __syncthreads();
 #pragma unroll
-    for (int w = 0; w < 8; w++) biggest = max(biggest, s_warp[w]);
+    for (int w = 0; w < kBinWarps; w++) biggest = max(biggest, s_warp[w]);
     return biggest;
 }
 
@@ -545,8 +546,7 @@ struct BinArgs {
 };
 
 constexpr uint32_t kHole = 0xffffffffu;      // tile word of a pair that is not listed
-constexpr int kBinWarps = 8;
-constexpr int kBinQueue = 512;       // clip queue of a CTA
+constexpr int kBinQueue = 64 * kBinWarps;       // clip queue of a CTA
 // Shared memory of a warp, in words: first the staging area of its records (pitch 5 quads for the 4 of a geometry
 // record, 7 for the 6 of half the warp's attribute records: 16-byte accesses of consecutive lanes then fall on different
 // banks), then, component-major, what the pairs need of its triangles: matrix 9, corners 6, depth plane 3, tile
@@ -570,7 +570,7 @@ __device__ __forceinline__ void write_pair(const BinArgs& bin, const float* tri,
 }
 
 template <bool CULL>
-__global__ void __launch_bounds__(32 * kBinWarps, 4) bin_kernel(const float4* __restrict__ vertices,
+__global__ void __launch_bounds__(32 * kBinWarps, 32 / kBinWarps) bin_kernel(const float4* __restrict__ vertices,
                                                                 const int* __restrict__ indices,
                                                                 const float* __restrict__ colors,
                                                                 const float* __restrict__ opacities, int T, int per_cta,
@@ -583,7 +583,7 @@ __global__ void __launch_bounds__(32 * kBinWarps, 4) bin_kernel(const float4* __
     __shared__ uint32_t s_qx[kBinQueue], s_qy[kBinQueue], s_qe[kBinQueue];   // tile column, tile row << 8 | triangle, pair
     __shared__ uint32_t s_first[kBinWarps + 1];       // first pair of every warp's triangles
     __shared__ uint32_t s_queued, s_base;
-    __shared__ uint32_t s_warp[8];
+    __shared__ uint32_t s_warp[kBinWarps];
     __shared__ bool s_last;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const unsigned below = (1u << lane) - 1u;
@@ -872,9 +872,9 @@ int bin_triangles(const float* vertices, const int32_t* indices, const float* co
     }
     const tg::BinArgs bin = {b.tile_counts, offsets, b.counters, b.info, info_host, b.pairs, list_capacity, tiles, tiles_x,
                              tiles_y, by_last_cta ? 1 : 0, b.tile_order ? 1 : 0, {b.tables, rows}};
-    // Triangles per CTA: 256 where that fills the GPU; fewer below, so that a mesh of few triangles that cover many tiles
-    // each still spreads over all SMs (four CTAs on each).
-    constexpr int kWave = 148 * 4;
+    // Triangles per CTA: 32 per warp where that fills the GPU; fewer below, so that a mesh of few triangles that cover many
+    // tiles each still spreads over all SMs (eight CTAs on each).
+    constexpr int kWave = 148 * 32 / tg::kBinWarps;
     const int per_cta = T >= 32 * tg::kBinWarps * kWave ? 32 * tg::kBinWarps : (T + kWave - 1) / kWave;
     const int grid = (T + per_cta - 1) / per_cta;
     auto inverse = [](int n) { return (n & (n - 1)) == 0 ? 1.0 / n : 0.0; };

@@ -6,12 +6,14 @@
 // Entries are uint64 words (ordered depth << 32 | triangle), already grouped by tile:
 // tile t owns entries[offsets[t] .. offsets[t+1]).
 //   n <= 128     one warp per tile, rank sort: every element counts the smaller ones (no exchange steps)
-//   n <= 1024    a CTA of 128 threads per tile (work list): bitonic network in shared memory, 8 words per
-//                thread kept in registers between trips to shared memory
-//   n <= 16384   the same network in 136 KB of shared memory, 1024 threads with 8 or 16 words each;
-//                tiles taken from a work list
-//   beyond       the same CTA sorts 16384-entry chunks in shared memory and runs the network's wide
+//   n <= 1024    a CTA of 128 threads per tile (work list): bucket sort in shared memory - about as many
+//                buckets as words; one thread sorts a bucket by insertion
+//   n <= 8192    the same with 1024 threads, two CTAs per SM
+//   n <= 24576   the same with one CTA per SM
+//   beyond       a CTA sorts 16384-entry chunks with a bitonic network in shared memory and runs the network's wide
 //                steps on the segment in global memory
+// Where so many depths of a tile are (nearly) equal that a bucket gets more than kBucketMax words, the bitonic network
+// sorts the segment, 8 or 16 words per thread kept in registers between trips to shared memory.
 // No kernel here waits on another CTA.
 #include <atomic>
 
@@ -164,8 +166,171 @@ __device__ __forceinline__ int log2_at_least(uint32_t n) {
     return b;
 }
 
-// Work lists in the sort's scratch: [0] long tiles, [1] next long item to hand out in the first round,
-// [2] mid tiles, [3] next mid item, [4] next long item of the second round, [5] unused (all zero before
+// ---- bucket sort ---------------------------------------------------------------------------------------
+// n <= NT * E words from seg into s_keys in ascending order, through 2^LOGB buckets of about n / 2^LOGB words each: the
+// words are counted in 256 cells of equal width in depth, and the counts' running sum, linear within a cell, says which
+// share of the words lies below a depth (a tile of a mesh has its depths in a few thin layers).  Subtraction, product, sum
+// and truncation are monotone, so the buckets are in order whatever the rounding.  Words with the depth of an empty clip
+// (1e30) form a cell of their own.  False, for all threads, when a bucket gets too many words (s_keys then holds nothing).
+// `s_count`: 2^LOGB + 1 words; `s_cell`: 258 words; `s_warp`: 32 words.  Every thread of the CTA must call.
+constexpr uint32_t kBucketMax = 24;
+constexpr int kCells = 256;
+__device__ __forceinline__ float depth_of(uint32_t ordered) {
+    return __uint_as_float((ordered & 0x80000000u) ? ordered & 0x7fffffffu : ~ordered);
+}
+
+// Exclusive scan over the CTA of one value per thread; `voted`: whether any thread passed `vote`.
+template <int NT>
+__device__ __forceinline__ uint32_t cta_exclusive(uint32_t mine, uint32_t* s_warp, int tid, bool vote, bool& voted) {
+    const int lane = tid & 31, warp = tid >> 5;
+    uint32_t incl = mine;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += y;
+    }
+    if (lane == 31) s_warp[warp] = incl;
+    voted = __syncthreads_or(vote);
+    uint32_t run = lane < NT / 32 ? s_warp[lane] : 0u;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, run, d);
+        if (lane >= d) run += y;
+    }
+    run = __shfl_sync(0xffffffffu, run, (warp + 31) & 31);
+    return (warp == 0 ? 0u : run) + incl - mine;
+}
+
+template <int NT, int E, int LOGB>
+__device__ bool bucket_sort(uint64_t* s_keys, uint32_t* s_count, uint32_t* s_cell, uint32_t* s_warp, const uint64_t* seg,
+                            uint32_t n, int tid) {
+    constexpr int B = 1 << LOGB, PER = B / NT, CPER = (kCells + 1 + NT - 1) / NT, WARPS = NT / 32;
+    static_assert(PER * NT == B && NT * E <= 32768 && LOGB <= 16, "bucket and rank share a word");
+    const int lane = tid & 31, warp = tid >> 5;
+    const uint32_t empty_clip = float_to_ordered(1e30f);
+    const uint32_t* depths = reinterpret_cast<const uint32_t*>(seg) + 1;      // the high words
+    uint32_t lo = 0xffffffffu, hi = 0;
+#pragma unroll
+    for (int r = 0; r < E; r++) {
+        const uint32_t i = tid + r * NT;
+        if (i < n) {
+            const uint32_t u = depths[2 * i];
+            lo = min(lo, u);
+            if (u < empty_clip) hi = max(hi, u);
+        }
+    }
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if (lane == 0) { s_warp[warp] = lo; s_cell[warp] = hi; }
+    __syncthreads();
+    lo = 0xffffffffu; hi = 0;
+    if (lane < WARPS) { lo = s_warp[lane]; hi = s_cell[lane]; }
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    __syncthreads();
+    for (int b = tid; b <= B; b += NT) s_count[b] = 0;
+    for (int b = tid; b <= kCells; b += NT) s_cell[b] = 0;
+    const float first = depth_of(lo), span = depth_of(hi) - first;
+    const float scale = (float)(kCells - 1) / span;
+    if (!(span > 0.f && scale < FLT_MAX && span < FLT_MAX)) return false;      // all equal, or not finite
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < E; r++) {
+        const uint32_t i = tid + r * NT;
+        if (i < n) {
+            const uint32_t u = depths[2 * i];
+            atomicAdd(&s_cell[u < empty_clip ? min(kCells - 1, (int)((depth_of(u) - first) * scale)) : kCells], 1u);
+        }
+    }
+    __syncthreads();
+    bool voted;
+    {
+        uint32_t c[CPER], mine = 0;
+#pragma unroll
+        for (int k = 0; k < CPER; k++) {
+            const int b = tid * CPER + k;
+            c[k] = b <= kCells ? s_cell[b] : 0u;
+            mine += c[k];
+        }
+        uint32_t run = cta_exclusive<NT>(mine, s_warp, tid, false, voted);
+#pragma unroll
+        for (int k = 0; k < CPER; k++) {
+            const int b = tid * CPER + k;
+            if (b <= kCells) s_cell[b] = run;
+            run += c[k];
+        }
+        if (tid == 0) s_cell[kCells + 1] = n;
+    }
+    __syncthreads();
+    const float per_word = (float)B / (float)n;
+    uint32_t where[E];               // bucket << 15 | rank in it
+#pragma unroll
+    for (int r = 0; r < E; r++) {
+        const uint32_t i = tid + r * NT;
+        where[r] = 0;
+        if (i < n) {
+            const uint32_t u = depths[2 * i];
+            const float x = u < empty_clip ? fminf((depth_of(u) - first) * scale, (float)kCells - 0.5f) : (float)kCells;
+            const int cell = (int)x;
+            const float below = (float)s_cell[cell];
+            const float share = fminf(fmaf(x - (float)cell, (float)s_cell[cell + 1] - below, below), (float)s_cell[cell + 1]);
+            const int b = min(B - 1, (int)(share * per_word));
+            where[r] = ((uint32_t)b << 15) | atomicAdd(&s_count[b], 1u);
+        }
+    }
+    __syncthreads();
+    uint32_t mine = 0, biggest = 0, c[PER];
+#pragma unroll
+    for (int k = 0; k < PER; k++) {
+        c[k] = s_count[tid * PER + k];
+        mine += c[k];
+        biggest = max(biggest, c[k]);
+    }
+    uint32_t run = cta_exclusive<NT>(mine, s_warp, tid, biggest > kBucketMax, voted);
+    if (voted) return false;
+#pragma unroll
+    for (int k = 0; k < PER; k++) {
+        s_count[tid * PER + k] = run;
+        run += c[k];
+    }
+    if (tid == NT - 1) s_count[B] = n;
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < E; r++) {
+        const uint32_t i = tid + r * NT;
+        if (i < n) s_keys[s_count[where[r] >> 15] + (where[r] & 0x7fffu)] = seg[i];
+    }
+    __syncthreads();
+    for (int b = tid; b < B; b += NT) {
+        const int beg = (int)s_count[b], end = (int)s_count[b + 1];
+        for (int i = beg + 1; i < end; i++) {
+            const uint64_t x = s_keys[i];
+            int at = i;
+            for (; at > beg; at--) {
+                const uint64_t y = s_keys[at - 1];
+                if (y <= x) break;
+                s_keys[at] = y;
+            }
+            s_keys[at] = x;
+        }
+    }
+    __syncthreads();
+    return true;
+}
+
+template <int NT>
+__device__ __forceinline__ void hand_out(const uint64_t* s_keys, uint64_t* seg, uint32_t n, int32_t* ids_out, bool write_back,
+                                         int tid) {
+    for (uint32_t i = tid; i < n; i += NT) {
+        const uint64_t x = s_keys[i];
+        ids_out[i] = (int32_t)(uint32_t)x;
+        if (write_back) seg[i] = x;
+    }
+    __syncthreads();
+}
+
+// Work lists in the sort's scratch: [0] long tiles, [1] next long item of the kernel for the longest,
+// [2] mid tiles, [3] next mid item, [4] next long item of the other one, [5] unused (all zero before
 // tile_sort_kernel), then `tiles` slots of long items and `tiles` slots of mid items.
 constexpr int kListHead = 6;
 __device__ __forceinline__ uint32_t* long_items(uint32_t* lists) { return lists + kListHead; }
@@ -232,6 +397,7 @@ __global__ void __launch_bounds__(kTileSortThreads) tile_sort_mid_kernel(uint64_
                                                                          int32_t* __restrict__ sorted_ids, uint32_t* lists,
                                                                          int write_back) {
     __shared__ uint64_t s_mid[kMidSmemWords];
+    __shared__ uint32_t s_count[kTileSortShort + 1], s_cell[kCells + 2], s_warp[32];
     __shared__ uint32_t s_item;
     const int tid = threadIdx.x;
     const uint32_t count = lists[2];
@@ -244,8 +410,11 @@ __global__ void __launch_bounds__(kTileSortThreads) tile_sort_mid_kernel(uint64_
         const int tile = (int)mid_items(lists, tiles)[w];
         const int beg = offsets[tile];
         const uint32_t n = (uint32_t)(offsets[tile + 1] - beg);
-        sort_segment_in_smem<3, kTileSortThreads>(s_mid, entries + beg, n, log2_at_least(n), sorted_ids + beg,
-                                                  write_back != 0, tid);
+        if (bucket_sort<kTileSortThreads, 8, 10>(s_mid, s_count, s_cell, s_warp, entries + beg, n, tid))
+            hand_out<kTileSortThreads>(s_mid, entries + beg, n, sorted_ids + beg, write_back != 0, tid);
+        else
+            sort_segment_in_smem<3, kTileSortThreads>(s_mid, entries + beg, n, log2_at_least(n), sorted_ids + beg,
+                                                      write_back != 0, tid);
     }
 }
 
@@ -265,22 +434,27 @@ __device__ __forceinline__ void global_step(uint64_t* seg, uint32_t n, uint32_t 
     __syncthreads();
 }
 
-// Persistent CTAs (one per SM) take the long tiles from the work list, next free item first.
-__global__ void __launch_bounds__(kTileSortLongThreads) tile_sort_long_kernel(uint64_t* entries,
-                                                                              const int32_t* __restrict__ offsets,
-                                                                              int32_t* __restrict__ sorted_ids,
-                                                                              uint32_t* lists, int write_back) {
+// Persistent CTAs take the long tiles from the work list, next free item first.  Two kernels share the list: BIG takes
+// the tiles above kTileSortHalf words with one CTA per SM, the other one the rest with two.
+constexpr int kTileSortHalf = 8192, kTileSortBig = 24 * kTileSortLongThreads;
+constexpr int kLongBuckets = 4096;
+constexpr size_t long_smem_bytes(bool big) {
+    return sizeof(uint64_t) * (size_t)(big ? kTileSortBig : kTileSortHalf + (kTileSortHalf >> 3)) + sizeof(uint32_t) * (kLongBuckets + 4);
+}
+static_assert(kTileSortBig >= kLongSmemWords, "the network's padded chunk fits as well");
+template <bool BIG>
+__global__ void __launch_bounds__(kTileSortLongThreads, BIG ? 1 : 2)
+    tile_sort_long_kernel(uint64_t* entries, const int32_t* __restrict__ offsets, int32_t* __restrict__ sorted_ids,
+                          uint32_t* lists, int write_back) {
     extern __shared__ __align__(16) uint64_t s_long[];
-    __shared__ uint32_t s_item;
+    uint32_t* s_count = reinterpret_cast<uint32_t*>(s_long + (BIG ? kTileSortBig : kTileSortHalf + (kTileSortHalf >> 3)));
+    __shared__ uint32_t s_item, s_cell[kCells + 2], s_warp[32];
     constexpr int kLogChunk = 14;
     static_assert((1 << kLogChunk) == kTileSortChunk && kTileSortLongThreads == 1024, "chunk = 1024 threads x 16 words");
     const int tid = threadIdx.x;
     const uint32_t count = lists[0];
-    // Two rounds over the list: the tiles above 8192 entries first, the shorter ones afterwards, so that
-    // the kernel does not end on a few SMs that drew a long tile late.
-    for (int round = 0; round < 2; round++)
     while (true) {
-        if (tid == 0) s_item = atomicAdd(&lists[round == 0 ? 1 : 4], 1u);
+        if (tid == 0) s_item = atomicAdd(&lists[BIG ? 1 : 4], 1u);
         __syncthreads();
         const uint32_t w = s_item;
         __syncthreads();
@@ -288,11 +462,17 @@ __global__ void __launch_bounds__(kTileSortLongThreads) tile_sort_long_kernel(ui
         const int tile = (int)long_items(lists)[w];
         const int beg = offsets[tile];
         const uint32_t n = (uint32_t)(offsets[tile + 1] - beg);
-        if ((n > 8192u) != (round == 0)) continue;
+        if ((n > (uint32_t)kTileSortHalf) != BIG) continue;
         uint64_t* seg = entries + beg;
-        if (n <= 8192u) {            // 8 words per thread: 256, 512 or 1024 threads take part
-            sort_segment_in_smem<3, kTileSortLongThreads>(s_long, seg, n, log2_at_least(n), sorted_ids + beg,
-                                                          write_back != 0, tid);
+        if (!BIG) {
+            if (bucket_sort<kTileSortLongThreads, 8, 12>(s_long, s_count, s_cell, s_warp, seg, n, tid))
+                hand_out<kTileSortLongThreads>(s_long, seg, n, sorted_ids + beg, write_back != 0, tid);
+            else             // 8 words per thread: 256, 512 or 1024 threads take part
+                sort_segment_in_smem<3, kTileSortLongThreads>(s_long, seg, n, log2_at_least(n), sorted_ids + beg,
+                                                              write_back != 0, tid);
+        } else if (n <= (uint32_t)kTileSortBig &&
+                   bucket_sort<kTileSortLongThreads, 24, 12>(s_long, s_count, s_cell, s_warp, seg, n, tid)) {
+            hand_out<kTileSortLongThreads>(s_long, seg, n, sorted_ids + beg, write_back != 0, tid);
         } else if (n <= (uint32_t)kTileSortChunk) {
             sort_segment_in_smem<4, kTileSortLongThreads>(s_long, seg, n, kLogChunk, sorted_ids + beg, write_back != 0,
                                                           tid);
@@ -349,15 +529,19 @@ int sort_tile_lists(uint64_t* entries, const int32_t* offsets, int tiles, int32_
                                                                         write_back ? 1 : 0);
         TG_LAUNCH_CHECK("tile_sort_mid_kernel");
     }
-    if (longest > (uint32_t)tg::kTileSortShort) {
-        static SmemAllowed allowed;
-        const size_t long_smem = sizeof(uint64_t) * tg::kLongSmemWords;
-        if (int st = allow_smem((const void*)tg::tile_sort_long_kernel, long_smem, allowed)) return st;
-        const int grid = tiles < 148 ? tiles : 148;
-        tg::tile_sort_long_kernel<<<grid, tg::kTileSortLongThreads, long_smem, s>>>(entries, offsets, sorted_ids, lists,
-                                                                                     write_back ? 1 : 0);
+    auto launch_long = [&](auto kernel, bool big, int ctas, SmemAllowed& allowed) -> int {
+        const size_t smem = tg::long_smem_bytes(big);
+        if (int st = allow_smem((const void*)kernel, smem, allowed)) return st;
+        kernel<<<tiles < ctas ? tiles : ctas, tg::kTileSortLongThreads, smem, s>>>(entries, offsets, sorted_ids, lists,
+                                                                                 write_back ? 1 : 0);
         TG_LAUNCH_CHECK("tile_sort_long_kernel");
-    }
+        return TG_OK;
+    };
+    static SmemAllowed allowed[2];
+    if (longest > (uint32_t)tg::kTileSortHalf)
+        if (int st = launch_long(tg::tile_sort_long_kernel<true>, true, 148, allowed[0])) return st;
+    if (longest > (uint32_t)tg::kTileSortShort)
+        if (int st = launch_long(tg::tile_sort_long_kernel<false>, false, 2 * 148, allowed[1])) return st;
     return TG_OK;
 }
 
