@@ -27,27 +27,26 @@ __device__ __forceinline__ ClipVertex to_clip(const float* __restrict__ points, 
     return {c[0], c[1], c[2], c[3]};
 }
 
-// Which case a triangle is, and the rotation (in, out1, out2) / (out, in1, in2) the reference uses.
+// How many of a triangle's vertices are inside, and which vertex comes first in the reference's order: (in, out1, out2)
+// with one inside, (out, in1, in2) with two, (0, 1, 2) otherwise.
 struct ClipCase {
-    int inside;      // number of inside vertices
-    int k0, k1, k2;  // inside == 1: (in, out1, out2); inside == 2: (out, in1, in2); else (0, 1, 2)
+    int inside, first;
 };
-
 __device__ __forceinline__ ClipCase classify(float d0, float d1, float d2) {
     const bool i0 = d0 >= 0.f, i1 = d1 >= 0.f, i2 = d2 >= 0.f;
     ClipCase c;
     c.inside = (int)i0 + (int)i1 + (int)i2;
-    c.k0 = 0; c.k1 = 1; c.k2 = 2;
-    if (c.inside == 1) {
-        if (i0) { c.k0 = 0; c.k1 = 1; c.k2 = 2; }
-        else if (i1) { c.k0 = 1; c.k1 = 2; c.k2 = 0; }
-        else { c.k0 = 2; c.k1 = 0; c.k2 = 1; }
-    } else if (c.inside == 2) {
-        if (!i0) { c.k0 = 0; c.k1 = 1; c.k2 = 2; }
-        else if (!i1) { c.k0 = 1; c.k1 = 2; c.k2 = 0; }
-        else { c.k0 = 2; c.k1 = 0; c.k2 = 1; }
-    }
+    c.first = 0;
+    if (c.inside == 1) c.first = i0 ? 0 : i1 ? 1 : 2;
+    if (c.inside == 2) c.first = !i0 ? 0 : !i1 ? 1 : 2;
     return c;
+}
+// (a, b, c) rotated so that element `first` comes first: selects, no indexed array (which would live in local memory).
+template <class T>
+__device__ __forceinline__ void rotate3(int first, T& a, T& b, T& c) {
+    const T x = a, y = b, z = c;
+    if (first == 1) { a = y; b = z; c = x; }
+    if (first == 2) { a = z; b = x; c = y; }
 }
 
 struct SoupVertex { ClipVertex v; float r, g, b, o; };
@@ -63,65 +62,92 @@ __device__ __forceinline__ SoupVertex lerp_vertex(const SoupVertex& a, const Sou
     return n;
 }
 
-__device__ __forceinline__ void store_soup(const SoupVertex& s, int slot, float4* __restrict__ out_vertices,
-                                           float* __restrict__ out_colors, float* __restrict__ out_opacities) {
-    out_vertices[slot] = make_float4(div(s.v.x, s.v.w), div(s.v.y, s.v.w), div(s.v.z, s.v.w), div(1.f, s.v.w));
-    out_colors[3 * (size_t)slot] = s.r; out_colors[3 * (size_t)slot + 1] = s.g; out_colors[3 * (size_t)slot + 2] = s.b;
-    out_opacities[slot] = s.o;
+// The triangle's vertices, rotated, with their signed distances to the near plane.
+struct ClipTriangle {
+    SoupVertex a, b, c;
+    float da, db, dc;
+    int va, vb, vc;
+    int inside;
+};
+__device__ __forceinline__ SoupVertex load_soup(const float* points, const float* colors, const float* opacities, int v,
+                                                const ClipMat& pv) {
+    SoupVertex s;
+    s.v = to_clip(points, v, pv);
+    s.r = colors[3 * (size_t)v]; s.g = colors[3 * (size_t)v + 1]; s.b = colors[3 * (size_t)v + 2];
+    s.o = opacities[v];
+    return s;
+}
+__device__ __forceinline__ ClipTriangle load_clip_triangle(int t, const float* points, const int* indices, const float* colors,
+                                                           const float* opacities, const ClipMat& pv) {
+    ClipTriangle c;
+    c.va = indices[3 * (size_t)t]; c.vb = indices[3 * (size_t)t + 1]; c.vc = indices[3 * (size_t)t + 2];
+    c.a = load_soup(points, colors, opacities, c.va, pv);
+    c.b = load_soup(points, colors, opacities, c.vb, pv);
+    c.c = load_soup(points, colors, opacities, c.vc, pv);
+    c.da = add(c.a.v.z, c.a.v.w); c.db = add(c.b.v.z, c.b.v.w); c.dc = add(c.c.v.z, c.c.v.w);
+    const ClipCase cc = classify(c.da, c.db, c.dc);
+    c.inside = cc.inside;
+    rotate3(cc.first, c.a, c.b, c.c);
+    rotate3(cc.first, c.da, c.db, c.dc);
+    rotate3(cc.first, c.va, c.vb, c.vc);
+    return c;
 }
 
-__device__ __forceinline__ void store_unused(int slot, float4* __restrict__ out_vertices, float* __restrict__ out_colors,
-                                             float* __restrict__ out_opacities) {
-    out_vertices[slot] = make_float4(0.f, 0.f, 0.f, 1.f);
-    out_colors[3 * (size_t)slot] = 0.f; out_colors[3 * (size_t)slot + 1] = 0.f; out_colors[3 * (size_t)slot + 2] = 0.f;
-    out_opacities[slot] = 0.f;
-}
-
-__global__ void __launch_bounds__(256) project_clip_kernel(const float* __restrict__ points, const int* __restrict__ indices,
-                                                           const float* __restrict__ colors,
-                                                           const float* __restrict__ opacities, int T, ClipMat pv,
-                                                           float4* __restrict__ out_vertices, int* __restrict__ out_indices,
-                                                           float* __restrict__ out_colors,
-                                                           float* __restrict__ out_opacities) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= T) return;
-    SoupVertex s[3];
-    float d[3];
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-        const int v = indices[3 * (size_t)t + k];
-        s[k].v = to_clip(points, v, pv);
-        s[k].r = colors[3 * (size_t)v]; s[k].g = colors[3 * (size_t)v + 1]; s[k].b = colors[3 * (size_t)v + 2];
-        s[k].o = opacities[v];
-        d[k] = add(s[k].v.z, s[k].v.w);
+// One thread per input triangle; its six output vertices leave through shared memory, so that the CTA's stores are whole
+// consecutive lines (stored by the threads themselves they were 16 bytes every 96, 4 bytes every 72 and every 24: 82k
+// triangles 24 us).
+constexpr int kClipThreads = 128;
+__global__ void __launch_bounds__(kClipThreads) project_clip_kernel(const float* __restrict__ points,
+                                                                    const int* __restrict__ indices,
+                                                                    const float* __restrict__ colors,
+                                                                    const float* __restrict__ opacities, int T, ClipMat pv,
+                                                                    float4* __restrict__ out_vertices,
+                                                                    int* __restrict__ out_indices,
+                                                                    float* __restrict__ out_colors,
+                                                                    float* __restrict__ out_opacities) {
+    // odd pitches: 7 quads for 6 vertices, 19 words for 18 colour components, 7 words for 6 opacities
+    __shared__ float4 s_v[kClipThreads * 7];
+    __shared__ float s_c[kClipThreads * 19];
+    __shared__ float s_o[kClipThreads * 7];
+    const int tid = threadIdx.x, t0 = blockIdx.x * kClipThreads, n = min(kClipThreads, T - t0);
+    if (tid < n) {
+        auto put = [&](int k, const SoupVertex& s) {
+            s_v[7 * tid + k] = make_float4(div(s.v.x, s.v.w), div(s.v.y, s.v.w), div(s.v.z, s.v.w), div(1.f, s.v.w));
+            s_c[19 * tid + 3 * k] = s.r; s_c[19 * tid + 3 * k + 1] = s.g; s_c[19 * tid + 3 * k + 2] = s.b;
+            s_o[7 * tid + k] = s.o;
+        };
+        auto unused = [&](int k) {
+            s_v[7 * tid + k] = make_float4(0.f, 0.f, 0.f, 1.f);
+            s_c[19 * tid + 3 * k] = s_c[19 * tid + 3 * k + 1] = s_c[19 * tid + 3 * k + 2] = 0.f;
+            s_o[7 * tid + k] = 0.f;
+        };
+        const ClipTriangle c = load_clip_triangle(t0 + tid, points, indices, colors, opacities, pv);
+        if (c.inside == 2) {              // a outside
+            const float t1 = div(c.db, sub(c.db, c.da)), t2 = div(c.dc, sub(c.dc, c.da));
+            const SoupVertex n1 = lerp_vertex(c.b, c.a, t1), n2 = lerp_vertex(c.c, c.a, t2);
+            put(0, c.b); put(1, c.c); put(2, n1);
+            put(3, n1); put(4, c.c); put(5, n2);
+        } else {
+            if (c.inside == 3) {
+                put(0, c.a); put(1, c.b); put(2, c.c);
+            } else if (c.inside == 1) {   // a inside
+                const float t1 = div(c.da, sub(c.da, c.db)), t2 = div(c.da, sub(c.da, c.dc));
+                put(0, c.a); put(1, lerp_vertex(c.a, c.b, t1)); put(2, lerp_vertex(c.a, c.c, t2));
+            } else {
+                unused(0); unused(1); unused(2);
+            }
+            unused(3); unused(4); unused(5);
+        }
     }
-    const int base = 6 * t;
-#pragma unroll
-    for (int k = 0; k < 6; k++) out_indices[base + k] = base + k;
-    const ClipCase cc = classify(d[0], d[1], d[2]);
-    SoupVertex o[6];
-    int used = 0;
-    if (cc.inside == 3) {
-        o[0] = s[0]; o[1] = s[1]; o[2] = s[2];
-        used = 3;
-    } else if (cc.inside == 1) {
-        const SoupVertex& in = s[cc.k0];
-        const float t1 = div(d[cc.k0], sub(d[cc.k0], d[cc.k1])), t2 = div(d[cc.k0], sub(d[cc.k0], d[cc.k2]));
-        o[0] = in; o[1] = lerp_vertex(in, s[cc.k1], t1); o[2] = lerp_vertex(in, s[cc.k2], t2);
-        used = 3;
-    } else if (cc.inside == 2) {
-        const SoupVertex &out = s[cc.k0], &in1 = s[cc.k1], &in2 = s[cc.k2];
-        const float t1 = div(d[cc.k1], sub(d[cc.k1], d[cc.k0])), t2 = div(d[cc.k2], sub(d[cc.k2], d[cc.k0]));
-        const SoupVertex n1 = lerp_vertex(in1, out, t1), n2 = lerp_vertex(in2, out, t2);
-        o[0] = in1; o[1] = in2; o[2] = n1;
-        o[3] = n1; o[4] = in2; o[5] = n2;
-        used = 6;
+    __syncthreads();
+    const size_t first = 6 * (size_t)t0;
+    for (int i = tid; i < 6 * n; i += kClipThreads) {
+        const int r = i / 6, k = i % 6;
+        out_vertices[first + i] = s_v[7 * r + k];
+        out_opacities[first + i] = s_o[7 * r + k];
+        out_indices[first + i] = (int)first + i;
     }
-#pragma unroll
-    for (int k = 0; k < 6; k++) {
-        if (k < used) store_soup(o[k], base + k, out_vertices, out_colors, out_opacities);
-        else store_unused(base + k, out_vertices, out_colors, out_opacities);
-    }
+    for (int i = tid; i < 18 * n; i += kClipThreads) out_colors[3 * first + i] = s_c[19 * (i / 18) + i % 18];
 }
 
 // ---- vector-Jacobian product ---------------------------------------------------------------------
@@ -168,64 +194,49 @@ __global__ void __launch_bounds__(256) project_clip_backward_kernel(
     float* __restrict__ grad_points, float* __restrict__ grad_colors, float* __restrict__ grad_opacities) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= T) return;
-    SoupVertex s[3];
-    float d[3];
-    int vid[3];
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-        const int v = indices[3 * (size_t)t + k];
-        vid[k] = v;
-        s[k].v = to_clip(points, v, pv);
-        s[k].r = colors[3 * (size_t)v]; s[k].g = colors[3 * (size_t)v + 1]; s[k].b = colors[3 * (size_t)v + 2];
-        s[k].o = opacities[v];
-        d[k] = add(s[k].v.z, s[k].v.w);
-    }
-    const ClipCase cc = classify(d[0], d[1], d[2]);
-    if (cc.inside == 0) return;
+    const ClipTriangle c = load_clip_triangle(t, points, indices, colors, opacities, pv);
+    if (c.inside == 0) return;
     const int base = 6 * t;
-    VertexGrad g[3];
-    if (cc.inside == 3) {
-#pragma unroll
-        for (int k = 0; k < 3; k++)
-            add_grad(g[k], load_soup_grad(s[k].v, base + k, grad_out_vertices, grad_out_colors, grad_out_opacities), 1.f);
-    } else if (cc.inside == 1) {
-        const SoupVertex &in = s[cc.k0], &o1 = s[cc.k1], &o2 = s[cc.k2];
-        const float t1 = div(d[cc.k0], sub(d[cc.k0], d[cc.k1])), t2 = div(d[cc.k0], sub(d[cc.k0], d[cc.k2]));
-        const SoupVertex n1 = lerp_vertex(in, o1, t1), n2 = lerp_vertex(in, o2, t2);
-        add_grad(g[cc.k0], load_soup_grad(in.v, base, grad_out_vertices, grad_out_colors, grad_out_opacities), 1.f);
-        lerp_backward(in, o1, d[cc.k0], d[cc.k1], t1,
-                      load_soup_grad(n1.v, base + 1, grad_out_vertices, grad_out_colors, grad_out_opacities), g[cc.k0], g[cc.k1]);
-        lerp_backward(in, o2, d[cc.k0], d[cc.k2], t2,
-                      load_soup_grad(n2.v, base + 2, grad_out_vertices, grad_out_colors, grad_out_opacities), g[cc.k0], g[cc.k2]);
-    } else {
-        const SoupVertex &out = s[cc.k0], &in1 = s[cc.k1], &in2 = s[cc.k2];
-        const float t1 = div(d[cc.k1], sub(d[cc.k1], d[cc.k0])), t2 = div(d[cc.k2], sub(d[cc.k2], d[cc.k0]));
-        const SoupVertex n1 = lerp_vertex(in1, out, t1), n2 = lerp_vertex(in2, out, t2);
-        // soup: (in1, in2, n1), (n1, in2, n2)
-        add_grad(g[cc.k1], load_soup_grad(in1.v, base, grad_out_vertices, grad_out_colors, grad_out_opacities), 1.f);
-        add_grad(g[cc.k2], load_soup_grad(in2.v, base + 1, grad_out_vertices, grad_out_colors, grad_out_opacities), 1.f);
-        add_grad(g[cc.k2], load_soup_grad(in2.v, base + 4, grad_out_vertices, grad_out_colors, grad_out_opacities), 1.f);
-        SoupGrad gn1 = load_soup_grad(n1.v, base + 2, grad_out_vertices, grad_out_colors, grad_out_opacities);
-        const SoupGrad gn1b = load_soup_grad(n1.v, base + 3, grad_out_vertices, grad_out_colors, grad_out_opacities);
-        gn1.x += gn1b.x; gn1.y += gn1b.y; gn1.z += gn1b.z; gn1.w += gn1b.w;
-        gn1.r += gn1b.r; gn1.g += gn1b.g; gn1.b += gn1b.b; gn1.o += gn1b.o;
-        lerp_backward(in1, out, d[cc.k1], d[cc.k0], t1, gn1, g[cc.k1], g[cc.k0]);
-        lerp_backward(in2, out, d[cc.k2], d[cc.k0], t2,
-                      load_soup_grad(n2.v, base + 5, grad_out_vertices, grad_out_colors, grad_out_opacities), g[cc.k2], g[cc.k0]);
+    VertexGrad ga, gb, gc;
+    auto upstream = [&](const ClipVertex& v, int k) {
+        return load_soup_grad(v, base + k, grad_out_vertices, grad_out_colors, grad_out_opacities);
+    };
+    if (c.inside == 3) {
+        add_grad(ga, upstream(c.a.v, 0), 1.f);
+        add_grad(gb, upstream(c.b.v, 1), 1.f);
+        add_grad(gc, upstream(c.c.v, 2), 1.f);
+    } else if (c.inside == 1) {           // a inside
+        const float t1 = div(c.da, sub(c.da, c.db)), t2 = div(c.da, sub(c.da, c.dc));
+        const SoupVertex n1 = lerp_vertex(c.a, c.b, t1), n2 = lerp_vertex(c.a, c.c, t2);
+        add_grad(ga, upstream(c.a.v, 0), 1.f);
+        lerp_backward(c.a, c.b, c.da, c.db, t1, upstream(n1.v, 1), ga, gb);
+        lerp_backward(c.a, c.c, c.da, c.dc, t2, upstream(n2.v, 2), ga, gc);
+    } else {                              // a outside; soup: (b, c, n1), (n1, c, n2)
+        const float t1 = div(c.db, sub(c.db, c.da)), t2 = div(c.dc, sub(c.dc, c.da));
+        const SoupVertex n1 = lerp_vertex(c.b, c.a, t1), n2 = lerp_vertex(c.c, c.a, t2);
+        add_grad(gb, upstream(c.b.v, 0), 1.f);
+        add_grad(gc, upstream(c.c.v, 1), 1.f);
+        add_grad(gc, upstream(c.c.v, 4), 1.f);
+        SoupGrad g1 = upstream(n1.v, 2);
+        const SoupGrad g1b = upstream(n1.v, 3);
+        g1.x += g1b.x; g1.y += g1b.y; g1.z += g1b.z; g1.w += g1b.w;
+        g1.r += g1b.r; g1.g += g1b.g; g1.b += g1b.b; g1.o += g1b.o;
+        lerp_backward(c.b, c.a, c.db, c.da, t1, g1, gb, ga);
+        lerp_backward(c.c, c.a, c.dc, c.da, t2, upstream(n2.v, 5), gc, ga);
     }
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-        const int v = vid[k];
+    auto add_to = [&](int v, const VertexGrad& g) {
         // clip -> world: clip = PV (p, 1)
 #pragma unroll
         for (int j = 0; j < 3; j++)
-            atomicAdd(grad_points + 3 * (size_t)v + j,
-                      g[k].x * pv.m[j] + g[k].y * pv.m[4 + j] + g[k].z * pv.m[8 + j] + g[k].w * pv.m[12 + j]);
-        atomicAdd(grad_colors + 3 * (size_t)v, g[k].r);
-        atomicAdd(grad_colors + 3 * (size_t)v + 1, g[k].g);
-        atomicAdd(grad_colors + 3 * (size_t)v + 2, g[k].b);
-        atomicAdd(grad_opacities + v, g[k].o);
-    }
+            atomicAdd(grad_points + 3 * (size_t)v + j, g.x * pv.m[j] + g.y * pv.m[4 + j] + g.z * pv.m[8 + j] + g.w * pv.m[12 + j]);
+        atomicAdd(grad_colors + 3 * (size_t)v, g.r);
+        atomicAdd(grad_colors + 3 * (size_t)v + 1, g.g);
+        atomicAdd(grad_colors + 3 * (size_t)v + 2, g.b);
+        atomicAdd(grad_opacities + v, g.o);
+    };
+    add_to(c.va, ga);
+    add_to(c.vb, gb);
+    add_to(c.vc, gc);
 }
 
 }  // namespace tg
@@ -243,7 +254,7 @@ int tg_project_clip(const float* points, const int32_t* indices, const float* co
     TG_REQUIRE(((uintptr_t)out_vertices & 15) == 0, "out_vertices must be 16-byte aligned");
     tg::ClipMat pv;
     for (int i = 0; i < 16; i++) pv.m[i] = pv_host[i];
-    tg::project_clip_kernel<<<(T + 255) / 256, 256, 0, (cudaStream_t)stream>>>(
+    tg::project_clip_kernel<<<(T + tg::kClipThreads - 1) / tg::kClipThreads, tg::kClipThreads, 0, (cudaStream_t)stream>>>(
         points, indices, colors, opacities, T, pv, (float4*)out_vertices, out_indices, out_colors, out_opacities);
     TG_LAUNCH_CHECK("project_clip_kernel");
     return TG_OK;
