@@ -587,6 +587,7 @@ __global__ void __launch_bounds__(32 * kBinWarps, 32 / kBinWarps) bin_kernel(con
     __shared__ bool s_last;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const unsigned below = (1u << lane) - 1u;
+    allow_dependents();
     const int per_warp = (per_cta + kBinWarps - 1) / kBinWarps;
     const int t_cta = blockIdx.x * per_cta, t0 = t_cta + warp * per_warp;
     const int ntri = min(min(per_warp, per_cta - warp * per_warp), T - t0);
@@ -753,6 +754,8 @@ __global__ void __launch_bounds__(256) scatter_entries_kernel(const uint4* __res
                                                               int tiles, uint32_t* __restrict__ tile_counts,
                                                               uint32_t* __restrict__ counters, uint32_t* __restrict__ list_heads) {
     __shared__ uint32_t s_hist[33];
+    allow_dependents();
+    await_prerequisites();
     // the binning kernel is done with its counters: zero for the next call
     const uint32_t me = blockIdx.x * 256 + threadIdx.x;
     for (uint32_t i = me; i < (uint32_t)tiles; i += gridDim.x * 256) tile_counts[i] = 0;
@@ -900,8 +903,8 @@ int scatter_entries(const BinBuffers& b, uint32_t list_capacity, const int32_t* 
     // K is not known on the host yet: as many CTAs as its upper bound fills, at most eight per SM, and one for the order
     const uint32_t want = (list_capacity + 1023) / 1024;
     const int grid = (int)(want < 148 * 8 ? want : 148 * 8) + 1;
-    tg::scatter_entries_kernel<<<grid, 256, 0, stream>>>(b.pairs, b.info, list_capacity, offsets, b.entries, b.tile_order, tiles,
-                                                              b.tile_counts, b.counters, b.list_heads);
+    TG_CUDA(launch_dependent(tg::scatter_entries_kernel, grid, 256, 0, stream, b.pairs, b.info, list_capacity, offsets, b.entries,
+                             b.tile_order, tiles, b.tile_counts, b.counters, b.list_heads));
     TG_LAUNCH_CHECK("scatter_entries_kernel");
     return TG_OK;
 }

@@ -616,6 +616,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (SORT ? 4 : 5) : 1) blend_
     __shared__ int s_rank[FUSED ? kFusedList : 1];
     __shared__ int s_list[FUSED ? kFusedList : 1];
     if (FUSED) {
+        await_prerequisites();
         // launched before the host knows: nothing to do when the lists are too long or incomplete
         const uint32_t slots = unsorted.info[2], longest = unsorted.info[1] & ~kOrderWrittenBit;
         if (slots > unsorted.capacity || longest > kFusedList) return;
@@ -1183,6 +1184,7 @@ __global__ void __launch_bounds__(MAXT, DEPTH ? 7 : 8) blend_backward_queued_ker
     PixelGrad pg;
     BackState st;
     float sq = 0.f;
+    allow_dependents();
     const int n = load_pixel_state<DEPTH>(c, P, in, pg, st, &sq);
     const size_t plane = (size_t)P.W * P.H, index = (size_t)c.iy * P.W + c.ix;
     const int lane = lane_id();
@@ -1334,6 +1336,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (SORT ? 3 : 4) : 1) blend_
     const TileCtx c = tile_context(P, s_coord);
     PixelGrad pg;
     BackState st;
+    allow_dependents();
     const int limit = load_pixel_state(c, P, in, pg, st);
 
     if (SORT) {
@@ -1574,6 +1577,7 @@ __global__ void __launch_bounds__(256) unpack_gradients_kernel(float4* __restric
                                                                float* __restrict__ gC, float* __restrict__ gO, int accumulate,
                                                                int clear, float* __restrict__ l2_partials,
                                                                float l2_loss_scale, float* __restrict__ l2_loss_out) {
+    await_prerequisites();
     unpack_loss(l2_partials, l2_loss_scale, l2_loss_out, accumulate != 0, clear != 0);
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= V) return;
@@ -1597,6 +1601,7 @@ __global__ void __launch_bounds__(256) unpack_gradients_rgba_kernel(float4* __re
                                                                     float4* __restrict__ gRGBA, int accumulate, int clear,
                                                                     float* __restrict__ l2_partials, float l2_loss_scale,
                                                                     float* __restrict__ l2_loss_out) {
+    await_prerequisites();
     unpack_loss(l2_partials, l2_loss_scale, l2_loss_out, accumulate != 0, clear != 0);
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= V) return;
@@ -1663,7 +1668,7 @@ int blend_forward_short(const float* tri_geo, const float* tri_attr, const uint6
                                                    : tg::blend_forward_kernel<false, 256, false, true>)
                                  : (per_pixel_sort ? tg::blend_forward_kernel<true, 1024, false, true>
                                                    : tg::blend_forward_kernel<false, 1024, false, true>);
-    kernel<<<tiles, threads, 0, s>>>(P, (float4*)image, depthmap, final_weights, ends, selection, lists);
+    TG_CUDA(launch_dependent(kernel, tiles, threads, 0, s, P, (float4*)image, depthmap, final_weights, ends, selection, lists));
     TG_LAUNCH_CHECK("blend_forward_kernel (short lists)");
     return TG_OK;
 }
@@ -1821,9 +1826,9 @@ int tg_unpack_gradients(void* scratch, size_t scratch_bytes, int V, float loss_s
         return TG_ERR_WORKSPACE;
     }
     float* partials = (float*)((char*)scratch + (size_t)V * 32);
-    tg::unpack_gradients_kernel<<<(V + 255) / 256, 256, 0, (cudaStream_t)stream>>>(
-        (float4*)scratch, V, (float4*)grad_vertices, grad_colors, grad_opacities, accumulate, clear, partials, loss_scale,
-        loss_out);
+    TG_CUDA(tg_host::launch_dependent(tg::unpack_gradients_kernel, (V + 255) / 256, 256, 0, (cudaStream_t)stream, (float4*)scratch,
+                                      V, (float4*)grad_vertices, grad_colors, grad_opacities, accumulate, clear, partials,
+                                      loss_scale, loss_out));
     TG_LAUNCH_CHECK("unpack_gradients_kernel");
     return TG_OK;
 }
@@ -1842,8 +1847,9 @@ int tg_unpack_gradients_rgba(void* scratch, size_t scratch_bytes, int V, float l
         return TG_ERR_WORKSPACE;
     }
     float* partials = (float*)((char*)scratch + (size_t)V * 32);
-    tg::unpack_gradients_rgba_kernel<<<(V + 255) / 256, 256, 0, (cudaStream_t)stream>>>(
-        (float4*)scratch, V, (float4*)grad_vertices, (float4*)grad_rgba, accumulate, clear, partials, loss_scale, loss_out);
+    TG_CUDA(tg_host::launch_dependent(tg::unpack_gradients_rgba_kernel, (V + 255) / 256, 256, 0, (cudaStream_t)stream,
+                                      (float4*)scratch, V, (float4*)grad_vertices, (float4*)grad_rgba, accumulate, clear,
+                                      partials, loss_scale, loss_out));
     TG_LAUNCH_CHECK("unpack_gradients_rgba_kernel");
     return TG_OK;
 }

@@ -138,6 +138,12 @@ __device__ __forceinline__ PixelRect tile_pixel_rect(int tx, int ty, int W, int 
     return R;
 }
 
+// Programmatic dependent launch: a kernel launched with launch_dependent() may start when all CTAs of the kernel before it
+// have started and called allow_dependents(); await_prerequisites() then waits until that kernel is complete and its
+// writes are visible.  Hides the launch latency between two small kernels.  Both do nothing in ordinary launches.
+__device__ __forceinline__ void allow_dependents() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void await_prerequisites() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31u; }
 
 }  // namespace tg
@@ -153,6 +159,20 @@ struct SmemAllowed {
     std::atomic<bool> set[kMaxDevices];
 };
 int allow_smem(const void* kernel, size_t bytes, SmemAllowed& allowed);
+template <class... Params, class... Args>
+cudaError_t launch_dependent(void (*kernel)(Params...), int grid, int block, size_t smem, cudaStream_t stream, Args... args) {
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3((unsigned)grid);
+    config.blockDim = dim3((unsigned)block);
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    cudaLaunchAttribute early;
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = &early;
+    config.numAttrs = 1;
+    return cudaLaunchKernelEx(&config, kernel, Params(args)...);
+}
 }  // namespace tg_host
 
 #define TG_CUDA(call)                                                   \
