@@ -799,7 +799,7 @@ def main() -> None:
 # DRAM bytes (read + write) of one launch of the dominant kernel from an ncu capture of the same kernel on the same
 # workload, with the summary the figure was read from; the kernels may have changed since that capture.
 NCU_DRAM_BYTES = {
-    ("blend_backward_queued_kernel (+ memset, unpack_gradients_kernel)", "cfg3"):
+    ("blend_backward_queued_kernel (+ unpack_gradients_kernel)", "cfg3"):
         (183.2e6 + 11.5e6 + 13.0e6 + 38.4e6, "profiles/blend_kernels_cfg3.md"),
     ("blend_forward_kernel", "cfg3"): (53.1e6 + 45.5e6, "profiles/blend_kernels_cfg3.md"),
     ("blend_forward_kernel", "cfg4"): (256.4e6 + 73.5e6, "profiles/blend_forward_cfg4_view.md"),
@@ -855,18 +855,18 @@ def measure_stages(torch, St, scene, verts_np, flush, reps: int) -> dict:
     K = int(sids.numel())
     fwd = (image, depth, fw, ends, sel)
     res = {}
-    res["init"] = {"kernel": "memset", "ms": med["init"], "bytes": 4 * tiles + 8 * ((T + 255) // 256)}
-    res["binning"] = {"kernel": "preprocess_count_kernel", "ms": med["bary_transforms"],
-                      "bytes": 12 * T + 32 * V + 164 * T + 8 * tiles}
-    res["emit_entries"] = {"kernel": "emit_keys_kernel<direct> (with the read-back of K)", "ms": med["per_tile_lists"],
-                           "bytes": 16 * T + 16 * V + 8 * K + 8 * tiles}
+    res["init"] = {"kernel": "none (interval between two events)", "ms": med["init"], "bytes": 0}
+    res["binning"] = {"kernel": "bin_kernel", "ms": med["bary_transforms"],
+                      "bytes": 12 * T + 32 * V + 164 * T + 16 * K + 8 * tiles}
+    res["emit_entries"] = {"kernel": "scatter_entries_kernel (with the wait for K)", "ms": med["per_tile_lists"],
+                           "bytes": 24 * K + 8 * tiles}
     res["tile_sort"] = {"kernel": "tile_sort_kernel (+ tile_sort_mid_kernel, tile_sort_long_kernel when needed)", "ms": med["sorting"],
                         "bytes": 12 * K + 8 * tiles}
     res["blend_forward"] = {"kernel": "blend_forward_kernel", "ms": med["rasterization"], "bytes": 100 * K + 28 * W * H}
     gi = torch.randn((H, W, 4), device="cuda")
     gd = torch.zeros((H, W), device="cuda")
     ms, _ = timed(lambda: St.blend_backward(sc, geo, attr, sids, offsets, fwd, gi, gd))
-    res["blend_backward"] = {"kernel": "blend_backward_queued_kernel (+ memset, unpack_gradients_kernel)", "ms": ms, "bytes": 100 * K + 48 * W * H + 32 * V}
+    res["blend_backward"] = {"kernel": "blend_backward_queued_kernel (+ unpack_gradients_kernel)", "ms": ms, "bytes": 100 * K + 48 * W * H + 32 * V}
     for s in res.values():
         s["gbs"] = s["bytes"] / (s["ms"] * 1e-3) / 1e9 if s["ms"] > 0 else 0.0
     res["_K"] = K
