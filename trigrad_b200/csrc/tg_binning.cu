@@ -254,8 +254,8 @@ __global__ void __launch_bounds__(256) bin_init_kernel(uint32_t* __restrict__ cl
 // 16 consecutive counts per thread and round, fetched by four independent 16-byte loads one round ahead: the rounds are
 // bound by the latency of those loads.
 constexpr int kBinWarps = 4;         // warps of a CTA of the binning kernel (two and eight: 3 to 7 % slower)
+constexpr int kFinishWarps = 16;      // of the kernel that scans the tile counts after a binning of several waves
 constexpr int kTileScanPer = 16;
-constexpr int kTileScanRound = 32 * kBinWarps * kTileScanPer;
 __device__ __forceinline__ void load_counts(const uint32_t* counts, int first, int tiles, uint4 (&v)[4]) {
 #pragma unroll
     for (int k = 0; k < 4; k++) {
@@ -270,8 +270,10 @@ __device__ __forceinline__ void load_counts(const uint32_t* counts, int first, i
         }
     }
 }
-__device__ uint32_t tile_offsets_by_one_cta(const uint32_t* counts, int32_t* offsets, int tiles, uint32_t* s_warp /*[kBinWarps]*/,
+template <int WARPS>
+__device__ uint32_t tile_offsets_by_one_cta(const uint32_t* counts, int32_t* offsets, int tiles, uint32_t* s_warp /*[WARPS]*/,
                                             uint32_t& total) {
+    constexpr int kTileScanRound = 32 * WARPS * kTileScanPer;
     const int tid = threadIdx.x, warp = tid >> 5;
     uint32_t carry = 0, biggest = 0;
     uint4 ahead[4];
@@ -295,7 +297,7 @@ __device__ uint32_t tile_offsets_by_one_cta(const uint32_t* counts, int32_t* off
         __syncthreads();
         uint32_t run = carry + incl - mine;
 #pragma unroll
-        for (int w = 0; w < kBinWarps; w++) {
+        for (int w = 0; w < WARPS; w++) {
             const uint32_t x = s_warp[w];
             if (w < warp) run += x;
             carry += x;
@@ -322,7 +324,7 @@ __device__ uint32_t tile_offsets_by_one_cta(const uint32_t* counts, int32_t* off
     if (lane_id() == 0) s_warp[warp] = biggest;
     __syncthreads();
 #pragma unroll
-    for (int w = 0; w < kBinWarps; w++) biggest = max(biggest, s_warp[w]);
+    for (int w = 0; w < WARPS; w++) biggest = max(biggest, s_warp[w]);
     return biggest;
 }
 
@@ -540,7 +542,8 @@ struct BinArgs {
     uint4* pairs;            // [capacity]
     uint32_t capacity;
     int tiles, tiles_x, tiles_y;
-    int scan_here;           // 1: the last CTA scans the tile counts; 0: the host launches a scan
+    int scan_here;           // 1: the CTA that finishes the binning scans the tile counts; 0: the host launches a scan
+    int finish_here;         // 1: the last CTA finishes the binning; 0: bin_finish_kernel does
     int want_order;
     TileTables tables;
 };
@@ -567,6 +570,32 @@ __device__ __forceinline__ void write_pair(const BinArgs& bin, const float* tri,
                                  poly, 32 * kBinWarps);
     if (pos < bin.capacity)              // the host checks K before anything that reads the entries is used
         bin.pairs[pos] = make_uint4((uint32_t)t, float_to_ordered(depth), tile, rank);
+}
+
+// After all pairs are counted, by one CTA: tile offsets, K, the longest list, and all of it to the host.
+template <int WARPS>
+__device__ __forceinline__ void finish_binning(const BinArgs& bin, uint32_t* s_warp) {
+    const uint32_t slots = __ldcg(bin.counters + 1);
+    uint32_t K = slots, longest = UINT32_MAX;            // longest: not known
+    if (bin.scan_here) {
+        longest = tile_offsets_by_one_cta<WARPS>(bin.tile_counts, bin.offsets, bin.tiles, s_warp, K);
+        // the launch order costs two passes over the offsets: only for images of at most 16384 tiles whose lists are
+        // long on average and uneven (the longest one at least 256 entries)
+        if (bin.want_order && bin.tiles <= kOrderMaxTiles && K >= kOrderMinMean * (uint32_t)bin.tiles && longest >= kOrderMinLongest)
+            longest |= kOrderWrittenBit;
+    }
+    if (threadIdx.x == 0) {
+        bin.info[0] = K;
+        bin.info[1] = longest;
+        bin.info[2] = slots;
+        if (bin.info_host) {                  // K last: the host watches that word
+            volatile uint32_t* h = bin.info_host;
+            h[1] = longest;
+            h[3] = slots;
+            __threadfence_system();
+            h[0] = K;
+        }
+    }
 }
 
 template <bool CULL>
@@ -715,6 +744,7 @@ __global__ void __launch_bounds__(32 * kBinWarps, 32 / kBinWarps) bin_kernel(con
         write_pair(bin, s_tri[ct >> 5] + (ct & 31), t_cta + (ct >> 5) * per_warp + (ct & 31), tx, ty, slot0 + s_qe[q],
                    __ldg(bin.tables.cols + tx), __ldg(bin.tables.rows + ty), s_poly + tid);
     }
+    if (!bin.finish_here) return;
     __syncthreads();                          // the CTA's counts are issued; one cumulative fence publishes them
     if (tid == 0) {
         __threadfence();
@@ -723,27 +753,15 @@ __global__ void __launch_bounds__(32 * kBinWarps, 32 / kBinWarps) bin_kernel(con
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    const uint32_t slots = __ldcg(bin.counters + 1);
-    uint32_t K = slots, longest = UINT32_MAX;            // longest: not known
-    if (bin.scan_here) {
-        longest = tile_offsets_by_one_cta(bin.tile_counts, bin.offsets, bin.tiles, s_warp, K);
-        // the launch order costs two passes over the offsets: only for images of at most 16384 tiles whose lists are
-        // long on average and uneven (the longest one at least 256 entries)
-        if (bin.want_order && bin.tiles <= kOrderMaxTiles && K >= kOrderMinMean * (uint32_t)bin.tiles && longest >= kOrderMinLongest)
-            longest |= kOrderWrittenBit;
-    }
-    if (tid == 0) {
-        bin.info[0] = K;
-        bin.info[1] = longest;
-        bin.info[2] = slots;
-        if (bin.info_host) {                  // K last: the host watches that word
-            volatile uint32_t* h = bin.info_host;
-            h[1] = longest;
-            h[3] = slots;
-            __threadfence_system();
-            h[0] = K;
-        }
-    }
+    finish_binning<kBinWarps>(bin, s_warp);
+}
+
+// The same as a kernel of its own, after a binning of several waves.
+__global__ void __launch_bounds__(32 * kFinishWarps) bin_finish_kernel(BinArgs bin) {
+    __shared__ uint32_t s_warp[kFinishWarps];
+    allow_dependents();
+    await_prerequisites();
+    finish_binning<kFinishWarps>(bin, s_warp);
 }
 
 // Every entry to its place: offset of its tile plus its rank there.  The last CTA makes the launch order of the
@@ -873,13 +891,18 @@ int bin_triangles(const float* vertices, const int32_t* indices, const float* co
         TG_CUDA(cudaMemsetAsync(offsets, 0, sizeof(int32_t) * ((size_t)tiles + 1), stream));
         return TG_OK;
     }
-    const tg::BinArgs bin = {b.tile_counts, offsets, b.counters, b.info, info_host, b.pairs, list_capacity, tiles, tiles_x,
-                             tiles_y, by_last_cta ? 1 : 0, b.tile_order ? 1 : 0, {b.tables, rows}};
     // Triangles per CTA: 32 per warp where that fills the GPU; fewer below, so that a mesh of few triangles that cover many
     // tiles each still spreads over all SMs (eight CTAs on each).
     constexpr int kWave = 148 * 32 / tg::kBinWarps;
     const int per_cta = T >= 32 * tg::kBinWarps * kWave ? 32 * tg::kBinWarps : (T + kWave - 1) / kWave;
     const int grid = (T + per_cta - 1) / per_cta;
+    // A grid of one wave is finished by its last CTA, which saves a launch (where there are few triangles both take the same).
+    // Beyond, the barrier, fence and atomic at the end of every CTA hold its slot for longer than a dependent launch
+    // takes, and sixteen warps scan the counts faster than four (1.3M triangles: 158 us against 141 and the scan, a step
+    // 620 against 613; 200k triangles, full HD, a view: 164.3 against 162.7).
+    constexpr int kFinishHere = kWave;
+    const tg::BinArgs bin = {b.tile_counts, offsets, b.counters, b.info, info_host, b.pairs, list_capacity, tiles, tiles_x,
+                             tiles_y, by_last_cta ? 1 : 0, grid <= kFinishHere ? 1 : 0, b.tile_order ? 1 : 0, {b.tables, rows}};
     auto inverse = [](int n) { return (n & (n - 1)) == 0 ? 1.0 / n : 0.0; };
     auto kernel = cull ? tg::bin_kernel<true> : tg::bin_kernel<false>;
     static SmemAllowed allowed[2];
@@ -888,6 +911,10 @@ int bin_triangles(const float* vertices, const int32_t* indices, const float* co
                                                     tw, th, inverse(tw), inverse(th), (float4*)tri_geo, (float4*)tri_attr,
                                                     bin, packed ? 1 : 0);
     TG_LAUNCH_CHECK("bin_kernel");
+    if (!bin.finish_here) {
+        TG_CUDA(launch_dependent(tg::bin_finish_kernel, 1, 32 * tg::kFinishWarps, 0, stream, bin));
+        TG_LAUNCH_CHECK("bin_finish_kernel");
+    }
     if (!by_last_cta) {
         const int parts = (tiles + tg::kScanTile - 1) / tg::kScanTile;
         tg::scan_kernel<<<parts, tg::kScanThreads, 0, stream>>>(b.tile_counts, (uint32_t*)offsets, tiles, parts,
