@@ -199,15 +199,29 @@ __device__ __forceinline__ void stage_chunk(const BlendParams& P, int first, int
     }
 }
 
-// The attribute quads the forward blend needs (opacities, colours, 1/w: the first four of the six), staged next to
-// the geometry when the whole tile list fits in one chunk: the blend of the selected fragments then reads its
-// records from shared memory instead of gathering 128 bytes per fragment and lane through L1.  Same 80-byte pitch.
-__device__ __forceinline__ void stage_attr_chunk(const BlendParams& P, int first, int n, float4* s_attr) {
+// 16-byte asynchronous copy global -> shared (completion awaited with cp_async_wait_all by the issuing thread, then
+// made visible to the CTA by a barrier).
+__device__ __forceinline__ void cp_async16(float4* smem_dst, const float4* gmem_src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem_dst)),
+                 "l"(gmem_src));
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+
+// A whole list of at most one chunk, and with it the attribute quads the forward blend needs (opacities, colours, 1/w: the
+// first four of the six): the blend of the selected fragments then reads its records from shared memory instead of
+// gathering 128 bytes per fragment and lane through L1.  Asynchronous, started as soon as the list is known and awaited
+// behind the set-up of the pixels: two load-then-store loops behind that and a barrier were up to four trips to L2 in a row
+// in the life of a CTA of some ten (200k triangles, full HD: forward kernel 109 -> 99 us).  Same 80-byte pitch.
+__device__ __forceinline__ void stage_list_async(const BlendParams& P, int first, int n, float4* s_geo, float4* s_attr, int* s_id) {
     for (int i = threadIdx.x; i < n * 4; i += blockDim.x) {
         const int rec = i >> 2, q = i & 3;
         const int id = P.ids[first + rec];
-        s_attr[staged_quad(rec, q)] = __ldg(P.attr + kAttrQuads * (size_t)id + q);
+        if (q == 0) s_id[rec] = id;
+        cp_async16(s_geo + staged_quad(rec, q), P.geo + 4 * (size_t)id + q);
+        cp_async16(s_attr + staged_quad(rec, q), P.attr + kAttrQuads * (size_t)id + q);
     }
+    cp_async_commit();
 }
 __device__ __forceinline__ AttrRec staged_attr(const float4* s_attr, int r) {
     const float4 q0 = s_attr[staged_quad(r, 0)], q1 = s_attr[staged_quad(r, 1)], q2 = s_attr[staged_quad(r, 2)],
@@ -254,15 +268,6 @@ __device__ __forceinline__ unsigned long long warp_cull(const float4* s_geo, int
     const unsigned m0 = __ballot_sync(0xffffffffu, k0), m1 = __ballot_sync(0xffffffffu, k1);
     return (unsigned long long)m0 | ((unsigned long long)m1 << 32);
 }
-
-// 16-byte asynchronous copy global -> shared (completion awaited with cp_async_wait_all by the issuing thread, then
-// made visible to the CTA by a barrier).
-__device__ __forceinline__ void cp_async16(float4* smem_dst, const float4* gmem_src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem_dst)),
-                 "l"(gmem_src));
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
 // The nearest fragments a pixel has collected in a sweep: at most `bs` words (ordered depth << 32 | list position),
 // ascending.  One word per fragment, because the array lives in local memory.
@@ -426,7 +431,7 @@ __device__ __forceinline__ void process_chunk(const TileCtx& c, bool go, int bs,
     }
 }
 
-// Shared memory of a sweep.  `attr`, when given, receives the attribute quads of the chunk as well (stage_attr_chunk).
+// Shared memory of a sweep.  `staged`: the list is one chunk and in `geo` and `id` already.
 // `geo2` / `id2`, when given, are a second pair of staging buffers: a list of more than one chunk is then streamed
 // (CTAs of 256 threads: one quad per thread and chunk) - the records of chunk k + 1 travel by asynchronous copies
 // while chunk k is processed, their ids having been fetched one iteration earlier still, and one barrier per chunk
@@ -442,7 +447,7 @@ struct SweepSmem {
     float4* geo;
     int* id;
     SweepScratch* scratch;
-    float4* attr;
+    bool staged;
     float4* geo2;
     int* id2;
 };
@@ -561,7 +566,7 @@ __device__ __forceinline__ void select_sweep(const BlendParams& P, const TileCtx
                 const int first2 = first + 2 * kChunk;
                 id_ahead = (first2 < c.end && my_rec < c.end - first2) ? P.ids[first2 + my_rec] : -1;
             }
-        } else {
+        } else if (!sm.staged) {
             if (!FILTER) {
                 __syncthreads();
             } else if (__syncthreads_and(full) && c.end - first > kChunk) {
@@ -569,7 +574,6 @@ __device__ __forceinline__ void select_sweep(const BlendParams& P, const TileCtx
                 break;
             }
             stage_chunk(P, first, n, sm.geo, sm.id);
-            if (sm.attr) stage_attr_chunk(P, first, n, sm.attr);
             __syncthreads();
         }
         if (warp_go) process_chunk(c, go, bs, last, s, dense, geo_now, n, first, nullptr, s_slot);
@@ -622,7 +626,8 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (SORT ? 4 : 5) : 1) blend_
         if (slots > unsorted.capacity || longest > kFusedList) return;
     }
     const int this_tile = tile_of_block(P);
-    if (P.offsets[this_tile] == P.offsets[this_tile + 1]) {
+    const int list_first = P.offsets[this_tile], list_n = P.offsets[this_tile + 1] - list_first;
+    if (list_n == 0) {
         // a tile without entries: background, and no need for pixel-centre coordinates (any pixel order will do)
         const int tx = this_tile % P.tiles_x, ty = this_tile / P.tiles_x;
         const int ix = tx * P.tw + (int)threadIdx.x % P.tw, iy = ty * P.th + (int)threadIdx.x / P.tw;
@@ -635,12 +640,14 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (SORT ? 4 : 5) : 1) blend_
         }
         return;
     }
+    const bool one_chunk = SORT && list_n <= kChunk;
     if (FUSED) {
-        const int first = P.offsets[this_tile], n = P.offsets[this_tile + 1] - first;
-        for (int i = threadIdx.x; i < n; i += blockDim.x) {
-            s_key[i] = unsorted.entries[first + i];
+        for (int i = threadIdx.x; i < list_n; i += blockDim.x) {
+            s_key[i] = unsorted.entries[list_first + i];
             s_rank[i] = 0;
         }
+    } else if (one_chunk) {
+        stage_list_async(P, list_first, list_n, s_geo, s_attr, s_id);
     }
     const TileCtx c = tile_context(P, s_coord);      // its barrier makes the words above visible
     if (FUSED) {
@@ -664,6 +671,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (SORT ? 4 : 5) : 1) blend_
         }
         P.ids = s_list - c.start;
         __syncthreads();
+        if (one_chunk) stage_list_async(P, c.start, n, s_geo, s_attr, s_id);
     }
     PixelAcc acc;
 
@@ -674,16 +682,11 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (SORT ? 4 : 5) : 1) blend_
         const size_t plane = (size_t)P.W * P.H, index = (size_t)c.iy * P.W + c.ix;
         while (true) {
             const bool go = want && acc.alpha > P.thr && acc.blended < P.max_layers;
+            cp_async_wait_all();                       // a list of one chunk; visible to all behind the barrier
             if (!__syncthreads_or(go)) break;
             const int bs = min(kBatchLayers, P.max_layers - acc.blended);
-            // A list of one chunk is still in shared memory after the sweep, and then its attribute quads were staged
-            // with it (while the geometry loads were in flight anyway): the blend reads its records from shared memory
-            // instead of gathering 128 bytes per fragment and lane through L1.  (Deciding after the sweep, from the
-            // number of pixels that found something, whether staging the attributes pays was slower: the loads then
-            // wait alone behind a barrier.)
-            const bool one_chunk = c.end - c.start <= kChunk;
             select_sweep<STREAM, (STREAM || MAXT > 256) && !FUSED>(P, c, go, bs, last, batch,
-                                 {s_geo, s_id, &s_scratch, one_chunk ? s_attr : nullptr, one_chunk ? nullptr : s_attr, s_id2});
+                                 {s_geo, s_id, &s_scratch, one_chunk, one_chunk ? nullptr : s_attr, s_id2});
             const int found = batch.found;
             if (go) {
                 const int n = min(found, P.max_layers - acc.blended);
@@ -1260,7 +1263,7 @@ __global__ void __launch_bounds__(MAXT, 4) blend_step_l2_kernel(BlendParams P, f
         const bool go = c.active && acc.alpha > P.thr && P.max_layers > 0;
         if (__syncthreads_or(go)) {
             const int bs = min(kBatchLayers, P.max_layers);
-            select_sweep(P, c, go, bs, 0, batch, {s_geo, s_id, &s_scratch, nullptr, nullptr, nullptr});
+            select_sweep(P, c, go, bs, 0, batch, {s_geo, s_id, &s_scratch, false, nullptr, nullptr});
             if (go) {
                 n = min(batch.found, P.max_layers);
                 for (int i = 0; i < n; i++) {
@@ -1348,7 +1351,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (SORT ? 3 : 4) : 1) blend_
             const bool go = remaining > 0;
             if (!__syncthreads_or(go)) break;
             const int bs = min(kBatchLayers, remaining);
-            select_sweep(P, c, go, bs, last, batch, {s_geo, s_id, &s_scratch, nullptr, nullptr, nullptr});
+            select_sweep(P, c, go, bs, last, batch, {s_geo, s_id, &s_scratch, false, nullptr, nullptr});
             const int n = go ? min(batch.found, remaining) : 0;
             const int rounds = __reduce_max_sync(0xffffffffu, n);
             // back to front inside the batch (reference render.cu:684-688); the first of the rounds starts at every lane's
@@ -1492,7 +1495,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (SORT ? 3 : 4) : 1) blend_
             const bool go = remaining > 0;
             if (!__syncthreads_or(go)) break;
             const int bs = min(kBatchLayers, remaining);
-            select_sweep(P, c, go, bs, last, batch, {s_geo, s_id, &s_scratch, nullptr, nullptr, nullptr});
+            select_sweep(P, c, go, bs, last, batch, {s_geo, s_id, &s_scratch, false, nullptr, nullptr});
             const int n = go ? min(batch.found, remaining) : 0;
             const int rounds = __reduce_max_sync(0xffffffffu, n);
             for (int i = 0; i < rounds; ++i) {
