@@ -617,6 +617,7 @@ __global__ void __launch_bounds__(32 * kBinWarps, 32 / kBinWarps) bin_kernel(con
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const unsigned below = (1u << lane) - 1u;
     allow_dependents();
+    await_prerequisites();
     const int per_warp = (per_cta + kBinWarps - 1) / kBinWarps;
     const int t_cta = blockIdx.x * per_cta, t0 = t_cta + warp * per_warp;
     const int ntri = min(min(per_warp, per_cta - warp * per_warp), T - t0);
@@ -907,9 +908,9 @@ int bin_triangles(const float* vertices, const int32_t* indices, const float* co
     auto kernel = cull ? tg::bin_kernel<true> : tg::bin_kernel<false>;
     static SmemAllowed allowed[2];
     if (int st = allow_smem((const void*)kernel, tg::kBinSmem, allowed[cull ? 1 : 0])) return st;
-    kernel<<<grid, 32 * tg::kBinWarps, tg::kBinSmem, stream>>>((const float4*)vertices, indices, colors, opacities, T, per_cta, W, H,
-                                                    tw, th, inverse(tw), inverse(th), (float4*)tri_geo, (float4*)tri_attr,
-                                                    bin, packed ? 1 : 0);
+    TG_CUDA(launch_dependent(kernel, grid, 32 * tg::kBinWarps, tg::kBinSmem, stream, (const float4*)vertices, indices, colors,
+                             opacities, T, per_cta, W, H, tw, th, inverse(tw), inverse(th), (float4*)tri_geo, (float4*)tri_attr,
+                             bin, packed ? 1 : 0));
     TG_LAUNCH_CHECK("bin_kernel");
     if (!bin.finish_here) {
         TG_CUDA(launch_dependent(tg::bin_finish_kernel, 1, 32 * tg::kFinishWarps, 0, stream, bin));

@@ -653,8 +653,9 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (SORT ? 4 : 5) : 1) blend_
     __shared__ uint64_t s_key[FUSED ? kFusedList : 1];
     __shared__ int s_rank[FUSED ? kFusedList : 1];
     __shared__ int s_list[FUSED ? kFusedList : 1];
+    allow_dependents();
+    await_prerequisites();
     if (FUSED) {
-        await_prerequisites();
         // launched before the host knows: nothing to do when the lists are too long or incomplete
         const uint32_t slots = unsorted.info[2], longest = unsorted.info[1] & ~kOrderWrittenBit;
         if (slots > unsorted.capacity || longest > kFusedList) return;
@@ -1224,11 +1225,12 @@ __global__ void __launch_bounds__(MAXT, DEPTH ? 7 : 8) blend_backward_queued_ker
     static_assert(MAXT % 32 == 0 && MAXT <= 256, "one queue per warp, at most 8 warps");
     __shared__ __align__(16) float s_coord[MAXT + 2];      // tile_w + tile_h <= tile_w * tile_h + 1 <= MAXT + 1
     __shared__ float4 s_queue[MAXT / 32][kQueueQuads];
+    allow_dependents();
+    await_prerequisites();
     const TileCtx c = tile_context(P, s_coord);
     PixelGrad pg;
     BackState st;
     float sq = 0.f;
-    allow_dependents();
     const int n = load_pixel_state<DEPTH>(c, P, in, pg, st, &sq);
     const size_t plane = (size_t)P.W * P.H, index = (size_t)c.iy * P.W + c.ix;
     const int lane = lane_id();
@@ -1630,6 +1632,7 @@ __global__ void __launch_bounds__(256) unpack_gradients_kernel(float4* __restric
                                                                float* __restrict__ gC, float* __restrict__ gO, int accumulate,
                                                                int clear, float* __restrict__ l2_partials,
                                                                float l2_loss_scale, float* __restrict__ l2_loss_out) {
+    allow_dependents();
     await_prerequisites();
     unpack_loss(l2_partials, l2_loss_scale, l2_loss_out, accumulate != 0, clear != 0);
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1654,6 +1657,7 @@ __global__ void __launch_bounds__(256) unpack_gradients_rgba_kernel(float4* __re
                                                                     float4* __restrict__ gRGBA, int accumulate, int clear,
                                                                     float* __restrict__ l2_partials, float l2_loss_scale,
                                                                     float* __restrict__ l2_loss_out) {
+    allow_dependents();
     await_prerequisites();
     unpack_loss(l2_partials, l2_loss_scale, l2_loss_out, accumulate != 0, clear != 0);
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1743,16 +1747,17 @@ int tg_blend_forward(const float* tri_geo, const float* tri_attr, const int32_t*
     const int threads = ((tw * th + 31) / 32) * 32;
     cudaStream_t s = (cudaStream_t)stream;
     float4* img = (float4*)image;
-    if (threads <= 256) {
-        // lists well beyond one staged chunk (the binning kernel of the same call reported the longest): stream them
-        if (per_pixel_sort && threads == 256 && tg_host::g_longest_list > 2u * tg::kChunk)
-            tg::blend_forward_kernel<true, 256, true><<<tiles, threads, 0, s>>>(P, img, depthmap, final_weights, ends, selection, {});
-        else if (per_pixel_sort) tg::blend_forward_kernel<true, 256><<<tiles, threads, 0, s>>>(P, img, depthmap, final_weights, ends, selection, {});
-        else tg::blend_forward_kernel<false, 256><<<tiles, threads, 0, s>>>(P, img, depthmap, final_weights, ends, nullptr, {});
-    } else {
-        if (per_pixel_sort) tg::blend_forward_kernel<true, 1024><<<tiles, threads, 0, s>>>(P, img, depthmap, final_weights, ends, selection, {});
-        else tg::blend_forward_kernel<false, 1024><<<tiles, threads, 0, s>>>(P, img, depthmap, final_weights, ends, nullptr, {});
-    }
+    // lists well beyond one staged chunk (the binning kernel of the same call reported the longest): stream them
+    const bool stream_lists = threads == 256 && tg_host::g_longest_list > 2u * tg::kChunk;
+    auto kernel = threads > 256 ? (per_pixel_sort ? tg::blend_forward_kernel<true, 1024> : tg::blend_forward_kernel<false, 1024>)
+                  : !per_pixel_sort ? tg::blend_forward_kernel<false, 256>
+                  : stream_lists ? tg::blend_forward_kernel<true, 256, true> : tg::blend_forward_kernel<true, 256>;
+    // Launched ahead of the end of the sort (200k triangles, full HD: a view 152 -> 146 us together with the sort's own early
+    // launch), but only behind the kernel for short lists: CTAs that come to an SM while a sort kernel with much shared
+    // memory is still there run with what L1 that leaves, and as the SM is never empty, to the end (2M triangles, 4K: 611 ->
+    // 917 us; lists of up to 1024 entries, 400k triangles, full HD: 486 -> 537).
+    TG_CUDA(tg_host::launch_early(tg_host::g_longest_list <= (uint32_t)tg::kTileSortRank, kernel, tiles, threads, 0, s, P, img, depthmap, final_weights, ends,
+                                      per_pixel_sort ? selection : nullptr, tg::UnsortedLists{}));
     TG_LAUNCH_CHECK("blend_forward_kernel");
     return TG_OK;
 }
@@ -1805,8 +1810,8 @@ static int backward_impl(const float* tri_geo, const float* tri_attr, const int3
         Q.tiles_x = (W + Q.tw - 1) / Q.tw;
         Q.offsets = nullptr; Q.ids = nullptr; Q.order = nullptr;
         const int blocks = Q.tiles_x * ((H + Q.th - 1) / Q.th);
-        if (grad_depthmap) tg::blend_backward_queued_kernel<128, true><<<blocks, 128, 0, s>>>(Q, in, selection, gpack);
-        else tg::blend_backward_queued_kernel<128, false><<<blocks, 128, 0, s>>>(Q, in, selection, gpack);
+        auto kernel = grad_depthmap ? tg::blend_backward_queued_kernel<128, true> : tg::blend_backward_queued_kernel<128, false>;
+        TG_CUDA(tg_host::launch_dependent(kernel, blocks, 128, 0, s, Q, in, selection, gpack));
     } else if (threads <= 256) {
         if (per_pixel_sort) tg::blend_backward_kernel<true, 256><<<tiles, threads, 0, s>>>(P, in, gpack);
         else tg::blend_backward_kernel<false, 256><<<tiles, threads, 0, s>>>(P, in, gpack);

@@ -159,19 +159,24 @@ struct SmemAllowed {
     std::atomic<bool> set[kMaxDevices];
 };
 int allow_smem(const void* kernel, size_t bytes, SmemAllowed& allowed);
+// `early`: as a dependent launch.
 template <class... Params, class... Args>
-cudaError_t launch_dependent(void (*kernel)(Params...), int grid, int block, size_t smem, cudaStream_t stream, Args... args) {
+cudaError_t launch_early(bool early, void (*kernel)(Params...), int grid, int block, size_t smem, cudaStream_t stream, Args... args) {
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3((unsigned)grid);
     config.blockDim = dim3((unsigned)block);
     config.dynamicSmemBytes = smem;
     config.stream = stream;
-    cudaLaunchAttribute early;
-    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    early.val.programmaticStreamSerializationAllowed = 1;
-    config.attrs = &early;
-    config.numAttrs = 1;
+    cudaLaunchAttribute serial;
+    serial.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    serial.val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = &serial;
+    config.numAttrs = early ? 1 : 0;
     return cudaLaunchKernelEx(&config, kernel, Params(args)...);
+}
+template <class... Params, class... Args>
+cudaError_t launch_dependent(void (*kernel)(Params...), int grid, int block, size_t smem, cudaStream_t stream, Args... args) {
+    return launch_early(true, kernel, grid, block, smem, stream, args...);
 }
 }  // namespace tg_host
 

@@ -11,6 +11,8 @@ struct Mat4 { float m[16]; };   // row-major
 
 __global__ void __launch_bounds__(256) project_kernel(const float* __restrict__ points, int V, Mat4 pv,
                                                       float4* __restrict__ vertices) {
+    allow_dependents();
+    await_prerequisites();
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= V) return;
     const float x = points[3 * (size_t)v], y = points[3 * (size_t)v + 1], z = points[3 * (size_t)v + 2];
@@ -56,6 +58,8 @@ __global__ void __launch_bounds__(256) unpack_project_backward_kernel(float4* __
                                                                       float* __restrict__ grad_opacities,
                                                                       float* __restrict__ partials, float loss_scale,
                                                                       float* __restrict__ loss_out) {
+    allow_dependents();
+    await_prerequisites();
     if (blockIdx.x == 0 && threadIdx.x < 32) {
         float x = partials[threadIdx.x] + partials[threadIdx.x + 32];
         partials[threadIdx.x] = 0.f;
@@ -98,7 +102,8 @@ int tg_project(const float* points, int V, const float* pv_host, float* vertices
     TG_REQUIRE(((uintptr_t)vertices & 15) == 0, "vertices must be 16-byte aligned");
     tg::Mat4 pv;
     for (int i = 0; i < 16; i++) pv.m[i] = pv_host[i];
-    tg::project_kernel<<<(V + 255) / 256, 256, 0, (cudaStream_t)stream>>>(points, V, pv, (float4*)vertices);
+    TG_CUDA(tg_host::launch_dependent(tg::project_kernel, (V + 255) / 256, 256, 0, (cudaStream_t)stream, points, V, pv,
+                                      (float4*)vertices));
     TG_LAUNCH_CHECK("project_kernel");
     return TG_OK;
 }
@@ -130,8 +135,9 @@ int tg_unpack_project_backward(void* scratch, size_t scratch_bytes, int V, const
     tg::Mat4 pv;
     for (int i = 0; i < 16; i++) pv.m[i] = pv_host[i];
     float* partials = (float*)((char*)scratch + (size_t)V * 32);
-    tg::unpack_project_backward_kernel<<<(V + 255) / 256, 256, 0, (cudaStream_t)stream>>>(
-        (float4*)scratch, V, points, pv, grad_points, grad_colors, grad_opacities, partials, loss_scale, loss_out);
+    TG_CUDA(tg_host::launch_dependent(tg::unpack_project_backward_kernel, (V + 255) / 256, 256, 0, (cudaStream_t)stream,
+                                      (float4*)scratch, V, points, pv, grad_points, grad_colors, grad_opacities, partials,
+                                      loss_scale, loss_out));
     TG_LAUNCH_CHECK("unpack_project_backward_kernel");
     return TG_OK;
 }

@@ -20,6 +20,8 @@ constexpr int kHistDoneWord = 8;
 constexpr int kTileScanByLastCta = 65536;
 // Top bit of the longest-list word the binning kernel reports: a launch order of the tiles was written.
 constexpr uint32_t kOrderWrittenBit = 0x80000000u;
+// Longest tile list that a warp sorts (tile_sort_kernel alone).
+constexpr int kTileSortRank = 128;
 // Longest tile list that the compositing kernel sorts itself, in images of at most kFusedTiles tiles: two waves of its
 // CTAs.  There a launch and a trip through memory count (1280 triangles, 256x256: 36 -> 27 us with the early launch); with
 // many waves the sort inside takes more of the SMs' time than the kernel of its own does (200k triangles, 1920x1080: 124 us

@@ -23,7 +23,6 @@ namespace tg {
 
 constexpr int kTileSortWarps = 4;                      // tiles per CTA of the short kernel
 constexpr int kTileSortThreads = 32 * kTileSortWarps;
-constexpr int kTileSortRank = 128;
 constexpr int kTileSortShort = 1024;
 constexpr int kTileSortLongThreads = 1024;
 constexpr int kTileSortChunk = 16384;
@@ -371,6 +370,8 @@ __global__ void __launch_bounds__(kTileSortThreads) tile_sort_kernel(uint64_t* _
                                                                      int32_t* __restrict__ sorted_ids,
                                                                      uint32_t* __restrict__ lists, int write_back) {
     __shared__ uint64_t s_all[kTileSortWarps][kTileSortRank];
+    allow_dependents();
+    await_prerequisites();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int tile = blockIdx.x * kTileSortWarps + warp;
     if (tile >= tiles) return;
@@ -396,6 +397,8 @@ __global__ void __launch_bounds__(kTileSortThreads) tile_sort_mid_kernel(uint64_
                                                                          const int32_t* __restrict__ offsets, int tiles,
                                                                          int32_t* __restrict__ sorted_ids, uint32_t* lists,
                                                                          int write_back) {
+    allow_dependents();
+    await_prerequisites();
     __shared__ uint64_t s_mid[kMidSmemWords];
     __shared__ uint32_t s_count[kTileSortShort + 1], s_cell[kCells + 2], s_warp[32];
     __shared__ uint32_t s_item;
@@ -446,6 +449,8 @@ template <bool BIG>
 __global__ void __launch_bounds__(kTileSortLongThreads, BIG ? 1 : 2)
     tile_sort_long_kernel(uint64_t* entries, const int32_t* __restrict__ offsets, int32_t* __restrict__ sorted_ids,
                           uint32_t* lists, int write_back) {
+    allow_dependents();
+    await_prerequisites();
     extern __shared__ __align__(16) uint64_t s_long[];
     uint32_t* s_count = reinterpret_cast<uint32_t*>(s_long + (BIG ? kTileSortBig : kTileSortHalf + (kTileSortHalf >> 3)));
     __shared__ uint32_t s_item, s_cell[kCells + 2], s_warp[32];
@@ -520,20 +525,20 @@ int sort_tile_lists(uint64_t* entries, const int32_t* offsets, int tiles, int32_
     if (tiles == 0) return TG_OK;
     TG_REQUIRE(entries && offsets && sorted_ids && lists, "null pointer");
     if (!scratch_prepared) TG_CUDA(cudaMemsetAsync(lists, 0, tg::kListHead * sizeof(uint32_t), s));
-    tg::tile_sort_kernel<<<(tiles + tg::kTileSortWarps - 1) / tg::kTileSortWarps, tg::kTileSortThreads, 0, s>>>(
-        entries, offsets, tiles, sorted_ids, lists, write_back ? 1 : 0);
+    TG_CUDA(launch_dependent(tg::tile_sort_kernel, (tiles + tg::kTileSortWarps - 1) / tg::kTileSortWarps, tg::kTileSortThreads, 0, s,
+                             entries, offsets, tiles, sorted_ids, lists, write_back ? 1 : 0));
     TG_LAUNCH_CHECK("tile_sort_kernel");
     if (longest > (uint32_t)tg::kTileSortRank) {
         const int grid = tiles < 148 * 12 ? tiles : 148 * 12;
-        tg::tile_sort_mid_kernel<<<grid, tg::kTileSortThreads, 0, s>>>(entries, offsets, tiles, sorted_ids, lists,
-                                                                        write_back ? 1 : 0);
+        TG_CUDA(launch_dependent(tg::tile_sort_mid_kernel, grid, tg::kTileSortThreads, 0, s, entries, offsets, tiles, sorted_ids,
+                                 lists, write_back ? 1 : 0));
         TG_LAUNCH_CHECK("tile_sort_mid_kernel");
     }
     auto launch_long = [&](auto kernel, bool big, int ctas, SmemAllowed& allowed) -> int {
         const size_t smem = tg::long_smem_bytes(big);
         if (int st = allow_smem((const void*)kernel, smem, allowed)) return st;
-        kernel<<<tiles < ctas ? tiles : ctas, tg::kTileSortLongThreads, smem, s>>>(entries, offsets, sorted_ids, lists,
-                                                                                 write_back ? 1 : 0);
+        TG_CUDA(launch_dependent(kernel, tiles < ctas ? tiles : ctas, tg::kTileSortLongThreads, smem, s, entries, offsets,
+                                 sorted_ids, lists, write_back ? 1 : 0));
         TG_LAUNCH_CHECK("tile_sort_long_kernel");
         return TG_OK;
     };
