@@ -864,6 +864,17 @@ int allow_smem(const void* kernel, size_t bytes, SmemAllowed& allowed) {
     return TG_OK;
 }
 
+int prefer_smem(const void* kernel, int kilobytes, SmemAllowed& preferred) {
+    int dev = 0;
+    TG_CUDA(cudaGetDevice(&dev));
+    TG_REQUIRE(dev >= 0 && dev < SmemAllowed::kMaxDevices, "device index outside the supported range");
+    if (!preferred.set[dev].load(std::memory_order_acquire)) {
+        TG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, kilobytes * 100 / 228));
+        preferred.set[dev].store(true, std::memory_order_release);
+    }
+    return TG_OK;
+}
+
 // Per-triangle records, (triangle, tile) pairs and tile offsets: bin_init_kernel, bin_kernel and scatter_entries_kernel
 // (declared in tg_common.cuh with what each argument is).
 int bin_triangles(const float* vertices, const int32_t* indices, const float* colors, const float* opacities, int T, int W,

@@ -472,12 +472,12 @@ struct SweepScratch {
     uint16_t keep[kFilterBatch];     // entries of a filtered batch, as offsets
     int j[kChunk];                   // list positions of a filtered chunk
     uint32_t count[33];              // per warp and quarter of a batch
-    uint8_t slot[32][64];            // per warp, see process_chunk
 };
 struct SweepSmem {
     float4* geo;
     int* id;
-    SweepScratch* scratch;
+    SweepScratch* scratch;     // of sweep_filtered
+    uint8_t* slots;            // 64 per warp, see process_chunk
     bool staged;
     float4* geo2;
     int* id2;
@@ -544,7 +544,7 @@ __device__ __forceinline__ void sweep_filtered(const BlendParams& P, const TileC
                 sm.geo[staged_quad(rec, q)] = __ldg(P.geo + 4 * (size_t)id + q);
             }
             __syncthreads();
-            if (warp_go) process_chunk(c, go, bs, last, s, dense, sm.geo, n, 0, x.j, x.slot[warp]);
+            if (warp_go) process_chunk(c, go, bs, last, s, dense, sm.geo, n, 0, x.j, sm.slots + 64 * warp);
             __syncthreads();
         }
     }
@@ -561,7 +561,7 @@ __device__ __forceinline__ void select_sweep(const BlendParams& P, const TileCtx
     s.dfar = -INFINITY;
     bool dense = false;         // see process_chunk
     const bool warp_go = __any_sync(0xffffffffu, go);
-    uint8_t* s_slot = sm.scratch->slot[threadIdx.x >> 5];
+    uint8_t* s_slot = sm.slots + 64 * (threadIdx.x >> 5);
     const bool streamed = STREAM && sm.geo2 != nullptr && c.end - c.start > kChunk && blockDim.x == 4 * kChunk;
     const int my_rec = threadIdx.x >> 2, my_q = threadIdx.x & 3;
     int id_ahead = -1;          // streamed: id of this thread's record in the chunk after the one being copied
@@ -648,8 +648,10 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (SORT ? 4 : 5) : 1) blend_
     float4* s_attr = s_geo + kChunk * kStagedQuads;      // lists of one chunk: attributes; of two: more geometry; longer: 2nd buffer
     __shared__ int s_id[kChunk];
     __shared__ int s_id2[STREAM ? kChunk : 1];
-    __shared__ __align__(16) float s_coord[kMaxTileCoords];
+    constexpr bool kFilter = (STREAM || MAXT > 256) && !FUSED;
+    __shared__ __align__(16) float s_coord[MAXT <= 256 ? 260 : kMaxTileCoords];      // tile_w + tile_h <= tile_w * tile_h + 1
     __shared__ SweepScratch s_scratch;
+    __shared__ uint8_t s_slots[SORT ? 2 * MAXT : 1];
     __shared__ uint64_t s_key[FUSED ? kFusedList : 1];
     __shared__ int s_rank[FUSED ? kFusedList : 1];
     __shared__ int s_list[FUSED ? kFusedList : 1];
@@ -726,8 +728,8 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (SORT ? 4 : 5) : 1) blend_
             cp_async_wait_all();                       // a staged list; visible to all behind the barrier
             if (!__syncthreads_or(go)) break;
             const int bs = min(kBatchLayers, P.max_layers - acc.blended);
-            select_sweep<STREAM, (STREAM || MAXT > 256) && !FUSED>(P, c, go, bs, last, batch,
-                                 {s_geo, s_id, &s_scratch, one_chunk || two_chunks, one_chunk ? nullptr : s_attr, s_id2});
+            select_sweep<STREAM, kFilter>(P, c, go, bs, last, batch,
+                                 {s_geo, s_id, kFilter ? &s_scratch : nullptr, s_slots, one_chunk || two_chunks, one_chunk ? nullptr : s_attr, s_id2});
             const int found = batch.found;
             if (go) {
                 const int n = min(found, P.max_layers - acc.blended);
@@ -960,31 +962,34 @@ struct QueuedFragment {
     float o_raw, cr, cg, cb, z;
     float uo, ur, ug, ub, uz;
 };
-// A warp's queue: 64 slots of 4 quads, 5 apart (the odd pitch spreads consecutive slots over the banks).
-constexpr int kQueueSlots = 64, kQueuePitch = 5, kQueueQuads = kQueueSlots * kQueuePitch;
+// A warp's queue: 64 slots of 4 quads, rotated so that a quad of consecutive slots lies on different banks.  (A pitch of 5
+// does that too, but every kilobyte of the eight CTAs is L1 taken from the gathers: 2M triangles, 4K, a step 2083 -> 2065 us.)
+constexpr int kQueueSlots = 64, kQueuePitch = 4, kQueueQuads = kQueueSlots * kQueuePitch;
 
 template <bool DEPTH>
 __device__ __forceinline__ void queue_push(float4* q, int slot, const QueuedFragment& f) {
     q += kQueuePitch * slot;
-    q[0] = make_float4(f.px, f.py, __int_as_float(f.id), f.bx);
-    q[1] = make_float4(f.by, f.bz, f.o_raw, f.cr);
-    q[2] = make_float4(f.cg, f.cb, f.uo, f.ur);
-    if (DEPTH) q[3] = make_float4(f.ug, f.ub, f.z, f.uz);
-    else *reinterpret_cast<float2*>(q + 3) = make_float2(f.ug, f.ub);
+    const int x = (slot >> 1) & 3;
+    q[x] = make_float4(f.px, f.py, __int_as_float(f.id), f.bx);
+    q[1 ^ x] = make_float4(f.by, f.bz, f.o_raw, f.cr);
+    q[2 ^ x] = make_float4(f.cg, f.cb, f.uo, f.ur);
+    if (DEPTH) q[3 ^ x] = make_float4(f.ug, f.ub, f.z, f.uz);
+    else *reinterpret_cast<float2*>(q + (3 ^ x)) = make_float2(f.ug, f.ub);
 }
 template <bool DEPTH>
 __device__ __forceinline__ QueuedFragment queue_pop(const float4* q, int slot) {
     QueuedFragment f;
     q += kQueuePitch * slot;
-    const float4 a = q[0], b = q[1], c = q[2];
+    const int x = (slot >> 1) & 3;
+    const float4 a = q[x], b = q[1 ^ x], c = q[2 ^ x];
     f.px = a.x; f.py = a.y; f.id = __float_as_int(a.z); f.bx = a.w;
     f.by = b.x; f.bz = b.y; f.o_raw = b.z; f.cr = b.w;
     f.cg = c.x; f.cb = c.y; f.uo = c.z; f.ur = c.w;
     if (DEPTH) {
-        const float4 d = q[3];
+        const float4 d = q[3 ^ x];
         f.ug = d.x; f.ub = d.y; f.z = d.z; f.uz = d.w;
     } else {
-        const float2 d = *reinterpret_cast<const float2*>(q + 3);
+        const float2 d = *reinterpret_cast<const float2*>(q + (3 ^ x));
         f.ug = d.x; f.ub = d.y; f.z = 0.f; f.uz = 0.f;
     }
     return f;
@@ -1295,6 +1300,7 @@ __global__ void __launch_bounds__(MAXT, 4) blend_step_l2_kernel(BlendParams P, f
     __shared__ int s_id[kChunk];
     __shared__ __align__(16) float s_coord[kMaxTileCoords];
     __shared__ SweepScratch s_scratch;
+    __shared__ uint8_t s_slots[2 * MAXT];
     extern __shared__ float4 s_step[];       // queues of the warps
     const TileCtx c = tile_context(P, s_coord);
     const int lane = lane_id();
@@ -1306,7 +1312,7 @@ __global__ void __launch_bounds__(MAXT, 4) blend_step_l2_kernel(BlendParams P, f
         const bool go = c.active && acc.alpha > P.thr && P.max_layers > 0;
         if (__syncthreads_or(go)) {
             const int bs = min(kBatchLayers, P.max_layers);
-            select_sweep(P, c, go, bs, 0, batch, {s_geo, s_id, &s_scratch, false, nullptr, nullptr});
+            select_sweep(P, c, go, bs, 0, batch, {s_geo, s_id, &s_scratch, s_slots, false, nullptr, nullptr});
             if (go) {
                 n = min(batch.found, P.max_layers);
                 for (int i = 0; i < n; i++) {
@@ -1381,7 +1387,7 @@ template <bool SORT, int MAXT>
 __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (SORT ? 3 : 4) : 1) blend_backward_kernel(BlendParams P, BackwardIn in, float4* __restrict__ gpack) {
     __shared__ float4 s_geo[(SORT ? kResident : kChunk) * kStagedQuads];
     __shared__ int s_id[kChunk];
-    __shared__ __align__(16) float s_coord[kMaxTileCoords];
+    __shared__ __align__(16) float s_coord[MAXT <= 256 ? 260 : kMaxTileCoords];
     const TileCtx c = tile_context(P, s_coord);
     const bool resident = SORT && c.end - c.start <= kResident;
     if (resident) stage_geo_async(P, c.start, c.end - c.start, s_geo);
@@ -1392,6 +1398,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (SORT ? 3 : 4) : 1) blend_
 
     if (SORT) {
         __shared__ SweepScratch s_scratch;
+        __shared__ uint8_t s_slots[2 * MAXT];
         Batch batch;
         uint64_t last = 0;
         int remaining = limit;
@@ -1400,7 +1407,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (SORT ? 3 : 4) : 1) blend_
             cp_async_wait_all();
             if (!__syncthreads_or(go)) break;
             const int bs = min(kBatchLayers, remaining);
-            select_sweep(P, c, go, bs, last, batch, {s_geo, s_id, &s_scratch, resident, nullptr, nullptr});
+            select_sweep(P, c, go, bs, last, batch, {s_geo, s_id, &s_scratch, s_slots, resident, nullptr, nullptr});
             const int n = go ? min(batch.found, remaining) : 0;
             const int rounds = __reduce_max_sync(0xffffffffu, n);
             // back to front inside the batch (reference render.cu:684-688); the first of the rounds starts at every lane's
@@ -1522,7 +1529,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (SORT ? 3 : 4) : 1) blend_
                                                                         float4* __restrict__ gpack) {
     __shared__ float4 s_geo[(SORT ? kResident : kChunk) * kStagedQuads];
     __shared__ int s_id[kChunk];
-    __shared__ __align__(16) float s_coord[kMaxTileCoords];
+    __shared__ __align__(16) float s_coord[MAXT <= 256 ? 260 : kMaxTileCoords];
     const TileCtx c = tile_context(P, s_coord);
     const bool resident = SORT && c.end - c.start <= kResident;
     if (resident) stage_geo_async(P, c.start, c.end - c.start, s_geo);
@@ -1539,6 +1546,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (SORT ? 3 : 4) : 1) blend_
 
     if (SORT) {
         __shared__ SweepScratch s_scratch;
+        __shared__ uint8_t s_slots[2 * MAXT];
         Batch batch;
         uint64_t last = 0;
         int remaining = limit;
@@ -1547,7 +1555,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (SORT ? 3 : 4) : 1) blend_
             cp_async_wait_all();
             if (!__syncthreads_or(go)) break;
             const int bs = min(kBatchLayers, remaining);
-            select_sweep(P, c, go, bs, last, batch, {s_geo, s_id, &s_scratch, resident, nullptr, nullptr});
+            select_sweep(P, c, go, bs, last, batch, {s_geo, s_id, &s_scratch, s_slots, resident, nullptr, nullptr});
             const int n = go ? min(batch.found, remaining) : 0;
             const int rounds = __reduce_max_sync(0xffffffffu, n);
             for (int i = 0; i < rounds; ++i) {
@@ -1725,6 +1733,9 @@ int blend_forward_short(const float* tri_geo, const float* tri_attr, const uint6
                                                    : tg::blend_forward_kernel<false, 256, false, true>)
                                  : (per_pixel_sort ? tg::blend_forward_kernel<true, 1024, false, true>
                                                    : tg::blend_forward_kernel<false, 1024, false, true>);
+    static SmemAllowed preferred;                 // L1 for the batches, as in tg_blend_forward
+    if (per_pixel_sort && threads <= 256)
+        if (int st = prefer_smem((const void*)kernel, 100, preferred)) return st;
     TG_CUDA(launch_dependent(kernel, tiles, threads, 0, s, P, (float4*)image, depthmap, final_weights, ends, selection, lists));
     TG_LAUNCH_CHECK("blend_forward_kernel (short lists)");
     return TG_OK;
@@ -1752,6 +1763,11 @@ int tg_blend_forward(const float* tri_geo, const float* tri_attr, const int32_t*
     auto kernel = threads > 256 ? (per_pixel_sort ? tg::blend_forward_kernel<true, 1024> : tg::blend_forward_kernel<false, 1024>)
                   : !per_pixel_sort ? tg::blend_forward_kernel<false, 256>
                   : stream_lists ? tg::blend_forward_kernel<true, 256, true> : tg::blend_forward_kernel<true, 256>;
+    // The batches live in local memory: what the CTAs leave of shared memory is L1 for them (2M triangles, 4K, a step:
+    // 2112 -> 2083 us with 64 KB and CTAs that fit it; 196 KB for shared memory: 2404).
+    static tg_host::SmemAllowed preferred[2];
+    if (per_pixel_sort && threads <= 256)
+        if (int st = tg_host::prefer_smem((const void*)kernel, 64, preferred[stream_lists])) return st;
     // Launched ahead of the end of the sort (200k triangles, full HD: a view 152 -> 146 us together with the sort's own early
     // launch), but only behind the kernel for short lists: CTAs that come to an SM while a sort kernel with much shared
     // memory is still there run with what L1 that leaves, and as the SM is never empty, to the end (2M triangles, 4K: 611 ->

@@ -159,6 +159,9 @@ struct SmemAllowed {
     std::atomic<bool> set[kMaxDevices];
 };
 int allow_smem(const void* kernel, size_t bytes, SmemAllowed& allowed);
+// The split of an SM's 256 KB between shared memory (this many of 228 KB, for all its CTAs) and L1, for a kernel that needs
+// the L1 and of which the runtime would give more than its CTAs use to shared memory.  Once per device.
+int prefer_smem(const void* kernel, int kilobytes, SmemAllowed& preferred);
 // `early`: as a dependent launch.
 template <class... Params, class... Args>
 cudaError_t launch_early(bool early, void (*kernel)(Params...), int grid, int block, size_t smem, cudaStream_t stream, Args... args) {
