@@ -5,6 +5,7 @@ import torch
 
 import helpers as Hh
 import oracle as O
+import trigrad_b200
 from trigrad_b200 import scenes as S
 from trigrad_b200 import wrapper as Wr
 
@@ -61,3 +62,31 @@ def test_forward_methods_agree_with_the_oracle(triangles, edge, width, height, t
         assert np.array_equal(out[1].cpu().numpy().view(np.uint32), of.depthmap.view(np.uint32))
     li = O.build_lists(sc.vertices, sc.indices, width, height, tile, tile, cull=True)
     assert np.array_equal(out[4].cpu().numpy(), li.offsets) and np.array_equal(out[3].cpu().numpy(), li.ids)
+
+
+@pytest.mark.parametrize("triangles", [64, 65, 128, 129, 256, 257])
+@pytest.mark.parametrize("per_pixel_sort", [True, False], ids=["per_pixel", "tile_order"])
+def test_lists_at_the_ends_of_chunks(triangles, per_pixel_sort):
+    """Faint triangles over a whole tile and a part of another, blended to the last one: lists of whole chunks, staged once
+    for all batches of 32 layers, and one entry more; forward and corrected backward."""
+    sc = S.random_triangles(triangles, 23, 16, 6.0, 0.05, name="chunks", seed=triangles)
+    op = (0.05 * sc.opacities).astype(np.float32)
+    image_of = lambda v, c, o: O.forward(v, sc.indices, c, o, 23, 16, 16, 16, 0.0, per_pixel_sort, triangles + 1)
+    of = image_of(sc.vertices, sc.colors, op)
+    v, i, c, o = (Hh.cuda(x) for x in (sc.vertices, sc.indices, sc.colors, op))
+    for x in (v, c, o):
+        x.requires_grad_()
+    image, depth = trigrad_b200.render_corrected(v, i, c, o, 23, 16, 16, 16, 0.0, False, per_pixel_sort, 0)
+    assert np.array_equal(image.detach().cpu().numpy().view(np.uint32), of.image.view(np.uint32))
+    assert np.array_equal(depth.detach().cpu().numpy().view(np.uint32), of.depthmap.view(np.uint32))
+    assert int(of.ends.max()) > min(triangles // 2, 60)
+    rng = np.random.default_rng(triangles)
+    gi = rng.normal(size=of.image.shape).astype(np.float32)
+    (image * Hh.cuda(gi)).sum().backward()
+    f64 = [np.asarray(x, np.float64) for x in (sc.vertices, sc.colors, op)]
+    of64 = image_of(*f64)
+    og = O.backward(f64[0], sc.indices, f64[1], f64[2], 23, 16, of64, gi.astype(np.float64), np.zeros((16, 23)), 16, 16,
+                    per_pixel_sort, triangles + 1, corrected=True)
+    if np.array_equal(of64.ends, of.ends):
+        for a, b in zip((v, c, o), og):
+            assert Hh.rel_l2(a.grad.cpu().numpy(), b) <= 2e-4
