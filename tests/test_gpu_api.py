@@ -120,6 +120,28 @@ def test_shape_and_dtype_errors():
         trigrad_b200.render(v, i, c, o, 64, 64, 64, 64)
 
 
+@pytest.mark.parametrize("tile", [(0, 16), (16, 0), (0, 0), (-16, 16), (-4, -4), (2 ** 32 + 16, 16), (2 ** 33, 2 ** 33)])
+def test_every_entry_point_rejects_tiles_that_are_none(tile):
+    from trigrad_b200 import views
+    sc = S.large_triangles(2)
+    v, i, c, o = Hh.scene_tensors(sc)
+    rgba, faces = trigrad_b200.pack_mesh(c, o, i)
+    target = torch.rand((32, 32, 4), device="cuda")
+    b4, b3 = (views.GradBuffer.allocate(v.shape[0], "cuda", p) for p in (4, 3))
+    pv = np.eye(4, dtype=np.float32)
+    for call in (lambda: trigrad_b200.render(v, i, c, o, 32, 32, *tile),
+                 lambda: trigrad_b200.render_corrected(v, i, c, o, 32, 32, *tile),
+                 lambda: trigrad_b200.render_packed(v, faces, rgba, 32, 32, *tile),
+                 lambda: trigrad_b200.Renderer.apply(v, i, c, o, 32, 32, *tile),
+                 lambda: views.l2_view_step(v, i, c, o, target, 32, 32, b4.points, b4.colors, b4.opacities, b4.loss, *tile),
+                 lambda: views.l2_world_view_step(v[:, :3].contiguous(), pv, i, c, o, target, 32, 32, b3.points, b3.colors,
+                                                  b3.opacities, b3.loss, *tile)):
+        with pytest.raises(ValueError):
+            call()
+    if max(tile) < 2 ** 31:                  # a mesh without triangles is not binned
+        assert trigrad_b200.render(v, i[:0], c, o, 32, 32, *tile)[0].shape == (32, 32, 4)
+
+
 def test_capacity_regrow_and_reuse():
     """A small scene first, then one with far more (triangle, tile) pairs, then the small one again."""
     small, big = S.large_triangles(2), S.full_screen_layers(50, width=640, height=480)

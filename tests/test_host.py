@@ -29,6 +29,15 @@ def test_render_rejects_oversized_tiles():
         trigrad_b200.render(v, i, c, o, 64, 64, 64, 32)
 
 
+@pytest.mark.parametrize("tile", [(0, 16), (16, 0), (0, 0), (-16, 16), (-4, -4), (2 ** 32 + 16, 16), (2 ** 33, 2 ** 33),
+                                  (2 ** 31, 2 ** 33), (-2 ** 40, 2 ** 40)])
+def test_forward_rejects_tiles_that_are_none(tile):
+    """A tile size of zero divides nothing, and a 64-bit one does not become a small one."""
+    from trigrad_b200 import wrapper as Wr
+    with pytest.raises(ValueError):
+        Wr.forward_native(*_scene_tensors(S.large_triangles(2)), 32, 32, *tile, 1 / 256, False, True, 32)
+
+
 def test_check_tensor_semantics():
     check = create_check("cpu", torch.float32)
     t = torch.zeros(5, 4)

@@ -9,6 +9,7 @@
 // module holds no device code.
 #include <dlfcn.h>
 
+#include <algorithm>
 #include <list>
 #include <memory>
 #include <mutex>
@@ -96,8 +97,11 @@ int need_int(int64_t v) {
     TORCH_CHECK(v >= 0 && v <= INT32_MAX, "size out of range");
     return (int)v;
 }
-void need_tile(int tw, int th) {
-    if ((int64_t)tw * th > 1024) throw py::value_error("tile_width * tile_height must be <= 1024");
+// The product as the caller's 64-bit numbers have it (the reference's check); the sign is view_of's to look at.
+void need_tile(int64_t tw, int64_t th) {
+    int64_t area = 0;
+    if (__builtin_mul_overflow(tw, th, &area) ? (tw < 0) == (th < 0) : area > 1024)
+        throw py::value_error("tile_width * tile_height must be <= 1024");
 }
 
 template <class T>
@@ -651,8 +655,20 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> project_clip(const Tensor& points_, c
 using Optional = std::optional<Tensor>;
 Tensor or_none(const Optional& t) { return t ? *t : Tensor(); }
 
-View view_of(int64_t W, int64_t H, int64_t tw, int64_t th, double thr, bool sort, int64_t layers) {
-    return {need_int(W), need_int(H), (int)tw, (int)th, thr, sort, (int)std::min<int64_t>(layers, INT32_MAX)};
+// `binned` false: a mesh without triangles, which no kernel sees; its tile size is not looked at.
+View view_of(bool binned, int64_t W, int64_t H, int64_t tw, int64_t th, double thr, bool sort, int64_t layers) {
+    need_int(W);
+    need_int(H);
+    if (binned) {
+        if (tw < 1 || th < 1) throw py::value_error("tile_width and tile_height must be positive");
+        need_tile(tw, th);                       // so both fit an int
+        // fewer than 2^31 tiles, and pixels on a side with the last tile rounded up
+        if (W > INT32_MAX - tw || H > INT32_MAX - th || ((W + tw - 1) / tw) * ((H + th - 1) / th) >= INT32_MAX)
+            throw py::value_error("too many tiles");
+    } else {
+        tw = th = 1;
+    }
+    return {(int)W, (int)H, (int)tw, (int)th, thr, sort, (int)std::clamp<int64_t>(layers, INT32_MIN, INT32_MAX)};
 }
 
 Matrix matrix_of(const py::buffer& b) {
@@ -667,7 +683,7 @@ Matrix matrix_of(const py::buffer& b) {
 py::object py_render(int kind, const Tensor& vertices, const Tensor& indices, const Tensor& colors,
                      const Optional& opacities_, int64_t W, int64_t H, int64_t tw, int64_t th, double thr, bool timing,
                      bool sort, int64_t layers, bool cull, int64_t selection_max_bytes) {
-    need_tile((int)tw, (int)th);
+    need_tile(tw, th);
     const Tensor opacities = or_none(opacities_);
     const int64_t V = rows(vertices, "vertices");
     need(vertices, "vertices", {V, 4});
@@ -679,7 +695,7 @@ py::object py_render(int kind, const Tensor& vertices, const Tensor& indices, co
         need(opacities, "opacities", {V});
         need(indices, "indices", {rows(indices, "indices"), 3}, at::kInt);
     }
-    const View v = view_of(W, H, tw, th, thr, sort, layers);
+    const View v = view_of(indices.size(0) > 0, W, H, tw, th, thr, sort, layers);
     ImageAndDepth r;
     {
         py::gil_scoped_release nogil;
@@ -702,7 +718,7 @@ Tensor part(const Saved& s, const void* p, at::ScalarType type, at::IntArrayRef 
 py::object py_forward(const Tensor& vertices, const Tensor& indices, const Tensor& colors, const Optional& opacities,
                       int64_t W, int64_t H, int64_t tw, int64_t th, double thr, bool timing, bool sort, int64_t layers,
                       bool save_selection, bool cull, int64_t selection_max_bytes) {
-    const View v = view_of(W, H, tw, th, thr, sort, layers);
+    const View v = view_of(true, W, H, tw, th, thr, sort, layers);
     ForwardOut f;
     Tensor fw, ids, off, geo, attr, ends;
     {
@@ -749,8 +765,8 @@ Tensor py_l2_step(const Tensor& vertices, const Tensor& indices, const Tensor& c
     const bool world = !pv.is_none();
     need_mesh(vertices, world ? "points" : "vertices", world ? 3 : 4, indices, colors, opacities);
     need(target, "target", {H, W, 4}, target.scalar_type() == at::kByte && !one_kernel ? at::kByte : at::kFloat);
-    need_tile((int)tw, (int)th);
-    const View v = view_of(W, H, tw, th, thr, true, layers);
+    need_tile(tw, th);
+    const View v = view_of(true, W, H, tw, th, thr, true, layers);
     const Grads to = {or_none(gV), or_none(gC), or_none(gO), or_none(loss), or_none(packed)};
     const Matrix m = world ? matrix_of(pv.cast<py::buffer>()) : Matrix{};
     py::gil_scoped_release nogil;
