@@ -15,7 +15,8 @@
  *   tiles      tiles_x = ceil(W/tile_w), tiles_y = ceil(H/tile_h), tile id = ty*tiles_x + tx
  *   All pointers are device pointers unless named *_host.  `stream` is a cudaStream_t.
  *   Every function returns TG_OK (0) or one of the TG_ERR_* codes; tg_last_error() gives text.
- *   The number of (triangle, tile) pairs K must stay below 2^31.
+ *   The number of (triangle, tile) pairs of the bounding rectangles must stay below 2^31
+ *   (tg_render_forward, tg_render_step_l2: TG_ERR_BAD_ARG otherwise).
  *
  * Threads and state.  Every entry point may be called from any host thread (the reference runs its
  * forward on the caller's thread and its backward on an autograd worker thread); work is ordered on

@@ -64,6 +64,24 @@ def test_forward_methods_agree_with_the_oracle(triangles, edge, width, height, t
     assert np.array_equal(out[4].cpu().numpy(), li.offsets) and np.array_equal(out[3].cpu().numpy(), li.ids)
 
 
+@pytest.mark.parametrize("triangles,side,tile", [(4097, 1024, 1), (4096, 1024, 1), (2049, 1024, 1), (65536 + 1, 1024, 4)])
+def test_more_pairs_than_a_list_can_hold(triangles, side, tile):
+    """Triangles over the whole image, 2^31 to 2^32 + 2^20 pairs: 32-bit sums of them are small numbers or zero.  The call is
+    refused and the next one on the stream finds its counters in order."""
+    corners = np.array([[-4, -4], [4, -4], [0, 4]], np.float32)
+    v = torch.ones((triangles, 3, 4), device="cuda")
+    v[..., :2] = Hh.cuda(corners)
+    v = v.reshape(-1, 4)
+    i = torch.arange(3 * triangles, dtype=torch.int32, device="cuda").reshape(-1, 3)
+    c, o = torch.rand((3 * triangles, 3), device="cuda"), torch.rand((3 * triangles,), device="cuda")
+    with pytest.raises(RuntimeError, match="pairs"):
+        trigrad_b200.render(v, i, c, o, side, side, tile, tile)
+    few = slice(0, 7)
+    image = trigrad_b200.render(v, i[few], c, o, 64, 48, tile, tile)[0].cpu().numpy()
+    of = O.forward(*(x.cpu().numpy() for x in (v, i[few], c, o)), 64, 48, tile, tile)
+    assert np.array_equal(image.view(np.uint32), of.image.view(np.uint32))
+
+
 @pytest.mark.parametrize("triangles", [64, 65, 128, 129, 256, 257])
 @pytest.mark.parametrize("per_pixel_sort", [True, False], ids=["per_pixel", "tile_order"])
 def test_lists_at_the_ends_of_chunks(triangles, per_pixel_sort):

@@ -30,7 +30,7 @@ struct ForwardWorkspace {
         bin.tables = (float4*)take(sizeof(float4) * ((size_t)tiles + 1));     // tiles_x + tiles_y <= tiles + 1
         // everything from `status` up to the end of the tile counts must be zero when the kernels start
         bin.status = (uint32_t*)take(sizeof(uint32_t) * 4);
-        bin.counters = (uint32_t*)take(sizeof(uint32_t) * 2);
+        bin.counters = (uint32_t*)take(sizeof(uint32_t) * 4);
         bin.tile_scan_scratch = take(device_scan ? tg_scan_scratch_bytes(tiles) : 0);
         bin.tile_counts = (uint32_t*)take(sizeof(uint32_t) * (size_t)tiles);
         bin.clear = bin.status;
@@ -153,6 +153,10 @@ struct TileLists {
         longest = info_host[1];
         if (have_order) order = ws.bin.tile_order;
         const uint32_t slots = info_host[3];            // K and the holes of culled pairs
+        if (K >= tg::kTooManyPairs || slots >= tg::kTooManyPairs) {
+            tg_host::set_error("the triangles' rectangles hold 2^31 or more (triangle, tile) pairs");
+            return TG_ERR_BAD_ARG;
+        }
         if (K > cap || slots > cap) {
             info_host[0] = K > slots ? K : slots;
             tg_host::set_error("%u entries and culled pairs exceed the list capacity %u", info_host[0], cap);

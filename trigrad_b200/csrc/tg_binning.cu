@@ -536,8 +536,9 @@ __global__ void __launch_bounds__(kEmitThreads) emit_keys_kernel(const float4* _
 struct BinArgs {
     uint32_t* tile_counts;   // [tiles], zero on entry
     int32_t* offsets;        // [tiles + 1], written when scan_here
-    uint32_t* counters;      // [2], zero on entry: finished CTAs, slots handed out
-    uint32_t* info;          // [3] K, when scan_here the longest list (kOrderWrittenBit: a launch order is wanted), slots
+    uint32_t* counters;      // [4], zero on entry: finished CTAs, -, slots handed out (64 bits)
+    uint32_t* info;          // [3] K, when scan_here the longest list (kOrderWrittenBit: a launch order is wanted), slots;
+                             // K and slots no larger than kTooManyPairs
     uint32_t* info_host;     // words 0, 1 and 3 of mapped host memory receive them too, or null
     uint4* pairs;            // [capacity]
     uint32_t capacity;
@@ -549,6 +550,9 @@ struct BinArgs {
 };
 
 constexpr uint32_t kHole = 0xffffffffu;      // tile word of a pair that is not listed
+__device__ __forceinline__ unsigned long long* slot_counter(const BinArgs& bin) {
+    return reinterpret_cast<unsigned long long*>(bin.counters + 2);
+}
 constexpr int kBinQueue = 64 * kBinWarps;       // clip queue of a CTA
 // Shared memory of a warp, in words: first the staging area of its records (pitch 5 quads for the 4 of a geometry
 // record, 7 for the 6 of half the warp's attribute records: 16-byte accesses of consecutive lanes then fall on different
@@ -575,7 +579,7 @@ __device__ __forceinline__ void write_pair(const BinArgs& bin, const float* tri,
 // After all pairs are counted, by one CTA: tile offsets, K, the longest list, and all of it to the host.
 template <int WARPS>
 __device__ __forceinline__ void finish_binning(const BinArgs& bin, uint32_t* s_warp) {
-    const uint32_t slots = __ldcg(bin.counters + 1);
+    const uint32_t slots = (uint32_t)min(__ldcg(slot_counter(bin)), (unsigned long long)kTooManyPairs);
     uint32_t K = slots, longest = UINT32_MAX;            // longest: not known
     if (bin.scan_here) {
         longest = tile_offsets_by_one_cta<WARPS>(bin.tile_counts, bin.offsets, bin.tiles, s_warp, K);
@@ -583,6 +587,7 @@ __device__ __forceinline__ void finish_binning(const BinArgs& bin, uint32_t* s_w
         // long on average and uneven (the longest one at least 256 entries)
         if (bin.want_order && bin.tiles <= kOrderMaxTiles && K >= kOrderMinMean * (uint32_t)bin.tiles && longest >= kOrderMinLongest)
             longest |= kOrderWrittenBit;
+        if (slots == kTooManyPairs) K = kTooManyPairs;   // the counts' sum is not the number of pairs then
     }
     if (threadIdx.x == 0) {
         bin.info[0] = K;
@@ -673,18 +678,24 @@ __global__ void __launch_bounds__(32 * kBinWarps, 32 / kBinWarps) bin_kernel(con
             const uint32_t y = __shfl_up_sync(0xffffffffu, incl, d);
             if (lane >= d) incl += y;
         }
-        total = __shfl_sync(0xffffffffu, incl, 31);
+        // A triangle has fewer than 2^31 pairs, but 32 of them can have more than 32 bits hold: the sum in halves, cut off
+        const uint32_t low = __reduce_add_sync(0xffffffffu, count & 0xffffu), high = __reduce_add_sync(0xffffffffu, count >> 16);
+        total = (uint32_t)min(((uint64_t)high << 16) + low, (uint64_t)UINT32_MAX);
         mine[32 * kTriFirst + lane] = __uint_as_float(incl - count);
     }
     if (lane == 0) s_warp[warp] = total;
     __syncthreads();
-    // Every pair of the rectangles has its slot; those that are not listed leave a hole there.
+    // Every pair of the rectangles has its slot; those that are not listed leave a hole there.  Slots are counted in 64 bits:
+    // in 32 the count of a call with 2^32 pairs wraps to one that passes for fitting the list, while the tile offsets point
+    // far behind it (3840x2160 in tiles of 4x4: 8300 triangles over the whole image).  Such a call is refused, so a CTA that
+    // finds it lists nothing.
     if (tid == 0) {
-        uint32_t sum = 0;
+        uint64_t sum = 0;
 #pragma unroll
-        for (int w = 0; w < kBinWarps; w++) { s_first[w] = sum; sum += s_warp[w]; }
-        s_first[kBinWarps] = sum;
-        s_base = sum ? atomicAdd(bin.counters + 1, sum) : 0u;
+        for (int w = 0; w < kBinWarps; w++) { s_first[w] = (uint32_t)sum; sum += s_warp[w]; }
+        const uint64_t at = sum ? atomicAdd(slot_counter(bin), (unsigned long long)sum) : 0;
+        s_first[kBinWarps] = at + sum < kTooManyPairs ? (uint32_t)sum : 0u;
+        s_base = (uint32_t)at;
     }
     __syncthreads();
     // The CTA's pairs in chunks of 32, whichever warp prepared the triangle
@@ -778,7 +789,7 @@ __global__ void __launch_bounds__(256) scatter_entries_kernel(const uint4* __res
     // the binning kernel is done with its counters: zero for the next call
     const uint32_t me = blockIdx.x * 256 + threadIdx.x;
     for (uint32_t i = me; i < (uint32_t)tiles; i += gridDim.x * 256) tile_counts[i] = 0;
-    if (me < 2) counters[me] = 0;
+    if (me < 4) counters[me] = 0;
     if (me < 6) list_heads[me] = 0;
     const uint32_t n = info[2];               // slots, holes included
     if (n > capacity) return;

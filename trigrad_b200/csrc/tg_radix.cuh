@@ -20,6 +20,8 @@ constexpr int kHistDoneWord = 8;
 constexpr int kTileScanByLastCta = 65536;
 // Top bit of the longest-list word the binning kernel reports: a launch order of the tiles was written.
 constexpr uint32_t kOrderWrittenBit = 0x80000000u;
+// What it reports as K and as slots from this many (triangle, tile) pairs on: more than any list capacity.
+constexpr uint32_t kTooManyPairs = 0x80000000u;
 // Longest tile list that a warp sorts (tile_sort_kernel alone).
 constexpr int kTileSortRank = 128;
 // Longest tile list that the compositing kernel sorts itself, in images of at most kFusedTiles tiles: two waves of its
@@ -108,7 +110,7 @@ struct BinBuffers {
     uint32_t* clear;             // zeroed by the first kernel: `clear_words` words that hold the next four
     size_t clear_words;
     uint32_t* status;            // device error word
-    uint32_t* counters;          // [2]
+    uint32_t* counters;          // [4], 8-byte aligned
     uint32_t* tile_counts;       // [tiles], 16-byte aligned
     void* tile_scan_scratch;     // device-wide scan of the tile counts, only beyond kTileScanByLastCta tiles; zeroed too
     float4* tables;              // [tiles_x + tiles_y]
