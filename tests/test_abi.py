@@ -46,6 +46,14 @@ def test_argument_errors_are_reported_before_any_device_work():
     # tile larger than 1024 threads
     st = lib.tg_blend_forward(None, None, None, None, 64, 64, 64, 64, 0.0, 1, 32, None, None, None, None, None, None)
     assert st == N.TG_ERR_BAD_ARG and b"1024" in lib.tg_last_error()
+    # sizes whose products do not fit 32 bits
+    for W, H, tile, said in ((64, 64, 1 << 16, b"1024"), (1 << 16, 1 << 16, 1, b"tiles"), (2 ** 31 - 1, 8, 16, b"tiles")):
+        st = lib.tg_blend_forward(None, None, None, None, W, H, tile, tile, 0.0, 1, 32, None, None, None, None, None, None)
+        assert st == N.TG_ERR_BAD_ARG and said in lib.tg_last_error()
+        p = C.c_void_p(256)             # never looked at: the sizes come first
+        st = lib.tg_render_forward(p, p, p, p, 1, W, H, tile, tile, 0.0, 1, 32, p, p, p, p, None, p, p, p, 64, p, p, 1 << 20, p,
+                                   None, 0, None)
+        assert st == N.TG_ERR_BAD_ARG and said in lib.tg_last_error()
     # max_layers must be >= 1 at the ABI (the Python layer maps <= 0 to T + 1)
     st = lib.tg_blend_forward(None, None, None, None, 64, 64, 16, 16, 0.0, 1, 0, None, None, None, None, None, None)
     assert st == N.TG_ERR_BAD_ARG

@@ -173,8 +173,8 @@ struct TileLists {
 
 static int check_forward_args(int T, int W, int H, int tw, int th, int max_layers, const void* workspace,
                               const void* info_host, const void* offsets, uint32_t list_capacity, unsigned flags) {
-    TG_REQUIRE(T >= 0 && W > 0 && H > 0 && tw > 0 && th > 0, "sizes");
-    TG_REQUIRE(tw * th <= 1024, "tile_width * tile_height must be <= 1024");
+    TG_REQUIRE(T >= 0, "T < 0");
+    if (int s = tg_host::check_sizes(W, H, tw, th)) return s;
     TG_REQUIRE(max_layers >= 1, "max_layers must be >= 1");
     TG_REQUIRE(workspace && info_host && offsets, "null pointer");
     TG_REQUIRE(((uintptr_t)workspace & 255) == 0, "workspace must be 256-byte aligned");
@@ -217,9 +217,9 @@ int tg_render_forward(const float* vertices, const int32_t* indices, const float
                       size_t workspace_bytes, uint32_t* info_host, float* stage_ms_host, unsigned flags,
                       tg_stream_t stream) {
     TG_REQUIRE(image && depthmap && final_weights && ends, "null pointer");
+    if (int st = check_forward_args(T, W, H, tw, th, max_layers, workspace, info_host, offsets, list_capacity, flags)) return st;
     cudaStream_t s = (cudaStream_t)stream;
     StageTimer timer(stage_ms_host != nullptr, s);
-    if (int st = check_forward_args(T, W, H, tw, th, max_layers, workspace, info_host, offsets, list_capacity, flags)) return st;
     TileLists lists(workspace, T, W, H, tw, th, list_capacity, flags);
     if (int st = lists.start(vertices, indices, colors, opacities, T, W, H, tw, th, tri_geo, tri_attr, sorted_ids, list_capacity,
                              offsets, workspace_bytes, info_host, flags, timer, s))
@@ -266,10 +266,10 @@ int tg_render_step_l2(const float* vertices, const int32_t* indices, const float
                       size_t scratch_bytes, uint32_t* info_host, float* stage_ms_host, unsigned flags,
                       tg_stream_t stream) {
     TG_REQUIRE(image && depthmap && final_weights && ends && target, "null pointer");
+    if (int st = check_forward_args(T, W, H, tw, th, max_layers, workspace, info_host, offsets, list_capacity, flags)) return st;
     TG_REQUIRE(tw * th <= 256 && max_layers <= 32, "the one-kernel step needs tiles of at most 256 pixels and max_layers <= 32");
     cudaStream_t s = (cudaStream_t)stream;
     StageTimer timer(stage_ms_host != nullptr, s);
-    if (int st = check_forward_args(T, W, H, tw, th, max_layers, workspace, info_host, offsets, list_capacity, flags)) return st;
     TileLists lists(workspace, T, W, H, tw, th, list_capacity, flags);
     int st = lists.start(vertices, indices, colors, opacities, T, W, H, tw, th, tri_geo, tri_attr, sorted_ids, list_capacity,
                          offsets, workspace_bytes, info_host, flags, timer, s);

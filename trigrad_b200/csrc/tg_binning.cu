@@ -856,11 +856,13 @@ int cuda_fail(cudaError_t e, const char* what) {
 }
 const char* last_error() { return g_err; }
 
-static int check_dims_internal(int T, int W, int H, int tw, int th) {
-    TG_REQUIRE(T >= 0, "T < 0");
+int check_sizes(int W, int H, int tw, int th) {
     TG_REQUIRE(W > 0 && H > 0, "image size must be positive");
     TG_REQUIRE(tw > 0 && th > 0, "tile size must be positive");
-    TG_REQUIRE(tw * th <= 1024, "tile_width * tile_height must be <= 1024");
+    TG_REQUIRE((int64_t)tw * th <= 1024, "tile_width * tile_height must be <= 1024");
+    TG_REQUIRE(W <= INT32_MAX - tw && H <= INT32_MAX - th &&
+                   (int64_t)((W + tw - 1) / tw) * ((H + th - 1) / th) < INT32_MAX,
+               "too many tiles");
     return TG_OK;
 }
 
@@ -891,7 +893,8 @@ int prefer_smem(const void* kernel, int kilobytes, SmemAllowed& preferred) {
 int bin_triangles(const float* vertices, const int32_t* indices, const float* colors, const float* opacities, int T, int W,
                   int H, int tw, int th, float* tri_geo, float* tri_attr, const BinBuffers& b, int32_t* offsets,
                   uint32_t list_capacity, uint32_t* info_host, bool cull, bool packed, bool ready, cudaStream_t stream) {
-    if (int s = check_dims_internal(T, W, H, tw, th)) return s;
+    TG_REQUIRE(T >= 0, "T < 0");
+    if (int s = check_sizes(W, H, tw, th)) return s;
     TG_REQUIRE(offsets, "null pointer");
     const int tiles_x = (W + tw - 1) / tw, tiles_y = (H + th - 1) / th;
     const int tiles = tiles_x * tiles_y;
@@ -985,10 +988,7 @@ const char* tg_status_string(int s) {
 
 static int check_dims(int T, int W, int H, int tw, int th) {
     TG_REQUIRE(T >= 0, "T < 0");
-    TG_REQUIRE(W > 0 && H > 0, "image size must be positive");
-    TG_REQUIRE(tw > 0 && th > 0, "tile size must be positive");
-    TG_REQUIRE(tw * th <= 1024, "tile_width * tile_height must be <= 1024");
-    return TG_OK;
+    return tg_host::check_sizes(W, H, tw, th);
 }
 
 int tg_preprocess(const float* vertices, const int32_t* indices, const float* colors, const float* opacities, int T,

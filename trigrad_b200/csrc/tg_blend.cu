@@ -1687,8 +1687,7 @@ __global__ void __launch_bounds__(256) unpack_gradients_rgba_kernel(float4* __re
 extern "C" {
 
 static int blend_args(int W, int H, int tw, int th, int max_layers) {
-    TG_REQUIRE(W > 0 && H > 0 && tw > 0 && th > 0, "sizes must be positive");
-    TG_REQUIRE(tw * th <= 1024, "tile_width * tile_height must be <= 1024");
+    if (int s = tg_host::check_sizes(W, H, tw, th)) return s;
     TG_REQUIRE(max_layers >= 1, "max_layers must be >= 1");
     return TG_OK;
 }

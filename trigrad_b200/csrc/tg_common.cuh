@@ -153,6 +153,8 @@ namespace tg_host {
 void set_error(const char* fmt, ...);
 int cuda_fail(cudaError_t e, const char* what);
 void count_launch();
+// Image and tile size of a call: positive, tiles of at most 1024 pixels, fewer than 2^31 of them.
+int check_sizes(int W, int H, int tw, int th);
 // Opt-in shared memory of a kernel, set once per device (setting it twice is harmless).
 struct SmemAllowed {
     static constexpr int kMaxDevices = 64;
