@@ -1,0 +1,105 @@
+"""What a render keeps for its backward is autograd's: saved-tensor hooks see all of it, and it is freed with the graph."""
+import numpy as np
+import pytest
+import torch
+
+import helpers as Hh
+import trigrad_b200
+from trigrad_b200 import scenes as S
+
+pytestmark = pytest.mark.gpu
+
+W, H = 200, 120
+
+
+def _leaves(packed=False):
+    sc = S.random_triangles(3000, W, H, 0.2, 0.4, name="saved", seed=4)
+    v, i, c, o = Hh.scene_tensors(sc)
+    if packed:
+        rgba, i = trigrad_b200.pack_mesh(c, o, i)
+        return i, [x.requires_grad_() for x in (v, rgba)]
+    return i, [x.requires_grad_() for x in (v, c, o)]
+
+
+CALLS = {
+    "render": lambda i, x: trigrad_b200.render(x[0], i, x[1], x[2], W, H),
+    "searched": lambda i, x: trigrad_b200.render(x[0], i, x[1], x[2], W, H, 16, 16, 1 / 256, False, True, 40),
+    "tile_order": lambda i, x: trigrad_b200.render(x[0], i, x[1], x[2], W, H, 16, 16, 1 / 256, False, False, 64),
+    "corrected": lambda i, x: trigrad_b200.render_corrected(x[0], i, x[1], x[2], W, H, 16, 16, 1 / 256, False, True, 0),
+    "packed": lambda i, x: trigrad_b200.render_packed(x[0], i, x[1], W, H),
+    "Renderer": lambda i, x: trigrad_b200.Renderer.apply(x[0], i, x[1], x[2], W, H),
+}
+
+
+def _loss(out):
+    weights = torch.linspace(0.5, 1.5, out[0].numel(), device="cuda").reshape(out[0].shape)
+    return (out[0] * weights).sum() + torch.where(torch.isfinite(out[1]), out[1], 0).sum()
+
+
+def _moved(t):
+    """The same values at an address and with strides of its own."""
+    room = torch.empty(2 * t.numel() + 1, dtype=t.dtype, device="cuda")
+    return room[1:].as_strided(t.shape, [2 * s for s in t.contiguous().stride()]).copy_(t)
+
+
+@pytest.mark.parametrize("call", list(CALLS))
+def test_hooks_see_and_move_all_that_is_saved(call):
+    i, leaves = _leaves(call == "packed")
+    want = torch.autograd.grad(_loss(CALLS[call](i, leaves)), leaves)
+    seen = []
+
+    def pack(t):
+        seen.append(t.numel() * t.element_size())
+        return t.cpu()
+
+    for unpack in (lambda t: t.cuda(), _moved):
+        seen.clear()
+        with torch.autograd.graph.saved_tensors_hooks(pack, unpack):
+            out = CALLS[call](i, leaves)
+        # image and depth map, final weights and ends, records of 160 bytes, and the selection where one is kept
+        least = 20 * W * H + 8 * W * H + 160 * i.shape[0]
+        if call in ("render", "packed", "Renderer"):
+            least += 4 * 32 * W * H
+        assert sum(seen) >= least
+        for a, b in zip(torch.autograd.grad(_loss(out), leaves), want):
+            assert Hh.rel_l2(a.cpu().numpy(), b.cpu().numpy()) <= 1e-5      # sums of atomics, in no fixed order
+
+
+@pytest.mark.parametrize("call", list(CALLS))
+def test_a_hook_that_changes_device_or_size_is_an_error(call):
+    i, leaves = _leaves(call == "packed")
+    for unpack in (lambda t: t, lambda t: t.cuda().flatten()[:-1] if t.numel() > 1 else t, lambda t: t.cuda().double()):
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: t.cpu(), unpack):
+            out = CALLS[call](i, leaves)
+        loss = _loss((out[0], out[1]))
+        with pytest.raises(RuntimeError):
+            torch.autograd.grad(loss, leaves)
+
+
+@pytest.mark.parametrize("call", list(CALLS))
+def test_saved_state_is_freed_by_a_backward_that_does_not_keep_the_graph(call):
+    i, leaves = _leaves(call == "packed")
+    torch.autograd.grad(_loss(CALLS[call](i, leaves)), leaves)          # the stream's own workspaces exist from here on
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    out = CALLS[call](i, leaves)
+    loss = _loss(out)
+    kept = torch.cuda.memory_allocated() - before
+    torch.autograd.grad(loss, leaves, retain_graph=True)
+    torch.autograd.grad(loss, leaves)
+    with pytest.raises(RuntimeError, match="second time"):
+        torch.autograd.grad(loss, leaves)
+    assert out[0].grad_fn is not None
+    freed = kept - (torch.cuda.memory_allocated() - before)
+    assert freed >= 160 * i.shape[0] + (4 * 32 * W * H if call in ("render", "packed", "Renderer") else 0)
+
+
+@pytest.mark.parametrize("call", list(CALLS))
+def test_second_backward_of_a_mesh_without_triangles(call):
+    i, leaves = _leaves(call == "packed")
+    out = CALLS[call](i[:0], leaves)
+    for keep in (True, False):
+        for g, x in zip(torch.autograd.grad(out[0].sum(), leaves, retain_graph=keep), leaves):
+            assert g.shape == x.shape and not bool(g.any())
+    with pytest.raises(RuntimeError, match="second time"):
+        torch.autograd.grad(out[0].sum(), leaves)

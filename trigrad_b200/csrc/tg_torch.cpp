@@ -231,21 +231,43 @@ struct View {       // the arguments of a render that are not tensors
     int64_t pixels() const { return (int64_t)W * H; }
 };
 
-// What a forward leaves for its backward, in one allocation (`blob`) beside the lists and the selection.
-struct Saved {
+// What a forward leaves for its backward: sizes and places (`Layout`), and three tensors - final weights, ends, records
+// and tile offsets in one allocation (`blob`), the lists, and the selection.  Between the passes the tensors belong to
+// autograd (SavedVariable, ctx.save_for_backward), which may move them; so places are offsets, never addresses.
+struct Layout {
     View v;
-    int V = 0, T = 0;
+    int V = 0, T = 0, planes = 0;
     int64_t K = 0;
+    size_t final_w = 0, ends = 0, geo = 0, attr = 0, offsets = 0, bytes = 0;      // of blob
+
+    Layout() = default;
+    Layout(const View& view, int n_vertices, int n_triangles) : v(view), V(n_vertices), T(n_triangles) {
+        const size_t px = (size_t)v.pixels();
+        auto take = [&](size_t n) { const size_t at = bytes; bytes += (n + 255) / 256 * 256; return at; };
+        final_w = take(4 * px);
+        ends = take(4 * px);
+        geo = take(4 * (size_t)T * TG_GEO_WORDS);
+        attr = take(4 * (size_t)T * TG_ATTR_WORDS);
+        offsets = take(4 * ((size_t)v.tiles() + 1));
+    }
+};
+struct Saved {
+    Layout l;
     Tensor blob, ids, selection;
-    float *final_w = nullptr, *geo = nullptr, *attr = nullptr;
-    int32_t *ends = nullptr, *offsets = nullptr;
-    const int32_t* id_list() const { return data<int32_t>(ids); }
-    const int32_t* sel() const { return data<int32_t>(selection); }
+    template <class X>
+    X* at(size_t place) const { return reinterpret_cast<X*>(data<char>(blob) + place); }
+    float* final_w() const { return at<float>(l.final_w); }
+    float* geo() const { return at<float>(l.geo); }
+    float* attr() const { return at<float>(l.attr); }
+    int32_t* ends() const { return at<int32_t>(l.ends); }
+    int32_t* offsets() const { return at<int32_t>(l.offsets); }
+    int32_t* id_list() const { return data<int32_t>(ids); }
+    int32_t* sel() const { return data<int32_t>(selection); }
 };
 
 struct ForwardOut {
     Tensor image, depthmap;
-    std::shared_ptr<Saved> saved;
+    Saved saved;
     std::vector<float> stage_ms;    // five, when asked for
 };
 
@@ -258,26 +280,6 @@ struct L2Step {     // forward, loss and gradients in one call (tg_render_step_l
 };
 
 constexpr uint32_t kShortList = 128;      // what the compositing kernel sorts itself
-constexpr size_t kAlign = 256;
-size_t up(size_t x) { return (x + kAlign - 1) / kAlign * kAlign; }
-
-std::shared_ptr<Saved> allocate_saved(const View& v, int V, int T, const at::TensorOptions& options) {
-    auto s = std::make_shared<Saved>();
-    s->v = v; s->V = V; s->T = T;
-    const size_t px = (size_t)v.pixels();
-    size_t off = 0;
-    auto take = [&](size_t bytes) { const size_t at = off; off += up(bytes); return at; };
-    const size_t o_fw = take(4 * px), o_ends = take(4 * px), o_geo = take(4 * (size_t)T * TG_GEO_WORDS),
-                 o_attr = take(4 * (size_t)T * TG_ATTR_WORDS), o_off = take(4 * ((size_t)v.tiles() + 1));
-    s->blob = at::empty({(int64_t)off}, options.dtype(at::kByte));
-    char* p = (char*)s->blob.data_ptr();
-    s->final_w = (float*)(p + o_fw);
-    s->ends = (int32_t*)(p + o_ends);
-    s->geo = (float*)(p + o_geo);
-    s->attr = (float*)(p + o_attr);
-    s->offsets = (int32_t*)(p + o_off);
-    return s;
-}
 
 // `opacities` undefined: packed inputs (indices [T,4], colors [V,4]).  Called without the interpreter lock.
 ForwardOut forward(const Tensor& vertices_, const Tensor& indices_, const Tensor& colors_, const Tensor& opacities_,
@@ -292,11 +294,14 @@ ForwardOut forward(const Tensor& vertices_, const Tensor& indices_, const Tensor
     ForwardOut out;
     out.image = at::empty({v.H, v.W, 4}, options);
     out.depthmap = at::empty({v.H, v.W}, options);
-    out.saved = allocate_saved(v, V, T, options);
-    Saved& s = *out.saved;
+    Saved& s = out.saved;
+    s.l = Layout(v, V, T);
+    s.blob = at::empty({(int64_t)s.l.bytes}, options.dtype(at::kByte));
     const int64_t planes = save_selection ? g.selection_planes(v.sort ? 1 : 0, v.layers) : 0;
-    if (planes > 0 && planes * v.pixels() * 4 <= selection_max_bytes)
+    if (planes > 0 && planes * v.pixels() * 4 <= selection_max_bytes) {
+        s.l.planes = (int)planes;
         s.selection = at::empty({planes, v.H, v.W}, options.dtype(at::kInt));
+    }
     if (record_timing) out.stage_ms.resize(5);
     const unsigned fixed_flags = (cull ? TG_FORWARD_CULL_TILES : 0u) | (packed ? TG_INPUT_PACKED : 0u) | TG_INFO_MAPPED;
     const auto state = state_of(w.device, w.stream);
@@ -319,24 +324,23 @@ ForwardOut forward(const Tensor& vertices_, const Tensor& indices_, const Tensor
             step ? g.render_step_l2(data<float>(vertices), data<int32_t>(indices), data<float>(colors), data<float>(opacities),
                                     T, V, v.W, v.H, v.tw, v.th, (float)v.thr, v.layers, step->target, (float)(2.0 / n),
                                     (float)(1.0 / n), step->loss, data<float>(out.image), data<float>(out.depthmap),
-                                    s.final_w, s.ends, s.geo, s.attr, data<int32_t>(s.ids), (uint32_t)cap, s.offsets,
+                                    s.final_w(), s.ends(), s.geo(), s.attr(), s.id_list(), (uint32_t)cap, s.offsets(),
                                     step->gV, step->gC, step->gO, step->mode, ws, have, step->scratch,
                                     step->scratch_bytes, (uint32_t*)info, ms, flags, w.stream)
                  : g.render_forward(data<float>(vertices), data<int32_t>(indices), data<float>(colors),
                                     data<float>(opacities), T, v.W, v.H, v.tw, v.th, (float)v.thr, v.sort ? 1 : 0,
-                                    v.layers, data<float>(out.image), data<float>(out.depthmap), s.final_w, s.ends,
-                                    data<int32_t>(s.selection), s.geo, s.attr, data<int32_t>(s.ids), (uint32_t)cap,
-                                    s.offsets, ws, have, (uint32_t*)info, ms, flags, w.stream);
-        s.K = (uint32_t)info[0];
+                                    v.layers, data<float>(out.image), data<float>(out.depthmap), s.final_w(), s.ends(),
+                                    s.sel(), s.geo(), s.attr(), s.id_list(), (uint32_t)cap, s.offsets(), ws, have, (uint32_t*)info, ms, flags, w.stream);
+        s.l.K = (uint32_t)info[0];
         if (status == TG_ERR_CAPACITY) {
-            cap = s.K + s.K / 4 + 1024;              // what the call says it needs
+            cap = s.l.K + s.l.K / 4 + 1024;              // what the call says it needs
             continue;
         }
         check(step ? "render_step_l2" : "render_forward", status);
         std::copy(key, key + 4, state->ready);
         state->short_lists = (uint32_t)info[1] <= kShortList;
         state->finish_call(slot);
-        state->k_estimate = std::max<int64_t>(s.K, (uint32_t)info[3]);
+        state->k_estimate = std::max<int64_t>(s.l.K, (uint32_t)info[3]);
         return out;
     }
 }
@@ -357,12 +361,14 @@ std::vector<Tensor> backward(Kind kind, const Saved& s, const Tensor& image, con
     check_last_forward(w);
     const auto options = image.options().requires_grad(false);
     std::vector<Tensor> out;
-    out.push_back(at::empty({s.V, 4}, options));
+    const View& v = s.l.v;
+    const int V = s.l.V;
+    out.push_back(at::empty({V, 4}, options));
     if (kind == Kind::kPacked) {
-        out.push_back(at::empty({s.V, 4}, options));
+        out.push_back(at::empty({V, 4}, options));
     } else {
-        out.push_back(at::empty({s.V, 3}, options));
-        out.push_back(at::empty({s.V}, options));
+        out.push_back(at::empty({V, 3}, options));
+        out.push_back(at::empty({V}, options));
     }
     if (!gi.defined() && !gd.defined()) {
         for (auto& t : out) t.zero_();
@@ -370,60 +376,85 @@ std::vector<Tensor> backward(Kind kind, const Saved& s, const Tensor& image, con
     }
     gi = gi.defined() ? gi.contiguous() : at::zeros_like(image);      // only the depth map was used downstream
     gd = gd.defined() ? gd.contiguous() : Tensor();                  // none: taken as zero by the kernel
-    const size_t nscratch = g.backward_scratch_bytes(s.V);
-    const View& v = s.v;
+    const size_t nscratch = g.backward_scratch_bytes(V);
     const auto state = state_of(w.device, w.stream);
     std::lock_guard<std::mutex> lock(state->use);
     if (kind == Kind::kCorrected) {
         const Tensor scratch = at::empty({(int64_t)nscratch}, options.dtype(at::kByte));
         check("blend_backward_corrected",
-              g.blend_backward_corrected(s.geo, s.attr, s.id_list(), s.offsets, s.V, v.W, v.H, v.tw, v.th, v.sort, v.layers,
+              g.blend_backward_corrected(s.geo(), s.attr(), s.id_list(), s.offsets(), V, v.W, v.H, v.tw, v.th, v.sort, v.layers,
                                          data<float>(gi), data<float>(gd), data<float>(image), data<float>(depthmap),
-                                         s.final_w, s.ends, data<float>(out[0]), data<float>(out[1]), data<float>(out[2]),
+                                         s.final_w(), s.ends(), data<float>(out[0]), data<float>(out[1]), data<float>(out[2]),
                                          0, scratch.data_ptr(), nscratch, w.stream));
         return out;
     }
     Accumulator sums(*state, nscratch, options.dtype(at::kByte));
-    check("blend_backward", g.blend_backward(s.geo, s.attr, s.id_list(), s.offsets, s.V, v.W, v.H, v.tw, v.th, v.sort,
+    check("blend_backward", g.blend_backward(s.geo(), s.attr(), s.id_list(), s.offsets(), V, v.W, v.H, v.tw, v.th, v.sort,
                                              v.layers, data<float>(gi), data<float>(gd), data<float>(image),
-                                             data<float>(depthmap), s.final_w, s.ends, s.sel(), nullptr, nullptr, nullptr,
+                                             data<float>(depthmap), s.final_w(), s.ends(), s.sel(), nullptr, nullptr, nullptr,
                                              TG_ACCUMULATE_PACKED, sums.t.data_ptr(), nscratch, w.stream));
     if (kind == Kind::kPacked)
-        check("unpack_gradients_rgba", g.unpack_gradients_rgba(sums.t.data_ptr(), nscratch, s.V, 0.f, nullptr, data<float>(out[0]),
+        check("unpack_gradients_rgba", g.unpack_gradients_rgba(sums.t.data_ptr(), nscratch, V, 0.f, nullptr, data<float>(out[0]),
                                                                data<float>(out[1]), TG_UNPACK_CLEAR, w.stream));
     else
-        check("unpack_gradients", g.unpack_gradients(sums.t.data_ptr(), nscratch, s.V, 0.f, nullptr, data<float>(out[0]),
+        check("unpack_gradients", g.unpack_gradients(sums.t.data_ptr(), nscratch, V, 0.f, nullptr, data<float>(out[0]),
                                                      data<float>(out[1]), data<float>(out[2]), TG_UNPACK_CLEAR, w.stream));
     sums.unpacked();
     return out;
 }
 
+// A tensor that autograd kept: what was saved, or what a saved-tensor hook made of it in between, which only has to have
+// the same device, type and number of elements (`at_least`: or more of them).
+Tensor kept(Tensor t, at::Device device, at::ScalarType type, int64_t numel, bool at_least = false) {
+    TORCH_CHECK(t.defined() && t.device() == device && t.scalar_type() == type &&
+                    (at_least ? t.numel() >= numel : t.numel() == numel),
+                "a tensor saved for backward came back with another device, type or size");
+    t = t.contiguous();
+    return ((uintptr_t)t.data_ptr() & 15) != 0 ? t.clone() : t;      // the kernels load 16 bytes at a time
+}
+struct Kept {
+    Tensor image, depthmap;
+    Saved saved;
+};
+Kept kept_all(const Layout& l, const Tensor& image, const Tensor& depthmap, const Tensor& blob, const Tensor& ids,
+              const Tensor& selection) {
+    const int64_t px = l.v.pixels();
+    const at::Device d = image.device();
+    return {kept(image, d, at::kFloat, 4 * px), kept(depthmap, d, at::kFloat, px),
+            {l, kept(blob, d, at::kByte, (int64_t)l.bytes), kept(ids, d, at::kInt, l.K, true),
+             l.planes > 0 ? kept(selection, d, at::kInt, l.planes * px) : Tensor()}};
+}
+
 struct RenderBackward : public Node {
     Kind kind = Kind::kReference;
-    std::shared_ptr<Saved> saved;      // null: a mesh without triangles
-    SavedVariable image, depthmap;     // outputs of this node
-    std::vector<Tensor> like;          // mesh without triangles: the shapes of the (zero) gradients
+    Layout layout;
+    SavedVariable image, depthmap;           // outputs of this node
+    SavedVariable blob, ids, selection;
+    struct Shape { at::DimVector sizes; at::TensorOptions options; };
+    std::vector<Shape> zeros;                // mesh without triangles: nothing saved, the gradients' shapes
+    bool released = false;
     std::mutex lock;
 
     std::string name() const override { return "RenderBackward"; }
     variable_list apply(variable_list&& grads) override {
         std::lock_guard<std::mutex> hold(lock);
         variable_list out;
-        if (!like.empty()) {
-            for (const auto& t : like) out.push_back(at::zeros_like(t));
+        TORCH_CHECK(!released, torch::autograd::ERR_BACKWARD_TWICE);
+        if (!zeros.empty()) {
+            for (const auto& z : zeros) out.push_back(at::zeros(z.sizes, z.options));
             return out;
         }
-        const Tensor im = image.unpack(shared_from_this()), dm = depthmap.unpack(shared_from_this());
-        TORCH_CHECK(saved, torch::autograd::ERR_BACKWARD_TWICE);
+        const Tensor im = image.unpack(shared_from_this()), dm = depthmap.unpack(shared_from_this()), bl = blob.unpack(),
+                     li = ids.unpack(), se = selection.unpack();
         at::AutoDispatchBelowADInplaceOrView below_autograd;
-        for (auto& t : backward(kind, *saved, im, dm, grads[0], grads[1])) out.push_back(std::move(t));
+        const Kept k = kept_all(layout, im, dm, bl, li, se);
+        for (auto& t : backward(kind, k.saved, k.image, k.depthmap, grads[0], grads[1])) out.push_back(std::move(t));
         return out;
     }
     void release_variables() override {
         std::lock_guard<std::mutex> hold(lock);
-        image.reset_data();
-        depthmap.reset_data();
-        saved.reset();
+        released = true;
+        for (SavedVariable* s : {&image, &depthmap, &blob, &ids, &selection}) s->reset_data();
     }
 };
 
@@ -448,6 +479,7 @@ ImageAndDepth render_graph(Kind kind, const Tensor& vertices, const Tensor& indi
         else node->set_next_edges(torch::autograd::collect_next_edges(vertices, colors, opacities));
     }
     ImageAndDepth r;
+    Saved saved;
     {
         at::AutoDispatchBelowADInplaceOrView below_autograd;
         if (T < 1) {
@@ -457,8 +489,8 @@ ImageAndDepth render_graph(Kind kind, const Tensor& vertices, const Tensor& indi
             r.image.select(2, 3).fill_(1.0);
             r.depthmap = at::full({v.H, v.W}, INFINITY, options);
             if (node) {
-                node->like = {vertices.detach(), colors.detach()};
-                if (kind != Kind::kPacked) node->like.push_back(opacities.detach());
+                for (const Tensor* t : {&vertices, &colors, &opacities})
+                    if (t->defined()) node->zeros.push_back({at::DimVector(t->sizes()), t->options().requires_grad(false)});
             }
         } else {
             // the corrected gradients walk the lists themselves and need no selection; nor does a render nobody differentiates
@@ -467,15 +499,19 @@ ImageAndDepth render_graph(Kind kind, const Tensor& vertices, const Tensor& indi
             r.image = std::move(f.image);
             r.depthmap = std::move(f.depthmap);
             r.stage_ms = std::move(f.stage_ms);
-            if (node) node->saved = std::move(f.saved);
+            saved = std::move(f.saved);
         }
     }
     if (node) {
         torch::autograd::set_history(r.image, node);
         torch::autograd::set_history(r.depthmap, node);
-        if (node->saved) {
+        if (saved.blob.defined()) {
+            node->layout = saved.l;
             node->image = SavedVariable(r.image, /*is_output=*/true);
             node->depthmap = SavedVariable(r.depthmap, /*is_output=*/true);
+            node->blob = SavedVariable(saved.blob, false);
+            node->ids = SavedVariable(saved.ids, false);
+            if (saved.selection.defined()) node->selection = SavedVariable(saved.selection, false);
         }
     }
     return r;
@@ -511,18 +547,18 @@ Tensor l2_step(const Tensor& vertices, const Tensor& indices, const Tensor& colo
         return forward(vertices, indices, colors, opacities, v, false, false, cull, 0, &step).image;
     }
     const ForwardOut f = forward(vertices, indices, colors, opacities, v, false, true, cull, selection_max_bytes);
-    const Saved& s = *f.saved;
+    const Saved& s = f.saved;
     TORCH_CHECK_VALUE(s.selection.defined(), "the fused L2 backward needs per_pixel_sort=True and max_layers <= 32");
     auto backward_into = [&](const Tensor& sums) {
         check("blend_backward_l2",
               target.scalar_type() == at::kByte
-                  ? g.blend_backward_l2_u8(s.geo, s.attr, s.id_list(), s.offsets, V, v.W, v.H, v.tw, v.th, 1, v.layers,
+                  ? g.blend_backward_l2_u8(s.geo(), s.attr(), s.id_list(), s.offsets(), V, v.W, v.H, v.tw, v.th, 1, v.layers,
                                            data<uint8_t>(target), (float)(2.0 / n), (float)(1.0 / n), nullptr,
-                                           data<float>(f.image), data<float>(f.depthmap), s.final_w, s.ends, s.sel(), nullptr,
+                                           data<float>(f.image), data<float>(f.depthmap), s.final_w(), s.ends(), s.sel(), nullptr,
                                            nullptr, nullptr, TG_ACCUMULATE_PACKED, sums.data_ptr(), (size_t)sums.numel(), w.stream)
-                  : g.blend_backward_l2(s.geo, s.attr, s.id_list(), s.offsets, V, v.W, v.H, v.tw, v.th, 1, v.layers,
+                  : g.blend_backward_l2(s.geo(), s.attr(), s.id_list(), s.offsets(), V, v.W, v.H, v.tw, v.th, 1, v.layers,
                                         data<float>(target), (float)(2.0 / n), (float)(1.0 / n), nullptr,
-                                        data<float>(f.image), data<float>(f.depthmap), s.final_w, s.ends, s.sel(), nullptr,
+                                        data<float>(f.image), data<float>(f.depthmap), s.final_w(), s.ends(), s.sel(), nullptr,
                                         nullptr, nullptr, TG_ACCUMULATE_PACKED, sums.data_ptr(), (size_t)sums.numel(), w.stream));
     };
     if (packed) {
@@ -707,11 +743,10 @@ py::object py_render(int kind, const Tensor& vertices, const Tensor& indices, co
 }
 
 // The separate tensors a caller of the forward alone gets: views of the one allocation.
-Tensor part(const Saved& s, const void* p, at::ScalarType type, at::IntArrayRef shape) {
-    const int64_t off = (const char*)p - (const char*)s.blob.data_ptr();
+Tensor part(const Saved& s, size_t place, at::ScalarType type, at::IntArrayRef shape) {
     int64_t n = 4;
     for (int64_t d : shape) n *= d;
-    return s.blob.narrow(0, off, n).view(type).view(shape);
+    return s.blob.narrow(0, (int64_t)place, n).view(type).view(shape);
 }
 
 // opacities None: packed inputs
@@ -725,26 +760,29 @@ py::object py_forward(const Tensor& vertices, const Tensor& indices, const Tenso
         py::gil_scoped_release nogil;
         at::AutoDispatchBelowADInplaceOrView below_autograd;
         f = forward(vertices, indices, colors, or_none(opacities), v, timing, save_selection, cull, selection_max_bytes);
-        const Saved& s = *f.saved;
-        fw = part(s, s.final_w, at::kFloat, {v.H, v.W});
-        ids = s.ids.narrow(0, 0, s.K);
-        off = part(s, s.offsets, at::kInt, {v.tiles() + 1});
-        geo = part(s, s.geo, at::kFloat, {s.T, TG_GEO_WORDS});
-        attr = part(s, s.attr, at::kFloat, {s.T, TG_ATTR_WORDS});
-        ends = part(s, s.ends, at::kInt, {v.H, v.W});
+        const Saved& s = f.saved;
+        const Layout& l = s.l;
+        fw = part(s, l.final_w, at::kFloat, {v.H, v.W});
+        ids = s.ids.narrow(0, 0, l.K);
+        off = part(s, l.offsets, at::kInt, {v.tiles() + 1});
+        geo = part(s, l.geo, at::kFloat, {l.T, TG_GEO_WORDS});
+        attr = part(s, l.attr, at::kFloat, {l.T, TG_ATTR_WORDS});
+        ends = part(s, l.ends, at::kInt, {v.H, v.W});
     }
     return py::make_tuple(f.image, f.depthmap, fw, ids, off, geo, attr, ends,
-                          f.saved->selection.defined() ? py::cast(f.saved->selection) : py::object(py::none()),
-                          timing ? py::cast(f.stage_ms) : py::object(py::none()), f.saved);
+                          f.saved.selection.defined() ? py::cast(f.saved.selection) : py::object(py::none()),
+                          timing ? py::cast(f.stage_ms) : py::object(py::none()), f.saved.l, f.saved.blob);
 }
 
-py::list py_backward(const std::shared_ptr<Saved>& saved, const Tensor& image, const Tensor& depthmap, const Optional& gi,
-                     const Optional& gd) {
+// `blob`, `ids` and `selection` as forward returned them with `layout`.
+py::list py_backward(const Layout& layout, const Tensor& image, const Tensor& depthmap, const Tensor& blob, const Tensor& ids,
+                     const Optional& selection, const Optional& gi, const Optional& gd) {
     std::vector<Tensor> out;
     {
         py::gil_scoped_release nogil;
         at::AutoDispatchBelowADInplaceOrView below_autograd;
-        out = backward(Kind::kReference, *saved, image, depthmap, or_none(gi), or_none(gd));
+        const Kept k = kept_all(layout, image, depthmap, blob, ids, or_none(selection));
+        out = backward(Kind::kReference, k.saved, k.image, k.depthmap, or_none(gi), or_none(gd));
     }
     return py::cast(out);
 }
@@ -843,7 +881,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
             PyErr_SetObject(g_native_error, error.ptr());
         }
     });
-    py::class_<Saved, std::shared_ptr<Saved>>(m, "Saved");
+    py::class_<Layout>(m, "Layout");
     py::class_<DeviceState, std::shared_ptr<DeviceState>>(m, "DeviceState")
         .def_readonly("info", &DeviceState::info)
         .def_readonly("last_slot", &DeviceState::last_slot)

@@ -93,7 +93,7 @@ class Renderer(Function):
         ctx.set_materialize_grads(False)
         timings = None
         if n < 1:
-            ctx.native = None
+            ctx.layout = None
             image = torch.zeros((height, width, 4), dtype=colors.dtype, device=colors.device)
             image[..., 3] = 1.0
             depthmap = torch.full((height, width), float("inf"), dtype=colors.dtype, device=colors.device)
@@ -102,18 +102,18 @@ class Renderer(Function):
             out = N.host().forward(vertices, indices, colors, opacities, width, height, tile_width, tile_height,
                                    early_stopping_threshold, record_timing, per_pixel_sort, max_layers, True,
                                    bool(per_pixel_sort) and CULL_TILES, SELECTION_MAX_BYTES)
-            image, depthmap, timings, ctx.native = out[0], out[1], _timings(out[9]), out[10]
-            ctx.save_for_backward(image, depthmap)
+            image, depthmap, timings, ctx.layout = out[0], out[1], _timings(out[9]), out[10]
+            ctx.save_for_backward(image, depthmap, out[11], out[3], out[8])      # image, depth map, blob, lists, selection
         if record_timing:
             return image, depthmap, timings
         return image, depthmap
 
     @staticmethod
     def backward(ctx, grad_image: torch.Tensor, grad_depthmap: torch.Tensor, grad_timings=None):
-        if ctx.native is None:
+        if ctx.layout is None:
             gV, gC, gO = (torch.zeros_like(t) for t in ctx.saved_tensors)
         else:
-            gV, gC, gO = N.host().backward(ctx.native, *ctx.saved_tensors, grad_image, grad_depthmap)
+            gV, gC, gO = N.host().backward(ctx.layout, *ctx.saved_tensors, grad_image, grad_depthmap)
         return (gV, None, gC, gO, None, None, None, None, None, None, None, None)
 
 
