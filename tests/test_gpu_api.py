@@ -142,6 +142,43 @@ def test_every_entry_point_rejects_tiles_that_are_none(tile):
         assert trigrad_b200.render(v, i[:0], c, o, 32, 32, *tile)[0].shape == (32, 32, 4)
 
 
+@pytest.mark.parametrize("triangles", [0, 2])
+def test_fused_steps_check_a_mesh_without_triangles_like_any_other(triangles):
+    from trigrad_b200 import views
+    v, i, c, o = Hh.scene_tensors(S.large_triangles(2))
+    i = i[:triangles]
+    target = torch.rand((24, 32, 4), device="cuda")
+
+    def step(positions=v, indices=i, colors=c, opacities=o, target=target, tile=16, **k):
+        b = views.GradBuffer.allocate(v.shape[0], "cuda", 4)
+        views.l2_view_step(positions, indices, colors, opacities, target, 32, 24, b.points, b.colors, b.opacities, b.loss, tile, 16, **k)
+        return float(b.loss)
+
+    def world(positions=v[:, :3].contiguous(), pv=np.eye(4), indices=i, colors=c, opacities=o, target=target, tile=16, **k):
+        b = views.GradBuffer.allocate(v.shape[0], "cuda", 3)
+        views.l2_world_view_step(positions, pv, indices, colors, opacities, target, 32, 24, b.points, b.colors, b.opacities, b.loss,
+                                 tile, 16, **k)
+        return float(b.loss)
+
+    for call in (step, world):
+        assert call() > 0
+        assert call(target=(target * 255).to(torch.uint8)) > 0
+        for bad in (dict(target=target[:23]), dict(target=target[..., :3].contiguous()), dict(indices=i[:, :2]),
+                    dict(tile=65), dict(colors=c[:1]), dict(opacities=o[:, None]), dict(max_layers=0),
+                    dict(target=(target * 255).to(torch.uint8), one_kernel=True)):
+            with pytest.raises(ValueError):
+                call(**bad)
+        for bad in (dict(indices=i.long()), dict(target=target.double()), dict(target=target.cpu()), dict(indices=i.cpu()),
+                    dict(positions=v.double())):
+            with pytest.raises(TypeError):
+                call(**bad)
+    with pytest.raises(ValueError):
+        world(pv=np.eye(3))
+    if not triangles:
+        with pytest.raises(ValueError):
+            step(packed=views.PackedGradients(v.shape[0], "cuda"))
+
+
 def test_capacity_regrow_and_reuse():
     """A small scene first, then one with far more (triangle, tile) pairs, then the small one again."""
     small, big = S.large_triangles(2), S.full_screen_layers(50, width=640, height=480)

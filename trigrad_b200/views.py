@@ -132,20 +132,26 @@ def l2_view_step(vertices: torch.Tensor, indices: torch.Tensor, colors: torch.Te
         # 8-bit RGBA target (value / 255): a quarter of the bytes per view; the two-kernel path reads it directly
         raise ValueError("the one-kernel step takes a float32 target")
     if indices.shape[0] < 1:
-        return _empty_mesh_step(vertices, 4, colors, opacities, target, packed, loss)
+        return _empty_mesh_step(vertices, "vertices", 4, indices, colors, opacities, target, width, height, tile_width,
+                                tile_height, packed, loss)
     return N.host().l2_step(vertices, indices, colors, opacities, target, width, height, tile_width, tile_height,
                             early_stopping_threshold, max_layers, grad_vertices, grad_colors, grad_opacities, loss,
                             None if packed is None else packed.scratch, one_kernel and tile_width * tile_height <= 256,
                             cull_tiles, _w.SELECTION_MAX_BYTES, None)
 
 
-def _empty_mesh_step(positions, components, colors, opacities, target, packed, loss):
-    """The background's loss; no gradients and no image."""
+def _empty_mesh_step(positions, name, components, indices, colors, opacities, target, width, height, tile_width, tile_height,
+                     packed, loss):
+    """The background's loss; no gradients and no image.  The arguments are checked as for any other mesh."""
     n, _ = positions.shape
-    _w.check_tensor(positions, "positions", (n, components))
+    _w.check_tensor(positions, name, (n, components))
     _w.check_tensor(colors, "colors", (n, 3))
     _w.check_tensor(opacities, "opacities", (n,))
-    _w.check_tensor(target, "target", dtype=None if target.dtype != torch.uint8 else torch.uint8)
+    m, _ = indices.shape
+    _w.check_tensor(indices, "indices", (m, 3), torch.int32)
+    _w.check_tensor(target, "target", (height, width, 4), None if target.dtype != torch.uint8 else torch.uint8)
+    if tile_width * tile_height > 1024:
+        raise ValueError("tile_width * tile_height must be <= 1024")
     if packed is not None:
         raise ValueError("a mesh without triangles cannot use the packed accumulator")
     tf = target.float() / 255 if target.dtype == torch.uint8 else target
@@ -195,12 +201,14 @@ def l2_world_view_step(points: torch.Tensor, pv, indices: torch.Tensor, colors: 
         raise ValueError("l2_world_view_step needs 1 <= max_layers <= 32")
     if one_kernel and target.dtype == torch.uint8:
         raise ValueError("the one-kernel step takes a float32 target")
+    pv = _pv_host(pv)
     if indices.shape[0] < 1:
-        return _empty_mesh_step(points, 3, colors, opacities, target, packed, loss)
+        return _empty_mesh_step(points, "points", 3, indices, colors, opacities, target, width, height, tile_width,
+                                tile_height, packed, loss)
     return N.host().l2_step(points, indices, colors, opacities, target, width, height, tile_width, tile_height,
                             early_stopping_threshold, max_layers, grad_points, grad_colors, grad_opacities, loss,
                             None if packed is None else packed.scratch, one_kernel and tile_width * tile_height <= 256,
-                            True, _w.SELECTION_MAX_BYTES, _pv_host(pv))
+                            True, _w.SELECTION_MAX_BYTES, pv)
 
 
 def allreduce_gradients(grads: GradBuffer, loss: torch.Tensor | None = None, group=None) -> None:
