@@ -17,6 +17,7 @@
 #include <vector>
 
 #include <ATen/Parallel.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/custom_function.h>
@@ -92,6 +93,20 @@ void need(const Tensor& t, const char* name, std::initializer_list<int64_t> shap
 int64_t rows(const Tensor& t, const char* name) {
     if (t.dim() != 2) throw py::value_error(std::string(name) + " must have two dimensions");
     return t.size(0);
+}
+void need_no_proxies() {
+    TORCH_CHECK(!c10::impl::TorchDispatchModeTLS::any_modes_set() ||
+                    !c10::impl::TorchDispatchModeTLS::get_mode(c10::impl::TorchDispatchModeKey::PROXY),
+                "trigrad_b200 cannot be traced by make_fx");
+}
+// Transforms that the autograd nodes here do not take part in: left alone they would drop tangents or see no kernel at all.
+void need_no_transform(std::initializer_list<const Tensor*> differentiable) {
+    for (const Tensor* t : differentiable)
+        TORCH_CHECK_NOT_IMPLEMENTED(!t->defined() || !t->_fw_grad(/*level=*/0).defined(),
+                                    "trigrad_b200 does not implement forward-mode automatic differentiation");
+    TORCH_CHECK(!c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode),
+                "trigrad_b200 cannot be used inside torch.func transforms (vmap, grad, jvp, jacrev, ...)");
+    need_no_proxies();
 }
 int need_int(int64_t v) {
     TORCH_CHECK(v >= 0 && v <= INT32_MAX, "size out of range");
@@ -721,6 +736,7 @@ py::object py_render(int kind, const Tensor& vertices, const Tensor& indices, co
                      bool sort, int64_t layers, bool cull, int64_t selection_max_bytes) {
     need_tile(tw, th);
     const Tensor opacities = or_none(opacities_);
+    need_no_transform({&vertices, &colors, &opacities});
     const int64_t V = rows(vertices, "vertices");
     need(vertices, "vertices", {V, 4});
     if ((Kind)kind == Kind::kPacked) {
@@ -753,6 +769,7 @@ Tensor part(const Saved& s, size_t place, at::ScalarType type, at::IntArrayRef s
 py::object py_forward(const Tensor& vertices, const Tensor& indices, const Tensor& colors, const Optional& opacities,
                       int64_t W, int64_t H, int64_t tw, int64_t th, double thr, bool timing, bool sort, int64_t layers,
                       bool save_selection, bool cull, int64_t selection_max_bytes) {
+    need_no_proxies();
     const View v = view_of(true, W, H, tw, th, thr, sort, layers);
     ForwardOut f;
     Tensor fw, ids, off, geo, attr, ends;
@@ -831,6 +848,7 @@ void py_project_backward(const Tensor& points, const py::buffer& pv, const Tenso
 
 py::tuple py_project_clip(const Tensor& points, const Tensor& indices, const Tensor& colors, const Tensor& opacities,
                           const py::buffer& pv) {
+    need_no_transform({&points, &colors, &opacities});
     need_mesh(points, "points", 3, indices, colors, opacities);
     const Matrix m = matrix_of(pv);
     std::tuple<Tensor, Tensor, Tensor, Tensor> r;
