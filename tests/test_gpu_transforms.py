@@ -51,3 +51,18 @@ def test_transforms_that_are_not_supported_are_refused(name, triangles):
         with pytest.raises(RuntimeError):
             make_fx(f)(x)
     assert f(x).shape == f(x.clone()).shape
+
+
+@pytest.mark.filterwarnings("ignore::torch.jit.TracerWarning", "ignore::DeprecationWarning")
+@pytest.mark.parametrize("triangles", [300, 0])
+@pytest.mark.parametrize("name", NAMES)
+def test_a_trace_renders_the_inputs_it_is_given(name, triangles):
+    f, x = _calls(triangles)[name]
+    for grad in (False, True):
+        traced = torch.jit.trace(f, (x.clone().requires_grad_(grad),), check_trace=False)
+        y = (0.5 * x).requires_grad_(grad)
+        a, b = traced(y), f(y)
+        assert torch.equal(a, b)
+        if grad:
+            (ga,), (gb,) = torch.autograd.grad(a.sum(), y), torch.autograd.grad(b.sum(), y)
+            assert ga.shape == gb.shape and Hh.rel_l2(ga.cpu().numpy(), gb.cpu().numpy()) <= 1e-5      # order of atomics

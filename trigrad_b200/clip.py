@@ -15,6 +15,7 @@ from __future__ import annotations
 
 import numpy as np
 import torch
+from torch.autograd import Function
 
 from . import _native as N
 
@@ -28,6 +29,23 @@ def _pv_host(pv):
     return m
 
 
+class ProjectClip(Function):
+    """What ``torch.jit.trace`` records of a ``project_clip``."""
+
+    @staticmethod
+    def forward(ctx, points, indices, colors, opacities, pv):
+        ctx.pv = pv
+        ctx.save_for_backward(points, indices, colors, opacities)
+        out = N.host().project_clip(points, indices, colors, opacities, pv)
+        ctx.mark_non_differentiable(out[1])
+        return out
+
+    @staticmethod
+    def backward(ctx, grad_vertices, _, grad_colors, grad_opacities):
+        gp, gc, go = N.host().project_clip_backward(*ctx.saved_tensors, ctx.pv, grad_vertices, grad_colors, grad_opacities)
+        return gp, None, gc, go, None
+
+
 def project_clip(points: torch.Tensor, indices: torch.Tensor, colors: torch.Tensor, opacities: torch.Tensor, pv):
     """World-space mesh -> render-space triangle soup clipped at the near plane.
 
@@ -36,4 +54,6 @@ def project_clip(points: torch.Tensor, indices: torch.Tensor, colors: torch.Tens
     Returns ``(vertices (6T,4), indices (2T,3), colors (6T,3), opacities (6T,))`` ready for ``render``; differentiable
     with respect to points, colours and opacities.
     """
+    if torch._C._get_tracing_state() is not None:
+        return ProjectClip.apply(points, indices, colors, opacities, _pv_host(pv))
     return N.host().project_clip(points, indices, colors, opacities, _pv_host(pv))

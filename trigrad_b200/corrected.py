@@ -11,7 +11,6 @@ number of layers.  In the default mode both functions return the same gradients.
 """
 from __future__ import annotations
 
-from . import _native as N
 from . import wrapper as _w
 
 
@@ -19,7 +18,5 @@ def render_corrected(vertices, indices, colors, opacities, width=500, height=500
                      early_stopping_threshold=1 / 256, record_timing=False, per_pixel_sort=True, max_layers=32):
     """Same contract as ``trigrad_b200.render`` (and the reference's ``trigrad.render``); the gradients are those of
     the rendered image in every mode, see the module docstring."""
-    out = N.host().render(_w.GRADIENTS_CORRECTED, vertices, indices, colors, opacities, width, height, tile_width,
-                          tile_height, early_stopping_threshold, record_timing, per_pixel_sort, max_layers, _w.CULL_TILES,
-                          _w.SELECTION_MAX_BYTES)
-    return (out[0], out[1], _w._timings(out[2])) if record_timing else out
+    return _w.render_of_kind(_w.GRADIENTS_CORRECTED, vertices, indices, colors, opacities, width, height, tile_width,
+                             tile_height, early_stopping_threshold, record_timing, per_pixel_sort, max_layers)

@@ -17,6 +17,7 @@
 #include <vector>
 
 #include <ATen/Parallel.h>
+#include <ATen/TracerMode.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
@@ -309,6 +310,8 @@ ForwardOut forward(const Tensor& vertices_, const Tensor& indices_, const Tensor
     ForwardOut out;
     out.image = at::empty({v.H, v.W, 4}, options);
     out.depthmap = at::empty({v.H, v.W}, options);
+    // a trace records the Python function around this call, for which its outputs have to be known; nothing else
+    at::tracer::impl::NoTracerDispatchMode untraced;
     Saved& s = out.saved;
     s.l = Layout(v, V, T);
     s.blob = at::empty({(int64_t)s.l.bytes}, options.dtype(at::kByte));
@@ -636,6 +639,24 @@ Tensor world_step(const Tensor& points_, const Matrix& pv, const Tensor& indices
 }
 
 // ---- projection with near-plane splitting --------------------------------------------------------------------------
+std::vector<Tensor> project_clip_backward(const Tensor& points, const Tensor& indices, const Tensor& colors,
+                                          const Tensor& opacities, const Matrix& pv, const Tensor& grad_vertices,
+                                          const Tensor& grad_colors, const Tensor& grad_opacities) {
+    at::AutoDispatchBelowADInplaceOrView below_autograd;
+    const Tensor p = points.contiguous(), i = indices.contiguous(), c = colors.contiguous(), o = opacities.contiguous();
+    const Where w(p);
+    const int64_t T = i.size(0);
+    const auto options = p.options().requires_grad(false);
+    auto upstream = [&](const Tensor& t, at::IntArrayRef shape) { return t.defined() ? t.contiguous() : at::zeros(shape, options); };
+    const Tensor gv = upstream(grad_vertices, {6 * T, 4}), gc = upstream(grad_colors, {6 * T, 3}), go = upstream(grad_opacities, {6 * T});
+    std::vector<Tensor> out = {at::zeros_like(p), at::zeros_like(c), at::zeros_like(o)};
+    check("project_clip_backward",
+          g.project_clip_backward(data<float>(p), data<int32_t>(i), data<float>(c), data<float>(o), need_int(T), pv.m,
+                                  data<float>(gv), data<float>(gc), data<float>(go), data<float>(out[0]),
+                                  data<float>(out[1]), data<float>(out[2]), w.stream));
+    return out;
+}
+
 struct ProjectClipBackward : public Node {
     SavedVariable points, indices, colors, opacities;
     Matrix pv;
@@ -644,20 +665,8 @@ struct ProjectClipBackward : public Node {
     std::string name() const override { return "ProjectClipBackward"; }
     variable_list apply(variable_list&& grads) override {
         std::lock_guard<std::mutex> hold(lock);
-        const Tensor p = points.unpack().detach(), i = indices.unpack(), c = colors.unpack().detach(),
-                     o = opacities.unpack().detach();
-        at::AutoDispatchBelowADInplaceOrView below_autograd;
-        const Where w(p);
-        const int64_t T = i.size(0);
-        const auto options = p.options().requires_grad(false);
-        auto upstream = [&](const Tensor& t, at::IntArrayRef shape) { return t.defined() ? t.contiguous() : at::zeros(shape, options); };
-        const Tensor gv = upstream(grads[0], {6 * T, 4}), gc = upstream(grads[1], {6 * T, 3}), go = upstream(grads[2], {6 * T});
-        variable_list out = {at::zeros_like(p), at::zeros_like(c), at::zeros_like(o)};
-        check("project_clip_backward",
-              g.project_clip_backward(data<float>(p), data<int32_t>(i), data<float>(c), data<float>(o), need_int(T), pv.m,
-                                      data<float>(gv), data<float>(gc), data<float>(go), data<float>(out[0]),
-                                      data<float>(out[1]), data<float>(out[2]), w.stream));
-        return out;
+        return project_clip_backward(points.unpack().detach(), indices.unpack(), colors.unpack().detach(),
+                                     opacities.unpack().detach(), pv, grads[0], grads[1], grads[2]);
     }
     void release_variables() override {
         std::lock_guard<std::mutex> hold(lock);
@@ -779,6 +788,7 @@ py::object py_forward(const Tensor& vertices, const Tensor& indices, const Tenso
         f = forward(vertices, indices, colors, or_none(opacities), v, timing, save_selection, cull, selection_max_bytes);
         const Saved& s = f.saved;
         const Layout& l = s.l;
+        at::tracer::impl::NoTracerDispatchMode untraced;
         fw = part(s, l.final_w, at::kFloat, {v.H, v.W});
         ids = s.ids.narrow(0, 0, l.K);
         off = part(s, l.offsets, at::kInt, {v.tiles() + 1});
@@ -792,14 +802,15 @@ py::object py_forward(const Tensor& vertices, const Tensor& indices, const Tenso
 }
 
 // `blob`, `ids` and `selection` as forward returned them with `layout`.
-py::list py_backward(const Layout& layout, const Tensor& image, const Tensor& depthmap, const Tensor& blob, const Tensor& ids,
+py::list py_backward(int kind, const Layout& layout, const Tensor& image, const Tensor& depthmap, const Tensor& blob, const Tensor& ids,
                      const Optional& selection, const Optional& gi, const Optional& gd) {
     std::vector<Tensor> out;
     {
         py::gil_scoped_release nogil;
         at::AutoDispatchBelowADInplaceOrView below_autograd;
         const Kept k = kept_all(layout, image, depthmap, blob, ids, or_none(selection));
-        out = backward(Kind::kReference, k.saved, k.image, k.depthmap, or_none(gi), or_none(gd));
+        at::tracer::impl::NoTracerDispatchMode untraced;
+        out = backward((Kind)kind, k.saved, k.image, k.depthmap, or_none(gi), or_none(gd));
     }
     return py::cast(out);
 }
@@ -859,6 +870,18 @@ py::tuple py_project_clip(const Tensor& points, const Tensor& indices, const Ten
     return py::make_tuple(std::get<0>(r), std::get<1>(r), std::get<2>(r), std::get<3>(r));
 }
 
+py::list py_project_clip_backward(const Tensor& points, const Tensor& indices, const Tensor& colors, const Tensor& opacities,
+                                  const py::buffer& pv, const Optional& gv, const Optional& gc, const Optional& go) {
+    const Matrix m = matrix_of(pv);
+    std::vector<Tensor> out;
+    {
+        py::gil_scoped_release nogil;
+        at::tracer::impl::NoTracerDispatchMode untraced;
+        out = project_clip_backward(points, indices, colors, opacities, m, or_none(gv), or_none(gc), or_none(go));
+    }
+    return py::cast(out);
+}
+
 py::tuple py_pack_mesh(const Tensor& colors_, const Tensor& opacities_, const Tensor& indices_) {
     const int64_t V = rows(colors_, "colors"), T = rows(indices_, "indices");
     need(colors_, "colors", {V, 3});
@@ -914,6 +937,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("project", &py_project);
     m.def("project_backward", &py_project_backward);
     m.def("project_clip", &py_project_clip);
+    m.def("project_clip_backward", &py_project_clip_backward);
     m.def("pack_mesh", &py_pack_mesh);
     m.def("unpack_gradients", &py_unpack_gradients);
 }

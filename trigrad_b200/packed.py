@@ -25,7 +25,5 @@ def render_packed(vertices: torch.Tensor, faces: torch.Tensor, rgba: torch.Tenso
     """``render`` for the packed layout: ``faces`` is ``[T,4]`` int32 (fourth column ignored), ``rgba`` is ``[V,4]``
     (r, g, b, opacity).  Same outputs as ``render(vertices, faces[:, :3], rgba[:, :3], rgba[:, 3], ...)``; gradients
     flow to ``vertices`` and ``rgba``."""
-    out = N.host().render(_w.GRADIENTS_PACKED, vertices, faces, rgba, None, width, height, tile_width, tile_height,
-                          early_stopping_threshold, record_timing, per_pixel_sort, max_layers,
-                          bool(per_pixel_sort) and _w.CULL_TILES, _w.SELECTION_MAX_BYTES)
-    return (out[0], out[1], _w._timings(out[2])) if record_timing else out
+    return _w.render_of_kind(_w.GRADIENTS_PACKED, vertices, faces, rgba, None, width, height, tile_width, tile_height,
+                             early_stopping_threshold, record_timing, per_pixel_sort, max_layers)

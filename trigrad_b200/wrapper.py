@@ -72,25 +72,34 @@ def forward_native(vertices, indices, colors, opacities, width, height, tile_wid
     return (*out[:9], _timings(out[9]))
 
 
-class Renderer(Function):
-    """The autograd function behind ``render``, for callers that use it directly (``Renderer.apply``)."""
+# which gradients a render's backward computes (the host path's enumeration)
+GRADIENTS_REFERENCE, GRADIENTS_CORRECTED, GRADIENTS_PACKED = range(3)
+
+
+class RendererOfKind(Function):
+    """The autograd function behind ``Renderer``, and behind every render that ``torch.jit.trace`` records: the trace keeps
+    a call of it, where it would see nothing of the host path's own nodes.  ``kind``: one of ``GRADIENTS_*``; with
+    ``GRADIENTS_PACKED`` the inputs are vertices, faces, rgba, None."""
 
     @staticmethod
-    def forward(ctx, vertices: torch.Tensor, indices: torch.Tensor, colors: torch.Tensor, opacities: torch.Tensor,
-                width: int = 500, height: int = 500, tile_width: int = 16, tile_height: int = 16,
-                early_stopping_threshold: float = 1 / 256, record_timing: bool = False, per_pixel_sort: bool = True,
-                max_layers: int = 32):
+    def forward(ctx, kind, vertices, indices, colors, opacities, width, height, tile_width, tile_height,
+                early_stopping_threshold, record_timing, per_pixel_sort, max_layers):
+        packed = kind == GRADIENTS_PACKED
         n, _ = vertices.shape
         check_tensor(vertices, "vertices", (n, 4))
-        check_tensor(colors, "colors", (n, 3))
-        check_tensor(opacities, "opacities", (n,))
+        if packed:
+            check_tensor(colors, "rgba", (n, 4))
+        else:
+            check_tensor(colors, "colors", (n, 3))
+            check_tensor(opacities, "opacities", (n,))
         n, _ = indices.shape
-        check_tensor(indices, "indices", (n, 3), torch.int32)
+        check_tensor(indices, "faces" if packed else "indices", (n, 4 if packed else 3), torch.int32)
         if max_layers <= 0:
             max_layers = n + 1
         # an output that was not used downstream arrives in backward as None instead of a tensor of zeros that
         # autograd would have to fill and the kernel to read (the depth map, in the usual image-only loss)
         ctx.set_materialize_grads(False)
+        ctx.kind = kind
         timings = None
         if n < 1:
             ctx.layout = None
@@ -100,8 +109,9 @@ class Renderer(Function):
             ctx.save_for_backward(vertices, colors, opacities)
         else:
             out = N.host().forward(vertices, indices, colors, opacities, width, height, tile_width, tile_height,
-                                   early_stopping_threshold, record_timing, per_pixel_sort, max_layers, True,
-                                   bool(per_pixel_sort) and CULL_TILES, SELECTION_MAX_BYTES)
+                                   early_stopping_threshold, record_timing, per_pixel_sort, max_layers,
+                                   kind != GRADIENTS_CORRECTED,
+                                   (kind == GRADIENTS_CORRECTED or bool(per_pixel_sort)) and CULL_TILES, SELECTION_MAX_BYTES)
             image, depthmap, timings, ctx.layout = out[0], out[1], _timings(out[9]), out[10]
             ctx.save_for_backward(image, depthmap, out[11], out[3], out[8])      # image, depth map, blob, lists, selection
         if record_timing:
@@ -109,16 +119,45 @@ class Renderer(Function):
         return image, depthmap
 
     @staticmethod
-    def backward(ctx, grad_image: torch.Tensor, grad_depthmap: torch.Tensor, grad_timings=None):
+    def backward(ctx, grad_image, grad_depthmap, grad_timings=None):
         if ctx.layout is None:
-            gV, gC, gO = (torch.zeros_like(t) for t in ctx.saved_tensors)
+            grads = [None if t is None else torch.zeros_like(t) for t in ctx.saved_tensors]
         else:
-            gV, gC, gO = N.host().backward(ctx.layout, *ctx.saved_tensors, grad_image, grad_depthmap)
-        return (gV, None, gC, gO, None, None, None, None, None, None, None, None)
+            grads = N.host().backward(ctx.kind, ctx.layout, *ctx.saved_tensors, grad_image, grad_depthmap)
+            if ctx.kind == GRADIENTS_PACKED:
+                grads = [*grads, None]
+        gV, gC, gO = grads
+        return (None, gV, None, gC, gO, None, None, None, None, None, None, None, None)
 
 
-# which gradients a render's backward computes (the host path's enumeration)
-GRADIENTS_REFERENCE, GRADIENTS_CORRECTED, GRADIENTS_PACKED = range(3)
+class Renderer(Function):
+    """The autograd function behind ``render``, for callers that use it directly (``Renderer.apply``)."""
+
+    @staticmethod
+    def forward(ctx, vertices: torch.Tensor, indices: torch.Tensor, colors: torch.Tensor, opacities: torch.Tensor,
+                width: int = 500, height: int = 500, tile_width: int = 16, tile_height: int = 16,
+                early_stopping_threshold: float = 1 / 256, record_timing: bool = False, per_pixel_sort: bool = True,
+                max_layers: int = 32):
+        return RendererOfKind.forward(ctx, GRADIENTS_REFERENCE, vertices, indices, colors, opacities, width, height, tile_width,
+                                      tile_height, early_stopping_threshold, record_timing, per_pixel_sort, max_layers)
+
+    @staticmethod
+    def backward(ctx, grad_image: torch.Tensor, grad_depthmap: torch.Tensor, grad_timings=None):
+        return RendererOfKind.backward(ctx, grad_image, grad_depthmap, grad_timings)[1:]
+
+
+def render_of_kind(kind, vertices, indices, colors, opacities, width, height, tile_width, tile_height,
+                   early_stopping_threshold, record_timing, per_pixel_sort, max_layers):
+    """The call behind ``render``, ``render_corrected`` and ``render_packed``."""
+    if torch._C._get_tracing_state() is not None:
+        if tile_width * tile_height > 1024:
+            raise ValueError("tile_width * tile_height must be <= 1024")
+        return RendererOfKind.apply(kind, vertices, indices, colors, opacities, width, height, tile_width, tile_height,
+                                    early_stopping_threshold, record_timing, per_pixel_sort, max_layers)
+    out = N.host().render(kind, vertices, indices, colors, opacities, width, height, tile_width, tile_height,
+                          early_stopping_threshold, record_timing, per_pixel_sort, max_layers,
+                          (kind == GRADIENTS_CORRECTED or bool(per_pixel_sort)) and CULL_TILES, SELECTION_MAX_BYTES)
+    return (out[0], out[1], _timings(out[2])) if record_timing else out
 
 
 def render(vertices: torch.Tensor, indices: torch.Tensor, colors: torch.Tensor, opacities: torch.Tensor,
@@ -140,7 +179,5 @@ def render(vertices: torch.Tensor, indices: torch.Tensor, colors: torch.Tensor, 
     planes of the image size alive per render until its backward has run (265 MB at 1920x1080), see
     ``SELECTION_MAX_BYTES`` in this module for the switch to the list-searching backward.
     """
-    out = N.host().render(GRADIENTS_REFERENCE, vertices, indices, colors, opacities, width, height, tile_width, tile_height,
-                          early_stopping_threshold, record_timing, per_pixel_sort, max_layers,
-                          bool(per_pixel_sort) and CULL_TILES, SELECTION_MAX_BYTES)
-    return (out[0], out[1], _timings(out[2])) if record_timing else out
+    return render_of_kind(GRADIENTS_REFERENCE, vertices, indices, colors, opacities, width, height, tile_width, tile_height,
+                          early_stopping_threshold, record_timing, per_pixel_sort, max_layers)
