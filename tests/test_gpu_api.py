@@ -179,6 +179,31 @@ def test_fused_steps_check_a_mesh_without_triangles_like_any_other(triangles):
             step(packed=views.PackedGradients(v.shape[0], "cuda"))
 
 
+@pytest.mark.parametrize("which", range(4))
+def test_gradient_tensors_that_kernels_add_to_are_checked(which):
+    from trigrad_b200 import views
+    v, i, c, o = Hh.scene_tensors(S.large_triangles(2))
+    V, target, points, pv = v.shape[0], torch.rand((24, 32, 4), device="cuda"), v[:, :3].contiguous(), np.eye(4)
+    packed = views.PackedGradients(V, "cuda")
+    for p, call in ((4, lambda *g: views.l2_view_step(v, i, c, o, target, 32, 24, *g)),
+                    (4, lambda *g: views.l2_view_step(v, i, c, o, target, 32, 24, *g, one_kernel=True)),
+                    (3, lambda *g: views.l2_world_view_step(points, pv, i, c, o, target, 32, 24, *g)),
+                    (3, lambda *g: views.l2_world_view_step(points, pv, i, c, o, target, 32, 24, *g, packed=packed)),
+                    (4, lambda *g: packed.unpack(32, 24, *g))):
+        b = views.GradBuffer.allocate(V, "cuda", p)
+        good = [b.points, b.colors, b.opacities, b.loss]
+        call(*good)
+        t = good[which]
+        bad = [t.double(), t.cpu(), t.flatten()[:-1]]
+        if t.dim():
+            bad.append(t.repeat_interleave(2, dim=0)[::2])
+        for x in bad:
+            with pytest.raises((TypeError, ValueError)):
+                call(*good[:which], x, *good[which + 1:])
+    with pytest.raises(ValueError):
+        views.project_backward_native(points, pv, torch.zeros_like(v), torch.zeros((3, V), device="cuda").t())
+
+
 def test_capacity_regrow_and_reuse():
     """A small scene first, then one with far more (triangle, tile) pairs, then the small one again."""
     small, big = S.large_triangles(2), S.full_screen_layers(50, width=640, height=480)

@@ -90,6 +90,13 @@ void need(const Tensor& t, const char* name, std::initializer_list<int64_t> shap
     py::reinterpret_borrow<py::object>(g_check_tensor)(t, name, want, py::module_::import("torch").attr(dt));
     throw py::value_error(std::string(name) + ": wrong tensor");
 }
+// A tensor that kernels write or add to, taken as so many consecutive floats.  None where a call can do without.
+void need_out(const Tensor& t, const char* name, int64_t numel) {
+    if (!t.defined()) return;
+    if (!t.is_cuda() || t.scalar_type() != at::kFloat) throw py::type_error(std::string(name) + " must be a float32 tensor on cuda");
+    if (!t.is_contiguous() || t.numel() < numel)
+        throw py::value_error(std::string(name) + " must be contiguous, with " + std::to_string(numel) + " elements");
+}
 // First dimension of a matrix argument (what `n, _ = t.shape` gives).
 int64_t rows(const Tensor& t, const char* name) {
     if (t.dim() != 2) throw py::value_error(std::string(name) + " must have two dimensions");
@@ -834,6 +841,13 @@ Tensor py_l2_step(const Tensor& vertices, const Tensor& indices, const Tensor& c
     need_tile(tw, th);
     const View v = view_of(true, W, H, tw, th, thr, true, layers);
     const Grads to = {or_none(gV), or_none(gC), or_none(gO), or_none(loss), or_none(packed)};
+    const int64_t V = vertices.size(0);
+    if (world || !to.packed.defined()) {
+        need_out(to.vertices, world ? "grad_points" : "grad_vertices", (world ? 3 : 4) * V);
+        need_out(to.colors, "grad_colors", 3 * V);
+        need_out(to.opacities, "grad_opacities", V);
+        need_out(to.loss, "loss", 1);
+    }
     const Matrix m = world ? matrix_of(pv.cast<py::buffer>()) : Matrix{};
     py::gil_scoped_release nogil;
     return world ? world_step(vertices, m, indices, colors, opacities, target, v, to, one_kernel, selection_max_bytes)
@@ -852,6 +866,7 @@ void py_project_backward(const Tensor& points, const py::buffer& pv, const Tenso
     need(points, "points", {V, 3});
     need(gv, "grad_vertices", {V, 4});
     need(gp, "grad_points", {V, 3});
+    need_out(gp, "grad_points", 3 * V);
     const Matrix m = matrix_of(pv);
     py::gil_scoped_release nogil;
     project_backward(points, m, gv, gp, accumulate);
@@ -903,6 +918,10 @@ py::tuple py_pack_mesh(const Tensor& colors_, const Tensor& opacities_, const Te
 
 void py_unpack_gradients(const Tensor& scratch, int64_t V, int64_t W, int64_t H, const Tensor& gV, const Tensor& gC,
                          const Tensor& gO, const Optional& loss, bool accumulate) {
+    need_out(gV, "grad_vertices", 4 * V);
+    need_out(gC, "grad_colors", 3 * V);
+    need_out(gO, "grad_opacities", V);
+    need_out(or_none(loss), "loss", 1);
     py::gil_scoped_release nogil;
     const Where w(gV);
     check("unpack_gradients",
