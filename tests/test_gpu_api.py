@@ -263,6 +263,42 @@ def test_fused_l2_view_step_matches_autograd(tile, one_kernel):
         assert Hh.rel_l2(a.cpu().numpy(), b.cpu().numpy()) <= 1e-5
 
 
+def test_negated_views_are_read_as_what_they_are():
+    """The imaginary part of a conjugate is a view with a flag; kernels see memory."""
+    from trigrad_b200 import views
+    sc = S.random_triangles(300, 64, 48, 0.3, 0.4, name="negated", seed=1)
+    v, i, c, o = Hh.scene_tensors(sc)
+
+    def negated(t):
+        n = torch.complex(torch.zeros_like(t), -t).conj().imag
+        assert n.is_neg() and torch.equal(n, t)
+        return n
+
+    image, depth = trigrad_b200.render(v, i, c, o, 64, 48)
+    for call in (trigrad_b200.render, trigrad_b200.render_corrected, trigrad_b200.Renderer.apply):
+        out = call(negated(v), i, negated(c), negated(o), 64, 48)
+        assert torch.equal(out[0], image) and torch.equal(out[1], depth)
+    x = [t.requires_grad_() for t in (v, c, o)]
+    out = trigrad_b200.render(v, i, c, o, 64, 48)
+    up = [torch.randn_like(t) for t in out]
+    want = torch.autograd.grad(out, x, up, retain_graph=True)
+    for a, b in zip(torch.autograd.grad(out, x, [negated(t) for t in up]), want):
+        assert Hh.rel_l2(a.cpu().numpy(), b.cpu().numpy()) <= 1e-5      # order of atomics
+    target = torch.rand_like(image)
+    steps = []
+    for t in (target, negated(target)):
+        b = views.GradBuffer.allocate(v.shape[0], "cuda", 4)
+        views.l2_view_step(v.detach(), i, c.detach(), o.detach(), t, 64, 48, b.points, b.colors, b.opacities, b.loss)
+        steps.append(b.flat.cpu().numpy())
+    assert Hh.rel_l2(*steps) <= 1e-5
+    pv = S.camera_ring(8)[1]
+    points = v.detach()[:, :3].contiguous()
+    for a, b in zip(trigrad_b200.project_clip(negated(points), i, negated(c.detach()), o.detach(), pv),
+                    trigrad_b200.project_clip(points, i, c.detach(), o.detach(), pv)):
+        assert torch.equal(a, b)
+    assert torch.equal(views.project_native(negated(points), pv), views.project_native(points, pv))
+
+
 def _reference():
     import build_ref
     try:

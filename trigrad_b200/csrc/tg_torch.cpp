@@ -127,6 +127,9 @@ void need_tile(int64_t tw, int64_t th) {
         throw py::value_error("tile_width * tile_height must be <= 1024");
 }
 
+// Its values in memory, in order: a negated view (torch._neg_view, the imaginary part of a conjugate) is not that.
+Tensor plain(const Tensor& t) { return (t.is_neg() ? t.resolve_neg() : t).contiguous(); }
+
 template <class T>
 T* data(const Tensor& t) { return t.defined() ? static_cast<T*>(t.data_ptr()) : nullptr; }
 
@@ -308,9 +311,9 @@ constexpr uint32_t kShortList = 128;      // what the compositing kernel sorts i
 ForwardOut forward(const Tensor& vertices_, const Tensor& indices_, const Tensor& colors_, const Tensor& opacities_,
                    const View& v, bool record_timing, bool save_selection, bool cull, int64_t selection_max_bytes,
                    const L2Step* step = nullptr) {
-    const Tensor vertices = vertices_.contiguous(), indices = indices_.contiguous(), colors = colors_.contiguous();
+    const Tensor vertices = plain(vertices_), indices = plain(indices_), colors = plain(colors_);
     const bool packed = !opacities_.defined();
-    const Tensor opacities = packed ? Tensor() : opacities_.contiguous();
+    const Tensor opacities = packed ? Tensor() : plain(opacities_);
     const Where w(vertices);
     const int T = need_int(indices.size(0)), V = need_int(vertices.size(0));
     const auto options = vertices.options().requires_grad(false);
@@ -399,8 +402,8 @@ std::vector<Tensor> backward(Kind kind, const Saved& s, const Tensor& image, con
         for (auto& t : out) t.zero_();
         return out;
     }
-    gi = gi.defined() ? gi.contiguous() : at::zeros_like(image);      // only the depth map was used downstream
-    gd = gd.defined() ? gd.contiguous() : Tensor();                  // none: taken as zero by the kernel
+    gi = gi.defined() ? plain(gi) : at::zeros_like(image);      // only the depth map was used downstream
+    gd = gd.defined() ? plain(gd) : Tensor();                  // none: taken as zero by the kernel
     const size_t nscratch = g.backward_scratch_bytes(V);
     const auto state = state_of(w.device, w.stream);
     std::lock_guard<std::mutex> lock(state->use);
@@ -434,7 +437,7 @@ Tensor kept(Tensor t, at::Device device, at::ScalarType type, int64_t numel, boo
     TORCH_CHECK(t.defined() && t.device() == device && t.scalar_type() == type &&
                     (at_least ? t.numel() >= numel : t.numel() == numel),
                 "a tensor saved for backward came back with another device, type or size");
-    t = t.contiguous();
+    t = plain(t);
     return ((uintptr_t)t.data_ptr() & 15) != 0 ? t.clone() : t;      // the kernels load 16 bytes at a time
 }
 struct Kept {
@@ -553,7 +556,7 @@ Tensor l2_step(const Tensor& vertices, const Tensor& indices, const Tensor& colo
     const at::AutoDispatchBelowADInplaceOrView below_autograd;
     const Where w(vertices);
     const int V = need_int(vertices.size(0));
-    const Tensor target = target_.contiguous();
+    const Tensor target = plain(target_);
     const size_t nscratch = g.backward_scratch_bytes(V);
     const bool packed = to.packed.defined();
     const double n = 4.0 * v.pixels();
@@ -606,7 +609,7 @@ struct Matrix { float m[16]; };
 
 Tensor project(const Tensor& points_, const Matrix& pv) {
     const at::AutoDispatchBelowADInplaceOrView below_autograd;
-    const Tensor points = points_.contiguous();
+    const Tensor points = plain(points_);
     const Where w(points);
     const Tensor out = at::empty({points.size(0), 4}, points.options().requires_grad(false));
     check("project", g.project(data<float>(points), need_int(points.size(0)), pv.m, data<float>(out), w.stream));
@@ -616,7 +619,7 @@ Tensor project(const Tensor& points_, const Matrix& pv) {
 void project_backward(const Tensor& points_, const Matrix& pv, const Tensor& grad_vertices_, const Tensor& grad_points,
                       bool accumulate) {
     const at::AutoDispatchBelowADInplaceOrView below_autograd;
-    const Tensor points = points_.contiguous(), grad_vertices = grad_vertices_.contiguous();
+    const Tensor points = plain(points_), grad_vertices = plain(grad_vertices_);
     const Where w(points);
     check("project_backward", g.project_backward(data<float>(points), need_int(points.size(0)), pv.m,
                                                  data<float>(grad_vertices), data<float>(grad_points), accumulate, w.stream));
@@ -626,7 +629,7 @@ Tensor world_step(const Tensor& points_, const Matrix& pv, const Tensor& indices
                   const Tensor& opacities, const Tensor& target, const View& v, const Grads& to, bool one_kernel,
                   int64_t selection_max_bytes) {
     const at::AutoDispatchBelowADInplaceOrView below_autograd;
-    const Tensor points = points_.contiguous();
+    const Tensor points = plain(points_);
     const Where w(points);
     const Tensor vertices = project(points, pv);
     if (!to.packed.defined()) {
@@ -650,11 +653,11 @@ std::vector<Tensor> project_clip_backward(const Tensor& points, const Tensor& in
                                           const Tensor& opacities, const Matrix& pv, const Tensor& grad_vertices,
                                           const Tensor& grad_colors, const Tensor& grad_opacities) {
     at::AutoDispatchBelowADInplaceOrView below_autograd;
-    const Tensor p = points.contiguous(), i = indices.contiguous(), c = colors.contiguous(), o = opacities.contiguous();
+    const Tensor p = plain(points), i = plain(indices), c = plain(colors), o = plain(opacities);
     const Where w(p);
     const int64_t T = i.size(0);
     const auto options = p.options().requires_grad(false);
-    auto upstream = [&](const Tensor& t, at::IntArrayRef shape) { return t.defined() ? t.contiguous() : at::zeros(shape, options); };
+    auto upstream = [&](const Tensor& t, at::IntArrayRef shape) { return t.defined() ? plain(t) : at::zeros(shape, options); };
     const Tensor gv = upstream(grad_vertices, {6 * T, 4}), gc = upstream(grad_colors, {6 * T, 3}), go = upstream(grad_opacities, {6 * T});
     std::vector<Tensor> out = {at::zeros_like(p), at::zeros_like(c), at::zeros_like(o)};
     check("project_clip_backward",
@@ -683,8 +686,8 @@ struct ProjectClipBackward : public Node {
 
 std::tuple<Tensor, Tensor, Tensor, Tensor> project_clip(const Tensor& points_, const Tensor& indices_, const Tensor& colors_,
                                                         const Tensor& opacities_, const Matrix& pv) {
-    const Tensor points = points_.contiguous(), indices = indices_.contiguous(), colors = colors_.contiguous(),
-                 opacities = opacities_.contiguous();
+    const Tensor points = plain(points_), indices = plain(indices_), colors = plain(colors_),
+                 opacities = plain(opacities_);
     std::shared_ptr<ProjectClipBackward> node;
     if (at::GradMode::is_enabled() && (points.requires_grad() || colors.requires_grad() || opacities.requires_grad())) {
         node = std::shared_ptr<ProjectClipBackward>(new ProjectClipBackward(), torch::autograd::deleteNode);
@@ -906,7 +909,7 @@ py::tuple py_pack_mesh(const Tensor& colors_, const Tensor& opacities_, const Te
     {
         py::gil_scoped_release nogil;
         const at::AutoDispatchBelowADInplaceOrView below_autograd;
-        const Tensor colors = colors_.contiguous(), opacities = opacities_.contiguous(), indices = indices_.contiguous();
+        const Tensor colors = plain(colors_), opacities = plain(opacities_), indices = plain(indices_);
         const Where w(colors);
         rgba = at::empty({V, 4}, colors.options().requires_grad(false));
         faces = at::empty({T, 4}, indices.options());
