@@ -1,0 +1,147 @@
+"""The state that the host path keeps per stream: shared by threads, by meshes of different size, and over failed calls."""
+import ctypes
+import threading
+
+import numpy as np
+import pytest
+import torch
+
+import helpers as Hh
+import trigrad_b200
+from trigrad_b200 import scenes as S
+from trigrad_b200 import views
+
+pytestmark = pytest.mark.gpu
+
+
+class Job:
+    """A render and its gradients, through autograd or the fused step, with the oracle-free expectation of a lone call."""
+
+    def __init__(self, triangles, width, height, fused, seed):
+        self.size, self.fused = (width, height), fused
+        self.v, self.i, self.c, self.o = Hh.scene_tensors(
+            S.random_triangles(triangles, width, height, 0.2, 0.4, name="host state", seed=seed))
+        self.target = torch.rand((height, width, 4), device="cuda", generator=torch.Generator("cuda").manual_seed(seed))
+        with torch.cuda.stream(torch.cuda.Stream()):
+            torch.cuda.current_stream().wait_stream(torch.cuda.default_stream())
+            self.expected = [t.clone() for t in self.run()]
+            torch.cuda.current_stream().synchronize()
+
+    def run(self):
+        if self.fused:
+            b = views.GradBuffer.allocate(self.v.shape[0], "cuda", 4)
+            image = views.l2_view_step(self.v, self.i, self.c, self.o, self.target, *self.size, b.points, b.colors, b.opacities, b.loss)
+            return image, b.points, b.colors, b.opacities
+        x = [t.detach().requires_grad_() for t in (self.v, self.c, self.o)]
+        image, _ = trigrad_b200.render(x[0], self.i, x[1], x[2], *self.size)
+        return image.detach(), *torch.autograd.grad(torch.mean((image - self.target) ** 2), x)
+
+    def check(self, got):
+        assert torch.equal(got[0], self.expected[0])
+        for a, b in zip(got[1:], self.expected[1:]):
+            assert Hh.rel_l2(a.cpu().numpy(), b.cpu().numpy()) <= 1e-5      # order of atomics
+
+
+def test_threads_that_render_on_one_stream():
+    """Four threads, two streams: two threads on each, with meshes, images and entry points of their own."""
+    jobs = [Job(40, 50, 40, False, 1), Job(20_000, 320, 200, True, 2), Job(3000, 100, 300, False, 3), Job(300, 64, 64, True, 4)]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    results, errors = [[] for _ in jobs], []
+
+    def work(k):
+        try:
+            with torch.cuda.stream(streams[k % 2]):
+                for _ in range(12):
+                    results[k].append(jobs[k].run())
+                torch.cuda.current_stream().synchronize()
+        except BaseException as e:
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(len(jobs))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors
+    for job, got in zip(jobs, results):
+        assert len(got) == 12
+        for g in got:
+            job.check(g)
+
+
+def test_meshes_of_different_size_take_turns_on_one_accumulator():
+    jobs = [Job(50, 64, 64, True, 1), Job(30_000, 400, 300, True, 2), Job(2000, 90, 70, False, 3), Job(60_000, 256, 256, False, 4)]
+    torch.cuda.synchronize()
+    with torch.cuda.stream(torch.cuda.Stream()):
+        for k in (0, 1, 0, 2, 3, 0, 1, 3, 2, 0):
+            jobs[k].check(jobs[k].run())
+
+
+@pytest.mark.parametrize("fused", [True, False])
+def test_an_accumulator_above_the_limit_is_not_kept(fused):
+    """9 million vertices, 288 MB of sums, of which the triangles use the last 3000."""
+    small = Job(1000, 64, 64, fused, 5)
+    n, used = 9_000_000, small.v.shape[0]
+    big = Job.__new__(Job)
+    big.size, big.fused, big.target = small.size, fused, small.target
+    big.i = small.i + (n - used)
+    big.v, big.c, big.o = (torch.zeros((n, *t.shape[1:]), device="cuda") for t in (small.v, small.c, small.o))
+    for b, t in zip((big.v, big.c, big.o), (small.v, small.c, small.o)):
+        b[n - used:] = t
+    small.check(small.run())
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    got = big.run()
+    small.check([got[0]] + [t[n - used:] for t in got[1:]])
+    assert not any(bool(t[:n - used].any()) for t in got[1:])
+    del got
+    assert torch.cuda.memory_allocated() - before < 64 << 20
+    small.check(small.run())
+
+
+def test_calls_after_a_failed_call():
+    job = Job(3000, 100, 80, True, 6)
+    fit = Job(500, 64, 48, False, 7)
+    V = job.v.shape[0]
+    flat = torch.zeros(8 * V + 2, device="cuda")
+    args = (job.v, job.i, job.c, job.o, job.target, *job.size)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(torch.cuda.Stream()):
+        for _ in range(2):
+            # refused by the unpacking, after the sums have been made: the accumulator is not left zero
+            with pytest.raises(RuntimeError, match="aligned"):
+                views.l2_view_step(*args, flat[1:4 * V + 1].view(V, 4), flat[4 * V + 1:7 * V + 1].view(V, 3), flat[7 * V + 1:8 * V + 1],
+                                   flat[8 * V + 1:].view(()))
+            fit.check(fit.run())
+            # refused behind the forward
+            old, trigrad_b200.wrapper.SELECTION_MAX_BYTES = trigrad_b200.wrapper.SELECTION_MAX_BYTES, 0
+            try:
+                with pytest.raises(ValueError):
+                    job.run()
+            finally:
+                trigrad_b200.wrapper.SELECTION_MAX_BYTES = old
+            # refused ahead of it
+            with pytest.raises(RuntimeError):
+                trigrad_b200.render(job.v, job.i, job.c, job.o, -1, 8)
+            job.check(job.run())
+
+
+def test_more_streams_than_states_are_kept():
+    """The state of the stream used least lately is given back, and made anew when the stream comes back."""
+    job = Job(500, 64, 48, False, 8)
+    torch.cuda.synchronize()
+    handles = []
+    for _ in range(140):
+        h = ctypes.c_void_p()
+        assert int(torch.cuda.cudart().cudaStreamCreate(ctypes.addressof(h))) == 0
+        handles.append(h.value)
+    results = []
+    for h in handles + handles[:3]:
+        with torch.cuda.stream(torch.cuda.ExternalStream(h)):
+            results.append(job.run())
+    torch.cuda.synchronize()
+    for got in results:
+        job.check(got)
+    for h in handles:
+        assert int(torch.cuda.cudart().cudaStreamDestroy(h)) == 0
