@@ -299,7 +299,7 @@ int tg_blend_step_l2(const float* tri_geo, const float* tri_attr, const int32_t*
  */
 #define TG_INFO_MAPPED 4u
 /*                TG_EXPECT_SHORT_LISTS: a guess of the caller's (from the call before, say) that no tile list is longer
- *                than 128 entries.  The compositing kernel, which in images of few tiles sorts lists of that length
+ *                than TG_SHORT_LIST entries.  The compositing kernel, which in images of few tiles sorts lists of that length
  *                itself, is then launched before K has reached the host; it does nothing when the guess was wrong, and
  *                the call goes on as without the flag.  Results do not depend on it.  Needs TG_INFO_MAPPED.
  *                TG_WORKSPACE_READY: the workspace was left behind by a successful call on the same stream with the
@@ -307,6 +307,7 @@ int tg_blend_step_l2(const float* tri_geo, const float* tri_attr, const int32_t*
  *                its counters are zero and its tables of tile borders are valid, and are not made again.
  */
 #define TG_EXPECT_SHORT_LISTS 8u
+#define TG_SHORT_LIST 128
 #define TG_WORKSPACE_READY 16u
 size_t tg_forward_workspace_bytes(int T, int tiles, uint32_t list_capacity);
 int tg_render_forward(const float* vertices, const int32_t* indices, const float* colors, const float* opacities,

@@ -16,7 +16,7 @@ constexpr int kSortWarps = kSortThreads / 32;
 constexpr size_t kHistBytes = (size_t)kMaxPasses * kRadix * sizeof(uint32_t);
 constexpr size_t kCtrBytes = 64;
 constexpr int kHistDoneWord = 8;
-// Up to this many tiles the CTA that finishes the fused preprocess kernel last scans the tile counts itself.
+// Up to this many tiles one CTA scans the tile counts: the binning kernel's last one, or bin_finish_kernel's.
 constexpr int kTileScanByLastCta = 65536;
 // Top bit of the longest-list word the binning kernel reports: a launch order of the tiles was written.
 constexpr uint32_t kOrderWrittenBit = 0x80000000u;
@@ -28,7 +28,7 @@ constexpr int kTileSortRank = 128;
 // CTAs.  There a launch and a trip through memory count (1280 triangles, 256x256: 36 -> 27 us with the early launch); with
 // many waves the sort inside takes more of the SMs' time than the kernel of its own does (200k triangles, 1920x1080: 124 us
 // against 110 + 6).
-constexpr uint32_t kFusedList = 128;
+constexpr uint32_t kFusedList = TG_SHORT_LIST;
 constexpr int kFusedTiles = 2 * 4 * 148;
 
 // Exclusive scan of one value per thread over the first 256 threads of a CTA (all threads of the CTA
@@ -54,7 +54,7 @@ __device__ __forceinline__ uint32_t block_exclusive_scan_256(uint32_t v, uint32_
 }
 
 struct HistArgs {
-    uint32_t* hist;           // [kMaxPasses][256] global counts, zeroed by the host; NULL = no histogram
+    uint32_t* hist;           // [kMaxPasses][256] global counts, zeroed by the host
     uint32_t* done_counter;   // zeroed by the host
     int begin_bit, end_bit, passes;
 };
@@ -93,10 +93,6 @@ __device__ __forceinline__ void hist_flush_and_finish(uint32_t* s_hist, uint32_t
 
 namespace tg_host {
 // Internal (not part of the C ABI): the pieces tg_render_forward strings together.
-int sort_pairs(uint64_t* keys_a, uint64_t* keys_b, uint32_t* vals_a, uint32_t* vals_b, uint32_t n, int begin_bit,
-               int end_bit, void* scratch, size_t scratch_bytes, uint32_t* status, int* result_in_b_host,
-               bool scratch_prepared, cudaStream_t stream);
-size_t sort_scratch_clear_bytes(uint32_t n, int passes);
 // Forward compositing with the sort of the tile lists (at most kFusedList entries each, `info` as the binning kernel left
 // it) in the same kernel, which does nothing when a list is longer or the slots exceed `capacity`.
 int blend_forward_short(const float* tri_geo, const float* tri_attr, const uint64_t* entries, const uint32_t* info,

@@ -264,21 +264,21 @@ __global__ void __launch_bounds__(kSmallThreads, 1) onesweep_all_passes_kernel(
 
 }  // namespace tg
 
-namespace tg_host {
-
 static inline int sort_passes(int begin_bit, int end_bit) { return (end_bit - begin_bit + tg::kRadixBits - 1) / tg::kRadixBits; }
 static inline size_t sort_parts(uint32_t n) { return ((size_t)n + tg::kSortTile - 1) / tg::kSortTile; }
 
-size_t sort_scratch_clear_bytes(uint32_t n, int passes) {
+static size_t sort_scratch_bytes(uint32_t n, int passes) {
     return tg::kHistBytes + tg::kCtrBytes + (size_t)passes * sort_parts(n) * tg::kRadix * sizeof(uint64_t);
 }
 
-// scratch_prepared: the caller has zeroed sort_scratch_clear_bytes(>= n) bytes and filled the digit
-// offsets (the key-emission kernel counts digits as it writes keys); then no clearing and no
-// histogram pass are needed here.
-int sort_pairs(uint64_t* keys_a, uint64_t* keys_b, uint32_t* vals_a, uint32_t* vals_b, uint32_t n, int begin_bit,
-               int end_bit, void* scratch, size_t scratch_bytes, uint32_t* status, int* result_in_b_host,
-               bool scratch_prepared, cudaStream_t s) {
+extern "C" {
+
+size_t tg_sort_scratch_bytes(uint32_t n) { return sort_scratch_bytes(n, tg::kMaxPasses); }
+
+int tg_sort_pairs(uint64_t* keys_a, uint64_t* keys_b, uint32_t* vals_a, uint32_t* vals_b, uint32_t n, int begin_bit,
+                  int end_bit, void* scratch, size_t scratch_bytes, uint32_t* status, int* result_in_b_host,
+                  tg_stream_t stream) {
+    cudaStream_t s = (cudaStream_t)stream;
     TG_REQUIRE(begin_bit >= 0 && end_bit <= 64 && begin_bit < end_bit, "bit range");
     TG_REQUIRE(n < 0x80000000u, "n must stay below 2^31");
     const int passes = sort_passes(begin_bit, end_bit);
@@ -288,23 +288,21 @@ int sort_pairs(uint64_t* keys_a, uint64_t* keys_b, uint32_t* vals_a, uint32_t* v
     TG_REQUIRE(keys_a && keys_b && vals_a && vals_b && scratch && status, "null pointer");
     TG_REQUIRE(((uintptr_t)scratch & 15) == 0, "scratch must be 16-byte aligned");
     const size_t parts = sort_parts(n);
-    const size_t need = sort_scratch_clear_bytes(n, passes);
+    const size_t need = sort_scratch_bytes(n, passes);
     if (scratch_bytes < need) {
-        set_error("sort scratch: need %zu bytes, got %zu", need, scratch_bytes);
+        tg_host::set_error("sort scratch: need %zu bytes, got %zu", need, scratch_bytes);
         return TG_ERR_WORKSPACE;
     }
     uint32_t* hist = (uint32_t*)scratch;
     uint32_t* ctr = (uint32_t*)((char*)scratch + tg::kHistBytes);   // [0..7] tickets, [8] histogram-done
     uint64_t* lookback = (uint64_t*)((char*)scratch + tg::kHistBytes + tg::kCtrBytes);
-    if (!scratch_prepared) {
-        TG_CUDA(cudaMemsetAsync(scratch, 0, need, s));
-        int hist_grid = (int)((n + tg::kSortThreads * 16 - 1) / (tg::kSortThreads * 16));
-        if (hist_grid > 148 * 8) hist_grid = 148 * 8;
-        if (hist_grid < 1) hist_grid = 1;
-        const tg::HistArgs h = {hist, ctr + tg::kHistDoneWord, begin_bit, end_bit, passes};
-        tg::sort_histogram_kernel<<<hist_grid, tg::kSortThreads, 0, s>>>(keys_a, n, h);
-        TG_LAUNCH_CHECK("sort_histogram_kernel");
-    }
+    TG_CUDA(cudaMemsetAsync(scratch, 0, need, s));
+    int hist_grid = (int)((n + tg::kSortThreads * 16 - 1) / (tg::kSortThreads * 16));
+    if (hist_grid > 148 * 8) hist_grid = 148 * 8;
+    if (hist_grid < 1) hist_grid = 1;
+    const tg::HistArgs h = {hist, ctr + tg::kHistDoneWord, begin_bit, end_bit, passes};
+    tg::sort_histogram_kernel<<<hist_grid, tg::kSortThreads, 0, s>>>(keys_a, n, h);
+    TG_LAUNCH_CHECK("sort_histogram_kernel");
     static thread_local int cfg_device = -1;
     static thread_local size_t max_resident = 0;      // tiles that can be resident at once (cooperative launch limit)
     int dev = 0;
@@ -349,20 +347,6 @@ int sort_pairs(uint64_t* keys_a, uint64_t* keys_b, uint32_t* vals_a, uint32_t* v
     }
     if (result_in_b_host) *result_in_b_host = passes & 1;
     return TG_OK;
-}
-
-}  // namespace tg_host
-
-extern "C" {
-
-
-size_t tg_sort_scratch_bytes(uint32_t n) { return tg_host::sort_scratch_clear_bytes(n, tg::kMaxPasses); }
-
-int tg_sort_pairs(uint64_t* keys_a, uint64_t* keys_b, uint32_t* vals_a, uint32_t* vals_b, uint32_t n, int begin_bit,
-                  int end_bit, void* scratch, size_t scratch_bytes, uint32_t* status, int* result_in_b_host,
-                  tg_stream_t stream) {
-    return tg_host::sort_pairs(keys_a, keys_b, vals_a, vals_b, n, begin_bit, end_bit, scratch, scratch_bytes, status,
-                               result_in_b_host, false, (cudaStream_t)stream);
 }
 
 }  // extern "C"

@@ -142,7 +142,7 @@ struct DeviceState {
     Tensor workspace, info;      // info [slots,4] int32 pinned: K, longest list, error word, -
     int slot = 0, last_slot = -1;
     int64_t k_estimate = 0;
-    bool short_lists = false;          // the last forward had no tile list beyond kShortList entries
+    bool short_lists = false;          // the last forward had no tile list beyond TG_SHORT_LIST entries
     // image and tile size of the last successful forward, whose counters and tables the workspace still holds; W = 0: none
     int ready[4] = {0, 0, 0, 0};
 
@@ -305,8 +305,6 @@ struct L2Step {     // forward, loss and gradients in one call (tg_render_step_l
     size_t scratch_bytes;
 };
 
-constexpr uint32_t kShortList = 128;      // what the compositing kernel sorts itself
-
 // `opacities` undefined: packed inputs (indices [T,4], colors [V,4]).  Called without the interpreter lock.
 ForwardOut forward(const Tensor& vertices_, const Tensor& indices_, const Tensor& colors_, const Tensor& opacities_,
                    const View& v, bool record_timing, bool save_selection, bool cull, int64_t selection_max_bytes,
@@ -366,7 +364,7 @@ ForwardOut forward(const Tensor& vertices_, const Tensor& indices_, const Tensor
         }
         check(step ? "render_step_l2" : "render_forward", status);
         std::copy(key, key + 4, state->ready);
-        state->short_lists = (uint32_t)info[1] <= kShortList;
+        state->short_lists = (uint32_t)info[1] <= TG_SHORT_LIST;
         state->finish_call(slot);
         state->k_estimate = std::max<int64_t>(s.l.K, (uint32_t)info[3]);
         return out;
