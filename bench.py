@@ -271,13 +271,14 @@ class ViewBatch:
     def render_view(self, v, target, si):
         """fwd + bwd of one view on the current stream (stream slot `si`)."""
         sc, Vw, g = self.scene, self.Vw, self.grads
+        one_kernel = self.one_kernel and target.dtype == self.torch.float32       # which takes no 8-bit targets
         if self.camera_ring:
             Vw.l2_world_view_step(self.points, v, self.i, self.c, self.o, target, self.W, self.H, g.points, g.colors,
-                                  g.opacities, g.loss, sc.tile_width, sc.tile_height, one_kernel=self.one_kernel,
+                                  g.opacities, g.loss, sc.tile_width, sc.tile_height, one_kernel=one_kernel,
                                   packed=self.packed[si])
         else:
             Vw.l2_view_step(v, self.i, self.c, self.o, target, self.W, self.H, None, None, None, None, sc.tile_width,
-                            sc.tile_height, one_kernel=self.one_kernel, packed=self.packed[0])
+                            sc.tile_height, one_kernel=one_kernel, packed=self.packed[0])
 
     def run(self, items):
         """Render (vertices or matrix, target, ready_event) items; returns the summed loss (a view into ``grads``)."""
@@ -800,9 +801,9 @@ def main() -> None:
 # workload, with the summary the figure was read from; the kernels may have changed since that capture.
 NCU_DRAM_BYTES = {
     ("blend_backward_queued_kernel (+ unpack_gradients_kernel)", "cfg3"):
-        (183.2e6 + 11.5e6 + 13.0e6 + 38.4e6, "profiles/blend_kernels_cfg3.md"),
-    ("blend_forward_kernel", "cfg3"): (53.1e6 + 45.5e6, "profiles/blend_kernels_cfg3.md"),
-    ("blend_forward_kernel", "cfg4"): (256.4e6 + 73.5e6, "profiles/blend_forward_cfg4_view.md"),
+        (164.1e6 + 7.1e6 + 38.4e6, "profiles/blend_kernels_cfg3.md"),
+    ("blend_forward_kernel", "cfg3"): (50.1e6 + 38.0e6, "profiles/blend_kernels_cfg3.md"),
+    ("blend_forward_kernel", "cfg4"): (258.1e6 + 26.7e6, "profiles/blend_forward_cfg4_view.md"),
 }
 
 
@@ -839,6 +840,7 @@ def measure_stages(torch, St, scene, verts_np, flush, reps: int) -> dict:
             ms.append(a.elapsed_time(b))
         return statistics.median(ms), out
 
+    from trigrad_b200 import _native as N
     from trigrad_b200 import wrapper as Wr
 
     # forward: the stage times come from events recorded inside the one forward call (L2 flushed before it)
@@ -856,17 +858,21 @@ def measure_stages(torch, St, scene, verts_np, flush, reps: int) -> dict:
     fwd = (image, depth, fw, ends, sel)
     res = {}
     res["init"] = {"kernel": "none (interval between two events)", "ms": med["init"], "bytes": 0}
-    res["binning"] = {"kernel": "bin_kernel", "ms": med["bary_transforms"],
+    res["binning"] = {"kernel": "bin_kernel (+ bin_finish_kernel)", "ms": med["bary_transforms"],
                       "bytes": 12 * T + 32 * V + 164 * T + 16 * K + 8 * tiles}
     res["emit_entries"] = {"kernel": "scatter_entries_kernel (with the wait for K)", "ms": med["per_tile_lists"],
                            "bytes": 24 * K + 8 * tiles}
     res["tile_sort"] = {"kernel": "tile_sort_kernel (+ tile_sort_mid_kernel, tile_sort_long_kernel when needed)", "ms": med["sorting"],
                         "bytes": 12 * K + 8 * tiles}
     res["blend_forward"] = {"kernel": "blend_forward_kernel", "ms": med["rasterization"], "bytes": 100 * K + 28 * W * H}
-    gi = torch.randn((H, W, 4), device="cuda")
-    gd = torch.zeros((H, W), device="cuda")
-    ms, _ = timed(lambda: St.blend_backward(sc, geo, attr, sids, offsets, fwd, gi, gd))
-    res["blend_backward"] = {"kernel": "blend_backward_queued_kernel (+ unpack_gradients_kernel)", "ms": ms, "bytes": 100 * K + 48 * W * H + 32 * V}
+    # the two launches of a single view's fused backward: no depth gradient, an accumulator that stays zero in between
+    target = torch.rand((H, W, 4), device="cuda")
+    sums = torch.zeros(N.lib().tg_backward_scratch_bytes(V), dtype=torch.uint8, device="cuda")
+    grads = [torch.zeros(s, device="cuda") for s in ((V, 4), (V, 3), (V,))]
+    loss = torch.zeros((), device="cuda")
+    ms, _ = timed(lambda: St.backward_l2(sc, geo, attr, sids, offsets, fwd, target, sums, grads, loss))
+    res["blend_backward"] = {"kernel": "blend_backward_queued_kernel (+ unpack_gradients_kernel)", "ms": ms,
+                             "bytes": 100 * K + 36 * W * H + 4 * int(ends.sum()) + 32 * V}
     for s in res.values():
         s["gbs"] = s["bytes"] / (s["ms"] * 1e-3) / 1e9 if s["ms"] > 0 else 0.0
     res["_K"] = K

@@ -13,6 +13,7 @@ LIB_PATH = os.environ.get("TRIGRAD_B200_LIB") or os.path.join(HERE, "libtrigrad_
 
 TG_OK, TG_ERR_BAD_ARG, TG_ERR_WORKSPACE, TG_ERR_CAPACITY, TG_ERR_DEVICE_FLAG, TG_ERR_CUDA = range(6)
 TG_ACCUMULATE_PACKED = 2   # accumulate mode of the backward entry points: the sums stay in the scratch
+TG_UNPACK_CLEAR = 4        # added to `accumulate` of tg_unpack_gradients: the accumulator is zero again afterwards
 TG_FORWARD_CULL_TILES = 1  # flag of the forward entry points: list a (triangle, tile) pair only if it can cover a pixel
 TG_INPUT_PACKED = 2        # flag of the forward entry points: faces [T,4] int32 and colours [V,4] (r, g, b, opacity)
 GEO_WORDS = 16

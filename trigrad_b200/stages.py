@@ -166,6 +166,19 @@ def blend_step_l2(sc, geo, attr, ids, offsets, target, thr=1 / 256, max_layers=3
     return (image, depth, fw, ends), (gV, gC, gO), loss
 
 
+def backward_l2(sc, geo, attr, ids, offsets, fwd, target, sums, grads, loss, max_layers=32):
+    """The backward of mean((image - target)^2) as ``views.l2_view_step`` runs it: into the packed accumulator ``sums``
+    (``tg_backward_scratch_bytes`` bytes, zero before and after), then added to ``grads`` = (gV, gC, gO) and ``loss``."""
+    image, depth, fw, ends, sel = fwd
+    V, npix, (gV, gC, gO) = sc.num_vertices, float(sc.width * sc.height * 4), grads
+    N.check("blend_backward_l2", N.lib().tg_blend_backward_l2(
+        ptr(geo), ptr(attr), ptr(ids), ptr(offsets), V, sc.width, sc.height, sc.tile_width, sc.tile_height, 1, int(max_layers),
+        ptr(target), 2.0 / npix, 1.0 / npix, None, ptr(image), ptr(depth), ptr(fw), ptr(ends), ptr(sel), None, None, None,
+        N.TG_ACCUMULATE_PACKED, ptr(sums), sums.numel(), stream()))
+    N.check("unpack_gradients", N.lib().tg_unpack_gradients(ptr(sums), sums.numel(), V, 1.0 / npix, ptr(loss), ptr(gV), ptr(gC),
+                                                            ptr(gO), 1 | N.TG_UNPACK_CLEAR, stream()))
+
+
 def blend_backward(sc, geo, attr, ids, offsets, fwd, gimage, gdepth, per_pixel_sort=True, max_layers=32):
     image, depth, fw, ends, sel = fwd
     V = sc.num_vertices
