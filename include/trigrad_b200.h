@@ -25,8 +25,8 @@
  *   - per host thread: the text behind tg_last_error(); one cudaEvent_t per device (marks "K has
  *     reached the host" inside tg_render_forward); the occupancy figures of the radix-sort kernels
  *     for the device last used by that thread;
- *   - per process: an atomic launch counter (tg_launch_count); per device, atomically, "the opt-in
- *     shared-memory size of the long tile sort has been set" and the device address of the fixed
+ *   - per process: an atomic launch counter (tg_launch_count); per device, atomically, which kernels'
+ *     shared-memory sizes and preferences have been set and the device address of the fixed
  *     array behind tg_scan_static.  These belong to the device's primary context: a program that
  *     resets a device (cudaDeviceReset) must not call the library on it afterwards.
  */

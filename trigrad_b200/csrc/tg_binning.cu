@@ -530,9 +530,10 @@ __global__ void __launch_bounds__(kEmitThreads) emit_keys_kernel(const float4* _
 // that need the polygon clipper are put off to the end of the CTA when they are few in a warp, and run there with full
 // warps.
 // The CTA that finishes last turns the counts into tile offsets; the scatter kernel then moves every entry to
-// offset + rank.  Against counting and writing in two kernels, which gathered, tested and searched twice, B200: 1.3M triangles of a pixel
-// each, full HD: 281 -> 188 us; 200k triangles, full HD: 65 -> 46; 2M triangles, 4K: 791 -> 510; 3000 triangles of 200
-// tiles each: 294 -> 28.  Bound by instruction issue and shared-memory wavefronts (61 %) in turns with the barriers.
+// offset + rank.  Against counting and writing in two kernels, which gathered, tested and searched twice, B200, with the
+// scatter: 1.3M triangles of a pixel each, full HD: 281 -> 170 us (this kernel 141); 200k triangles, full HD: 65 -> 36 (31);
+// 2M triangles, 4K: 791 -> 477 (387).  Bound by latency: at 52 % of the issue slots, 38 % of L1 and 8 % of DRAM (200k
+// triangles) its warps wait first for the gathers and for the rank atomics, then for one another at the barriers.
 struct BinArgs {
     uint32_t* tile_counts;   // [tiles], zero on entry
     int32_t* offsets;        // [tiles + 1], written when scan_here
@@ -889,7 +890,7 @@ int prefer_smem(const void* kernel, int kilobytes, SmemAllowed& preferred) {
 }
 
 // Per-triangle records, (triangle, tile) pairs and tile offsets: bin_init_kernel, bin_kernel and scatter_entries_kernel
-// (declared in tg_common.cuh with what each argument is).
+// (declared in tg_radix.cuh with what each argument is).
 int bin_triangles(const float* vertices, const int32_t* indices, const float* colors, const float* opacities, int T, int W,
                   int H, int tw, int th, float* tri_geo, float* tri_attr, const BinBuffers& b, int32_t* offsets,
                   uint32_t list_capacity, uint32_t* info_host, bool cull, bool packed, bool ready, cudaStream_t stream) {

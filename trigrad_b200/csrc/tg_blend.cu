@@ -16,9 +16,10 @@
 //     the CTA leaves the list as soon as every warp voted "done".
 //
 // Backward: per pixel the recorded fragments are walked last to first with the reference's
-// recurrences; every lane adds its contribution with 128-bit vector reductions
-// (red.global.add.v4.f32) into a packed per-vertex buffer (x, y, w, opacity | r, g, b, -) that a
-// small kernel then unpacks into grad_vertices / grad_colors / grad_opacities.
+// recurrences; the contributions of a warp's lanes are summed per triangle, and the sums go to a packed
+// per-vertex buffer (x, y, w, opacity | r, g, b, -), mostly with one 24-lane atomic addition per triangle
+// (lanes of which too few share a triangle add for themselves, with red.global.add.v4.f32).  A small kernel
+// unpacks the buffer into grad_vertices / grad_colors / grad_opacities.
 #include "tg_radix.cuh"
 
 namespace tg {
@@ -369,7 +370,8 @@ __device__ __forceinline__ unsigned cover_rows(const float* m, const float* s_x 
     return cover;
 }
 
-// 32x32 bit matrix, one row per lane, transposed: bit k of lane p becomes bit p of lane k.
+// 32x32 bit matrix, one row per lane, transposed: bit k of lane p becomes bit p of lane k.  The recursive exchange of
+// blocks of H. S. Warren, Hacker's Delight, section 7-3, with the rows in lanes.
 __device__ __forceinline__ unsigned transpose_bits(unsigned x) {
     const unsigned lane = lane_id();
     unsigned m = 0x0000ffffu;
@@ -953,7 +955,8 @@ __device__ __forceinline__ int load_pixel_state(const TileCtx& c, const BlendPar
 // gradients of the fragment's interpolations; these go into a queue in shared memory; part B (the
 // expensive barycentric partials and the 21 per-vertex outputs) pops 32 queued fragments at a time and
 // so runs with full warps.  A warp whose lanes are busy anyway (deep overlap, or one opaque layer everywhere) skips the
-// queue.  (Bound by L1 data wavefronts, 78 %, and by the latency of the gathers.)
+// queue.  (200k triangles, full HD: 148 us at 70 % of L1, 64 % of the issue slots and 14 % of DRAM; bound by the latency of
+// the gathers, fifteen of 16 bytes per fragment, and by L1 together.)
 // DEPTH = false (everywhere below): no gradient flows into the depth map, the terms that it feeds are left out.
 struct QueuedFragment {
     float px, py;
@@ -1289,6 +1292,11 @@ __global__ void __launch_bounds__(MAXT, DEPTH ? 7 : 8) blend_backward_queued_ker
 // fragment (opacity, colour, 1/w, barycentrics) are kept in local memory and feed the recurrence
 // directly: no second pass over geometry and attributes for it, no selection planes, no re-read of the
 // image; the per-vertex outputs go through the per-warp queue as in blend_backward_queued_kernel.
+// Slower than the two kernels in most places by now, as it has none of their staging ahead of the pixel set-up, streamed
+// lists and dependent launches, and its half for the forward runs with the registers of both (a step, B200: 200k triangles,
+// full HD 317 us in two kernels against 355 in one; 2M triangles, 4K 2038 against 2301; 10k, 512x512 60 against 73; four
+// streams of views, full HD 277 against 296 per view).  Faster where triangles are a pixel each and a pixel blends one
+// fragment or none (1.3M triangles, full HD 594 against 561).  Used on request only.
 template <int MAXT>
 __global__ void __launch_bounds__(MAXT, 4) blend_step_l2_kernel(BlendParams P, float4* __restrict__ image,
                                                                 float* __restrict__ depthmap, float* __restrict__ final_w,
@@ -1757,7 +1765,12 @@ int tg_blend_forward(const float* tri_geo, const float* tri_attr, const int32_t*
     const int threads = ((tw * th + 31) / 32) * 32;
     cudaStream_t s = (cudaStream_t)stream;
     float4* img = (float4*)image;
-    // lists well beyond one staged chunk (the binning kernel of the same call reported the longest): stream them
+    // Lists well beyond one staged chunk (the binning kernel of the same call reported the longest): stream them, and filter
+    // them by depth once the batches are full.  Streaming moves a chunk with one quad per thread, which takes 256 threads.
+    // The filter alone in smaller CTAs gains where almost all of a list lies behind the batches and loses elsewhere, with
+    // its barriers over the few records that a small tile's chunk leaves to each warp (forward, 8x8 tiles: 2M triangles
+    // piled up, 4K 1612 -> 1468 us, but 200k piled up, full HD 585 -> 700, 300k spread, 1001x777 748 -> 1124, 20k, 512x512,
+    // lists of 375 205 -> 258; 4x4 tiles, 400k, full HD 4115 -> 6640); CTAs of more than 256 threads have it always.
     const bool stream_lists = threads == 256 && tg_host::g_longest_list > 2u * tg::kChunk;
     auto kernel = threads > 256 ? (per_pixel_sort ? tg::blend_forward_kernel<true, 1024> : tg::blend_forward_kernel<false, 1024>)
                   : !per_pixel_sort ? tg::blend_forward_kernel<false, 256>
@@ -1818,8 +1831,8 @@ static int backward_impl(const float* tri_geo, const float* tri_attr, const int3
     if (saved) {
         // The queued kernel walks the per-pixel selection, not the tile lists, so its blocks need not be the
         // forward's tiles: 16x8 pixels (four warps) finish more evenly than whole tiles do, and a block's
-        // registers come free only when its slowest warp is done (config 3: 179 -> 173 µs; 64 threads the
-        // same, 32 threads slower again).
+        // registers come free only when its slowest warp is done (200k triangles, full HD, when it was made: 179 -> 173
+        // us; 64 threads the same, 32 threads slower again).
         tg::BlendParams Q = P;
         Q.tw = 16; Q.th = 8;
         Q.tiles_x = (W + Q.tw - 1) / Q.tw;

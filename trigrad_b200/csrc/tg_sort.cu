@@ -1,12 +1,11 @@
 // Stage 4: onesweep least-significant-digit radix sort of (uint64 key, uint32 value) pairs.
 //
-// The digits of every pass are counted in a single read of the keys (here, or on the fly by the
-// key-emission kernel) and turned into global digit offsets.  Then one kernel per pass: each CTA
+// The digits of every pass are counted in a single read of the keys and turned into global digit offsets.  Then one kernel per pass: each CTA
 // takes a tile of pairs (ticket order), ranks them stably by the pass digit (per-warp ballots, one
 // per digit bit), publishes its per-digit counts, obtains the counts of all earlier tiles by
 // decoupled look-back (one thread per digit, bounded waits) and scatters keys and values through
 // shared memory so that global writes are contiguous runs per digit.  Every pass reads 12 B and
-// writes 12 B per pair: HBM-bound.
+// writes 12 B per pair; at 2^27 pairs that runs at 39 % of the copy rate.
 #include "tg_radix.cuh"
 
 #ifndef TG_SORT_THREADS
@@ -62,7 +61,7 @@ struct SortSmemT {
     uint32_t fail;
 };
 using SortSmem = SortSmemT<kPassThreads, kPassItems>;
-// Shape of the single-launch path for small inputs.  Measured on config 3 (338k pairs): 256x16 tiles 13 us
+// Shape of the single-launch path for small inputs.  Measured at 338k pairs: 256x16 tiles 13 us
 // per pass, 512x16 with all peer masks computed up front 15 us - the per-item ballot + offset chain
 // (about 0.25 us per item and warp) and the prefix chain between tiles dominate, not the launches.
 constexpr int kSmallThreads = 256;
