@@ -11,6 +11,7 @@ number of layers.  In the default mode both functions return the same gradients.
 """
 from __future__ import annotations
 
+from . import _native as N
 from . import wrapper as _w
 
 
@@ -18,5 +19,10 @@ def render_corrected(vertices, indices, colors, opacities, width=500, height=500
                      early_stopping_threshold=1 / 256, record_timing=False, per_pixel_sort=True, max_layers=32):
     """Same contract as ``trigrad_b200.render`` (and the reference's ``trigrad.render``); the gradients are those of
     the rendered image in every mode, see the module docstring."""
-    return _w.render_of_kind(_w.GRADIENTS_CORRECTED, vertices, indices, colors, opacities, width, height, tile_width,
-                             tile_height, early_stopping_threshold, record_timing, per_pixel_sort, max_layers)
+    out = N.host().render(_w.GRADIENTS_CORRECTED, vertices, indices, colors, opacities, width, height, tile_width,
+                          tile_height, early_stopping_threshold, record_timing, per_pixel_sort, max_layers, _w.CULL_TILES,
+                          _w.SELECTION_MAX_BYTES)
+    if record_timing or out is None:
+        return _w.finish_render(out, _w.GRADIENTS_CORRECTED, vertices, indices, colors, opacities, width, height, tile_width,
+                                tile_height, early_stopping_threshold, record_timing, per_pixel_sort, max_layers)
+    return out

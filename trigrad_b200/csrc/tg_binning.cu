@@ -679,9 +679,12 @@ __global__ void __launch_bounds__(32 * kBinWarps, 32 / kBinWarps) bin_kernel(con
             const uint32_t y = __shfl_up_sync(0xffffffffu, incl, d);
             if (lane >= d) incl += y;
         }
-        // A triangle has fewer than 2^31 pairs, but 32 of them can have more than 32 bits hold: the sum in halves, cut off
-        const uint32_t low = __reduce_add_sync(0xffffffffu, count & 0xffffu), high = __reduce_add_sync(0xffffffffu, count >> 16);
-        total = (uint32_t)min(((uint64_t)high << 16) + low, (uint64_t)UINT32_MAX);
+        total = __shfl_sync(0xffffffffu, incl, 31);
+        if (__any_sync(0xffffffffu, count >= 1u << 27)) {
+            // A triangle has fewer than 2^31 pairs, but 32 of them can have more than 32 bits hold: the sum in halves, cut off
+            const uint32_t low = __reduce_add_sync(0xffffffffu, count & 0xffffu), high = __reduce_add_sync(0xffffffffu, count >> 16);
+            total = (uint32_t)min(((uint64_t)high << 16) + low, (uint64_t)UINT32_MAX);
+        }
         mine[32 * kTriFirst + lane] = __uint_as_float(incl - count);
     }
     if (lane == 0) s_warp[warp] = total;
@@ -694,7 +697,7 @@ __global__ void __launch_bounds__(32 * kBinWarps, 32 / kBinWarps) bin_kernel(con
         uint64_t sum = 0;
 #pragma unroll
         for (int w = 0; w < kBinWarps; w++) { s_first[w] = (uint32_t)sum; sum += s_warp[w]; }
-        const uint64_t at = sum ? atomicAdd(slot_counter(bin), (unsigned long long)sum) : 0;
+        const uint64_t at = atomicAdd(slot_counter(bin), (unsigned long long)sum);
         s_first[kBinWarps] = at + sum < kTooManyPairs ? (uint32_t)sum : 0u;
         s_base = (uint32_t)at;
     }

@@ -24,6 +24,7 @@
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/extension.h>
 
 #include "../../include/trigrad_b200.h"
@@ -752,6 +753,7 @@ py::object py_render(int kind, const Tensor& vertices, const Tensor& indices, co
                      const Optional& opacities_, int64_t W, int64_t H, int64_t tw, int64_t th, double thr, bool timing,
                      bool sort, int64_t layers, bool cull, int64_t selection_max_bytes) {
     need_tile(tw, th);
+    if (torch::jit::tracer::isTracing()) return py::none();          // the caller's autograd function is what a trace can hold
     const Tensor opacities = or_none(opacities_);
     need_no_transform({&vertices, &colors, &opacities});
     const int64_t V = rows(vertices, "vertices");

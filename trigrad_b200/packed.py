@@ -25,5 +25,10 @@ def render_packed(vertices: torch.Tensor, faces: torch.Tensor, rgba: torch.Tenso
     """``render`` for the packed layout: ``faces`` is ``[T,4]`` int32 (fourth column ignored), ``rgba`` is ``[V,4]``
     (r, g, b, opacity).  Same outputs as ``render(vertices, faces[:, :3], rgba[:, :3], rgba[:, 3], ...)``; gradients
     flow to ``vertices`` and ``rgba``."""
-    return _w.render_of_kind(_w.GRADIENTS_PACKED, vertices, faces, rgba, None, width, height, tile_width, tile_height,
-                             early_stopping_threshold, record_timing, per_pixel_sort, max_layers)
+    out = N.host().render(_w.GRADIENTS_PACKED, vertices, faces, rgba, None, width, height, tile_width, tile_height,
+                          early_stopping_threshold, record_timing, per_pixel_sort, max_layers,
+                          bool(per_pixel_sort) and _w.CULL_TILES, _w.SELECTION_MAX_BYTES)
+    if record_timing or out is None:
+        return _w.finish_render(out, _w.GRADIENTS_PACKED, vertices, faces, rgba, None, width, height, tile_width, tile_height,
+                                early_stopping_threshold, record_timing, per_pixel_sort, max_layers)
+    return out

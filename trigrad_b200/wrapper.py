@@ -146,18 +146,12 @@ class Renderer(Function):
         return RendererOfKind.backward(ctx, grad_image, grad_depthmap, grad_timings)[1:]
 
 
-def render_of_kind(kind, vertices, indices, colors, opacities, width, height, tile_width, tile_height,
-                   early_stopping_threshold, record_timing, per_pixel_sort, max_layers):
-    """The call behind ``render``, ``render_corrected`` and ``render_packed``."""
-    if torch._C._get_tracing_state() is not None:
-        if tile_width * tile_height > 1024:
-            raise ValueError("tile_width * tile_height must be <= 1024")
-        return RendererOfKind.apply(kind, vertices, indices, colors, opacities, width, height, tile_width, tile_height,
-                                    early_stopping_threshold, record_timing, per_pixel_sort, max_layers)
-    out = N.host().render(kind, vertices, indices, colors, opacities, width, height, tile_width, tile_height,
-                          early_stopping_threshold, record_timing, per_pixel_sort, max_layers,
-                          (kind == GRADIENTS_CORRECTED or bool(per_pixel_sort)) and CULL_TILES, SELECTION_MAX_BYTES)
-    return (out[0], out[1], _timings(out[2])) if record_timing else out
+def finish_render(out, *args):
+    """What the host path's ``render`` does not return by itself: stage times as a dict, and nothing while a trace is being
+    recorded - the call then goes through a node that the trace sees.  ``args``: those of ``RendererOfKind``."""
+    if out is None:
+        return RendererOfKind.apply(*args)
+    return out[0], out[1], _timings(out[2])
 
 
 def render(vertices: torch.Tensor, indices: torch.Tensor, colors: torch.Tensor, opacities: torch.Tensor,
@@ -179,5 +173,10 @@ def render(vertices: torch.Tensor, indices: torch.Tensor, colors: torch.Tensor, 
     planes of the image size alive per render until its backward has run (265 MB at 1920x1080), see
     ``SELECTION_MAX_BYTES`` in this module for the switch to the list-searching backward.
     """
-    return render_of_kind(GRADIENTS_REFERENCE, vertices, indices, colors, opacities, width, height, tile_width, tile_height,
-                          early_stopping_threshold, record_timing, per_pixel_sort, max_layers)
+    out = N.host().render(GRADIENTS_REFERENCE, vertices, indices, colors, opacities, width, height, tile_width, tile_height,
+                          early_stopping_threshold, record_timing, per_pixel_sort, max_layers,
+                          bool(per_pixel_sort) and CULL_TILES, SELECTION_MAX_BYTES)
+    if record_timing or out is None:
+        return finish_render(out, GRADIENTS_REFERENCE, vertices, indices, colors, opacities, width, height, tile_width, tile_height,
+                             early_stopping_threshold, record_timing, per_pixel_sort, max_layers)
+    return out
