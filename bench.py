@@ -858,11 +858,11 @@ def measure_stages(torch, St, scene, verts_np, flush, reps: int) -> dict:
     fwd = (image, depth, fw, ends, sel)
     res = {}
     res["init"] = {"kernel": "none (interval between two events)", "ms": med["init"], "bytes": 0}
-    res["binning"] = {"kernel": "bin_kernel (+ bin_finish_kernel)", "ms": med["bary_transforms"],
+    res["binning"] = {"kernel": "bin_kernel", "ms": med["bary_transforms"],
                       "bytes": 12 * T + 32 * V + 164 * T + 16 * K + 8 * tiles}
-    res["emit_entries"] = {"kernel": "scatter_entries_kernel (with the wait for K)", "ms": med["per_tile_lists"],
+    res["emit_entries"] = {"kernel": "place_entries_kernel", "ms": med["per_tile_lists"],
                            "bytes": 24 * K + 8 * tiles}
-    res["tile_sort"] = {"kernel": "tile_sort_kernel (+ tile_sort_mid_kernel, tile_sort_long_kernel when needed)", "ms": med["sorting"],
+    res["tile_sort"] = {"kernel": "tile_sort_kernel (+ tile_sort_mid_kernel, tile_sort_long_kernel when needed; with the wait for K)", "ms": med["sorting"],
                         "bytes": 12 * K + 8 * tiles}
     res["blend_forward"] = {"kernel": "blend_forward_kernel", "ms": med["rasterization"], "bytes": 100 * K + 28 * W * H}
     # the two launches of a single view's fused backward: no depth gradient, an accumulator that stays zero in between

@@ -149,7 +149,7 @@ def test_forward_entry_lists_bit_exact(pipeline):
 
 
 def test_forward_entry_more_tiles_than_one_cta_scans():
-    """Beyond 65536 tiles the tile offsets come from the device-wide scan instead of the last CTA."""
+    """Beyond 65536 tiles the tile offsets come from the device-wide scan instead of one CTA."""
     sc = S.random_triangles(6000, 2100, 2100, 0.02, 0.6, name="many_tiles")
     sc.tile_width = sc.tile_height = 8
     assert Hh.num_tiles(sc) > 65536
@@ -157,6 +157,38 @@ def test_forward_entry_more_tiles_than_one_cta_scans():
     li = O.build_lists(sc.vertices, sc.indices, sc.width, sc.height, sc.tile_width, sc.tile_height)
     assert np.array_equal(offsets, li.offsets)
     assert np.array_equal(ids, li.ids)
+
+
+@pytest.mark.parametrize("tiles_x, tiles_y", [
+    (1, 1), (7, 73), (16, 32), (19, 27),                  # 511, 512, 513: a round of one warp
+    (64, 128), (3, 2731), (128, 128), (145, 113),         # 8192, 8193: a round of 512 threads; 16384, 16385: the larger CTA
+    (220, 256), (220, 257),                               # the most tiles every CTA scans, and more
+])
+def test_offsets_and_places_by_number_of_tiles(tiles_x, tiles_y):
+    """Tile offsets and entries at the edges of the scan's rounds and of the kernels' ranges; three calls in a row, which
+    find the counters as the one before left them."""
+    for seed in range(3):
+        sc = S.random_triangles(3000 - 1000 * seed, 4 * tiles_x - 1, 4 * tiles_y - 2, 0.03, 0.6, name=f"tiles_{seed}", seed=seed)
+        sc.tile_width = sc.tile_height = 4
+        ids, offsets, _ = _forward_entry_lists(sc)
+        li = O.build_lists(sc.vertices, sc.indices, sc.width, sc.height, sc.tile_width, sc.tile_height)
+        assert np.array_equal(offsets, li.offsets)
+        assert np.array_equal(ids, li.ids)
+
+
+@pytest.mark.parametrize("width, height", [(300, 205), (2048, 33), (97, 31)])
+def test_launch_order_takes_every_tile_once(width, height):
+    """Long and uneven lists, for which the tiles are launched by length: every length class, tile counts off any round."""
+    sc = S.random_triangles(12_000, width, height, 0.3, 0.9, name="order", seed=width)
+    sc.vertices[::2, :2] *= 0.3                           # half of them piled up in the middle
+    ids, offsets, image = _forward_entry_lists(sc)
+    li = O.build_lists(sc.vertices, sc.indices, sc.width, sc.height, sc.tile_width, sc.tile_height)
+    n = np.diff(li.offsets)
+    assert n.max() >= 256 and n.mean() >= 64              # what an order is made for
+    assert np.array_equal(ids, li.ids)
+    of = O.forward(sc.vertices, sc.indices, sc.colors, sc.opacities, sc.width, sc.height, sc.tile_width, sc.tile_height,
+                   1 / 256, True, 32)
+    assert np.array_equal(image.view(np.uint32), of.image.view(np.uint32))
 
 
 def test_forward_entry_very_long_tile_lists():

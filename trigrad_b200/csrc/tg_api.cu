@@ -25,7 +25,7 @@ struct ForwardWorkspace {
             off += align_up(bytes ? bytes : 1);
             return p;
         };
-        const bool device_scan = tiles > tg::kTileScanByLastCta;
+        const bool device_scan = tiles > tg::kTileScanByOneCta;
         // what outlives a call (TG_WORKSPACE_READY) lies first, at places that do not depend on the list capacity
         bin.tables = (float4*)take(sizeof(float4) * ((size_t)tiles + 1));     // tiles_x + tiles_y <= tiles + 1
         // everything from `status` up to the end of the tile counts must be zero when the kernels start
@@ -88,7 +88,7 @@ struct TileLists {
 
     TileLists(void* workspace, int T, int W, int H, int tw, int th, uint32_t cap, unsigned flags)
         : ws(workspace, ((W + tw - 1) / tw) * ((H + th - 1) / th), cap), tiles(((W + tw - 1) / tw) * ((H + th - 1) / th)),
-          device_scan(tiles > tg::kTileScanByLastCta), mapped((flags & TG_INFO_MAPPED) != 0 && T > 0),
+          device_scan(tiles > tg::kTileScanByOneCta), mapped((flags & TG_INFO_MAPPED) != 0 && T > 0),
           device_status(device_scan ? ws.bin.status : nullptr) {}       // only the scan waits
 
     int start(const float* vertices, const int32_t* indices, const float* colors, const float* opacities, int T, int W, int H,
@@ -107,20 +107,20 @@ struct TileLists {
         const bool cull = (flags & TG_FORWARD_CULL_TILES) != 0 && !device_scan;
         timer.mark();                                                    // [0] start of "init"
         timer.mark();                                                    // [1] start of "bary_transforms"
-        // per-triangle records, (triangle, tile) pairs with their depth keys, tile offsets
+        // per-triangle records, (triangle, tile) pairs with their depth keys
         if (int st = tg_host::bin_triangles(vertices, indices, colors, opacities, T, W, H, tw, th, tri_geo, tri_attr, ws.bin,
-                                            offsets, cap, mapped ? info_host : nullptr, cull, (flags & TG_INPUT_PACKED) != 0,
+                                            offsets, cap, cull, (flags & TG_INPUT_PACKED) != 0,
                                             (flags & TG_WORKSPACE_READY) != 0, s))
             return st;
         timer.mark();                                                    // [2] start of "per_tile_lists"
+        if (int st = tg_host::place_entries(ws.bin, T, W, H, tw, th, offsets, cap, mapped ? info_host : nullptr, s)) return st;
         if (!mapped) {
             // [3] first: the host watches the word K arrives in
             TG_CUDA(cudaMemcpyAsync(&info_host[3], ws.bin.info + 2, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
             TG_CUDA(cudaMemcpyAsync(&info_host[0], ws.bin.info, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
             TG_CUDA(cudaEventRecord(k_ready, s));
         }
-        // The entries move to their tiles while K travels to the host: the kernel does nothing when K exceeds the capacity.
-        return tg_host::scatter_entries(ws.bin, cap, offsets, tiles, T, s);
+        return TG_OK;
     }
 
     // K arrives in (preferably pinned) host memory.  Watching the word itself is quicker than waking up from
@@ -165,9 +165,14 @@ struct TileLists {
         return TG_OK;
     }
 
-    int sort(int32_t* sorted_ids, const int32_t* offsets, cudaStream_t s) {
+    // Before wait(): the lists are sorted while K travels to the host, where they turn out to be complete.
+    int sort_short(int32_t* sorted_ids, const int32_t* offsets, uint32_t cap, int T, cudaStream_t s) {
+        if (T == 0 || cap == 0) return TG_OK;
+        return tg_host::sort_short_lists(ws.bin.entries, offsets, tiles, sorted_ids, ws.long_list, false, &ws.bin, cap, s);
+    }
+    int sort_long(int32_t* sorted_ids, const int32_t* offsets, cudaStream_t s) {
         if (K == 0) return TG_OK;
-        return tg_host::sort_tile_lists(ws.bin.entries, offsets, tiles, sorted_ids, ws.long_list, true, false, longest, s);
+        return tg_host::sort_long_lists(ws.bin.entries, offsets, tiles, sorted_ids, ws.long_list, false, longest, s);
     }
 };
 
@@ -191,9 +196,9 @@ static int finish_timing(StageTimer& timer, float* stage_ms_host, const uint32_t
     float ms[5];
     for (int i = 0; i < 5; i++) TG_CUDA(cudaEventElapsedTime(&ms[i], timer.ev[i], timer.ev[i + 1]));
     stage_ms_host[0] = ms[0];   // init
-    stage_ms_host[1] = ms[2];   // per_tile_lists: K read-back + entry emission
-    stage_ms_host[2] = ms[3];   // sorting: per-tile sort
-    stage_ms_host[3] = ms[1];   // bary_transforms: preprocess + scan + tile counts and offsets
+    stage_ms_host[1] = ms[2];   // per_tile_lists: tile offsets, entries to their places
+    stage_ms_host[2] = ms[3];   // sorting: per-tile sort, K read-back meanwhile
+    stage_ms_host[3] = ms[1];   // bary_transforms: records, pairs, tile counts
     stage_ms_host[4] = ms[4];   // rasterization
     if (info_host[2]) {
         tg_host::set_error("device error word = %u", info_host[2]);
@@ -224,26 +229,19 @@ int tg_render_forward(const float* vertices, const int32_t* indices, const float
     if (int st = lists.start(vertices, indices, colors, opacities, T, W, H, tw, th, tri_geo, tri_attr, sorted_ids, list_capacity,
                              offsets, workspace_bytes, info_host, flags, timer, s))
         return st;
-    // Lists of up to kFusedList entries are sorted by the compositing kernel itself in images of few tiles.  Where the
-    // caller expects nothing longer it is launched right away, and checks on the device what the host is told afterwards.
-    auto composite_short = [&]() {
-        return tg_host::blend_forward_short(tri_geo, tri_attr, lists.ws.bin.entries, lists.ws.bin.info, list_capacity, sorted_ids,
-                                            offsets, W, H, tw, th, thr, per_pixel_sort, max_layers, image, depthmap,
-                                            final_weights, ends, selection, s);
-    };
-    const bool can = lists.tiles <= tg::kFusedTiles && T > 0;
-    const bool early = can && (flags & TG_EXPECT_SHORT_LISTS) != 0 && stage_ms_host == nullptr;
-    if (early)
-        if (int st = composite_short()) return st;
-    if (int st = lists.wait(list_capacity, info_host, s)) return st;
+    // Lists of up to kFusedList entries are sorted by the compositing kernel itself in images of few tiles, where the caller
+    // expects nothing longer: it checks on the device what the host is told afterwards.
+    const bool early = lists.tiles <= tg::kFusedTiles && T > 0 && (flags & TG_EXPECT_SHORT_LISTS) != 0 && stage_ms_host == nullptr;
     timer.mark();                                                    // [3] start of "sorting"
-    int st = TG_OK;
-    if (can && lists.longest <= tg::kFusedList) {
+    int st = early ? tg_host::blend_forward_short(tri_geo, tri_attr, lists.ws.bin, list_capacity, sorted_ids, offsets, W, H, tw, th,
+                                                  thr, per_pixel_sort, max_layers, image, depthmap, final_weights, ends, selection, s)
+                   : lists.sort_short(sorted_ids, offsets, list_capacity, T, s);
+    if (st) return st;
+    if ((st = lists.wait(list_capacity, info_host, s))) return st;
+    if (!early || lists.longest > tg::kFusedList) {
+        if (early && (st = lists.sort_short(sorted_ids, offsets, list_capacity, T, s))) return st;
+        if ((st = lists.sort_long(sorted_ids, offsets, s))) return st;
         timer.mark();                                                // [4] start of "rasterization"
-        if (!early) st = composite_short();
-    } else {
-        if ((st = lists.sort(sorted_ids, offsets, s))) return st;
-        timer.mark();                                                // [4]
         tg_host::set_tile_order(lists.order, lists.longest);         // with the longest list: long lists are streamed
         st = tg_blend_forward(tri_geo, tri_attr, sorted_ids, offsets, W, H, tw, th, thr, per_pixel_sort, max_layers, image,
                               depthmap, final_weights, ends, selection, stream);
@@ -274,9 +272,10 @@ int tg_render_step_l2(const float* vertices, const int32_t* indices, const float
     int st = lists.start(vertices, indices, colors, opacities, T, W, H, tw, th, tri_geo, tri_attr, sorted_ids, list_capacity,
                          offsets, workspace_bytes, info_host, flags, timer, s);
     if (st) return st;
-    if ((st = lists.wait(list_capacity, info_host, s))) return st;
     timer.mark();                                                    // [3] start of "sorting"
-    if ((st = lists.sort(sorted_ids, offsets, s))) return st;
+    if ((st = lists.sort_short(sorted_ids, offsets, list_capacity, T, s))) return st;
+    if ((st = lists.wait(list_capacity, info_host, s))) return st;
+    if ((st = lists.sort_long(sorted_ids, offsets, s))) return st;
     timer.mark();                                                    // [4] start of "rasterization" (here: forward + backward)
     tg_host::set_tile_order(lists.order);
     st = tg_blend_step_l2(tri_geo, tri_attr, sorted_ids, offsets, V, W, H, tw, th, thr, max_layers, target, grad_scale,

@@ -249,17 +249,15 @@ __global__ void __launch_bounds__(256) bin_init_kernel(uint32_t* __restrict__ cl
     else if (i < (size_t)tiles_x + tiles_y) rows[i - tiles_x] = tile_span((int)(i - tiles_x), th, H);
 }
 
-// Exclusive scan of counts[0..tiles) by one CTA of the binning kernel into offsets[0..tiles]; returns the largest count,
-// the sum in `total`.
-// 16 consecutive counts per thread and round, fetched by four independent 16-byte loads one round ahead: the rounds are
-// bound by the latency of those loads.
+// Exclusive scan of counts[0..tiles) by one CTA into offsets[0..tiles] (global or shared memory); the sum in `total`.  Returns
+// the largest count where `want_biggest` (uniform over the CTA).
+// A warp takes 512 counts per round, four independent 16-byte loads per lane one round ahead: bound by the latency of those.
 constexpr int kBinWarps = 4;         // warps of a CTA of the binning kernel (two and eight: 3 to 7 % slower)
-constexpr int kFinishWarps = 16;      // of the kernel that scans the tile counts after a binning of several waves
-constexpr int kTileScanPer = 16;
+constexpr int kFinishWarps = 16;     // of the kernel that scans the tile counts of images with very many tiles
 __device__ __forceinline__ void load_counts(const uint32_t* counts, int first, int tiles, uint4 (&v)[4]) {
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-        const int i = first + 4 * k;
+        const int i = first + 128 * k;
         if (i + 3 < tiles) {
             v[k] = __ldcg(reinterpret_cast<const uint4*>(counts + i));
         } else {
@@ -271,43 +269,54 @@ __device__ __forceinline__ void load_counts(const uint32_t* counts, int first, i
     }
 }
 template <int WARPS>
-__device__ uint32_t tile_offsets_by_one_cta(const uint32_t* counts, int32_t* offsets, int tiles, uint32_t* s_warp /*[WARPS]*/,
-                                            uint32_t& total) {
-    constexpr int kTileScanRound = 32 * WARPS * kTileScanPer;
-    const int tid = threadIdx.x, warp = tid >> 5;
+__device__ __forceinline__ uint32_t tile_offsets_by_one_cta(const uint32_t* counts, int32_t* offsets, int tiles,
+                                                            uint32_t* s_warp /*[WARPS]*/, bool want_biggest, uint32_t& total) {
+    static_assert(WARPS <= 32, "a lane per warp");
+    constexpr int kRound = 512 * WARPS;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, mine = 512 * warp + 4 * lane;
+    const bool aligned = ((uintptr_t)offsets & 15) == 0;
     uint32_t carry = 0, biggest = 0;
     uint4 ahead[4];
-    load_counts(counts, tid * kTileScanPer, tiles, ahead);
-    for (int base = 0; base < tiles; base += kTileScanRound) {
-        const int first = base + tid * kTileScanPer;
-        uint32_t v[kTileScanPer], mine = 0;
+    load_counts(counts, mine, tiles, ahead);
+    for (int base = 0; base < tiles; base += kRound) {
+        uint4 v[4];
+        uint32_t excl[4], run = 0;              // of this lane's counts in the warp's 128; sum of the warp's 128s before
 #pragma unroll
-        for (int k = 0; k < 4; k++) { v[4 * k] = ahead[k].x; v[4 * k + 1] = ahead[k].y; v[4 * k + 2] = ahead[k].z; v[4 * k + 3] = ahead[k].w; }
-        if (base + kTileScanRound < tiles) load_counts(counts, first + kTileScanRound, tiles, ahead);
+        for (int k = 0; k < 4; k++) v[k] = ahead[k];
+        if (base + kRound < tiles) load_counts(counts, base + kRound + mine, tiles, ahead);
 #pragma unroll
-        for (int k = 0; k < kTileScanPer; k++) { mine += v[k]; biggest = max(biggest, v[k]); }
-        uint32_t incl = mine;
+        for (int k = 0; k < 4; k++) {
+            const uint32_t sum = v[k].x + v[k].y + v[k].z + v[k].w;
+            biggest = max(max(biggest, max(v[k].x, v[k].y)), max(v[k].z, v[k].w));
+            uint32_t incl = sum;
 #pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            uint32_t y = __shfl_up_sync(0xffffffffu, incl, d);
-            if (lane_id() >= (unsigned)d) incl += y;
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, incl, d);
+                if (lane >= d) incl += y;
+            }
+            excl[k] = incl - sum + run;
+            run += __shfl_sync(0xffffffffu, incl, 31);
         }
         __syncthreads();                      // s_warp free again
-        if (lane_id() == 31) s_warp[warp] = incl;
+        if (lane == 0) s_warp[warp] = run;
         __syncthreads();
-        uint32_t run = carry + incl - mine;
+        uint32_t incl = lane < WARPS ? s_warp[lane] : 0u;
 #pragma unroll
-        for (int w = 0; w < WARPS; w++) {
-            const uint32_t x = s_warp[w];
-            if (w < warp) run += x;
-            carry += x;
+        for (int d = 1; d < WARPS; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= d) incl += y;
         }
+        const uint32_t before = carry + __shfl_sync(0xffffffffu, incl, warp) - run;
+        carry += __shfl_sync(0xffffffffu, incl, WARPS - 1);
 #pragma unroll
-        for (int k = 0; k < kTileScanPer; k += 4) {
-            const uint4 o = make_uint4(run, run + v[k], run + v[k] + v[k + 1], run + v[k] + v[k + 1] + v[k + 2]);
-            run = o.w + v[k + 3];
-            const int i = first + k;
-            if (i + 3 < tiles && ((uintptr_t)offsets & 15) == 0) {
+        for (int k = 0; k < 4; k++) {
+            const int i = base + mine + 128 * k;
+            uint4 o;
+            o.x = before + excl[k];
+            o.y = o.x + v[k].x;
+            o.z = o.y + v[k].y;
+            o.w = o.z + v[k].z;
+            if (i + 3 < tiles && aligned) {
                 *reinterpret_cast<uint4*>(offsets + i) = o;
             } else {
                 if (i < tiles) offsets[i] = (int32_t)o.x;
@@ -317,51 +326,74 @@ __device__ uint32_t tile_offsets_by_one_cta(const uint32_t* counts, int32_t* off
             }
         }
     }
-    if (tid == 0) offsets[tiles] = (int32_t)carry;
+    if (threadIdx.x == 0) offsets[tiles] = (int32_t)carry;
     total = carry;
+    __syncthreads();                          // offsets visible to the CTA
+    if (!want_biggest) return 0;
     biggest = __reduce_max_sync(0xffffffffu, biggest);
+    if (lane == 0) s_warp[warp] = biggest;
     __syncthreads();
-    if (lane_id() == 0) s_warp[warp] = biggest;
-    __syncthreads();
-#pragma unroll
-    for (int w = 0; w < WARPS; w++) biggest = max(biggest, s_warp[w]);
-    return biggest;
+    return __reduce_max_sync(0xffffffffu, lane < WARPS ? s_warp[lane] : 0u);
 }
 
-// Launch order for the compositing kernel: tiles grouped by the class floor(log2(length)) + 1 of their list length,
-// longest class first (empty tiles last).  With one CTA per tile in scan order a tile whose list is as long as
-// everything else an SM processes can start late and leave the other SMs idle (a view of a fine mesh: 28 % of the
-// SM time); long lists first removes that tail.  Worth its two passes over the offsets only when lists are long and
-// uneven and the tiles are few enough for one CTA (a 1920x1080 image: 8160 tiles, 5 us); an extra CTA of the scatter kernel
-// makes it while the others move the entries.
+// Launch order for the compositing kernel: tiles grouped by the length class of their lists, longest class first.  With one
+// CTA per tile in scan order a tile whose list is as long as everything else an SM processes can start late and leave the
+// other SMs idle (a view of a fine mesh: 28 % of the SM time); long lists first removes that tail.  Worth its passes over the
+// offsets only when lists are long and uneven and the tiles are few enough for one CTA, which makes it while the others move
+// the entries: every thread counts its tiles per class, eight 16-bit sums in four words, and a scan of the words over the CTA
+// says where each thread's tiles of a class go (1920x1080, 8160 tiles: under 2 us; with an atomic per class and warp 10).
 constexpr uint32_t kOrderMinLongest = 256;
-constexpr int kOrderMaxTiles = 16384;
 constexpr uint32_t kOrderMinMean = 64;
-__device__ void tile_order_by_one_cta(const int32_t* offsets, int tiles, uint32_t* order, uint32_t* s_hist /*[33]*/) {
-    const int tid = threadIdx.x;
-    const unsigned lane = lane_id(), lt_mask = (1u << lane) - 1u;
-    if (tid < 33) s_hist[tid] = 0;
-    __syncthreads();
-    const int padded = (tiles + 255) & ~255;
-    for (int i = tid; i < padded; i += 256) {
-        const int cls = (i < tiles) ? 32 - __clz((uint32_t)(offsets[i + 1] - offsets[i])) : 33;
-        const unsigned peers = __match_any_sync(0xffffffffu, cls);          // one shared-memory atomic per class and warp
-        if (cls <= 32 && (peers & lt_mask) == 0) atomicAdd(&s_hist[cls], (uint32_t)__popc(peers));
+constexpr int kOrderMaxTiles = kPlaceTilesSmall;
+static_assert(kOrderMaxTiles < 65536, "16-bit sums");
+// 7: empty, 6: below 64 entries, 5: below 128, ... 0: 2048 and more
+__device__ __forceinline__ int length_class(int n) { return n <= 0 ? 7 : min(6, max(0, __clz(n) - 20)); }
+template <int NT>
+__device__ __forceinline__ void tile_order_by_one_cta(const int32_t* s_off, int tiles, uint32_t* order, uint4* s_sums /*[NT / 32]*/) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t c[4] = {0, 0, 0, 0};
+    auto field = [](int cls) { return 1u << (16 * (cls & 1)); };
+    for (int i = threadIdx.x; i < tiles; i += NT) {
+        const int cls = length_class(s_off[i + 1] - s_off[i]);
+#pragma unroll
+        for (int k = 0; k < 4; k++) c[k] += (cls >> 1) == k ? field(cls) : 0u;
     }
-    __syncthreads();
-    if (tid == 0) {
-        uint32_t run = 0;
-        for (int c = 32; c >= 0; c--) { const uint32_t n = s_hist[c]; s_hist[c] = run; run += n; }
+    uint32_t incl[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        incl[k] = c[k];
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl[k], d);
+            if (lane >= d) incl[k] += y;
+        }
     }
+    if (lane == 31) s_sums[warp] = make_uint4(incl[0], incl[1], incl[2], incl[3]);
     __syncthreads();
-    for (int i = tid; i < padded; i += 256) {
-        const int cls = (i < tiles) ? 32 - __clz((uint32_t)(offsets[i + 1] - offsets[i])) : 33;
-        const unsigned peers = __match_any_sync(0xffffffffu, cls);
-        const int leader = __ffs(peers) - 1;
-        uint32_t base = 0;
-        if (cls <= 32 && (int)lane == leader) base = atomicAdd(&s_hist[cls], (uint32_t)__popc(peers));
-        base = __shfl_sync(0xffffffffu, base, leader);
-        if (cls <= 32) order[base + __popc(peers & lt_mask)] = (uint32_t)i;
+    uint32_t all[4] = {0, 0, 0, 0};
+    for (int w = 0; w < NT / 32; w++) {
+        const uint4 x = s_sums[w];
+        const uint32_t y[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            if (w < warp) incl[k] += y[k];
+            all[k] += y[k];
+        }
+    }
+    uint32_t at[8], run = 0;            // where this thread's next tile of a class goes
+#pragma unroll
+    for (int cls = 0; cls < 8; cls++) {
+        const int k = cls >> 1, shift = 16 * (cls & 1);
+        at[cls] = run + (((incl[k] - c[k]) >> shift) & 0xffffu);
+        run += (all[k] >> shift) & 0xffffu;
+    }
+    for (int i = threadIdx.x; i < tiles; i += NT) {
+        const int cls = length_class(s_off[i + 1] - s_off[i]);
+        uint32_t to = 0;
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            if (cls == k) to = at[k]++;
+        order[to] = (uint32_t)i;
     }
 }
 
@@ -529,7 +561,7 @@ __global__ void __launch_bounds__(kEmitThreads) emit_keys_kernel(const float4* _
 // (issued before the depth key, which hides its latency) and leave one 16-byte record (key, triangle, tile, rank).  Pairs
 // that need the polygon clipper are put off to the end of the CTA when they are few in a warp, and run there with full
 // warps.
-// The CTA that finishes last turns the counts into tile offsets; the scatter kernel then moves every entry to
+// place_entries_kernel turns the counts into tile offsets and moves every entry to
 // offset + rank.  Against counting and writing in two kernels, which gathered, tested and searched twice, B200, with the
 // scatter: 1.3M triangles of a pixel each, full HD: 281 -> 170 us (this kernel 141); 200k triangles, full HD: 65 -> 36 (31);
 // 2M triangles, 4K: 791 -> 477 (387).  Bound by latency: at 52 % of the issue slots, 38 % of L1 and 8 % of DRAM (200k
@@ -537,15 +569,14 @@ __global__ void __launch_bounds__(kEmitThreads) emit_keys_kernel(const float4* _
 struct BinArgs {
     uint32_t* tile_counts;   // [tiles], zero on entry
     int32_t* offsets;        // [tiles + 1], written when scan_here
-    uint32_t* counters;      // [4], zero on entry: finished CTAs, -, slots handed out (64 bits)
+    uint32_t* counters;      // [4], zero on entry: -, -, slots handed out (64 bits)
     uint32_t* info;          // [3] K, when scan_here the longest list (kOrderWrittenBit: a launch order is wanted), slots;
                              // K and slots no larger than kTooManyPairs
     uint32_t* info_host;     // words 0, 1 and 3 of mapped host memory receive them too, or null
     uint4* pairs;            // [capacity]
     uint32_t capacity;
     int tiles, tiles_x, tiles_y;
-    int scan_here;           // 1: the CTA that finishes the binning scans the tile counts; 0: the host launches a scan
-    int finish_here;         // 1: the last CTA finishes the binning; 0: bin_finish_kernel does
+    int scan_here;           // 0: the host launches a device-wide scan of the tile counts
     int want_order;
     TileTables tables;
 };
@@ -577,31 +608,26 @@ __device__ __forceinline__ void write_pair(const BinArgs& bin, const float* tri,
         bin.pairs[pos] = make_uint4((uint32_t)t, float_to_ordered(depth), tile, rank);
 }
 
-// After all pairs are counted, by one CTA: tile offsets, K, the longest list, and all of it to the host.
-template <int WARPS>
-__device__ __forceinline__ void finish_binning(const BinArgs& bin, uint32_t* s_warp) {
-    const uint32_t slots = (uint32_t)min(__ldcg(slot_counter(bin)), (unsigned long long)kTooManyPairs);
-    uint32_t K = slots, longest = UINT32_MAX;            // longest: not known
-    if (bin.scan_here) {
-        longest = tile_offsets_by_one_cta<WARPS>(bin.tile_counts, bin.offsets, bin.tiles, s_warp, K);
-        // the launch order costs two passes over the offsets: only for images of at most 16384 tiles whose lists are
-        // long on average and uneven (the longest one at least 256 entries)
-        if (bin.want_order && bin.tiles <= kOrderMaxTiles && K >= kOrderMinMean * (uint32_t)bin.tiles && longest >= kOrderMinLongest)
-            longest |= kOrderWrittenBit;
-        if (slots == kTooManyPairs) K = kTooManyPairs;   // the counts' sum is not the number of pairs then
+// K, the longest list and the number of slots, for the kernels behind and for the host.  By one thread.
+__device__ __forceinline__ void publish_counts(const BinArgs& bin, uint32_t K, uint32_t longest, uint32_t slots) {
+    bin.info[0] = K;
+    bin.info[1] = longest;
+    bin.info[2] = slots;
+    if (bin.info_host) {                  // K last: the host watches that word
+        volatile uint32_t* h = bin.info_host;
+        h[1] = longest;
+        h[3] = slots;
+        __threadfence_system();
+        h[0] = K;
     }
-    if (threadIdx.x == 0) {
-        bin.info[0] = K;
-        bin.info[1] = longest;
-        bin.info[2] = slots;
-        if (bin.info_host) {                  // K last: the host watches that word
-            volatile uint32_t* h = bin.info_host;
-            h[1] = longest;
-            h[3] = slots;
-            __threadfence_system();
-            h[0] = K;
-        }
-    }
+}
+__device__ __forceinline__ uint32_t slots_used(const BinArgs& bin) {
+    return (uint32_t)min(__ldcg(slot_counter(bin)), (unsigned long long)kTooManyPairs);
+}
+// Whether a launch order of the tiles is worth its two passes over the offsets: only for images of at most 16384 tiles
+// whose lists are long on average and uneven (the longest one at least 256 entries).
+__device__ __forceinline__ bool order_wanted(const BinArgs& bin, uint32_t K, uint32_t longest) {
+    return bin.want_order && bin.tiles <= kOrderMaxTiles && K >= kOrderMinMean * (uint32_t)bin.tiles && longest >= kOrderMinLongest;
 }
 
 template <bool CULL>
@@ -619,7 +645,6 @@ __global__ void __launch_bounds__(32 * kBinWarps, 32 / kBinWarps) bin_kernel(con
     __shared__ uint32_t s_first[kBinWarps + 1];       // first pair of every warp's triangles
     __shared__ uint32_t s_queued, s_base;
     __shared__ uint32_t s_warp[kBinWarps];
-    __shared__ bool s_last;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const unsigned below = (1u << lane) - 1u;
     allow_dependents();
@@ -760,34 +785,81 @@ __global__ void __launch_bounds__(32 * kBinWarps, 32 / kBinWarps) bin_kernel(con
         write_pair(bin, s_tri[ct >> 5] + (ct & 31), t_cta + (ct >> 5) * per_warp + (ct & 31), tx, ty, slot0 + s_qe[q],
                    __ldg(bin.tables.cols + tx), __ldg(bin.tables.rows + ty), s_poly + tid);
     }
-    if (!bin.finish_here) return;
-    __syncthreads();                          // the CTA's counts are issued; one cumulative fence publishes them
-    if (tid == 0) {
-        __threadfence();
-        s_last = (atomicAdd(bin.counters, 1u) == gridDim.x - 1u);
-    }
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    finish_binning<kBinWarps>(bin, s_warp);
 }
 
-// The same as a kernel of its own, after a binning of several waves.
+// Images of more tiles than place_entries_kernel has shared memory for: one CTA turns the counts into tile offsets (unless a
+// device-wide scan follows), and scatter_entries_kernel moves the entries.
 __global__ void __launch_bounds__(32 * kFinishWarps) bin_finish_kernel(BinArgs bin) {
     __shared__ uint32_t s_warp[kFinishWarps];
     allow_dependents();
     await_prerequisites();
-    finish_binning<kFinishWarps>(bin, s_warp);
+    const uint32_t slots = slots_used(bin);
+    uint32_t K = slots, longest = UINT32_MAX;            // longest: not known
+    if (bin.scan_here) {
+        longest = tile_offsets_by_one_cta<kFinishWarps>(bin.tile_counts, bin.offsets, bin.tiles, s_warp, true, K);
+        if (slots == kTooManyPairs) K = kTooManyPairs;   // the counts' sum is not the number of pairs then
+    }
+    if (threadIdx.x == 0) publish_counts(bin, K, longest, slots);
 }
 
-// Every entry to its place: offset of its tile plus its rank there.  The last CTA makes the launch order of the
-// compositing kernel instead when one is wanted.
+// Counts to tile offsets, and every entry to its place: offset of its tile plus its rank there.  Every CTA makes the offsets
+// for itself, in shared memory, while its first pairs are on their way; the first one leaves them for the kernels behind, with K, the
+// longest list and the launch order of the tiles, instead of moving entries.
+// Against the scan by one CTA (the binning kernel's last, or a kernel of its own) and a scatter that looked the offsets up in
+// memory, B200: 200k triangles, 1920x1080 13.4 -> 6.7 us; 1.3M triangles, the same image, with the launch order 39 -> 16;
+// 2M triangles, 3840x2160 102 -> 92; 1280 triangles, 256x256, with the binning 15.6 -> 12.2.  Latency: half of the 6.7 us are
+// the scan's loads and barriers; the large one is bound by the scattered stores of 8 bytes.
+template <int NT>
+__global__ void __launch_bounds__(NT) place_entries_kernel(BinArgs bin, uint64_t* __restrict__ entries, uint32_t* __restrict__ order,
+                                                           uint32_t* __restrict__ list_heads) {
+    extern __shared__ __align__(16) int32_t s_off[];            // [tiles + 1]
+    __shared__ uint32_t s_warp[NT / 32];
+    __shared__ uint4 s_sums[NT / 32];
+    constexpr uint32_t kPer = 4;                                // pairs of a thread in flight
+    const uint32_t tid = threadIdx.x, stride = (gridDim.x - 1) * kPer * NT;
+    allow_dependents();
+    await_prerequisites();
+    const bool tables = blockIdx.x == 0;
+    uint32_t first = (blockIdx.x - 1) * kPer * NT + tid;
+    uint4 p[kPer];
+#pragma unroll
+    for (uint32_t k = 0; k < kPer; k++)
+        if (!tables && first + NT * k < bin.capacity) p[k] = __ldcs(bin.pairs + first + NT * k);
+    const uint32_t n = slots_used(bin);                         // holes included
+    uint32_t K = 0;
+    const uint32_t longest = tile_offsets_by_one_cta<NT / 32>(bin.tile_counts, s_off, bin.tiles, s_warp, tables, K);
+    if (tables) {
+        if (n == kTooManyPairs) K = kTooManyPairs;              // the counts' sum is not the number of pairs then
+        const bool ordered = order_wanted(bin, K, longest);
+        if (tid == 0) publish_counts(bin, K, ordered ? longest | kOrderWrittenBit : longest, n);
+        if (tid < 6) list_heads[tid] = 0;
+        for (int i = tid; i <= bin.tiles; i += NT) bin.offsets[i] = s_off[i];
+        if (ordered) tile_order_by_one_cta<NT>(s_off, bin.tiles, order, s_sums);
+        return;
+    }
+    if (n > bin.capacity) return;
+    for (; first < n; first += stride) {
+        uint32_t to[kPer];
+#pragma unroll
+        for (uint32_t k = 0; k < kPer; k++) {
+            if (first + NT * k >= n) p[k].z = kHole;
+            to[k] = p[k].z != kHole ? (uint32_t)s_off[p[k].z] + p[k].w : 0u;
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < kPer; k++) {
+            if (p[k].z != kHole) entries[to[k]] = ((uint64_t)p[k].y << 32) | p[k].x;
+            const uint32_t next = first + stride + NT * k;
+            if (next < n) p[k] = __ldcs(bin.pairs + next);
+        }
+    }
+}
+
+// Every entry to its place.
 __global__ void __launch_bounds__(256) scatter_entries_kernel(const uint4* __restrict__ pairs, const uint32_t* __restrict__ info,
                                                               uint32_t capacity, const int32_t* __restrict__ offsets,
-                                                              uint64_t* __restrict__ entries, uint32_t* __restrict__ order,
+                                                              uint64_t* __restrict__ entries,
                                                               int tiles, uint32_t* __restrict__ tile_counts,
                                                               uint32_t* __restrict__ counters, uint32_t* __restrict__ list_heads) {
-    __shared__ uint32_t s_hist[33];
     allow_dependents();
     await_prerequisites();
     // the binning kernel is done with its counters: zero for the next call
@@ -797,12 +869,8 @@ __global__ void __launch_bounds__(256) scatter_entries_kernel(const uint4* __res
     if (me < 6) list_heads[me] = 0;
     const uint32_t n = info[2];               // slots, holes included
     if (n > capacity) return;
-    if (blockIdx.x == gridDim.x - 1) {
-        if (order && info[1] != UINT32_MAX && (info[1] & kOrderWrittenBit)) tile_order_by_one_cta(offsets, tiles, order, s_hist);
-        return;
-    }
     // four entries per thread in flight: each is a chain of two loads and a scattered store
-    const uint32_t stride = (gridDim.x - 1) * 1024;
+    const uint32_t stride = gridDim.x * 1024;
     for (uint32_t i = blockIdx.x * 1024 + threadIdx.x; i < n; i += stride) {
         uint4 p[4];
         uint32_t off[4];
@@ -892,11 +960,18 @@ int prefer_smem(const void* kernel, int kilobytes, SmemAllowed& preferred) {
     return TG_OK;
 }
 
-// Per-triangle records, (triangle, tile) pairs and tile offsets: bin_init_kernel, bin_kernel and scatter_entries_kernel
-// (declared in tg_radix.cuh with what each argument is).
+static tg::BinArgs bin_args(const BinBuffers& b, int W, int H, int tw, int th, int32_t* offsets, uint32_t list_capacity,
+                            uint32_t* info_host) {
+    const int tiles_x = (W + tw - 1) / tw, tiles_y = (H + th - 1) / th, tiles = tiles_x * tiles_y;
+    return {b.tile_counts, offsets, b.counters, b.info, info_host, b.pairs, list_capacity, tiles, tiles_x, tiles_y,
+            tiles <= tg::kTileScanByOneCta ? 1 : 0, b.tile_order ? 1 : 0, {b.tables, b.tables + tiles_x}};
+}
+
+// Per-triangle records and (triangle, tile) pairs: bin_init_kernel and bin_kernel (declared in tg_radix.cuh with what each
+// argument is).
 int bin_triangles(const float* vertices, const int32_t* indices, const float* colors, const float* opacities, int T, int W,
                   int H, int tw, int th, float* tri_geo, float* tri_attr, const BinBuffers& b, int32_t* offsets,
-                  uint32_t list_capacity, uint32_t* info_host, bool cull, bool packed, bool ready, cudaStream_t stream) {
+                  uint32_t list_capacity, bool cull, bool packed, bool ready, cudaStream_t stream) {
     TG_REQUIRE(T >= 0, "T < 0");
     if (int s = check_sizes(W, H, tw, th)) return s;
     TG_REQUIRE(offsets, "null pointer");
@@ -907,10 +982,10 @@ int bin_triangles(const float* vertices, const int32_t* indices, const float* co
                "vertices / tri_geo / tri_attr must be 16-byte aligned");
     TG_REQUIRE(!packed || ((((uintptr_t)indices | (uintptr_t)colors) & 15) == 0),
                "packed faces [T,4] and colours [V,4] must be 16-byte aligned");
-    const bool by_last_cta = tiles <= tg::kTileScanByLastCta;
-    TG_REQUIRE(!cull || by_last_cta, "tile culling is limited to 65536 tiles");
+    const bool by_one_cta = tiles <= tg::kTileScanByOneCta;
+    TG_REQUIRE(!cull || by_one_cta, "tile culling is limited to 65536 tiles");
     float4* rows = b.tables + tiles_x;
-    if (!ready || !by_last_cta) {
+    if (!ready || !by_one_cta) {
         const size_t init = b.clear_words > (size_t)tiles_x + tiles_y ? b.clear_words : (size_t)tiles_x + tiles_y;
         tg::bin_init_kernel<<<(unsigned)((init + 255) / 256), 256, 0, stream>>>(b.clear, b.clear_words, b.tables, rows, tiles_x,
                                                                               tiles_y, W, H, tw, th);
@@ -926,42 +1001,55 @@ int bin_triangles(const float* vertices, const int32_t* indices, const float* co
     constexpr int kWave = 148 * 32 / tg::kBinWarps;
     const int per_cta = T >= 32 * tg::kBinWarps * kWave ? 32 * tg::kBinWarps : (T + kWave - 1) / kWave;
     const int grid = (T + per_cta - 1) / per_cta;
-    // A grid of one wave is finished by its last CTA, which saves a launch (where there are few triangles both take the same).
-    // Beyond, the barrier, fence and atomic at the end of every CTA hold its slot for longer than a dependent launch
-    // takes, and sixteen warps scan the counts faster than four (1.3M triangles: 158 us against 141 and the scan, a step
-    // 620 against 613; 200k triangles, full HD, a view: 164.3 against 162.7).
-    constexpr int kFinishHere = kWave;
-    const tg::BinArgs bin = {b.tile_counts, offsets, b.counters, b.info, info_host, b.pairs, list_capacity, tiles, tiles_x,
-                             tiles_y, by_last_cta ? 1 : 0, grid <= kFinishHere ? 1 : 0, b.tile_order ? 1 : 0, {b.tables, rows}};
+    const tg::BinArgs bin = bin_args(b, W, H, tw, th, offsets, list_capacity, nullptr);
     auto inverse = [](int n) { return (n & (n - 1)) == 0 ? 1.0 / n : 0.0; };
     auto kernel = cull ? tg::bin_kernel<true> : tg::bin_kernel<false>;
-    static SmemAllowed allowed[2];
-    if (int st = allow_smem((const void*)kernel, tg::kBinSmem, allowed[cull ? 1 : 0])) return st;
+    static SmemAllowed bin_allowed[2];
+    if (int st = allow_smem((const void*)kernel, tg::kBinSmem, bin_allowed[cull ? 1 : 0])) return st;
     TG_CUDA(launch_dependent(kernel, grid, 32 * tg::kBinWarps, tg::kBinSmem, stream, (const float4*)vertices, indices, colors,
                              opacities, T, per_cta, W, H, tw, th, inverse(tw), inverse(th), (float4*)tri_geo, (float4*)tri_attr,
                              bin, packed ? 1 : 0));
     TG_LAUNCH_CHECK("bin_kernel");
-    if (!bin.finish_here) {
-        TG_CUDA(launch_dependent(tg::bin_finish_kernel, 1, 32 * tg::kFinishWarps, 0, stream, bin));
-        TG_LAUNCH_CHECK("bin_finish_kernel");
+    return TG_OK;
+}
+
+int place_entries(const BinBuffers& b, int T, int W, int H, int tw, int th, int32_t* offsets, uint32_t list_capacity,
+                  uint32_t* info_host, cudaStream_t stream) {
+    if (T == 0) return TG_OK;
+    const tg::BinArgs bin = bin_args(b, W, H, tw, th, offsets, list_capacity, info_host);
+    const int tiles = bin.tiles;
+    if (tiles <= tg::kPlaceTiles) {
+        // One CTA per SM, and no more than the list capacity, which is what the host knows of the number of pairs, fills; the
+        // first moves none.  More of them read the counts more often than the loop gains (two per SM: 8.0 us against 6.7,
+        // 200k triangles, 1920x1080).  The offsets of very many tiles leave an SM room for one CTA, which then has 1024
+        // threads (2M triangles, 3840x2160, 32400 tiles: 92 us; 8160 tiles with 1024 threads: 7.2 against 6.7).
+        const bool big = tiles > tg::kPlaceTilesSmall;
+        const int threads = big ? 1024 : 512;
+        const uint32_t want = (list_capacity + 4 * threads - 1) / (4 * threads);
+        const int ctas = (int)(want < 147 ? want + 1 : 148);
+        const size_t smem = sizeof(int32_t) * ((size_t)tiles + 1);
+        static SmemAllowed place_allowed[2];
+        auto place = big ? tg::place_entries_kernel<1024> : tg::place_entries_kernel<512>;
+        if (int st = allow_smem((const void*)place, sizeof(int32_t) * ((big ? tg::kPlaceTiles : tg::kPlaceTilesSmall) + 1), place_allowed[big]))
+            return st;
+        TG_CUDA(launch_dependent(place, ctas, threads, smem, stream, bin, b.entries, b.tile_order, b.list_heads));
+        TG_LAUNCH_CHECK("place_entries_kernel");
+        return TG_OK;
     }
-    if (!by_last_cta) {
+    TG_CUDA(launch_dependent(tg::bin_finish_kernel, 1, 32 * tg::kFinishWarps, 0, stream, bin));
+    TG_LAUNCH_CHECK("bin_finish_kernel");
+    if (!bin.scan_here) {
         const int parts = (tiles + tg::kScanTile - 1) / tg::kScanTile;
         tg::scan_kernel<<<parts, tg::kScanThreads, 0, stream>>>(b.tile_counts, (uint32_t*)offsets, tiles, parts,
                                                                  (uint32_t*)b.tile_scan_scratch,
                                                                  (uint64_t*)((char*)b.tile_scan_scratch + 8), b.status);
         TG_LAUNCH_CHECK("scan_kernel");
     }
-    return TG_OK;
-}
-
-int scatter_entries(const BinBuffers& b, uint32_t list_capacity, const int32_t* offsets, int tiles, int T, cudaStream_t stream) {
-    if (T == 0) return TG_OK;
-    // K is not known on the host yet: as many CTAs as its upper bound fills, at most eight per SM, and one for the order
+    // K is not known on the host yet: as many CTAs as its upper bound fills, at most eight per SM
     const uint32_t want = (list_capacity + 1023) / 1024;
-    const int grid = (int)(want < 148 * 8 ? want : 148 * 8) + 1;
-    TG_CUDA(launch_dependent(tg::scatter_entries_kernel, grid, 256, 0, stream, b.pairs, b.info, list_capacity, offsets, b.entries,
-                             b.tile_order, tiles, b.tile_counts, b.counters, b.list_heads));
+    const int ctas = want < 1 ? 1 : (int)(want < 148 * 8 ? want : 148 * 8);
+    TG_CUDA(launch_dependent(tg::scatter_entries_kernel, ctas, 256, 0, stream, b.pairs, b.info, list_capacity, offsets, b.entries,
+                             tiles, b.tile_counts, b.counters, b.list_heads));
     TG_LAUNCH_CHECK("scatter_entries_kernel");
     return TG_OK;
 }

@@ -637,8 +637,7 @@ __device__ __forceinline__ void store_pixel(const TileCtx& c, const BlendParams&
 static_assert(kFusedList <= 2 * kChunk, "staged as a whole");
 struct UnsortedLists {
     const uint64_t* entries;      // ordered depth << 32 | triangle, grouped by tile
-    const uint32_t* info;         // K, longest list, slots
-    uint32_t capacity;
+    AfterBinning bin;
     int* sorted_ids;
 };
 template <bool SORT, int MAXT, bool STREAM = false, bool FUSED = false>
@@ -661,8 +660,9 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (SORT ? 4 : 5) : 1) blend_
     await_prerequisites();
     if (FUSED) {
         // launched before the host knows: nothing to do when the lists are too long or incomplete
-        const uint32_t slots = unsorted.info[2], longest = unsorted.info[1] & ~kOrderWrittenBit;
-        if (slots > unsorted.capacity || longest > kFusedList) return;
+        unsorted.bin.clear((int)blockIdx.x, threadIdx.x == 0);
+        const uint32_t longest = unsorted.bin.info[1] & ~kOrderWrittenBit;
+        if (unsorted.bin.incomplete() || longest > kFusedList) return;
     }
     const int this_tile = tile_of_block(P);
     const int list_first = P.offsets[this_tile], list_n = P.offsets[this_tile + 1] - list_first;
@@ -1726,15 +1726,14 @@ void set_tile_order(const uint32_t* order, uint32_t longest_list) {
     g_longest_list = longest_list;
 }
 
-int blend_forward_short(const float* tri_geo, const float* tri_attr, const uint64_t* entries, const uint32_t* info,
-                        uint32_t capacity, int32_t* sorted_ids, const int32_t* offsets, int W, int H, int tw, int th, float thr,
+int blend_forward_short(const float* tri_geo, const float* tri_attr, const BinBuffers& b, uint32_t capacity, int32_t* sorted_ids, const int32_t* offsets, int W, int H, int tw, int th, float thr,
                         int per_pixel_sort, int max_layers, float* image, float* depthmap, float* final_weights,
                         int32_t* ends, int32_t* selection, cudaStream_t s) {
     TG_REQUIRE(((uintptr_t)image & 15) == 0, "image must be 16-byte aligned");
     if (tg_selection_planes(per_pixel_sort, max_layers) == 0) selection = nullptr;
     const tg::BlendParams P = make_params(tri_geo, tri_attr, nullptr, offsets, W, H, tw, th, thr, max_layers);
-    const tg::UnsortedLists lists = {entries, info, capacity, sorted_ids};
     const int tiles = P.tiles_x * ((H + th - 1) / th);
+    const tg::UnsortedLists lists = {b.entries, after_binning(&b, tiles, capacity), sorted_ids};
     const int threads = ((tw * th + 31) / 32) * 32;
     auto kernel = threads <= 256 ? (per_pixel_sort ? tg::blend_forward_kernel<true, 256, false, true>
                                                    : tg::blend_forward_kernel<false, 256, false, true>)

@@ -16,8 +16,10 @@ constexpr int kSortWarps = kSortThreads / 32;
 constexpr size_t kHistBytes = (size_t)kMaxPasses * kRadix * sizeof(uint32_t);
 constexpr size_t kCtrBytes = 64;
 constexpr int kHistDoneWord = 8;
-// Up to this many tiles one CTA scans the tile counts: the binning kernel's last one, or bin_finish_kernel's.
-constexpr int kTileScanByLastCta = 65536;
+// Up to this many tiles one CTA scans the tile counts.
+constexpr int kTileScanByOneCta = 65536;
+// Up to this many every CTA that places entries does so for itself, in 220 KB of shared memory (64 KB up to the lower number).
+constexpr int kPlaceTiles = 55 * 1024, kPlaceTilesSmall = 16384;
 // Top bit of the longest-list word the binning kernel reports: a launch order of the tiles was written.
 constexpr uint32_t kOrderWrittenBit = 0x80000000u;
 // What it reports as K and as slots from this many (triangle, tile) pairs on: more than any list capacity.
@@ -89,39 +91,65 @@ __device__ __forceinline__ void hist_flush_and_finish(uint32_t* s_hist, uint32_t
     }
 }
 
+// What a kernel behind the binning is told: whether the lists are complete, and counts and counters to zero for the next call.
+struct AfterBinning {
+    const uint32_t* info;         // K, longest list, slots; null: the lists are known to be complete
+    uint32_t capacity;
+    uint32_t* tile_counts;        // null: nothing to clear
+    uint32_t* counters;           // [4]
+    __device__ __forceinline__ bool incomplete() const { return info != nullptr && info[2] > capacity; }
+    __device__ __forceinline__ void clear(int tile, bool one_thread) const {
+        if (tile_counts == nullptr || !one_thread) return;
+        tile_counts[tile] = 0;
+        if (tile == 0) *reinterpret_cast<uint4*>(counters) = make_uint4(0, 0, 0, 0);
+    }
+};
+
 }  // namespace tg
 
 namespace tg_host {
 // Internal (not part of the C ABI): the pieces tg_render_forward strings together.
-// Forward compositing with the sort of the tile lists (at most kFusedList entries each, `info` as the binning kernel left
-// it) in the same kernel, which does nothing when a list is longer or the slots exceed `capacity`.
-int blend_forward_short(const float* tri_geo, const float* tri_attr, const uint64_t* entries, const uint32_t* info,
-                        uint32_t capacity, int32_t* sorted_ids, const int32_t* offsets, int W, int H, int tw, int th, float thr,
-                        int per_pixel_sort, int max_layers, float* image, float* depthmap, float* final_weights,
-                        int32_t* ends, int32_t* selection, cudaStream_t stream);
 void set_tile_order(const uint32_t* order, uint32_t longest_list = 0);
 size_t tile_sort_scratch_bytes(int tiles);
-// Workspace of the binning kernels (bin_triangles, scatter_entries).
+// Workspace of the binning kernels (bin_triangles, place_entries).
 struct BinBuffers {
     uint32_t* clear;             // zeroed by the first kernel: `clear_words` words that hold the next four
     size_t clear_words;
     uint32_t* status;            // device error word
     uint32_t* counters;          // [4], 8-byte aligned
     uint32_t* tile_counts;       // [tiles], 16-byte aligned
-    void* tile_scan_scratch;     // device-wide scan of the tile counts, only beyond kTileScanByLastCta tiles; zeroed too
+    void* tile_scan_scratch;     // device-wide scan of the tile counts, only beyond kTileScanByOneCta tiles; zeroed too
     float4* tables;              // [tiles_x + tiles_y]
     uint32_t* info;              // [3] K, longest list (UINT32_MAX: not known), slots of `pairs` in use
     uint4* pairs;                // [list capacity]
     uint64_t* entries;           // [list capacity]
     uint32_t* tile_order;        // [tiles] or null
-    uint32_t* list_heads;        // [6] heads of the tile sort's work lists, zeroed by scatter_entries
+    uint32_t* list_heads;        // [6] heads of the tile sort's work lists, zeroed by place_entries
 };
-// `ready`: the counters are zero and the tables valid from a call before (scatter_entries leaves them so).
-// `info_host`: mapped host memory whose words 0, 1 and 3 receive the three info words (K last), or null.
+// Records and pairs.  `ready`: the counters are zero and the tables valid from a call before.
 int bin_triangles(const float* vertices, const int32_t* indices, const float* colors, const float* opacities, int T, int W,
                   int H, int tw, int th, float* tri_geo, float* tri_attr, const BinBuffers& b, int32_t* offsets,
-                  uint32_t list_capacity, uint32_t* info_host, bool cull, bool packed, bool ready, cudaStream_t stream);
-int scatter_entries(const BinBuffers& b, uint32_t list_capacity, const int32_t* offsets, int tiles, int T, cudaStream_t stream);
-int sort_tile_lists(uint64_t* entries, const int32_t* offsets, int tiles, int32_t* sorted_ids, uint32_t* lists,
-                    bool scratch_prepared, bool write_back, uint32_t longest, cudaStream_t stream);
+                  uint32_t list_capacity, bool cull, bool packed, bool ready, cudaStream_t stream);
+// Entries grouped by tile, offsets, info, launch order.  `info_host`: mapped host memory whose words 0, 1 and 3 receive the
+// three info words (K last), or null.  Counts and counters of images of at most kPlaceTiles tiles are left to the kernel
+// behind to clear (the sort's first one, or the compositing kernel that sorts short lists itself).
+int place_entries(const BinBuffers& b, int T, int W, int H, int tw, int th, int32_t* offsets, uint32_t list_capacity,
+                  uint32_t* info_host, cudaStream_t stream);
+// The sort in two steps.  The first launch sorts lists of up to kTileSortRank entries and makes work lists of the others; it
+// needs nothing from the host: given `b`, it does nothing where the slots exceed `capacity`, and clears the counts and
+// counters (see above).  The second, when the longest list is known, launches what the other length classes need.
+int sort_short_lists(uint64_t* entries, const int32_t* offsets, int tiles, int32_t* sorted_ids, uint32_t* lists, bool write_back,
+                     const BinBuffers* b, uint32_t capacity, cudaStream_t stream);
+inline tg::AfterBinning after_binning(const BinBuffers* b, int tiles, uint32_t capacity) {
+    if (b == nullptr) return {};
+    const bool clear = tiles <= tg::kPlaceTiles;
+    return {b->info, capacity, clear ? b->tile_counts : nullptr, b->counters};
+}
+int sort_long_lists(uint64_t* entries, const int32_t* offsets, int tiles, int32_t* sorted_ids, uint32_t* lists, bool write_back,
+                    uint32_t longest, cudaStream_t stream);
+// Forward compositing with the sort of the tile lists (at most kFusedList entries each, `info` as the binning kernel left
+// it) in the same kernel, which does nothing when a list is longer or the slots exceed `capacity`.
+int blend_forward_short(const float* tri_geo, const float* tri_attr, const BinBuffers& b, uint32_t capacity, int32_t* sorted_ids, const int32_t* offsets, int W, int H, int tw, int th, float thr,
+                        int per_pixel_sort, int max_layers, float* image, float* depthmap, float* final_weights,
+                        int32_t* ends, int32_t* selection, cudaStream_t stream);
 }  // namespace tg_host

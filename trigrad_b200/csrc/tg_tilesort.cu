@@ -368,13 +368,15 @@ __device__ __forceinline__ void rank_sort_warp(uint64_t* s, uint64_t* __restrict
 __global__ void __launch_bounds__(kTileSortThreads) tile_sort_kernel(uint64_t* __restrict__ entries,
                                                                      const int32_t* __restrict__ offsets, int tiles,
                                                                      int32_t* __restrict__ sorted_ids,
-                                                                     uint32_t* __restrict__ lists, int write_back) {
+                                                                     uint32_t* __restrict__ lists, int write_back, AfterBinning bin) {
     __shared__ uint64_t s_all[kTileSortWarps][kTileSortRank];
     allow_dependents();
     await_prerequisites();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int tile = blockIdx.x * kTileSortWarps + warp;
     if (tile >= tiles) return;
+    bin.clear(tile, lane == 0);
+    if (bin.incomplete()) return;
     const int edge = (lane < 2) ? offsets[tile + lane] : 0;
     const int beg = __shfl_sync(0xffffffffu, edge, 0);
     const int n = __shfl_sync(0xffffffffu, edge, 1) - beg;
@@ -516,18 +518,19 @@ namespace tg_host {
 
 size_t tile_sort_scratch_bytes(int tiles) { return sizeof(uint32_t) * (2 * (size_t)(tiles > 0 ? tiles : 0) + tg::kListHead); }
 
-// `scratch_prepared`: the caller has zeroed the first six words of `lists`.  `longest`: an upper bound
-// of the longest tile list when the caller knows one (the kernels of the length classes above it are
-// not launched), UINT32_MAX otherwise.
-int sort_tile_lists(uint64_t* entries, const int32_t* offsets, int tiles, int32_t* sorted_ids, uint32_t* lists,
-                    bool scratch_prepared, bool write_back, uint32_t longest, cudaStream_t s) {
+int sort_short_lists(uint64_t* entries, const int32_t* offsets, int tiles, int32_t* sorted_ids, uint32_t* lists, bool write_back,
+                     const BinBuffers* b, uint32_t capacity, cudaStream_t s) {
     TG_REQUIRE(tiles >= 0, "tiles < 0");
     if (tiles == 0) return TG_OK;
     TG_REQUIRE(entries && offsets && sorted_ids && lists, "null pointer");
-    if (!scratch_prepared) TG_CUDA(cudaMemsetAsync(lists, 0, tg::kListHead * sizeof(uint32_t), s));
     TG_CUDA(launch_dependent(tg::tile_sort_kernel, (tiles + tg::kTileSortWarps - 1) / tg::kTileSortWarps, tg::kTileSortThreads, 0, s,
-                             entries, offsets, tiles, sorted_ids, lists, write_back ? 1 : 0));
+                             entries, offsets, tiles, sorted_ids, lists, write_back ? 1 : 0, after_binning(b, tiles, capacity)));
     TG_LAUNCH_CHECK("tile_sort_kernel");
+    return TG_OK;
+}
+
+int sort_long_lists(uint64_t* entries, const int32_t* offsets, int tiles, int32_t* sorted_ids, uint32_t* lists, bool write_back,
+                    uint32_t longest, cudaStream_t s) {
     if (longest > (uint32_t)tg::kTileSortRank) {
         const int grid = tiles < 148 * 12 ? tiles : 148 * 12;
         TG_CUDA(launch_dependent(tg::tile_sort_mid_kernel, grid, tg::kTileSortThreads, 0, s, entries, offsets, tiles, sorted_ids,
@@ -564,8 +567,11 @@ int tg_sort_tile_lists(uint64_t* entries, const int32_t* offsets, int tiles, int
         return TG_ERR_WORKSPACE;
     }
     TG_REQUIRE(((uintptr_t)scratch & 3) == 0 && ((uintptr_t)entries & 7) == 0, "alignment");
-    return tg_host::sort_tile_lists(entries, offsets, tiles, sorted_ids, (uint32_t*)scratch, false, true, UINT32_MAX,
-                                    (cudaStream_t)stream);
+    cudaStream_t s = (cudaStream_t)stream;
+    if (tiles > 0) TG_CUDA(cudaMemsetAsync(scratch, 0, tg::kListHead * sizeof(uint32_t), s));
+    if (int st = tg_host::sort_short_lists(entries, offsets, tiles, sorted_ids, (uint32_t*)scratch, true, nullptr, 0, s)) return st;
+    if (tiles == 0) return TG_OK;
+    return tg_host::sort_long_lists(entries, offsets, tiles, sorted_ids, (uint32_t*)scratch, true, UINT32_MAX, s);
 }
 
 }  // extern "C"
