@@ -280,6 +280,32 @@ def test_forward_and_backward_vs_oracle(pipeline, mode):
         assert err_max <= GRAD_TOL_MAX, f"grad_{name} ({path}): worst element {err_max:.3e}"
 
 
+@pytest.mark.parametrize("height", [1336, 1345, 1353, 1361])     # 167 strips of blocks: one pass; 169, 170, 171: three
+@pytest.mark.parametrize("depth_too", [False, True])
+def test_backward_in_several_passes_vs_oracle(height, depth_too):
+    """Large images, whose CTAs take several blocks of pixels one after the other: strips that do not divide by the number of
+    passes, ragged columns, and warps that take either path (a third of the image lies under three opaque-ish layers)."""
+    import trigrad_b200
+
+    W = 1021 if height == 1336 else 2045
+    sc = S.random_triangles(20_000, W, height, 0.02, 0.6, name="passes", seed=height)
+    sc.vertices[:9, 0] = np.tile([-3, 3, 3], 3)
+    sc.vertices[:9, 1] = np.tile([0.2, 0.2, 5], 3) + np.repeat([0, 0.1, 0.3], 3)
+    rng = np.random.default_rng(height)
+    gi = rng.normal(size=(height, W, 4)).astype(np.float32)
+    gd = rng.normal(size=(height, W)).astype(np.float32) * depth_too
+    v, i, c, o = Hh.scene_tensors(sc)
+    leaves = [t.requires_grad_() for t in (v, c, o)]
+    image, depth = trigrad_b200.render(leaves[0], i, leaves[1], leaves[2], W, height)
+    of = O.forward(sc.vertices, sc.indices, sc.colors, sc.opacities, W, height)
+    assert np.array_equal(image.detach().cpu().numpy().view(np.uint32), of.image.view(np.uint32))
+    got = torch.autograd.grad((image, depth) if depth_too else (image,), leaves,
+                              (Hh.cuda(gi), Hh.cuda(gd)) if depth_too else (Hh.cuda(gi),))
+    want = O.backward(sc.vertices, sc.indices, sc.colors, sc.opacities, W, height, of, gi, gd)
+    for name, a, b in zip(("vertices", "colors", "opacities"), got, want):
+        assert Hh.rel_l2(a.cpu().numpy(), b) <= GRAD_TOL, name
+
+
 @pytest.mark.parametrize("max_layers", [32, 5])
 def test_one_kernel_step_vs_oracle(pipeline, max_layers):
     """tg_blend_step_l2 (forward + backward of the mean squared error in one kernel): image identical to the

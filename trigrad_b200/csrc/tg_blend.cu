@@ -955,8 +955,8 @@ __device__ __forceinline__ int load_pixel_state(const TileCtx& c, const BlendPar
 // gradients of the fragment's interpolations; these go into a queue in shared memory; part B (the
 // expensive barycentric partials and the 21 per-vertex outputs) pops 32 queued fragments at a time and
 // so runs with full warps.  A warp whose lanes are busy anyway (deep overlap, or one opaque layer everywhere) skips the
-// queue.  (200k triangles, full HD: 148 us at 70 % of L1, 64 % of the issue slots and 14 % of DRAM; bound by the latency of
-// the gathers, fifteen of 16 bytes per fragment, and by L1 together.)
+// queue.  (200k triangles, full HD: 140 us at 70 % of L1, 63 % of the issue slots and 13 % of DRAM; bound by the latency of
+// the gathers, fifteen of 16 bytes per fragment, and by L1 together, half of whose work is shared memory's.)
 // DEPTH = false (everywhere below): no gradient flows into the depth map, the terms that it feeds are left out.
 struct QueuedFragment {
     float px, py;
@@ -1226,64 +1226,93 @@ __device__ __noinline__ void backward_rounds_direct(const BlendParams& P, float 
     }
 }
 
-template <int MAXT, bool DEPTH>
-__global__ void __launch_bounds__(MAXT, DEPTH ? 7 : 8) blend_backward_queued_kernel(BlendParams P, BackwardIn in,
+// A CTA takes a block of kQueueCols x kQueueRows pixels, a warp 8x4 of them, and then PASSES - 1 blocks more, each the same
+// number of rows further down; the queues go on through all of them.  What a warp does for 32 pixels of a layer or two is
+// short against the start of a CTA and ends in a queue that is not full: three passes instead of one, B200, kernel: 1.3M
+// triangles of a pixel, full HD 159 -> 115 us; 200k triangles, full HD 163 -> 153; 2M triangles, 4K 822 -> 806.  (Two, four, six
+// passes: 126, 116, 129; 154, 154, 157; 821, 808, 836.  Blocks next to each other: 4K 850 with two, as the deep blocks all lie in
+// the same CTAs and the last of them run alone.  In a loop of a number of passes known at run time the compiler spills.)
+constexpr int kQueueCols = 16, kQueueRows = 8;
+
+template <int PASSES, bool DEPTH>
+__global__ void __launch_bounds__(kQueueCols * kQueueRows, DEPTH ? 7 : 8) blend_backward_queued_kernel(BlendParams P, BackwardIn in,
                                                                         const int* __restrict__ sel,
                                                                         float4* __restrict__ gpack) {
-    static_assert(MAXT % 32 == 0 && MAXT <= 256, "one queue per warp, at most 8 warps");
-    __shared__ __align__(16) float s_coord[MAXT + 2];      // tile_w + tile_h <= tile_w * tile_h + 1 <= MAXT + 1
-    __shared__ float4 s_queue[MAXT / 32][kQueueQuads];
+    constexpr int kWarps = kQueueCols * kQueueRows / 32;
+    __shared__ __align__(16) float s_coord[kQueueCols + PASSES * kQueueRows];
+    __shared__ float4 s_queue[kWarps][kQueueQuads];
     allow_dependents();
-    await_prerequisites();
-    const TileCtx c = tile_context(P, s_coord);
-    PixelGrad pg;
-    BackState st;
-    float sq = 0.f;
-    const int n = load_pixel_state<DEPTH>(c, P, in, pg, st, &sq);
-    const size_t plane = (size_t)P.W * P.H, index = (size_t)c.iy * P.W + c.ix;
-    const int lane = lane_id();
-    float4* q = s_queue[threadIdx.x >> 5];
-    int id_next = (n > 0) ? sel[(size_t)(n - 1) * plane + index] : 0;   // ids are fetched one fragment ahead
-    if (in.l2_target || in.l2_target_u8) {
-        // loss: warp sum, then one atomic per warp into one of 64 partial sums (spread addresses)
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, d);
-        if (lane == 0 && sq != 0.f) atomicAdd(in.l2_partials + ((blockIdx.x * 8 + (threadIdx.x >> 5)) & (kLossPartials - 1)), sq);
+    const int lane = lane_id(), warp = threadIdx.x >> 5;
+    const int x0 = ((int)blockIdx.x % P.tiles_x) * kQueueCols, y0 = ((int)blockIdx.x / P.tiles_x) * kQueueRows;
+    const int apart = ((P.H + kQueueRows - 1) / kQueueRows + PASSES - 1) / PASSES * kQueueRows;      // rows between passes
+    if ((int)threadIdx.x < kQueueCols) s_coord[threadIdx.x] = pixel_coord(x0 + threadIdx.x, P.W);
+    else if ((int)threadIdx.x < kQueueCols + PASSES * kQueueRows) {
+        const int r = (int)threadIdx.x - kQueueCols;
+        s_coord[threadIdx.x] = pixel_coord(y0 + (r / kQueueRows) * apart + r % kQueueRows, P.H);
     }
-    const int nmax = __reduce_max_sync(0xffffffffu, n), nsum = __reduce_add_sync(0xffffffffu, n);
-    if (nsum * 10 >= nmax * 32 * 9) {
-        // Nearly all lanes have a fragment in every round (90 % or more): the queue would cost more than the idle
-        // lanes do.
-        backward_rounds_direct<DEPTH>(P, c.px, c.py, pg, st, n, nmax, id_next, sel + index, plane, q, gpack);
-        return;
-    }
+    const int lx = 8 * (warp & 1) + (lane & 7);
+    TileCtx c;
+    c.ix = x0 + lx;
+    const size_t plane = (size_t)P.W * P.H;
+    float4* q = s_queue[warp];
     int queued = 0;                                    // uniform over the warp
-    for (int s = 0; s < nmax; s++) {
-        const int k = n - 1 - s;
-        const bool has = k >= 0;
-        const int id = id_next;
-        if (k > 0) id_next = sel[(size_t)(k - 1) * plane + index];
-        const unsigned pushing = __ballot_sync(0xffffffffu, has);
-        if (has) {
-            float m[9], w[3];
-            load_geo(P.geo, id, m, w);
-            const AttrRec a = load_attr<false>(P.attr, id);
-            if (k > 0) prefetch_record(P, id_next);
-            const Bary b = apply_bary(m, c.px, c.py);
-            QueuedFragment f;
-            f.px = c.px; f.py = c.py; f.id = id;
-            backward_state<DEPTH>(w, a, b, pg, st, f);
-            queue_push<DEPTH>(q, queued + __popc(pushing & ((1u << lane) - 1u)), f);
+    float sq_sum = 0.f;
+    __syncthreads();
+    c.px = s_coord[lx];
+    await_prerequisites();
+#pragma unroll 1
+    for (int pass = 0; pass < PASSES; pass++) {
+        const int ly = pass * kQueueRows + 4 * (warp >> 1) + (lane >> 3);
+        c.iy = y0 + pass * apart + ly - pass * kQueueRows;
+        c.active = c.ix < P.W && c.iy < P.H;
+        c.py = s_coord[kQueueCols + ly];
+        PixelGrad pg;
+        BackState st;
+        float sq = 0.f;
+        const int n = load_pixel_state<DEPTH>(c, P, in, pg, st, &sq);
+        sq_sum += sq;
+        const size_t index = (size_t)c.iy * P.W + c.ix;
+        int id_next = (n > 0) ? sel[(size_t)(n - 1) * plane + index] : 0;   // ids are fetched one fragment ahead
+        const int nmax = __reduce_max_sync(0xffffffffu, n), nsum = __reduce_add_sync(0xffffffffu, n);
+        if (nsum * 10 >= nmax * 32 * 9) {
+            // Nearly all lanes have a fragment in every round (90 % or more): the queue would cost more than the idle
+            // lanes do.
+            backward_rounds_direct<DEPTH>(P, c.px, c.py, pg, st, n, nmax, id_next, sel + index, plane, q + kQueuePitch * queued, gpack);
+            continue;
         }
-        queued += __popc(pushing);
-        __syncwarp();
-        if (queued >= 32) {
-            queued -= 32;
-            drain_queue<DEPTH>(P, q, queued, 32, gpack);
+        for (int s = 0; s < nmax; s++) {
+            const int k = n - 1 - s;
+            const bool has = k >= 0;
+            const int id = id_next;
+            if (k > 0) id_next = sel[(size_t)(k - 1) * plane + index];
+            const unsigned pushing = __ballot_sync(0xffffffffu, has);
+            if (has) {
+                float m[9], w[3];
+                load_geo(P.geo, id, m, w);
+                const AttrRec a = load_attr<false>(P.attr, id);
+                if (k > 0) prefetch_record(P, id_next);
+                const Bary b = apply_bary(m, c.px, c.py);
+                QueuedFragment f;
+                f.px = c.px; f.py = c.py; f.id = id;
+                backward_state<DEPTH>(w, a, b, pg, st, f);
+                queue_push<DEPTH>(q, queued + __popc(pushing & ((1u << lane) - 1u)), f);
+            }
+            queued += __popc(pushing);
             __syncwarp();
+            if (queued >= 32) {
+                queued -= 32;
+                drain_queue<DEPTH>(P, q, queued, 32, gpack);
+                __syncwarp();
+            }
         }
     }
     if (queued > 0) drain_queue<DEPTH>(P, q, 0, queued, gpack);
+    if (in.l2_target || in.l2_target_u8) {
+        // loss: warp sum, then one atomic per warp into one of 64 partial sums (spread addresses)
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) sq_sum += __shfl_xor_sync(0xffffffffu, sq_sum, d);
+        if (lane == 0 && sq_sum != 0.f) atomicAdd(in.l2_partials + ((blockIdx.x * kWarps + warp) & (kLossPartials - 1)), sq_sum);
+    }
 }
 
 // ---- one optimisation step of one view in a single kernel -------------------------------------------
@@ -1833,12 +1862,16 @@ static int backward_impl(const float* tri_geo, const float* tri_attr, const int3
         // registers come free only when its slowest warp is done (200k triangles, full HD, when it was made: 179 -> 173
         // us; 64 threads the same, 32 threads slower again).
         tg::BlendParams Q = P;
-        Q.tw = 16; Q.th = 8;
-        Q.tiles_x = (W + Q.tw - 1) / Q.tw;
+        Q.tiles_x = (W + tg::kQueueCols - 1) / tg::kQueueCols;
         Q.offsets = nullptr; Q.ids = nullptr; Q.order = nullptr;
-        const int blocks = Q.tiles_x * ((H + Q.th - 1) / Q.th);
-        auto kernel = grad_depthmap ? tg::blend_backward_queued_kernel<128, true> : tg::blend_backward_queued_kernel<128, false>;
-        TG_CUDA(tg_host::launch_dependent(kernel, blocks, 128, 0, s, Q, in, selection, gpack));
+        // Three passes where they leave three waves of CTAs (eight per SM): 1280x720, 2.3 waves, 40 us in one pass, 42 in three.
+        constexpr int kPasses = 3;
+        const int strips = (H + tg::kQueueRows - 1) / tg::kQueueRows;
+        const bool many = (int64_t)Q.tiles_x * strips >= (int64_t)kPasses * 3 * 8 * 148;
+        const int blocks = Q.tiles_x * (many ? (strips + kPasses - 1) / kPasses : strips);
+        auto kernel = many ? (grad_depthmap ? tg::blend_backward_queued_kernel<kPasses, true> : tg::blend_backward_queued_kernel<kPasses, false>)
+                           : (grad_depthmap ? tg::blend_backward_queued_kernel<1, true> : tg::blend_backward_queued_kernel<1, false>);
+        TG_CUDA(tg_host::launch_dependent(kernel, blocks, tg::kQueueCols * tg::kQueueRows, 0, s, Q, in, selection, gpack));
     } else if (threads <= 256) {
         if (per_pixel_sort) tg::blend_backward_kernel<true, 256><<<tiles, threads, 0, s>>>(P, in, gpack);
         else tg::blend_backward_kernel<false, 256><<<tiles, threads, 0, s>>>(P, in, gpack);
