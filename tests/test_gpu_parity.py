@@ -230,6 +230,30 @@ def test_sort_tile_lists_segment_lengths(lengths):
     assert np.array_equal(ids.cpu().numpy().view(np.uint32), (expect & np.uint64(0xFFFFFFFF)).astype(np.uint32))
 
 
+@pytest.mark.parametrize("n, equal", [
+    (129, 129), (129, 1), (300, 25), (1024, 511), (1024, 512), (1024, 513), (1025, 512), (5000, 513), (8192, 512),
+    (8193, 512), (24_576, 512), (24_576, 2000), (24_577, 10),
+])
+def test_sort_tile_lists_equal_depths(n, equal):
+    """Depths of a real tile, `equal` of them the same: buckets below, at and above the most that are worked off one against
+    the other, in every length class that has buckets.  Two segments with other neighbours, a tenth with the key of an empty
+    clip in the second."""
+    rng = np.random.default_rng(n + equal)
+    depth = rng.uniform(0.1, 10.0, 2 * n).astype(np.float32)
+    depth[rng.permutation(n)[:equal]] = 3.25
+    depth[n:][rng.permutation(n)[:equal]] = 3.25
+    depth[n:][::10] = 1e30
+    hi = O.float_to_ordered_u32(depth).astype(np.uint64)
+    lo = np.concatenate([rng.permutation(n), rng.permutation(n)]).astype(np.uint64)
+    entries = (hi << np.uint64(32)) | lo
+    expect = np.concatenate([np.sort(entries[:n]), np.sort(entries[n:])])
+    dev = Hh.cuda(entries.view(np.int64))
+    ids = Hh.sort_tile_lists(dev, Hh.cuda(np.array([0, n, n, 2 * n], np.int32)))
+    torch.cuda.synchronize()
+    assert np.array_equal(dev.cpu().numpy().view(np.uint64), expect)
+    assert np.array_equal(ids.cpu().numpy().view(np.uint32), (expect & np.uint64(0xFFFFFFFF)).astype(np.uint32))
+
+
 MODES = [
     dict(per_pixel_sort=True, max_layers=32, thr=1 / 256),    # the reference default
     dict(per_pixel_sort=False, max_layers=32, thr=1 / 256),

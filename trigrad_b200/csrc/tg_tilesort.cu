@@ -6,14 +6,14 @@
 // Entries are uint64 words (ordered depth << 32 | triangle), already grouped by tile:
 // tile t owns entries[offsets[t] .. offsets[t+1]).
 //   n <= 128     one warp per tile, rank sort: every element counts the smaller ones (no exchange steps)
-//   n <= 1024    a CTA of 128 threads per tile (work list): bucket sort in shared memory - about as many
-//                buckets as words; one thread sorts a bucket by insertion
+//   n <= 1024    a CTA of 256 threads per tile (work list): bucket sort in shared memory - about as many
+//                buckets as words; in its bucket every word counts the smaller ones
 //   n <= 8192    the same with 1024 threads, two CTAs per SM
 //   n <= 24576   the same with one CTA per SM
 //   beyond       a CTA sorts 16384-entry chunks with a bitonic network in shared memory and runs the network's wide
 //                steps on the segment in global memory
-// Where so many depths of a tile are (nearly) equal that a bucket gets more than kBucketMax words, the bitonic network
-// sorts the segment, 8 or 16 words per thread kept in registers between trips to shared memory.
+// Where so many depths of a tile are (nearly) equal that a bucket gets more than kBucketMax words (the counting, linear in that
+// for every word, then takes as long as the network), or all are equal, the bitonic network sorts the segment, 8 or 16 words per thread kept in registers between trips to shared memory.
 // No kernel here waits on another CTA.
 #include <atomic>
 
@@ -23,6 +23,7 @@ namespace tg {
 
 constexpr int kTileSortWarps = 4;                      // tiles per CTA of the short kernel
 constexpr int kTileSortThreads = 32 * kTileSortWarps;
+constexpr int kTileSortMidThreads = 256;
 constexpr int kTileSortShort = 1024;
 constexpr int kTileSortLongThreads = 1024;
 constexpr int kTileSortChunk = 16384;
@@ -166,13 +167,18 @@ __device__ __forceinline__ int log2_at_least(uint32_t n) {
 }
 
 // ---- bucket sort ---------------------------------------------------------------------------------------
-// n <= NT * E words from seg into s_keys in ascending order, through 2^LOGB buckets of about n / 2^LOGB words each: the
+// n <= NT * E words of seg in ascending order to ids_out (and back), through 2^LOGB buckets of about n / 2^LOGB words each: the
 // words are counted in 256 cells of equal width in depth, and the counts' running sum, linear within a cell, says which
 // share of the words lies below a depth (a tile of a mesh has its depths in a few thin layers).  Subtraction, product, sum
 // and truncation are monotone, so the buckets are in order whatever the rounding.  Words with the depth of an empty clip
-// (1e30) form a cell of their own.  False, for all threads, when a bucket gets too many words (s_keys then holds nothing).
-// `s_count`: 2^LOGB + 1 words; `s_cell`: 258 words; `s_warp`: 32 words.  Every thread of the CTA must call.
-constexpr uint32_t kBucketMax = 24;
+// (1e30) form a cell of their own.  Within its bucket every word counts the smaller ones, all threads at once: a thread per
+// bucket that sorted it by insertion took a quarter of a tile's time, up to 11 of its 20 us where a bucket was full, and gave up
+// beyond 24 words (B200: tiles of 129 to 1024 words of a view of 1.3M triangles 26 -> 20 us, the longer ones, among them one
+// that then went to the network, 25 -> 12; 2M triangles piled up, 4K: 14 -> 12 us, 54 -> 49 and, beyond 8192 words, 57 -> 50).
+// KEEP: the words stay in registers from the first step on, E of them per thread (with 1024 threads they do not fit).
+// False, for all threads, when a bucket gets too many words (nothing has been written then).
+// `s_keys`: n words; `s_count`: 2^LOGB + 1 words; `s_cell`: 258 words; `s_warp`: 32 words.  Every thread of the CTA must call.
+constexpr uint32_t kBucketMax = 512;
 constexpr int kCells = 256;
 __device__ __forceinline__ float depth_of(uint32_t ordered) {
     return __uint_as_float((ordered & 0x80000000u) ? ordered & 0x7fffffffu : ~ordered);
@@ -200,24 +206,31 @@ __device__ __forceinline__ uint32_t cta_exclusive(uint32_t mine, uint32_t* s_war
     return (warp == 0 ? 0u : run) + incl - mine;
 }
 
-template <int NT, int E, int LOGB>
-__device__ bool bucket_sort(uint64_t* s_keys, uint32_t* s_count, uint32_t* s_cell, uint32_t* s_warp, const uint64_t* seg,
-                            uint32_t n, int tid) {
+template <int NT, int E, int LOGB, bool KEEP>
+__device__ __forceinline__ bool bucket_sort(uint64_t* s_keys, uint32_t* s_count, uint32_t* s_cell, uint32_t* s_warp, uint64_t* seg,
+                                            uint32_t n, int32_t* ids_out, bool write_back, int tid) {
     constexpr int B = 1 << LOGB, PER = B / NT, CPER = (kCells + 1 + NT - 1) / NT, WARPS = NT / 32;
     static_assert(PER * NT == B && NT * E <= 32768 && LOGB <= 16, "bucket and rank share a word");
     const int lane = tid & 31, warp = tid >> 5;
     const uint32_t empty_clip = float_to_ordered(1e30f);
-    const uint32_t* depths = reinterpret_cast<const uint32_t*>(seg) + 1;      // the high words
+    uint64_t word[KEEP ? E : 1];
+    if (KEEP) {
+#pragma unroll
+        for (int r = 0; r < E; r++) word[r] = tid + r * NT < n ? seg[tid + r * NT] : 0;
+    }
+    auto depth_word = [&](int r) {            // the high word
+        return KEEP ? (uint32_t)(word[KEEP ? r : 0] >> 32) : reinterpret_cast<const uint32_t*>(seg)[2 * (tid + r * NT) + 1];
+    };
     uint32_t lo = 0xffffffffu, hi = 0;
 #pragma unroll
     for (int r = 0; r < E; r++) {
-        const uint32_t i = tid + r * NT;
-        if (i < n) {
-            const uint32_t u = depths[2 * i];
+        if (tid + r * NT < n) {
+            const uint32_t u = depth_word(r);
             lo = min(lo, u);
             if (u < empty_clip) hi = max(hi, u);
         }
     }
+    for (int b = tid; b <= B; b += NT) s_count[b] = 0;
     lo = __reduce_min_sync(0xffffffffu, lo);
     hi = __reduce_max_sync(0xffffffffu, hi);
     if (lane == 0) { s_warp[warp] = lo; s_cell[warp] = hi; }
@@ -227,7 +240,6 @@ __device__ bool bucket_sort(uint64_t* s_keys, uint32_t* s_count, uint32_t* s_cel
     lo = __reduce_min_sync(0xffffffffu, lo);
     hi = __reduce_max_sync(0xffffffffu, hi);
     __syncthreads();
-    for (int b = tid; b <= B; b += NT) s_count[b] = 0;
     for (int b = tid; b <= kCells; b += NT) s_cell[b] = 0;
     const float first = depth_of(lo), span = depth_of(hi) - first;
     const float scale = (float)(kCells - 1) / span;
@@ -235,9 +247,8 @@ __device__ bool bucket_sort(uint64_t* s_keys, uint32_t* s_count, uint32_t* s_cel
     __syncthreads();
 #pragma unroll
     for (int r = 0; r < E; r++) {
-        const uint32_t i = tid + r * NT;
-        if (i < n) {
-            const uint32_t u = depths[2 * i];
+        if (tid + r * NT < n) {
+            const uint32_t u = depth_word(r);
             atomicAdd(&s_cell[u < empty_clip ? min(kCells - 1, (int)((depth_of(u) - first) * scale)) : kCells], 1u);
         }
     }
@@ -262,18 +273,19 @@ __device__ bool bucket_sort(uint64_t* s_keys, uint32_t* s_count, uint32_t* s_cel
     }
     __syncthreads();
     const float per_word = (float)B / (float)n;
+    auto bucket_of = [&](uint32_t u) {
+        const float x = u < empty_clip ? fminf((depth_of(u) - first) * scale, (float)kCells - 0.5f) : (float)kCells;
+        const int cell = (int)x;
+        const float below = (float)s_cell[cell];
+        const float share = fminf(fmaf(x - (float)cell, (float)s_cell[cell + 1] - below, below), (float)s_cell[cell + 1]);
+        return min(B - 1, (int)(share * per_word));
+    };
     uint32_t where[E];               // bucket << 15 | rank in it
 #pragma unroll
     for (int r = 0; r < E; r++) {
-        const uint32_t i = tid + r * NT;
         where[r] = 0;
-        if (i < n) {
-            const uint32_t u = depths[2 * i];
-            const float x = u < empty_clip ? fminf((depth_of(u) - first) * scale, (float)kCells - 0.5f) : (float)kCells;
-            const int cell = (int)x;
-            const float below = (float)s_cell[cell];
-            const float share = fminf(fmaf(x - (float)cell, (float)s_cell[cell + 1] - below, below), (float)s_cell[cell + 1]);
-            const int b = min(B - 1, (int)(share * per_word));
+        if (tid + r * NT < n) {
+            const int b = bucket_of(depth_word(r));
             where[r] = ((uint32_t)b << 15) | atomicAdd(&s_count[b], 1u);
         }
     }
@@ -295,37 +307,20 @@ __device__ bool bucket_sort(uint64_t* s_keys, uint32_t* s_count, uint32_t* s_cel
     if (tid == NT - 1) s_count[B] = n;
     __syncthreads();
 #pragma unroll
-    for (int r = 0; r < E; r++) {
-        const uint32_t i = tid + r * NT;
-        if (i < n) s_keys[s_count[where[r] >> 15] + (where[r] & 0x7fffu)] = seg[i];
-    }
-    __syncthreads();
-    for (int b = tid; b < B; b += NT) {
-        const int beg = (int)s_count[b], end = (int)s_count[b + 1];
-        for (int i = beg + 1; i < end; i++) {
-            const uint64_t x = s_keys[i];
-            int at = i;
-            for (; at > beg; at--) {
-                const uint64_t y = s_keys[at - 1];
-                if (y <= x) break;
-                s_keys[at] = y;
-            }
-            s_keys[at] = x;
-        }
-    }
-    __syncthreads();
-    return true;
-}
-
-template <int NT>
-__device__ __forceinline__ void hand_out(const uint64_t* s_keys, uint64_t* seg, uint32_t n, int32_t* ids_out, bool write_back,
-                                         int tid) {
+    for (int r = 0; r < E; r++)
+        if (tid + r * NT < n) s_keys[s_count[where[r] >> 15] + (where[r] & 0x7fffu)] = KEEP ? word[KEEP ? r : 0] : seg[tid + r * NT];
+    __syncthreads();                          // nobody reads seg from here on
+    // the words in the order of their buckets, so that neighbouring threads write next to each other
     for (uint32_t i = tid; i < n; i += NT) {
         const uint64_t x = s_keys[i];
-        ids_out[i] = (int32_t)(uint32_t)x;
-        if (write_back) seg[i] = x;
+        const int b = bucket_of((uint32_t)(x >> 32)), end = (int)s_count[b + 1];
+        int at = (int)s_count[b];
+        for (int k = at; k < end; k++) at += s_keys[k] < x ? 1 : 0;
+        ids_out[at] = (int32_t)(uint32_t)x;
+        if (write_back) seg[at] = x;
     }
-    __syncthreads();
+    __syncthreads();                          // the shared arrays are the next tile's
+    return true;
 }
 
 // Work lists in the sort's scratch: [0] long tiles, [1] next long item of the kernel for the longest,
@@ -394,8 +389,9 @@ __global__ void __launch_bounds__(kTileSortThreads) tile_sort_kernel(uint64_t* _
     else rank_sort_warp<kTileSortRank / 32>(s, entries, sorted_ids, beg, n, lane, write_back);
 }
 
-// Tiles of kTileSortRank < n <= kTileSortShort entries: persistent CTAs of 128 threads, next free item first.
-__global__ void __launch_bounds__(kTileSortThreads) tile_sort_mid_kernel(uint64_t* entries,
+// Tiles of kTileSortRank < n <= kTileSortShort entries: persistent CTAs of 256 threads (128 take 10 % longer, 64 half as
+// long again), next free item first.
+__global__ void __launch_bounds__(kTileSortMidThreads) tile_sort_mid_kernel(uint64_t* entries,
                                                                          const int32_t* __restrict__ offsets, int tiles,
                                                                          int32_t* __restrict__ sorted_ids, uint32_t* lists,
                                                                          int write_back) {
@@ -415,10 +411,8 @@ __global__ void __launch_bounds__(kTileSortThreads) tile_sort_mid_kernel(uint64_
         const int tile = (int)mid_items(lists, tiles)[w];
         const int beg = offsets[tile];
         const uint32_t n = (uint32_t)(offsets[tile + 1] - beg);
-        if (bucket_sort<kTileSortThreads, 8, 10>(s_mid, s_count, s_cell, s_warp, entries + beg, n, tid))
-            hand_out<kTileSortThreads>(s_mid, entries + beg, n, sorted_ids + beg, write_back != 0, tid);
-        else
-            sort_segment_in_smem<3, kTileSortThreads>(s_mid, entries + beg, n, log2_at_least(n), sorted_ids + beg,
+        if (!bucket_sort<kTileSortMidThreads, 4, 10, true>(s_mid, s_count, s_cell, s_warp, entries + beg, n, sorted_ids + beg, write_back != 0, tid))
+            sort_segment_in_smem<3, kTileSortMidThreads>(s_mid, entries + beg, n, log2_at_least(n), sorted_ids + beg,
                                                       write_back != 0, tid);
     }
 }
@@ -472,14 +466,14 @@ __global__ void __launch_bounds__(kTileSortLongThreads, BIG ? 1 : 2)
         if ((n > (uint32_t)kTileSortHalf) != BIG) continue;
         uint64_t* seg = entries + beg;
         if (!BIG) {
-            if (bucket_sort<kTileSortLongThreads, 8, 12>(s_long, s_count, s_cell, s_warp, seg, n, tid))
-                hand_out<kTileSortLongThreads>(s_long, seg, n, sorted_ids + beg, write_back != 0, tid);
-            else             // 8 words per thread: 256, 512 or 1024 threads take part
+            if (!bucket_sort<kTileSortLongThreads, 8, 12, false>(s_long, s_count, s_cell, s_warp, seg, n, sorted_ids + beg, write_back != 0, tid))
+                // 8 words per thread: 256, 512 or 1024 threads take part
                 sort_segment_in_smem<3, kTileSortLongThreads>(s_long, seg, n, log2_at_least(n), sorted_ids + beg,
                                                               write_back != 0, tid);
         } else if (n <= (uint32_t)kTileSortBig &&
-                   bucket_sort<kTileSortLongThreads, 24, 12>(s_long, s_count, s_cell, s_warp, seg, n, tid)) {
-            hand_out<kTileSortLongThreads>(s_long, seg, n, sorted_ids + beg, write_back != 0, tid);
+                   bucket_sort<kTileSortLongThreads, 24, 12, false>(s_long, s_count, s_cell, s_warp, seg, n, sorted_ids + beg,
+                                                                    write_back != 0, tid)) {
+            // sorted
         } else if (n <= (uint32_t)kTileSortChunk) {
             sort_segment_in_smem<4, kTileSortLongThreads>(s_long, seg, n, kLogChunk, sorted_ids + beg, write_back != 0,
                                                           tid);
@@ -532,8 +526,8 @@ int sort_short_lists(uint64_t* entries, const int32_t* offsets, int tiles, int32
 int sort_long_lists(uint64_t* entries, const int32_t* offsets, int tiles, int32_t* sorted_ids, uint32_t* lists, bool write_back,
                     uint32_t longest, cudaStream_t s) {
     if (longest > (uint32_t)tg::kTileSortRank) {
-        const int grid = tiles < 148 * 12 ? tiles : 148 * 12;
-        TG_CUDA(launch_dependent(tg::tile_sort_mid_kernel, grid, tg::kTileSortThreads, 0, s, entries, offsets, tiles, sorted_ids,
+        const int grid = tiles < 148 * 8 ? tiles : 148 * 8;
+        TG_CUDA(launch_dependent(tg::tile_sort_mid_kernel, grid, tg::kTileSortMidThreads, 0, s, entries, offsets, tiles, sorted_ids,
                                  lists, write_back ? 1 : 0));
         TG_LAUNCH_CHECK("tile_sort_mid_kernel");
     }
