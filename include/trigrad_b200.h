@@ -309,6 +309,15 @@ int tg_blend_step_l2(const float* tri_geo, const float* tri_attr, const int32_t*
 #define TG_EXPECT_SHORT_LISTS 8u
 #define TG_SHORT_LIST 128
 #define TG_WORKSPACE_READY 16u
+/*                TG_NO_COUNT: the call returns without waiting for K.  For renders so small that the largest K there can be is
+ *                no matter: T <= TG_NO_COUNT_TRIANGLES, list_capacity >= T * tiles, at most 1184 tiles, TG_INFO_MAPPED, no
+ *                stage_ms_host, and not while the stream is being captured (otherwise TG_ERR_BAD_ARG).  info_host is not
+ *                waited for and receives nothing but, in [1], the length of the longest list where that is beyond
+ *                TG_SHORT_LIST, whenever the binning gets there: such lists are sorted slowly, so a caller that finds it
+ *                had better do without the flag for a while.  Results do not depend on it.
+ */
+#define TG_NO_COUNT 32u
+#define TG_NO_COUNT_TRIANGLES 4096
 size_t tg_forward_workspace_bytes(int T, int tiles, uint32_t list_capacity);
 int tg_render_forward(const float* vertices, const int32_t* indices, const float* colors, const float* opacities,
                       int T, int W, int H, int tile_w, int tile_h, float early_stopping_threshold,

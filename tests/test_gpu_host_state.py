@@ -7,6 +7,7 @@ import pytest
 import torch
 
 import helpers as Hh
+import oracle as O
 import trigrad_b200
 from trigrad_b200 import scenes as S
 from trigrad_b200 import views
@@ -145,3 +146,55 @@ def test_more_streams_than_states_are_kept():
         job.check(got)
     for h in handles:
         assert int(torch.cuda.cudart().cudaStreamDestroy(h)) == 0
+
+
+@pytest.mark.parametrize("tile", [16, 8, 32])
+@pytest.mark.parametrize("sort", [True, False])
+def test_lists_that_grow_beyond_what_the_calls_before_had(tile, sort):
+    """Small renders behind one with short lists do not wait for the number of entries; the first with long lists gets them
+    sorted where they are, later ones as any others, and short ones again go back to not waiting."""
+    w, h = 197, 121
+    short = S.random_triangles(300, w, h, 0.05, 0.4, name="short", seed=tile)
+    long = S.random_triangles(2000, w, h, 0.6, 0.4, name="long", seed=tile + 1)
+    rng = np.random.default_rng(5)
+    gi, gd = rng.normal(size=(h, w, 4)).astype(np.float32), rng.normal(size=(h, w)).astype(np.float32)
+    with torch.cuda.stream(torch.cuda.Stream()):
+        outs = []
+        for sc in (short, short, short, long, long, long, short, short, long):
+            v, i, c, o = Hh.scene_tensors(sc)
+            leaves = [t.requires_grad_() for t in (v, c, o)]
+            out = trigrad_b200.render(leaves[0], i, leaves[1], leaves[2], w, h, tile, tile, per_pixel_sort=sort)
+            outs.append((sc, out[0], torch.autograd.grad(out, leaves, (Hh.cuda(gi), Hh.cuda(gd)))))
+        torch.cuda.synchronize()
+    for sc in (short, long):
+        of = O.forward(sc.vertices, sc.indices, sc.colors, sc.opacities, w, h, tile, tile, 1 / 256, sort)
+        assert (np.diff(of.lists.offsets).max() > 128) == (sc is long)
+        og = O.backward(sc.vertices, sc.indices, sc.colors, sc.opacities, w, h, of, gi, gd, tile, tile, sort)
+        for image, grads in ((x[1], x[2]) for x in outs if x[0] is sc):
+            assert np.array_equal(image.detach().cpu().numpy().view(np.uint32), of.image.view(np.uint32))
+            for a, b in zip(grads, og):
+                assert Hh.rel_l2(a.cpu().numpy(), b) <= 1e-4
+
+
+@pytest.mark.parametrize("triangles, capacity, flags", [
+    (4097, 4097 * 64, 4 | 32),       # more triangles than the flag is for
+    (100, 100 * 64 - 1, 4 | 32),     # a list that could overflow
+    (100, 100 * 64, 32),             # host memory that kernels cannot write
+])
+def test_not_counting_is_refused_where_it_is_not_safe(triangles, capacity, flags):
+    from trigrad_b200 import _native as N
+
+    sc = S.random_triangles(triangles, 128, 128, 0.05, 0.4, name="refused")
+    out = trigrad_b200.wrapper.forward_native(*Hh.scene_tensors(sc), 128, 128, 16, 16, 1 / 256, False, True, 32)
+    ptr = lambda t: ctypes.c_void_p(t.data_ptr())
+    lib = N.lib()
+    size = lib.tg_forward_workspace_bytes(triangles, 64, capacity)
+    ws = torch.empty(size + 256, dtype=torch.uint8, device="cuda")
+    info = torch.zeros(4, dtype=torch.int32).pin_memory()
+    image, depth, fw, ids, off, geo, attr, ends, sel = out[:9]
+    ids = torch.empty(capacity, dtype=torch.int32, device="cuda")
+    t = Hh.scene_tensors(sc)
+    status = lib.tg_render_forward(*(ptr(x) for x in (t[0], t[1], t[2], t[3])), triangles, 128, 128, 16, 16, 1 / 256, 1, 32, ptr(image),
+                                   ptr(depth), ptr(fw), ptr(ends), ptr(sel), ptr(geo), ptr(attr), ptr(ids), capacity, ptr(off),
+                                   ctypes.c_void_p((ws.data_ptr() + 255) // 256 * 256), size, ptr(info), None, flags, ctypes.c_void_p(0))
+    assert status == 1

@@ -80,7 +80,7 @@ struct StageTimer {
 struct TileLists {
     ForwardWorkspace ws;
     int tiles;
-    bool device_scan, mapped;
+    bool device_scan, mapped, no_count;
     cudaEvent_t k_ready = nullptr;
     uint32_t* device_status;               // error word, null where no kernel of the path can raise it
     uint32_t K = 0, longest = 0;
@@ -88,7 +88,7 @@ struct TileLists {
 
     TileLists(void* workspace, int T, int W, int H, int tw, int th, uint32_t cap, unsigned flags)
         : ws(workspace, ((W + tw - 1) / tw) * ((H + th - 1) / th), cap), tiles(((W + tw - 1) / tw) * ((H + th - 1) / th)),
-          device_scan(tiles > tg::kTileScanByOneCta), mapped((flags & TG_INFO_MAPPED) != 0 && T > 0),
+          device_scan(tiles > tg::kTileScanByOneCta), mapped((flags & TG_INFO_MAPPED) != 0 && T > 0), no_count((flags & TG_NO_COUNT) != 0),
           device_status(device_scan ? ws.bin.status : nullptr) {}       // only the scan waits
 
     int start(const float* vertices, const int32_t* indices, const float* colors, const float* opacities, int T, int W, int H,
@@ -99,8 +99,10 @@ struct TileLists {
             return TG_ERR_WORKSPACE;
         }
         TG_REQUIRE(cap == 0 || sorted_ids != nullptr, "null sorted_ids");
-        info_host[0] = kNotArrived;     // K < 2^31, so this value means "K has not landed yet"
-        info_host[1] = info_host[2] = info_host[3] = 0;
+        if (!no_count) {
+            info_host[0] = kNotArrived;     // K < 2^31, so this value means "K has not landed yet"
+            info_host[1] = info_host[2] = info_host[3] = 0;
+        }
         if (!mapped)
             if (int st = scratch_event(&k_ready)) return st;
         // beyond 65536 tiles the lists are the reference's
@@ -113,7 +115,9 @@ struct TileLists {
                                             (flags & TG_WORKSPACE_READY) != 0, s))
             return st;
         timer.mark();                                                    // [2] start of "per_tile_lists"
-        if (int st = tg_host::place_entries(ws.bin, T, W, H, tw, th, offsets, cap, mapped ? info_host : nullptr, s)) return st;
+        if (int st = tg_host::place_entries(ws.bin, T, W, H, tw, th, offsets, cap, mapped && !no_count ? info_host : nullptr,
+                                            no_count ? info_host + 1 : nullptr, s))
+            return st;
         if (!mapped) {
             // [3] first: the host watches the word K arrives in
             TG_CUDA(cudaMemcpyAsync(&info_host[3], ws.bin.info + 2, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
@@ -184,7 +188,7 @@ static int check_forward_args(int T, int W, int H, int tw, int th, int max_layer
     TG_REQUIRE(workspace && info_host && offsets, "null pointer");
     TG_REQUIRE(((uintptr_t)workspace & 255) == 0, "workspace must be 256-byte aligned");
     TG_REQUIRE(list_capacity < 0x80000000u, "list capacity must stay below 2^31");
-    TG_REQUIRE((flags & ~31u) == 0, "unknown flag");
+    TG_REQUIRE((flags & ~63u) == 0, "unknown flag");
     TG_REQUIRE(!(flags & TG_EXPECT_SHORT_LISTS) || (flags & TG_INFO_MAPPED), "TG_EXPECT_SHORT_LISTS needs TG_INFO_MAPPED");
     return TG_OK;
 }
@@ -226,17 +230,25 @@ int tg_render_forward(const float* vertices, const int32_t* indices, const float
     cudaStream_t s = (cudaStream_t)stream;
     StageTimer timer(stage_ms_host != nullptr, s);
     TileLists lists(workspace, T, W, H, tw, th, list_capacity, flags);
+    if (lists.no_count) {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        TG_CUDA(cudaStreamIsCapturing(s, &capture));
+        TG_REQUIRE(T > 0 && T <= tg::kNoCountTriangles && lists.tiles <= tg::kFusedTiles && (flags & TG_INFO_MAPPED) &&
+                       (uint64_t)list_capacity >= (uint64_t)T * lists.tiles && stage_ms_host == nullptr &&
+                       capture == cudaStreamCaptureStatusNone,
+                   "TG_NO_COUNT is for small renders with room for every list, see the header");
+    }
     if (int st = lists.start(vertices, indices, colors, opacities, T, W, H, tw, th, tri_geo, tri_attr, sorted_ids, list_capacity,
                              offsets, workspace_bytes, info_host, flags, timer, s))
         return st;
     // Lists of up to kFusedList entries are sorted by the compositing kernel itself in images of few tiles, where the caller
     // expects nothing longer: it checks on the device what the host is told afterwards.
-    const bool early = lists.tiles <= tg::kFusedTiles && T > 0 && (flags & TG_EXPECT_SHORT_LISTS) != 0 && stage_ms_host == nullptr;
+    const bool early = lists.tiles <= tg::kFusedTiles && T > 0 && (flags & (TG_EXPECT_SHORT_LISTS | TG_NO_COUNT)) != 0 && stage_ms_host == nullptr;
     timer.mark();                                                    // [3] start of "sorting"
-    int st = early ? tg_host::blend_forward_short(tri_geo, tri_attr, lists.ws.bin, list_capacity, sorted_ids, offsets, W, H, tw, th,
-                                                  thr, per_pixel_sort, max_layers, image, depthmap, final_weights, ends, selection, s)
+    int st = early ? tg_host::blend_forward_short(tri_geo, tri_attr, lists.ws.bin, list_capacity, lists.no_count, sorted_ids, offsets, W,
+                                                  H, tw, th, thr, per_pixel_sort, max_layers, image, depthmap, final_weights, ends, selection, s)
                    : lists.sort_short(sorted_ids, offsets, list_capacity, T, s);
-    if (st) return st;
+    if (st || lists.no_count) return st;
     if ((st = lists.wait(list_capacity, info_host, s))) return st;
     if (!early || lists.longest > tg::kFusedList) {
         if (early && (st = lists.sort_short(sorted_ids, offsets, list_capacity, T, s))) return st;
@@ -265,6 +277,7 @@ int tg_render_step_l2(const float* vertices, const int32_t* indices, const float
                       tg_stream_t stream) {
     TG_REQUIRE(image && depthmap && final_weights && ends && target, "null pointer");
     if (int st = check_forward_args(T, W, H, tw, th, max_layers, workspace, info_host, offsets, list_capacity, flags)) return st;
+    TG_REQUIRE(!(flags & TG_NO_COUNT), "the one-kernel step waits for the number of entries");
     TG_REQUIRE(tw * th <= 256 && max_layers <= 32, "the one-kernel step needs tiles of at most 256 pixels and max_layers <= 32");
     cudaStream_t s = (cudaStream_t)stream;
     StageTimer timer(stage_ms_host != nullptr, s);

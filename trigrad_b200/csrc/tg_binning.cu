@@ -573,6 +573,7 @@ struct BinArgs {
     uint32_t* info;          // [3] K, when scan_here the longest list (kOrderWrittenBit: a launch order is wanted), slots;
                              // K and slots no larger than kTooManyPairs
     uint32_t* info_host;     // words 0, 1 and 3 of mapped host memory receive them too, or null
+    uint32_t* long_host;     // mapped host memory that receives the longest list if it has more than kFusedList entries, or null
     uint4* pairs;            // [capacity]
     uint32_t capacity;
     int tiles, tiles_x, tiles_y;
@@ -620,6 +621,7 @@ __device__ __forceinline__ void publish_counts(const BinArgs& bin, uint32_t K, u
         __threadfence_system();
         h[0] = K;
     }
+    if (bin.long_host && (longest & ~kOrderWrittenBit) > kFusedList) *(volatile uint32_t*)bin.long_host = longest & ~kOrderWrittenBit;
 }
 __device__ __forceinline__ uint32_t slots_used(const BinArgs& bin) {
     return (uint32_t)min(__ldcg(slot_counter(bin)), (unsigned long long)kTooManyPairs);
@@ -961,9 +963,9 @@ int prefer_smem(const void* kernel, int kilobytes, SmemAllowed& preferred) {
 }
 
 static tg::BinArgs bin_args(const BinBuffers& b, int W, int H, int tw, int th, int32_t* offsets, uint32_t list_capacity,
-                            uint32_t* info_host) {
+                            uint32_t* info_host, uint32_t* long_host) {
     const int tiles_x = (W + tw - 1) / tw, tiles_y = (H + th - 1) / th, tiles = tiles_x * tiles_y;
-    return {b.tile_counts, offsets, b.counters, b.info, info_host, b.pairs, list_capacity, tiles, tiles_x, tiles_y,
+    return {b.tile_counts, offsets, b.counters, b.info, info_host, long_host, b.pairs, list_capacity, tiles, tiles_x, tiles_y,
             tiles <= tg::kTileScanByOneCta ? 1 : 0, b.tile_order ? 1 : 0, {b.tables, b.tables + tiles_x}};
 }
 
@@ -1001,7 +1003,7 @@ int bin_triangles(const float* vertices, const int32_t* indices, const float* co
     constexpr int kWave = 148 * 32 / tg::kBinWarps;
     const int per_cta = T >= 32 * tg::kBinWarps * kWave ? 32 * tg::kBinWarps : (T + kWave - 1) / kWave;
     const int grid = (T + per_cta - 1) / per_cta;
-    const tg::BinArgs bin = bin_args(b, W, H, tw, th, offsets, list_capacity, nullptr);
+    const tg::BinArgs bin = bin_args(b, W, H, tw, th, offsets, list_capacity, nullptr, nullptr);
     auto inverse = [](int n) { return (n & (n - 1)) == 0 ? 1.0 / n : 0.0; };
     auto kernel = cull ? tg::bin_kernel<true> : tg::bin_kernel<false>;
     static SmemAllowed bin_allowed[2];
@@ -1014,9 +1016,9 @@ int bin_triangles(const float* vertices, const int32_t* indices, const float* co
 }
 
 int place_entries(const BinBuffers& b, int T, int W, int H, int tw, int th, int32_t* offsets, uint32_t list_capacity,
-                  uint32_t* info_host, cudaStream_t stream) {
+                  uint32_t* info_host, uint32_t* long_host, cudaStream_t stream) {
     if (T == 0) return TG_OK;
-    const tg::BinArgs bin = bin_args(b, W, H, tw, th, offsets, list_capacity, info_host);
+    const tg::BinArgs bin = bin_args(b, W, H, tw, th, offsets, list_capacity, info_host, long_host);
     const int tiles = bin.tiles;
     if (tiles <= tg::kPlaceTiles) {
         // One CTA per SM, and no more than the list capacity, which is what the host knows of the number of pairs, fills; the

@@ -639,6 +639,7 @@ struct UnsortedLists {
     const uint64_t* entries;      // ordered depth << 32 | triangle, grouped by tile
     AfterBinning bin;
     int* sorted_ids;
+    bool any_length;              // false: the host launches other kernels when a list is longer than kFusedList
 };
 template <bool SORT, int MAXT, bool STREAM = false, bool FUSED = false>
 __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (SORT ? 4 : 5) : 1) blend_forward_kernel(BlendParams P, float4* __restrict__ image,
@@ -662,7 +663,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (SORT ? 4 : 5) : 1) blend_
         // launched before the host knows: nothing to do when the lists are too long or incomplete
         unsorted.bin.clear((int)blockIdx.x, threadIdx.x == 0);
         const uint32_t longest = unsorted.bin.info[1] & ~kOrderWrittenBit;
-        if (unsorted.bin.incomplete() || longest > kFusedList) return;
+        if (unsorted.bin.incomplete() || (longest > kFusedList && !unsorted.any_length)) return;
     }
     const int this_tile = tile_of_block(P);
     const int list_first = P.offsets[this_tile], list_n = P.offsets[this_tile + 1] - list_first;
@@ -681,7 +682,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (SORT ? 4 : 5) : 1) blend_
     }
     const bool one_chunk = SORT && list_n <= kChunk, two_chunks = SORT && !STREAM && !one_chunk && list_n <= 2 * kChunk;
     if (FUSED) {
-        for (int i = threadIdx.x; i < list_n; i += blockDim.x) {
+        for (int i = threadIdx.x; i < min(list_n, (int)kFusedList); i += blockDim.x) {
             s_key[i] = unsorted.entries[list_first + i];
             s_rank[i] = 0;
         }
@@ -693,7 +694,19 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (SORT ? 4 : 5) : 1) blend_
         stage_geo_async(P, list_first, list_n, s_geo);
     }
     const TileCtx c = tile_context(P, s_coord);      // its barrier makes the words above visible
-    if (FUSED) {
+    if (FUSED && list_n > (int)kFusedList) {
+        // rare (see TG_NO_COUNT): every word counts the smaller ones of the whole list, in memory
+        const uint64_t* words = unsorted.entries + c.start;
+        for (int i = threadIdx.x; i < list_n; i += blockDim.x) {
+            const uint64_t mine = words[i];
+            int at = 0;
+            for (int j = 0; j < list_n; j++) at += words[j] < mine ? 1 : 0;
+            unsorted.sorted_ids[c.start + at] = (int)(uint32_t)mine;
+        }
+        P.ids = unsorted.sorted_ids;
+        __syncthreads();
+        if (!SORT) ListPipe{s_geo}.copy(P, 0, c.start, kChunk);
+    } else if (FUSED) {
         const int n = c.end - c.start, nt = blockDim.x;
         // several threads per word where the CTA has them, each counting over a part of the list
         const int words = n <= 32 ? 32 : n <= 64 ? 64 : (int)kFusedList, parts = max(1, nt / words);
@@ -1755,14 +1768,15 @@ void set_tile_order(const uint32_t* order, uint32_t longest_list) {
     g_longest_list = longest_list;
 }
 
-int blend_forward_short(const float* tri_geo, const float* tri_attr, const BinBuffers& b, uint32_t capacity, int32_t* sorted_ids, const int32_t* offsets, int W, int H, int tw, int th, float thr,
+int blend_forward_short(const float* tri_geo, const float* tri_attr, const BinBuffers& b, uint32_t capacity, bool any_length,
+                        int32_t* sorted_ids, const int32_t* offsets, int W, int H, int tw, int th, float thr,
                         int per_pixel_sort, int max_layers, float* image, float* depthmap, float* final_weights,
                         int32_t* ends, int32_t* selection, cudaStream_t s) {
     TG_REQUIRE(((uintptr_t)image & 15) == 0, "image must be 16-byte aligned");
     if (tg_selection_planes(per_pixel_sort, max_layers) == 0) selection = nullptr;
     const tg::BlendParams P = make_params(tri_geo, tri_attr, nullptr, offsets, W, H, tw, th, thr, max_layers);
     const int tiles = P.tiles_x * ((H + th - 1) / th);
-    const tg::UnsortedLists lists = {b.entries, after_binning(&b, tiles, capacity), sorted_ids};
+    const tg::UnsortedLists lists = {b.entries, after_binning(&b, tiles, capacity), sorted_ids, any_length};
     const int threads = ((tw * th + 31) / 32) * 32;
     auto kernel = threads <= 256 ? (per_pixel_sort ? tg::blend_forward_kernel<true, 256, false, true>
                                                    : tg::blend_forward_kernel<false, 256, false, true>)

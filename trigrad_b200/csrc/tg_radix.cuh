@@ -32,6 +32,9 @@ constexpr int kTileSortRank = 128;
 // against 110 + 6).
 constexpr uint32_t kFusedList = TG_SHORT_LIST;
 constexpr int kFusedTiles = 2 * 4 * 148;
+// A call that does not wait for the number of entries (TG_NO_COUNT) has at most this many triangles, which is also the
+// longest list that its compositing kernel can meet.
+constexpr int kNoCountTriangles = TG_NO_COUNT_TRIANGLES;
 
 // Exclusive scan of one value per thread over the first 256 threads of a CTA (all threads of the CTA
 // must call it; threads beyond 256 pass 0 and ignore the result).
@@ -131,10 +134,11 @@ int bin_triangles(const float* vertices, const int32_t* indices, const float* co
                   int H, int tw, int th, float* tri_geo, float* tri_attr, const BinBuffers& b, int32_t* offsets,
                   uint32_t list_capacity, bool cull, bool packed, bool ready, cudaStream_t stream);
 // Entries grouped by tile, offsets, info, launch order.  `info_host`: mapped host memory whose words 0, 1 and 3 receive the
-// three info words (K last), or null.  Counts and counters of images of at most kPlaceTiles tiles are left to the kernel
+// three info words (K last), or null; `long_host`: one that receives the longest list where it has more than kFusedList
+// entries, or null.  Counts and counters of images of at most kPlaceTiles tiles are left to the kernel
 // behind to clear (the sort's first one, or the compositing kernel that sorts short lists itself).
 int place_entries(const BinBuffers& b, int T, int W, int H, int tw, int th, int32_t* offsets, uint32_t list_capacity,
-                  uint32_t* info_host, cudaStream_t stream);
+                  uint32_t* info_host, uint32_t* long_host, cudaStream_t stream);
 // The sort in two steps.  The first launch sorts lists of up to kTileSortRank entries and makes work lists of the others; it
 // needs nothing from the host: given `b`, it does nothing where the slots exceed `capacity`, and clears the counts and
 // counters (see above).  The second, when the longest list is known, launches what the other length classes need.
@@ -147,9 +151,11 @@ inline tg::AfterBinning after_binning(const BinBuffers* b, int tiles, uint32_t c
 }
 int sort_long_lists(uint64_t* entries, const int32_t* offsets, int tiles, int32_t* sorted_ids, uint32_t* lists, bool write_back,
                     uint32_t longest, cudaStream_t stream);
-// Forward compositing with the sort of the tile lists (at most kFusedList entries each, `info` as the binning kernel left
-// it) in the same kernel, which does nothing when a list is longer or the slots exceed `capacity`.
-int blend_forward_short(const float* tri_geo, const float* tri_attr, const BinBuffers& b, uint32_t capacity, int32_t* sorted_ids, const int32_t* offsets, int W, int H, int tw, int th, float thr,
+// Forward compositing with the sort of the tile lists (at most kFusedList entries each, `info` as the binning left it) in the
+// same kernel, which does nothing when the slots exceed `capacity` or a list is longer; with `any_length` it sorts longer
+// ones too, slowly.
+int blend_forward_short(const float* tri_geo, const float* tri_attr, const BinBuffers& b, uint32_t capacity, bool any_length,
+                        int32_t* sorted_ids, const int32_t* offsets, int W, int H, int tw, int th, float thr,
                         int per_pixel_sort, int max_layers, float* image, float* depthmap, float* final_weights,
                         int32_t* ends, int32_t* selection, cudaStream_t stream);
 }  // namespace tg_host

@@ -19,6 +19,7 @@
 #include <ATen/Parallel.h>
 #include <ATen/TracerMode.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/custom_function.h>
@@ -140,7 +141,7 @@ T* data(const Tensor& t) { return t.defined() ? static_cast<T*>(t.data_ptr()) : 
 struct DeviceState {
     static constexpr int kSlots = 256;
     std::mutex use;
-    Tensor workspace, info;      // info [slots,4] int32 pinned: K, longest list, error word, -
+    Tensor workspace, info;      // info [slots + 1,4] int32 pinned: K, longest list, error word, slots; last row: see no_count
     int slot = 0, last_slot = -1;
     int64_t k_estimate = 0;
     bool short_lists = false;          // the last forward had no tile list beyond TG_SHORT_LIST entries
@@ -154,7 +155,7 @@ struct DeviceState {
 
     explicit DeviceState(at::Device device) {
         workspace = at::empty({0}, at::TensorOptions().dtype(at::kByte).device(device));
-        info = at::zeros({kSlots, 4}, at::TensorOptions().dtype(at::kInt)).pin_memory();
+        info = at::zeros({kSlots + 1, 4}, at::TensorOptions().dtype(at::kInt)).pin_memory();
     }
     int32_t* words(int s) { return info.data_ptr<int32_t>() + 4 * s; }
     int next_slot() {
@@ -173,6 +174,19 @@ struct DeviceState {
         throw std::runtime_error("trigrad_b200: an earlier render reported device error word " + std::to_string(stale) +
                                  " (a bounded wait ran out inside a kernel); its outputs are not valid");
     }
+    // Whether a call can do without the number of entries on the host (TG_NO_COUNT): the lists were short when last looked at
+    // (the kernels of calls that did not wait say so, in the row that is theirs alone, as soon as they no longer are), and
+    // the room for every pair of triangle and tile is small.  28 bytes each, so 14 MB.
+    static constexpr int64_t kNoCountPairs = int64_t(1) << 19;
+    bool no_count(int64_t T, int64_t tiles) {
+        volatile int32_t* longest = words(kSlots) + 1;
+        if (*longest) {
+            *longest = 0;
+            short_lists = false;
+        }
+        return short_lists && T <= TG_NO_COUNT_TRIANGLES && T * tiles <= kNoCountPairs && tiles <= kNoCountTiles;
+    }
+    static constexpr int64_t kNoCountTiles = 1184;
     // After a forward call that used slot `s` has returned: it waited for work recorded after the previous call's on
     // this stream, so the previous call's error word has arrived.
     void finish_call(int s) {
@@ -307,8 +321,9 @@ struct L2Step {     // forward, loss and gradients in one call (tg_render_step_l
 };
 
 // `opacities` undefined: packed inputs (indices [T,4], colors [V,4]).  Called without the interpreter lock.
+// `count` false: the caller can do without the number of list entries (Layout::K is then the room for them).
 ForwardOut forward(const Tensor& vertices_, const Tensor& indices_, const Tensor& colors_, const Tensor& opacities_,
-                   const View& v, bool record_timing, bool save_selection, bool cull, int64_t selection_max_bytes,
+                   const View& v, bool record_timing, bool save_selection, bool cull, int64_t selection_max_bytes, bool count,
                    const L2Step* step = nullptr) {
     const Tensor vertices = plain(vertices_), indices = plain(indices_), colors = plain(colors_);
     const bool packed = !opacities_.defined();
@@ -333,7 +348,10 @@ ForwardOut forward(const Tensor& vertices_, const Tensor& indices_, const Tensor
     const unsigned fixed_flags = (cull ? TG_FORWARD_CULL_TILES : 0u) | (packed ? TG_INPUT_PACKED : 0u) | TG_INFO_MAPPED;
     const auto state = state_of(w.device, w.stream);
     std::lock_guard<std::mutex> lock(state->use);
-    int64_t cap = std::max<int64_t>(state->k_estimate + state->k_estimate / 4 + 1024, 2 * (int64_t)T + 1024);
+    const bool no_count = state->no_count(T, v.tiles()) && !count && !record_timing && !step &&
+                          c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None;
+    int64_t cap = no_count ? (int64_t)T * v.tiles()
+                           : std::max<int64_t>(state->k_estimate + state->k_estimate / 4 + 1024, 2 * (int64_t)T + 1024);
     while (true) {
         s.ids = at::empty({cap}, options.dtype(at::kInt));
         size_t have = 0;
@@ -342,8 +360,8 @@ ForwardOut forward(const Tensor& vertices_, const Tensor& indices_, const Tensor
         const bool ready = std::equal(key, key + 4, state->ready);
         state->ready[0] = 0;                     // until this call has succeeded
         const unsigned flags = fixed_flags | (ready ? TG_WORKSPACE_READY : 0u) |
-                               (state->short_lists && !step ? TG_EXPECT_SHORT_LISTS : 0u);
-        const int slot = state->next_slot();
+                               (no_count ? TG_NO_COUNT : state->short_lists && !step ? TG_EXPECT_SHORT_LISTS : 0u);
+        const int slot = no_count ? DeviceState::kSlots : state->next_slot();
         int32_t* info = state->words(slot);
         float* ms = record_timing ? out.stage_ms.data() : nullptr;
         const double n = 4.0 * v.pixels();
@@ -358,6 +376,13 @@ ForwardOut forward(const Tensor& vertices_, const Tensor& indices_, const Tensor
                                     data<float>(opacities), T, v.W, v.H, v.tw, v.th, (float)v.thr, v.sort ? 1 : 0,
                                     v.layers, data<float>(out.image), data<float>(out.depthmap), s.final_w(), s.ends(),
                                     s.sel(), s.geo(), s.attr(), s.id_list(), (uint32_t)cap, s.offsets(), ws, have, (uint32_t*)info, ms, flags, w.stream);
+        if (no_count) {
+            check("render_forward", status);
+            std::copy(key, key + 4, state->ready);
+            state->check_error_word(state->last_slot);       // of an earlier call that counted; may yet arrive
+            s.l.K = cap;
+            return out;
+        }
         s.l.K = (uint32_t)info[0];
         if (status == TG_ERR_CAPACITY) {
             cap = s.l.K + s.l.K / 4 + 1024;              // what the call says it needs
@@ -522,7 +547,7 @@ ImageAndDepth render_graph(Kind kind, const Tensor& vertices, const Tensor& indi
         } else {
             // the corrected gradients walk the lists themselves and need no selection; nor does a render nobody differentiates
             ForwardOut f = forward(vertices, indices, colors, opacities, v, record_timing,
-                                   wants_grad && kind != Kind::kCorrected, cull_tiles, selection_max_bytes);
+                                   wants_grad && kind != Kind::kCorrected, cull_tiles, selection_max_bytes, false);
             r.image = std::move(f.image);
             r.depthmap = std::move(f.depthmap);
             r.stage_ms = std::move(f.stage_ms);
@@ -571,9 +596,9 @@ Tensor l2_step(const Tensor& vertices, const Tensor& indices, const Tensor& colo
         step.gO = packed ? nullptr : data<float>(to.opacities);
         step.scratch = scratch.data_ptr();
         step.scratch_bytes = (size_t)scratch.numel();
-        return forward(vertices, indices, colors, opacities, v, false, false, cull, 0, &step).image;
+        return forward(vertices, indices, colors, opacities, v, false, false, cull, 0, true, &step).image;
     }
-    const ForwardOut f = forward(vertices, indices, colors, opacities, v, false, true, cull, selection_max_bytes);
+    const ForwardOut f = forward(vertices, indices, colors, opacities, v, false, true, cull, selection_max_bytes, false);
     const Saved& s = f.saved;
     TORCH_CHECK_VALUE(s.selection.defined(), "the fused L2 backward needs per_pixel_sort=True and max_layers <= 32");
     auto backward_into = [&](const Tensor& sums) {
@@ -795,7 +820,7 @@ py::object py_forward(const Tensor& vertices, const Tensor& indices, const Tenso
     {
         py::gil_scoped_release nogil;
         at::AutoDispatchBelowADInplaceOrView below_autograd;
-        f = forward(vertices, indices, colors, or_none(opacities), v, timing, save_selection, cull, selection_max_bytes);
+        f = forward(vertices, indices, colors, or_none(opacities), v, timing, save_selection, cull, selection_max_bytes, true);
         const Saved& s = f.saved;
         const Layout& l = s.l;
         at::tracer::impl::NoTracerDispatchMode untraced;
