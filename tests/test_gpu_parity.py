@@ -304,7 +304,7 @@ def test_forward_and_backward_vs_oracle(pipeline, mode):
         assert err_max <= GRAD_TOL_MAX, f"grad_{name} ({path}): worst element {err_max:.3e}"
 
 
-@pytest.mark.parametrize("height", [1336, 1345, 1353, 1361])     # 167 strips of blocks: one pass; 169, 170, 171: three
+@pytest.mark.parametrize("height", [1336, 1345, 1353, 1361])     # 167 strips of 64 blocks: one pass; 169, 170, 171 of 128: three
 @pytest.mark.parametrize("depth_too", [False, True])
 def test_backward_in_several_passes_vs_oracle(height, depth_too):
     """Large images, whose CTAs take several blocks of pixels one after the other: strips that do not divide by the number of

@@ -1878,10 +1878,12 @@ static int backward_impl(const float* tri_geo, const float* tri_attr, const int3
         tg::BlendParams Q = P;
         Q.tiles_x = (W + tg::kQueueCols - 1) / tg::kQueueCols;
         Q.offsets = nullptr; Q.ids = nullptr; Q.order = nullptr;
-        // Three passes where they leave three waves of CTAs (eight per SM): 1280x720, 2.3 waves, 40 us in one pass, 42 in three.
+        // Three passes where they leave five waves of CTAs (seven or eight per SM): with a depth gradient 1280x720, 2.3 waves,
+        // 40 us in one pass, 42 in three; 669k triangles, 1382x1036, 3.6 waves, 193 and 202; inside a mesh, full HD, 5.2 waves, 86
+        // and 80.
         constexpr int kPasses = 3;
         const int strips = (H + tg::kQueueRows - 1) / tg::kQueueRows;
-        const bool many = (int64_t)Q.tiles_x * strips >= (int64_t)kPasses * 3 * 8 * 148;
+        const bool many = (int64_t)Q.tiles_x * strips >= (int64_t)kPasses * 5 * 7 * 148;
         const int blocks = Q.tiles_x * (many ? (strips + kPasses - 1) / kPasses : strips);
         auto kernel = many ? (grad_depthmap ? tg::blend_backward_queued_kernel<kPasses, true> : tg::blend_backward_queued_kernel<kPasses, false>)
                            : (grad_depthmap ? tg::blend_backward_queued_kernel<1, true> : tg::blend_backward_queued_kernel<1, false>);
