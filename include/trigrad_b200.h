@@ -376,6 +376,9 @@ int tg_project_clip_backward(const float* points, const int32_t* indices, const 
                              int T, const float* pv_host, const float* grad_out_vertices, const float* grad_out_colors,
                              const float* grad_out_opacities, float* grad_points, float* grad_colors,
                              float* grad_opacities, tg_stream_t stream);
+/* Zeroes grad_points [V,3], grad_colors [V,3] and grad_opacities [V] with one launch. */
+int tg_clear_gradients(float* grad_points, float* grad_colors, float* grad_opacities, int V, tg_stream_t stream);
+
 
 /* One view's packed accumulator (filled by the backward entry points with TG_ACCUMULATE_PACKED) straight to
  * world space: tg_unpack_gradients and tg_project_backward in one kernel.  The render-space vertex gradient

@@ -61,6 +61,7 @@ SIGNATURES = {
     "tg_project_backward": (_i, [_vp, _i, _vp, _vp, _vp, _i, _vp]),
     "tg_project_clip": (_i, [_vp, _vp, _vp, _vp, _i, _vp, _vp, _vp, _vp, _vp, _vp]),
     "tg_project_clip_backward": (_i, [_vp, _vp, _vp, _vp, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
+    "tg_clear_gradients": (_i, [_vp, _vp, _vp, _i, _vp]),
     "tg_unpack_project_backward": (_i, [_vp, _sz, _i, _vp, _vp, _f, _vp, _vp, _vp, _vp, _vp]),
     "tg_render_step_l2": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _i, _vp, _f, _f, _vp, _vp, _vp, _vp, _vp, _vp,
                                _vp, _vp, _u32, _vp, _vp, _vp, _vp, _i, _vp, _sz, _vp, _sz, _vp, _vp, C.c_uint, _vp]),

@@ -45,7 +45,7 @@ struct Api {
     F(last_error) F(status_string) F(selection_planes) F(forward_workspace_bytes) F(render_forward)                  \
     F(render_step_l2) F(backward_scratch_bytes) F(blend_backward) F(blend_backward_corrected) F(blend_backward_l2)   \
     F(blend_backward_l2_u8) F(unpack_gradients) F(unpack_gradients_rgba) F(project) F(project_backward)              \
-    F(project_clip) F(project_clip_backward) F(unpack_project_backward) F(pack_inputs)
+    F(project_clip) F(project_clip_backward) F(clear_gradients) F(unpack_project_backward) F(pack_inputs)
     TG_FUNCTIONS(TG_FN)
 #undef TG_FN
 };
@@ -685,7 +685,9 @@ std::vector<Tensor> project_clip_backward(const Tensor& points, const Tensor& in
     const auto options = p.options().requires_grad(false);
     auto upstream = [&](const Tensor& t, at::IntArrayRef shape) { return t.defined() ? plain(t) : at::zeros(shape, options); };
     const Tensor gv = upstream(grad_vertices, {6 * T, 4}), gc = upstream(grad_colors, {6 * T, 3}), go = upstream(grad_opacities, {6 * T});
-    std::vector<Tensor> out = {at::zeros_like(p), at::zeros_like(c), at::zeros_like(o)};
+    std::vector<Tensor> out = {at::empty_like(p), at::empty_like(c), at::empty_like(o)};
+    check("clear_gradients", g.clear_gradients(data<float>(out[0]), data<float>(out[1]), data<float>(out[2]), need_int(p.size(0)),
+                                               w.stream));
     check("project_clip_backward",
           g.project_clip_backward(data<float>(p), data<int32_t>(i), data<float>(c), data<float>(o), need_int(T), pv.m,
                                   data<float>(gv), data<float>(gc), data<float>(go), data<float>(out[0]),
