@@ -10,6 +10,7 @@
 #include <dlfcn.h>
 
 #include <algorithm>
+#include <atomic>
 #include <list>
 #include <memory>
 #include <mutex>
@@ -141,7 +142,7 @@ T* data(const Tensor& t) { return t.defined() ? static_cast<T*>(t.data_ptr()) : 
 struct DeviceState {
     static constexpr int kSlots = 256;
     std::mutex use;
-    Tensor workspace, info;      // info [slots + 1,4] int32 pinned: K, longest list, error word, slots; last row: see no_count
+    Tensor workspace, info;      // info [slots,4] int32 pinned: K, longest list, error word, slots
     int slot = 0, last_slot = -1;
     int64_t k_estimate = 0;
     bool short_lists = false;          // the last forward had no tile list beyond TG_SHORT_LIST entries
@@ -155,7 +156,7 @@ struct DeviceState {
 
     explicit DeviceState(at::Device device) {
         workspace = at::empty({0}, at::TensorOptions().dtype(at::kByte).device(device));
-        info = at::zeros({kSlots + 1, 4}, at::TensorOptions().dtype(at::kInt)).pin_memory();
+        info = at::zeros({kSlots, 4}, at::TensorOptions().dtype(at::kInt)).pin_memory();
     }
     int32_t* words(int s) { return info.data_ptr<int32_t>() + 4 * s; }
     int next_slot() {
@@ -175,13 +176,22 @@ struct DeviceState {
                                  " (a bounded wait ran out inside a kernel); its outputs are not valid");
     }
     // Whether a call can do without the number of entries on the host (TG_NO_COUNT): the lists were short when last looked at
-    // (the kernels of calls that did not wait say so, in the row that is theirs alone, as soon as they no longer are), and
-    // the room for every pair of triangle and tile is small.  28 bytes each, so 14 MB.  The wait was the length of the binning
-    // and a trip over PCIe in every small call (B200: ten squares, 50x50, forward and backward 99 -> 84 us; 1280 triangles,
-    // 256x256, forward 25.3 -> 19.9, with a loss and backward 171 -> 161).
+    // (the kernels of calls that did not wait say so, in `long_row`, as soon as they no longer are), and the room for every
+    // pair of triangle and tile is small.  28 bytes each, so 14 MB.  The wait was the length of the binning and a trip over
+    // PCIe in every small call (B200: ten squares, 50x50, forward and backward 99 -> 84 us; 1280 triangles, 256x256, forward
+    // 25.3 -> 19.9, with a loss and backward 171 -> 161).
+    // Such a kernel may write its word after the state is gone, so the rows are nobody's to free: a fixed table, whose rows
+    // states that come and go share.  A word that another state's kernel wrote costs a call that waits.
+    int32_t* const long_row = next_long_row();
+    static int32_t* next_long_row() {
+        constexpr int kRows = 2 * 128;
+        static Tensor& table = *new Tensor(at::zeros({kRows, 4}, at::TensorOptions().dtype(at::kInt)).pin_memory());
+        static std::atomic<unsigned> next{0};
+        return table.data_ptr<int32_t>() + 4 * (next++ % kRows);
+    }
     static constexpr int64_t kNoCountPairs = int64_t(1) << 19;
     bool no_count(int64_t T, int64_t tiles) {
-        volatile int32_t* longest = words(kSlots) + 1;
+        volatile int32_t* longest = long_row + 1;
         if (*longest) {
             *longest = 0;
             short_lists = false;
@@ -363,8 +373,8 @@ ForwardOut forward(const Tensor& vertices_, const Tensor& indices_, const Tensor
         state->ready[0] = 0;                     // until this call has succeeded
         const unsigned flags = fixed_flags | (ready ? TG_WORKSPACE_READY : 0u) |
                                (no_count ? TG_NO_COUNT : state->short_lists && !step ? TG_EXPECT_SHORT_LISTS : 0u);
-        const int slot = no_count ? DeviceState::kSlots : state->next_slot();
-        int32_t* info = state->words(slot);
+        const int slot = no_count ? -1 : state->next_slot();
+        int32_t* info = no_count ? state->long_row : state->words(slot);
         float* ms = record_timing ? out.stage_ms.data() : nullptr;
         const double n = 4.0 * v.pixels();
         const int status =
