@@ -313,7 +313,8 @@ int tg_blend_step_l2(const float* tri_geo, const float* tri_attr, const int32_t*
  *                no matter: T <= TG_NO_COUNT_TRIANGLES, list_capacity >= T * tiles, at most 1184 tiles, TG_INFO_MAPPED, no
  *                stage_ms_host, and not while the stream is being captured (otherwise TG_ERR_BAD_ARG).  info_host is not
  *                waited for and receives nothing but, in [1], the length of the longest list where that is beyond
- *                TG_SHORT_LIST, whenever the binning gets there: such lists are sorted slowly, so a caller that finds it
+ *                TG_SHORT_LIST, whenever the binning gets there: such lists are sorted inside the compositing kernel and not
+ *                filtered there (lists of 3300 entries: 100 to 200 us more than without the flag), so a caller that finds it
  *                had better do without the flag for a while.  Results do not depend on it.
  */
 #define TG_NO_COUNT 32u

@@ -202,3 +202,38 @@ def test_not_counting_is_refused_where_it_is_not_safe(triangles, capacity, flags
                                    ptr(depth), ptr(fw), ptr(ends), ptr(sel), ptr(geo), ptr(attr), ptr(ids), capacity, ptr(off),
                                    ctypes.c_void_p((ws.data_ptr() + 255) // 256 * 256), size, ptr(info), None, flags, ctypes.c_void_p(0))
     assert status == 1
+
+
+def _stacked(n, w, h, seed):
+    """n triangles over the whole image, at few depths, so that order is the triangles' in part."""
+    rng = np.random.default_rng(seed)
+    xy = np.array([[-3, -3], [3, -3], [0, 5]], np.float32) + rng.normal(size=(n, 1, 2)).astype(np.float32) * 0.01
+    z = rng.integers(2, 9, size=(n, 1, 1)).astype(np.float32).repeat(3, axis=1)
+    v = np.concatenate([xy, z, 1 / z], axis=2).reshape(3 * n, 4)
+    c = rng.random((3 * n, 3), dtype=np.float32)
+    o = np.full(3 * n, min(0.5, 20 / n), np.float32)
+    return [Hh.cuda(np.ascontiguousarray(x)) for x in (v, np.arange(3 * n, dtype=np.int32).reshape(n, 3), c, o)]
+
+
+@pytest.mark.parametrize("n", [129, 1023, 1024, 1025, 2049, 4096])
+@pytest.mark.parametrize("tile", [16, 8, 32])
+@pytest.mark.parametrize("sort", [True, False])
+def test_long_lists_of_a_call_that_does_not_count(n, tile, sort):
+    """The order of a list at the edges of the chunks it is sorted in, all of it seen in tile order, the first layers otherwise."""
+    from trigrad_b200 import _native as N
+
+    w, h = 20, 13
+    few, many = _stacked(20, w, h, 1), _stacked(n, w, h, n)
+    options = dict(tile_width=tile, tile_height=tile, early_stopping_threshold=0.0, per_pixel_sort=sort, max_layers=32 if sort else 0)
+    with torch.cuda.stream(torch.cuda.Stream()), torch.no_grad():
+        state = N.host().state(0, torch.cuda.current_stream().cuda_stream)
+        for _ in range(65):                                   # the stream may have met long lists before
+            trigrad_b200.render(*few, w, h, **options)
+        before = state.last_slot
+        got = trigrad_b200.render(*many, w, h, **options)
+        assert state.last_slot == before                      # went without the count
+        want = trigrad_b200.render(*many, w, h, record_timing=True, **options)
+        assert state.last_slot != before
+        torch.cuda.current_stream().synchronize()
+    for a, b in zip(got, want):
+        assert torch.equal(a.view(torch.int32), b.view(torch.int32))

@@ -153,7 +153,7 @@ int sort_long_lists(uint64_t* entries, const int32_t* offsets, int tiles, int32_
                     uint32_t longest, cudaStream_t stream);
 // Forward compositing with the sort of the tile lists (at most kFusedList entries each, `info` as the binning left it) in the
 // same kernel, which does nothing when the slots exceed `capacity` or a list is longer; with `any_length` it sorts longer
-// ones too, slowly.
+// ones too (sort_words), and does not filter them.
 int blend_forward_short(const float* tri_geo, const float* tri_attr, const BinBuffers& b, uint32_t capacity, bool any_length,
                         int32_t* sorted_ids, const int32_t* offsets, int W, int H, int tw, int th, float thr,
                         int per_pixel_sort, int max_layers, float* image, float* depthmap, float* final_weights,
