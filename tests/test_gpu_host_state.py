@@ -237,3 +237,30 @@ def test_long_lists_of_a_call_that_does_not_count(n, tile, sort):
         torch.cuda.current_stream().synchronize()
     for a, b in zip(got, want):
         assert torch.equal(a.view(torch.int32), b.view(torch.int32))
+
+
+def test_lists_that_change_between_short_and_long():
+    """Calls that meet a long list without having counted get rarer, whatever the pattern; where lists stay short, no call counts."""
+    from trigrad_b200 import _native as N
+
+    w, h = 64, 64
+    few, many = _stacked(20, w, h, 1), _stacked(300, w, h, 2)
+    with torch.cuda.stream(torch.cuda.Stream()), torch.no_grad():
+        state = N.host().state(0, torch.cuda.current_stream().cuda_stream)
+
+        def counts(mesh):
+            before = state.last_slot
+            trigrad_b200.render(*mesh, w, h)
+            torch.cuda.current_stream().synchronize()
+            return state.last_slot != before
+
+        for short in (1, 2, 5, 16):
+            uncounted = 0
+            for _ in range(40):
+                for _ in range(short):
+                    counts(few)
+                uncounted += not counts(many)
+            assert uncounted <= 3
+        for _ in range(64):
+            counts(few)
+        assert not any(counts(few) for _ in range(300))

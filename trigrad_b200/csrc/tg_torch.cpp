@@ -175,13 +175,18 @@ struct DeviceState {
         throw std::runtime_error("trigrad_b200: an earlier render reported device error word " + std::to_string(stale) +
                                  " (a bounded wait ran out inside a kernel); its outputs are not valid");
     }
-    // Whether a call can do without the number of entries on the host (TG_NO_COUNT): the lists were short when last looked at
-    // (the kernels of calls that did not wait say so, in `long_row`, as soon as they no longer are), and the room for every
-    // pair of triangle and tile is small.  28 bytes each, so 14 MB.  The wait was the length of the binning and a trip over
-    // PCIe in every small call (B200: ten squares, 50x50, forward and backward 99 -> 84 us; 1280 triangles, 256x256, forward
-    // 25.3 -> 19.9, with a loss and backward 171 -> 161).
+    // Whether a call can do without the number of entries on the host (TG_NO_COUNT): the lists of the last few calls that counted
+    // were short, no kernel of a call that did not has said otherwise since (in `long_row`), and the room for every pair of
+    // triangle and tile is small.  28 bytes each, so 14 MB.  The wait was the length of the binning and a trip over PCIe in
+    // every small call (B200: ten squares, 50x50, forward and backward 99 -> 84 us; 1280 triangles, 256x256, forward 25.3 ->
+    // 19.9, with a loss and backward 171 -> 161).
+    // "The last few": one at first, twice as many (up to kCountedMax) each time a call that did not count met a long list, which
+    // costs it 100 to 200 us where lists have 3300 entries (see sort_words in tg_blend.cu).  So a program whose lists change
+    // between short and long pays that a few times and not at every change, and one that has long lists now and then keeps most
+    // of the gain (short and such lists in turn, 160x160: 538 us a call when one short call was enough, 108 now, 110 with every
+    // call waiting).
     // Such a kernel may write its word after the state is gone, so the rows are nobody's to free: a fixed table, whose rows
-    // states that come and go share.  A word that another state's kernel wrote costs a call that waits.
+    // states that come and go share.  A word that another state's kernel wrote costs a few calls that wait.
     int32_t* const long_row = next_long_row();
     static int32_t* next_long_row() {
         constexpr int kRows = 2 * 128;
@@ -190,13 +195,21 @@ struct DeviceState {
         return table.data_ptr<int32_t>() + 4 * (next++ % kRows);
     }
     static constexpr int64_t kNoCountPairs = int64_t(1) << 19;
+    static constexpr int kCountedMax = 64;
+    int counted_short = 0, counted_needed = 1;
     bool no_count(int64_t T, int64_t tiles) {
         volatile int32_t* longest = long_row + 1;
         if (*longest) {
             *longest = 0;
             short_lists = false;
+            counted_short = 0;
+            counted_needed = std::min(2 * counted_needed, kCountedMax);
         }
-        return short_lists && T <= TG_NO_COUNT_TRIANGLES && T * tiles <= kNoCountPairs && tiles <= kNoCountTiles;
+        return counted_short >= counted_needed && T <= TG_NO_COUNT_TRIANGLES && T * tiles <= kNoCountPairs && tiles <= kNoCountTiles;
+    }
+    void counted(bool all_short) {
+        short_lists = all_short;
+        counted_short = all_short ? std::min(counted_short + 1, kCountedMax) : 0;
     }
     static constexpr int64_t kNoCountTiles = 1184;
     // After a forward call that used slot `s` has returned: it waited for work recorded after the previous call's on
@@ -402,7 +415,7 @@ ForwardOut forward(const Tensor& vertices_, const Tensor& indices_, const Tensor
         }
         check(step ? "render_step_l2" : "render_forward", status);
         std::copy(key, key + 4, state->ready);
-        state->short_lists = (uint32_t)info[1] <= TG_SHORT_LIST;
+        state->counted((uint32_t)info[1] <= TG_SHORT_LIST);
         state->finish_call(slot);
         state->k_estimate = std::max<int64_t>(s.l.K, (uint32_t)info[3]);
         return out;
