@@ -103,3 +103,56 @@ def test_second_backward_of_a_mesh_without_triangles(call):
             assert g.shape == x.shape and not bool(g.any())
     with pytest.raises(RuntimeError, match="second time"):
         torch.autograd.grad(out[0].sum(), leaves)
+
+
+@pytest.mark.parametrize("call", list(CALLS))
+def test_lists_are_kept_only_for_a_backward_that_reads_them(call):
+    i, leaves = _leaves(call == "packed")
+    sizes = []
+
+    def pack(t):
+        sizes.append(t.numel() * t.element_size())
+        return t
+
+    with torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t):
+        CALLS[call](i, leaves)
+    blob = 8 * W * H + 160 * i.shape[0] + 4 * (13 * 8 + 1) + 5 * 256
+    selection = 4 * 32 * W * H if call in ("render", "packed", "Renderer") else 0
+    lists = sum(sizes) - 20 * W * H - selection
+    if selection:
+        assert lists <= blob                  # nothing but final weights, ends, records and offsets
+    else:
+        assert lists >= 8 * W * H + 160 * i.shape[0] + 4 * i.shape[0]
+
+
+@pytest.mark.parametrize("triangles, width, height, tile", [(20, 50, 50, 4), (1280, 256, 256, 16), (4000, 120, 100, 16), (300, 40, 40, 2)])
+@pytest.mark.parametrize("call", ["render", "tile_order", "corrected"])
+def test_small_renders_keep_little_more_than_image_records_and_selection(call, triangles, width, height, tile):
+    """A hundred live graphs of calls that may go without the number of list entries, whose lists have room for every pair."""
+    sc = S.random_triangles(triangles, width, height, 0.05, 0.4, name="live", seed=4)
+    v, i, c, o = Hh.scene_tensors(sc)
+    leaves = [x.requires_grad_() for x in (v, c, o)]
+    options = dict(tile_order=dict(per_pixel_sort=False), corrected={}, render={})[call]
+    function = trigrad_b200.render_corrected if call == "corrected" else trigrad_b200.render
+    render = lambda: function(leaves[0], i, leaves[1], leaves[2], width, height, tile, tile, **options)
+    with torch.cuda.stream(torch.cuda.Stream()):
+        for _ in range(70):
+            torch.autograd.grad(render()[0].sum(), leaves)
+        torch.cuda.current_stream().synchronize()
+        before = torch.cuda.memory_allocated()
+        live = [render() for _ in range(100)]
+        kept = (torch.cuda.memory_allocated() - before) / len(live)
+    tiles = -(-width // tile) * -(-height // tile)
+    px = width * height
+    rest = 28 * px + 160 * triangles + 4 * (tiles + 1) + 5 * 256
+    # the lists: none, up to a quarter of the rest, or what a call that counts has room for
+    lists = 0 if call == "render" else max(rest // 4, 4 * max(2 * triangles, 5 * int(_entries(v, i, c, o, width, height, tile)) // 4) + 4096)
+    selection = 4 * 32 * px if call == "render" else 0
+    # blocks are rounded up to 512 bytes; of the 20 MB segments that blocks above 1 MB come from, less than 1 MB is given away unsplit
+    unsplit = (1 << 20) / ((20 << 20) // selection) if selection > 1 << 20 else 0
+    assert kept <= rest + selection + lists + 5 * 512 + unsplit
+
+
+def _entries(v, i, c, o, width, height, tile):
+    out = trigrad_b200.wrapper.forward_native(v.detach(), i, c.detach(), o.detach(), width, height, tile, tile, 1 / 256, False, True, 32)
+    return out[3].numel()

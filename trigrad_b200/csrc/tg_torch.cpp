@@ -297,8 +297,8 @@ struct View {       // the arguments of a render that are not tensors
     int64_t pixels() const { return (int64_t)W * H; }
 };
 
-// What a forward leaves for its backward: sizes and places (`Layout`), and three tensors - final weights, ends, records
-// and tile offsets in one allocation (`blob`), the lists, and the selection.  Between the passes the tensors belong to
+// What a forward leaves for its backward: sizes and places (`Layout`), and two tensors - final weights, ends, records
+// and tile offsets in one allocation (`blob`), and the selection, or the lists where there is none.  Between the passes they belong to
 // autograd (SavedVariable, ctx.save_for_backward), which may move them; so places are offsets, never addresses.
 struct Layout {
     View v;
@@ -346,9 +346,10 @@ struct L2Step {     // forward, loss and gradients in one call (tg_render_step_l
 };
 
 // `opacities` undefined: packed inputs (indices [T,4], colors [V,4]).  Called without the interpreter lock.
-// `count` false: the caller can do without the number of list entries (Layout::K is then the room for them).
+// `count`: whether the caller needs the number of list entries (otherwise Layout::K may be the room for them).
+enum class Count { kAlways, kUnlessSmall, kUnlessSmallKeepLists };      // the last one: and may keep the lists for a backward
 ForwardOut forward(const Tensor& vertices_, const Tensor& indices_, const Tensor& colors_, const Tensor& opacities_,
-                   const View& v, bool record_timing, bool save_selection, bool cull, int64_t selection_max_bytes, bool count,
+                   const View& v, bool record_timing, bool save_selection, bool cull, int64_t selection_max_bytes, Count count,
                    const L2Step* step = nullptr) {
     const Tensor vertices = plain(vertices_), indices = plain(indices_), colors = plain(colors_);
     const bool packed = !opacities_.defined();
@@ -373,7 +374,12 @@ ForwardOut forward(const Tensor& vertices_, const Tensor& indices_, const Tensor
     const unsigned fixed_flags = (cull ? TG_FORWARD_CULL_TILES : 0u) | (packed ? TG_INPUT_PACKED : 0u) | TG_INFO_MAPPED;
     const auto state = state_of(w.device, w.stream);
     std::lock_guard<std::mutex> lock(state->use);
-    const bool no_count = state->no_count(T, v.tiles()) && !count && !record_timing && !step &&
+    // Without the count the lists have room for every pair, however few there are.  Where they are kept for a backward that is
+    // let be up to a quarter of what the graph keeps anyway (image, depth map, blob); beyond it the call counts, as keeping the
+    // lists of 1280 triangles at 256x256, 1.3 MB instead of 15 KB, added 60 % to every live graph.
+    const bool lists_small = count != Count::kUnlessSmallKeepLists || s.selection.defined() ||
+                             16 * (int64_t)T * v.tiles() <= 20 * v.pixels() + (int64_t)s.l.bytes;
+    const bool no_count = state->no_count(T, v.tiles()) && count != Count::kAlways && lists_small && !record_timing && !step &&
                           c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None;
     int64_t cap = no_count ? (int64_t)T * v.tiles()
                            : std::max<int64_t>(state->k_estimate + state->k_estimate / 4 + 1024, 2 * (int64_t)T + 1024);
@@ -498,7 +504,7 @@ Kept kept_all(const Layout& l, const Tensor& image, const Tensor& depthmap, cons
     const int64_t px = l.v.pixels();
     const at::Device d = image.device();
     return {kept(image, d, at::kFloat, 4 * px), kept(depthmap, d, at::kFloat, px),
-            {l, kept(blob, d, at::kByte, (int64_t)l.bytes), kept(ids, d, at::kInt, l.K, true),
+            {l, kept(blob, d, at::kByte, (int64_t)l.bytes), l.planes > 0 ? Tensor() : kept(ids, d, at::kInt, l.K, true),
              l.planes > 0 ? kept(selection, d, at::kInt, l.planes * px) : Tensor()}};
 }
 
@@ -506,7 +512,7 @@ struct RenderBackward : public Node {
     Kind kind = Kind::kReference;
     Layout layout;
     SavedVariable image, depthmap;           // outputs of this node
-    SavedVariable blob, ids, selection;
+    SavedVariable blob, ids, selection;      // the lists or the selection
     struct Shape { at::DimVector sizes; at::TensorOptions options; };
     std::vector<Shape> zeros;                // mesh without triangles: nothing saved, the gradients' shapes
     bool released = false;
@@ -572,7 +578,8 @@ ImageAndDepth render_graph(Kind kind, const Tensor& vertices, const Tensor& indi
         } else {
             // the corrected gradients walk the lists themselves and need no selection; nor does a render nobody differentiates
             ForwardOut f = forward(vertices, indices, colors, opacities, v, record_timing,
-                                   wants_grad && kind != Kind::kCorrected, cull_tiles, selection_max_bytes, false);
+                                   wants_grad && kind != Kind::kCorrected, cull_tiles, selection_max_bytes,
+                                   wants_grad ? Count::kUnlessSmallKeepLists : Count::kUnlessSmall);
             r.image = std::move(f.image);
             r.depthmap = std::move(f.depthmap);
             r.stage_ms = std::move(f.stage_ms);
@@ -587,8 +594,8 @@ ImageAndDepth render_graph(Kind kind, const Tensor& vertices, const Tensor& indi
             node->image = SavedVariable(r.image, /*is_output=*/true);
             node->depthmap = SavedVariable(r.depthmap, /*is_output=*/true);
             node->blob = SavedVariable(saved.blob, false);
-            node->ids = SavedVariable(saved.ids, false);
             if (saved.selection.defined()) node->selection = SavedVariable(saved.selection, false);
+            else node->ids = SavedVariable(saved.ids, false);
         }
     }
     return r;
@@ -621,9 +628,9 @@ Tensor l2_step(const Tensor& vertices, const Tensor& indices, const Tensor& colo
         step.gO = packed ? nullptr : data<float>(to.opacities);
         step.scratch = scratch.data_ptr();
         step.scratch_bytes = (size_t)scratch.numel();
-        return forward(vertices, indices, colors, opacities, v, false, false, cull, 0, true, &step).image;
+        return forward(vertices, indices, colors, opacities, v, false, false, cull, 0, Count::kAlways, &step).image;
     }
-    const ForwardOut f = forward(vertices, indices, colors, opacities, v, false, true, cull, selection_max_bytes, false);
+    const ForwardOut f = forward(vertices, indices, colors, opacities, v, false, true, cull, selection_max_bytes, Count::kUnlessSmall);
     const Saved& s = f.saved;
     TORCH_CHECK_VALUE(s.selection.defined(), "the fused L2 backward needs per_pixel_sort=True and max_layers <= 32");
     auto backward_into = [&](const Tensor& sums) {
@@ -847,7 +854,7 @@ py::object py_forward(const Tensor& vertices, const Tensor& indices, const Tenso
     {
         py::gil_scoped_release nogil;
         at::AutoDispatchBelowADInplaceOrView below_autograd;
-        f = forward(vertices, indices, colors, or_none(opacities), v, timing, save_selection, cull, selection_max_bytes, true);
+        f = forward(vertices, indices, colors, or_none(opacities), v, timing, save_selection, cull, selection_max_bytes, Count::kAlways);
         const Saved& s = f.saved;
         const Layout& l = s.l;
         at::tracer::impl::NoTracerDispatchMode untraced;
@@ -863,14 +870,14 @@ py::object py_forward(const Tensor& vertices, const Tensor& indices, const Tenso
                           timing ? py::cast(f.stage_ms) : py::object(py::none()), f.saved.l, f.saved.blob);
 }
 
-// `blob`, `ids` and `selection` as forward returned them with `layout`.
-py::list py_backward(int kind, const Layout& layout, const Tensor& image, const Tensor& depthmap, const Tensor& blob, const Tensor& ids,
-                     const Optional& selection, const Optional& gi, const Optional& gd) {
+// `blob`, `ids` and `selection` as forward returned them with `layout`; the lists are not looked at when there is a selection.
+py::list py_backward(int kind, const Layout& layout, const Tensor& image, const Tensor& depthmap, const Tensor& blob,
+                     const Optional& ids, const Optional& selection, const Optional& gi, const Optional& gd) {
     std::vector<Tensor> out;
     {
         py::gil_scoped_release nogil;
         at::AutoDispatchBelowADInplaceOrView below_autograd;
-        const Kept k = kept_all(layout, image, depthmap, blob, ids, or_none(selection));
+        const Kept k = kept_all(layout, image, depthmap, blob, or_none(ids), or_none(selection));
         at::tracer::impl::NoTracerDispatchMode untraced;
         out = backward((Kind)kind, k.saved, k.image, k.depthmap, or_none(gi), or_none(gd));
     }

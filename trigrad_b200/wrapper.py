@@ -113,7 +113,8 @@ class RendererOfKind(Function):
                                    kind != GRADIENTS_CORRECTED,
                                    (kind == GRADIENTS_CORRECTED or bool(per_pixel_sort)) and CULL_TILES, SELECTION_MAX_BYTES)
             image, depthmap, timings, ctx.layout = out[0], out[1], _timings(out[9]), out[10]
-            ctx.save_for_backward(image, depthmap, out[11], out[3], out[8])      # image, depth map, blob, lists, selection
+            # image, depth map, blob, and the selection or, where there is none, the lists
+            ctx.save_for_backward(image, depthmap, out[11], None if out[8] is not None else out[3], out[8])
         if record_timing:
             return image, depthmap, timings
         return image, depthmap
