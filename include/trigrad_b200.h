@@ -222,7 +222,7 @@ int tg_blend_backward_l2_u8(const float* tri_geo, const float* tri_attr, const i
 /* ---- gradients of several views in one packed accumulator ------------------------------------------
  * With accumulate = TG_ACCUMULATE_PACKED the backward entry points (tg_blend_backward, tg_blend_backward_l2,
  * tg_blend_step_l2, tg_render_step_l2) neither clear `scratch` nor write the three gradient tensors
- * (which may then be NULL, like loss_out): the packed per-vertex sums and the loss partials stay in
+ * (which may then be NULL, like loss_out): the packed per-vertex sums and the sums of the loss stay in
  * `scratch` and keep growing call after call - also from calls on several streams, the additions are
  * atomic.  The caller clears the tg_backward_scratch_bytes(V) bytes once (cudaMemsetAsync), runs the
  * views, orders the streams, and calls tg_unpack_gradients once: grad_* = (accumulate ? grad_* : 0) +
@@ -385,7 +385,7 @@ int tg_clear_gradients(float* grad_points, float* grad_colors, float* grad_opaci
  * world space: tg_unpack_gradients and tg_project_backward in one kernel.  The render-space vertex gradient
  * of every vertex goes through the VJP of tg_project (same points, same pv_host) and is ADDED to
  * grad_points [V,3]; colour and opacity gradients are ADDED to grad_colors [V,3] / grad_opacities [V]; the
- * view's loss (sum of its partials * loss_scale) is ADDED to *loss_out (may be NULL).  All additions are
+ * view's loss (its sums * loss_scale) is ADDED to *loss_out (may be NULL).  All additions are
  * atomic, so views rendered on several streams may add into the same tensors; the caller clears them once
  * per batch.  The accumulator is zero again when the kernel ends: clear it once
  * (tg_backward_scratch_bytes(V) bytes) before the first view and reuse it, one accumulator per stream.

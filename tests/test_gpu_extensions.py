@@ -256,3 +256,28 @@ def test_obj_mesh_renders_like_the_oracle():
     of = O.forward(verts.cpu().numpy(), faces, col, op, 256, 192)
     assert np.array_equal(image.cpu().numpy().view(np.uint32), of.image.view(np.uint32))
     assert int(of.ends.max()) == 2          # front and back face
+
+
+@pytest.mark.parametrize("width, height", [(7, 3), (200, 120), (1600, 990), (2048, 977)])     # one block; one pass; 12400 blocks: one; 15744: three
+@pytest.mark.parametrize("one_kernel", [False, True])
+def test_loss_of_a_step_vs_64_bits(width, height, one_kernel):
+    """The squared differences of many warps in a few sums, taken and cleared by each of three calls on one stream, through the
+    accumulator that the stream keeps and through one of the caller's."""
+    sc = S.random_triangles(3000, width, height, 0.1, 0.5, name="loss", seed=width)
+    v, i, c, o = Hh.scene_tensors(sc)
+    target = torch.rand((height, width, 4), device="cuda", generator=torch.Generator("cuda").manual_seed(3))
+    # additions of positive numbers, one rounding each: four squares, five shuffles, warps / 256 atomics, the total, the scale
+    bound = (width * height / 32 / 256 + 32) * 2.0 ** -23
+    points = v[:, :3].contiguous()
+    pv = torch.eye(4)
+    packed = views.PackedGradients(v.shape[0], "cuda")
+    for _ in range(3):
+        b = views.GradBuffer.allocate(v.shape[0], "cuda", 4)
+        image = views.l2_view_step(v, i, c, o, target, width, height, b.points, b.colors, b.opacities, b.loss, one_kernel=one_kernel)
+        want = float(torch.mean((image.double() - target.double()) ** 2))
+        assert abs(float(b.loss) - want) <= bound * want
+        b = views.GradBuffer.allocate(v.shape[0], "cuda", 3)
+        image = views.l2_world_view_step(points, pv, i, c, o, target, width, height, b.points, b.colors, b.opacities, b.loss,
+                                         one_kernel=one_kernel, packed=packed)
+        want = float(torch.mean((image.double() - target.double()) ** 2))
+        assert abs(float(b.loss) - want) <= bound * want

@@ -956,15 +956,14 @@ struct BackwardIn {
     const int* ends;
     // fused mean-squared-error loss: when l2_target is set, the upstream gradient of the image is
     // l2_grad_scale * (image - target), the depth-map gradient is zero and the squared differences are
-    // summed into l2_partials[64] (no gradient image is ever materialised)
+    // summed into l2_sums (add_loss; no gradient image is ever materialised)
     const float4* l2_target;
     float l2_grad_scale;
-    float* l2_partials;
+    float* l2_sums;
     // the same target as 8-bit RGBA (value / 255, correctly rounded division: what `u8.float() / 255` gives);
     // at most one of l2_target / l2_target_u8 is set
     const uchar4* l2_target_u8;
 };
-constexpr int kLossPartials = 64;
 
 // DEPTH = false: no gradient flows into the depth map, so neither it nor the final weight is read.
 template <bool DEPTH = true>
@@ -1374,10 +1373,10 @@ __global__ void __launch_bounds__(kQueueCols * kQueueRows, DEPTH ? 7 : 8) blend_
     }
     if (queued > 0) drain_queue<DEPTH>(P, q, 0, queued, gpack);
     if (in.l2_target || in.l2_target_u8) {
-        // loss: warp sum, then one atomic per warp into one of 64 partial sums (spread addresses)
+        // loss: warp sum, then one atomic per warp
 #pragma unroll
         for (int d = 16; d > 0; d >>= 1) sq_sum += __shfl_xor_sync(0xffffffffu, sq_sum, d);
-        if (lane == 0 && sq_sum != 0.f) atomicAdd(in.l2_partials + ((blockIdx.x * kWarps + warp) & (kLossPartials - 1)), sq_sum);
+        if (lane == 0 && sq_sum != 0.f) add_loss(in.l2_sums, blockIdx.x * kWarps + warp, sq_sum);
     }
 }
 
@@ -1396,7 +1395,7 @@ template <int MAXT>
 __global__ void __launch_bounds__(MAXT, 4) blend_step_l2_kernel(BlendParams P, float4* __restrict__ image,
                                                                 float* __restrict__ depthmap, float* __restrict__ final_w,
                                                                 int* __restrict__ ends, const float4* __restrict__ target,
-                                                                float grad_scale, float* __restrict__ l2_partials,
+                                                                float grad_scale, float* __restrict__ l2_sums,
                                                                 float4* __restrict__ gpack) {
     static_assert(MAXT == 256, "the per-warp queues are sized for 8 warps");
     __shared__ float4 s_geo[kChunk * kStagedQuads];
@@ -1454,7 +1453,7 @@ __global__ void __launch_bounds__(MAXT, 4) blend_step_l2_kernel(BlendParams P, f
     }
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, d);
-    if (lane == 0 && sq != 0.f) atomicAdd(l2_partials + ((blockIdx.x * 8 + (threadIdx.x >> 5)) & (kLossPartials - 1)), sq);
+    if (lane == 0 && sq != 0.f) add_loss(l2_sums, blockIdx.x * 8 + (threadIdx.x >> 5), sq);
 
     float4* q = s_step + kQueueQuads * (threadIdx.x >> 5);
     const int nmax = __reduce_max_sync(0xffffffffu, n);
@@ -1725,15 +1724,9 @@ __device__ __forceinline__ bool take_vertex(float4* gpack, int v, bool clear, fl
     }
     return any;
 }
-__device__ __forceinline__ void unpack_loss(float* partials, float scale, float* loss_out, bool accumulate, bool clear) {
+__device__ __forceinline__ void unpack_loss(float* sums, float scale, float* loss_out, bool accumulate, bool clear) {
     if (blockIdx.x != 0 || threadIdx.x >= 32 || (!loss_out && !clear)) return;
-    float x = partials[threadIdx.x] + partials[threadIdx.x + 32];
-    if (clear) {
-        partials[threadIdx.x] = 0.f;
-        partials[threadIdx.x + 32] = 0.f;
-    }
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) x += __shfl_xor_sync(0xffffffffu, x, d);
+    const float x = take_loss(sums, clear);
     if (threadIdx.x == 0 && loss_out) *loss_out = (accumulate ? *loss_out : 0.f) + x * scale;
 }
 
@@ -1741,11 +1734,11 @@ __device__ __forceinline__ void unpack_loss(float* partials, float scale, float*
 // vertex, and 32 written or, adding to the tensors, touched only for vertices that received something.
 __global__ void __launch_bounds__(256) unpack_gradients_kernel(float4* __restrict__ gpack, int V, float4* __restrict__ gV,
                                                                float* __restrict__ gC, float* __restrict__ gO, int accumulate,
-                                                               int clear, float* __restrict__ l2_partials,
+                                                               int clear, float* __restrict__ l2_sums,
                                                                float l2_loss_scale, float* __restrict__ l2_loss_out) {
     allow_dependents();
     await_prerequisites();
-    unpack_loss(l2_partials, l2_loss_scale, l2_loss_out, accumulate != 0, clear != 0);
+    unpack_loss(l2_sums, l2_loss_scale, l2_loss_out, accumulate != 0, clear != 0);
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= V) return;
     float4 a, b;
@@ -1766,11 +1759,11 @@ __global__ void __launch_bounds__(256) unpack_gradients_kernel(float4* __restric
 // The same for the packed input layout: colour and opacity gradients as one [V,4] array (dr, dg, db, dopacity).
 __global__ void __launch_bounds__(256) unpack_gradients_rgba_kernel(float4* __restrict__ gpack, int V, float4* __restrict__ gV,
                                                                     float4* __restrict__ gRGBA, int accumulate, int clear,
-                                                                    float* __restrict__ l2_partials, float l2_loss_scale,
+                                                                    float* __restrict__ l2_sums, float l2_loss_scale,
                                                                     float* __restrict__ l2_loss_out) {
     allow_dependents();
     await_prerequisites();
-    unpack_loss(l2_partials, l2_loss_scale, l2_loss_out, accumulate != 0, clear != 0);
+    unpack_loss(l2_sums, l2_loss_scale, l2_loss_out, accumulate != 0, clear != 0);
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= V) return;
     float4 a, b;
@@ -1885,7 +1878,7 @@ int tg_blend_forward(const float* tri_geo, const float* tri_attr, const int32_t*
     return TG_OK;
 }
 
-size_t tg_backward_scratch_bytes(int V) { return (size_t)(V > 0 ? V : 0) * 32 + 512; }
+size_t tg_backward_scratch_bytes(int V) { return (size_t)(V > 0 ? V : 0) * 32 + tg::kLossBytes; }
 
 static int backward_impl(const float* tri_geo, const float* tri_attr, const int32_t* sorted_ids, const int32_t* offsets,
                          int V, int W, int H, int tw, int th, int per_pixel_sort, int max_layers,
@@ -1915,13 +1908,13 @@ static int backward_impl(const float* tri_geo, const float* tri_attr, const int3
     TG_REQUIRE(!l2_target || saved, "the fused L2 backward needs the selection saved by the forward pass (default mode)");
     cudaStream_t s = (cudaStream_t)stream;
     float4* gpack = (float4*)scratch;
-    float* partials = (float*)((char*)scratch + (size_t)V * 32);
-    if (!packed) TG_CUDA(cudaMemsetAsync(gpack, 0, (size_t)V * 32 + sizeof(float) * tg::kLossPartials, s));
+    float* loss_sums = (float*)((char*)scratch + (size_t)V * 32);
+    if (!packed) TG_CUDA(cudaMemsetAsync(gpack, 0, (size_t)V * 32 + tg::kLossBytes, s));
     const tg::BlendParams P = make_params(tri_geo, tri_attr, sorted_ids, offsets, W, H, tw, th, 0.f, max_layers);
     const int tiles = P.tiles_x * ((H + th - 1) / th);
     const int threads = ((tw * th + 31) / 32) * 32;
     const tg::BackwardIn in = {(const float4*)grad_image, grad_depthmap, (const float4*)image, depthmap, final_weights,
-                               ends, target_u8 ? nullptr : (const float4*)l2_target, l2_grad_scale, partials,
+                               ends, target_u8 ? nullptr : (const float4*)l2_target, l2_grad_scale, loss_sums,
                                target_u8 ? (const uchar4*)l2_target : nullptr};
     if (saved) {
         // The queued kernel walks the per-pixel selection, not the tile lists, so its blocks need not be the
@@ -1951,7 +1944,7 @@ static int backward_impl(const float* tri_geo, const float* tri_attr, const int3
     TG_LAUNCH_CHECK("blend_backward_kernel");
     if (packed) return TG_OK;
     tg::unpack_gradients_kernel<<<(V + 255) / 256, 256, 0, s>>>(gpack, V, (float4*)grad_vertices, grad_colors,
-                                                              grad_opacities, accumulate, 0, partials, l2_loss_scale,
+                                                              grad_opacities, accumulate, 0, loss_sums, l2_loss_scale,
                                                               l2_target ? l2_loss_out : nullptr);
     TG_LAUNCH_CHECK("unpack_gradients_kernel");
     return TG_OK;
@@ -1979,8 +1972,8 @@ int tg_blend_step_l2(const float* tri_geo, const float* tri_attr, const int32_t*
     }
     cudaStream_t s = (cudaStream_t)stream;
     float4* gpack = (float4*)scratch;
-    float* partials = (float*)((char*)scratch + (size_t)V * 32);
-    if (!packed) TG_CUDA(cudaMemsetAsync(gpack, 0, (size_t)V * 32 + sizeof(float) * tg::kLossPartials, s));
+    float* loss_sums = (float*)((char*)scratch + (size_t)V * 32);
+    if (!packed) TG_CUDA(cudaMemsetAsync(gpack, 0, (size_t)V * 32 + tg::kLossBytes, s));
     tg::BlendParams P = make_params(tri_geo, tri_attr, sorted_ids, offsets, W, H, tw, th, thr, max_layers);
     P.order = tg_host::g_tile_order;
     const int tiles = P.tiles_x * ((H + th - 1) / th);
@@ -1989,11 +1982,11 @@ int tg_blend_step_l2(const float* tri_geo, const float* tri_attr, const int32_t*
     constexpr size_t smem = 8 * sizeof(float4) * tg::kQueueQuads;
     if (int st = tg_host::allow_smem((const void*)tg::blend_step_l2_kernel<256>, smem, allowed)) return st;
     tg::blend_step_l2_kernel<256><<<tiles, threads, smem, s>>>(P, (float4*)image, depthmap, final_weights, ends,
-                                                            (const float4*)target, grad_scale, partials, gpack);
+                                                            (const float4*)target, grad_scale, loss_sums, gpack);
     TG_LAUNCH_CHECK("blend_step_l2_kernel");
     if (packed) return TG_OK;
     tg::unpack_gradients_kernel<<<(V + 255) / 256, 256, 0, s>>>(gpack, V, (float4*)grad_vertices, grad_colors,
-                                                              grad_opacities, accumulate, 0, partials, loss_scale, loss_out);
+                                                              grad_opacities, accumulate, 0, loss_sums, loss_scale, loss_out);
     TG_LAUNCH_CHECK("unpack_gradients_kernel");
     return TG_OK;
 }
@@ -2012,9 +2005,9 @@ int tg_unpack_gradients(void* scratch, size_t scratch_bytes, int V, float loss_s
         tg_host::set_error("backward scratch: need %zu bytes, got %zu", tg_backward_scratch_bytes(V), scratch_bytes);
         return TG_ERR_WORKSPACE;
     }
-    float* partials = (float*)((char*)scratch + (size_t)V * 32);
+    float* loss_sums = (float*)((char*)scratch + (size_t)V * 32);
     TG_CUDA(tg_host::launch_dependent(tg::unpack_gradients_kernel, (V + 255) / 256, 256, 0, (cudaStream_t)stream, (float4*)scratch,
-                                      V, (float4*)grad_vertices, grad_colors, grad_opacities, accumulate, clear, partials,
+                                      V, (float4*)grad_vertices, grad_colors, grad_opacities, accumulate, clear, loss_sums,
                                       loss_scale, loss_out));
     TG_LAUNCH_CHECK("unpack_gradients_kernel");
     return TG_OK;
@@ -2033,10 +2026,10 @@ int tg_unpack_gradients_rgba(void* scratch, size_t scratch_bytes, int V, float l
         tg_host::set_error("backward scratch: need %zu bytes, got %zu", tg_backward_scratch_bytes(V), scratch_bytes);
         return TG_ERR_WORKSPACE;
     }
-    float* partials = (float*)((char*)scratch + (size_t)V * 32);
+    float* loss_sums = (float*)((char*)scratch + (size_t)V * 32);
     TG_CUDA(tg_host::launch_dependent(tg::unpack_gradients_rgba_kernel, (V + 255) / 256, 256, 0, (cudaStream_t)stream,
                                       (float4*)scratch, V, (float4*)grad_vertices, (float4*)grad_rgba, accumulate, clear,
-                                      partials, loss_scale, loss_out));
+                                      loss_sums, loss_scale, loss_out));
     TG_LAUNCH_CHECK("unpack_gradients_rgba_kernel");
     return TG_OK;
 }
@@ -2073,13 +2066,13 @@ int tg_blend_backward_corrected(const float* tri_geo, const float* tri_attr, con
     }
     cudaStream_t s = (cudaStream_t)stream;
     float4* gpack = (float4*)scratch;
-    float* partials = (float*)((char*)scratch + (size_t)V * 32);
-    TG_CUDA(cudaMemsetAsync(gpack, 0, (size_t)V * 32 + sizeof(float) * tg::kLossPartials, s));
+    float* loss_sums = (float*)((char*)scratch + (size_t)V * 32);
+    TG_CUDA(cudaMemsetAsync(gpack, 0, (size_t)V * 32 + tg::kLossBytes, s));
     const tg::BlendParams P = make_params(tri_geo, tri_attr, sorted_ids, offsets, W, H, tw, th, 0.f, max_layers);
     const int tiles = P.tiles_x * ((H + th - 1) / th);
     const int threads = ((tw * th + 31) / 32) * 32;
     const tg::BackwardIn in = {(const float4*)grad_image, grad_depthmap, (const float4*)image, depthmap, final_weights,
-                               ends, nullptr, 0.f, partials, nullptr};
+                               ends, nullptr, 0.f, loss_sums, nullptr};
     if (threads <= 256) {
         if (per_pixel_sort) tg::blend_backward_corrected_kernel<true, 256><<<tiles, threads, 0, s>>>(P, in, gpack);
         else tg::blend_backward_corrected_kernel<false, 256><<<tiles, threads, 0, s>>>(P, in, gpack);
@@ -2089,7 +2082,7 @@ int tg_blend_backward_corrected(const float* tri_geo, const float* tri_attr, con
     }
     TG_LAUNCH_CHECK("blend_backward_corrected_kernel");
     tg::unpack_gradients_kernel<<<(V + 255) / 256, 256, 0, s>>>(gpack, V, (float4*)grad_vertices, grad_colors,
-                                                              grad_opacities, accumulate, 0, partials, 0.f, nullptr);
+                                                              grad_opacities, accumulate, 0, loss_sums, 0.f, nullptr);
     TG_LAUNCH_CHECK("unpack_gradients_kernel");
     return TG_OK;
 }

@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(256) project_backward_kernel(const float* __re
 }
 
 // The packed accumulator of ONE view (what the gradient kernels leave with TG_ACCUMULATE_PACKED: per vertex
-// (d/dx, d/dy, d/dw, d/dopacity | d/dr, d/dg, d/db, -), then 64 loss partials) straight to world space: the
+// (d/dx, d/dy, d/dw, d/dopacity | d/dr, d/dg, d/db, -), then the sums of the loss) straight to world space: the
 // render-space vertex gradient goes through the projection's VJP and is ADDED to grad_points, colours and
 // opacities are added as they are, and the accumulator is cleared on the way out so that the next view needs no
 // memset.  All additions are atomic reductions: several streams may add their views into the same three
@@ -56,16 +56,12 @@ __global__ void __launch_bounds__(256) unpack_project_backward_kernel(float4* __
                                                                       float* __restrict__ grad_points,
                                                                       float* __restrict__ grad_colors,
                                                                       float* __restrict__ grad_opacities,
-                                                                      float* __restrict__ partials, float loss_scale,
+                                                                      float* __restrict__ loss_sums, float loss_scale,
                                                                       float* __restrict__ loss_out) {
     allow_dependents();
     await_prerequisites();
     if (blockIdx.x == 0 && threadIdx.x < 32) {
-        float x = partials[threadIdx.x] + partials[threadIdx.x + 32];
-        partials[threadIdx.x] = 0.f;
-        partials[threadIdx.x + 32] = 0.f;
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) x += __shfl_xor_sync(0xffffffffu, x, d);
+        const float x = take_loss(loss_sums, true);
         if (threadIdx.x == 0 && loss_out) atomicAdd(loss_out, x * loss_scale);
     }
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
@@ -134,9 +130,9 @@ int tg_unpack_project_backward(void* scratch, size_t scratch_bytes, int V, const
     }
     tg::Mat4 pv;
     for (int i = 0; i < 16; i++) pv.m[i] = pv_host[i];
-    float* partials = (float*)((char*)scratch + (size_t)V * 32);
+    float* loss_sums = (float*)((char*)scratch + (size_t)V * 32);
     TG_CUDA(tg_host::launch_dependent(tg::unpack_project_backward_kernel, (V + 255) / 256, 256, 0, (cudaStream_t)stream,
-                                      (float4*)scratch, V, points, pv, grad_points, grad_colors, grad_opacities, partials,
+                                      (float4*)scratch, V, points, pv, grad_points, grad_colors, grad_opacities, loss_sums,
                                       loss_scale, loss_out));
     TG_LAUNCH_CHECK("unpack_project_backward_kernel");
     return TG_OK;
