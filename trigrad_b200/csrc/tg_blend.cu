@@ -1293,9 +1293,10 @@ __device__ __noinline__ void backward_rounds_direct(const BlendParams& P, float 
 
 // A CTA takes a block of kQueueCols x kQueueRows pixels, a warp 8x4 of them, and then PASSES - 1 blocks more, each the same
 // number of rows further down; the queues go on through all of them.  What a warp does for 32 pixels of a layer or two is
-// short against the start of a CTA and ends in a queue that is not full: three passes instead of one, B200, kernel: 1.3M
-// triangles of a pixel, full HD 159 -> 115 us; 200k triangles, full HD 163 -> 153; 2M triangles, 4K 822 -> 806.  (Two, four, six
-// passes: 126, 116, 129; 154, 154, 157; 821, 808, 836.  Blocks next to each other: 4K 850 with two, as the deep blocks all lie in
+// short against the start of a CTA and ends in a queue that is not full; against that, the last CTAs end later.  One, two,
+// three, four, six passes, a fused step, B200, kernel as a trace has it: 200k triangles, 1920x1080 164, 154, 153, 154, 158 us; 1.3M
+// triangles of a pixel, the same image 111, 111, 116, 119, 136; 2M piled up, 3840x2160 786, 814, 798, 799, 824.  So three, and by
+// the size of the image (backward_impl).  (Blocks next to each other: 3840x2160 850 with two, as the deep blocks all lie in
 // the same CTAs and the last of them run alone.  In a loop of a number of passes known at run time the compiler spills.)
 constexpr int kQueueCols = 16, kQueueRows = 8;
 
@@ -1924,12 +1925,19 @@ static int backward_impl(const float* tri_geo, const float* tri_attr, const int3
         tg::BlendParams Q = P;
         Q.tiles_x = (W + tg::kQueueCols - 1) / tg::kQueueCols;
         Q.offsets = nullptr; Q.ids = nullptr; Q.order = nullptr;
-        // Three passes where they leave five waves of CTAs (seven or eight per SM): with a depth gradient 1280x720, 2.3 waves,
-        // 40 us in one pass, 42 in three; 669k triangles, 1382x1036, 3.6 waves, 193 and 202; inside a mesh, full HD, 5.2 waves, 86
-        // and 80.
+        // Three passes from the numbers of waves on that were measured to pay, B200, whole calls, one pass -> three, us.
+        // No depth gradient, 8 CTAs per SM (fused steps; the same renders through autograd are alike): 2.0 waves (1280x720) 1.3M
+        // triangles of a pixel 480 -> 486, 89k random triangles 153 -> 157, 100k piled up in the middle 241 -> 274; 3.2 (1600x900)
+        // 492 -> 497, 221 -> 218, 258 -> 260; 3.8 (1760x990) 474 -> 477, 268 -> 259, 274 -> 275; 4.6 (1920x1080) 488 -> 491, 310 ->
+        // 304, 290 -> 291; 8.1 (2560x1440) 590 -> 587, 530 -> 508, 381 -> 384; 18 (3840x2160) 879 -> 863, 1162 -> 1102, 718 -> 698.
+        // With one, 7 per SM (through autograd): 3.6 waves (1600x900) 494 -> 495, 237 -> 236, 267 -> 275; 5.2 (1920x1080) 492 ->
+        // 493, 333 -> 331, 301 -> 311; 9.3 (2560x1440) 597 -> 594, 565 -> 551, 402 -> 418; 21 (3840x2160) 892 -> 879, 1241 -> 1196,
+        // 758 -> 761; 100k light triangles spread evenly 179 -> 172, 233 -> 223, 363 -> 337, 709 -> 646.  Triangles piled up in the
+        // middle of the image lose with a depth gradient, up to 5 % of the call, and gain only beyond 3840x2160.
         constexpr int kPasses = 3;
         const int strips = (H + tg::kQueueRows - 1) / tg::kQueueRows;
-        const bool many = (int64_t)Q.tiles_x * strips >= (int64_t)kPasses * 5 * 7 * 148;
+        const int64_t wanted = grad_depthmap ? kPasses * 5 * 7 * 148 : kPasses * 7 * 8 * 148 / 2;      // 5 waves, 3.5 waves
+        const bool many = (int64_t)Q.tiles_x * strips >= wanted;
         const int blocks = Q.tiles_x * (many ? (strips + kPasses - 1) / kPasses : strips);
         auto kernel = many ? (grad_depthmap ? tg::blend_backward_queued_kernel<kPasses, true> : tg::blend_backward_queued_kernel<kPasses, false>)
                            : (grad_depthmap ? tg::blend_backward_queued_kernel<1, true> : tg::blend_backward_queued_kernel<1, false>);
