@@ -204,6 +204,46 @@ def test_not_counting_is_refused_where_it_is_not_safe(triangles, capacity, flags
     assert status == 1
 
 
+@pytest.mark.filterwarnings("ignore:The CUDA Graph is empty")
+def test_not_counting_is_refused_while_the_stream_is_captured():
+    from trigrad_b200 import _native as N
+
+    T, tiles = 100, 64
+    capacity = T * tiles
+    t = Hh.scene_tensors(S.random_triangles(T, 128, 128, 0.05, 0.4, name="captured"))
+    out = trigrad_b200.wrapper.forward_native(*t, 128, 128, 16, 16, 1 / 256, False, True, 32)
+    image, depth, fw, _, off, geo, attr, ends, sel = out[:9]
+    want = image.clone()
+    ptr = lambda t: ctypes.c_void_p(t.data_ptr())
+    lib = N.lib()
+    size = lib.tg_forward_workspace_bytes(T, tiles, capacity)
+    ws = torch.empty(size + 256, dtype=torch.uint8, device="cuda")
+    ids = torch.empty(capacity, dtype=torch.int32, device="cuda")
+    info = torch.zeros(4, dtype=torch.int32).pin_memory()
+    stream = torch.cuda.Stream()
+
+    def call():
+        return lib.tg_render_forward(*(ptr(x) for x in t), T, 128, 128, 16, 16, 1 / 256, 1, 32, ptr(image), ptr(depth), ptr(fw), ptr(ends),
+                                     ptr(sel), ptr(geo), ptr(attr), ptr(ids), capacity, ptr(off),
+                                     ctypes.c_void_p((ws.data_ptr() + 255) // 256 * 256), size, ptr(info), None, 4 | 32,
+                                     ctypes.c_void_p(stream.cuda_stream))
+
+    image.zero_()
+    torch.cuda.synchronize()
+    launches = lib.tg_launch_count()
+    with torch.cuda.stream(stream):
+        graph = torch.cuda.CUDAGraph()
+        graph.capture_begin()
+        status = call()
+        graph.capture_end()
+    assert status == N.TG_ERR_BAD_ARG and lib.tg_launch_count() == launches
+    torch.cuda.synchronize()
+    assert not bool(image.any())
+    assert call() == N.TG_OK
+    torch.cuda.synchronize()
+    assert torch.equal(image, want) and not bool(info.any())
+
+
 def _stacked(n, w, h, seed):
     """n triangles over the whole image, at few depths, so that order is the triangles' in part."""
     rng = np.random.default_rng(seed)
@@ -264,3 +304,114 @@ def test_lists_that_change_between_short_and_long():
         for _ in range(64):
             counts(few)
         assert not any(counts(few) for _ in range(300))
+
+
+def _uncounted_routes():
+    w, h = 72, 40
+
+    def packed(m, target):
+        rgba, faces = trigrad_b200.pack_mesh(m[2], m[3], m[1])
+        x = [m[0].detach().requires_grad_(), rgba.requires_grad_()]
+        image, depth = trigrad_b200.render_packed(x[0], faces, x[1], w, h)
+        return image.detach(), *torch.autograd.grad((image * target).sum() + depth[torch.isfinite(depth)].sum(), x)
+
+    def step(u8):
+        def f(m, target):
+            b = views.GradBuffer.allocate(m[0].shape[0], "cuda", 4)
+            target = (target * 255).to(torch.uint8) if u8 else target
+            image = views.l2_view_step(m[0], m[1], m[2], m[3], target, w, h, b.points, b.colors, b.opacities, b.loss)
+            return image, b.points, b.colors, b.opacities, b.loss.reshape(1)
+        return f
+
+    def world(kept):
+        def f(m, target):
+            b = views.GradBuffer.allocate(m[0].shape[0], "cuda", 3)
+            p = views.PackedGradients(m[0].shape[0], "cuda") if kept else None
+            image = views.l2_world_view_step(m[0][:, :3].contiguous(), torch.eye(4), m[1], m[2], m[3], target, w, h, b.points, b.colors,
+                                             b.opacities, b.loss, packed=p)
+            return image, b.points, b.colors, b.opacities, b.loss.reshape(1)
+        return f
+
+    return w, h, {"packed": packed, "step": step(False), "step_u8": step(True), "world": world(False), "world_packed": world(True)}
+
+
+@pytest.mark.parametrize("route", ["packed", "step", "step_u8", "world", "world_packed"])
+def test_every_route_without_the_count(route):
+    """Packed inputs and the fused steps, lists short and long, against the same call when it counts."""
+    from trigrad_b200 import _native as N
+
+    w, h, routes = _uncounted_routes()
+    run = routes[route]
+    few, many = _stacked(20, w, h, 1), _stacked(700, w, h, 2)
+    target = torch.rand((h, w, 4), device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    state_here = lambda: N.host().state(0, torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    want = {}
+    with torch.cuda.stream(torch.cuda.Stream()):
+        for name, mesh in (("few", few), ("many", many)):
+            trigrad_b200.wrapper.forward_native(*many, w, h, 16, 16, 1 / 256, False, True, 32)      # long: the next call counts
+            before = state_here().last_slot
+            want[name] = run(mesh, target)
+            assert state_here().last_slot != before
+        torch.cuda.current_stream().synchronize()
+    with torch.cuda.stream(torch.cuda.Stream()):
+        for _ in range(65):
+            run(few, target)
+        torch.cuda.current_stream().synchronize()
+        before = state_here().last_slot
+        got = {"few": run(few, target), "many": run(many, target)}
+        assert state_here().last_slot == before
+        torch.cuda.current_stream().synchronize()
+    for name in want:
+        assert torch.equal(got[name][0], want[name][0])
+        for a, b in zip(got[name][1:], want[name][1:]):
+            assert Hh.rel_l2(a.cpu().numpy(), b.cpu().numpy()) <= 1e-5      # order of atomics
+
+
+def test_states_that_share_a_row_of_the_table_of_long_lists():
+    """More states have been made than the table has rows: a word that one state's kernel writes is another's to find."""
+    from trigrad_b200 import _native as N
+
+    w, h = 50, 40
+    few, many = _stacked(20, w, h, 1), _stacked(400, w, h, 2)
+    want = {name: trigrad_b200.render(*m, w, h, record_timing=True)[0] for name, m in (("few", few), ("many", many))}
+    torch.cuda.synchronize()
+    handles = []
+
+    def new_stream():
+        s = ctypes.c_void_p()
+        assert int(torch.cuda.cudart().cudaStreamCreate(ctypes.addressof(s))) == 0
+        handles.append(s.value)
+        return s.value
+
+    first = new_stream()
+    row = N.host().state(0, first).long_row
+    for _ in range(600):
+        second = new_stream()
+        if N.host().state(0, second).long_row == row:
+            break
+        assert N.host().state(0, first).long_row == row             # the one used least lately is given back: not this one
+    else:
+        raise AssertionError("no two states share a row")
+    state = {h_: N.host().state(0, h_) for h_ in (first, second)}
+
+    def counts(handle, name):
+        before = state[handle].last_slot
+        with torch.cuda.stream(torch.cuda.ExternalStream(handle)), torch.no_grad():
+            image = trigrad_b200.render(*(few if name == "few" else many), w, h)[0]
+            torch.cuda.current_stream().synchronize()
+        assert torch.equal(image, want[name])
+        return state[handle].last_slot != before
+
+    for handle in (first, second):
+        while counts(handle, "few"):
+            pass
+    assert not counts(first, "many")
+    assert counts(second, "few")                   # found the other's word
+    for _ in range(6):
+        for handle in (first, second, first):
+            counts(handle, "many")
+            counts(handle, "few")
+    torch.cuda.synchronize()
+    for handle in handles:
+        assert int(torch.cuda.cudart().cudaStreamDestroy(handle)) == 0

@@ -1008,6 +1008,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         .def_readonly("info", &DeviceState::info)
         .def_readonly("last_slot", &DeviceState::last_slot)
         .def_readonly("k_estimate", &DeviceState::k_estimate)
+        .def_property_readonly("long_row", [](const DeviceState& s) { return (uintptr_t)s.long_row; })
         .def("check_error_word", &DeviceState::check_error_word);
     m.def("bind", &bind);
     m.def("state", [](int device, int64_t stream) { return state_of(device, (cudaStream_t)stream); });
