@@ -272,7 +272,8 @@ int tg_blend_step_l2(const float* tri_geo, const float* tri_attr, const int32_t*
  *                synchronises the stream.  [3] receives, with K, the number of list slots the call used: K plus the
  *                pairs that TG_FORWARD_CULL_TILES dropped.
  *   stage_ms_host  NULL or float[5]: milliseconds of {init, per_tile_lists, sorting,
- *                bary_transforms, rasterization} measured with CUDA events (synchronises)
+ *                bary_transforms, rasterization} measured with CUDA events (synchronises).  Sorting and compositing are two
+ *                kernels then, also in a small render that without the times would do both in one.
  * If the slots exceed list_capacity nothing past the binning is run and TG_ERR_CAPACITY is returned with the
  * capacity needed in info_host[0]; call again with a larger list and workspace.
  *   flags        0, or TG_FORWARD_CULL_TILES: a (triangle, tile) pair of the bounding rectangle is listed only if

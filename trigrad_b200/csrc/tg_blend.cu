@@ -1010,8 +1010,8 @@ __device__ __forceinline__ int load_pixel_state(const TileCtx& c, const BlendPar
 // gradients of the fragment's interpolations; these go into a queue in shared memory; part B (the
 // expensive barycentric partials and the 21 per-vertex outputs) pops 32 queued fragments at a time and
 // so runs with full warps.  A warp whose lanes are busy anyway (deep overlap, or one opaque layer everywhere) skips the
-// queue.  (200k triangles, full HD: 140 us at 70 % of L1, 63 % of the issue slots and 13 % of DRAM; bound by the latency of
-// the gathers, fifteen of 16 bytes per fragment, and by L1 together, half of whose work is shared memory's.)
+// queue.  (200k triangles, full HD: 153 us with L1 75 % busy and 64 % of the issue slots used; bound by the latency of the
+// gathers, fifteen of 16 bytes per fragment, and by L1 together, half of whose work is shared memory's.)
 // DEPTH = false (everywhere below): no gradient flows into the depth map, the terms that it feeds are left out.
 struct QueuedFragment {
     float px, py;
@@ -1389,9 +1389,9 @@ __global__ void __launch_bounds__(kQueueCols * kQueueRows, DEPTH ? 7 : 8) blend_
 // image; the per-vertex outputs go through the per-warp queue as in blend_backward_queued_kernel.
 // Slower than the two kernels in most places by now, as it has none of their staging ahead of the pixel set-up, streamed
 // lists and dependent launches, and its half for the forward runs with the registers of both (a step, B200: 200k triangles,
-// full HD 317 us in two kernels against 355 in one; 2M triangles, 4K 2038 against 2301; 10k, 512x512 60 against 73; four
-// streams of views, full HD 277 against 296 per view).  Faster where triangles are a pixel each and a pixel blends one
-// fragment or none (1.3M triangles, full HD 594 against 561).  Used on request only.
+// full HD 306 us in two kernels against 353 in one; 2M triangles, 4K 2028 against 2267; 10k, 512x512 55 against 62; four
+// streams of views, full HD 257 against 293 per view).  As fast where triangles are a pixel each and a pixel blends one
+// fragment or none (1.3M triangles, full HD 505 against 503).  Used on request only.
 template <int MAXT>
 __global__ void __launch_bounds__(MAXT, 4) blend_step_l2_kernel(BlendParams P, float4* __restrict__ image,
                                                                 float* __restrict__ depthmap, float* __restrict__ final_w,

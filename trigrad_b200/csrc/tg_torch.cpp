@@ -179,7 +179,8 @@ struct DeviceState {
     // were short, no kernel of a call that did not has said otherwise since (in `long_row`), and the room for every pair of
     // triangle and tile is small.  28 bytes each, so 14 MB.  The wait was the length of the binning and a trip over PCIe in
     // every small call (B200: ten squares, 50x50, forward and backward 99 -> 84 us; 1280 triangles, 256x256, forward 25.3 ->
-    // 19.9, with a loss and backward 171 -> 161).
+    // 19.9, with a loss and backward 171 -> 161), by overlap with the calls around it: a caller that waits for every image gains
+    // nothing here.
     // "The last few": one at first, twice as many (up to kCountedMax) each time a call that did not count met a long list, which
     // costs it 100 to 200 us where lists have 3300 entries (see sort_words in tg_blend.cu).  So a program whose lists change
     // between short and long pays that a few times and not at every change, and one that has long lists now and then keeps most
