@@ -145,8 +145,8 @@ def test_small_renders_keep_little_more_than_image_records_and_selection(call, t
     tiles = -(-width // tile) * -(-height // tile)
     px = width * height
     rest = 28 * px + 160 * triangles + 4 * (tiles + 1) + 5 * 256
-    # the lists: none, up to a quarter of the rest, or what a call that counts has room for
-    lists = 0 if call == "render" else max(rest // 4, 4 * max(2 * triangles, 5 * int(_entries(v, i, c, o, width, height, tile)) // 4) + 4096)
+    # the lists: none, up to as much as the rest, or what a call that counts has room for
+    lists = 0 if call == "render" else max(rest, 4 * max(2 * triangles, 5 * int(_entries(v, i, c, o, width, height, tile)) // 4) + 4096)
     selection = 4 * 32 * px if call == "render" else 0
     # blocks are rounded up to 512 bytes; of the 20 MB segments that blocks above 1 MB come from, less than 1 MB is given away unsplit
     unsplit = (1 << 20) / ((20 << 20) // selection) if selection > 1 << 20 else 0

@@ -376,10 +376,11 @@ ForwardOut forward(const Tensor& vertices_, const Tensor& indices_, const Tensor
     const auto state = state_of(w.device, w.stream);
     std::lock_guard<std::mutex> lock(state->use);
     // Without the count the lists have room for every pair, however few there are.  Where they are kept for a backward that is
-    // let be up to a quarter of what the graph keeps anyway (image, depth map, blob); beyond it the call counts, as keeping the
-    // lists of 1280 triangles at 256x256, 1.3 MB instead of 15 KB, added 60 % to every live graph.
+    // let be up to as much as the graph keeps anyway (image, depth map, blob), so a live graph at most doubles, by 2 MB at most;
+    // beyond it the call counts.  (Corrected gradients, forward and backward, B200: 604 triangles, 142x104, a third of the rest,
+    // 90 us without the count against 99 with it; 1140, 346x192, six tenths, 135 against 139.)
     const bool lists_small = count != Count::kUnlessSmallKeepLists || s.selection.defined() ||
-                             16 * (int64_t)T * v.tiles() <= 20 * v.pixels() + (int64_t)s.l.bytes;
+                             4 * (int64_t)T * v.tiles() <= 20 * v.pixels() + (int64_t)s.l.bytes;
     const bool no_count = state->no_count(T, v.tiles()) && count != Count::kAlways && lists_small && !record_timing && !step &&
                           c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None;
     int64_t cap = no_count ? (int64_t)T * v.tiles()
