@@ -317,8 +317,13 @@ int tg_blend_step_l2(const float* tri_geo, const float* tri_attr, const int32_t*
  *                TG_SHORT_LIST, whenever the binning gets there: such lists are sorted inside the compositing kernel and not
  *                filtered there (lists of 3300 entries: 100 to 200 us more than without the flag), so a caller that finds it
  *                had better do without the flag for a while.  Results do not depend on it.
+ *                TG_LISTS_UNUSED: the caller does not read `sorted_ids` and `offsets`, nor hands them to a backward that
+ *                walks the lists (one without `selection`): they are left unwritten where a call has no need of them (today
+ *                with TG_NO_COUNT, whose lists then lie with room for every triangle in each tile and are not moved
+ *                together).  Both have to have their full size.
  */
 #define TG_NO_COUNT 32u
+#define TG_LISTS_UNUSED 64u
 #define TG_NO_COUNT_TRIANGLES 4096
 size_t tg_forward_workspace_bytes(int T, int tiles, uint32_t list_capacity);
 int tg_render_forward(const float* vertices, const int32_t* indices, const float* colors, const float* opacities,

@@ -279,6 +279,49 @@ def test_long_lists_of_a_call_that_does_not_count(n, tile, sort):
         assert torch.equal(a.view(torch.int32), b.view(torch.int32))
 
 
+@pytest.mark.parametrize("n", [1, 31, 33, 64, 65, 127, 128, 129])
+@pytest.mark.parametrize("w, h, tile", [(20, 13, 32), (97, 61, 16), (250, 130, 8)])
+def test_lists_that_are_not_moved_together(n, w, h, tile):
+    """Entries that go straight to their lists, in turn with calls that keep the lists or count on the same workspace."""
+    from trigrad_b200 import _native as N
+
+    mesh = _stacked(n, w, h, n)
+    size = (w, h, tile, tile)
+    gi = torch.rand((h, w, 4), device="cuda", generator=torch.Generator("cuda").manual_seed(n))
+
+    def gradients(function, **options):
+        leaves = [x.detach().requires_grad_() for x in (mesh[0], mesh[2], mesh[3])]
+        image, _ = function(leaves[0], mesh[1], leaves[1], leaves[2], *size, **options)
+        return [image.detach(), *torch.autograd.grad(image, leaves, gi)]
+
+    calls = {"look": lambda: trigrad_b200.render(*mesh, *size), "fit": lambda: gradients(trigrad_b200.render),
+             "lists": lambda: gradients(trigrad_b200.render, per_pixel_sort=False),
+             "corrected": lambda: gradients(trigrad_b200.render_corrected)}
+    with torch.cuda.stream(torch.cuda.Stream()):
+        state = N.host().state(0, torch.cuda.current_stream().cuda_stream)
+        want = {}
+        for name, call in calls.items():
+            state_before = state.last_slot
+            trigrad_b200.wrapper.forward_native(*_stacked(150, w, h, 9), w, h, tile, tile, 1 / 256, False, True, 32)     # the next call counts
+            want[name] = call()
+            assert state.last_slot != state_before
+        for _ in range(65):
+            with torch.no_grad():
+                trigrad_b200.render(*_stacked(3, w, h, 3), *size)
+        torch.cuda.current_stream().synchronize()
+        for name in ("look", "fit", "look", "lists", "look", "corrected", "fit", "look"):
+            got = calls[name]()
+            assert torch.equal(got[0], want[name][0])
+            for a, b in zip(got[1:], want[name][1:]):
+                if name == "look":
+                    assert torch.equal(a, b)
+                else:
+                    assert Hh.rel_l2(a.cpu().numpy(), b.cpu().numpy()) <= 1e-5      # order of atomics
+        trigrad_b200.wrapper.forward_native(*mesh, w, h, tile, tile, 1 / 256, False, True, 32)
+        assert torch.equal(trigrad_b200.render(*mesh, *size, record_timing=True)[0], want["look"][0])
+        torch.cuda.current_stream().synchronize()
+
+
 def test_lists_that_change_between_short_and_long():
     """Calls that meet a long list without having counted get rarer, whatever the pattern; where lists stay short, no call counts."""
     from trigrad_b200 import _native as N

@@ -81,6 +81,7 @@ struct TileLists {
     ForwardWorkspace ws;
     int tiles;
     bool device_scan, mapped, no_count;
+    bool in_place;                         // entries go straight to their lists, each with room for all triangles
     cudaEvent_t k_ready = nullptr;
     uint32_t* device_status;               // error word, null where no kernel of the path can raise it
     uint32_t K = 0, longest = 0;
@@ -89,6 +90,7 @@ struct TileLists {
     TileLists(void* workspace, int T, int W, int H, int tw, int th, uint32_t cap, unsigned flags)
         : ws(workspace, ((W + tw - 1) / tw) * ((H + th - 1) / th), cap), tiles(((W + tw - 1) / tw) * ((H + th - 1) / th)),
           device_scan(tiles > tg::kTileScanByOneCta), mapped((flags & TG_INFO_MAPPED) != 0 && T > 0), no_count((flags & TG_NO_COUNT) != 0),
+          in_place(no_count && (flags & TG_LISTS_UNUSED) != 0),
           device_status(device_scan ? ws.bin.status : nullptr) {}       // only the scan waits
 
     int start(const float* vertices, const int32_t* indices, const float* colors, const float* opacities, int T, int W, int H,
@@ -112,9 +114,10 @@ struct TileLists {
         // per-triangle records, (triangle, tile) pairs with their depth keys
         if (int st = tg_host::bin_triangles(vertices, indices, colors, opacities, T, W, H, tw, th, tri_geo, tri_attr, ws.bin,
                                             offsets, cap, cull, (flags & TG_INPUT_PACKED) != 0,
-                                            (flags & TG_WORKSPACE_READY) != 0, s))
+                                            (flags & TG_WORKSPACE_READY) != 0, in_place, s))
             return st;
         timer.mark();                                                    // [2] start of "per_tile_lists"
+        if (in_place) return TG_OK;
         if (int st = tg_host::place_entries(ws.bin, T, W, H, tw, th, offsets, cap, mapped && !no_count ? info_host : nullptr,
                                             no_count ? info_host + 1 : nullptr, s))
             return st;
@@ -188,7 +191,7 @@ static int check_forward_args(int T, int W, int H, int tw, int th, int max_layer
     TG_REQUIRE(workspace && info_host && offsets, "null pointer");
     TG_REQUIRE(((uintptr_t)workspace & 255) == 0, "workspace must be 256-byte aligned");
     TG_REQUIRE(list_capacity < 0x80000000u, "list capacity must stay below 2^31");
-    TG_REQUIRE((flags & ~63u) == 0, "unknown flag");
+    TG_REQUIRE((flags & ~127u) == 0, "unknown flag");
     TG_REQUIRE(!(flags & TG_EXPECT_SHORT_LISTS) || (flags & TG_INFO_MAPPED), "TG_EXPECT_SHORT_LISTS needs TG_INFO_MAPPED");
     return TG_OK;
 }
@@ -245,8 +248,8 @@ int tg_render_forward(const float* vertices, const int32_t* indices, const float
     // expects nothing longer: it checks on the device what the host is told afterwards.
     const bool early = lists.tiles <= tg::kFusedTiles && T > 0 && (flags & (TG_EXPECT_SHORT_LISTS | TG_NO_COUNT)) != 0 && stage_ms_host == nullptr;
     timer.mark();                                                    // [3] start of "sorting"
-    int st = early ? tg_host::blend_forward_short(tri_geo, tri_attr, lists.ws.bin, list_capacity, lists.no_count, sorted_ids, offsets, W,
-                                                  H, tw, th, thr, per_pixel_sort, max_layers, image, depthmap, final_weights, ends, selection, s)
+    int st = early ? tg_host::blend_forward_short(tri_geo, tri_attr, lists.ws.bin, list_capacity, lists.no_count, lists.in_place ? T : 0,
+                                                  info_host + 1, sorted_ids, offsets, W, H, tw, th, thr, per_pixel_sort, max_layers, image, depthmap, final_weights, ends, selection, s)
                    : lists.sort_short(sorted_ids, offsets, list_capacity, T, s);
     if (st || lists.no_count) return st;
     if ((st = lists.wait(list_capacity, info_host, s))) return st;

@@ -575,6 +575,8 @@ struct BinArgs {
     uint32_t* info_host;     // words 0, 1 and 3 of mapped host memory receive them too, or null
     uint32_t* long_host;     // mapped host memory that receives the longest list if it has more than kFusedList entries, or null
     uint4* pairs;            // [capacity]
+    uint64_t* lists;         // [tiles][room], for entries that go straight to their lists, or null
+    uint32_t room;
     uint32_t capacity;
     int tiles, tiles_x, tiles_y;
     int scan_here;           // 0: the host launches a device-wide scan of the tile counts
@@ -605,6 +607,10 @@ __device__ __forceinline__ void write_pair(const BinArgs& bin, const float* tri,
     const float* p = tri + 32 * kTriPlane;
     const float depth = tile_key({v[0], v[32], v[64], v[96], v[128], v[160]}, {p[0], p[32], p[64]}, cx.z, cx.w, cy.z, cy.w,
                                  poly, 32 * kBinWarps);
+    if (bin.lists != nullptr) {          // a triangle is in a tile's list once, so rank < room, which is T
+        bin.lists[(size_t)tile * bin.room + rank] = ((uint64_t)float_to_ordered(depth) << 32) | (uint32_t)t;
+        return;
+    }
     if (pos < bin.capacity)              // the host checks K before anything that reads the entries is used
         bin.pairs[pos] = make_uint4((uint32_t)t, float_to_ordered(depth), tile, rank);
 }
@@ -724,7 +730,7 @@ __global__ void __launch_bounds__(32 * kBinWarps, 32 / kBinWarps) bin_kernel(con
         uint64_t sum = 0;
 #pragma unroll
         for (int w = 0; w < kBinWarps; w++) { s_first[w] = (uint32_t)sum; sum += s_warp[w]; }
-        const uint64_t at = atomicAdd(slot_counter(bin), (unsigned long long)sum);
+        const uint64_t at = bin.lists != nullptr ? 0 : atomicAdd(slot_counter(bin), (unsigned long long)sum);
         s_first[kBinWarps] = at + sum < kTooManyPairs ? (uint32_t)sum : 0u;
         s_base = (uint32_t)at;
     }
@@ -756,7 +762,7 @@ __global__ void __launch_bounds__(32 * kBinWarps, 32 / kBinWarps) bin_kernel(con
 #pragma unroll
                 for (int k = 0; k < 9; k++) m[k] = d[32 * (kTriMatrix + k)];
                 keep = rect_may_cover(m, {cx.x, cx.y, cy.x, cy.y});
-                if (!keep && slot0 + e < bin.capacity) bin.pairs[slot0 + e] = make_uint4(0, 0, kHole, 0);
+                if (!keep && bin.lists == nullptr && slot0 + e < bin.capacity) bin.pairs[slot0 + e] = make_uint4(0, 0, kHole, 0);
             }
             const float* v = d + 32 * kTriCorners;
             inside = inside_tile({v[0], v[32], v[64], v[96], v[128], v[160]}, cx.z, cx.w, cy.z, cy.w);
@@ -965,7 +971,7 @@ int prefer_smem(const void* kernel, int kilobytes, SmemAllowed& preferred) {
 static tg::BinArgs bin_args(const BinBuffers& b, int W, int H, int tw, int th, int32_t* offsets, uint32_t list_capacity,
                             uint32_t* info_host, uint32_t* long_host) {
     const int tiles_x = (W + tw - 1) / tw, tiles_y = (H + th - 1) / th, tiles = tiles_x * tiles_y;
-    return {b.tile_counts, offsets, b.counters, b.info, info_host, long_host, b.pairs, list_capacity, tiles, tiles_x, tiles_y,
+    return {b.tile_counts, offsets, b.counters, b.info, info_host, long_host, b.pairs, nullptr, 0, list_capacity, tiles, tiles_x, tiles_y,
             tiles <= tg::kTileScanByOneCta ? 1 : 0, b.tile_order ? 1 : 0, {b.tables, b.tables + tiles_x}};
 }
 
@@ -973,7 +979,7 @@ static tg::BinArgs bin_args(const BinBuffers& b, int W, int H, int tw, int th, i
 // argument is).
 int bin_triangles(const float* vertices, const int32_t* indices, const float* colors, const float* opacities, int T, int W,
                   int H, int tw, int th, float* tri_geo, float* tri_attr, const BinBuffers& b, int32_t* offsets,
-                  uint32_t list_capacity, bool cull, bool packed, bool ready, cudaStream_t stream) {
+                  uint32_t list_capacity, bool cull, bool packed, bool ready, bool in_place, cudaStream_t stream) {
     TG_REQUIRE(T >= 0, "T < 0");
     if (int s = check_sizes(W, H, tw, th)) return s;
     TG_REQUIRE(offsets, "null pointer");
@@ -1003,7 +1009,12 @@ int bin_triangles(const float* vertices, const int32_t* indices, const float* co
     constexpr int kWave = 148 * 32 / tg::kBinWarps;
     const int per_cta = T >= 32 * tg::kBinWarps * kWave ? 32 * tg::kBinWarps : (T + kWave - 1) / kWave;
     const int grid = (T + per_cta - 1) / per_cta;
-    const tg::BinArgs bin = bin_args(b, W, H, tw, th, offsets, list_capacity, nullptr, nullptr);
+    tg::BinArgs bin = bin_args(b, W, H, tw, th, offsets, list_capacity, nullptr, nullptr);
+    if (in_place) {
+        TG_REQUIRE((uint64_t)T * tiles <= list_capacity, "no room for every pair");
+        bin.lists = b.entries;
+        bin.room = (uint32_t)T;
+    }
     auto inverse = [](int n) { return (n & (n - 1)) == 0 ? 1.0 / n : 0.0; };
     auto kernel = cull ? tg::bin_kernel<true> : tg::bin_kernel<false>;
     static SmemAllowed bin_allowed[2];

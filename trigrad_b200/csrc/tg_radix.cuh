@@ -129,10 +129,11 @@ struct BinBuffers {
     uint32_t* tile_order;        // [tiles] or null
     uint32_t* list_heads;        // [6] heads of the tile sort's work lists, zeroed by place_entries
 };
-// Records and pairs.  `ready`: the counters are zero and the tables valid from a call before.
+// Records and pairs.  `ready`: the counters are zero and the tables valid from a call before.  `in_place`: no pairs, but every
+// entry at once in `entries`, tile * T + rank (the caller has room for T * tiles; place_entries is not called).
 int bin_triangles(const float* vertices, const int32_t* indices, const float* colors, const float* opacities, int T, int W,
                   int H, int tw, int th, float* tri_geo, float* tri_attr, const BinBuffers& b, int32_t* offsets,
-                  uint32_t list_capacity, bool cull, bool packed, bool ready, cudaStream_t stream);
+                  uint32_t list_capacity, bool cull, bool packed, bool ready, bool in_place, cudaStream_t stream);
 // Entries grouped by tile, offsets, info, launch order.  `info_host`: mapped host memory whose words 0, 1 and 3 receive the
 // three info words (K last), or null; `long_host`: one that receives the longest list where it has more than kFusedList
 // entries, or null.  Counts and counters of images of at most kPlaceTiles tiles are left to the kernel
@@ -153,9 +154,10 @@ int sort_long_lists(uint64_t* entries, const int32_t* offsets, int tiles, int32_
                     uint32_t longest, cudaStream_t stream);
 // Forward compositing with the sort of the tile lists (at most kFusedList entries each, `info` as the binning left it) in the
 // same kernel, which does nothing when the slots exceed `capacity` or a list is longer; with `any_length` it sorts longer
-// ones too (sort_words), and does not filter them.
+// ones too (sort_words), and does not filter them.  `room` > 0: the lists lie `room` entries apart, as bin_triangles leaves them
+// in place, complete; `long_host` as for place_entries, which is then not called.
 int blend_forward_short(const float* tri_geo, const float* tri_attr, const BinBuffers& b, uint32_t capacity, bool any_length,
-                        int32_t* sorted_ids, const int32_t* offsets, int W, int H, int tw, int th, float thr,
+                        int room, uint32_t* long_host, int32_t* sorted_ids, const int32_t* offsets, int W, int H, int tw, int th, float thr,
                         int per_pixel_sort, int max_layers, float* image, float* depthmap, float* final_weights,
                         int32_t* ends, int32_t* selection, cudaStream_t stream);
 }  // namespace tg_host

@@ -383,6 +383,7 @@ ForwardOut forward(const Tensor& vertices_, const Tensor& indices_, const Tensor
                              4 * (int64_t)T * v.tiles() <= 20 * v.pixels() + (int64_t)s.l.bytes;
     const bool no_count = state->no_count(T, v.tiles()) && count != Count::kAlways && lists_small && !record_timing && !step &&
                           c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None;
+    const unsigned lists_unused = count == Count::kUnlessSmall || s.selection.defined() ? TG_LISTS_UNUSED : 0u;
     int64_t cap = no_count ? (int64_t)T * v.tiles()
                            : std::max<int64_t>(state->k_estimate + state->k_estimate / 4 + 1024, 2 * (int64_t)T + 1024);
     while (true) {
@@ -393,7 +394,7 @@ ForwardOut forward(const Tensor& vertices_, const Tensor& indices_, const Tensor
         const bool ready = std::equal(key, key + 4, state->ready);
         state->ready[0] = 0;                     // until this call has succeeded
         const unsigned flags = fixed_flags | (ready ? TG_WORKSPACE_READY : 0u) |
-                               (no_count ? TG_NO_COUNT : state->short_lists && !step ? TG_EXPECT_SHORT_LISTS : 0u);
+                               (no_count ? TG_NO_COUNT | lists_unused : state->short_lists && !step ? TG_EXPECT_SHORT_LISTS : 0u);
         const int slot = no_count ? -1 : state->next_slot();
         int32_t* info = no_count ? state->long_row : state->words(slot);
         float* ms = record_timing ? out.stage_ms.data() : nullptr;
