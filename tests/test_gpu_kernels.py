@@ -108,3 +108,32 @@ def test_lists_at_the_ends_of_chunks(triangles, per_pixel_sort):
                     per_pixel_sort, triangles + 1, corrected=True)
     for a, b in zip((v, c, o), og):
         assert Hh.rel_l2(a.grad.cpu().numpy(), b) <= 2e-4
+
+
+@pytest.mark.parametrize("columns", [[1], [1, 6], [6, 7], [7, 7, 7, 1], [8, 7, 6, 5, 4, 3, 2, 1], [2] * 13 + [8], [1] * 31 + [8]],
+                         ids=lambda x: f"{len(x)}_layers_{4 * sum(x)}")
+@pytest.mark.parametrize("depth_gradient", [False, True])
+def test_fragments_that_a_warp_keeps_for_its_next_round(columns, depth_gradient):
+    """One warp of 8x4 pixels; layer k is a slanted rectangle over its first columns[k] columns."""
+    W, H, rng = 8, 4, np.random.default_rng(len(columns))
+    vertices, faces = [], []
+    for k, n in enumerate(columns):
+        right, z = 2 * n / W - 1, 1 + 0.1 * k
+        depth = z + 0.01 * rng.random(4)
+        xy = [(-1.1, -1.1), (right, -1.1), (right, 1.1), (-1.1, 1.1)]
+        faces += [[4 * k, 4 * k + 1, 4 * k + 2], [4 * k, 4 * k + 2, 4 * k + 3]]
+        vertices += [(x, y, d, 1 / d) for (x, y), d in zip(xy, depth)]
+    v, i = np.array(vertices, np.float32), np.array(faces, np.int32)
+    c, o = rng.random((len(v), 3), dtype=np.float32), rng.uniform(0.1, 0.5, len(v)).astype(np.float32)
+    of = O.forward(v, i, c, o, W, H, 16, 16, 1 / 256, True, 32)
+    assert int(of.ends.sum()) == 4 * sum(columns)
+    gi = rng.standard_normal((H, W, 4)).astype(np.float32)
+    gd = rng.standard_normal((H, W)).astype(np.float32) if depth_gradient else np.zeros((H, W), np.float32)
+    og = O.backward(v, i, c, o, W, H, of, gi, np.where(np.isfinite(of.depthmap.reshape(H, W)), gd, 0).astype(np.float32), 16, 16, True, 32)
+    leaves = [Hh.cuda(x).requires_grad_() for x in (v, c, o)]
+    image, depth = trigrad_b200.render(leaves[0], Hh.cuda(i), leaves[1], leaves[2], W, H, 16, 16)
+    outputs = [(image, Hh.cuda(gi))] + ([(depth, Hh.cuda(gd))] if depth_gradient else [])
+    got = torch.autograd.grad([x for x, _ in outputs], leaves, [g for _, g in outputs])
+    for a, b in zip(got, og):
+        # sums of at most 32 fragments per vertex; the barycentric partials of triangles this large lose about two digits
+        assert Hh.rel_l2(a.cpu().numpy(), b) <= 1e-4

@@ -1037,9 +1037,19 @@ struct QueuedFragment {
     float o_raw, cr, cg, cb, z;
     float uo, ur, ug, ub, uz;
 };
-// A warp's queue: 64 slots of 4 quads, rotated so that a quad of consecutive slots lies on different banks.  (A pitch of 5
-// does that too, but every kilobyte of the eight CTAs is L1 taken from the gathers: 2M triangles, 4K, a step 2083 -> 2065 us.)
-constexpr int kQueueSlots = 64, kQueuePitch = 4, kQueueQuads = kQueueSlots * kQueuePitch;
+// A warp's queue: slots of 4 quads, rotated so that a quad of consecutive slots lies on different banks.  Up to kLeft fragments stay
+// behind when a round ends; the slots above hold that round's, and, once these are in registers, the table of emit_lanes.  Every
+// kilobyte of the seven or eight CTAs is L1 taken from the gathers: with kLeft = 26 and columns of 34 words eight CTAs take 163 KB
+// and the SM is split at 164; with 31 slots and columns of 36, which are read four words at a time, it is split at 196, and fine
+// meshes lose (kernel, 200k triangles 1920x1080 / 1.3M triangles of a pixel 1920x1080 / 2M piled up 3840x2160: 146 / 108 / 722
+// us against 149 / 118 / 802; with 23 slots and 36 words, whose rounds end less full, 148 / 110 / 732).  Seven CTAs have room for both.
+constexpr int kQueuePitch = 4;
+template <bool DEPTH>
+struct QueueShape {
+    static constexpr int kLeft = DEPTH ? 31 : 26, kColumn = DEPTH ? 36 : 34;
+    static constexpr int kTable = 24 * kColumn / 4;                       // quads
+    static constexpr int kQuads = kLeft * kQueuePitch + (kTable > 32 * kQueuePitch ? kTable : 32 * kQueuePitch);
+};
 
 template <bool DEPTH>
 __device__ __forceinline__ void queue_push(float4* q, int slot, const QueuedFragment& f) {
@@ -1206,14 +1216,18 @@ __device__ __forceinline__ void backward_one(const float* w, const AttrRec& a, c
 }
 
 // Contributions of a warp's lanes (triangles `id`) with as few atomics as their triangles allow.  All lanes must call.
-// The lanes' rows go to shared memory ordered by triangle, sixteen at a time; 24 lanes add the columns up and send each
-// triangle's three 32-byte slots with one instruction.  The vertex ids ride in the unused eighth word of every slot.
-// (Adding up to four neighbouring lanes with 42 shuffles and six vector reductions per run took as long where a triangle
+// The lanes' outputs go to a table in shared memory, one column of 32 words per value, the lanes ordered by triangle; 24 lanes add the
+// columns up and send each triangle's three 32-byte slots with one instruction.  The vertex ids ride in the unused eighth value
+// of every slot.  Columns and not rows: a store then has the lanes in one column, 32 banks whatever their order, where rows, two
+// times sixteen of them as there was less room, took 72 passes through shared memory instead of 24 and were most of what the
+// kernel asked of L1, which it waits for where many triangles overlap (200k triangles, 1920x1080 154 -> 146 us; 1.3M
+// triangles of a pixel, the same image 111 -> 108; 2M piled up, 3840x2160 807 -> 722).
+// (Adding up to four neighbouring lanes with 42 shuffles and six vector reductions per run took as long as rows where a triangle
 // has one or two of the 32 fragments, and 17 % longer where a few triangles have them all: 2M overlapping triangles, 4K,
-// 944 us against 804.)
-// `rows`: kRowsQuads quads of shared memory of this warp.
-constexpr int kRowQuads = 7;                  // 6 used; the odd pitch spreads the rows over the banks
-constexpr int kRowsQuads = 16 * kRowQuads;
+// 944 us against 804.  Sums of four values per lane, for five triangles at a time, which leave as vector reductions: 185 against
+// 154 and 981 against 807 - reductions of 16 bytes to one 32-byte slot are not merged.)
+// `rows`: 24 * COLUMN words of this warp.  COLUMN: 36, or 34, which is read two words at a time.
+template <int COLUMN>
 __device__ __forceinline__ void emit_lanes(const Contrib& c, bool valid, int id, float4* rows, float4* __restrict__ gpack) {
     const int lane = lane_id();
     const unsigned peers = __match_any_sync(0xffffffffu, valid ? id : -1 - lane);      // distinct negatives never match
@@ -1229,46 +1243,46 @@ __device__ __forceinline__ void emit_lanes(const Contrib& c, bool valid, int id,
     const int total = __shfl_sync(0xffffffffu, incl, 31);
     const int place = __shfl_sync(0xffffffffu, incl - size, __ffs(peers) - 1) + __popc(peers & below);
     const unsigned ends = __reduce_or_sync(0xffffffffu, leads ? 1u << (incl - 1) : 0u);   // last row of every triangle
-    const float* column = reinterpret_cast<const float*>(rows) + min(lane, 4 * kRowQuads - 1);
-    const int* ids = reinterpret_cast<const int*>(rows) + (min(lane, 23) | 7);
+    float* table = reinterpret_cast<float*>(rows);
+    const float* column = table + COLUMN * min(lane, 23);
+    const int* ids = reinterpret_cast<const int*>(table) + COLUMN * (min(lane, 23) | 7);
     const bool adds = lane < 24 && (lane & 7) != 7;
+    if (valid) {
+        float* at = table + place;
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+#pragma unroll
+            for (int i = 0; i < 7; i++) at[COLUMN * (8 * k + i)] = c.v[k][i];
+            at[COLUMN * (8 * k + 7)] = __int_as_float(c.vid[k]);
+        }
+    }
+    __syncwarp();
     float sum = 0.f;
 #pragma unroll 1
-    for (int half = 0; half < total; half += 16) {
-        __syncwarp();                     // the rows before have been added up
-        if (valid && place >= half && place < half + 16) {
-            float4* row = rows + kRowQuads * (place - half);
-#pragma unroll
-            for (int k = 0; k < 3; k++) {
-                row[2 * k] = make_float4(c.v[k][0], c.v[k][1], c.v[k][2], c.v[k][3]);
-                row[2 * k + 1] = make_float4(c.v[k][4], c.v[k][5], c.v[k][6], __int_as_float(c.vid[k]));
-            }
+    for (int j = 0; j < total; j += 4) {
+        float x[4];                       // rows past `total` end no triangle
+        if (COLUMN % 4 == 0) {
+            const float4 q = *reinterpret_cast<const float4*>(column + j);
+            x[0] = q.x; x[1] = q.y; x[2] = q.z; x[3] = q.w;
+        } else {
+            const float2 q = *reinterpret_cast<const float2*>(column + j), r = *reinterpret_cast<const float2*>(column + j + 2);
+            x[0] = q.x; x[1] = q.y; x[2] = r.x; x[3] = r.y;
         }
-        __syncwarp();
-        const int n = min(16, total - half);
-        const unsigned end_bits = ends >> half;
-#pragma unroll 1
-        for (int j = 0; j < n; j += 4) {
-            float x[4];
 #pragma unroll
-            for (int k = 0; k < 4; k++) x[k] = column[4 * kRowQuads * (j + k)];     // rows past `total` end no triangle
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                sum += x[k];
-                if ((end_bits >> (j + k)) & 1u) {
-                    const int vid = ids[4 * kRowQuads * (j + k)];
-                    if (adds) atomicAdd(reinterpret_cast<float*>(gpack + 2 * (size_t)vid) + (lane & 7), sum);
-                    sum = 0.f;
-                }
+        for (int k = 0; k < 4; k++) {
+            sum += x[k];
+            if ((ends >> (j + k)) & 1u) {
+                const int vid = ids[j + k];
+                if (adds) atomicAdd(reinterpret_cast<float*>(gpack + 2 * (size_t)vid) + (lane & 7), sum);
+                sum = 0.f;
             }
         }
     }
     __syncwarp();
 }
 
-// Part B for the fragments in queue slots first .. first + count - 1 (count <= 32), one per lane.  The slots from `first`
-// on, at least 33 of them, are free once the fragments are in registers.
-static_assert(kRowsQuads <= 33 * kQueuePitch, "rows in the free part of the queue");
+// Part B for the fragments in queue slots first .. first + count - 1 (count <= 32, first <= kLeft), one per lane.  The slots from
+// `first` on are free once the fragments are in registers.
 template <bool DEPTH>
 __device__ __forceinline__ void drain_queue(const BlendParams& P, float4* q, int first, int count, float4* __restrict__ gpack) {
     const int lane = lane_id();
@@ -1282,7 +1296,7 @@ __device__ __forceinline__ void drain_queue(const BlendParams& P, float4* q, int
         backward_outputs<DEPTH>(w, a, f, ct);
     }
     __syncwarp();
-    emit_lanes(ct, valid, f.id, q + kQueuePitch * first, gpack);
+    emit_lanes<QueueShape<DEPTH>::kColumn>(ct, valid, f.id, q + kQueuePitch * first, gpack);
 }
 
 // Whole fragments per round, for warps whose lanes are busy anyway.  Kept out of line so that it does not weigh on the
@@ -1304,7 +1318,7 @@ __device__ __noinline__ void backward_rounds_direct(const BlendParams& P, float 
             const Bary b = apply_bary(m, px, py);
             backward_one<DEPTH>(w, a, b, px, py, pg, st, ct);
         }
-        emit_lanes(ct, has, id, rows, gpack);
+        emit_lanes<QueueShape<DEPTH>::kColumn>(ct, has, id, rows, gpack);
     }
 }
 
@@ -1323,7 +1337,7 @@ __global__ void __launch_bounds__(kQueueCols * kQueueRows, DEPTH ? 7 : 8) blend_
                                                                         float4* __restrict__ gpack) {
     constexpr int kWarps = kQueueCols * kQueueRows / 32;
     __shared__ __align__(16) float s_coord[kQueueCols + PASSES * kQueueRows];
-    __shared__ float4 s_queue[kWarps][kQueueQuads];
+    __shared__ float4 s_queue[kWarps][QueueShape<DEPTH>::kQuads];
     allow_dependents();
     const int lane = lane_id(), warp = threadIdx.x >> 5;
     const int x0 = ((int)blockIdx.x % P.tiles_x) * kQueueCols, y0 = ((int)blockIdx.x / P.tiles_x) * kQueueRows;
@@ -1382,9 +1396,10 @@ __global__ void __launch_bounds__(kQueueCols * kQueueRows, DEPTH ? 7 : 8) blend_
             }
             queued += __popc(pushing);
             __syncwarp();
-            if (queued >= 32) {
-                queued -= 32;
-                drain_queue<DEPTH>(P, q, queued, 32, gpack);
+            if (queued > QueueShape<DEPTH>::kLeft) {
+                const int count = min(queued, 32);
+                queued -= count;
+                drain_queue<DEPTH>(P, q, queued, count, gpack);
                 __syncwarp();
             }
         }
@@ -1406,7 +1421,7 @@ __global__ void __launch_bounds__(kQueueCols * kQueueRows, DEPTH ? 7 : 8) blend_
 // image; the per-vertex outputs go through the per-warp queue as in blend_backward_queued_kernel.
 // Slower than the two kernels in most places by now, as it has none of their staging ahead of the pixel set-up, streamed
 // lists and dependent launches, and its half for the forward runs with the registers of both (a step, B200: 200k triangles,
-// full HD 306 us in two kernels against 353 in one; 2M triangles, 4K 2028 against 2267; 10k, 512x512 55 against 62; four
+// full HD 301 us in two kernels against 330 in one; 2M triangles, 4K 1948 against 2153; 10k, 512x512 55 against 62; four
 // streams of views, full HD 257 against 293 per view).  As fast where triangles are a pixel each and a pixel blends one
 // fragment or none (1.3M triangles, full HD 505 against 503).  Used on request only.
 template <int MAXT>
@@ -1418,7 +1433,7 @@ __global__ void __launch_bounds__(MAXT, 4) blend_step_l2_kernel(BlendParams P, f
     static_assert(MAXT == 256, "the per-warp queues are sized for 8 warps");
     __shared__ float4 s_geo[kChunk * kStagedQuads];
     __shared__ int s_id[kChunk];
-    __shared__ __align__(16) float s_coord[kMaxTileCoords];
+    __shared__ __align__(16) float s_coord[260];       // four CTAs take 195 KB, the SM is split at 196 (at 228: 2M triangles, 4K, a step 2242 -> 2423 us)
     __shared__ SweepScratch s_scratch;
     __shared__ uint8_t s_slots[2 * MAXT];
     extern __shared__ float4 s_step[];       // queues of the warps
@@ -1473,7 +1488,7 @@ __global__ void __launch_bounds__(MAXT, 4) blend_step_l2_kernel(BlendParams P, f
     for (int d = 16; d > 0; d >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, d);
     if (lane == 0 && sq != 0.f) add_loss(l2_sums, blockIdx.x * 8 + (threadIdx.x >> 5), sq);
 
-    float4* q = s_step + kQueueQuads * (threadIdx.x >> 5);
+    float4* q = s_step + QueueShape<false>::kQuads * (threadIdx.x >> 5);
     const int nmax = __reduce_max_sync(0xffffffffu, n);
     int queued = 0;                                    // uniform over the warp
     for (int s = 0; s < nmax; s++) {
@@ -1490,9 +1505,10 @@ __global__ void __launch_bounds__(MAXT, 4) blend_step_l2_kernel(BlendParams P, f
         }
         queued += __popc(pushing);
         __syncwarp();
-        if (queued >= 32) {
-            queued -= 32;
-            drain_queue<false>(P, q, queued, 32, gpack);
+        if (queued > QueueShape<false>::kLeft) {
+            const int count = min(queued, 32);
+            queued -= count;
+            drain_queue<false>(P, q, queued, count, gpack);
             __syncwarp();
         }
     }
@@ -2004,7 +2020,7 @@ int tg_blend_step_l2(const float* tri_geo, const float* tri_attr, const int32_t*
     const int tiles = P.tiles_x * ((H + th - 1) / th);
     const int threads = ((tw * th + 31) / 32) * 32;
     static tg_host::SmemAllowed allowed;
-    constexpr size_t smem = 8 * sizeof(float4) * tg::kQueueQuads;
+    constexpr size_t smem = 8 * sizeof(float4) * tg::QueueShape<false>::kQuads;
     if (int st = tg_host::allow_smem((const void*)tg::blend_step_l2_kernel<256>, smem, allowed)) return st;
     tg::blend_step_l2_kernel<256><<<tiles, threads, smem, s>>>(P, (float4*)image, depthmap, final_weights, ends,
                                                             (const float4*)target, grad_scale, loss_sums, gpack);
