@@ -112,9 +112,10 @@ def test_lists_at_the_ends_of_chunks(triangles, per_pixel_sort):
 
 @pytest.mark.parametrize("columns", [[1], [1, 6], [6, 7], [7, 7, 7, 1], [8, 7, 6, 5, 4, 3, 2, 1], [2] * 13 + [8], [1] * 31 + [8]],
                          ids=lambda x: f"{len(x)}_layers_{4 * sum(x)}")
-@pytest.mark.parametrize("depth_gradient", [False, True])
-def test_fragments_that_a_warp_keeps_for_its_next_round(columns, depth_gradient):
-    """One warp of 8x4 pixels; layer k is a slanted rectangle over its first columns[k] columns."""
+@pytest.mark.parametrize("depth_gradient, layers", [(False, 32), (True, 32), (True, 40)])
+def test_fragments_that_a_warp_keeps_for_its_next_round(columns, depth_gradient, layers):
+    """One warp of 8x4 pixels; layer k is a slanted rectangle over its first columns[k] columns.  With more than 32 layers allowed
+    the backward walks the list, in rounds of 4 * columns lanes."""
     W, H, rng = 8, 4, np.random.default_rng(len(columns))
     vertices, faces = [], []
     for k, n in enumerate(columns):
@@ -125,15 +126,39 @@ def test_fragments_that_a_warp_keeps_for_its_next_round(columns, depth_gradient)
         vertices += [(x, y, d, 1 / d) for (x, y), d in zip(xy, depth)]
     v, i = np.array(vertices, np.float32), np.array(faces, np.int32)
     c, o = rng.random((len(v), 3), dtype=np.float32), rng.uniform(0.1, 0.5, len(v)).astype(np.float32)
-    of = O.forward(v, i, c, o, W, H, 16, 16, 1 / 256, True, 32)
+    of = O.forward(v, i, c, o, W, H, 16, 16, 1 / 256, True, layers)
     assert int(of.ends.sum()) == 4 * sum(columns)
     gi = rng.standard_normal((H, W, 4)).astype(np.float32)
     gd = rng.standard_normal((H, W)).astype(np.float32) if depth_gradient else np.zeros((H, W), np.float32)
-    og = O.backward(v, i, c, o, W, H, of, gi, np.where(np.isfinite(of.depthmap.reshape(H, W)), gd, 0).astype(np.float32), 16, 16, True, 32)
+    og = O.backward(v, i, c, o, W, H, of, gi, np.where(np.isfinite(of.depthmap.reshape(H, W)), gd, 0).astype(np.float32), 16, 16, True, layers)
     leaves = [Hh.cuda(x).requires_grad_() for x in (v, c, o)]
-    image, depth = trigrad_b200.render(leaves[0], Hh.cuda(i), leaves[1], leaves[2], W, H, 16, 16)
+    image, depth = trigrad_b200.render(leaves[0], Hh.cuda(i), leaves[1], leaves[2], W, H, 16, 16, max_layers=layers)
     outputs = [(image, Hh.cuda(gi))] + ([(depth, Hh.cuda(gd))] if depth_gradient else [])
     got = torch.autograd.grad([x for x, _ in outputs], leaves, [g for _, g in outputs])
     for a, b in zip(got, og):
         # sums of at most 32 fragments per vertex; the barycentric partials of triangles this large lose about two digits
         assert Hh.rel_l2(a.cpu().numpy(), b) <= 1e-4
+
+
+@pytest.mark.parametrize("triangles, tile", [(128, 16), (129, 16), (192, 8), (256, 32), (257, 32)])
+def test_lists_that_stay_in_shared_memory_for_all_sweeps(triangles, tile):
+    """Every triangle covers the image's one tile or most of it: lists around the number of records that are kept."""
+    rng = np.random.default_rng(triangles)
+    angle = rng.uniform(0, 2 * np.pi, (triangles, 1)) + np.arange(3) * (2 * np.pi / 3)
+    depth = rng.uniform(0.5, 10, (triangles, 1)) * np.ones(3)
+    v = np.stack([3 * np.cos(angle), 3 * np.sin(angle), depth, 1 / depth], 2).reshape(-1, 4).astype(np.float32)
+    i = np.arange(3 * triangles, dtype=np.int32).reshape(-1, 3)
+    c, o = rng.random((len(v), 3), dtype=np.float32), rng.uniform(0.01, 0.03, len(v)).astype(np.float32)
+    size = (tile, tile, tile, tile)
+    li = O.build_lists(v, i, *size)
+    assert li.offsets[-1] == triangles
+    gi = rng.standard_normal((tile, tile, 4)).astype(np.float32)
+    gd = rng.standard_normal((tile, tile)).astype(np.float32)
+    of = O.forward(v, i, c, o, *size, 1 / 256, True, 1000)
+    for function, corrected in ((trigrad_b200.render, False), (trigrad_b200.render_corrected, True)):
+        og = O.backward(v, i, c, o, tile, tile, of, gi, gd, tile, tile, True, 1000, corrected=corrected)
+        leaves = [Hh.cuda(x).requires_grad_() for x in (v, c, o)]
+        image, depth = function(leaves[0], Hh.cuda(i), leaves[1], leaves[2], *size, max_layers=1000)
+        for a, b in zip(torch.autograd.grad((image, depth), leaves, (Hh.cuda(gi), Hh.cuda(gd))), og):
+            # the recurrences' divisions by 1 - opacity, a few hundred in a row, on both sides in 32 bits
+            assert Hh.rel_l2(a.cpu().numpy(), b) <= 2e-4

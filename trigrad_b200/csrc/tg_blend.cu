@@ -282,6 +282,14 @@ __device__ __forceinline__ StagedGeo load_staged(const float4* s_geo, int r) {
     return g;
 }
 
+__device__ __forceinline__ void load_geo_staged(const float4* s_geo, int r, float* m, float* w) {
+    const StagedGeo g = load_staged(s_geo, r);
+#pragma unroll
+    for (int k = 0; k < 9; k++) m[k] = g.m[k];
+#pragma unroll
+    for (int k = 0; k < 3; k++) w[k] = g.w[k];
+}
+
 // Bit mask (64 records) of the staged records that may matter to this warp: the triangle may cover one
 // of its pixels (corner test) and, when `depth_cut` is finite, its depth lower bound is below the cut
 // (every lane already holds a full batch of nearer fragments otherwise).
@@ -951,23 +959,6 @@ __device__ __forceinline__ void emit_uniform(const Contrib& c, bool has, float4*
     __syncwarp();
 }
 
-// The same for lanes with triangles of their own (`id`): pixels next to each other under large triangles mostly blend the
-// same triangle at the same place of their sequences.  All lanes must call.
-__device__ __forceinline__ void emit_warp(const Contrib& c, bool has, int id, float4* __restrict__ gpack) {
-    const unsigned peers = __match_any_sync(0xffffffffu, has ? id : -1 - (int)lane_id());
-    const bool big = has && __popc(peers) >= kGroupMin;
-    unsigned todo = __ballot_sync(0xffffffffu, big);
-#pragma unroll 1
-    for (int it = 0; it < 32 / kGroupMin && todo != 0; ++it) {
-        const int leader = __ffs(todo) - 1;
-        const unsigned group = __shfl_sync(0xffffffffu, peers, leader);
-        todo &= ~group;
-        reduce_group(c, (group >> lane_id()) & 1u, leader, gpack);
-    }
-    if (has && !big) emit_contrib(c, gpack);
-    __syncwarp();
-}
-
 struct BackwardIn {
     const float4* gimage;
     const float* gdepth;
@@ -1520,16 +1511,32 @@ __global__ void __launch_bounds__(MAXT, 4) blend_step_l2_kernel(BlendParams P, f
 }
 
 // General path (any max_layers, both modes): searches the list again as the reference does.
-// Per-pixel mode, batch after batch sweeping the list: lists of up to kResident records are staged once for all sweeps
-// (3000 triangles about 90 layers deep, corrected gradients: 316 -> 313 us).  20 KB; three CTAs' worth leaves L1 its share.
-constexpr int kResident = 4 * kChunk;
+// Per-pixel mode, batch after batch sweeping the list: lists of up to kListRecords records are staged once for all sweeps, and for
+// the gradients of the fragments found.  A warp's outputs leave as in the queued kernel, through a table of columns: its lanes
+// hold a handful of triangles each round, and a reduction by halves for each (100 instructions, a lane's own six vector reductions
+// where few lanes share one) took longer.  B200, corrected gradients, kernel: 3000 triangles about 90 layers deep, 637x421,
+// tiles of 16 307 -> 272 us, of 32 377 -> 318, of 8 349 -> 296 (with 256 records instead of 128 376: the shared memory of small
+// CTAs); 300 triangles, 480x360, at most 64 layers 104 -> 97; 100k small triangles in one or two layers 113 -> 114; 400
+// triangles, 200x150, a CTA per SM, so that what counts is how long a round takes 48 -> 52.  Bound by issue, 24 warps on an SM.
+template <bool SORT, int MAXT>
+constexpr int kListRecords = !SORT ? kChunk : MAXT <= 256 ? 2 * kChunk : 4 * kChunk;
+constexpr int kListColumn = 36, kListTable = 24 * kListColumn / 4;      // quads per warp
+constexpr size_t list_tables(int threads) { return sizeof(float4) * kListTable * (threads / 32); }
+// A round's contributions.  From 12 lanes on the table is cheaper than the lanes' own vector reductions, below it a little dearer
+// (100k small triangles in one or two layers 122 -> 114 us, deep stacks 1 % slower; 16 and 20 lanes: 300 triangles 95 -> 107, 119).
+constexpr int kTableMin = 12;
+__device__ __forceinline__ void emit_round(const Contrib& c, bool has, int id, float4* rows, float4* __restrict__ gpack) {
+    if (__popc(__ballot_sync(0xffffffffu, has)) >= kTableMin) emit_lanes<kListColumn>(c, has, id, rows, gpack);
+    else if (has) emit_contrib(c, gpack);
+}
 template <bool SORT, int MAXT>
 __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (SORT ? 3 : 4) : 1) blend_backward_kernel(BlendParams P, BackwardIn in, float4* __restrict__ gpack) {
-    __shared__ float4 s_geo[(SORT ? kResident : kChunk) * kStagedQuads];
+    __shared__ float4 s_geo[kListRecords<SORT, MAXT> * kStagedQuads];
     __shared__ int s_id[kChunk];
+    extern __shared__ float4 s_tables[];             // SORT: kListTable quads per warp
     __shared__ __align__(16) float s_coord[MAXT <= 256 ? 260 : kMaxTileCoords];
     const TileCtx c = tile_context(P, s_coord);
-    const bool resident = SORT && c.end - c.start <= kResident;
+    const bool resident = SORT && c.end - c.start <= kListRecords<SORT, MAXT>;
     if (resident) stage_geo_async(P, c.start, c.end - c.start, s_geo);
     PixelGrad pg;
     BackState st;
@@ -1552,19 +1559,26 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (SORT ? 3 : 4) : 1) blend_
             const int rounds = __reduce_max_sync(0xffffffffu, n);
             // back to front inside the batch (reference render.cu:684-688); the first of the rounds starts at every lane's
             // last fragment
+            int ahead = n > 0 ? (int)(uint32_t)batch.key[n - 1] : 0, id_ahead = n > 0 ? P.ids[ahead] : 0;
             for (int s = 0; s < rounds; ++s) {
                 const int i = n - 1 - s;
                 int id = -1;
                 Contrib ct = {};
                 if (i >= 0) {
-                    id = P.ids[(uint32_t)batch.key[i]];
+                    const int j = ahead;
+                    id = id_ahead;
+                    if (i > 0) {
+                        ahead = (int)(uint32_t)batch.key[i - 1];
+                        id_ahead = P.ids[ahead];
+                    }
                     float m[9], w[3];
-                    load_geo(P.geo, id, m, w);
+                    if (resident) load_geo_staged(s_geo, j - c.start, m, w);
+                    else load_geo(P.geo, id, m, w);
                     const Bary b = apply_bary(m, c.px, c.py);
                     const AttrRec a = load_attr<true>(P.attr, id);
                     backward_one(w, a, b, c.px, c.py, pg, st, ct);
                 }
-                emit_warp(ct, i >= 0, id, gpack);
+                emit_round(ct, i >= 0, id, s_tables + kListTable * (threadIdx.x >> 5), gpack);
             }
             if (go) {
                 if (n > 0) {
@@ -1667,11 +1681,12 @@ __device__ __forceinline__ void backward_one_prefix(const float* w, const AttrRe
 template <bool SORT, int MAXT>
 __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (SORT ? 3 : 4) : 1) blend_backward_corrected_kernel(BlendParams P, BackwardIn in,
                                                                         float4* __restrict__ gpack) {
-    __shared__ float4 s_geo[(SORT ? kResident : kChunk) * kStagedQuads];
+    __shared__ float4 s_geo[kListRecords<SORT, MAXT> * kStagedQuads];
     __shared__ int s_id[kChunk];
+    extern __shared__ float4 s_tables[];             // SORT: kListTable quads per warp
     __shared__ __align__(16) float s_coord[MAXT <= 256 ? 260 : kMaxTileCoords];
     const TileCtx c = tile_context(P, s_coord);
-    const bool resident = SORT && c.end - c.start <= kResident;
+    const bool resident = SORT && c.end - c.start <= kListRecords<SORT, MAXT>;
     if (resident) stage_geo_async(P, c.start, c.end - c.start, s_geo);
     PixelGrad pg;
     BackState unused;
@@ -1698,18 +1713,25 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (SORT ? 3 : 4) : 1) blend_
             select_sweep(P, c, go, bs, last, batch, {s_geo, s_id, &s_scratch, s_slots, resident, nullptr, nullptr});
             const int n = go ? min(batch.found, remaining) : 0;
             const int rounds = __reduce_max_sync(0xffffffffu, n);
+            int ahead = n > 0 ? (int)(uint32_t)batch.key[0] : 0, id_ahead = n > 0 ? P.ids[ahead] : 0;
             for (int i = 0; i < rounds; ++i) {
                 int id = -1;
                 Contrib ct = {};
                 if (i < n) {
-                    id = P.ids[(uint32_t)batch.key[i]];
+                    const int j = ahead;
+                    id = id_ahead;
+                    if (i + 1 < n) {
+                        ahead = (int)(uint32_t)batch.key[i + 1];
+                        id_ahead = P.ids[ahead];
+                    }
                     float m[9], w[3];
-                    load_geo(P.geo, id, m, w);
+                    if (resident) load_geo_staged(s_geo, j - c.start, m, w);
+                    else load_geo(P.geo, id, m, w);
                     const Bary b = apply_bary(m, c.px, c.py);
                     const AttrRec a = load_attr<true>(P.attr, id);
                     backward_one_prefix(w, a, b, c.px, c.py, pg, fin, pf, ct);
                 }
-                emit_warp(ct, i < n, id, gpack);
+                emit_round(ct, i < n, id, s_tables + kListTable * (threadIdx.x >> 5), gpack);
             }
             if (go) {
                 if (n > 0) {
@@ -1918,6 +1940,26 @@ int tg_blend_forward(const float* tri_geo, const float* tri_attr, const int32_t*
 
 size_t tg_backward_scratch_bytes(int V) { return (size_t)(V > 0 ? V : 0) * 32 + tg::kLossBytes; }
 
+}  // extern "C"
+// The kernels that walk the tile lists: the reference's backward or the corrected one.
+template <bool CORRECTED>
+static int launch_list_kernel(const tg::BlendParams& P, const tg::BackwardIn& in, float4* gpack, int tiles, int threads, bool sort, cudaStream_t s) {
+    const bool large = threads > 256;
+    void (*kernel)(tg::BlendParams, tg::BackwardIn, float4*);
+    if (CORRECTED)
+        kernel = large ? (sort ? tg::blend_backward_corrected_kernel<true, 1024> : tg::blend_backward_corrected_kernel<false, 1024>)
+                       : (sort ? tg::blend_backward_corrected_kernel<true, 256> : tg::blend_backward_corrected_kernel<false, 256>);
+    else
+        kernel = large ? (sort ? tg::blend_backward_kernel<true, 1024> : tg::blend_backward_kernel<false, 1024>)
+                       : (sort ? tg::blend_backward_kernel<true, 256> : tg::blend_backward_kernel<false, 256>);
+    static tg_host::SmemAllowed allowed[2];
+    if (sort)
+        if (int st = tg_host::allow_smem((const void*)kernel, tg::list_tables(large ? 1024 : 256), allowed[large])) return st;
+    kernel<<<tiles, threads, sort ? tg::list_tables(threads) : 0, s>>>(P, in, gpack);
+    return TG_OK;
+}
+extern "C" {
+
 static int backward_impl(const float* tri_geo, const float* tri_attr, const int32_t* sorted_ids, const int32_t* offsets,
                          int V, int W, int H, int tw, int th, int per_pixel_sort, int max_layers,
                          const float* grad_image, const float* grad_depthmap, const void* l2_target, bool target_u8,
@@ -1979,12 +2021,8 @@ static int backward_impl(const float* tri_geo, const float* tri_attr, const int3
         auto kernel = many ? (grad_depthmap ? tg::blend_backward_queued_kernel<kPasses, true> : tg::blend_backward_queued_kernel<kPasses, false>)
                            : (grad_depthmap ? tg::blend_backward_queued_kernel<1, true> : tg::blend_backward_queued_kernel<1, false>);
         TG_CUDA(tg_host::launch_dependent(kernel, blocks, tg::kQueueCols * tg::kQueueRows, 0, s, Q, in, selection, gpack));
-    } else if (threads <= 256) {
-        if (per_pixel_sort) tg::blend_backward_kernel<true, 256><<<tiles, threads, 0, s>>>(P, in, gpack);
-        else tg::blend_backward_kernel<false, 256><<<tiles, threads, 0, s>>>(P, in, gpack);
     } else {
-        if (per_pixel_sort) tg::blend_backward_kernel<true, 1024><<<tiles, threads, 0, s>>>(P, in, gpack);
-        else tg::blend_backward_kernel<false, 1024><<<tiles, threads, 0, s>>>(P, in, gpack);
+        if (int st = launch_list_kernel<false>(P, in, gpack, tiles, threads, per_pixel_sort, s)) return st;
     }
     TG_LAUNCH_CHECK("blend_backward_kernel");
     if (packed) return TG_OK;
@@ -2118,13 +2156,7 @@ int tg_blend_backward_corrected(const float* tri_geo, const float* tri_attr, con
     const int threads = ((tw * th + 31) / 32) * 32;
     const tg::BackwardIn in = {(const float4*)grad_image, grad_depthmap, (const float4*)image, depthmap, final_weights,
                                ends, nullptr, 0.f, loss_sums, nullptr};
-    if (threads <= 256) {
-        if (per_pixel_sort) tg::blend_backward_corrected_kernel<true, 256><<<tiles, threads, 0, s>>>(P, in, gpack);
-        else tg::blend_backward_corrected_kernel<false, 256><<<tiles, threads, 0, s>>>(P, in, gpack);
-    } else {
-        if (per_pixel_sort) tg::blend_backward_corrected_kernel<true, 1024><<<tiles, threads, 0, s>>>(P, in, gpack);
-        else tg::blend_backward_corrected_kernel<false, 1024><<<tiles, threads, 0, s>>>(P, in, gpack);
-    }
+    if (int st = launch_list_kernel<true>(P, in, gpack, tiles, threads, per_pixel_sort, s)) return st;
     TG_LAUNCH_CHECK("blend_backward_corrected_kernel");
     tg::unpack_gradients_kernel<<<(V + 255) / 256, 256, 0, s>>>(gpack, V, (float4*)grad_vertices, grad_colors,
                                                               grad_opacities, accumulate, 0, loss_sums, 0.f, nullptr);
