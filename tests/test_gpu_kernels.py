@@ -162,3 +162,20 @@ def test_lists_that_stay_in_shared_memory_for_all_sweeps(triangles, tile):
         for a, b in zip(torch.autograd.grad((image, depth), leaves, (Hh.cuda(gi), Hh.cuda(gd))), og):
             # the recurrences' divisions by 1 - opacity, a few hundred in a row, on both sides in 32 bits
             assert Hh.rel_l2(a.cpu().numpy(), b) <= 2e-4
+
+
+@pytest.mark.parametrize("scale", [3.0, 1e3, 1e5, 3e6, 1e8])
+@pytest.mark.parametrize("cull", [False, True])
+def test_keys_of_triangles_far_larger_than_the_image(scale, cull):
+    """Intersections that miss their border by more than a tile leave polygons that are not convex: keys as the oracle's."""
+    rng, T, W, H, tile = np.random.default_rng(int(scale)), 400, 96, 80, 8
+    xy = rng.standard_normal((T, 3, 2)) * scale * 10 ** rng.uniform(-2, 0, (T, 3, 1)) + rng.uniform(-1, 1, (T, 1, 2))
+    d = rng.uniform(0.5, 10, (T, 3, 1))
+    v = np.concatenate([xy, d, 1 / d], 2).reshape(-1, 4).astype(np.float32)
+    i = np.arange(3 * T, dtype=np.int32).reshape(-1, 3)
+    c, o = rng.random((len(v), 3), dtype=np.float32), rng.random(len(v), dtype=np.float32)
+    li = O.build_lists(v, i, W, H, tile, tile, cull=cull)
+    assert li.offsets[-1] > 1000
+    out = Wr.forward_native(*map(Hh.cuda, (v, i, c, o)), W, H, tile, tile, 1 / 256, False, True, 32, cull_tiles=cull)
+    assert np.array_equal(out[4].cpu().numpy(), li.offsets)
+    assert np.array_equal(out[3].cpu().numpy()[:li.offsets[-1]], li.ids)

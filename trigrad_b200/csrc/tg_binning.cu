@@ -588,7 +588,9 @@ constexpr uint32_t kHole = 0xffffffffu;      // tile word of a pair that is not 
 __device__ __forceinline__ unsigned long long* slot_counter(const BinArgs& bin) {
     return reinterpret_cast<unsigned long long*>(bin.counters + 2);
 }
-constexpr int kBinQueue = 64 * kBinWarps;       // clip queue of a CTA
+// Clip queue of a CTA.  Twice as many took longer (1.3M triangles of a pixel 146 us against 143, 200k triangles 35.9 against 35.1,
+// 2M piled up the same), with the clips later and 1.5 KB more of shared memory in each of the eight CTAs; half as many 143, 35.7.
+constexpr int kBinQueue = 32 * kBinWarps;
 // Shared memory of a warp, in words: first the staging area of its records (pitch 5 quads for the 4 of a geometry
 // record, 7 for the 6 of half the warp's attribute records: 16-byte accesses of consecutive lanes then fall on different
 // banks), then, component-major, what the pairs need of its triangles: matrix 9, corners 6, depth plane 3, tile
