@@ -1216,7 +1216,8 @@ __device__ __forceinline__ void backward_one(const float* w, const AttrRec& a, c
 // of every slot.  Columns and not rows: a store then has the lanes in one column, 32 banks whatever their order, where rows, two
 // times sixteen of them as there was less room, took 72 passes through shared memory instead of 24 and were most of what the
 // kernel asked of L1, which it waits for where many triangles overlap (200k triangles, 1920x1080 154 -> 146 us; 1.3M
-// triangles of a pixel, the same image 111 -> 108; 2M piled up, 3840x2160 807 -> 722).
+// triangles of a pixel, the same image 111 -> 106; 2M piled up, 3840x2160 807 -> 706; the three vertices' ids on one or two
+// banks instead of three 146, 108, 715).
 // (Adding up to four neighbouring lanes with 42 shuffles and six vector reductions per run took as long as rows where a triangle
 // has one or two of the 32 fragments, and 17 % longer where a few triangles have them all: 2M overlapping triangles, 4K,
 // 944 us against 804.  Sums of four values per lane, for five triangles at a time, which leave as vector reductions: 185 against
@@ -1240,7 +1241,7 @@ __device__ __forceinline__ void emit_lanes(const Contrib& c, bool valid, int id,
     const unsigned ends = __reduce_or_sync(0xffffffffu, leads ? 1u << (incl - 1) : 0u);   // last row of every triangle
     float* table = reinterpret_cast<float*>(rows);
     const float* column = table + COLUMN * min(lane, 23);
-    const int* ids = reinterpret_cast<const int*>(table) + COLUMN * (min(lane, 23) | 7);
+    const int* ids = reinterpret_cast<const int*>(table) + COLUMN * (min(lane, 23) | 7) + (min(lane, 23) >> 3);    // on three banks
     const bool adds = lane < 24 && (lane & 7) != 7;
     if (valid) {
         float* at = table + place;
@@ -1248,7 +1249,7 @@ __device__ __forceinline__ void emit_lanes(const Contrib& c, bool valid, int id,
         for (int k = 0; k < 3; k++) {
 #pragma unroll
             for (int i = 0; i < 7; i++) at[COLUMN * (8 * k + i)] = c.v[k][i];
-            at[COLUMN * (8 * k + 7)] = __int_as_float(c.vid[k]);
+            at[COLUMN * (8 * k + 7) + k] = __int_as_float(c.vid[k]);
         }
     }
     __syncwarp();
