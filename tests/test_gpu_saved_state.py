@@ -156,3 +156,18 @@ def test_small_renders_keep_little_more_than_image_records_and_selection(call, t
 def _entries(v, i, c, o, width, height, tile):
     out = trigrad_b200.wrapper.forward_native(v.detach(), i, c.detach(), o.detach(), width, height, tile, tile, 1 / 256, False, True, 32)
     return out[3].numel()
+
+
+def test_a_backward_that_walks_the_lists_needs_them():
+    """With a selection the lists may not be there; the corrected gradients walk them all the same."""
+    from trigrad_b200 import _native as N
+    from trigrad_b200 import wrapper as Wr
+
+    i, (v, c, o) = _leaves()
+    out = N.host().forward(v.detach(), i, c.detach(), o.detach(), W, H, 16, 16, 1 / 256, False, True, 32, True, True, Wr.SELECTION_MAX_BYTES)
+    image, depth, ids, selection, layout, blob = *out[:2], out[3], out[8], out[10], out[11]
+    gi = torch.ones_like(image)
+    for kind in (Wr.GRADIENTS_REFERENCE, Wr.GRADIENTS_PACKED):
+        N.host().backward(kind, layout, image, depth, blob, None, selection, gi, None)
+    with pytest.raises(RuntimeError, match="tile lists"):
+        N.host().backward(Wr.GRADIENTS_CORRECTED, layout, image, depth, blob, None, selection, gi, None)

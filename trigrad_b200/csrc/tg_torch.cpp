@@ -348,7 +348,11 @@ struct L2Step {     // forward, loss and gradients in one call (tg_render_step_l
 
 // `opacities` undefined: packed inputs (indices [T,4], colors [V,4]).  Called without the interpreter lock.
 // `count`: whether the caller needs the number of list entries (otherwise Layout::K may be the room for them).
-enum class Count { kAlways, kUnlessSmall, kUnlessSmallKeepLists };      // the last one: and may keep the lists for a backward
+//   kAlways                it does
+//   kUnlessSmall           it needs neither it nor the lists: tile offsets and ids may be left unwritten
+//   kUnlessSmallKeepLists  it may walk the lists later, where there is no selection
+// Where the lists are left unwritten Saved::ids is undefined, and backward() refuses to walk them.
+enum class Count { kAlways, kUnlessSmall, kUnlessSmallKeepLists };
 ForwardOut forward(const Tensor& vertices_, const Tensor& indices_, const Tensor& colors_, const Tensor& opacities_,
                    const View& v, bool record_timing, bool save_selection, bool cull, int64_t selection_max_bytes, Count count,
                    const L2Step* step = nullptr) {
@@ -415,6 +419,7 @@ ForwardOut forward(const Tensor& vertices_, const Tensor& indices_, const Tensor
             std::copy(key, key + 4, state->ready);
             state->check_error_word(state->last_slot);       // of an earlier call that counted; may yet arrive
             s.l.K = cap;
+            if (lists_unused) s.ids = Tensor();
             return out;
         }
         s.l.K = (uint32_t)info[0];
@@ -445,6 +450,8 @@ void check_last_forward(const Where& w) {
 std::vector<Tensor> backward(Kind kind, const Saved& s, const Tensor& image, const Tensor& depthmap, Tensor gi, Tensor gd) {
     const Where w(image);
     check_last_forward(w);
+    TORCH_CHECK(s.ids.defined() || (s.selection.defined() && kind != Kind::kCorrected),
+                "this backward walks the tile lists, which the forward did not leave");
     const auto options = image.options().requires_grad(false);
     std::vector<Tensor> out;
     const View& v = s.l.v;
