@@ -320,7 +320,9 @@ int tg_blend_step_l2(const float* tri_geo, const float* tri_attr, const int32_t*
  *                TG_LISTS_UNUSED: the caller does not read `sorted_ids` and `offsets`, nor hands them to a backward that
  *                walks the lists (one without `selection`): they are left unwritten where a call has no need of them (today
  *                with TG_NO_COUNT, whose lists then lie with room for every triangle in each tile and are not moved
- *                together).  Both have to have their full size.
+ *                together).  Both have to have their full size.  info_host[1] of a call with TG_NO_COUNT then receives the
+ *                length of some list beyond TG_SHORT_LIST, not of the longest, from the compositing kernel: nothing but
+ *                that there is one is to be taken from it.
  */
 #define TG_NO_COUNT 32u
 #define TG_LISTS_UNUSED 64u
