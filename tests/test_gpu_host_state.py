@@ -305,12 +305,24 @@ def test_lists_that_are_not_moved_together(n, w, h, tile):
             trigrad_b200.wrapper.forward_native(*_stacked(150, w, h, 9), w, h, tile, tile, 1 / 256, False, True, 32)     # the next call counts
             want[name] = call()
             assert state.last_slot != state_before
-        for _ in range(65):
+        few, long_list = _stacked(3, w, h, 3), ctypes.c_uint32.from_address(state.long_row + 4)
+
+        def after_short_lists():
             with torch.no_grad():
-                trigrad_b200.render(*_stacked(3, w, h, 3), *size)
-        torch.cuda.current_stream().synchronize()
+                for _ in range(65):
+                    trigrad_b200.render(*few, *size)
+            torch.cuda.current_stream().synchronize()
+
+        after_short_lists()
         for name in ("look", "fit", "look", "lists", "look", "corrected", "fit", "look"):
+            if n > 128:
+                after_short_lists()                           # the call before met long lists
+            assert long_list.value == 0
+            before = state.last_slot
             got = calls[name]()
+            torch.cuda.current_stream().synchronize()
+            assert state.last_slot == before                  # went without the count
+            assert long_list.value == (n if n > 128 else 0)   # every list has all the triangles
             assert torch.equal(got[0], want[name][0])
             for a, b in zip(got[1:], want[name][1:]):
                 if name == "look":
