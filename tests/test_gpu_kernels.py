@@ -179,3 +179,29 @@ def test_keys_of_triangles_far_larger_than_the_image(scale, cull):
     out = Wr.forward_native(*map(Hh.cuda, (v, i, c, o)), W, H, tile, tile, 1 / 256, False, True, 32, cull_tiles=cull)
     assert np.array_equal(out[4].cpu().numpy(), li.offsets)
     assert np.array_equal(out[3].cpu().numpy()[:li.offsets[-1]], li.ids)
+
+
+@pytest.mark.parametrize("tile, across, down", [(16, 37, 4), (16, 149, 1), (8, 37, 16), (8, 593, 1), (4, 37, 32), (4, 1185, 1), (16, 1, 1)])
+@pytest.mark.parametrize("triangles", [40, 256, 257])
+def test_walked_lists_at_the_number_of_tiles_that_chooses_the_sums(tile, across, down, triangles):
+    """Eight warps on each of 148 multiprocessors and one tile more; the last column and row of tiles ragged."""
+    W, H, rng = tile * across - tile // 2, tile * down - 1, np.random.default_rng(triangles + across)
+    angle = rng.uniform(0, 2 * np.pi, (triangles, 1)) + np.arange(3) * (2 * np.pi / 3)
+    radius = np.where(np.arange(triangles) % 4 == 0, rng.uniform(0.02, 0.5, triangles), 4.0)[:, None]      # some small, most over all
+    centre = np.where(radius < 1, rng.uniform(-1, 1, (triangles, 2)), 0.0)
+    depth = rng.uniform(0.5, 10, (triangles, 1)) * np.ones(3)
+    v = np.stack([centre[:, :1] + radius * np.cos(angle), centre[:, 1:] + radius * np.sin(angle), depth, 1 / depth], 2)
+    v, i = v.reshape(-1, 4).astype(np.float32), np.arange(3 * triangles, dtype=np.int32).reshape(-1, 3)
+    c, o = rng.random((len(v), 3), dtype=np.float32), rng.uniform(0.01, 0.03, len(v)).astype(np.float32)
+    size = (W, H, tile, tile)
+    of = O.forward(v, i, c, o, *size, 1 / 256, True, 1000)
+    assert of.ends.min() >= 30
+    gi = rng.standard_normal((H, W, 4)).astype(np.float32)
+    gd = rng.standard_normal((H, W)).astype(np.float32)
+    for function, corrected in ((trigrad_b200.render, False), (trigrad_b200.render_corrected, True)):
+        og = O.backward(v, i, c, o, W, H, of, gi, gd, tile, tile, True, 1000, corrected=corrected)
+        leaves = [Hh.cuda(x).requires_grad_() for x in (v, c, o)]
+        image, depth = function(leaves[0], Hh.cuda(i), leaves[1], leaves[2], *size, max_layers=1000)
+        for a, b in zip(torch.autograd.grad((image, depth), leaves, (Hh.cuda(gi), Hh.cuda(gd))), og):
+            # as for the lists that stay in shared memory: a few hundred divisions by 1 - opacity, on both sides in 32 bits
+            assert Hh.rel_l2(a.cpu().numpy(), b) <= 2e-4

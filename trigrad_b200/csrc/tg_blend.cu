@@ -959,6 +959,23 @@ __device__ __forceinline__ void emit_uniform(const Contrib& c, bool has, float4*
     __syncwarp();
 }
 
+// The same for lanes with triangles of their own (`id`): pixels next to each other under large triangles mostly blend the
+// same triangle at the same place of their sequences.  All lanes must call.
+__device__ __forceinline__ void emit_groups(const Contrib& c, bool has, int id, float4* __restrict__ gpack) {
+    const unsigned peers = __match_any_sync(0xffffffffu, has ? id : -1 - (int)lane_id());
+    const bool big = has && __popc(peers) >= kGroupMin;
+    unsigned todo = __ballot_sync(0xffffffffu, big);
+#pragma unroll 1
+    for (int it = 0; it < 32 / kGroupMin && todo != 0; ++it) {
+        const int leader = __ffs(todo) - 1;
+        const unsigned group = __shfl_sync(0xffffffffu, peers, leader);
+        todo &= ~group;
+        reduce_group(c, (group >> lane_id()) & 1u, leader, gpack);
+    }
+    if (has && !big) emit_contrib(c, gpack);
+    __syncwarp();
+}
+
 struct BackwardIn {
     const float4* gimage;
     const float* gdepth;
@@ -1516,28 +1533,41 @@ __global__ void __launch_bounds__(MAXT, 4) blend_step_l2_kernel(BlendParams P, f
 // the gradients of the fragments found.  A warp's outputs leave as in the queued kernel, through a table of columns: its lanes
 // hold a handful of triangles each round, and a reduction by halves for each (100 instructions, a lane's own six vector reductions
 // where few lanes share one) took longer.  B200, corrected gradients, kernel: 3000 triangles about 90 layers deep, 637x421,
-// tiles of 16 307 -> 272 us, of 32 377 -> 318, of 8 349 -> 296 (with 256 records instead of 128 376: the shared memory of small
-// CTAs); 300 triangles, 480x360, at most 64 layers 104 -> 97; 100k small triangles in one or two layers 113 -> 114; 400
-// triangles, 200x150, a CTA per SM, so that what counts is how long a round takes 48 -> 52.  Bound by issue, 24 warps on an SM.
-template <bool SORT, int MAXT>
-constexpr int kListRecords = !SORT ? kChunk : MAXT <= 256 ? 2 * kChunk : 4 * kChunk;
+// tiles of 16 304 -> 270 us, of 32 368 -> 314, of 8 346 -> 291; 300 triangles, 480x360 102 -> 93; the reference's gradients 320 -> 270,
+// 354 -> 304, 358 -> 290, 105 -> 94.  Bound by issue, 24 warps on an SM.  Where a pixel has a layer or two the table is the dearer
+// one: 200k triangles, 1920x1080, 199 -> 205 (the reference's gradients 207 -> 205); 2000 light ones, the same image, 75 -> 79.  Both
+// ways in one kernel, chosen by the rounds of a batch, take 290 for the 270.
+// 128 records in tiles of up to 256 pixels, 256 in larger ones.  With 256 in tiles of 8 the shared memory of small CTAs costs more
+// than it gives, 291 -> 369; in tiles of 16, with a list of 33 records on average 93 -> 94, 71 231 -> 235, 142 270 -> 272, 192
+// 279 -> 276, 239 285 -> 278, 287 293 -> 283.
+// FEW: at most eight warps on an SM, where a round's latency counts and not its instructions: the lanes' own reductions, all the
+// registers a thread wants and 256 records.  4000 triangles, 160x160 (100 tiles of 16) 99 -> 80 us, with the reductions alone
+// 85; 3000, 96x96 90 -> 62; 400, 200x150 (130 tiles) 55 -> 51, in tiles of 8 (475 of two warps) 58 -> 43; 1500, 96x96 in tiles of 4
+// 74 -> 50.  With more warps the table is ahead or much as fast: 400, 304x200 (247 tiles, two to an SM, whose registers are for one
+// of FEW) 57 against 60, 200x200 in tiles of 8 (625, five) 60 against 61, the reference's gradients 58 against 56; and ahead
+// with tiles of more than 256 pixels, whose CTA has more warps by itself (1500, 160x160 in tiles of 32 177 against 203).
+constexpr int kFewWarps = 8;
+template <bool SORT, int MAXT, bool FEW>
+constexpr int kListRecords = !SORT ? kChunk : MAXT <= 256 && !FEW ? 2 * kChunk : 4 * kChunk;
 constexpr int kListColumn = 36, kListTable = 24 * kListColumn / 4;      // quads per warp
 constexpr size_t list_tables(int threads) { return sizeof(float4) * kListTable * (threads / 32); }
 // A round's contributions.  From 12 lanes on the table is cheaper than the lanes' own vector reductions, below it a little dearer
 // (100k small triangles in one or two layers 122 -> 114 us, deep stacks 1 % slower; 16 and 20 lanes: 300 triangles 95 -> 107, 119).
 constexpr int kTableMin = 12;
+template <bool FEW>
 __device__ __forceinline__ void emit_round(const Contrib& c, bool has, int id, float4* rows, float4* __restrict__ gpack) {
-    if (__popc(__ballot_sync(0xffffffffu, has)) >= kTableMin) emit_lanes<kListColumn>(c, has, id, rows, gpack);
+    if (FEW) emit_groups(c, has, id, gpack);
+    else if (__popc(__ballot_sync(0xffffffffu, has)) >= kTableMin) emit_lanes<kListColumn>(c, has, id, rows, gpack);
     else if (has) emit_contrib(c, gpack);
 }
-template <bool SORT, int MAXT>
-__global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (SORT ? 3 : 4) : 1) blend_backward_kernel(BlendParams P, BackwardIn in, float4* __restrict__ gpack) {
-    __shared__ float4 s_geo[kListRecords<SORT, MAXT> * kStagedQuads];
+template <bool SORT, int MAXT, bool FEW = false>
+__global__ void __launch_bounds__(MAXT, MAXT <= 256 && !FEW ? (SORT ? 3 : 4) : 1) blend_backward_kernel(BlendParams P, BackwardIn in, float4* __restrict__ gpack) {
+    __shared__ float4 s_geo[kListRecords<SORT, MAXT, FEW> * kStagedQuads];
     __shared__ int s_id[kChunk];
-    extern __shared__ float4 s_tables[];             // SORT: kListTable quads per warp
+    extern __shared__ float4 s_tables[];             // SORT and not FEW: kListTable quads per warp
     __shared__ __align__(16) float s_coord[MAXT <= 256 ? 260 : kMaxTileCoords];
     const TileCtx c = tile_context(P, s_coord);
-    const bool resident = SORT && c.end - c.start <= kListRecords<SORT, MAXT>;
+    const bool resident = SORT && c.end - c.start <= kListRecords<SORT, MAXT, FEW>;
     if (resident) stage_geo_async(P, c.start, c.end - c.start, s_geo);
     PixelGrad pg;
     BackState st;
@@ -1579,7 +1609,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (SORT ? 3 : 4) : 1) blend_
                     const AttrRec a = load_attr<true>(P.attr, id);
                     backward_one(w, a, b, c.px, c.py, pg, st, ct);
                 }
-                emit_round(ct, i >= 0, id, s_tables + kListTable * (threadIdx.x >> 5), gpack);
+                emit_round<FEW>(ct, i >= 0, id, s_tables + kListTable * (threadIdx.x >> 5), gpack);
             }
             if (go) {
                 if (n > 0) {
@@ -1679,15 +1709,15 @@ __device__ __forceinline__ void backward_one_prefix(const float* w, const AttrRe
     backward_outputs<true, false>(w, a, f, out);
 }
 
-template <bool SORT, int MAXT>
-__global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (SORT ? 3 : 4) : 1) blend_backward_corrected_kernel(BlendParams P, BackwardIn in,
+template <bool SORT, int MAXT, bool FEW = false>
+__global__ void __launch_bounds__(MAXT, MAXT <= 256 && !FEW ? (SORT ? 3 : 4) : 1) blend_backward_corrected_kernel(BlendParams P, BackwardIn in,
                                                                         float4* __restrict__ gpack) {
-    __shared__ float4 s_geo[kListRecords<SORT, MAXT> * kStagedQuads];
+    __shared__ float4 s_geo[kListRecords<SORT, MAXT, FEW> * kStagedQuads];
     __shared__ int s_id[kChunk];
-    extern __shared__ float4 s_tables[];             // SORT: kListTable quads per warp
+    extern __shared__ float4 s_tables[];             // SORT and not FEW: kListTable quads per warp
     __shared__ __align__(16) float s_coord[MAXT <= 256 ? 260 : kMaxTileCoords];
     const TileCtx c = tile_context(P, s_coord);
-    const bool resident = SORT && c.end - c.start <= kListRecords<SORT, MAXT>;
+    const bool resident = SORT && c.end - c.start <= kListRecords<SORT, MAXT, FEW>;
     if (resident) stage_geo_async(P, c.start, c.end - c.start, s_geo);
     PixelGrad pg;
     BackState unused;
@@ -1732,7 +1762,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? (SORT ? 3 : 4) : 1) blend_
                     const AttrRec a = load_attr<true>(P.attr, id);
                     backward_one_prefix(w, a, b, c.px, c.py, pg, fin, pf, ct);
                 }
-                emit_round(ct, i < n, id, s_tables + kListTable * (threadIdx.x >> 5), gpack);
+                emit_round<FEW>(ct, i < n, id, s_tables + kListTable * (threadIdx.x >> 5), gpack);
             }
             if (go) {
                 if (n > 0) {
@@ -1946,17 +1976,21 @@ size_t tg_backward_scratch_bytes(int V) { return (size_t)(V > 0 ? V : 0) * 32 + 
 template <bool CORRECTED>
 static int launch_list_kernel(const tg::BlendParams& P, const tg::BackwardIn& in, float4* gpack, int tiles, int threads, bool sort, cudaStream_t s) {
     const bool large = threads > 256;
+    const bool few = sort && !large && (tiles + 147) / 148 * (threads / 32) <= tg::kFewWarps;
     void (*kernel)(tg::BlendParams, tg::BackwardIn, float4*);
     if (CORRECTED)
         kernel = large ? (sort ? tg::blend_backward_corrected_kernel<true, 1024> : tg::blend_backward_corrected_kernel<false, 1024>)
+                 : few ? tg::blend_backward_corrected_kernel<true, 256, true>
                        : (sort ? tg::blend_backward_corrected_kernel<true, 256> : tg::blend_backward_corrected_kernel<false, 256>);
     else
         kernel = large ? (sort ? tg::blend_backward_kernel<true, 1024> : tg::blend_backward_kernel<false, 1024>)
+                 : few ? tg::blend_backward_kernel<true, 256, true>
                        : (sort ? tg::blend_backward_kernel<true, 256> : tg::blend_backward_kernel<false, 256>);
+    const bool tables = sort && !few;
     static tg_host::SmemAllowed allowed[2];
-    if (sort)
+    if (tables)
         if (int st = tg_host::allow_smem((const void*)kernel, tg::list_tables(large ? 1024 : 256), allowed[large])) return st;
-    kernel<<<tiles, threads, sort ? tg::list_tables(threads) : 0, s>>>(P, in, gpack);
+    kernel<<<tiles, threads, tables ? tg::list_tables(threads) : 0, s>>>(P, in, gpack);
     return TG_OK;
 }
 extern "C" {
