@@ -1239,8 +1239,9 @@ __device__ __forceinline__ void backward_one(const float* w, const AttrRec& a, c
 // has one or two of the 32 fragments, and 17 % longer where a few triangles have them all: 2M overlapping triangles, 4K,
 // 944 us against 804.  Sums of four values per lane, for five triangles at a time, which leave as vector reductions: 185 against
 // 154 and 981 against 807 - reductions of 16 bytes to one 32-byte slot are not merged.)
-// `rows`: 24 * COLUMN words of this warp.  COLUMN: 36, or 34, which is read two words at a time.
-template <int COLUMN>
+// `rows`: 24 * COLUMN words of this warp.  COLUMN: 36, or 34, which is read two words at a time.  WHOLE: where all lanes have
+// one and the same triangle the columns are read at once.
+template <int COLUMN, bool WHOLE = false>
 __device__ __forceinline__ void emit_lanes(const Contrib& c, bool valid, int id, float4* rows, float4* __restrict__ gpack) {
     const int lane = lane_id();
     const unsigned peers = __match_any_sync(0xffffffffu, valid ? id : -1 - lane);      // distinct negatives never match
@@ -1260,6 +1261,7 @@ __device__ __forceinline__ void emit_lanes(const Contrib& c, bool valid, int id,
     const float* column = table + COLUMN * min(lane, 23);
     const int* ids = reinterpret_cast<const int*>(table) + COLUMN * (min(lane, 23) | 7) + (min(lane, 23) >> 3);    // on three banks
     const bool adds = lane < 24 && (lane & 7) != 7;
+    static_assert(!WHOLE || COLUMN % 4 == 0, "read four words at a time");
     if (valid) {
         float* at = table + place;
 #pragma unroll
@@ -1270,6 +1272,19 @@ __device__ __forceinline__ void emit_lanes(const Contrib& c, bool valid, int id,
         }
     }
     __syncwarp();
+    if (WHOLE && ends == 0x80000000u) {
+        float4 even = make_float4(0.f, 0.f, 0.f, 0.f), odd = even;
+#pragma unroll
+        for (int j = 0; j < 32; j += 8) {
+            const float4 q = *reinterpret_cast<const float4*>(column + j), r = *reinterpret_cast<const float4*>(column + j + 4);
+            even.x += q.x; even.y += q.y; even.z += q.z; even.w += q.w;
+            odd.x += r.x; odd.y += r.y; odd.z += r.z; odd.w += r.w;
+        }
+        if (adds) atomicAdd(reinterpret_cast<float*>(gpack + 2 * (size_t)ids[31]) + (lane & 7),
+                            ((even.x + odd.x) + (even.y + odd.y)) + ((even.z + odd.z) + (even.w + odd.w)));
+        __syncwarp();
+        return;
+    }
     float sum = 0.f;
 #pragma unroll 1
     for (int j = 0; j < total; j += 4) {
@@ -1533,10 +1548,13 @@ __global__ void __launch_bounds__(MAXT, 4) blend_step_l2_kernel(BlendParams P, f
 // the gradients of the fragments found.  A warp's outputs leave as in the queued kernel, through a table of columns: its lanes
 // hold a handful of triangles each round, and a reduction by halves for each (100 instructions, a lane's own six vector reductions
 // where few lanes share one) took longer.  B200, corrected gradients, kernel: 3000 triangles about 90 layers deep, 637x421,
-// tiles of 16 304 -> 270 us, of 32 368 -> 314, of 8 346 -> 291; 300 triangles, 480x360 102 -> 93; the reference's gradients 320 -> 270,
-// 354 -> 304, 358 -> 290, 105 -> 94.  Bound by issue, 24 warps on an SM.  Where a pixel has a layer or two the table is the dearer
-// one: 200k triangles, 1920x1080, 199 -> 205 (the reference's gradients 207 -> 205); 2000 light ones, the same image, 75 -> 79.  Both
-// ways in one kernel, chosen by the rounds of a batch, take 290 for the 270.
+// tiles of 16 306 -> 266 us, of 32 367 -> 299, of 8 346 -> 288; 300 triangles, 480x360 102 -> 90; the reference's gradients 321 -> 267,
+// 354 -> 285, 358 -> 287, 105 -> 92.  (Before the columns of a round with one triangle in all lanes were read at once, the table
+// took 270, 314, 292, 94, 270, 304, 290, 95; 700 large triangles, 1280x720, 333, now 316, the reductions by halves 327.)  Bound
+// by issue, 24 warps on an SM.  Where a pixel has a layer or two the table is the dearer one, corrected gradients above all: 200k
+// triangles, 1920x1080, 199 -> 205 (the reference's 207 -> 205), 2000, the same image, 75 -> 79 (84 -> 79), in tiles of 32 124 -> 128
+// (110 -> 113).  Not cured: both ways in one kernel, chosen by the number of rounds, take 290 for the 270, with the shorter one out
+// of line all take longer; the groups of 6 or 8 lanes and more through the table instead of 12, 214 and 211 for the 205.
 // 128 records in tiles of up to 256 pixels, 256 in larger ones.  With 256 in tiles of 8 the shared memory of small CTAs costs more
 // than it gives, 291 -> 369; in tiles of 16, with a list of 33 records on average 93 -> 94, 71 231 -> 235, 142 270 -> 272, 192
 // 279 -> 276, 239 285 -> 278, 287 293 -> 283.
@@ -1557,7 +1575,7 @@ constexpr int kTableMin = 12;
 template <bool FEW>
 __device__ __forceinline__ void emit_round(const Contrib& c, bool has, int id, float4* rows, float4* __restrict__ gpack) {
     if (FEW) emit_groups(c, has, id, gpack);
-    else if (__popc(__ballot_sync(0xffffffffu, has)) >= kTableMin) emit_lanes<kListColumn>(c, has, id, rows, gpack);
+    else if (__popc(__ballot_sync(0xffffffffu, has)) >= kTableMin) emit_lanes<kListColumn, true>(c, has, id, rows, gpack);
     else if (has) emit_contrib(c, gpack);
 }
 template <bool SORT, int MAXT, bool FEW = false>
