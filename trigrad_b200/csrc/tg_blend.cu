@@ -1039,8 +1039,8 @@ __device__ __forceinline__ int load_pixel_state(const TileCtx& c, const BlendPar
 // gradients of the fragment's interpolations; these go into a queue in shared memory; part B (the
 // expensive barycentric partials and the 21 per-vertex outputs) pops 32 queued fragments at a time and
 // so runs with full warps.  A warp whose lanes are busy anyway (deep overlap, or one opaque layer everywhere) skips the
-// queue.  (200k triangles, full HD: 153 us with L1 75 % busy and 64 % of the issue slots used; bound by the latency of the
-// gathers, fifteen of 16 bytes per fragment, and by L1 together, half of whose work is shared memory's.)
+// queue.  (200k triangles, full HD: 146 us with L1 75 % busy and 63 % of the issue slots used; bound by the latency of the
+// gathers, fourteen of 16 bytes per fragment, and by L1 together, which does shared memory's work too.)
 // DEPTH = false (everywhere below): no gradient flows into the depth map, the terms that it feeds are left out.
 struct QueuedFragment {
     float px, py;
@@ -1352,9 +1352,10 @@ __device__ __noinline__ void backward_rounds_direct(const BlendParams& P, float 
 
 // A CTA takes a block of kQueueCols x kQueueRows pixels, a warp 8x4 of them, and then PASSES - 1 blocks more, each the same
 // number of rows further down; the queues go on through all of them.  What a warp does for 32 pixels of a layer or two is
-// short against the start of a CTA and ends in a queue that is not full; against that, the last CTAs end later.  One, two,
-// three, four, six passes, a fused step, B200, kernel as a trace has it: 200k triangles, 1920x1080 164, 154, 153, 154, 158 us; 1.3M
-// triangles of a pixel, the same image 111, 111, 116, 119, 136; 2M piled up, 3840x2160 786, 814, 798, 799, 824.  So three, and by
+// short against the start of a CTA and ends in a queue that is not full; against that, the last CTAs end later.  One and three
+// passes, a fused step, B200, kernel as a trace has it: 200k triangles, 1920x1080 159, 146 us; 1.3M triangles of a pixel, the same
+// image 107, 106; 2M piled up, 3840x2160 708, 699.  (With sums by rows instead of columns, one, two, three, four, six passes took 164,
+// 154, 153, 154, 158; 111, 111, 116, 119, 136; 786, 814, 798, 799, 824, so three was the number.)  So three, and by
 // the size of the image (backward_impl).  (Blocks next to each other: 3840x2160 850 with two, as the deep blocks all lie in
 // the same CTAs and the last of them run alone.  In a loop of a number of passes known at run time the compiler spills.)
 constexpr int kQueueCols = 16, kQueueRows = 8;
@@ -1449,9 +1450,9 @@ __global__ void __launch_bounds__(kQueueCols * kQueueRows, DEPTH ? 7 : 8) blend_
 // image; the per-vertex outputs go through the per-warp queue as in blend_backward_queued_kernel.
 // Slower than the two kernels in most places by now, as it has none of their staging ahead of the pixel set-up, streamed
 // lists and dependent launches, and its half for the forward runs with the registers of both (a step, B200: 200k triangles,
-// full HD 301 us in two kernels against 330 in one; 2M triangles, 4K 1948 against 2153; 10k, 512x512 55 against 62; four
-// streams of views, full HD 257 against 293 per view).  As fast where triangles are a pixel each and a pixel blends one
-// fragment or none (1.3M triangles, full HD 505 against 503).  Used on request only.
+// full HD 300 us in two kernels against 335 in one; 2M triangles, 4K 1914 against 2165; 10k, 512x512 54 against 59; four
+// streams of views, full HD 250 against 278 per view).  Nearly as fast where triangles are a pixel each and a pixel blends one
+// fragment or none (1.3M triangles, full HD 502 against 508).  Used on request only.
 template <int MAXT>
 __global__ void __launch_bounds__(MAXT, 4) blend_step_l2_kernel(BlendParams P, float4* __restrict__ image,
                                                                 float* __restrict__ depthmap, float* __restrict__ final_w,
@@ -2059,13 +2060,13 @@ static int backward_impl(const float* tri_geo, const float* tri_attr, const int3
         Q.offsets = nullptr; Q.ids = nullptr; Q.order = nullptr;
         // Three passes from the numbers of waves on that were measured to pay, B200, whole calls, one pass -> three, us.
         // No depth gradient, 8 CTAs per SM (fused steps; the same renders through autograd are alike): 2.0 waves (1280x720) 1.3M
-        // triangles of a pixel 480 -> 486, 89k random triangles 153 -> 157, 100k piled up in the middle 241 -> 274; 3.2 (1600x900)
-        // 492 -> 497, 221 -> 218, 258 -> 260; 3.8 (1760x990) 474 -> 477, 268 -> 259, 274 -> 275; 4.6 (1920x1080) 488 -> 491, 310 ->
-        // 304, 290 -> 291; 8.1 (2560x1440) 590 -> 587, 530 -> 508, 381 -> 384; 18 (3840x2160) 879 -> 863, 1162 -> 1102, 718 -> 698.
-        // With one, 7 per SM (through autograd): 3.6 waves (1600x900) 494 -> 495, 237 -> 236, 267 -> 275; 5.2 (1920x1080) 492 ->
-        // 493, 333 -> 331, 301 -> 311; 9.3 (2560x1440) 597 -> 594, 565 -> 551, 402 -> 418; 21 (3840x2160) 892 -> 879, 1241 -> 1196,
-        // 758 -> 761; 100k light triangles spread evenly 179 -> 172, 233 -> 223, 363 -> 337, 709 -> 646.  Triangles piled up in the
-        // middle of the image lose with a depth gradient, up to 5 % of the call, and gain only beyond 3840x2160.
+        // triangles of a pixel 489 -> 494, 89k random triangles 156 -> 158, 100k piled up in the middle 362 -> 415; 3.2 (1600x900)
+        // 502 -> 504, 225 -> 218, 364 -> 390; 3.8 (1760x990) 486 -> 487, 271 -> 257, 376 -> 387; 4.6 (1920x1080) 499 -> 500, 313 ->
+        // 300, 384 -> 384; 8.1 (2560x1440) 599 -> 595, 530 -> 498, 425 -> 423; 18 (3840x2160) 878 -> 862, 1161 -> 1080, 686 -> 665.
+        // With one, 7 per SM (through autograd; random, piled up, and 100k light triangles spread evenly): 3.6 waves (1600x900) 228 ->
+        // 221, 366 -> 372, 170 -> 160; 5.2 (1920x1080) 319 -> 308, 381 -> 381, 222 -> 209; 9.3 (2560x1440) 543 -> 513, 434 -> 436,
+        // 346 -> 313; 21 (3840x2160) 1193 -> 1115, 708 -> 688, 670 -> 594.  Between 3.6 and 5.2 one stands against the other.  Triangles piled up in the middle of a small image
+        // lose: the passes of their CTAs hold what one pass spreads over all.
         constexpr int kPasses = 3;
         const int strips = (H + tg::kQueueRows - 1) / tg::kQueueRows;
         const int64_t wanted = grad_depthmap ? kPasses * 5 * 7 * 148 : kPasses * 7 * 8 * 148 / 2;      // 5 waves, 3.5 waves

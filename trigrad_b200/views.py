@@ -114,8 +114,8 @@ def l2_view_step(vertices: torch.Tensor, indices: torch.Tensor, colors: torch.Te
                  packed: "PackedGradients | None" = None, cull_tiles: bool = True) -> torch.Tensor:
     """One view of a multi-view optimisation step without autograd: forward, then the backward of
     ``mean((image - target)**2)`` fused into the gradient kernel.  With ``one_kernel`` (tiles of up to 256 pixels)
-    both directions run in one compositing kernel: as fast on fine meshes whose triangles are about a pixel large,
-    10 to 15 % slower on everything else measured (B200; larger triangles, small images, several streams of views).
+    both directions run in one compositing kernel: 1 % slower on fine meshes whose triangles are about a pixel large,
+    8 to 13 % on everything else measured (B200; larger triangles, small images, several streams of views).
 
     Adds the view's gradients to ``grad_vertices [V,4]`` (render-space x, y, z, w), ``grad_colors [V,3]``,
     ``grad_opacities [V]`` and its loss to the 0-d float32 tensor ``loss`` - no gradient image, no per-view
